@@ -30,6 +30,7 @@
 #include "dsk_mega.cuh"
 #include "dsk_hybrid.cuh"
 #include "dsk_linattn.cuh"
+#include "dsk_tc5.cuh"
 
 using namespace dsk;
 

@@ -284,18 +284,37 @@ struct GemmP {
   const void *sW1, *sW2;   // [sN][sK], packed
   const float* As;
   float* Cs;
+  // gemm_tc5 only.  n_expert: experts behind W (tile lists);  A16: the activations as packed bf16 rows in the product's row order (null: rounded
+  // from A by a pass of its own);  C16: results go there as packed bf16 rows in the product's row order instead of to C
+  int n_expert;
+  const __nv_bfloat16* A16;
+  __nv_bfloat16* C16;
 };
+
+// the epilogues that join two matrices' results, and those that are a function of one result and its column
+template <int EPI>
+__device__ __forceinline__ float dual_value(const GemmP& P, float v, float v2) {
+  if (EPI == HEPI_GEGLU) return gelu_tanh_f(v) * v2;
+  if (EPI == HEPI_SWIGLU) return silu_f(v) * v2;
+  const float g = fminf(v, P.lim), u = fminf(fmaxf(v2, -P.lim), P.lim);   // HEPI_GLU
+  return g * sigmoid_f(1.702f * g) * (u + 1.f);
+}
+template <int EPI>
+__device__ __forceinline__ float epi_value(const GemmP& P, int n, float v) {   // (joined results come as they are)
+  if (epi_dual(EPI)) return v;
+  if (P.bias) v += P.bias[n];
+  if (EPI == HEPI_XIELU) return v > 0.f ? fmaf(P.act_a * v, v, 0.5f * v) : fmaf(P.act_b, expm1f(v) - v, 0.5f * v);
+  if (EPI == HEPI_RELU2) { const float r = fmaxf(v, 0.f); return r * r; }
+  return P.alpha * v;
+}
 
 template <typename WT, int EPI>
 __device__ __forceinline__ void gemm_epilogue(const GemmP& P, float* __restrict__ crow, int cr, int n, float v, float v2) {
+  if (EPI == HEPI_STORE || EPI == HEPI_XIELU || EPI == HEPI_RELU2) { crow[n] = epi_value<EPI>(P, n, v); return; }
   if (P.bias) v += P.bias[n];
-  if (EPI == HEPI_STORE) crow[n] = P.alpha * v;
-  else if (EPI == HEPI_ADD) crow[n] += P.alpha * v;
-  else if (EPI == HEPI_XIELU) crow[n] = v > 0.f ? fmaf(P.act_a * v, v, 0.5f * v) : fmaf(P.act_b, expm1f(v) - v, 0.5f * v);
-  else if (EPI == HEPI_GEGLU) crow[n] = gelu_tanh_f(v) * v2;
-  else if (EPI == HEPI_SWIGLU) crow[n] = silu_f(v) * v2;
+  if (EPI == HEPI_ADD) crow[n] += P.alpha * v;
+  else if (epi_dual(EPI)) crow[n] = dual_value<EPI>(P, v, v2);
   else if (EPI == HEPI_SIGMUL) crow[n] *= sigmoid_f(v);
-  else if (EPI == HEPI_RELU2) { const float r = fmaxf(v, 0.f); crow[n] = r * r; }
   else if (EPI == HEPI_SILU_SIG) crow[n] = n < P.aux_off ? silu_f(v) : sigmoid_f(v);
   else if (EPI == HEPI_SOFTCAP) crow[n] = P.lim * tanhf(P.alpha * v / P.lim);
   else if (EPI == HEPI_LINGATE) {
@@ -304,10 +323,7 @@ __device__ __forceinline__ void gemm_epilogue(const GemmP& P, float* __restrict_
     else if (n < 2 * hn) { const float lo = reinterpret_cast<const float*>(P.aux)[n - hn]; crow[n] = fmaf(1.f - lo, sigmoid_f(v), lo); }
     else crow[n] = v;
   }
-  else if (EPI == HEPI_GLU) {
-    const float g = fminf(v, P.lim), u = fminf(fmaxf(v2, -P.lim), P.lim);
-    crow[n] = g * sigmoid_f(1.702f * g) * (u + 1.f);
-  } else {
+  else {
     const WT* aux = reinterpret_cast<const WT*>(P.aux);
     crow[n] = gelu_tanh_f(v) * to_f<WT>(aux[(size_t)P.aux_row[cr] * P.aux_ld + P.aux_off + n]);
   }

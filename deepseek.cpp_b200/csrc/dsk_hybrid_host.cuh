@@ -157,6 +157,11 @@ struct State {
   int* d_prev = nullptr;                     // the sequence's last token (bigram embedding)
   float *x = nullptr, *h = nullptr, *b0 = nullptr, *b1 = nullptr, *b2 = nullptr, *b3 = nullptr, *wgt = nullptr, *logits = nullptr;
   int *h_tok = nullptr, *h_want = nullptr;   // pinned staging of a chunk's token ids / wanted rows
+  // bf16 products of portions: activations rounded for the product that follows, hidden rows of a feed-forward, and a host word that a wait
+  // which gave up sets
+  __nv_bfloat16 *a16 = nullptr, *hid16 = nullptr;
+  size_t a16_elems = 0, hid16_elems = 0;
+  int* h_err = nullptr;
   std::vector<void*> allocs;
   // side-by-side mixers run on two streams, forked and joined by events
   cudaStream_t side = nullptr;
@@ -377,6 +382,10 @@ static void set_kernel_attrs() {
   DSK_LSCAN_ATTR(8, 1, 2); DSK_LSCAN_ATTR(16, 1, 2); DSK_LSCAN_ATTR(32, 1, 2); DSK_LSCAN_ATTR(8, 1, 4); DSK_LSCAN_ATTR(16, 1, 4); DSK_LSCAN_ATTR(32, 1, 4); DSK_LSCAN_ATTR(32, 2, 4);
 #undef DSK_LSCAN_ATTR
   cudaFuncSetAttribute(gemm_mma<HEPI_SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMmaSmem);
+#define DSK_TC5_ATTR(E) cudaFuncSetAttribute(gemm_tc5<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem)
+  DSK_TC5_ATTR(HEPI_STORE); DSK_TC5_ATTR(HEPI_ADD); DSK_TC5_ATTR(HEPI_GLU); DSK_TC5_ATTR(HEPI_XIELU); DSK_TC5_ATTR(HEPI_GEGLU); DSK_TC5_ATTR(HEPI_SIGMUL);
+  DSK_TC5_ATTR(HEPI_RELU2); DSK_TC5_ATTR(HEPI_LINGATE); DSK_TC5_ATTR(HEPI_SILU_SIG); DSK_TC5_ATTR(HEPI_SOFTCAP); DSK_TC5_ATTR(HEPI_SWIGLU); DSK_TC5_ATTR(HEPI_GELU_MUL);
+#undef DSK_TC5_ATTR
   cudaFuncSetAttribute(gqa_attn, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(mix_heads, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   done = true;
@@ -1235,6 +1244,11 @@ static dsk_state* state_create(dsk_model* m) {
     mx1 = std::max<size_t>(mx1, c.side_dim);
   }
   S->max_tiles = (int)(Tc * mxTop / 64 + mxE + 1);
+  size_t mxHid = 0, mxRouted = 0;   // hidden rows of a feed-forward per token; inputs of routed rows per token
+  for (const HLayer& L : M->L) {
+    if (L.sp.ff_kind == DSK_FF_MOE) { mxHid = std::max<size_t>(mxHid, (size_t)L.sp.ff_top * L.sp.ff_hidden + L.sp.ff_shared); mxRouted = std::max<size_t>(mxRouted, (size_t)L.sp.ff_top * c.dim); }
+    if (L.sp.ff_kind == DSK_FF_DENSE) mxHid = std::max<size_t>(mxHid, L.sp.ff_hidden);
+  }
   int rc = 0;
   size_t mxPart = 0;
   for (const HLayer& L : M->L) {
@@ -1288,6 +1302,16 @@ static dsk_state* state_create(dsk_model* m) {
   rc |= salloc(S, (void**)&S->d_tiles, (size_t)S->max_tiles * sizeof(int4)) | salloc(S, (void**)&S->d_ntiles, 16);
   rc |= salloc(S, (void**)&S->d_tok, Tc * 4) | salloc(S, (void**)&S->d_want, Tc * 4) | salloc(S, (void**)&S->d_ctl, 16);
   S->head_rows = (int)std::min<size_t>(Tc, 256);
+  if (c.quant == DSK_BF16 && Tc > 4) {
+    // a product's input is one of b0 .. b3, a row of 2 x width values (loop products), or latents of the visible keys
+    size_t rank = 0;
+    for (const HLayer& L : M->L) rank = std::max<size_t>(rank, has_attn(L.sp) && L.sp.mixer != DSK_MIX_GQA ? L.sp.att_kv_rank : 0);
+    S->a16_elems = std::max(Tc * std::max({mx0, mx1, mx2, mx3, (size_t)2 * c.dim, mxRouted}), (size_t)S->prefill_keys * rank);
+    S->hid16_elems = Tc * mxHid;
+    rc |= salloc(S, (void**)&S->a16, S->a16_elems * 2) | salloc(S, (void**)&S->hid16, S->hid16_elems * 2);
+  }
+  if (cudaHostAlloc((void**)&S->h_err, sizeof(int), cudaHostAllocMapped) != cudaSuccess) { fail(-2, "pinned allocation failed"); return nullptr; }
+  *S->h_err = 0;
   rc |= salloc(S, (void**)&S->logits, (size_t)S->head_rows * c.vocab_size * 4);
   if (rc) { fail(-2, "state allocation failed"); return nullptr; }
   if (cudaMallocHost((void**)&S->h_tok, Tc * 4) != cudaSuccess || cudaMallocHost((void**)&S->h_want, Tc * 4) != cudaSuccess) { fail(-2, "pinned allocation failed"); return nullptr; }
@@ -1302,7 +1326,7 @@ static void state_free(dsk_state* s) {
   if (S->side) { cudaStreamSynchronize(S->side); cudaStreamDestroy(S->side); cudaEventDestroy(S->ev_fork); cudaEventDestroy(S->ev_join); }
   for (cudaEvent_t e : S->tl_events) cudaEventDestroy(e);
   for (void* p : S->allocs) cudaFree(p);
-  cudaFreeHost(S->h_tok); cudaFreeHost(S->h_want);
+  cudaFreeHost(S->h_tok); cudaFreeHost(S->h_want); cudaFreeHost(S->h_err);
   delete S;
   s->hy = nullptr;
 }
@@ -1357,6 +1381,72 @@ static void launch_gemm_mma(int epi, const GemmP& P, int Z, int tile_cap, cudaSt
     case HEPI_SWIGLU: gemm_mma<HEPI_SWIGLU><<<grid, 256, kMmaSmem, st>>>(P); break;
     default: gemm_mma<HEPI_GELU_MUL><<<grid, 256, kMmaSmem, st>>>(P); break;
   }
+}
+
+// ---- portions on the tensor cores (gemm_tc5) ----
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
+                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+static EncodeTiledFn encode_tiled() {
+  static EncodeTiledFn fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) p = nullptr;
+    return (EncodeTiledFn)p;
+  }();
+  return fn;
+}
+// bf16 rows x cols matrix of pitch ld, copied in boxes of box_rows x 64 (elements past its edges read as zeros)
+static bool tile_map(CUtensorMap* m, const void* p, long long rows, long long cols, long long ld, int box_rows) {
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)ld * 2};
+  const cuuint32_t box[2] = {(cuuint32_t)kTcDepth, (cuuint32_t)box_rows}, one[2] = {1, 1};
+  return encode_tiled()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(p), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// Whether a product of more than four rows runs on gemm_tc5: bf16 matrices whose rows TMA can address (16-byte base and pitch), one batch,
+// and room for the rounded activations.  gemm_mma takes the others (odd sizes, per-head batches).
+static bool tc_ok(const State* S, bool bf16, int epi, const GemmP& P, int Z) {
+  auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  if (!bf16 || Z != 1 || P.z_expert || (!P.tiles && (P.M <= 4 || P.N <= 96)) || !encode_tiled()) return false;
+  if (P.K % 8 || P.ldw % 8 || !al(P.W) || (epi_dual(epi) && (!al(P.W2) || P.bias))) return false;
+  if (P.tiles && P.sW % P.ldw) return false;
+  return P.A16 || (size_t)P.M * P.K <= S->a16_elems;
+}
+static void launch_tc5(State* S, int epi, const GemmP& P, int tile_cap, cudaStream_t st) {
+  const __nv_bfloat16* A16 = P.A16;
+  if (!A16) {
+    const int vec = P.lda % 4 == 0 && (reinterpret_cast<uintptr_t>(P.A) & 15) == 0;
+    const long long n = (long long)P.M * (P.K / 8);
+    bf16_rows<<<(unsigned)std::min<long long>((n + 255) / 256, 148 * 8), 256, 0, st>>>(P.A, P.lda, P.a_map, P.a_div, S->a16, P.M, P.K, vec);
+    S->launches++;
+    A16 = S->a16;
+  }
+  // column tile: rounds of the grid times (columns + what a slice of the activations costs, about 64 columns)
+  const bool dual = epi_dual(epi);
+  const int mt = P.tiles ? tile_cap : (P.M + kTcRows - 1) / kTcRows;
+  TcP T{};
+  long long best = -1, grid = 1;
+  for (int bn = 256; bn >= 32; bn /= 2) {
+    if (dual && bn < 64) break;
+    const int cols = dual ? bn / 2 : bn;
+    const long long tiles = (long long)mt * ((P.N + cols - 1) / cols), cost = (tiles + 147) / 148 * (bn + 64);
+    if (best < 0 || cost < best) { best = cost; T.bn = bn; grid = std::min<long long>(tiles, 148); }
+  }
+  T.stages = std::min(kTcMaxStages, kTcRing / ((kTcRows + T.bn) * kTcDepth * 2));
+  T.n_mt = mt; T.rows_per_expert = P.tiles ? (int)(P.sW / P.ldw) : 0;
+  T.C16 = P.C16; T.ldc16 = P.N; T.err = S->h_err;
+  const int brows = dual ? T.bn / 2 : T.bn;
+  const long long wrows = P.tiles ? (long long)T.rows_per_expert * P.n_expert : P.N;
+  CUtensorMap mA, mB, mB2;
+  if (!tile_map(&mA, A16, P.M, P.K, P.K, kTcRows) || !tile_map(&mB, P.W, wrows, P.K, P.ldw, brows) || !tile_map(&mB2, dual ? P.W2 : P.W, wrows, P.K, P.ldw, brows)) {
+    *S->h_err = 2;
+    return;
+  }
+#define DSK_TC5(E) case E: gemm_tc5<E><<<(unsigned)grid, kTcThreads, kTcSmem, st>>>(P, T, mA, mB, mB2); break
+  switch (epi) {
+    DSK_TC5(HEPI_STORE); DSK_TC5(HEPI_ADD); DSK_TC5(HEPI_GLU); DSK_TC5(HEPI_XIELU); DSK_TC5(HEPI_GEGLU); DSK_TC5(HEPI_SIGMUL);
+    DSK_TC5(HEPI_RELU2); DSK_TC5(HEPI_LINGATE); DSK_TC5(HEPI_SILU_SIG); DSK_TC5(HEPI_SOFTCAP); DSK_TC5(HEPI_SWIGLU); DSK_TC5(HEPI_GELU_MUL);
+  }
+#undef DSK_TC5
 }
 
 template <typename WT>
@@ -1427,10 +1517,22 @@ static void linear(State* S, bool bf16, int epi, const GemmP& P, int Z, cudaStre
     S->launches++;
     return;
   }
-  if (bf16 && !small) launch_gemm_mma(epi, P, Z, tile_cap, st);
+  if (tc_ok(S, bf16, epi, P, Z)) launch_tc5(S, epi, P, tile_cap, st);
+  else if (bf16 && !small) launch_gemm_mma(epi, P, Z, tile_cap, st);
   else if (bf16) launch_gemm_t<__nv_bfloat16>(epi, P, Z, small, tile_cap, st);
   else launch_gemm_t<float>(epi, P, Z, small, tile_cap, st);
   S->launches++;
+}
+
+// A feed-forward whose two products both run on gemm_tc5 keeps its hidden rows in bf16, in the row order of the products (the second one
+// would round them anyway).
+static void hidden16(State* S, bool bf16, int epi_up, GemmP& up, int epi_down, GemmP& down, __nv_bfloat16* buf) {
+  if (!S->hid16 || (reinterpret_cast<uintptr_t>(buf) & 15) || !tc_ok(S, bf16, epi_up, up, 1)) return;
+  GemmP d = down;
+  d.A16 = buf;
+  if (!tc_ok(S, bf16, epi_down, d, 1)) return;
+  up.C16 = buf;
+  down.A16 = buf;
 }
 
 static void launch_scan(const dsk_layer_spec& sp, const float* proj, int ld_proj, const float* xbc, int ld_xbc, const HLayer& L,
@@ -2077,20 +2179,23 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       const int ff = sp.ff_hidden;
       GemmP U = gp(hin, W, L.gate_d.p, W, S->b2, ff, T, ff, W);
       U.W2 = L.up.p; U.lim = sp.ff_limit;
-      linear(S, bf, sp.ff_act == DSK_ACT_GLU_CLAMPED ? HEPI_GLU : sp.ff_act == DSK_ACT_SWIGLU ? HEPI_SWIGLU : HEPI_GEGLU, U, 1, st);
-      MK("ff.up");
       GemmP Dn = gp(S->b2, ff, L.down.p, ff, sink.C, W, T, W, ff);
       Dn.alpha = sink.alpha;
+      const int act = sp.ff_act == DSK_ACT_GLU_CLAMPED ? HEPI_GLU : sp.ff_act == DSK_ACT_SWIGLU ? HEPI_SWIGLU : HEPI_GEGLU;
+      hidden16(S, bf, act, U, sink.epi, Dn, S->hid16);
+      linear(S, bf, act, U, 1, st);
+      MK("ff.up");
       linear(S, bf, sink.epi, Dn, 1, st);
       MK("ff.down");
     } else if (sp.ff_kind == DSK_FF_DENSE) {
       const int ff = sp.ff_hidden;
       GemmP U = gp(hin, W, L.up.p, W, S->b2, ff, T, ff, W);
       U.bias = L.up_b; U.act_a = L.act_a; U.act_b = L.act_b;
-      linear(S, bf, HEPI_XIELU, U, 1, st);
-      MK("ff.up");
       GemmP Dn = gp(S->b2, ff, L.down.p, ff, sink.C, W, T, W, ff);
       Dn.bias = L.down_b; Dn.alpha = sink.alpha;
+      hidden16(S, bf, HEPI_XIELU, U, sink.epi, Dn, S->hid16);
+      linear(S, bf, HEPI_XIELU, U, 1, st);
+      MK("ff.up");
       linear(S, bf, sink.epi, Dn, 1, st);
       MK("ff.down");
     }
@@ -2130,6 +2235,8 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         G.tiles = S->d_tiles; G.n_tiles = S->d_ntiles; G.a_map = S->d_perm; G.a_div = top; G.c_map = S->d_perm;
         Dn.tiles = S->d_tiles; Dn.n_tiles = S->d_ntiles; Dn.a_map = S->d_perm; Dn.a_div = 1; Dn.c_map = S->d_perm;
         const int cap = std::min(S->max_tiles, pairs / bm + E + 1);
+        G.n_expert = Dn.n_expert = E;
+        hidden16(S, bf, epi_up, G, HEPI_STORE, Dn, S->hid16);
         MK("moe.plan");
         linear(S, bf, epi_up, G, 1, st, cap);
         MK("moe.glu");
@@ -2138,8 +2245,10 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         if (shared) {
           GemmP Us = gp(hin, W, L.gate_sh.p, W, hsh, ffs, T, ffs, W);
           Us.W2 = L.up_sh.p; Us.lim = sp.ff_limit;
+          GemmP Ds = gp(hsh, ffs, L.down_sh.p, ffs, ysh, W, T, W, ffs);
+          hidden16(S, bf, epi_up, Us, HEPI_STORE, Ds, S->hid16 + (size_t)pairs * ff);
           linear(S, bf, epi_up, Us, 1, st);
-          linear(S, bf, HEPI_STORE, gp(hsh, ffs, L.down_sh.p, ffs, ysh, W, T, W, ffs), 1, st);
+          linear(S, bf, HEPI_STORE, Ds, 1, st);
           MK("moe.shared");
         }
       }
@@ -2237,6 +2346,7 @@ static int forward_chunk(dsk_model* m, dsk_state* s, const int32_t* tokens, int 
   }
   CK(cudaStreamSynchronize(s->stream));
   CK(cudaGetLastError());
+  if (*(volatile int*)S->h_err) { const int e = *S->h_err; *S->h_err = 0; return fail(-2, e == 2 ? "a product's tensor map was refused" : "a wait inside a matrix product gave up"); }
   S->next_pos = pos0 + n;
   s->last_pos = pos0 + n - 1;
   s->have_logits = n_want > 0 && want[n_want - 1] == n - 1;

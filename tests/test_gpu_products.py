@@ -1,0 +1,37 @@
+"""bf16 products of portions on the tensor cores, at the edges of their tiles (128 rows; 32 to 256 columns; 64-deep slices; experts with
+no row, one tile and several), against the float64 statement of a small model made of them."""
+import numpy as np
+import pytest
+
+from test_gpu_netusun import close_bf16, mk, no, tokens_for  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+# width: depth of most products (72 and 136 end inside a 64-deep slice), ff: their columns (104 and 264 end inside a column tile; gated ones take
+# half a tile), tokens: rows (5 is the smallest portion that takes this path; 128 is one row tile)
+@pytest.mark.parametrize("width,ff,tokens", [(72, 104, 5), (136, 264, 127), (128, 256, 128), (64, 1032, 129), (136, 104, 257)])
+def test_dense_edges(mk, no, width, ff, tokens):  # noqa: F811
+    cfg = no.model_config([no.att(heads=4, dim=32, vdim=24, size=40, mlp=no.dense(ff)), no.lat(mlp=no.dense(2 * ff))], width=width, vocab=211)
+    m, W = mk(cfg, seed=width + tokens, quant="bf16", chunk=512)
+    toks = tokens_for(cfg, tokens, 3)
+    assert close_bf16(m.forward_chunk(toks, 0, range(tokens)), no.run(cfg, W, toks)[0], no.rounding_noise(cfg, W, toks))
+
+
+@pytest.mark.parametrize("experts,top,ff,tokens", [(3, 1, 40, 5), (2, 2, 72, 130), (8, 2, 104, 200), (40, 3, 8, 64)])
+def test_routed_edges(mk, no, experts, top, ff, tokens):  # noqa: F811
+    cfg = no.model_config([no.att(heads=2, dim=16, vdim=16, mlp=no.moe(experts=experts, top=top, ff=ff, shared=ff + 32))], width=88, vocab=131)
+    m, W = mk(cfg, seed=experts, quant="bf16", chunk=256)
+    toks = tokens_for(cfg, tokens, 4)
+    assert close_bf16(m.forward_chunk(toks, 0, range(tokens)), no.run(cfg, W, toks)[0], no.rounding_noise(cfg, W, toks))
+
+
+def test_unaligned_depth_and_short_steps(mk, no):  # noqa: F811
+    """Depths that TMA cannot address (not a multiple of 8) and the steps of up to four rows keep their own kernels."""
+    cfg = no.model_config([no.att(heads=3, dim=10, vdim=6, mlp=no.dense(98))], width=84, vocab=61)
+    m, W = mk(cfg, seed=9, quant="bf16", chunk=64)
+    toks = tokens_for(cfg, 40, 5)
+    exp, noise = no.run(cfg, W, toks)[0], no.rounding_noise(cfg, W, toks)
+    assert close_bf16(m.forward_chunk(toks, 0, range(40)), exp, noise)
+    rows = np.concatenate([m.forward_chunk(toks[p:p + 4], p, range(4)) for p in range(0, 40, 4)])
+    assert close_bf16(rows, exp, noise)
