@@ -98,8 +98,8 @@ __global__ void convert_kernel(const ST* __restrict__ src, DT* __restrict__ dst,
 // control words of a chunk: ctl[0] = absolute position of the chunk's first token.  Kept in device memory so that a captured
 // decode step can be replayed: advance_ctl moves it on.
 // ---------------------------------------------------------------------------------------------------------------------
-__global__ void set_ctl(int* ctl, int pos0) { ctl[0] = pos0; }
-__global__ void advance_ctl(int* ctl, int by) { ctl[0] += by; }
+__global__ void set_ctl(int* ctl, int pos0) { grid_enter(); ctl[0] = pos0; }
+__global__ void advance_ctl(int* ctl, int by) { grid_enter(); ctl[0] += by; }
 
 // x[t] = scale * table[tok[t]] (+ bigram[row]).  The second table is indexed by the pair (previous token, token): row
 // (prev * mul_prev + tok * mul_cur) mod buckets, and row `buckets` for the first token of a sequence (position ctl[0] + t == 0).
@@ -109,6 +109,7 @@ template <typename WT>
 __global__ void embed_rows(const int* __restrict__ tok, const WT* __restrict__ table, int width, float* __restrict__ x, float scale,
                            const WT* __restrict__ bigram, int buckets, int mul_prev, int mul_cur, const int* __restrict__ ctl,
                            const int* __restrict__ carried, float* __restrict__ x_keep = nullptr, int ld_keep = 0) {
+  grid_enter();
   const int t = blockIdx.x;
   const WT* row = table + (size_t)tok[t] * width;
   if (!bigram) {
@@ -133,6 +134,7 @@ __global__ void embed_rows(const int* __restrict__ tok, const WT* __restrict__ t
 }
 // the ring rows of the last taps - 1 positions of a step of T >= taps - 1 tokens (see canon_conv)
 __global__ void canon_history(const float* __restrict__ x, int ld, float* __restrict__ hist, int T, int ch, int taps, const int* __restrict__ ctl) {
+  grid_enter();
   const int c = blockIdx.x * blockDim.x + threadIdx.x, back = taps - 1;
   if (c >= ch) return;
   for (int j = 0; j < back; j++) {
@@ -140,7 +142,7 @@ __global__ void canon_history(const float* __restrict__ x, int ld, float* __rest
     hist[(size_t)((ctl[0] + tau) % back) * ch + c] = x[(size_t)tau * ld + c];
   }
 }
-__global__ void carry_token(const int* __restrict__ tok, int T, int* __restrict__ carried) { carried[0] = tok[T - 1]; }
+__global__ void carry_token(const int* __restrict__ tok, int T, int* __restrict__ carried) { grid_enter(); carried[0] = tok[T - 1]; }
 
 // ---------------------------------------------------------------------------------------------------------------------
 // Causal per-channel convolution in front of a sublayer, added to its input:  u_t = x_t + sum_j w[c][j] x_(t - taps + 1 + j)
@@ -153,6 +155,7 @@ __global__ void carry_token(const int* __restrict__ tok, int T, int* __restrict_
 constexpr int kCanonTokens = 32, kCanonMaxTaps = 17;
 __global__ void __launch_bounds__(128) canon_conv(const float* __restrict__ x, int ld, const float* __restrict__ w, float* __restrict__ hist,
                                                   float* __restrict__ u, int ldu, int T, int ch, int taps, const int* __restrict__ ctl) {
+  grid_enter();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ch) return;
   const int t0 = blockIdx.y * kCanonTokens, t1 = min(T, t0 + kCanonTokens), pos0 = ctl[0], back = taps - 1;
@@ -204,6 +207,7 @@ __global__ void __launch_bounds__(256) group_rmsnorm(const float* __restrict__ i
                                                      OT* __restrict__ out, int ld_out, int n, int groups, float eps, int mode,
                                                      float alpha, const int* __restrict__ ctl, int ring,
                                                      const float* __restrict__ gate = nullptr, int ld_gate = 0) {
+  grid_enter();
   __shared__ float red[33];
   const int t = blockIdx.x;
   const float* x = in + (size_t)t * ld_in;
@@ -332,6 +336,7 @@ __device__ __forceinline__ void gemm_epilogue(const GemmP& P, float* __restrict_
 // 64 x 64 output tile, K in steps of 16, 256 threads with a 4 x 4 micro-tile each; plain fp32 FMA on fp32 activations.
 template <typename WT, int EPI>
 __global__ void __launch_bounds__(256) gemm_tiled(const GemmP P) {
+  grid_enter();
   constexpr int BM = 64, BN = 64, BK = 16;
   constexpr bool DUAL = epi_dual(EPI);
   __shared__ __align__(16) float As[BK][BM + 4];
@@ -451,6 +456,7 @@ constexpr size_t kMmaSmem = (size_t)(1 + kMmaStages) * 128 * kMmaPitch * 2;
 
 template <int EPI>
 __global__ void __launch_bounds__(256) gemm_mma(const GemmP P) {
+  grid_enter();
   typedef __nv_bfloat16 bf;
   constexpr int BM = 128, BT = 128, BK = 32, PITCH = kMmaPitch, ST = kMmaStages;
   constexpr bool DUAL = epi_dual(EPI);
@@ -611,6 +617,7 @@ constexpr int kCloseOpenTokens = 8;
 __global__ void __launch_bounds__(128) close_open_small(const float* __restrict__ y, const float* __restrict__ cw, float alpha, float eps,
                                                         float* __restrict__ x, int ld, const float* __restrict__ w, float* __restrict__ hist,
                                                         float* __restrict__ u, int T, int ch, int taps, const int* __restrict__ ctl) {
+  grid_enter();
   __shared__ float red[33];
   float sc[kCloseOpenTokens];
 #pragma unroll
@@ -672,6 +679,7 @@ __global__ void __launch_bounds__(128) close_open_small(const float* __restrict_
 __global__ void __launch_bounds__(128) rms_add_shift_small(const float* __restrict__ y, const float* __restrict__ w, float alpha, float eps,
                                                            float* __restrict__ x, int ld, const float* __restrict__ mu, float* __restrict__ carry,
                                                            float* __restrict__ hs, int T, int ch, const int* __restrict__ ctl) {
+  grid_enter();
   __shared__ float red[33];
   float sc[kCloseOpenTokens];
 #pragma unroll
@@ -729,6 +737,7 @@ __device__ __forceinline__ uint4 ldg_stream(const void* p) {   // 16 read-only b
 // M <= 4 rows: one warp per weight row, lanes stride over K with 16-byte loads when pitches and bases allow it.
 template <typename WT, int EPI>
 __global__ void __launch_bounds__(256) gemv_rows(const GemmP P) {
+  grid_enter();
   constexpr bool DUAL = epi_dual(EPI);
   constexpr int MR = 4, V = WVec<WT>::N;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, z = blockIdx.y;
@@ -831,18 +840,25 @@ __global__ void __launch_bounds__(256) gemv_one(const GemmP P) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, z = blockIdx.y;
   int N = P.N, K = P.K, ldw = P.ldw, cr = 0;
   const WT *W, *W2 = nullptr;
-  const float* A;
-  float* C;
-  if (P.z_expert && P.n_shared > 0 && z >= P.z_shared) {
+  const float* A = nullptr;
+  float* C = nullptr;
+  // the first weights of a product whose matrix is known are asked for while the kernel ahead still runs; a routed one has to wait for its router
+  bool ready = P.z_expert != nullptr;
+  if (ready) grid_enter();
+  const bool shared = P.z_expert && P.n_shared > 0 && z >= P.z_shared;
+  if (shared) {
     N = P.sN; K = P.sK; ldw = P.sK;
     W = reinterpret_cast<const WT*>(P.sW1); W2 = reinterpret_cast<const WT*>(P.sW2);
-    A = P.As + (size_t)(z - P.z_shared) * P.s_lda;
-    C = P.Cs + (size_t)(z - P.z_shared) * P.s_ldc;
   } else {
     const long long woff = P.z_expert ? (long long)P.z_expert[z] * P.sW : (long long)(z / P.z_wdiv) * P.sW;
     W = reinterpret_cast<const WT*>(P.W) + woff;
     if (DUAL) W2 = reinterpret_cast<const WT*>(P.W2) + woff;
-    if (P.z_expert) {
+  }
+  auto rows = [&] {
+    if (shared) {
+      A = P.As + (size_t)(z - P.z_shared) * P.s_lda;
+      C = P.Cs + (size_t)(z - P.z_shared) * P.s_ldc;
+    } else if (P.z_expert) {
       A = P.A + (size_t)(z / P.z_adiv) * P.lda;
       C = P.C + (size_t)z * P.ldc;
     } else {
@@ -850,7 +866,8 @@ __global__ void __launch_bounds__(256) gemv_one(const GemmP P) {
       A = P.A + (long long)z * P.sA + (size_t)(P.a_map ? P.a_map[0] / P.a_div : 0) * P.lda;
       C = P.C + (long long)z * P.sC + (size_t)cr * P.ldc;
     }
-  }
+  };
+  if (ready) rows();
   for (int n0 = (blockIdx.x * 8 + warp) * R; n0 < N; n0 += gridDim.x * 8 * R) {
     const WT* w[R][NM];
     float acc[R][NM];
@@ -862,7 +879,7 @@ __global__ void __launch_bounds__(256) gemv_one(const GemmP P) {
 #pragma unroll
       for (int m = 0; m < NM; m++) acc[r][m] = 0.f;
     }
-    for (int k0 = lane * V; k0 < K; k0 += 32 * V * U) {
+    for (int k0 = lane * V; k0 < K || !ready; k0 += 32 * V * U) {   // (a lane without a first slice still has to wait)
       uint4 raw[U][R][NM];
 #pragma unroll
       for (int u = 0; u < U; u++)
@@ -870,6 +887,7 @@ __global__ void __launch_bounds__(256) gemv_one(const GemmP P) {
         for (int r = 0; r < R; r++)
 #pragma unroll
           for (int m = 0; m < NM; m++) raw[u][r][m] = k0 + u * 32 * V < K ? ldg_stream(w[r][m] + k0 + u * 32 * V) : make_uint4(0u, 0u, 0u, 0u);
+      if (!ready) { grid_enter(); rows(); ready = true; }
 #pragma unroll
       for (int u = 0; u < U; u++) {
         const int k = k0 + u * 32 * V;
@@ -899,6 +917,7 @@ __global__ void __launch_bounds__(256) gemv_one(const GemmP P) {
       if (lane == 0 && n0 + r < N) gemm_epilogue<WT, EPI>(P, C, cr, n0 + r, v, v2);
     }
   }
+  if (!ready) grid_enter();   // a warp without a row
 }
 // whether gemv_one's 16-byte loads are aligned for every batch
 template <typename WT>
@@ -916,6 +935,7 @@ inline bool gemv_one_ok(const GemmP& P) {
 // ---------------------------------------------------------------------------------------------------------------------
 __global__ void causal_conv_silu(const float* __restrict__ in, int ld_in, const float* __restrict__ w, const float* __restrict__ b,
                                  const float* __restrict__ hist, float* __restrict__ out, int ld_out, int T, int ch, int taps) {
+  grid_enter();
   const int t = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ch) return;
   float acc = b[c];
@@ -927,6 +947,7 @@ __global__ void causal_conv_silu(const float* __restrict__ in, int ld_in, const 
   out[(size_t)t * ld_out + c] = silu_f(acc);
 }
 __global__ void conv_history_update(const float* __restrict__ in, int ld_in, float* __restrict__ hist, int T, int ch, int taps) {
+  grid_enter();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ch) return;
   for (int j = 0; j < taps - 1; j++) {   // ascending: slot j is read (as slot T + j of the old history) before it is written
@@ -948,6 +969,7 @@ __global__ void __launch_bounds__(512) ssd_scan(const float* __restrict__ proj, 
                                                 const float* __restrict__ dt_bias, const float* __restrict__ A_log,
                                                 const float* __restrict__ Dskip, float* __restrict__ state,
                                                 float* __restrict__ out, int ld_out, int T, int H, int P, int N, int G, int PB, int TB) {
+  grid_enter();
   extern __shared__ __align__(16) float sm[];
   const int NP = (N + 3) & ~3;      // staged B / C rows are padded to whole float4s
   float* s_B = sm;                  // [TB][NP]
@@ -1055,6 +1077,7 @@ __global__ void __launch_bounds__(512) ssd_scan(const float* __restrict__ proj, 
 // ---------------------------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(128) token_shift(const float* __restrict__ x, int ld, const float* __restrict__ mu, float* __restrict__ carry,
                                                    float* __restrict__ h, int ldh, int T, int ch, const int* __restrict__ ctl) {
+  grid_enter();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ch) return;
   const int t0 = blockIdx.y * kCanonTokens, t1 = min(T, t0 + kCanonTokens);
@@ -1068,6 +1091,7 @@ __global__ void __launch_bounds__(128) token_shift(const float* __restrict__ x, 
   if (gridDim.y == 1) carry[c] = prev;
 }
 __global__ void shift_carry(const float* __restrict__ x, int ld, float* __restrict__ carry, int T, int ch) {
+  grid_enter();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c < ch) carry[c] = x[(size_t)(T - 1) * ld + c];
 }
@@ -1085,6 +1109,7 @@ template <int RQ, int TPC>
 __global__ void __launch_bounds__(512, 1) hgrn2_scan(const float* __restrict__ proj, int ld, int q_off, int f_off, int v_off,
                                                   float* __restrict__ state, float* __restrict__ out,
                                                   int ld_out, int T, int H, int N, int P, int PB, int TB) {
+  grid_enter();
   extern __shared__ __align__(16) float sm[];
   const int NP = (N + 3) & ~3;      // staged rows are padded to whole float4s
   const int per = TB * (2 * NP + PB);   // floats of one staging buffer: f [TB][NP], q [TB][NP], v [TB][PB]
@@ -1222,6 +1247,7 @@ template <typename CT, int RV>
 __global__ void __launch_bounds__(256) latent_swa_attn(const float* __restrict__ qa, const CT* __restrict__ cache, float* __restrict__ out,
                                                        int T, int H, int R, const int* __restrict__ ctl, int mask, int window, int ring,
                                                        float scale, int TQ, int NS, float* __restrict__ part, const float* __restrict__ sink) {
+  grid_enter();
   extern __shared__ float sm[];
   const int NW = 8, HB = NW / TQ;
   float* qs = sm;                 // [NW][R]
@@ -1328,6 +1354,7 @@ __global__ void __launch_bounds__(256) latent_swa_attn(const float* __restrict__
 __global__ void __launch_bounds__(128) latent_swa_merge(const float* __restrict__ part, float* __restrict__ out, int R, int NS,
                                                         const float* __restrict__ gate = nullptr, int ld_gate = 0, int H = 1,
                                                         int gate_head = 0, int ld_out = 0, float alpha = 1.f) {
+  grid_enter();
   __shared__ float wts[64], ms[64], ls[64];   // NS <= 64 (kAttnSplitMax)
   const size_t th = blockIdx.x;
   const float* pp = part + th * NS * (R + 2);
@@ -1360,6 +1387,7 @@ __global__ void __launch_bounds__(128) latent_swa_merge(const float* __restrict_
 // out[t][c] *= sigmoid(gate[t][c / per]) for the n columns of T rows (an output gate whose raw values came out of a stacked
 // projection; per: columns that share a gate)
 __global__ void gate_rows(float* __restrict__ out, int ld_out, const float* __restrict__ gate, int ld_gate, int n, int per) {
+  grid_enter();
   float* o = out + (size_t)blockIdx.x * ld_out;
   const float* g = gate + (size_t)blockIdx.x * ld_gate;
   for (int c = threadIdx.x; c < n; c += blockDim.x) o[c] *= sigmoid_f(g[per == 1 ? c : c / per]);
@@ -1373,6 +1401,7 @@ __global__ void gate_rows(float* __restrict__ out, int ld_out, const float* __re
 // product kernels), and the softmax over the band 0 <= i - j < window of a [head][query][key] score array.
 // ---------------------------------------------------------------------------------------------------------------------
 __global__ void ring_rows(int first, int n, int ring, int* __restrict__ rows) {
+  grid_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) rows[i] = (first + i) % ring;
 }
@@ -1380,6 +1409,7 @@ __global__ void ring_rows(int first, int n, int ring, int* __restrict__ rows) {
 template <typename WT>
 __global__ void pack_keys_values(const float* __restrict__ kf, const float* __restrict__ vf, WT* __restrict__ kb, WT* __restrict__ vt,
                                  int Lk, int H, int D, int V) {
+  grid_enter();
   const int j = blockIdx.x;
   for (int e = threadIdx.x; e < H * D; e += blockDim.x) {
     const int h = e / D, d = e - h * D;
@@ -1396,6 +1426,7 @@ __global__ void pack_keys_values(const float* __restrict__ kf, const float* __re
 // positions.  Visible scores are modified (ScoreMods) and normalised, hidden entries become 0.
 __global__ void __launch_bounds__(128) softmax_band(float* __restrict__ S, int Tq, int Lk, int first, int qpos0, int mask, int window,
                                                     int nk, ScoreMods sm) {
+  grid_enter();
   __shared__ float red[33];
   const int t = blockIdx.x, h = blockIdx.y, H = gridDim.y;
   float* row = S + ((size_t)h * Tq + t) * Lk;
@@ -1450,6 +1481,7 @@ __device__ __forceinline__ void ln_stats(const float (&v)[kLnRegs], const float*
 __global__ void __launch_bounds__(256) layer_norm(const float* __restrict__ in, int ld_in, const float* __restrict__ w, const float* __restrict__ b,
                                                   float* __restrict__ out, int ld_out, int n, float eps, int mode, float alpha,
                                                   const float* __restrict__ wgt, int top) {
+  grid_enter();
   __shared__ float red[33];
   const int t = blockIdx.x;
   const float* x = in + (size_t)t * (wgt ? top : 1) * ld_in;
@@ -1482,6 +1514,7 @@ __global__ void __launch_bounds__(256) layer_norm(const float* __restrict__ in, 
 __global__ void __launch_bounds__(256) layer_norm_add_norm(const float* __restrict__ y, const float* __restrict__ wy, float* __restrict__ x,
                                                            const float* __restrict__ row, const float* __restrict__ wh,
                                                            float* __restrict__ h, int n, float eps, float alpha) {
+  grid_enter();
   __shared__ float red[33];
   const size_t t = blockIdx.x;
   const float* yr = y + t * n;
@@ -1512,6 +1545,7 @@ __global__ void __launch_bounds__(256) layer_norm_add_norm(const float* __restri
 // h = x / sqrt(mean(x^2) + eps) * w.  The row stays in registers up to 256 * kLnRegs values.
 __global__ void __launch_bounds__(256) rms_open(float* __restrict__ x, const float* __restrict__ e, const float* __restrict__ row,
                                                 const float* __restrict__ w, float* __restrict__ h, int n, float eps) {
+  grid_enter();
   __shared__ float red[33];
   float* xr = x + (size_t)blockIdx.x * n;
   const float* er = e ? e + (size_t)blockIdx.x * n : nullptr;
@@ -1549,6 +1583,7 @@ __global__ void __launch_bounds__(NT) rms_add_norm(const float* __restrict__ y, 
                                                     const float* __restrict__ wsh, const float* __restrict__ wy, const float* x, float* xo, int ldxo,
                                                     const float* __restrict__ wh, float* __restrict__ h, int n,
                                                     float eps, float alpha) {
+  grid_enter();
   __shared__ float red[33];
   const size_t t = blockIdx.x;
   constexpr int KR = NT * kLnRegs / NT;
@@ -1597,6 +1632,7 @@ __global__ void __launch_bounds__(NT) rms_add_norm(const float* __restrict__ y, 
 
 // the T rows of a step (pitch ls) copied to rows of pitch ld
 __global__ void copy_rows(const float* __restrict__ src, int ls, float* __restrict__ dst, int ld, int n) {
+  grid_enter();
   for (int i = threadIdx.x; i < n; i += blockDim.x) dst[(size_t)blockIdx.x * ld + i] = src[(size_t)blockIdx.x * ls + i];
 }
 
@@ -1608,6 +1644,7 @@ __global__ void __launch_bounds__(256) head_rmsnorm(const float* __restrict__ in
                                                     int ld_out, int T, int H, int P, float eps, const float* __restrict__ gate = nullptr,
                                                     int ld_gate = 0, float alpha = 1.f, int w_stride = 0, int gate_sig = 0,
                                                     const float* __restrict__ den = nullptr, const float* __restrict__ mrow = nullptr) {
+  grid_enter();
   const int lane = threadIdx.x & 31;
   const long long id = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (id >= (long long)T * H) return;
@@ -1628,6 +1665,7 @@ __global__ void __launch_bounds__(256) head_rmsnorm(const float* __restrict__ in
 
 // x[t][:] += row[:] for the T rows of a step (the per-pass vector of a layer loop)
 __global__ void add_row(float* __restrict__ x, int ld, const float* __restrict__ row, int n) {
+  grid_enter();
   float* o = x + (size_t)blockIdx.x * ld;
   for (int i = threadIdx.x; i < n; i += blockDim.x) o[i] += row[i];
 }
@@ -1709,6 +1747,7 @@ __global__ void __launch_bounds__(256) qk_norm_rope(const float* __restrict__ q,
                                                     const int* __restrict__ ctl, float* __restrict__ kcache,
                                                     float* __restrict__ vcache, int ring, int keep, const float* __restrict__ v_first,
                                                     float lam, float* __restrict__ v_keep, int layout, int head_norm, const ConvP cv) {
+  grid_enter();
   extern __shared__ float cs[];   // [8][D] convolved head rows (cv.w)
   __shared__ float red[33];
   const int t = blockIdx.x, pos = ctl[0] + t;
@@ -1809,6 +1848,7 @@ __global__ void __launch_bounds__(256) gqa_attn(const float* __restrict__ q, con
                                                 int Dv, const int* __restrict__ ctl, int mask, int span, int ring, float scale, int NS,
                                                 float* __restrict__ part, ScoreMods mods, const float* __restrict__ gate, int ld_gate, int gate_head,
                                                 int ld_out, float alpha) {
+  grid_enter();
   extern __shared__ float sm[];
   const int GD = G * D, GV = G * Dv, rep = H / G;
   const int GL = G / (int)gridDim.z, g0 = (int)blockIdx.z * GL, h0 = g0 * rep, HL = GL * rep, GDl = GL * D;   // this CTA's key heads and query heads
@@ -1951,6 +1991,7 @@ __global__ void __launch_bounds__(256) gqa_attn(const float* __restrict__ q, con
 template <typename WT>
 __global__ void pack_ring_kv(const float* __restrict__ kc, const float* __restrict__ vc, WT* __restrict__ kb, WT* __restrict__ vt,
                              int first, int Lk, int ring, int G, int D, int Dv, int nk, int keep) {
+  grid_enter();
   const int j = blockIdx.x;
   const size_t row = (size_t)cache_row(j < nk ? j : first + j - nk, keep, ring);
   for (int e = threadIdx.x; e < G * D; e += blockDim.x) {
@@ -1976,6 +2017,7 @@ __global__ void __launch_bounds__(256) mla_prepare(const float* __restrict__ dkv
                                                    float* __restrict__ q, float* __restrict__ qa_rot, int H, int D, int Rd, int R,
                                                    int rot_dims, const float* __restrict__ freq, float mag, int layout, const int* __restrict__ ctl,
                                                    float* __restrict__ cache, int ring) {
+  grid_enter();
   __shared__ float red[33];
   const int t = blockIdx.x, pos = ctl[0] + t, RW = R + Rd;
   const float* src = dkv + (size_t)t * ld_dkv;
@@ -2016,6 +2058,7 @@ __global__ void __launch_bounds__(256) mla_prepare(const float* __restrict__ dkv
 __global__ void pack_mla_kv(const float* __restrict__ kf, const float* __restrict__ vf, const float* __restrict__ cache,
                             const int* __restrict__ rows, float* __restrict__ kb, float* __restrict__ vt, int Lk, int H, int D, int Rd,
                             int R, int V) {
+  grid_enter();
   const int j = blockIdx.x, DK = D + Rd;
   const float* kr = cache + (size_t)rows[j] * (R + Rd) + R;
   for (int e = threadIdx.x; e < H * DK; e += blockDim.x) {
@@ -2031,6 +2074,7 @@ __global__ void pack_mla_kv(const float* __restrict__ kf, const float* __restric
 // out[h][e] = sum_g talk[h][g] in[g][e] for the n = Tq * Lk entries of every head; a CTA takes 128 consecutive entries
 __global__ void __launch_bounds__(128) mix_heads(const float* __restrict__ in, float* __restrict__ out, const float* __restrict__ talk,
                                                  int H, long long n) {
+  grid_enter();
   extern __shared__ float sm[];
   float* tk = sm;              // [H][H]
   float* col = sm + H * H;     // [H][128]
@@ -2056,6 +2100,7 @@ __global__ void __launch_bounds__(128) mix_heads(const float* __restrict__ in, f
 // ---------------------------------------------------------------------------------------------------------------------
 __global__ void moe_route(const float* __restrict__ logits, int ldz, const float* __restrict__ correction, int E, int top, float scale,
                           int* __restrict__ idx, float* __restrict__ wgt, int mode, int groups, int keep, float* __restrict__ wsh) {
+  grid_enter();
   extern __shared__ float sm[];
   __shared__ float red[33];
   float* sc = sm;            // [E]
@@ -2120,6 +2165,7 @@ __global__ void moe_route(const float* __restrict__ logits, int ldz, const float
 // {expert, first index into perm, rows}.  One CTA: histogram, serial scan over the experts, placement.
 __global__ void __launch_bounds__(1024) moe_plan(const int* __restrict__ idx, int pairs, int E, int bm, int* __restrict__ perm,
                                                  int4* __restrict__ tiles, int* __restrict__ n_tiles) {
+  grid_enter();
   extern __shared__ int smi[];
   int* cnt = smi;            // [E]
   int* off = smi + E;        // [E]
@@ -2143,6 +2189,7 @@ __global__ void __launch_bounds__(1024) moe_plan(const int* __restrict__ idx, in
 // ysh (nullable, [T][width]): a shared expert's output, added with the weight wsh[t]
 __global__ void moe_combine(float* __restrict__ x, int ldx, const float* __restrict__ y, const float* __restrict__ wgt, int top,
                             int width, float alpha, int add, const float* __restrict__ ysh = nullptr, const float* __restrict__ wsh = nullptr) {
+  grid_enter();
   const int t = blockIdx.x;
   for (int c = threadIdx.x; c < width; c += blockDim.x) {
     float s = 0.f;
@@ -2152,20 +2199,22 @@ __global__ void moe_combine(float* __restrict__ x, int ldx, const float* __restr
   }
 }
 
-// arg-max of one logits row -> Ctrl::argmax_key (lowest index on ties), optionally feeding the next token of a device-side
-// greedy loop: tok_out[0] = arg-max, log[step] = arg-max.
-__global__ void __launch_bounds__(1024) argmax_row(const float* __restrict__ logits, int vocab, Ctrl* __restrict__ ctrl, int* tok_out,
-                                                   int* log, int step) {
-  __shared__ unsigned long long best[32];
+// arg-max of one logits row -> Ctrl::argmax_key (lowest index on ties), joined over the CTAs by an atomic maximum on a key that is 0 ahead of
+// the launch.
+__global__ void __launch_bounds__(256) argmax_row(const float* __restrict__ logits, int vocab, Ctrl* __restrict__ ctrl) {
+  grid_enter();
+  __shared__ unsigned long long best[8];
   unsigned long long b = 0ull;
   auto see = [&](float v, int i) {
     const unsigned long long key = ((unsigned long long)orderable(v) << 32) | (unsigned long long)(0xFFFFFFFFu - (unsigned)i);
     if (key > b) b = key;
   };
-  int done = 0;
+  const int per = (vocab + (int)gridDim.x * 16 - 1) / ((int)gridDim.x * 16) * 16;   // a CTA's share, whole 16-byte loads
+  const int end = min(vocab, ((int)blockIdx.x + 1) * per);
+  int done = (int)blockIdx.x * per;
   if ((reinterpret_cast<uintptr_t>(logits) & 15) == 0) {   // whole rounds of four 16-byte loads per thread, all in flight together
     const int round = 16 * (int)blockDim.x;
-    for (; done + round <= vocab; done += round) {
+    for (; done + round <= end; done += round) {
       float4 v[4];
 #pragma unroll
       for (int u = 0; u < 4; u++) v[u] = *reinterpret_cast<const float4*>(logits + done + 4 * (u * (int)blockDim.x + (int)threadIdx.x));
@@ -2176,22 +2225,21 @@ __global__ void __launch_bounds__(1024) argmax_row(const float* __restrict__ log
       }
     }
   }
-  for (int i = done + threadIdx.x; i < vocab; i += blockDim.x) see(logits[i], i);
+  for (int i = done + threadIdx.x; i < end; i += blockDim.x) see(logits[i], i);
   for (int o = 16; o; o >>= 1) { const unsigned long long v = __shfl_xor_sync(0xffffffffu, b, o); if (v > b) b = v; }
   if ((threadIdx.x & 31) == 0) best[threadIdx.x >> 5] = b;
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); w++) if (best[w] > b) b = best[w];
-    ctrl->argmax_key = b;
-    const int tok = (int)(0xFFFFFFFFu - (unsigned)(b & 0xFFFFFFFFull));
-    if (tok_out) tok_out[0] = tok;
-    if (log) log[step] = tok;
+    for (int w = 1; w < 8; w++) if (best[w] > b) b = best[w];
+    atomicMax(&ctrl->argmax_key, b);
   }
 }
 
 // device-side greedy loop: the token of the last arg-max becomes the next chunk's only token and is logged
-__global__ void greedy_feed(const Ctrl* __restrict__ ctrl, int* __restrict__ tok, int* __restrict__ log, int* __restrict__ step) {
+__global__ void greedy_feed(Ctrl* __restrict__ ctrl, int* __restrict__ tok, int* __restrict__ log, int* __restrict__ step) {
+  grid_enter();
   const int t = (int)(0xFFFFFFFFu - (unsigned)(ctrl->argmax_key & 0xFFFFFFFFull));
+  ctrl->argmax_key = 0ull;   // (for the step's own arg-max)
   tok[0] = t;
   log[*step] = t;
   *step += 1;

@@ -1357,6 +1357,33 @@ static void timeline_report(State* S, int T) {
   S->tl_used = 0;
 }
 
+// Launches a kernel as a programmatic dependent of the one ahead of it in the stream: it is set up, and runs up to its grid_wait, while
+// that one still runs.  Only in short steps (chain_step): their kernels take a few microseconds, about what a launch takes (a decoded token 10 -
+// 15 % less, 45 tokens 436 -> 359 us).  In long ones the waiting CTAs take the places that the running kernel leaves, not one per SM: a
+// 600-token step in fp32, whose products are about one CTA per SM, went from 1.88 to 2.56 ms.  plain_next: the coming launch waits
+// as usual (it joins another stream).
+static thread_local bool chain_step = false, plain_next = false;
+template <typename... KA> struct Launch {
+  void (*kernel)(KA...);
+  cudaLaunchConfig_t cfg;
+  template <typename... A> void operator()(A&&... a) const {
+    static_assert(sizeof...(A) == sizeof...(KA), "every argument of a kernel is given");
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = cfg;
+    if (chain_step && !plain_next) { c.attrs = &at; c.numAttrs = 1; }
+    plain_next = false;
+    cudaLaunchKernelEx(&c, kernel, static_cast<KA>(a)...);
+  }
+};
+template <typename... KA>
+static Launch<KA...> launch_next(void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t st) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = st;
+  return {kernel, c};
+}
+
 static GemmP gp(const float* A, int lda, const void* W, int ldw, float* C, int ldc, int M, int N, int K) {
   GemmP P{};
   P.A = A; P.lda = lda; P.W = W; P.ldw = ldw; P.C = C; P.ldc = ldc; P.M = M; P.N = N; P.K = K;
@@ -1368,18 +1395,18 @@ static void launch_gemm_mma(int epi, const GemmP& P, int Z, int tile_cap, cudaSt
   const int bn = epi_dual(epi) ? 64 : 128;
   const dim3 grid((unsigned)((P.N + bn - 1) / bn), (unsigned)(P.tiles ? tile_cap : (P.M + 127) / 128), (unsigned)Z);
   switch (epi) {
-    case HEPI_STORE: gemm_mma<HEPI_STORE><<<grid, 256, kMmaSmem, st>>>(P); break;
-    case HEPI_ADD: gemm_mma<HEPI_ADD><<<grid, 256, kMmaSmem, st>>>(P); break;
-    case HEPI_GLU: gemm_mma<HEPI_GLU><<<grid, 256, kMmaSmem, st>>>(P); break;
-    case HEPI_XIELU: gemm_mma<HEPI_XIELU><<<grid, 256, kMmaSmem, st>>>(P); break;
-    case HEPI_GEGLU: gemm_mma<HEPI_GEGLU><<<grid, 256, kMmaSmem, st>>>(P); break;
-    case HEPI_SIGMUL: gemm_mma<HEPI_SIGMUL><<<grid, 256, kMmaSmem, st>>>(P); break;
-    case HEPI_RELU2: gemm_mma<HEPI_RELU2><<<grid, 256, kMmaSmem, st>>>(P); break;
-    case HEPI_LINGATE: gemm_mma<HEPI_LINGATE><<<grid, 256, kMmaSmem, st>>>(P); break;
-    case HEPI_SILU_SIG: gemm_mma<HEPI_SILU_SIG><<<grid, 256, kMmaSmem, st>>>(P); break;
-    case HEPI_SOFTCAP: gemm_mma<HEPI_SOFTCAP><<<grid, 256, kMmaSmem, st>>>(P); break;
-    case HEPI_SWIGLU: gemm_mma<HEPI_SWIGLU><<<grid, 256, kMmaSmem, st>>>(P); break;
-    default: gemm_mma<HEPI_GELU_MUL><<<grid, 256, kMmaSmem, st>>>(P); break;
+    case HEPI_STORE: launch_next(gemm_mma<HEPI_STORE>, grid, 256, kMmaSmem, st)(P); break;
+    case HEPI_ADD: launch_next(gemm_mma<HEPI_ADD>, grid, 256, kMmaSmem, st)(P); break;
+    case HEPI_GLU: launch_next(gemm_mma<HEPI_GLU>, grid, 256, kMmaSmem, st)(P); break;
+    case HEPI_XIELU: launch_next(gemm_mma<HEPI_XIELU>, grid, 256, kMmaSmem, st)(P); break;
+    case HEPI_GEGLU: launch_next(gemm_mma<HEPI_GEGLU>, grid, 256, kMmaSmem, st)(P); break;
+    case HEPI_SIGMUL: launch_next(gemm_mma<HEPI_SIGMUL>, grid, 256, kMmaSmem, st)(P); break;
+    case HEPI_RELU2: launch_next(gemm_mma<HEPI_RELU2>, grid, 256, kMmaSmem, st)(P); break;
+    case HEPI_LINGATE: launch_next(gemm_mma<HEPI_LINGATE>, grid, 256, kMmaSmem, st)(P); break;
+    case HEPI_SILU_SIG: launch_next(gemm_mma<HEPI_SILU_SIG>, grid, 256, kMmaSmem, st)(P); break;
+    case HEPI_SOFTCAP: launch_next(gemm_mma<HEPI_SOFTCAP>, grid, 256, kMmaSmem, st)(P); break;
+    case HEPI_SWIGLU: launch_next(gemm_mma<HEPI_SWIGLU>, grid, 256, kMmaSmem, st)(P); break;
+    default: launch_next(gemm_mma<HEPI_GELU_MUL>, grid, 256, kMmaSmem, st)(P); break;
   }
 }
 
@@ -1416,7 +1443,7 @@ static void launch_tc5(State* S, int epi, const GemmP& P, int tile_cap, cudaStre
   if (!A16) {
     const int vec = P.lda % 4 == 0 && (reinterpret_cast<uintptr_t>(P.A) & 15) == 0;
     const long long n = (long long)P.M * (P.K / 8);
-    bf16_rows<<<(unsigned)std::min<long long>((n + 255) / 256, 148 * 8), 256, 0, st>>>(P.A, P.lda, P.a_map, P.a_div, S->a16, P.M, P.K, vec);
+    launch_next(bf16_rows, (unsigned)std::min<long long>((n + 255) / 256, 148 * 8), 256, 0, st)(P.A, P.lda, P.a_map, P.a_div, S->a16, P.M, P.K, vec);
     S->launches++;
     A16 = S->a16;
   }
@@ -1441,7 +1468,7 @@ static void launch_tc5(State* S, int epi, const GemmP& P, int tile_cap, cudaStre
     *S->h_err = 2;
     return;
   }
-#define DSK_TC5(E) case E: gemm_tc5<E><<<(unsigned)grid, kTcThreads, kTcSmem, st>>>(P, T, mA, mB, mB2); break
+#define DSK_TC5(E) case E: launch_next(gemm_tc5<E>, (unsigned)grid, kTcThreads, kTcSmem, st)(P, T, mA, mB, mB2); break
   switch (epi) {
     DSK_TC5(HEPI_STORE); DSK_TC5(HEPI_ADD); DSK_TC5(HEPI_GLU); DSK_TC5(HEPI_XIELU); DSK_TC5(HEPI_GEGLU); DSK_TC5(HEPI_SIGMUL);
     DSK_TC5(HEPI_RELU2); DSK_TC5(HEPI_LINGATE); DSK_TC5(HEPI_SILU_SIG); DSK_TC5(HEPI_SOFTCAP); DSK_TC5(HEPI_SWIGLU); DSK_TC5(HEPI_GELU_MUL);
@@ -1455,7 +1482,7 @@ static void launch_gemm_t(int epi, const GemmP& P, int Z, bool small, int tile_c
     const int n = std::max(P.N, P.n_shared > 0 ? P.sN : 0);
     const int R = (long long)n * Z >= 16384 && Z == 1 ? 2 : 1;   // rows per warp
     const dim3 grid((unsigned)std::max(1, std::min((n + 8 * R - 1) / (8 * R), 148 * 8)), (unsigned)Z);
-#define DSK_GEMV1(E) do { if (R == 2) gemv_one<WT, E, 2><<<grid, 256, 0, st>>>(P); else gemv_one<WT, E, 1><<<grid, 256, 0, st>>>(P); } while (0)
+#define DSK_GEMV1(E) do { if (R == 2) launch_next(gemv_one<WT, E, 2>, grid, 256, 0, st)(P); else launch_next(gemv_one<WT, E, 1>, grid, 256, 0, st)(P); } while (0)
     switch (epi) {
       case HEPI_STORE: DSK_GEMV1(HEPI_STORE); break;
       case HEPI_ADD: DSK_GEMV1(HEPI_ADD); break;
@@ -1474,34 +1501,34 @@ static void launch_gemm_t(int epi, const GemmP& P, int Z, bool small, int tile_c
   } else if (small) {
     const dim3 grid((unsigned)std::max(1, std::min((std::max(P.N, P.n_shared > 0 ? P.sN : 0) + 7) / 8, 148 * 8)), (unsigned)Z);
     switch (epi) {
-      case HEPI_STORE: gemv_rows<WT, HEPI_STORE><<<grid, 256, 0, st>>>(P); break;
-      case HEPI_ADD: gemv_rows<WT, HEPI_ADD><<<grid, 256, 0, st>>>(P); break;
-      case HEPI_GLU: gemv_rows<WT, HEPI_GLU><<<grid, 256, 0, st>>>(P); break;
-      case HEPI_XIELU: gemv_rows<WT, HEPI_XIELU><<<grid, 256, 0, st>>>(P); break;
-      case HEPI_GEGLU: gemv_rows<WT, HEPI_GEGLU><<<grid, 256, 0, st>>>(P); break;
-      case HEPI_SIGMUL: gemv_rows<WT, HEPI_SIGMUL><<<grid, 256, 0, st>>>(P); break;
-      case HEPI_RELU2: gemv_rows<WT, HEPI_RELU2><<<grid, 256, 0, st>>>(P); break;
-      case HEPI_LINGATE: gemv_rows<WT, HEPI_LINGATE><<<grid, 256, 0, st>>>(P); break;
-      case HEPI_SILU_SIG: gemv_rows<WT, HEPI_SILU_SIG><<<grid, 256, 0, st>>>(P); break;
-      case HEPI_SOFTCAP: gemv_rows<WT, HEPI_SOFTCAP><<<grid, 256, 0, st>>>(P); break;
-      case HEPI_SWIGLU: gemv_rows<WT, HEPI_SWIGLU><<<grid, 256, 0, st>>>(P); break;
-      default: gemv_rows<WT, HEPI_GELU_MUL><<<grid, 256, 0, st>>>(P); break;
+      case HEPI_STORE: launch_next(gemv_rows<WT, HEPI_STORE>, grid, 256, 0, st)(P); break;
+      case HEPI_ADD: launch_next(gemv_rows<WT, HEPI_ADD>, grid, 256, 0, st)(P); break;
+      case HEPI_GLU: launch_next(gemv_rows<WT, HEPI_GLU>, grid, 256, 0, st)(P); break;
+      case HEPI_XIELU: launch_next(gemv_rows<WT, HEPI_XIELU>, grid, 256, 0, st)(P); break;
+      case HEPI_GEGLU: launch_next(gemv_rows<WT, HEPI_GEGLU>, grid, 256, 0, st)(P); break;
+      case HEPI_SIGMUL: launch_next(gemv_rows<WT, HEPI_SIGMUL>, grid, 256, 0, st)(P); break;
+      case HEPI_RELU2: launch_next(gemv_rows<WT, HEPI_RELU2>, grid, 256, 0, st)(P); break;
+      case HEPI_LINGATE: launch_next(gemv_rows<WT, HEPI_LINGATE>, grid, 256, 0, st)(P); break;
+      case HEPI_SILU_SIG: launch_next(gemv_rows<WT, HEPI_SILU_SIG>, grid, 256, 0, st)(P); break;
+      case HEPI_SOFTCAP: launch_next(gemv_rows<WT, HEPI_SOFTCAP>, grid, 256, 0, st)(P); break;
+      case HEPI_SWIGLU: launch_next(gemv_rows<WT, HEPI_SWIGLU>, grid, 256, 0, st)(P); break;
+      default: launch_next(gemv_rows<WT, HEPI_GELU_MUL>, grid, 256, 0, st)(P); break;
     }
   } else {
     const dim3 grid((unsigned)((P.N + 63) / 64), (unsigned)(P.tiles ? tile_cap : (P.M + 63) / 64), (unsigned)Z);
     switch (epi) {
-      case HEPI_STORE: gemm_tiled<WT, HEPI_STORE><<<grid, 256, 0, st>>>(P); break;
-      case HEPI_ADD: gemm_tiled<WT, HEPI_ADD><<<grid, 256, 0, st>>>(P); break;
-      case HEPI_GLU: gemm_tiled<WT, HEPI_GLU><<<grid, 256, 0, st>>>(P); break;
-      case HEPI_XIELU: gemm_tiled<WT, HEPI_XIELU><<<grid, 256, 0, st>>>(P); break;
-      case HEPI_GEGLU: gemm_tiled<WT, HEPI_GEGLU><<<grid, 256, 0, st>>>(P); break;
-      case HEPI_SIGMUL: gemm_tiled<WT, HEPI_SIGMUL><<<grid, 256, 0, st>>>(P); break;
-      case HEPI_RELU2: gemm_tiled<WT, HEPI_RELU2><<<grid, 256, 0, st>>>(P); break;
-      case HEPI_LINGATE: gemm_tiled<WT, HEPI_LINGATE><<<grid, 256, 0, st>>>(P); break;
-      case HEPI_SILU_SIG: gemm_tiled<WT, HEPI_SILU_SIG><<<grid, 256, 0, st>>>(P); break;
-      case HEPI_SOFTCAP: gemm_tiled<WT, HEPI_SOFTCAP><<<grid, 256, 0, st>>>(P); break;
-      case HEPI_SWIGLU: gemm_tiled<WT, HEPI_SWIGLU><<<grid, 256, 0, st>>>(P); break;
-      default: gemm_tiled<WT, HEPI_GELU_MUL><<<grid, 256, 0, st>>>(P); break;
+      case HEPI_STORE: launch_next(gemm_tiled<WT, HEPI_STORE>, grid, 256, 0, st)(P); break;
+      case HEPI_ADD: launch_next(gemm_tiled<WT, HEPI_ADD>, grid, 256, 0, st)(P); break;
+      case HEPI_GLU: launch_next(gemm_tiled<WT, HEPI_GLU>, grid, 256, 0, st)(P); break;
+      case HEPI_XIELU: launch_next(gemm_tiled<WT, HEPI_XIELU>, grid, 256, 0, st)(P); break;
+      case HEPI_GEGLU: launch_next(gemm_tiled<WT, HEPI_GEGLU>, grid, 256, 0, st)(P); break;
+      case HEPI_SIGMUL: launch_next(gemm_tiled<WT, HEPI_SIGMUL>, grid, 256, 0, st)(P); break;
+      case HEPI_RELU2: launch_next(gemm_tiled<WT, HEPI_RELU2>, grid, 256, 0, st)(P); break;
+      case HEPI_LINGATE: launch_next(gemm_tiled<WT, HEPI_LINGATE>, grid, 256, 0, st)(P); break;
+      case HEPI_SILU_SIG: launch_next(gemm_tiled<WT, HEPI_SILU_SIG>, grid, 256, 0, st)(P); break;
+      case HEPI_SOFTCAP: launch_next(gemm_tiled<WT, HEPI_SOFTCAP>, grid, 256, 0, st)(P); break;
+      case HEPI_SWIGLU: launch_next(gemm_tiled<WT, HEPI_SWIGLU>, grid, 256, 0, st)(P); break;
+      default: launch_next(gemm_tiled<WT, HEPI_GELU_MUL>, grid, 256, 0, st)(P); break;
     }
   }
 }
@@ -1548,7 +1575,7 @@ static void launch_scan(const dsk_layer_spec& sp, const float* proj, int ld_proj
   const int NP = (N + 3) & ~3;
   const size_t smem = (size_t)TB * (2 + 2 * NP + 2 * PB) * 4;
   const int need = (N + 31) / 32;     // float4 groups of state per thread
-#define DSK_SCAN(RQ) ssd_scan<RQ><<<grid, threads, smem, st>>>(proj, ld_proj, 0, inner + (int)ssd_channels(sp), xbc, ld_xbc, 0, inner, inner + G * N, \
+#define DSK_SCAN(RQ) launch_next(ssd_scan<RQ>, grid, threads, smem, st)(proj, ld_proj, 0, inner + (int)ssd_channels(sp), xbc, ld_xbc, 0, inner, inner + G * N, \
                                                                L.dt_bias, L.A_log, L.D, state, out, inner, T, H, P, N, G, PB, TB)
   if (need <= 1) DSK_SCAN(1); else if (need <= 2) DSK_SCAN(2); else if (need <= 3) DSK_SCAN(3); else if (need <= 4) DSK_SCAN(4);
   else if (need <= 6) DSK_SCAN(6); else DSK_SCAN(8);
@@ -1572,7 +1599,7 @@ static void launch_hgrn2(const dsk_layer_spec& sp, const float* proj, int ld, fl
   while (TB > 16 && (size_t)2 * TB * (2 * NP + PB) * 4 > 160 * 1024) TB /= 2;
   const size_t smem = (size_t)2 * TB * (2 * NP + PB) * 4;
   const int need = (N + 4 * TPC - 1) / (4 * TPC);     // float4 groups of state per thread
-#define DSK_LIN(RQ, C) hgrn2_scan<RQ, C><<<grid, threads, smem, st>>>(proj, ld, 0, H * N, 2 * H * N, state, out, H * P, T, H, N, P, PB, TB)
+#define DSK_LIN(RQ, C) launch_next(hgrn2_scan<RQ, C>, grid, threads, smem, st)(proj, ld, 0, H * N, 2 * H * N, state, out, H * P, T, H, N, P, PB, TB)
   if (TPC == 32) { if (need <= 1) DSK_LIN(1, 32); else DSK_LIN(2, 32); }
   else if (TPC == 16) { if (need <= 1) DSK_LIN(1, 16); else if (need <= 2) DSK_LIN(2, 16); else if (need <= 3) DSK_LIN(3, 16); else DSK_LIN(4, 16); }
   else if (need <= 1) DSK_LIN(1, 8); else if (need <= 2) DSK_LIN(2, 8); else if (need <= 3) DSK_LIN(3, 8); else if (need <= 4) DSK_LIN(4, 8);
@@ -1593,7 +1620,7 @@ static void launch_lin_scan(bool delta, const float* q, const float* k, int ldq,
   const int PB = warps * CW;
   const dim3 grid((unsigned)H, (unsigned)((P + (nst ? 1 : 0) + PB - 1) / PB));
   const size_t smem = lin_scan_smem(4 * TPC * RQ, PB, warps, CW);
-#define DSK_LSCAN(D, A, B, C) lin_scan<D, A, B, C><<<grid, 32 * (warps + kLinStage), smem, st>>>(q, k, ldq, hs, rep, v, ldv, rec, state, out, ldo, T, H, N, P, PB, nst, den)
+#define DSK_LSCAN(D, A, B, C) launch_next(lin_scan<D, A, B, C>, grid, 32 * (warps + kLinStage), smem, st)(q, k, ldq, hs, rep, v, ldv, rec, state, out, ldo, T, H, N, P, PB, nst, den)
 #define DSK_LSCANS(D) do { if (N > 128) DSK_LSCAN(D, 32, 2, 4); else if (CPT == 2) { if (N <= 32) DSK_LSCAN(D, 8, 1, 2); else if (N <= 64) DSK_LSCAN(D, 16, 1, 2); else DSK_LSCAN(D, 32, 1, 2); } \
   else { if (N <= 32) DSK_LSCAN(D, 8, 1, 4); else if (N <= 64) DSK_LSCAN(D, 16, 1, 4); else DSK_LSCAN(D, 32, 1, 4); } } while (0)
   if (delta) DSK_LSCANS(true); else DSK_LSCANS(false);
@@ -1605,7 +1632,7 @@ static void launch_lin_decode(int mode, const GdnP& D, const float* decay, float
                               float* out, int ldo, cudaStream_t st, const MlstmP& memory = MlstmP{1.f, nullptr, nullptr}) {
   const int NG = std::min(kLinDecodeThreads / ((D.P + 3) / 4), D.N), need = (D.N + NG - 1) / NG;
   const size_t smem = lin_decode_smem(D.N, D.P);
-#define DSK_LDEC(X, R) lin_decode<X, R><<<D.H, kLinDecodeThreads, smem, st>>>(D, decay, state, norm_w, eps, gate_off, alpha, out, ldo, memory)
+#define DSK_LDEC(X, R) launch_next(lin_decode<X, R>, D.H, kLinDecodeThreads, smem, st)(D, decay, state, norm_w, eps, gate_off, alpha, out, ldo, memory)
 #define DSK_LDECS(X) do { if (need <= 1) DSK_LDEC(X, 1); else if (need <= 2) DSK_LDEC(X, 2); else if (need <= 4) DSK_LDEC(X, 4); else if (need <= 8) DSK_LDEC(X, 8); else DSK_LDEC(X, 16); } while (0)
   if (mode == LIN_DELTA) DSK_LDECS(LIN_DELTA); else if (mode == LIN_MLSTM) DSK_LDECS(LIN_MLSTM); else DSK_LDECS(LIN_PLAIN);
 #undef DSK_LDECS
@@ -1624,10 +1651,10 @@ static void gdn_forward(State* S, const HLayer& L, LayerState& ls, int ldp, cons
   }
   const int nb = (T + kLinBlk - 1) / kLinBlk;
   const size_t smem = (size_t)(2 * kLinBlk * (NP + 4) + 2 * kLinBlk * kLinBlk + 8 * kLinBlk * kLinBlk) * 4;
-  gdn_prepare<<<dim3((unsigned)nb, (unsigned)(G + (RV + 255) / 256)), 256, smem, st>>>(D, S->lq, S->lk, S->lv, NP, S->lrec);
+  launch_next(gdn_prepare, dim3((unsigned)nb, (unsigned)(G + (RV + 255) / 256)), 256, smem, st)(D, S->lq, S->lk, S->lv, NP, S->lrec);
   launch_lin_scan(true, S->lq, S->lk, G * NP, NP, H / G, S->lv, RV, S->lrec, ls.lin, S->lout, RV, T, H, N, P, st);
-  if (sp.gdn_conv > 1) { conv_ring_store<<<(CH + 127) / 128, 128, 0, st>>>(S->b0, ldp, (int)a.dq, ls.hist, D.ring, T, CH, sp.gdn_conv, S->d_ctl); S->launches++; }
-  head_rmsnorm<<<(unsigned)(((long long)T * H + 7) / 8), 256, 0, st>>>(S->lout, RV, L.lin_norm, out, ldo, T, H, P, eps, S->b0 + a.dg, ldp, alpha);
+  if (sp.gdn_conv > 1) { launch_next(conv_ring_store, (CH + 127) / 128, 128, 0, st)(S->b0, ldp, (int)a.dq, ls.hist, D.ring, T, CH, sp.gdn_conv, S->d_ctl); S->launches++; }
+  launch_next(head_rmsnorm, (unsigned)(((long long)T * H + 7) / 8), 256, 0, st)(S->lout, RV, L.lin_norm, out, ldo, T, H, P, eps, S->b0 + a.dg, ldp, alpha, 0, 0, nullptr, nullptr);
   S->launches += 3;
 }
 
@@ -1641,7 +1668,7 @@ static void lightning_forward(State* S, const HLayer& L, LayerState& ls, int ldp
     S->launches++;
     return;
   }
-  lin_gram<<<dim3((unsigned)((T + kLinBlk - 1) / kLinBlk), (unsigned)H), 256, (size_t)2 * kLinBlk * (((N + 3) & ~3) + 4) * 4, st>>>(S->b0, S->b0 + HN, ldp, L.log_decay, T, H, N, S->lrec);
+  launch_next(lin_gram, dim3((unsigned)((T + kLinBlk - 1) / kLinBlk), (unsigned)H), 256, (size_t)2 * kLinBlk * (((N + 3) & ~3) + 4) * 4, st)(S->b0, S->b0 + HN, ldp, L.log_decay, T, H, N, S->lrec);
   launch_lin_scan(false, S->b0, S->b0 + HN, ldp, N, 1, S->b0 + 2 * HN, ldp, S->lrec, ls.lin, S->lout, HP, T, H, N, P, st);
   S->launches += 2;
 }
@@ -1658,10 +1685,10 @@ static void mlstm_forward(State* S, const HLayer& L, LayerState& ls, int ldp, co
     return;
   }
   float *gi = S->lgate, *gf = gi + (size_t)H * T, *gm = gf + (size_t)H * T;
-  mlstm_gates<<<H, 256, 0, st>>>(S->b0, ldp, (int)a.i, (int)a.f, sp.lin_gate_cap, T, H, gi, gf, gm, mst);
-  mlstm_gram<<<dim3((unsigned)((T + kLinBlk - 1) / kLinBlk), (unsigned)H), 256, (size_t)2 * kLinBlk * (((N + 3) & ~3) + 4) * 4, st>>>(S->b0, S->b0 + HN, ldp, gi, gf, gm, T, H, N, S->lrec);
+  launch_next(mlstm_gates, H, 256, 0, st)(S->b0, ldp, (int)a.i, (int)a.f, sp.lin_gate_cap, T, H, gi, gf, gm, mst);
+  launch_next(mlstm_gram, dim3((unsigned)((T + kLinBlk - 1) / kLinBlk), (unsigned)H), 256, (size_t)2 * kLinBlk * (((N + 3) & ~3) + 4) * 4, st)(S->b0, S->b0 + HN, ldp, gi, gf, gm, T, H, N, S->lrec);
   launch_lin_scan(false, S->b0, S->b0 + HN, ldp, N, 1, S->b0 + 2 * HN, ldp, S->lrec, ls.lin, S->lout, HP, T, H, N, P, st, nst, S->lden);
-  head_rmsnorm<<<(unsigned)(((long long)T * H + 7) / 8), 256, 0, st>>>(S->lout, HP, L.mnorm, out, HP, T, H, P, eps, S->b0 + a.g, ldp, 1.f, P, 1, S->lden, gm);
+  launch_next(head_rmsnorm, (unsigned)(((long long)T * H + 7) / 8), 256, 0, st)(S->lout, HP, L.mnorm, out, HP, T, H, P, eps, S->b0 + a.g, ldp, 1.f, P, 1, S->lden, gm);
   S->launches += 4;
 }
 
@@ -1677,35 +1704,35 @@ static void launch_attn(const float* qa, const float* cache, float* out, int T, 
   }
   const dim3 grid((unsigned)((T + TQ - 1) / TQ), (unsigned)((H + HB - 1) / HB), (unsigned)NS);
   const size_t smem = ((size_t)8 * R + (size_t)32 * (R + 1)) * 4;
-  if (R <= 128) latent_swa_attn<float, 4><<<grid, 256, smem, st>>>(qa, cache, out, T, H, R, ctl, mask, window, ring, scale, TQ, NS, part, sink);
-  else if (R <= 256) latent_swa_attn<float, 8><<<grid, 256, smem, st>>>(qa, cache, out, T, H, R, ctl, mask, window, ring, scale, TQ, NS, part, sink);
-  else if (R <= 512) latent_swa_attn<float, 16><<<grid, 256, smem, st>>>(qa, cache, out, T, H, R, ctl, mask, window, ring, scale, TQ, NS, part, sink);
-  else latent_swa_attn<float, 32><<<grid, 256, smem, st>>>(qa, cache, out, T, H, R, ctl, mask, window, ring, scale, TQ, NS, part, sink);
-  if (NS > 1) latent_swa_merge<<<dim3((unsigned)(T * H), (unsigned)((R + 127) / 128)), 128, 0, st>>>(part, out, R, NS);
+  if (R <= 128) launch_next(latent_swa_attn<float, 4>, grid, 256, smem, st)(qa, cache, out, T, H, R, ctl, mask, window, ring, scale, TQ, NS, part, sink);
+  else if (R <= 256) launch_next(latent_swa_attn<float, 8>, grid, 256, smem, st)(qa, cache, out, T, H, R, ctl, mask, window, ring, scale, TQ, NS, part, sink);
+  else if (R <= 512) launch_next(latent_swa_attn<float, 16>, grid, 256, smem, st)(qa, cache, out, T, H, R, ctl, mask, window, ring, scale, TQ, NS, part, sink);
+  else launch_next(latent_swa_attn<float, 32>, grid, 256, smem, st)(qa, cache, out, T, H, R, ctl, mask, window, ring, scale, TQ, NS, part, sink);
+  if (NS > 1) launch_next(latent_swa_merge, dim3((unsigned)(T * H), (unsigned)((R + 127) / 128)), 128, 0, st)(part, out, R, NS, nullptr, 0, 1, 0, 0, 1.f);
 }
 
 // LM head on the wanted rows [first, first + count) of the chunk whose normalised rows are in S->h -> S->logits [count][vocab]
-static void enqueue_head(dsk_model* m, dsk_state* s, int first, int count, cudaStream_t st) {
+static void enqueue_head(dsk_model* m, dsk_state* s, int first, int count, float* logits, cudaStream_t st) {
   Model* M = m->hy;
   State* S = s->hy;
   const dsk_hybrid_config& c = M->c;
-  GemmP P = gp(S->h, c.dim, c.tie_head ? M->embed.p : M->head.p, c.dim, S->logits, c.vocab_size, count, c.vocab_size, c.dim);
+  GemmP P = gp(S->h, c.dim, c.tie_head ? M->embed.p : M->head.p, c.dim, logits, c.vocab_size, count, c.vocab_size, c.dim);
   P.a_map = S->d_want + first; P.alpha = c.logit_scale; P.lim = c.logit_softcap;
   linear(S, c.quant == DSK_BF16, c.logit_softcap > 0.f ? HEPI_SOFTCAP : HEPI_STORE, P, 1, st);
 }
 
 // the model's norm over the T rows of `in` (width values each): stored into `out`, or added into it times alpha (mode 1)
 static void norm_rows(const dsk_hybrid_config& c, State* S, const float* in, const float* w, const float* b, float* out, int T, int mode, float alpha, cudaStream_t st) {
-  if (c.norm_kind == DSK_NORM_LAYER) layer_norm<<<T, 256, 0, st>>>(in, c.dim, w, b, out, c.dim, c.dim, c.norm_eps, mode, alpha, nullptr, 0);
-  else if (mode == 0 && c.norm_groups == 1) rms_open<<<T, 256, 0, st>>>(const_cast<float*>(in), nullptr, nullptr, w, out, c.dim, c.norm_eps);   // (adds nothing: the row is only read)
-  else group_rmsnorm<float><<<T, 256, 0, st>>>(in, c.dim, w, out, c.dim, c.dim, c.norm_groups, c.norm_eps, mode, alpha, nullptr, 0);
+  if (c.norm_kind == DSK_NORM_LAYER) launch_next(layer_norm, T, 256, 0, st)(in, c.dim, w, b, out, c.dim, c.dim, c.norm_eps, mode, alpha, nullptr, 0);
+  else if (mode == 0 && c.norm_groups == 1) launch_next(rms_open, T, 256, 0, st)(const_cast<float*>(in), nullptr, nullptr, w, out, c.dim, c.norm_eps);   // (adds nothing: the row is only read)
+  else launch_next(group_rmsnorm<float>, T, 256, 0, st)(in, c.dim, w, out, c.dim, c.dim, c.norm_groups, c.norm_eps, mode, alpha, nullptr, 0, nullptr, 0);
   S->launches++;
 }
 
 template <typename... A>
 static void launch_rms_add_norm(int T, cudaStream_t st, A... a) {
-  if (T <= kAttnSplitTokens) rms_add_norm<1024><<<T, 1024, 0, st>>>(a...);
-  else rms_add_norm<256><<<T, 256, 0, st>>>(a...);
+  if (T <= kAttnSplitTokens) launch_next(rms_add_norm<1024>, T, 1024, 0, st)(a...);
+  else launch_next(rms_add_norm<256>, T, 256, 0, st)(a...);
 }
 
 static bool fused_norms(const dsk_hybrid_config& c) {
@@ -1726,6 +1753,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
   State* S = s->hy;
   const dsk_hybrid_config& c = M->c;
   const bool bf = c.quant == DSK_BF16;
+  chain_step = T <= kAttnSplitTokens || (bf && T <= 256);
   const bool sandwich = c.block == DSK_BLOCK_SANDWICH, post = c.block == DSK_BLOCK_POST, pre = c.block == DSK_BLOCK_PRE;
   const int W = c.dim;
   const float mult = c.residual_mult;
@@ -1733,12 +1761,12 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
   const int nb = c.bigram_buckets;
   float* keep_emb = S->xin ? S->xin + W : S->emb;   // the embedding output again, for a layer loop
   const int ld_keep = S->xin ? 2 * W : W;
-  if (bf) embed_rows<__nv_bfloat16><<<T, 256, 0, st>>>(S->d_tok, (const __nv_bfloat16*)M->embed.p, W, S->x, es, nb > 0 ? (const __nv_bfloat16*)M->bigram.p : nullptr,
+  if (bf) launch_next(embed_rows<__nv_bfloat16>, T, 256, 0, st)(S->d_tok, (const __nv_bfloat16*)M->embed.p, W, S->x, es, nb > 0 ? (const __nv_bfloat16*)M->bigram.p : nullptr,
                                                        nb, c.bigram_mul_prev, c.bigram_mul_cur, S->d_ctl, S->d_prev, keep_emb, ld_keep);
-  else embed_rows<float><<<T, 256, 0, st>>>(S->d_tok, (const float*)M->embed.p, W, S->x, es, nb > 0 ? (const float*)M->bigram.p : nullptr, nb, c.bigram_mul_prev,
+  else launch_next(embed_rows<float>, T, 256, 0, st)(S->d_tok, (const float*)M->embed.p, W, S->x, es, nb > 0 ? (const float*)M->bigram.p : nullptr, nb, c.bigram_mul_prev,
                                             c.bigram_mul_cur, S->d_ctl, S->d_prev, keep_emb, ld_keep);
   S->launches++;
-  if (nb > 0) { carry_token<<<1, 1, 0, st>>>(S->d_tok, T, S->d_prev); S->launches++; }   // the next step's first token pairs with this step's last
+  if (nb > 0) { launch_next(carry_token, 1, 1, 0, st)(S->d_tok, T, S->d_prev); S->launches++; }   // the next step's first token pairs with this step's last
   if (pos0 < 0) S->tl_used = 0;   // a captured step records no events
   const bool tl = S->timeline && pos0 >= 0;
   auto MK = [&](const char* label) { if (tl) mark(S, label, st); };
@@ -1761,9 +1789,9 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       if (c.canon_taps <= 0) return S->x;
       float* ring = ls.canon ? ls.canon + (size_t)which * (c.canon_taps - 1) * W : nullptr;
       const int ty = (T + kCanonTokens - 1) / kCanonTokens;
-      canon_conv<<<dim3((unsigned)((W + 127) / 128), (unsigned)ty), 128, 0, st>>>(S->x, W, taps, ring, S->h, W, T, W, c.canon_taps, S->d_ctl);
+      launch_next(canon_conv, dim3((unsigned)((W + 127) / 128), (unsigned)ty), 128, 0, st)(S->x, W, taps, ring, S->h, W, T, W, c.canon_taps, S->d_ctl);
       S->launches++;
-      if (ty > 1 && c.canon_taps > 1) { canon_history<<<(W + 127) / 128, 128, 0, st>>>(S->x, W, ring, T, W, c.canon_taps, S->d_ctl); S->launches++; }
+      if (ty > 1 && c.canon_taps > 1) { launch_next(canon_history, (W + 127) / 128, 128, 0, st)(S->x, W, ring, T, W, c.canon_taps, S->d_ctl); S->launches++; }
       return S->h;
     };
     auto close_post = [&](const HTensor& rg, const float* rg_b, const float* close_w, const float* close_b) {
@@ -1783,7 +1811,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         G.bias = rg_b;
         linear(S, bf, HEPI_SIGMUL, G, 1, st);
       }
-      close_open_small<<<(W + 127) / 128, 128, 0, st>>>(S->y, close_w, mult, c.norm_eps, S->x, W, next_taps, next_ring, S->h, T, W, c.canon_taps, S->d_ctl);
+      launch_next(close_open_small, (W + 127) / 128, 128, 0, st)(S->y, close_w, mult, c.norm_eps, S->x, W, next_taps, next_ring, S->h, T, W, c.canon_taps, S->d_ctl);
       S->launches++;
     };
     auto ring_of = [&](size_t run_i, int which) { return S->L[run_i].canon ? S->L[run_i].canon + (size_t)which * (c.canon_taps - 1) * W : nullptr; };
@@ -1792,18 +1820,18 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
     if (post) { if (!h_ready) hin = open_post(L.canon1, 0); }
     else if (pre) {   // a pass of the layer loop opens with its vector (and, but for the first, the embedding) added to the stream
       const bool again = c.loop_embed && run.pass > 0;
-      rms_open<<<T, 256, 0, st>>>(S->x, again ? S->emb : nullptr, run.pass >= 0 ? M->loop_step + (size_t)run.pass * W : nullptr, L.norm1, S->h, W, c.norm_eps);
+      launch_next(rms_open, T, 256, 0, st)(S->x, again ? S->emb : nullptr, run.pass >= 0 ? M->loop_step + (size_t)run.pass * W : nullptr, L.norm1, S->h, W, c.norm_eps);
       S->launches++;
     } else if (!h_ready) {
       if (run.pass >= 0 && c.loop_in) {   // a pass of the layer loop opens with a product over [stream | embedding], its vector as the bias
-        if (!xin_ready) { copy_rows<<<T, 256, 0, st>>>(S->x, W, S->xin, 2 * W, W); S->launches++; }
+        if (!xin_ready) { launch_next(copy_rows, T, 256, 0, st)(S->x, W, S->xin, 2 * W, W); S->launches++; }
         xin_ready = false;
         GemmP In = gp(S->xin, 2 * W, M->loop_in.p, 2 * W, S->x, W, T, W, 2 * W);
         In.bias = M->loop_step + (size_t)run.pass * W;
         linear(S, bf, HEPI_STORE, In, 1, st);
         MK("loop.in");
       } else if (run.pass >= 0) {   // a pass of the layer loop opens with its own vector added to the residual stream
-        add_row<<<T, 256, 0, st>>>(S->x, W, M->loop_step + (size_t)run.pass * W, W);
+        launch_next(add_row, T, 256, 0, st)(S->x, W, M->loop_step + (size_t)run.pass * W, W);
         S->launches++;
       }
       norm_rows(c, S, S->x, L.norm1, L.norm1_bias, S->h, T, 0, 0.f, st);
@@ -1813,9 +1841,9 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
     if (c.token_shift && hs_ready) { hin = S->hs; hs_ready = false; }   // the previous run's last kernel shifted already
     else if (c.token_shift) {      // the mixer reads its input blended with the previous token's; the step's last row is carried on
       const int ty = (T + kCanonTokens - 1) / kCanonTokens;
-      token_shift<<<dim3((unsigned)((W + 127) / 128), (unsigned)ty), 128, 0, st>>>(hin, W, L.shift, ls.shift, S->hs, W, T, W, S->d_ctl);
+      launch_next(token_shift, dim3((unsigned)((W + 127) / 128), (unsigned)ty), 128, 0, st)(hin, W, L.shift, ls.shift, S->hs, W, T, W, S->d_ctl);
       S->launches++;
-      if (ty > 1) { shift_carry<<<(W + 127) / 128, 128, 0, st>>>(hin, W, ls.shift, T, W); S->launches++; }
+      if (ty > 1) { launch_next(shift_carry, (W + 127) / 128, 128, 0, st)(hin, W, ls.shift, T, W); S->launches++; }
       hin = S->hs;
     }
     // the closing norm of this run's last sublayer, fused with what opens the next run (its pass vector and first norm) or the head
@@ -1834,7 +1862,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         return;
       }
       const float* row = next && next->pass >= 0 ? M->loop_step + (size_t)next->pass * W : nullptr;
-      layer_norm_add_norm<<<T, 256, 0, st>>>(S->y, wb, S->x, row, next ? M->L[next->layer].norm1 : M->final_norm, S->h, W, c.norm_eps, mult);
+      launch_next(layer_norm_add_norm, T, 256, 0, st)(S->y, wb, S->x, row, next ? M->L[next->layer].norm1 : M->final_norm, S->h, W, c.norm_eps, mult);
       S->launches++;
       h_ready = true;
     };
@@ -1861,7 +1889,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       if (reads) {
         linear(S, bf, HEPI_STORE, gp(hin, W, L.qkv.p, W, S->b0, ldp, T, ldp, W), 1, st);
         MK("att.qk");
-        qk_norm_rope<<<qk_grid, 256, 0, st>>>(S->b0, S->b2, HD, nullptr, nullptr, GD, GV, ldp, 0, 0, L.q_norm, nullptr, c.norm_eps, D, sp.rot_dims, L.rot_freq,
+        launch_next(qk_norm_rope, qk_grid, 256, 0, st)(S->b0, S->b2, HD, nullptr, nullptr, GD, GV, ldp, 0, 0, L.q_norm, nullptr, c.norm_eps, D, sp.rot_dims, L.rot_freq,
                                         L.rot_mag, S->d_ctl, nullptr, nullptr, ring, keep, nullptr, 0.f, nullptr, sp.rot_layout, sp.att_qk_norm, ConvP{nullptr, nullptr, 0, 1, 0});
       } else if (sp.att_value_proj) {   // one product for the stacked q / k / v rows; the first value-mixing layer keeps its values for the later ones
         const int ld = ldp;
@@ -1872,24 +1900,26 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         if (sp.mixer2 == DSK_MIX_GDN && !tl) {   // the second mixer on its own stream: it shares nothing with the first but the projections
           CKL(cudaEventRecord(S->ev_fork, st));
           CKL(cudaStreamWaitEvent(S->side, S->ev_fork, 0));
+          plain_next = true;
           gdn_forward(S, L, ls, ldp, lay, S->b3 + H * V, ldo, sp.mix2_scale, c.norm_eps, T, S->side);
           CKL(cudaEventRecord(S->ev_join, S->side));
+          plain_next = true;
         }
         const bool blend = sp.att_vmix && li != M->vmix_first;
         ConvP cv{nullptr, nullptr, 0, 1, 0};
         if (sp.att_conv > 0) cv = ConvP{L.conv_w, ls.hist, sp.att_conv, sp.att_conv - 1 + kConvSpare, sp.att_conv > 1 && T <= kConvSpare};
-        qk_norm_rope<<<qk_grid, 256, cv.w ? (size_t)8 * D * 4 : 0, st>>>(S->b0, S->b2, HD, S->b0 + HD, S->b0 + HD + GD, GD, GV, ld, ld, ld, L.q_norm, L.k_norm, c.norm_eps, D, sp.rot_dims,
+        launch_next(qk_norm_rope, qk_grid, 256, cv.w ? (size_t)8 * D * 4 : 0, st)(S->b0, S->b2, HD, S->b0 + HD, S->b0 + HD + GD, GD, GV, ld, ld, ld, L.q_norm, L.k_norm, c.norm_eps, D, sp.rot_dims,
                                         L.rot_freq, L.rot_mag, S->d_ctl, kc, vc, ring, keep, blend ? S->vfirst : nullptr, L.vmix,
                                         sp.att_vmix && li == M->vmix_first ? S->vfirst : nullptr, sp.rot_layout, sp.att_qk_norm, cv);
         if (sp.att_conv > 1 && !cv.store) {   // a long step stores its last inputs after its convolutions
-          conv_ring_store<<<(HD + GD + GV + 127) / 128, 128, 0, st>>>(S->b0, ld, 0, ls.hist, cv.ring, T, HD + GD + GV, sp.att_conv, S->d_ctl);
+          launch_next(conv_ring_store, (HD + GD + GV + 127) / 128, 128, 0, st)(S->b0, ld, 0, ls.hist, cv.ring, T, HD + GD + GV, sp.att_conv, S->d_ctl);
           S->launches++;
         }
       } else {
         linear(S, bf, HEPI_STORE, gp(hin, W, L.q.p, W, S->b0, HD, T, HD, W), 1, st);
         linear(S, bf, HEPI_STORE, gp(hin, W, L.kproj.p, W, S->b1, GD, T, GD, W), 1, st);
         MK("att.qk");
-        qk_norm_rope<<<qk_grid, 256, 0, st>>>(S->b0, S->b2, HD, S->b1, nullptr, GD, GV, HD, GD, GD, L.q_norm, L.k_norm, c.norm_eps, D, sp.rot_dims, L.rot_freq,
+        launch_next(qk_norm_rope, qk_grid, 256, 0, st)(S->b0, S->b2, HD, S->b1, nullptr, GD, GV, HD, GD, GD, L.q_norm, L.k_norm, c.norm_eps, D, sp.rot_dims, L.rot_freq,
                                         L.rot_mag, S->d_ctl, kc, vc, ring, keep, nullptr, 0.f, nullptr, sp.rot_layout, sp.att_qk_norm, ConvP{nullptr, nullptr, 0, 1, 0});
       }
       S->launches++;
@@ -1899,7 +1929,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         for (int t0 = 0; t0 < T; t0 += kPrefillQ) {
           const int Tq = std::min(kPrefillQ, T - t0), qpos0 = pos0 + t0;
           const int first = mask_first(sp.att_mask, sp.att_window, qpos0), nk = std::min(keep, first), Lk = nk + qpos0 + Tq - first;
-          pack_ring_kv<float><<<Lk, 256, 0, st>>>(kc, vc, S->kf, S->vf, first, Lk, ring, G, D, V, nk, keep);
+          launch_next(pack_ring_kv<float>, Lk, 256, 0, st)(kc, vc, S->kf, S->vf, first, Lk, ring, G, D, V, nk, keep);
           S->launches++;
           MK("att.pack");
           GemmP Sc = gp(S->b2 + (size_t)t0 * HD, HD, S->kf, D, S->sc, Lk, Tq, Lk, D);
@@ -1909,11 +1939,11 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
           float* pr = S->sc;
           if (sp.att_talk) {
             const long long n = (long long)Tq * Lk;
-            mix_heads<<<(unsigned)((n + 127) / 128), 128, (size_t)(H * H + H * 128) * 4, st>>>(S->sc, S->sc2, L.talk, H, n);
+            launch_next(mix_heads, (unsigned)((n + 127) / 128), 128, (size_t)(H * H + H * 128) * 4, st)(S->sc, S->sc2, L.talk, H, n);
             S->launches++;
             pr = S->sc2;
           }
-          softmax_band<<<dim3((unsigned)Tq, (unsigned)H), 128, 0, st>>>(pr, Tq, Lk, first, qpos0, sp.att_mask, sp.att_window, nk, sm);
+          launch_next(softmax_band, dim3((unsigned)Tq, (unsigned)H), 128, 0, st)(pr, Tq, Lk, first, qpos0, sp.att_mask, sp.att_window, nk, sm);
           S->launches++;
           MK("att.softmax");
           GemmP Ov = gp(pr, Lk, S->vf, Lk, S->b3 + (size_t)t0 * ldo, ldo, Tq, V, Lk);
@@ -1921,19 +1951,19 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
           linear(S, false, HEPI_STORE, Ov, H, st);
           MK("att.pv");
         }
-        if (gate) { gate_rows<<<T, 256, 0, st>>>(S->b3, ldo, gate, ldp, H * V, gate_head ? V : 1); S->launches++; }   // heads *= sigmoid(g h)
+        if (gate) { launch_next(gate_rows, T, 256, 0, st)(S->b3, ldo, gate, ldp, H * V, gate_head ? V : 1); S->launches++; }   // heads *= sigmoid(g h)
       } else {
         int NS = 1;
         if (T <= kAttnSplitTokens) NS = std::max(1, std::min((std::min(sp.att_window, ring) + keep + 31) / 32, kAttnSplitMax));
         const int GL = gqa_key_heads(H, G, sp.att_talk != 0);   // without score mixing the key heads are dealt over CTAs
-        gqa_attn<<<dim3((unsigned)T, (unsigned)NS, (unsigned)(G / GL)), 256, gqa_attn_smem_floats(GL * rep, GL, D, V, sp.att_talk != 0) * 4, st>>>(
+        launch_next(gqa_attn, dim3((unsigned)T, (unsigned)NS, (unsigned)(G / GL)), 256, gqa_attn_smem_floats(GL * rep, GL, D, V, sp.att_talk != 0) * 4, st)(
             S->b2, kc, vc, S->b3, sp.att_talk ? L.talk : nullptr, T, H, G, D, V, S->d_ctl, sp.att_mask, sp.att_window, ring, sp.att_scale, NS, S->part, sm,
             NS > 1 ? nullptr : gate, ldp, gate_head, ldo, lscale);
-        if (NS > 1) latent_swa_merge<<<dim3((unsigned)(T * H), (unsigned)((V + 127) / 128)), 128, 0, st>>>(S->part, S->b3, V, NS, gate, ldp, H, gate_head, ldo, lscale);
+        if (NS > 1) launch_next(latent_swa_merge, dim3((unsigned)(T * H), (unsigned)((V + 127) / 128)), 128, 0, st)(S->part, S->b3, V, NS, gate, ldp, H, gate_head, ldo, lscale);
         S->launches += NS > 1 ? 2 : 1;
         MK("att.decode");
       }
-      if (sp.mixer2 == DSK_MIX_GDN && !tl) CKL(cudaStreamWaitEvent(st, S->ev_join, 0));
+      if (sp.mixer2 == DSK_MIX_GDN && !tl) { CKL(cudaStreamWaitEvent(st, S->ev_join, 0)); plain_next = true; }
       else if (sp.mixer2 == DSK_MIX_GDN) {   // timeline: one after the other
         gdn_forward(S, L, ls, ldp, lay, S->b3 + H * V, ldo, sp.mix2_scale, c.norm_eps, T, st);
         MK("gdn");
@@ -1948,11 +1978,11 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       const int ldi = Q + RW;
       MK("norm");
       linear(S, bf, HEPI_STORE, gp(hin, W, L.in2.p, W, S->b1, ldi, T, ldi, W), 1, st);              // [query latent | key / value latent | rotated key part]
-      group_rmsnorm<float><<<T, 256, 0, st>>>(S->b1, ldi, L.dq_norm, S->b2, Q, Q, 1, c.norm_eps, 0, 0.f, nullptr, 0);
+      launch_next(group_rmsnorm<float>, T, 256, 0, st)(S->b1, ldi, L.dq_norm, S->b2, Q, Q, 1, c.norm_eps, 0, 0.f, nullptr, 0, nullptr, 0);
       S->launches++;
       linear(S, bf, HEPI_STORE, gp(S->b2, Q, L.uq.p, Q, S->b0, H * DK, T, H * DK, Q), 1, st);       // q [T][H][D | Rd]
       const bool portion = pos0 >= 0 && T >= kPrefillMin && S->prefill_keys > 0;
-      mla_prepare<<<T, 256, 0, st>>>(S->b1 + Q, ldi, L.dkv_norm, c.norm_eps, S->b0, portion ? nullptr : S->b2, H, D, Rd, R, sp.rot_dims, L.rot_freq,
+      launch_next(mla_prepare, T, 256, 0, st)(S->b1 + Q, ldi, L.dkv_norm, c.norm_eps, S->b0, portion ? nullptr : S->b2, H, D, Rd, R, sp.rot_dims, L.rot_freq,
                                      L.rot_mag, sp.rot_layout, S->d_ctl, cache, L.ring);
       S->launches++;
       MK("att.q+latent");
@@ -1965,7 +1995,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         for (int t0 = 0; t0 < T; t0 += kPrefillQ) {
           const int Tq = std::min(kPrefillQ, T - t0), qpos0 = pos0 + t0;
           const int first = mask_first(sp.att_mask, sp.att_window, qpos0), Lk = qpos0 + Tq - first;
-          ring_rows<<<(Lk + 255) / 256, 256, 0, st>>>(first, Lk, L.ring, S->d_rows);
+          launch_next(ring_rows, (Lk + 255) / 256, 256, 0, st)(first, Lk, L.ring, S->d_rows);
           GemmP K = gp(cache, RW, L.uk.p, R, S->kf, H * D, Lk, H * D, R);
           K.a_map = S->d_rows;
           linear(S, bf, HEPI_STORE, K, 1, st);
@@ -1973,13 +2003,13 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
           Vp.a_map = S->d_rows;
           linear(S, bf, HEPI_STORE, Vp, 1, st);
           MK("att.kv_up");
-          pack_mla_kv<<<Lk, 256, 0, st>>>(S->kf, S->vf, cache, S->d_rows, (float*)S->kb, (float*)S->vt, Lk, H, D, Rd, R, V);
+          launch_next(pack_mla_kv, Lk, 256, 0, st)(S->kf, S->vf, cache, S->d_rows, (float*)S->kb, (float*)S->vt, Lk, H, D, Rd, R, V);
           MK("att.pack");
           GemmP Sc = gp(S->b0 + (size_t)t0 * H * DK, H * DK, S->kb, DK, S->sc, Lk, Tq, Lk, DK);
           Sc.sA = DK; Sc.sW = (long long)Lk * DK; Sc.sC = (long long)Tq * Lk; Sc.alpha = sp.att_scale;
           linear(S, false, HEPI_STORE, Sc, H, st);
           MK("att.scores");
-          softmax_band<<<dim3((unsigned)Tq, (unsigned)H), 128, 0, st>>>(S->sc, Tq, Lk, first, qpos0, sp.att_mask, sp.att_window, 0, sm);
+          launch_next(softmax_band, dim3((unsigned)Tq, (unsigned)H), 128, 0, st)(S->sc, Tq, Lk, first, qpos0, sp.att_mask, sp.att_window, 0, sm);
           MK("att.softmax");
           GemmP Ov = gp(S->sc, Lk, S->vt, Lk, S->b3 + (size_t)t0 * H * V, H * V, Tq, V, Lk);
           Ov.sA = (long long)Tq * Lk; Ov.sW = (long long)V * Lk; Ov.sC = V;
@@ -2043,7 +2073,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       MK("lin.in");
       lightning_forward(S, L, ls, pw, T, st);
       MK("lin.scan");
-      group_rmsnorm<float><<<T, 256, 0, st>>>(S->lout, HP, L.mnorm, S->b3, HP, HP, 1, c.norm_eps, 0, 0.f, nullptr, 0, S->b0 + 2 * HN + HP, pw);
+      launch_next(group_rmsnorm<float>, T, 256, 0, st)(S->lout, HP, L.mnorm, S->b3, HP, HP, 1, c.norm_eps, 0, 0.f, nullptr, 0, S->b0 + 2 * HN + HP, pw);
       S->launches++;
       MK("lin.norm");
       GemmP P = gp(S->b3, HP, L.o.p, HP, sink.C, W, T, W, HP);
@@ -2059,7 +2089,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       MK("lin.in");
       launch_hgrn2(sp, S->b0, pw, ls.lin, S->b2, T, st);
       MK("lin.scan");
-      head_rmsnorm<<<(unsigned)(((long long)T * H + 7) / 8), 256, 0, st>>>(S->b2, HP, L.lin_norm, S->b3, HP, T, H, sp.lin_vdim, c.norm_eps);
+      launch_next(head_rmsnorm, (unsigned)(((long long)T * H + 7) / 8), 256, 0, st)(S->b2, HP, L.lin_norm, S->b3, HP, T, H, sp.lin_vdim, c.norm_eps, nullptr, 0, 1.f, 0, 0, nullptr, nullptr);
       S->launches += 2;
       MK("lin.norm");
       GemmP P = gp(S->b3, HP, L.o.p, HP, sink.C, W, T, W, HP);
@@ -2071,12 +2101,12 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       MK("norm");
       linear(S, bf, HEPI_STORE, gp(hin, W, L.in.p, W, S->b0, pw, T, pw, W), 1, st);
       MK("ssd.in");
-      causal_conv_silu<<<dim3((unsigned)((ch + 127) / 128), (unsigned)T), 128, 0, st>>>(S->b0 + inner, pw, L.conv_w, L.conv_b, ls.hist, S->b1, ch, T, ch, sp.ssm_conv);
-      if (sp.ssm_conv > 1) conv_history_update<<<(ch + 127) / 128, 128, 0, st>>>(S->b0 + inner, pw, ls.hist, T, ch, sp.ssm_conv);
+      launch_next(causal_conv_silu, dim3((unsigned)((ch + 127) / 128), (unsigned)T), 128, 0, st)(S->b0 + inner, pw, L.conv_w, L.conv_b, ls.hist, S->b1, ch, T, ch, sp.ssm_conv);
+      if (sp.ssm_conv > 1) launch_next(conv_history_update, (ch + 127) / 128, 128, 0, st)(S->b0 + inner, pw, ls.hist, T, ch, sp.ssm_conv);
       MK("ssd.conv");
       launch_scan(sp, S->b0, pw, S->b1, ch, L, ls.ssm, S->b2, T, st);
       MK("ssd.scan");
-      group_rmsnorm<float><<<T, 256, 0, st>>>(S->b2, inner, L.mnorm, S->b3, inner, inner, sp.ssm_norm_groups, c.norm_eps, 0, 0.f, nullptr, 0);
+      launch_next(group_rmsnorm<float>, T, 256, 0, st)(S->b2, inner, L.mnorm, S->b3, inner, inner, sp.ssm_norm_groups, c.norm_eps, 0, 0.f, nullptr, 0, nullptr, 0);
       S->launches += 4;
       MK("ssd.norm");
       GemmP P = gp(S->b3, inner, L.o.p, inner, sink.C, W, T, W, inner);
@@ -2091,7 +2121,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       linear(S, bf, HEPI_STORE, gp(hin, W, L.q.p, W, S->b0, H * D, T, H * D, W), 1, st);
       if (L.owner == li) {
         linear(S, bf, HEPI_STORE, gp(hin, W, L.dkv.p, W, S->b1, R, T, R, W), 1, st);
-        group_rmsnorm<float><<<T, 256, 0, st>>>(S->b1, R, L.dkv_norm, cache, R, R, 1, c.norm_eps, 0, 0.f, S->d_ctl, O.ring);
+        launch_next(group_rmsnorm<float>, T, 256, 0, st)(S->b1, R, L.dkv_norm, cache, R, R, 1, c.norm_eps, 0, 0.f, S->d_ctl, O.ring, nullptr, 0);
         S->launches++;
       }
       MK("att.q+latent");
@@ -2102,7 +2132,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         for (int t0 = 0; t0 < T; t0 += kPrefillQ) {
           const int Tq = std::min(kPrefillQ, T - t0), qpos0 = pos0 + t0;
           const int first = mask_first(sp.att_mask, sp.att_window, qpos0), Lk = qpos0 + Tq - first;
-          ring_rows<<<(Lk + 255) / 256, 256, 0, st>>>(first, Lk, O.ring, S->d_rows);
+          launch_next(ring_rows, (Lk + 255) / 256, 256, 0, st)(first, Lk, O.ring, S->d_rows);
           GemmP K = gp(cache, R, L.uk.p, R, S->kf, H * D, Lk, H * D, R);
           K.a_map = S->d_rows;
           linear(S, bf, HEPI_STORE, K, 1, st);
@@ -2110,14 +2140,14 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
           Vp.a_map = S->d_rows;
           linear(S, bf, HEPI_STORE, Vp, 1, st);
           MK("att.kv_up");
-          if (bf) pack_keys_values<__nv_bfloat16><<<Lk, 256, 0, st>>>(S->kf, S->vf, (__nv_bfloat16*)S->kb, (__nv_bfloat16*)S->vt, Lk, H, D, V);
-          else pack_keys_values<float><<<Lk, 256, 0, st>>>(S->kf, S->vf, (float*)S->kb, (float*)S->vt, Lk, H, D, V);
+          if (bf) launch_next(pack_keys_values<__nv_bfloat16>, Lk, 256, 0, st)(S->kf, S->vf, (__nv_bfloat16*)S->kb, (__nv_bfloat16*)S->vt, Lk, H, D, V);
+          else launch_next(pack_keys_values<float>, Lk, 256, 0, st)(S->kf, S->vf, (float*)S->kb, (float*)S->vt, Lk, H, D, V);
           GemmP Sc = gp(S->b0 + (size_t)t0 * H * D, H * D, S->kb, D, S->sc, Lk, Tq, Lk, D);
           Sc.sA = D; Sc.sW = (long long)Lk * D; Sc.sC = (long long)Tq * Lk; Sc.alpha = sp.att_scale;
           MK("att.pack");
           linear(S, bf, HEPI_STORE, Sc, H, st);
           MK("att.scores");
-          softmax_band<<<dim3((unsigned)Tq, (unsigned)H), 128, 0, st>>>(S->sc, Tq, Lk, first, qpos0, sp.att_mask, sp.att_window, 0, ScoreMods{});
+          launch_next(softmax_band, dim3((unsigned)Tq, (unsigned)H), 128, 0, st)(S->sc, Tq, Lk, first, qpos0, sp.att_mask, sp.att_window, 0, ScoreMods{});
           GemmP Ov = gp(S->sc, Lk, S->vt, Lk, S->b3 + (size_t)t0 * H * V, H * V, Tq, V, Lk);
           Ov.sA = (long long)Tq * Lk; Ov.sW = (long long)V * Lk; Ov.sC = V;
           MK("att.softmax");
@@ -2161,7 +2191,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         launch_rms_add_norm(T, st, S->y, nullptr, 0, nullptr, nullptr, L.close1, S->x, S->x, W, L.norm2, S->h, W, c.norm_eps, mult);
         S->launches++;
       } else if (fuse) {
-        layer_norm_add_norm<<<T, 256, 0, st>>>(S->y, L.close1, S->x, nullptr, L.norm2, S->h, W, c.norm_eps, mult);
+        launch_next(layer_norm_add_norm, T, 256, 0, st)(S->y, L.close1, S->x, nullptr, L.norm2, S->h, W, c.norm_eps, mult);
         S->launches++;
       } else {
         norm_rows(c, S, S->y, L.close1, nullptr, S->x, T, 1, mult, st);
@@ -2170,7 +2200,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       MK("norm");
     }
     if (pre && sp.ff_kind != DSK_FF_NONE) {
-      rms_open<<<T, 256, 0, st>>>(S->x, nullptr, nullptr, L.norm2, S->h, W, c.norm_eps);
+      launch_next(rms_open, T, 256, 0, st)(S->x, nullptr, nullptr, L.norm2, S->h, W, c.norm_eps);
       S->launches++;
       hin = S->h;
       MK("norm");
@@ -2206,7 +2236,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       GemmP Rt = gp(hin, W, L.router, W, S->b0, ldz, T, ldz, W);   // router: fp32 weights in every mode (and the shared expert's weight)
       Rt.bias = sp.ff_router == DSK_ROUTER_TOP_SOFTMAX ? L.router_b : nullptr;
       linear(S, false, HEPI_STORE, Rt, 1, st);
-      moe_route<<<T, 128, (size_t)(2 * E + top + groups) * 4, st>>>(S->b0, ldz, sp.ff_router == DSK_ROUTER_SIGMOID ? L.correction : nullptr, E, top, sp.ff_router_scale,
+      launch_next(moe_route, T, 128, (size_t)(2 * E + top + groups) * 4, st)(S->b0, ldz, sp.ff_router == DSK_ROUTER_SIGMOID ? L.correction : nullptr, E, top, sp.ff_router_scale,
                                                                     S->d_idx, S->wgt, sp.ff_router == DSK_ROUTER_SOFTMAX_GROUPS ? 2 : sp.ff_router == DSK_ROUTER_TOP_SOFTMAX ? 1 : 0,
                                                                     groups, sp.ff_groups > 0 ? sp.ff_groups_keep : 1, shared ? S->wsh : nullptr);
       S->launches++;
@@ -2230,7 +2260,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         MK("moe.down");
       } else {
         const int bm = bf ? 128 : 64;   // rows per tile of the product kernel that follows (gemm_mma / gemm_tiled)
-        moe_plan<<<1, 1024, (size_t)2 * E * 4, st>>>(S->d_idx, pairs, E, bm, S->d_perm, S->d_tiles, S->d_ntiles);
+        launch_next(moe_plan, 1, 1024, (size_t)2 * E * 4, st)(S->d_idx, pairs, E, bm, S->d_perm, S->d_tiles, S->d_ntiles);
         S->launches++;
         G.tiles = S->d_tiles; G.n_tiles = S->d_ntiles; G.a_map = S->d_perm; G.a_div = top; G.c_map = S->d_perm;
         Dn.tiles = S->d_tiles; Dn.n_tiles = S->d_ntiles; Dn.a_map = S->d_perm; Dn.a_div = 1; Dn.c_map = S->d_perm;
@@ -2253,10 +2283,10 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         }
       }
       if (combine_in_norm) {   // x += ln(sum_k w_k y_k): the weighted sum of the experts' outputs is taken by the closing layer norm as it reads its row
-        layer_norm<<<T, 256, 0, st>>>(S->b3, W, L.close2, L.norm2_bias, S->x, W, W, c.norm_eps, 1, mult, S->wgt, top);
+        launch_next(layer_norm, T, 256, 0, st)(S->b3, W, L.close2, L.norm2_bias, S->x, W, W, c.norm_eps, 1, mult, S->wgt, top);
         S->launches++;
       } else if (!frms) {   // (sandwich blocks of RMS norms combine as they close)
-        moe_combine<<<T, 256, 0, st>>>(sink.C, W, S->b3, S->wgt, top, W, sink.alpha, sink.epi == HEPI_ADD ? 1 : 0, shared ? ysh : nullptr, S->wsh);
+        launch_next(moe_combine, T, 256, 0, st)(sink.C, W, S->b3, S->wgt, top, W, sink.alpha, sink.epi == HEPI_ADD ? 1 : 0, shared ? ysh : nullptr, S->wsh);
         S->launches++;
       }
       MK("moe.combine");
@@ -2279,23 +2309,28 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       // decode-sized steps of post-norm blocks: the normed addition and the next layer's token shift in one launch over 128-channel CTAs
       if (post && c.canon_taps <= 0 && T <= kCloseOpenTokens && !trace) {
         const bool next_shift = c.token_shift && has_next;
-        rms_add_shift_small<<<(W + 127) / 128, 128, 0, st>>>(S->h, L.snorm, mult, c.norm_eps, S->x, W, next_shift ? M->L[M->runs[ri + 1].layer].shift : nullptr,
+        launch_next(rms_add_shift_small, (W + 127) / 128, 128, 0, st)(S->h, L.snorm, mult, c.norm_eps, S->x, W, next_shift ? M->L[M->runs[ri + 1].layer].shift : nullptr,
                                                              next_shift ? S->L[ri + 1].shift : nullptr, S->hs, T, W, S->d_ctl);
         hs_ready = next_shift;
-      } else group_rmsnorm<float><<<T, 256, 0, st>>>(S->h, W, L.snorm, S->x, W, W, 1, c.norm_eps, 1, mult, nullptr, 0);
+      } else launch_next(group_rmsnorm<float>, T, 256, 0, st)(S->h, W, L.snorm, S->x, W, W, 1, c.norm_eps, 1, mult, nullptr, 0, nullptr, 0);
       S->launches++;
       MK("side");
     }
     if (trace) CKL(cudaMemcpyAsync(trace + ri * (size_t)T * W, S->x, (size_t)T * W * 4, cudaMemcpyDeviceToDevice, st));
   }
   if (n_want > 0) {   // final norm of every row, LM head on the first group of wanted rows (enqueue_head does the others)
-    if (pre) { rms_open<<<T, 256, 0, st>>>(S->x, nullptr, nullptr, M->final_norm, S->h, W, c.norm_eps); S->launches++; }
+    if (pre) { launch_next(rms_open, T, 256, 0, st)(S->x, nullptr, nullptr, M->final_norm, S->h, W, c.norm_eps); S->launches++; }
     else if (!h_ready) norm_rows(c, S, S->x, M->final_norm, M->final_norm_b, S->h, T, 0, 0.f, st);
-    enqueue_head(m, s, 0, std::min(n_want, S->head_rows), st);
+    enqueue_head(m, s, 0, std::min(n_want, S->head_rows), pos0 < 0 ? s->logits : S->logits, st);   // a captured step leaves its one row in the state
     MK("head");
   }
   CKL(cudaGetLastError());
   return 0;
+}
+
+// arg-max of the state's logits into Ctrl::argmax_key, which is 0 ahead of it; a few CTAs: one takes 13 us for 100 k logits, mostly waiting
+static void launch_argmax(dsk_state* s, int vocab) {
+  launch_next(argmax_row, (unsigned)std::max(1, std::min(vocab / 4096, 32)), 256, 0, s->stream)(s->logits, vocab, s->ctrl);
 }
 
 // tokens [n] at positions pos0.. of the state's sequence; want: ascending indices into tokens whose logits go to host_logits
@@ -2323,17 +2358,18 @@ static int forward_chunk(dsk_model* m, dsk_state* s, const int32_t* tokens, int 
     while (wi + nw < n_want && want[wi + nw] < o + T) { S->h_want[nw] = want[wi + nw] - o; nw++; }
     CK(cudaMemcpyAsync(S->d_tok, S->h_tok, (size_t)T * 4, cudaMemcpyHostToDevice, s->stream));
     if (nw) CK(cudaMemcpyAsync(S->d_want, S->h_want, (size_t)nw * 4, cudaMemcpyHostToDevice, s->stream));
-    set_ctl<<<1, 1, 0, s->stream>>>(S->d_ctl, pos0 + o);
+    launch_next(set_ctl, 1, 1, 0, s->stream)(S->d_ctl, pos0 + o);
     if (host_layers) { CK(cudaMalloc((void**)&d_trace, M->runs.size() * (size_t)T * c.dim * 4)); }
     if (enqueue_chunk(m, s, T, nw, d_trace, s->stream, pos0 + o)) { if (d_trace) cudaFree(d_trace); return -2; }
     for (int g0 = 0; g0 < nw; g0 += S->head_rows) {   // the LM head in groups of head_rows wanted rows
       const int gn = std::min(S->head_rows, nw - g0);
-      if (g0 > 0) enqueue_head(m, s, g0, gn, s->stream);
+      if (g0 > 0) enqueue_head(m, s, g0, gn, S->logits, s->stream);
       if (host_logits) CK(cudaMemcpyAsync(host_logits + (size_t)(wi + g0) * c.vocab_size, S->logits, (size_t)gn * c.vocab_size * 4, cudaMemcpyDeviceToHost, s->stream));
     }
     if (nw) {   // the last wanted row stays in the state for the samplers
       CK(cudaMemcpyAsync(s->logits, S->logits + (size_t)((nw - 1) % S->head_rows) * c.vocab_size, (size_t)c.vocab_size * 4, cudaMemcpyDeviceToDevice, s->stream));
-      argmax_row<<<1, 1024, 0, s->stream>>>(s->logits, c.vocab_size, s->ctrl, nullptr, nullptr, 0);
+      CK(cudaMemsetAsync(&s->ctrl->argmax_key, 0, sizeof(s->ctrl->argmax_key), s->stream));
+      launch_argmax(s, c.vocab_size);
     }
     timeline_report(S, T);
     if (host_layers) {
@@ -2362,17 +2398,16 @@ static int decode_greedy(dsk_model* m, dsk_state* s, int start_pos, int n_steps,
   if (start_pos != S->next_pos) return fail(-4, "dsk_decode_greedy: start_pos %d must follow the state's sequence (at %d)", start_pos, S->next_pos);
   const int one = 0;
   CK(cudaMemcpyAsync(S->d_want, &one, 4, cudaMemcpyHostToDevice, s->stream));
-  set_ctl<<<1, 1, 0, s->stream>>>(S->d_ctl, start_pos);
+  launch_next(set_ctl, 1, 1, 0, s->stream)(S->d_ctl, start_pos);
   CK(cudaMemsetAsync(s->step, 0, sizeof(int), s->stream));
   CK(cudaStreamSynchronize(s->stream));
   if (!S->step_graph) {
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-    greedy_feed<<<1, 1, 0, s->stream>>>(s->ctrl, S->d_tok, s->token_log, s->step);
+    launch_next(greedy_feed, 1, 1, 0, s->stream)(s->ctrl, S->d_tok, s->token_log, s->step);
     int rc = enqueue_chunk(m, s, 1, 1, nullptr, s->stream);
-    cudaMemcpyAsync(s->logits, S->logits, (size_t)c.vocab_size * 4, cudaMemcpyDeviceToDevice, s->stream);
-    argmax_row<<<1, 1024, 0, s->stream>>>(s->logits, c.vocab_size, s->ctrl, nullptr, nullptr, 0);
-    advance_ctl<<<1, 1, 0, s->stream>>>(S->d_ctl, 1);
+    launch_argmax(s, c.vocab_size);
+    launch_next(advance_ctl, 1, 1, 0, s->stream)(S->d_ctl, 1);
     cudaError_t e = cudaStreamEndCapture(s->stream, &g);
     if (rc || e != cudaSuccess) return fail(-2, "capturing the decode step failed: %s", cudaGetErrorString(e));
     CK(cudaGraphInstantiate(&S->step_graph, g, 0));

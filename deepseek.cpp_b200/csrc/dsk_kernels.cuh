@@ -63,6 +63,13 @@ __device__ __forceinline__ void mbar_wait(uint32_t bar, uint32_t parity) {
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   }
 }
+// Kernels of one stream that are launched as programmatic dependents (launch_next in dsk_hybrid_host.cuh): grid_wait returns once the kernel ahead
+// has finished and its writes are visible; grid_release lets the kernel behind start, up to its own grid_wait.  Every kernel of such a chain
+// runs grid_wait in every thread ahead of its first access to memory that a kernel writes, so that the end of a kernel implies the
+// end of all kernels ahead of it.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_enter() { grid_wait(); grid_release(); }
 __device__ __forceinline__ uint4 lds128(uint32_t a) {
   uint4 r;
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "r"(a));

@@ -46,6 +46,7 @@ __device__ __forceinline__ float conv_silu_at(const float* __restrict__ proj, in
 // stores the step's last taps - 1 inputs in the history ring (steps longer than kConvSpare tokens, after their convolutions)
 __global__ void conv_ring_store(const float* __restrict__ proj, int ld, int off, float* __restrict__ hist, int ring, int T, int ch, int taps,
                                 const int* __restrict__ ctl) {
+  grid_enter();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ch) return;
   for (int tau = max(0, T - (taps - 1)); tau < T; tau++) hist[(size_t)((ctl[0] + tau) % ring) * ch + c] = proj[(size_t)tau * ld + off + c];
@@ -84,6 +85,7 @@ struct GdnP {
 };
 __global__ void __launch_bounds__(256) gdn_prepare(const GdnP D, float* __restrict__ qn, float* __restrict__ kn, float* __restrict__ vn, int NP,
                                                    float* __restrict__ rec) {
+  grid_enter();
   extern __shared__ __align__(16) float sm[];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, blk = blockIdx.x, t0 = blk * kLinBlk, nt = min(kLinBlk, D.T - t0);
   const int pos0 = D.ctl[0], KD = D.G * D.N, CH = 2 * KD + D.H * D.P;
@@ -164,6 +166,7 @@ __global__ void __launch_bounds__(256) gdn_prepare(const GdnP D, float* __restri
 // Plain form: the records of a step (M and the decays) from q and k as they are.  Grid (blocks, heads).
 __global__ void __launch_bounds__(256) lin_gram(const float* __restrict__ q, const float* __restrict__ k, int ld, const float* __restrict__ log_decay,
                                                 int T, int H, int N, float* __restrict__ rec) {
+  grid_enter();
   extern __shared__ __align__(16) float sm[];
   const int pitch = ((N + 3) & ~3) + 4, tid = threadIdx.x, t0 = blockIdx.x * kLinBlk, nt = min(kLinBlk, T - t0), h = blockIdx.y;
   float* sq = sm;
@@ -191,6 +194,7 @@ __global__ void __launch_bounds__(256) lin_gram(const float* __restrict__ q, con
 __device__ __forceinline__ float log_sigmoid_f(float z) { return fminf(z, 0.f) - log1pf(expf(-fabsf(z))); }
 __global__ void __launch_bounds__(256) mlstm_gates(const float* __restrict__ proj, int ld, int i_off, int f_off, float cap, int T, int H,
                                                    float* __restrict__ gi, float* __restrict__ gf, float* __restrict__ gm, float* __restrict__ m) {
+  grid_enter();
   __shared__ float sF[256], sB[256];
   const int h = blockIdx.x, tid = threadIdx.x, per = (T + 255) / 256, t0 = min(T, tid * per), t1 = min(T, t0 + per);
   float F = 0.f, B = -INFINITY;
@@ -222,6 +226,7 @@ __global__ void __launch_bounds__(256) mlstm_gates(const float* __restrict__ pro
 // mLSTM: the records of a step from q and k as they are (q is scaled by 1 / sqrt(N) here) and the gates above.  Grid (blocks, heads).
 __global__ void __launch_bounds__(256) mlstm_gram(const float* __restrict__ q, const float* __restrict__ k, int ld, const float* __restrict__ gi,
                                                   const float* __restrict__ gf, const float* __restrict__ gm, int T, int H, int N, float* __restrict__ rec) {
+  grid_enter();
   extern __shared__ __align__(16) float sm[];
   __shared__ float sf[kLinBlk], si[kLinBlk], sx[kLinBlk + 1];
   const int pitch = ((N + 3) & ~3) + 4, tid = threadIdx.x, t0 = blockIdx.x * kLinBlk, nt = min(kLinBlk, T - t0), h = blockIdx.y;
@@ -295,6 +300,7 @@ template <bool DELTA, int TPC, int RQ, int CPT>
 __global__ void __launch_bounds__(320) lin_scan(const float* __restrict__ q, const float* __restrict__ k, int ldq, int hs, int rep,
                                                 const float* __restrict__ v, int ldv, const float* __restrict__ rec, float* __restrict__ state,
                                                 float* __restrict__ out, int ldo, int T, int H, int N, int P, int PB, float* __restrict__ nst, float* __restrict__ den) {
+  grid_enter();
   extern __shared__ __align__(16) float sm[];
   constexpr int C = kLinBlk, PITCH = 4 * TPC * RQ, CW = CPT * (32 / TPC), VB = 32 / CPT;
   const int per = 2 * C * PITCH + C * PB + kRecFloats;     // one buffer: k [C][PITCH], q [C][PITCH], v [C][PB], record
@@ -510,6 +516,7 @@ template <int MODE, int RN>
 __global__ void __launch_bounds__(kLinDecodeThreads) lin_decode(const GdnP D, const float* __restrict__ decay, float* __restrict__ state,
                                                                 const float* __restrict__ norm_w, float eps, int gate_off, float alpha,
                                                                 float* __restrict__ out, int ldo, const MlstmP X) {
+  grid_enter();
   constexpr bool DELTA = MODE == LIN_DELTA, MLSTM = MODE == LIN_MLSTM;
   extern __shared__ __align__(16) float sm[];
   __shared__ float red[33], gb[5];

@@ -90,6 +90,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc5(const GemmP P, const T
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  grid_enter();                                              // barriers and TMEM are set up under the kernel ahead
   const int n_mt = P.tiles ? *P.n_tiles : T.n_mt;
   const int cols = DUAL ? T.bn / 2 : T.bn;                   // output columns of a tile
   const int n_nt = (P.N + cols - 1) / cols, total = n_mt * n_nt, nk = (P.K + kTcDepth - 1) / kTcDepth;
@@ -198,6 +199,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc5(const GemmP P, const T
 // out[i] = bf16(A[a_map ? a_map[i] / a_div : i]), K values each (K a multiple of 8), eight per thread
 __global__ void __launch_bounds__(256) bf16_rows(const float* __restrict__ A, int lda, const int* __restrict__ a_map, int a_div, __nv_bfloat16* __restrict__ out,
                                                  int rows, int K, int vec) {
+  grid_enter();
   const int per = K / 8;
   const long long n = (long long)rows * per;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
