@@ -14,7 +14,7 @@
 //   gemv_one          the same for one row (a decoded token): eight 16-byte weight loads in flight per lane
 //   causal_conv_silu  depthwise causal convolution over the chunk continuing from the carried (taps - 1) inputs, + SiLU
 //   ssd_scan          the state-space recurrence S <- exp(-exp(A_log) dt) S + dt B x^T, y = S^T C + D x, gated by silu(z)
-//   latent_swa_attn   softmax attention over a sliding window of cached latents with absorbed key up-projection
+//   decode_attn       softmax attention of decode-sized steps over cached keys and values, or cached latents with absorbed key up-projection
 //   layer_norm        (x - mean) / sqrt(var + eps) * w, stored or added into the residual
 //   qk_norm_rope      RMS norm over a whole query / key projection, partial interleaved rotary positions from a frequency table,
 //                     keys and values written into their ring caches
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(128) canon_conv(const float* __restrict__ x, i
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// RMS norm in groups.  Row t of `in` (n values) is cut into `groups` equal consecutive parts; each part is divided by
+// RMS norm in groups, grid (rows, groups).  Row t of `in` (n values) is cut into `groups` equal consecutive parts; each part is divided by
 // sqrt(mean(part^2) + eps) and the row is multiplied by w.  mode 0: out[row] = result, where row = (ctl ? ctl[0] : 0) + t,
 // taken modulo `ring` (a ring cache of latents; ring = 0 means rows are not wrapped).  mode 1: out[t] += alpha * result.
 // gate (nullable, row pitch ld_gate): the result is multiplied by it entry by entry.
@@ -233,18 +233,38 @@ __global__ void __launch_bounds__(256) group_rmsnorm(const float* __restrict__ i
     }
     return;
   }
-  for (int g = 0; g < groups; g++) {
-    float ss = 0.f;
-    for (int i = threadIdx.x; i < gs; i += blockDim.x) { const float v = x[g * gs + i]; ss += v * v; }
-    ss = block_sum(ss, red);
-    const float sc = 1.f / sqrtf(ss / (float)gs + eps);
-    for (int i = threadIdx.x; i < gs; i += blockDim.x) {
-      const int c = g * gs + i;
-      float v = x[c] * sc * w[c];
-      if (gate) v *= gate[(size_t)t * ld_gate + c];
-      if (mode == 0) o[c] = from_f<OT>(v);
-      else o[c] = from_f<OT>(to_f<OT>(o[c]) + alpha * v);
+  // a CTA per group, everything it reads in flight ahead of the sum (a decoded token's 4 groups one after the other, each with two waits for
+  // memory, took 12 to 20 us; side by side 5)
+  const int c0 = (int)blockIdx.y * gs;
+  constexpr int NV = 4;
+  float v[NV], wt[NV], old[NV], ss = 0.f;
+  const bool cached = gs <= 256 * NV;
+  if (cached) {
+#pragma unroll
+    for (int k = 0; k < NV; k++) {
+      const int i = threadIdx.x + 256 * k;
+      v[k] = i < gs ? x[c0 + i] : 0.f;
+      wt[k] = i < gs ? w[c0 + i] : 0.f;
+      old[k] = i < gs && mode != 0 ? to_f<OT>(o[c0 + i]) : 0.f;
     }
+#pragma unroll
+    for (int k = 0; k < NV; k++) ss = fmaf(v[k], v[k], ss);
+  } else {
+#pragma unroll 8
+    for (int i = threadIdx.x; i < gs; i += 256) { const float xv = x[c0 + i]; ss = fmaf(xv, xv, ss); }
+  }
+  const float sc = 1.f / sqrtf(block_sum(ss, red) / (float)gs + eps);
+  auto put = [&](int i, float xv, float wv, float ov) {
+    float r = xv * sc * wv;
+    if (gate) r *= gate[(size_t)t * ld_gate + c0 + i];
+    o[c0 + i] = from_f<OT>(mode == 0 ? r : ov + alpha * r);
+  };
+  if (cached) {
+#pragma unroll
+    for (int k = 0; k < NV; k++) { const int i = threadIdx.x + 256 * k; if (i < gs) put(i, v[k], wt[k], old[k]); }
+  } else {
+#pragma unroll 4
+    for (int i = threadIdx.x; i < gs; i += 256) put(i, x[c0 + i], w[c0 + i], mode != 0 ? to_f<OT>(o[c0 + i]) : 0.f);
   }
 }
 
@@ -946,6 +966,37 @@ __global__ void causal_conv_silu(const float* __restrict__ in, int ld_in, const 
   }
   out[(size_t)t * ld_out + c] = silu_f(acc);
 }
+// The same for steps of at most kConvShort tokens, history included: thread = channel
+constexpr int kConvShort = 4;
+__global__ void __launch_bounds__(128) causal_conv_silu_short(const float* __restrict__ in, int ld_in, const float* __restrict__ w, const float* __restrict__ b,
+                                                              float* __restrict__ hist, float* __restrict__ out, int ld_out, int T, int ch, int taps) {
+  grid_enter();
+  const int c = blockIdx.x * blockDim.x + threadIdx.x, back = taps - 1;
+  if (c >= ch) return;
+  float cur[kConvShort];
+#pragma unroll
+  for (int t = 0; t < kConvShort; t++) cur[t] = t < T ? in[(size_t)t * ld_in + c] : 0.f;
+  const float bias = b[c];
+  float acc[kConvShort];
+#pragma unroll
+  for (int t = 0; t < kConvShort; t++) acc[t] = bias;
+  // inputs in time order: back carried ones, then the step's; input u is under tap u - t of output t
+#pragma unroll 4
+  for (int u = 0; u < back + T; u++) {
+    float v = 0.f;
+    if (u < back) v = hist[(size_t)u * ch + c];
+    else {
+#pragma unroll
+      for (int t = 0; t < kConvShort; t++) if (u - back == t) v = cur[t];
+    }
+#pragma unroll
+    for (int t = 0; t < kConvShort; t++)
+      if (t < T && u >= t && u - t < taps) acc[t] = fmaf(w[(size_t)c * taps + u - t], v, acc[t]);
+    if (u >= T) hist[(size_t)(u - T) * ch + c] = v;   // (ascending: slot u - T has been read)
+  }
+#pragma unroll
+  for (int t = 0; t < kConvShort; t++) if (t < T) out[(size_t)t * ld_out + c] = silu_f(acc[t]);
+}
 __global__ void conv_history_update(const float* __restrict__ in, int ld_in, float* __restrict__ hist, int T, int ch, int taps) {
   grid_enter();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1243,109 +1294,166 @@ __device__ __forceinline__ float mod_score(const ScoreMods& sm, float s, int dis
   return s;
 }
 
-template <typename CT, int RV>
-__global__ void __launch_bounds__(256) latent_swa_attn(const float* __restrict__ qa, const CT* __restrict__ cache, float* __restrict__ out,
-                                                       int T, int H, int R, const int* __restrict__ ctl, int mask, int window, int ring,
-                                                       float scale, int TQ, int NS, float* __restrict__ part, const float* __restrict__ sink) {
+// ---------------------------------------------------------------------------------------------------------------------
+// Softmax attention of decode-sized steps over cached rows (no mixing of the heads): a CTA holds up to 8 query rows that share their keys (heads
+// of one key group x neighbouring tokens) and walks its share of the visible keys in tiles of 32.  Key and value rows of a tile arrive together
+// (cp.async, everything in flight).  Scores: lane = key, the warps share the depth, so that a key value read from shared memory serves all
+// query rows, and the warps' parts are joined there; then warp w holds row w's softmax state; values: thread = columns, a value serves all rows.
+// (One warp per row, as before, read every key and value of the tile once per row: 8 x the shared-memory traffic, which bounded the kernel.)
+// KV: keys and values are the same rows (absorbed latents: Dv = D).
+// ---------------------------------------------------------------------------------------------------------------------
+struct DecodeAttn {
+  const float *q, *kc, *vc;      // q rows [token][head][D]; caches of row pitch ldk / ldv, key group g at column g * D / g * Dv
+  float *out, *part;
+  const int* ctl;
+  const float* gate;             // (see gqa_attn)
+  int T, H, G, D, Dv, ldk, ldv, mask, span, ring, TQ, HB, NS, ld_gate, gate_head, ld_out;
+  float scale, alpha;
+  ScoreMods mods;
+};
+__host__ __device__ inline int attn_pitch(int n) { return ((n + 3) & ~3) + 4; }
+__host__ __device__ inline size_t decode_attn_floats(int D, int Dv, bool kv) {
+  return (size_t)40 * attn_pitch(D) + (kv ? 0 : (size_t)32 * attn_pitch(Dv)) + 8 * 8 * 32 + 32 * 8 + 3 * 8;
+}
+template <bool KV, int CV>   // CV: value columns per thread (CV * 256 >= Dv)
+__global__ void __launch_bounds__(256) decode_attn(const DecodeAttn P) {
+  extern __shared__ __align__(16) float sm[];
+  const int D = P.D, Dv = P.Dv, pd = attn_pitch(D), pv = KV ? pd : attn_pitch(Dv), rep = P.H / P.G, hblocks = (rep + P.HB - 1) / P.HB;
+  float* qs = sm;                                    // [8][pd]
+  float* ks = qs + 8 * pd;                           // [32][pd]
+  float* vs = KV ? ks : ks + 32 * pd;                // [32][pv]
+  float* red = (KV ? ks + 32 * pd : vs + 32 * pv);   // [8 warps][8 rows][32 keys]
+  float* pt = red + 8 * 8 * 32;                      // [32 keys][8 rows] weights
+  float* corr = pt + 32 * 8;                         // [8], then m [8] and l [8] at the end
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int g = (int)blockIdx.y / hblocks, hb = (int)blockIdx.y % hblocks, tq0 = (int)blockIdx.x * P.TQ;
+  // query row r of the CTA: token tq0 + r % TQ, head hb * HB + r / TQ of the group
+  auto row_t = [&](int r) { return tq0 + r % P.TQ; };
+  auto row_h = [&](int r) { return hb * P.HB + r / P.TQ; };
+  auto live = [&](int r) { return r < P.TQ * P.HB && row_t(r) < P.T && row_h(r) < rep; };
   grid_enter();
-  extern __shared__ float sm[];
-  const int NW = 8, HB = NW / TQ;
-  float* qs = sm;                 // [NW][R]
-  float* ks = sm + NW * R;        // [32][R + 1]
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int tq0 = blockIdx.x * TQ, t = tq0 + (w % TQ), h = blockIdx.y * HB + w / TQ;
-  const bool active = t < T && h < H;
-  const int pos0 = ctl[0];
-  for (int r = lane; r < R; r += 32) qs[w * R + r] = active ? qa[((size_t)t * H + h) * R + r] * scale : 0.f;
-  const int i = pos0 + t;
-  const int lo_w = mask_first(mask, window, i), hi_w = i;
-  int lo = mask_first(mask, window, pos0 + tq0), hi = pos0 + min(T, tq0 + TQ) - 1;
-  if (NS > 1) {   // this CTA's share of the key range (whole tiles of 32)
-    const int tiles = (hi - lo + 32) / 32, per = (tiles + NS - 1) / NS;
-    const int lo_s = lo + (int)blockIdx.z * per * 32;
-    hi = min(hi, lo_s + per * 32 - 1);
-    lo = lo_s;
+  const int pos0 = P.ctl[0], keep = P.mods.keep;
+  const int j_lo = mask_first(P.mask, P.span, pos0 + tq0), nk = min(keep, j_lo);
+  int lo = 0, hi = nk + pos0 + min(P.T, tq0 + P.TQ) - 1 - j_lo;   // visible keys of all rows in one index space: kept ones, then the range
+  if (P.NS > 1) {
+    const int tiles = (hi + 32) / 32, per = (tiles + P.NS - 1) / P.NS;
+    lo = (int)blockIdx.z * per * 32;
+    hi = min(hi, lo + per * 32 - 1);
   }
-  float m = -1e30f, l = 0.f, acc[RV];
+  const bool vk = (D & 3) == 0 && (P.ldk & 3) == 0, vv = (Dv & 3) == 0 && (P.ldv & 3) == 0;   // cudaMalloc'd caches: rows on 16-byte boundaries
+  auto stage = [&](float* dst, const float* src, int ld, int off, int n, int pitch, bool vec, int j0) {
+    for (int jj = w; jj < 32; jj += 8) {
+      const int v = j0 + jj;
+      float* d = dst + jj * pitch;
+      if (v > hi) { for (int r = lane; r < n; r += 32) d[r] = 0.f; continue; }
+      const float* s = src + (size_t)cache_row(v < nk ? v : j_lo + v - nk, keep, P.ring) * ld + off;
+      if (vec) { for (int r = lane * 4; r < n; r += 128) cp_async_16(d + r, s + r, 16); }
+      else for (int r = lane; r < n; r += 32) d[r] = s[r];
+    }
+  };
+  const int d4 = (D + 3) >> 2;
+  for (int r = 0; r < 8; r++) {
+    const bool on = live(r);
+    const float* src = P.q + ((size_t)row_t(r) * P.H + g * rep + row_h(r)) * D;
+    for (int e = tid; e < 4 * d4; e += 256) qs[r * pd + e] = on && e < D ? src[e] * P.scale : 0.f;
+  }
+  if (D & 3) for (int jj = tid; jj < 32; jj += 256) for (int e = D; e < 4 * d4; e++) ks[jj * pd + e] = 0.f;   // (a depth that ends inside a group of four)
+  const bool mine = live(w);
+  const int i_w = pos0 + row_t(w), lo_w = mask_first(P.mask, P.span, i_w), h_w = g * rep + row_h(w);
+  float m = -1e30f, l = 0.f, acc[8][CV];
 #pragma unroll
-  for (int k = 0; k < RV; k++) acc[k] = 0.f;
+  for (int r = 0; r < 8; r++)
+#pragma unroll
+    for (int k = 0; k < CV; k++) acc[r][k] = 0.f;
   for (int j0 = lo; j0 <= hi; j0 += 32) {
     __syncthreads();
-    // warp w stages the tile's rows w, w + 8, ..: one ring row index per row, then (fp32 caches of a width that is a multiple of 4)
-    // 16-byte loads with all of a lane's loads in flight before the first store
-    for (int jj = w; jj < 32; jj += 8) {
-      const int j = j0 + jj;
-      float* dst = ks + jj * (R + 1);
-      if (j > hi) { for (int r = lane; r < R; r += 32) dst[r] = 0.f; continue; }
-      const CT* src = cache + (size_t)(j % ring) * R;
-      if (sizeof(CT) == 4 && (R & 3) == 0) {
-        const float4* s4 = reinterpret_cast<const float4*>(src);
-        const int n4 = R >> 2;
-#pragma unroll 8
-        for (int q = lane; q < n4; q += 32) {
-          const float4 v = s4[q];
-          dst[4 * q] = v.x; dst[4 * q + 1] = v.y; dst[4 * q + 2] = v.z; dst[4 * q + 3] = v.w;
+    stage(ks, P.kc, P.ldk, g * D, D, pd, vk, j0);
+    cp_async_commit();
+    if (!KV) stage(vs, P.vc, P.ldv, g * Dv, Dv, pv, vv, j0);
+    cp_async_commit();
+    cp_async_wait<KV ? 0 : 1>();
+    __syncthreads();
+    {   // this warp's share of the depth for all 8 rows
+      float s[8];
+#pragma unroll
+      for (int r = 0; r < 8; r++) s[r] = 0.f;
+      const float4* k4 = reinterpret_cast<const float4*>(ks + lane * pd);
+#pragma unroll 2
+      for (int u = w; u < d4; u += 8) {
+        const float4 kv = k4[u];
+#pragma unroll
+        for (int r = 0; r < 8; r++) {
+          const float4 qv = reinterpret_cast<const float4*>(qs + r * pd)[u];
+          s[r] = fmaf(qv.x, kv.x, s[r]); s[r] = fmaf(qv.y, kv.y, s[r]); s[r] = fmaf(qv.z, kv.z, s[r]); s[r] = fmaf(qv.w, kv.w, s[r]);
         }
-      } else {
-        for (int r = lane; r < R; r += 32) dst[r] = to_f<CT>(src[r]);
       }
+#pragma unroll
+      for (int r = 0; r < 8; r++) red[(w * 8 + r) * 32 + lane] = s[r];
     }
     __syncthreads();
-    const int j = j0 + lane;
-    const bool valid = active && j >= lo_w && j <= hi_w && j <= hi;
-    if (!__any_sync(0xffffffffu, valid)) continue;
-    const float* kr = ks + lane * (R + 1);
-    const float* qr = qs + w * R;
-    float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;   // four chains: the dot product is latency-bound otherwise
-    int r = 0;
-    for (; r + 4 <= R; r += 4) {
-      s0 = fmaf(qr[r], kr[r], s0); s1 = fmaf(qr[r + 1], kr[r + 1], s1);
-      s2 = fmaf(qr[r + 2], kr[r + 2], s2); s3 = fmaf(qr[r + 3], kr[r + 3], s3);
+    {
+      float s = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; k++) s += red[(k * 8 + w) * 32 + lane];
+      const int v = j0 + lane, p = v < nk ? v : j_lo + v - nk;
+      const bool ok = mine && v <= hi && p <= i_w && (p >= lo_w || p < keep);
+      s = ok ? mod_score(P.mods, s, i_w - p, h_w, P.H) : -1e30f;
+      const float m_new = fmaxf(m, warp_max(s));
+      const float c = expf(m - m_new), pr = ok ? expf(s - m_new) : 0.f;
+      l = l * c + warp_sum(pr);
+      m = m_new;
+      pt[lane * 8 + w] = pr;
+      if (lane == 0) corr[w] = c;
     }
-    for (; r < R; r++) s0 = fmaf(qr[r], kr[r], s0);
-    float s = (s0 + s1) + (s2 + s3);
-    s = valid ? s : -1e30f;
-    const float m_new = fmaxf(m, warp_max(s));
-    const float corr = expf(m - m_new);
-    const float p = valid ? expf(s - m_new) : 0.f;
-    l = l * corr + warp_sum(p);
+    cp_async_wait<0>();
+    __syncthreads();
 #pragma unroll
-    for (int k = 0; k < RV; k++) acc[k] *= corr;
+    for (int r = 0; r < 8; r++) {
+      const float c = corr[r];
+#pragma unroll
+      for (int k = 0; k < CV; k++) acc[r][k] *= c;
+    }
+#pragma unroll 4
     for (int jj = 0; jj < 32; jj++) {
-      const float pj = __shfl_sync(0xffffffffu, p, jj);
-      if (pj == 0.f) continue;
-      const float* c = ks + jj * (R + 1);
+      const float4 p0 = *reinterpret_cast<const float4*>(pt + jj * 8), p1 = *reinterpret_cast<const float4*>(pt + jj * 8 + 4);
 #pragma unroll
-      for (int k = 0; k < RV; k++) {
-        const int r = lane + 32 * k;
-        if (r < R) acc[k] = fmaf(pj, c[r], acc[k]);
+      for (int k = 0; k < CV; k++) {
+        const int c = tid + 256 * k;
+        const float v = c < Dv ? vs[jj * pv + c] : 0.f;
+        acc[0][k] = fmaf(p0.x, v, acc[0][k]); acc[1][k] = fmaf(p0.y, v, acc[1][k]); acc[2][k] = fmaf(p0.z, v, acc[2][k]); acc[3][k] = fmaf(p0.w, v, acc[3][k]);
+        acc[4][k] = fmaf(p1.x, v, acc[4][k]); acc[5][k] = fmaf(p1.y, v, acc[5][k]); acc[6][k] = fmaf(p1.z, v, acc[6][k]); acc[7][k] = fmaf(p1.w, v, acc[7][k]);
       }
     }
+  }
+  float c_end = 1.f;
+  if (P.mods.sink && blockIdx.z == 0 && mine) {   // the sink joins the first share like a key with a zero value vector
+    const float sk = P.mods.sink[h_w], m_new = fmaxf(m, sk);
+    c_end = expf(m - m_new);
+    l = l * c_end + expf(sk - m_new);
     m = m_new;
   }
-  if (!active) return;
-  if (sink && blockIdx.z == 0) {   // the sink joins the first share like a key with a zero value vector
-    const float sk = sink[h], m_new = fmaxf(m, sk), corr = expf(m - m_new);
-    l = l * corr + expf(sk - m_new);
+  __syncthreads();
+  if (lane == 0) { corr[w] = c_end; corr[8 + w] = m; corr[16 + w] = l; }
+  __syncthreads();
 #pragma unroll
-    for (int k = 0; k < RV; k++) acc[k] *= corr;
-    m = m_new;
-  }
-  if (NS > 1) {   // partial result of this key range: [t][h][split] -> {m, l, acc[R]} (not normalised); latent_swa_merge finishes
-    float* pp = part + (((size_t)t * H + h) * NS + blockIdx.z) * (R + 2);
-    if (lane == 0) { pp[0] = m; pp[1] = l; }
+  for (int r = 0; r < 8; r++) {
+    if (!live(r)) continue;
+    const int t = row_t(r), h = g * rep + row_h(r);
+    if (P.NS > 1) {   // partial result of this key range: [t][h][split] -> {m, l, acc} (not normalised); latent_swa_merge finishes
+      float* pp = P.part + (((size_t)t * P.H + h) * P.NS + blockIdx.z) * (Dv + 2);
+      if (tid == 0) { pp[0] = corr[8 + r]; pp[1] = corr[16 + r]; }
 #pragma unroll
-    for (int k = 0; k < RV; k++) {
-      const int r = lane + 32 * k;
-      if (r < R) pp[2 + r] = acc[k];
+      for (int k = 0; k < CV; k++) { const int c = tid + 256 * k; if (c < Dv) pp[2 + c] = acc[r][k] * corr[r]; }
+    } else {
+      const float inv = corr[r] / corr[16 + r] * P.alpha;
+#pragma unroll
+      for (int k = 0; k < CV; k++) {
+        const int c = tid + 256 * k;
+        if (c >= Dv) continue;
+        const float gt = P.gate ? sigmoid_f(P.gate[(size_t)t * P.ld_gate + (P.gate_head ? (size_t)h : (size_t)h * Dv + c)]) : 1.f;
+        P.out[(size_t)t * P.ld_out + (size_t)h * Dv + c] = acc[r][k] * inv * gt;
+      }
     }
-    return;
-  }
-  const float inv = 1.f / l;
-#pragma unroll
-  for (int k = 0; k < RV; k++) {
-    const int r = lane + 32 * k;
-    if (r < R) out[((size_t)t * H + h) * R + r] = acc[k] * inv;
   }
 }
 
@@ -1491,10 +1599,17 @@ __global__ void __launch_bounds__(256) layer_norm(const float* __restrict__ in, 
 #pragma unroll
   for (int k = 0; k < kLnRegs; k++) { const int i = threadIdx.x + 256 * k; v[k] = cached && i < n && !wgt ? x[i] : 0.f; }
   if (wgt)
-    for (int e = 0; e < top; e++) {
-      const float we = wgt[(size_t)t * top + e];
+    for (int e0 = 0; e0 < top; e0 += 2) {   // two rows' loads in flight together
+      const float w0 = wgt[(size_t)t * top + e0], w1 = e0 + 1 < top ? wgt[(size_t)t * top + e0 + 1] : 0.f;
+      float r0[kLnRegs], r1[kLnRegs];
 #pragma unroll
-      for (int k = 0; k < kLnRegs; k++) { const int i = threadIdx.x + 256 * k; if (i < n) v[k] = fmaf(we, x[(size_t)e * ld_in + i], v[k]); }
+      for (int k = 0; k < kLnRegs; k++) {
+        const int i = threadIdx.x + 256 * k;
+        r0[k] = i < n ? x[(size_t)e0 * ld_in + i] : 0.f;
+        r1[k] = i < n && e0 + 1 < top ? x[(size_t)(e0 + 1) * ld_in + i] : 0.f;
+      }
+#pragma unroll
+      for (int k = 0; k < kLnRegs; k++) { v[k] = fmaf(w0, r0[k], v[k]); if (e0 + 1 < top) v[k] = fmaf(w1, r1[k], v[k]); }
     }
   float mean, sc;
   ln_stats(v, x, n, eps, red, mean, sc);
@@ -1586,7 +1701,7 @@ __global__ void __launch_bounds__(NT) rms_add_norm(const float* __restrict__ y, 
   grid_enter();
   __shared__ float red[33];
   const size_t t = blockIdx.x;
-  constexpr int KR = NT * kLnRegs / NT;
+  constexpr int KR = 256 * kLnRegs / NT;
   float v[KR], u[KR], ss = 0.f;
 #pragma unroll
   for (int k = 0; k < KR; k++) {
@@ -1595,7 +1710,7 @@ __global__ void __launch_bounds__(NT) rms_add_norm(const float* __restrict__ y, 
     u[k] = i < n ? x[t * n + i] : 0.f;
   }
   if (wgt) {
-    constexpr int EB = KR >= 16 ? 1 : 16 / KR;   // rows whose loads are in flight together
+    constexpr int EB = KR >= 16 ? 2 : 32 / KR;   // rows whose loads are in flight together
     for (int e0 = 0; e0 < top; e0 += EB) {
       float r[EB][KR];
 #pragma unroll
@@ -2190,13 +2305,14 @@ __global__ void __launch_bounds__(1024) moe_plan(const int* __restrict__ idx, in
 __global__ void moe_combine(float* __restrict__ x, int ldx, const float* __restrict__ y, const float* __restrict__ wgt, int top,
                             int width, float alpha, int add, const float* __restrict__ ysh = nullptr, const float* __restrict__ wsh = nullptr) {
   grid_enter();
-  const int t = blockIdx.x;
-  for (int c = threadIdx.x; c < width; c += blockDim.x) {
-    float s = 0.f;
-    for (int k = 0; k < top; k++) s = fmaf(wgt[(size_t)t * top + k], y[((size_t)t * top + k) * width + c], s);
-    if (ysh) s = fmaf(wsh[t], ysh[(size_t)t * width + c], s);
-    x[(size_t)t * ldx + c] = add ? x[(size_t)t * ldx + c] + alpha * s : alpha * s;
-  }
+  const int t = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;   // a column per thread: the rows' loads are in flight together
+  if (c >= width) return;
+  const float old = add ? x[(size_t)t * ldx + c] : 0.f;
+  float s = 0.f;
+#pragma unroll 8
+  for (int k = 0; k < top; k++) s = fmaf(wgt[(size_t)t * top + k], y[((size_t)t * top + k) * width + c], s);
+  if (ysh) s = fmaf(wsh[t], ysh[(size_t)t * width + c], s);
+  x[(size_t)t * ldx + c] = add ? old + alpha * s : alpha * s;
 }
 
 // arg-max of one logits row -> Ctrl::argmax_key (lowest index on ties), joined over the CTAs by an atomic maximum on a key that is 0 ahead of

@@ -156,7 +156,7 @@ struct State {
   float* vfirst = nullptr;                   // [chunk][kv_heads * vdim] values of the step's tokens in the first value-mixing layer
   int* d_prev = nullptr;                     // the sequence's last token (bigram embedding)
   float *x = nullptr, *h = nullptr, *b0 = nullptr, *b1 = nullptr, *b2 = nullptr, *b3 = nullptr, *wgt = nullptr, *logits = nullptr;
-  int *h_tok = nullptr, *h_want = nullptr;   // pinned staging of a chunk's token ids / wanted rows
+  int *h_tok = nullptr, *h_want = nullptr;   // pinned staging of a chunk's token ids / wanted rows (one allocation, with h_err)
   // bf16 products of portions: activations rounded for the product that follows, hidden rows of a feed-forward, and a host word that a wait
   // which gave up sets
   __nv_bfloat16 *a16 = nullptr, *hid16 = nullptr;
@@ -352,10 +352,6 @@ static void set_kernel_attrs() {
   static bool done = false;
   if (done) return;
   const int big = 200 * 1024;
-  cudaFuncSetAttribute(latent_swa_attn<float, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(latent_swa_attn<float, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(latent_swa_attn<float, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(latent_swa_attn<float, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(ssd_scan<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big); cudaFuncSetAttribute(ssd_scan<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(ssd_scan<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, big); cudaFuncSetAttribute(ssd_scan<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(ssd_scan<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, big); cudaFuncSetAttribute(ssd_scan<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
@@ -386,6 +382,9 @@ static void set_kernel_attrs() {
   DSK_TC5_ATTR(HEPI_STORE); DSK_TC5_ATTR(HEPI_ADD); DSK_TC5_ATTR(HEPI_GLU); DSK_TC5_ATTR(HEPI_XIELU); DSK_TC5_ATTR(HEPI_GEGLU); DSK_TC5_ATTR(HEPI_SIGMUL);
   DSK_TC5_ATTR(HEPI_RELU2); DSK_TC5_ATTR(HEPI_LINGATE); DSK_TC5_ATTR(HEPI_SILU_SIG); DSK_TC5_ATTR(HEPI_SOFTCAP); DSK_TC5_ATTR(HEPI_SWIGLU); DSK_TC5_ATTR(HEPI_GELU_MUL);
 #undef DSK_TC5_ATTR
+  cudaFuncSetAttribute(decode_attn<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big); cudaFuncSetAttribute(decode_attn<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(decode_attn<true, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big); cudaFuncSetAttribute(decode_attn<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(decode_attn<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big); cudaFuncSetAttribute(decode_attn<false, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(gqa_attn, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(mix_heads, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   done = true;
@@ -1091,7 +1090,7 @@ static int launches_per_token(const dsk_model* m) {
     else if (s.mixer == DSK_MIX_HGRN2) n += 4;   // stacked projection, recurrence, head norm, o
     else if (s.mixer == DSK_MIX_GQA) n += s.att_value_proj ? 5 : 6;   // q, k (or one stacked q / k / v (/ gate) product), norm + rotation, attention, merge, o
     else if (s.mixer == DSK_MIX_MLA) n += 9 + (s.att_out_gate ? 1 : 0);   // down-projections, query norm, query up, latent preparation, absorbed query, attention, merge, value up, (gate,) o
-    else n += is_ssd(s) ? 5 + (s.ssm_conv > 1 ? 1 : 0) : 5 + (s.att_kv_from < 0 ? 2 : 0);
+    else n += is_ssd(s) ? 5 : 5 + (s.att_kv_from < 0 ? 2 : 0);
     if (s.ff_kind == DSK_FF_MOE) n += (post && M->c.norm_kind == DSK_NORM_LAYER && !M->c.res_gate && M->c.dim <= 256 * kLnRegs && s.ff_shared == 0) || rms_fused(M->c) ? 4 : 5;
     if (R.pass >= 0 && M->c.loop_in) n += 1 + (&R != &M->runs[0] && fused_norms(M->c) ? 1 : 0);   // product, its norm
     if (s.ff_kind == DSK_FF_DENSE) n += 2;
@@ -1310,11 +1309,11 @@ static dsk_state* state_create(dsk_model* m) {
     S->hid16_elems = Tc * mxHid;
     rc |= salloc(S, (void**)&S->a16, S->a16_elems * 2) | salloc(S, (void**)&S->hid16, S->hid16_elems * 2);
   }
-  if (cudaHostAlloc((void**)&S->h_err, sizeof(int), cudaHostAllocMapped) != cudaSuccess) { fail(-2, "pinned allocation failed"); return nullptr; }
-  *S->h_err = 0;
   rc |= salloc(S, (void**)&S->logits, (size_t)S->head_rows * c.vocab_size * 4);
   if (rc) { fail(-2, "state allocation failed"); return nullptr; }
-  if (cudaMallocHost((void**)&S->h_tok, Tc * 4) != cudaSuccess || cudaMallocHost((void**)&S->h_want, Tc * 4) != cudaSuccess) { fail(-2, "pinned allocation failed"); return nullptr; }
+  if (cudaMallocHost((void**)&S->h_tok, (2 * Tc + 1) * 4) != cudaSuccess) { fail(-2, "pinned allocation failed"); return nullptr; }
+  S->h_want = S->h_tok + Tc; S->h_err = S->h_tok + 2 * Tc;
+  *S->h_err = 0;
   m->n_states++;
   return s;
 }
@@ -1326,7 +1325,7 @@ static void state_free(dsk_state* s) {
   if (S->side) { cudaStreamSynchronize(S->side); cudaStreamDestroy(S->side); cudaEventDestroy(S->ev_fork); cudaEventDestroy(S->ev_join); }
   for (cudaEvent_t e : S->tl_events) cudaEventDestroy(e);
   for (void* p : S->allocs) cudaFree(p);
-  cudaFreeHost(S->h_tok); cudaFreeHost(S->h_want); cudaFreeHost(S->h_err);
+  cudaFreeHost(S->h_tok);
   delete S;
   s->hy = nullptr;
 }
@@ -1694,21 +1693,45 @@ static void mlstm_forward(State* S, const HLayer& L, LayerState& ls, int ldp, co
 
 static int R0(const Model* M, size_t ri) { return M->runs[ri].owner_run; }
 
-static void launch_attn(const float* qa, const float* cache, float* out, int T, int H, int R, const int* ctl, int mask, int window, int ring,
-                        float scale, float* part, cudaStream_t st, const float* sink = nullptr) {
-  const int TQ = T >= 8 ? 8 : T >= 4 ? 4 : T >= 2 ? 2 : 1, HB = 8 / TQ;
-  int NS = 1;
-  if (T <= kAttnSplitTokens) {   // the widest key range a CTA can meet is window + TQ - 1 keys
-    const int tiles = (std::min(window, ring) + TQ - 1 + 31) / 32;
-    NS = std::max(1, std::min(tiles, kAttnSplitMax));
+// whether a tile of 32 keys and values fits decode_attn (gqa_attn takes larger heads, and mixed ones)
+static bool decode_attn_fits(int D, int Dv) { return Dv <= 1024 && decode_attn_floats(D, Dv, false) * 4 <= 200 * 1024; }
+// decode-sized attention (P.T, sizes, caches, mask and gate given): the split of rows and keys over CTAs, and the merge of key shares
+static void launch_decode_attn(State* S, DecodeAttn P, bool latent, cudaStream_t st) {
+  const int T = P.T, rep = P.H / P.G;
+  P.TQ = T >= 8 ? 8 : T >= 4 ? 4 : T >= 2 ? 2 : 1;
+  P.HB = std::min(rep, 8 / P.TQ);
+  P.NS = 1;
+  if (T <= kAttnSplitTokens) {   // the widest key range a CTA can meet is span + kept + TQ - 1 keys
+    const int tiles = (std::min(P.span, P.ring) + P.mods.keep + P.TQ - 1 + 31) / 32;
+    P.NS = std::max(1, std::min(tiles, kAttnSplitMax));
   }
-  const dim3 grid((unsigned)((T + TQ - 1) / TQ), (unsigned)((H + HB - 1) / HB), (unsigned)NS);
-  const size_t smem = ((size_t)8 * R + (size_t)32 * (R + 1)) * 4;
-  if (R <= 128) launch_next(latent_swa_attn<float, 4>, grid, 256, smem, st)(qa, cache, out, T, H, R, ctl, mask, window, ring, scale, TQ, NS, part, sink);
-  else if (R <= 256) launch_next(latent_swa_attn<float, 8>, grid, 256, smem, st)(qa, cache, out, T, H, R, ctl, mask, window, ring, scale, TQ, NS, part, sink);
-  else if (R <= 512) launch_next(latent_swa_attn<float, 16>, grid, 256, smem, st)(qa, cache, out, T, H, R, ctl, mask, window, ring, scale, TQ, NS, part, sink);
-  else launch_next(latent_swa_attn<float, 32>, grid, 256, smem, st)(qa, cache, out, T, H, R, ctl, mask, window, ring, scale, TQ, NS, part, sink);
-  if (NS > 1) launch_next(latent_swa_merge, dim3((unsigned)(T * H), (unsigned)((R + 127) / 128)), 128, 0, st)(part, out, R, NS, nullptr, 0, 1, 0, 0, 1.f);
+  P.part = S->part;
+  const dim3 grid((unsigned)((T + P.TQ - 1) / P.TQ), (unsigned)(P.G * ((rep + P.HB - 1) / P.HB)), (unsigned)P.NS);
+  const size_t smem = decode_attn_floats(P.D, P.Dv, latent) * 4;
+  const int cv = P.Dv <= 256 ? 1 : P.Dv <= 512 ? 2 : 4;
+  if (latent) {
+    if (cv == 1) launch_next(decode_attn<true, 1>, grid, 256, smem, st)(P);
+    else if (cv == 2) launch_next(decode_attn<true, 2>, grid, 256, smem, st)(P);
+    else launch_next(decode_attn<true, 4>, grid, 256, smem, st)(P);
+  } else {
+    if (cv == 1) launch_next(decode_attn<false, 1>, grid, 256, smem, st)(P);
+    else if (cv == 2) launch_next(decode_attn<false, 2>, grid, 256, smem, st)(P);
+    else launch_next(decode_attn<false, 4>, grid, 256, smem, st)(P);
+  }
+  S->launches++;
+  if (P.NS > 1) {
+    launch_next(latent_swa_merge, dim3((unsigned)(T * P.H), (unsigned)((P.Dv + 127) / 128)), 128, 0, st)(S->part, P.out, P.Dv, P.NS, P.gate, P.ld_gate, P.H, P.gate_head,
+                                                                                                        P.ld_out, P.alpha);
+    S->launches++;
+  }
+}
+// the same over cached latents with absorbed queries qa [T][H][R]
+static void launch_latent_attn(State* S, const float* qa, const float* cache, float* out, int T, int H, int R, int mask, int window, int ring, float scale, const float* sink,
+                               cudaStream_t st) {
+  DecodeAttn P{};
+  P.q = qa; P.kc = P.vc = cache; P.out = out; P.ctl = S->d_ctl; P.T = T; P.H = H; P.G = 1; P.D = P.Dv = P.ldk = P.ldv = R; P.mask = mask; P.span = window; P.ring = ring;
+  P.scale = scale; P.alpha = 1.f; P.ld_out = H * R; P.mods.sink = sink;
+  launch_decode_attn(S, P, true, st);
 }
 
 // LM head on the wanted rows [first, first + count) of the chunk whose normalised rows are in S->h -> S->logits [count][vocab]
@@ -1725,7 +1748,7 @@ static void enqueue_head(dsk_model* m, dsk_state* s, int first, int count, float
 static void norm_rows(const dsk_hybrid_config& c, State* S, const float* in, const float* w, const float* b, float* out, int T, int mode, float alpha, cudaStream_t st) {
   if (c.norm_kind == DSK_NORM_LAYER) launch_next(layer_norm, T, 256, 0, st)(in, c.dim, w, b, out, c.dim, c.dim, c.norm_eps, mode, alpha, nullptr, 0);
   else if (mode == 0 && c.norm_groups == 1) launch_next(rms_open, T, 256, 0, st)(const_cast<float*>(in), nullptr, nullptr, w, out, c.dim, c.norm_eps);   // (adds nothing: the row is only read)
-  else launch_next(group_rmsnorm<float>, T, 256, 0, st)(in, c.dim, w, out, c.dim, c.dim, c.norm_groups, c.norm_eps, mode, alpha, nullptr, 0, nullptr, 0);
+  else launch_next(group_rmsnorm<float>, dim3((unsigned)T, (unsigned)c.norm_groups), 256, 0, st)(in, c.dim, w, out, c.dim, c.dim, c.norm_groups, c.norm_eps, mode, alpha, nullptr, 0, nullptr, 0);
   S->launches++;
 }
 
@@ -1952,6 +1975,12 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
           MK("att.pv");
         }
         if (gate) { launch_next(gate_rows, T, 256, 0, st)(S->b3, ldo, gate, ldp, H * V, gate_head ? V : 1); S->launches++; }   // heads *= sigmoid(g h)
+      } else if (!sp.att_talk && decode_attn_fits(D, V)) {
+        DecodeAttn A{};
+        A.q = S->b2; A.kc = kc; A.vc = vc; A.out = S->b3; A.ctl = S->d_ctl; A.gate = gate; A.T = T; A.H = H; A.G = G; A.D = D; A.Dv = V; A.ldk = GD; A.ldv = GV;
+        A.mask = sp.att_mask; A.span = sp.att_window; A.ring = ring; A.ld_gate = ldp; A.gate_head = gate_head; A.ld_out = ldo; A.scale = sp.att_scale; A.alpha = lscale; A.mods = sm;
+        launch_decode_attn(S, A, false, st);
+        MK("att.decode");
       } else {
         int NS = 1;
         if (T <= kAttnSplitTokens) NS = std::max(1, std::min((std::min(sp.att_window, ring) + keep + 31) / 32, kAttnSplitMax));
@@ -2023,8 +2052,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
           P.sA = DK; P.sW = (long long)R * D; P.sC = RW;
           linear(S, bf, HEPI_STORE, P, H, st);
         }
-        launch_attn(S->b2, cache, S->b3, T, H, RW, S->d_ctl, sp.att_mask, sp.att_window, L.ring, sp.att_scale, S->part, st, sm.sink);
-        S->launches++;
+        launch_latent_attn(S, S->b2, cache, S->b3, T, H, RW, sp.att_mask, sp.att_window, L.ring, sp.att_scale, sm.sink, st);
         {  // value up-projection per head from the first R entries of the weighted cache rows
           GemmP P = gp(S->b3, H * RW, L.uv.p, R, S->b0, H * V, T, V, R);
           P.sA = RW; P.sW = (long long)V * R; P.sC = V;
@@ -2101,12 +2129,15 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       MK("norm");
       linear(S, bf, HEPI_STORE, gp(hin, W, L.in.p, W, S->b0, pw, T, pw, W), 1, st);
       MK("ssd.in");
-      launch_next(causal_conv_silu, dim3((unsigned)((ch + 127) / 128), (unsigned)T), 128, 0, st)(S->b0 + inner, pw, L.conv_w, L.conv_b, ls.hist, S->b1, ch, T, ch, sp.ssm_conv);
-      if (sp.ssm_conv > 1) launch_next(conv_history_update, (ch + 127) / 128, 128, 0, st)(S->b0 + inner, pw, ls.hist, T, ch, sp.ssm_conv);
+      if (T <= kConvShort) launch_next(causal_conv_silu_short, (ch + 127) / 128, 128, 0, st)(S->b0 + inner, pw, L.conv_w, L.conv_b, ls.hist, S->b1, ch, T, ch, sp.ssm_conv);
+      else {
+        launch_next(causal_conv_silu, dim3((unsigned)((ch + 127) / 128), (unsigned)T), 128, 0, st)(S->b0 + inner, pw, L.conv_w, L.conv_b, ls.hist, S->b1, ch, T, ch, sp.ssm_conv);
+        if (sp.ssm_conv > 1) launch_next(conv_history_update, (ch + 127) / 128, 128, 0, st)(S->b0 + inner, pw, ls.hist, T, ch, sp.ssm_conv);
+      }
       MK("ssd.conv");
       launch_scan(sp, S->b0, pw, S->b1, ch, L, ls.ssm, S->b2, T, st);
       MK("ssd.scan");
-      launch_next(group_rmsnorm<float>, T, 256, 0, st)(S->b2, inner, L.mnorm, S->b3, inner, inner, sp.ssm_norm_groups, c.norm_eps, 0, 0.f, nullptr, 0, nullptr, 0);
+      launch_next(group_rmsnorm<float>, dim3((unsigned)T, (unsigned)sp.ssm_norm_groups), 256, 0, st)(S->b2, inner, L.mnorm, S->b3, inner, inner, sp.ssm_norm_groups, c.norm_eps, 0, 0.f, nullptr, 0, nullptr, 0);
       S->launches += 4;
       MK("ssd.norm");
       GemmP P = gp(S->b3, inner, L.o.p, inner, sink.C, W, T, W, inner);
@@ -2161,8 +2192,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
           P.sA = D; P.sW = (long long)R * D; P.sC = R;
           linear(S, bf, HEPI_STORE, P, H, st);
         }
-        launch_attn(S->b2, cache, S->b3, T, H, R, S->d_ctl, sp.att_mask, sp.att_window, O.ring, sp.att_scale, S->part, st);
-        S->launches++;
+        launch_latent_attn(S, S->b2, cache, S->b3, T, H, R, sp.att_mask, sp.att_window, O.ring, sp.att_scale, nullptr, st);
         {  // value up-projection per head: ov[t][h][:] = W_uv[h] o[t][h][:]
           GemmP P = gp(S->b3, H * R, L.uv.p, R, S->b0, H * V, T, V, R);
           P.sA = R; P.sW = (long long)V * R; P.sC = V;
@@ -2286,7 +2316,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         launch_next(layer_norm, T, 256, 0, st)(S->b3, W, L.close2, L.norm2_bias, S->x, W, W, c.norm_eps, 1, mult, S->wgt, top);
         S->launches++;
       } else if (!frms) {   // (sandwich blocks of RMS norms combine as they close)
-        launch_next(moe_combine, T, 256, 0, st)(sink.C, W, S->b3, S->wgt, top, W, sink.alpha, sink.epi == HEPI_ADD ? 1 : 0, shared ? ysh : nullptr, S->wsh);
+        launch_next(moe_combine, dim3((unsigned)T, (unsigned)((W + 255) / 256)), 256, 0, st)(sink.C, W, S->b3, S->wgt, top, W, sink.alpha, sink.epi == HEPI_ADD ? 1 : 0, shared ? ysh : nullptr, S->wsh);
         S->launches++;
       }
       MK("moe.combine");
