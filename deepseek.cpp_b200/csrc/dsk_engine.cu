@@ -31,6 +31,7 @@
 #include "dsk_hybrid.cuh"
 #include "dsk_linattn.cuh"
 #include "dsk_tc5.cuh"
+#include "dsk_pattn.cuh"
 
 using namespace dsk;
 

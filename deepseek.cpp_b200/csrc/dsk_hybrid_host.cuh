@@ -157,6 +157,9 @@ struct State {
   int* d_prev = nullptr;                     // the sequence's last token (bigram embedding)
   float *x = nullptr, *h = nullptr, *b0 = nullptr, *b1 = nullptr, *b2 = nullptr, *b3 = nullptr, *wgt = nullptr, *logits = nullptr;
   int *h_tok = nullptr, *h_want = nullptr;   // pinned staging of a chunk's token ids / wanted rows (one allocation, with h_err)
+  // attention of portions in one kernel (pattn): split keys and values of the visible positions, queries it takes at a time
+  __nv_bfloat16 *k16 = nullptr, *v16 = nullptr;
+  int pattn_q = 0;
   // bf16 products of portions: activations rounded for the product that follows, hidden rows of a feed-forward, and a host word that a wait
   // which gave up sets
   __nv_bfloat16 *a16 = nullptr, *hid16 = nullptr;
@@ -348,6 +351,24 @@ static int validate(const dsk_hybrid_config& c, const dsk_layer_spec* L) {
   return 0;
 }
 
+// attention of portions in one kernel: sizes and the layers that take it (no mixing of the heads' scores, a tile of keys that fits)
+static constexpr int kPattnSmemMax = 220 * 1024;
+struct PattnSize { int parts, G, D, V, Dp, Vp, VN; };
+static PattnSize pattn_size(const dsk_layer_spec& s, bool bf16) {
+  PattnSize z;
+  z.parts = s.mixer == DSK_MIX_LATENT_SWA && bf16 ? 1 : 3;
+  z.G = s.mixer == DSK_MIX_GQA ? s.att_kv_heads : s.att_heads;
+  z.D = s.att_dim + (s.mixer == DSK_MIX_MLA ? s.att_rot_dim : 0); z.V = s.att_vdim;
+  z.VN = z.V <= 64 ? 8 : 16;
+  z.Dp = (z.D + 15) / 16 * 16; z.Vp = (z.V + z.VN * 8 - 1) / (z.VN * 8) * (z.VN * 8);
+  return z;
+}
+static bool takes_pattn(const dsk_layer_spec& s, bool bf16) {
+  if (!has_attn(s) || (s.mixer == DSK_MIX_GQA && s.att_talk)) return false;
+  const PattnSize z = pattn_size(s, bf16);
+  return pattn_smem(z.parts, 2, z.Dp, z.VN) <= (size_t)kPattnSmemMax;
+}
+
 static void set_kernel_attrs() {
   static bool done = false;
   if (done) return;
@@ -378,6 +399,8 @@ static void set_kernel_attrs() {
   DSK_LSCAN_ATTR(8, 1, 2); DSK_LSCAN_ATTR(16, 1, 2); DSK_LSCAN_ATTR(32, 1, 2); DSK_LSCAN_ATTR(8, 1, 4); DSK_LSCAN_ATTR(16, 1, 4); DSK_LSCAN_ATTR(32, 1, 4); DSK_LSCAN_ATTR(32, 2, 4);
 #undef DSK_LSCAN_ATTR
   cudaFuncSetAttribute(gemm_mma<HEPI_SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMmaSmem);
+  cudaFuncSetAttribute(pattn<1, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax); cudaFuncSetAttribute(pattn<1, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax);
+  cudaFuncSetAttribute(pattn<3, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax); cudaFuncSetAttribute(pattn<3, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax);
 #define DSK_TC5_ATTR(E) cudaFuncSetAttribute(gemm_tc5<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem)
   DSK_TC5_ATTR(HEPI_STORE); DSK_TC5_ATTR(HEPI_ADD); DSK_TC5_ATTR(HEPI_GLU); DSK_TC5_ATTR(HEPI_XIELU); DSK_TC5_ATTR(HEPI_GEGLU); DSK_TC5_ATTR(HEPI_SIGMUL);
   DSK_TC5_ATTR(HEPI_RELU2); DSK_TC5_ATTR(HEPI_LINGATE); DSK_TC5_ATTR(HEPI_SILU_SIG); DSK_TC5_ATTR(HEPI_SOFTCAP); DSK_TC5_ATTR(HEPI_SWIGLU); DSK_TC5_ATTR(HEPI_GELU_MUL);
@@ -1275,11 +1298,34 @@ static dsk_state* state_create(dsk_model* m) {
     }
     const size_t bytes = keys * (hd + hv) * (4 + (latent ? pack_es : 0)) + heads * kPrefillQ * keys * 4 * (any_talk ? 2 : 1);
     if (keys > 0 && bytes <= ((size_t)4 << 30)) {
-      S->prefill_keys = (int)keys;
-      rc |= salloc(S, (void**)&S->kf, keys * hd * 4) | salloc(S, (void**)&S->vf, keys * hv * 4);
-      if (latent) rc |= salloc(S, &S->kb, keys * hd * pack_es) | salloc(S, &S->vt, keys * hv * pack_es);
-      rc |= salloc(S, (void**)&S->sc, heads * kPrefillQ * keys * 4) | salloc(S, (void**)&S->d_rows, keys * 4);
-      if (any_talk) rc |= salloc(S, (void**)&S->sc2, heads * kPrefillQ * keys * 4);
+      // layers that run pattn: the visible keys of a whole step split into bf16 parts, behind the up-projected fp32 rows of latent layers (blocks of
+      // kPrefillQ queries where a step's keys would take over 4 GB)
+      const bool bf16 = c.quant == DSK_BF16;
+      size_t k16 = 0, v16 = 0, kup = 0, vup = 0, rows = keys;
+      bool old = false;
+      for (S->pattn_q = (int)Tc;; S->pattn_q = kPrefillQ) {
+        k16 = v16 = kup = vup = 0; rows = keys; old = false;
+        for (const HLayer& L : M->L) {
+          if (!has_attn(L.sp)) continue;
+          if (!takes_pattn(L.sp, bf16)) { old = true; continue; }
+          const PattnSize z = pattn_size(L.sp, bf16);
+          const size_t n = (size_t)std::min<long long>((long long)L.sp.att_window - 1, (long long)c.max_seq_len) + std::min<size_t>(Tc, S->pattn_q) +
+                           (L.sp.mixer == DSK_MIX_GQA ? L.sp.att_keep_first : 0);
+          k16 = std::max(k16, n * z.G * z.Dp * z.parts); v16 = std::max(v16, n * z.G * z.Vp * z.parts);
+          if (L.sp.mixer != DSK_MIX_GQA) { kup = std::max(kup, n * z.G * L.sp.att_dim); vup = std::max(vup, n * z.G * z.V); }
+          rows = std::max(rows, n);
+        }
+        if (2 * (k16 + v16) + 4 * (kup + vup) <= ((size_t)4 << 30) || S->pattn_q <= kPrefillQ) break;
+      }
+      S->prefill_keys = (int)rows;
+      if (k16) rc |= salloc(S, (void**)&S->k16, k16 * 2) | salloc(S, (void**)&S->v16, v16 * 2);
+      rc |= salloc(S, (void**)&S->kf, std::max(kup, old ? keys * hd : 0) * 4) | salloc(S, (void**)&S->vf, std::max(vup, old ? keys * hv : 0) * 4);
+      rc |= salloc(S, (void**)&S->d_rows, rows * 4);
+      if (old) {
+        if (latent) rc |= salloc(S, &S->kb, keys * hd * pack_es) | salloc(S, &S->vt, keys * hv * pack_es);
+        rc |= salloc(S, (void**)&S->sc, heads * kPrefillQ * keys * 4);
+        if (any_talk) rc |= salloc(S, (void**)&S->sc2, heads * kPrefillQ * keys * 4);
+      }
     }
   }
   rc |= salloc(S, (void**)&S->x, Tc * c.dim * 4) | salloc(S, (void**)&S->h, Tc * c.dim * 4);
@@ -1734,6 +1780,25 @@ static void launch_latent_attn(State* S, const float* qa, const float* cache, fl
   launch_decode_attn(S, P, true, st);
 }
 
+// Attention of Tq queries in one kernel: K (keys, values and the visible range given) is split into bf16 parts, then A runs over it.
+static void portion_attn(State* S, const PattnSize& z, PackP K, PattnP A, cudaStream_t st) {
+  K.V = z.V; K.Dp = z.Dp; K.Vp = z.Vp; K.G = z.G; K.kb = S->k16; K.vb = S->v16;
+  A.kb = S->k16; A.vb = S->v16; A.G = z.G; A.D = z.D; A.Dp = z.Dp; A.V = z.V; A.Vp = z.Vp; A.Lk = K.Lk; A.nk = K.nk; A.first = K.first; A.mods.keep = K.keep;
+  if (z.parts == 1) launch_next(pattn_pack<1>, K.Lk, 256, 0, st)(K);
+  else launch_next(pattn_pack<3>, K.Lk, 256, 0, st)(K);
+  // 16 query rows per warp: as many warps as shared memory holds, fewer where that leaves SMs idle (a warp's share of a tile's copy grows)
+  const int zc = z.Vp / (z.VN * 8);
+  int w = 8;
+  while (w > 2 && (pattn_smem(z.parts, w, z.Dp, z.VN) > (size_t)kPattnSmemMax || (long long)((A.T + 16 * w - 1) / (16 * w)) * A.H * zc < 148)) w /= 2;
+  const dim3 grid((unsigned)((A.T + 16 * w - 1) / (16 * w)), (unsigned)A.H, (unsigned)zc);
+  const size_t smem = pattn_smem(z.parts, w, z.Dp, z.VN);
+  if (z.parts == 1 && z.VN == 8) launch_next(pattn<1, 8>, grid, 32 * w, smem, st)(A);
+  else if (z.parts == 1) launch_next(pattn<1, 16>, grid, 32 * w, smem, st)(A);
+  else if (z.VN == 8) launch_next(pattn<3, 8>, grid, 32 * w, smem, st)(A);
+  else launch_next(pattn<3, 16>, grid, 32 * w, smem, st)(A);
+  S->launches += 2;
+}
+
 // LM head on the wanted rows [first, first + count) of the chunk whose normalised rows are in S->h -> S->logits [count][vocab]
 static void enqueue_head(dsk_model* m, dsk_state* s, int first, int count, float* logits, cudaStream_t st) {
   Model* M = m->hy;
@@ -1948,6 +2013,20 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       S->launches++;
       MK("att.norm+rot");
       if (pos0 >= 0 && T >= kPrefillMin && S->prefill_keys > 0) {
+        if (takes_pattn(sp, bf)) {
+          const PattnSize z = pattn_size(sp, bf);
+          for (int t0 = 0; t0 < T; t0 += S->pattn_q) {
+            const int Tq = std::min(S->pattn_q, T - t0), qpos0 = pos0 + t0;
+            PackP K{};
+            K.first = mask_first(sp.att_mask, sp.att_window, qpos0); K.nk = std::min(keep, K.first); K.Lk = K.nk + qpos0 + Tq - K.first; K.keep = keep; K.ring = ring;
+            K.k = kc; K.v = vc; K.ldk = GD; K.ldv = GV; K.D0 = D; K.kv_cached = 1;
+            PattnP A{};
+            A.q = S->b2 + (size_t)t0 * HD; A.ldq = HD; A.out = S->b3 + (size_t)t0 * ldo; A.ld_out = ldo; A.gate = gate ? gate + (size_t)t0 * ldp : nullptr; A.ld_gate = ldp;
+            A.gate_head = gate_head; A.T = Tq; A.H = H; A.pos0 = qpos0; A.mask = sp.att_mask; A.span = sp.att_window; A.scale = sp.att_scale; A.alpha = lscale; A.mods = sm;
+            portion_attn(S, z, K, A, st);
+          }
+          MK("att.fused");
+        } else {
         // a portion: blocks of kPrefillQ queries, each as  scores = q k^T per head (fp32);  mixing of the heads;  masked softmax;  o = P v
         for (int t0 = 0; t0 < T; t0 += kPrefillQ) {
           const int Tq = std::min(kPrefillQ, T - t0), qpos0 = pos0 + t0;
@@ -1975,6 +2054,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
           MK("att.pv");
         }
         if (gate) { launch_next(gate_rows, T, 256, 0, st)(S->b3, ldo, gate, ldp, H * V, gate_head ? V : 1); S->launches++; }   // heads *= sigmoid(g h)
+        }
       } else if (!sp.att_talk && decode_attn_fits(D, V)) {
         DecodeAttn A{};
         A.q = S->b2; A.kc = kc; A.vc = vc; A.out = S->b3; A.ctl = S->d_ctl; A.gate = gate; A.T = T; A.H = H; A.G = G; A.D = D; A.Dv = V; A.ldk = GD; A.ldv = GV;
@@ -2018,7 +2098,29 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       float* ov = S->b3;   // [T][H*V] heads' outputs
       ScoreMods sm{};
       sm.sink = sp.att_sink ? L.sink : nullptr;
-      if (portion) {
+      if (portion && takes_pattn(sp, bf)) {   // plain keys and values up-projected from the visible latents, the rotated key part shared by the heads
+        const PattnSize z = pattn_size(sp, bf);
+        for (int t0 = 0; t0 < T; t0 += S->pattn_q) {
+          const int Tq = std::min(S->pattn_q, T - t0), qpos0 = pos0 + t0;
+          PackP P{};
+          P.first = mask_first(sp.att_mask, sp.att_window, qpos0); P.Lk = qpos0 + Tq - P.first; P.ring = L.ring;
+          launch_next(ring_rows, (P.Lk + 255) / 256, 256, 0, st)(P.first, P.Lk, L.ring, S->d_rows);
+          GemmP K = gp(cache, RW, L.uk.p, R, S->kf, H * D, P.Lk, H * D, R);
+          K.a_map = S->d_rows;
+          linear(S, bf, HEPI_STORE, K, 1, st);
+          GemmP Vp = gp(cache, RW, L.uv.p, R, S->vf, H * V, P.Lk, H * V, R);
+          Vp.a_map = S->d_rows;
+          linear(S, bf, HEPI_STORE, Vp, 1, st);
+          MK("att.kv_up");
+          P.k = S->kf; P.v = S->vf; P.krot = cache + R; P.ldk = H * D; P.ldv = H * V; P.ldr = RW; P.D0 = D; P.Rd = Rd;
+          PattnP A{};
+          A.q = S->b0 + (size_t)t0 * H * DK; A.ldq = H * DK; A.out = S->b3 + (size_t)t0 * H * V; A.ld_out = H * V; A.T = Tq; A.H = H; A.pos0 = qpos0; A.mask = sp.att_mask;
+          A.span = sp.att_window; A.scale = sp.att_scale; A.alpha = 1.f; A.mods = sm;
+          portion_attn(S, z, P, A, st);
+          S->launches++;
+        }
+        MK("att.fused");
+      } else if (portion) {
         // blocks of kPrefillQ queries: plain keys and values up-projected from the visible latents, the rotated key part appended to every
         // head's keys; scores, softmax and the value product in fp32
         for (int t0 = 0; t0 < T; t0 += kPrefillQ) {
@@ -2160,6 +2262,29 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       if (pos0 >= 0 && T >= kPrefillMin && S->prefill_keys > 0) {
         // a portion: blocks of kPrefillQ queries, each as  k, v = up-projections of the visible latents;  P = softmax_band(q k^T);  o = P v
         ov = S->b3;
+        if (takes_pattn(sp, bf)) {
+          const PattnSize z = pattn_size(sp, bf);
+          for (int t0 = 0; t0 < T; t0 += S->pattn_q) {
+            const int Tq = std::min(S->pattn_q, T - t0), qpos0 = pos0 + t0;
+            PackP P{};
+            P.first = mask_first(sp.att_mask, sp.att_window, qpos0); P.Lk = qpos0 + Tq - P.first; P.ring = O.ring;
+            launch_next(ring_rows, (P.Lk + 255) / 256, 256, 0, st)(P.first, P.Lk, O.ring, S->d_rows);
+            GemmP K = gp(cache, R, L.uk.p, R, S->kf, H * D, P.Lk, H * D, R);
+            K.a_map = S->d_rows;
+            linear(S, bf, HEPI_STORE, K, 1, st);
+            GemmP Vp = gp(cache, R, L.uv.p, R, S->vf, H * V, P.Lk, H * V, R);
+            Vp.a_map = S->d_rows;
+            linear(S, bf, HEPI_STORE, Vp, 1, st);
+            MK("att.kv_up");
+            P.k = S->kf; P.v = S->vf; P.ldk = H * D; P.ldv = H * V; P.D0 = D;
+            PattnP A{};
+            A.q = S->b0 + (size_t)t0 * H * D; A.ldq = H * D; A.out = S->b3 + (size_t)t0 * H * V; A.ld_out = H * V; A.T = Tq; A.H = H; A.pos0 = qpos0; A.mask = sp.att_mask;
+            A.span = sp.att_window; A.scale = sp.att_scale; A.alpha = 1.f;
+            portion_attn(S, z, P, A, st);
+            S->launches++;
+          }
+          MK("att.fused");
+        } else
         for (int t0 = 0; t0 < T; t0 += kPrefillQ) {
           const int Tq = std::min(kPrefillQ, T - t0), qpos0 = pos0 + t0;
           const int first = mask_first(sp.att_mask, sp.att_window, qpos0), Lk = qpos0 + Tq - first;

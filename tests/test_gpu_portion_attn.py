@@ -1,0 +1,30 @@
+"""Attention of portions in one kernel at the edges of its tiles (16 query rows a warp, 32 keys, depths padded to 16, value columns in groups of 64
+or 128), against the float64 statement: steps that continue a sequence inside a window, several column groups, heads too deep for the kernel."""
+import pytest
+
+from test_gpu_netusun import F32_TOL, close_bf16, in_portions, mk, no, rel, tokens_for  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,size", [(3, 1, 10, 6, 1), (4, 2, 33, 65, 40), (2, 2, 128, 128, 33), (6, 3, 16, 300, None), (1, 1, 300, 20, 50)])
+def test_grouped_heads(mk, no, heads, kv_heads, dim, vdim, size):  # noqa: F811
+    cfg = no.model_config([no.att(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, size=size)] * 2, width=48, vocab=97)
+    m, W = mk(cfg, seed=heads + dim, chunk=160)
+    toks = tokens_for(cfg, 210, 8)
+    exp = no.run(cfg, W, toks)[0]
+    for sizes in ([160, 50], [33, 32, 129], [32, 160]):
+        assert rel(in_portions(m, toks, sizes), exp) < F32_TOL
+
+
+@pytest.mark.parametrize("heads,dim,rot_dim,vdim", [(3, 7, 4, 5), (2, 128, 64, 128), (2, 40, 8, 129)])
+def test_latents(mk, no, heads, dim, rot_dim, vdim):  # noqa: F811
+    cfg = no.model_config([no.lat(heads=heads, dim=dim, rot_dim=rot_dim, vdim=vdim)], width=40, vocab=97)
+    toks = tokens_for(cfg, 200, 9)
+    for quant in ("fp32", "bf16"):
+        m, W = mk(cfg, seed=dim, chunk=128, quant=quant)
+        exp = no.run(cfg, W, toks)[0]
+        noise = no.rounding_noise(cfg, W, toks) if quant == "bf16" else None
+        for sizes in ([128, 72], [33, 95, 65]):
+            got = in_portions(m, toks, sizes)
+            assert rel(got, exp) < F32_TOL if quant == "fp32" else close_bf16(got, exp, noise)
