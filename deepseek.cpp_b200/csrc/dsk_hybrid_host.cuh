@@ -366,7 +366,7 @@ static PattnSize pattn_size(const dsk_layer_spec& s, bool bf16) {
 static bool takes_pattn(const dsk_layer_spec& s, bool bf16) {
   if (!has_attn(s) || (s.mixer == DSK_MIX_GQA && s.att_talk)) return false;
   const PattnSize z = pattn_size(s, bf16);
-  return pattn_smem(z.parts, 2, z.Dp, z.VN) <= (size_t)kPattnSmemMax;
+  return pattn_smem(z.parts, 2, z.Dp, z.VN, 4) <= (size_t)kPattnSmemMax;
 }
 
 static void set_kernel_attrs() {
@@ -399,8 +399,9 @@ static void set_kernel_attrs() {
   DSK_LSCAN_ATTR(8, 1, 2); DSK_LSCAN_ATTR(16, 1, 2); DSK_LSCAN_ATTR(32, 1, 2); DSK_LSCAN_ATTR(8, 1, 4); DSK_LSCAN_ATTR(16, 1, 4); DSK_LSCAN_ATTR(32, 1, 4); DSK_LSCAN_ATTR(32, 2, 4);
 #undef DSK_LSCAN_ATTR
   cudaFuncSetAttribute(gemm_mma<HEPI_SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMmaSmem);
-  cudaFuncSetAttribute(pattn<1, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax); cudaFuncSetAttribute(pattn<1, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax);
-  cudaFuncSetAttribute(pattn<3, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax); cudaFuncSetAttribute(pattn<3, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax);
+#define DSK_PATTN_ATTR(A, B) cudaFuncSetAttribute(pattn<A, B, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax); cudaFuncSetAttribute(pattn<A, B, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax)
+  DSK_PATTN_ATTR(1, 8); DSK_PATTN_ATTR(1, 16); DSK_PATTN_ATTR(3, 8); DSK_PATTN_ATTR(3, 16);
+#undef DSK_PATTN_ATTR
 #define DSK_TC5_ATTR(E) cudaFuncSetAttribute(gemm_tc5<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem)
   DSK_TC5_ATTR(HEPI_STORE); DSK_TC5_ATTR(HEPI_ADD); DSK_TC5_ATTR(HEPI_GLU); DSK_TC5_ATTR(HEPI_XIELU); DSK_TC5_ATTR(HEPI_GEGLU); DSK_TC5_ATTR(HEPI_SIGMUL);
   DSK_TC5_ATTR(HEPI_RELU2); DSK_TC5_ATTR(HEPI_LINGATE); DSK_TC5_ATTR(HEPI_SILU_SIG); DSK_TC5_ATTR(HEPI_SOFTCAP); DSK_TC5_ATTR(HEPI_SWIGLU); DSK_TC5_ATTR(HEPI_GELU_MUL);
@@ -1525,7 +1526,7 @@ template <typename WT>
 static void launch_gemm_t(int epi, const GemmP& P, int Z, bool small, int tile_cap, cudaStream_t st) {
   if (small && gemv_one_ok<WT>(P)) {
     const int n = std::max(P.N, P.n_shared > 0 ? P.sN : 0);
-    const int R = (long long)n * Z >= 16384 && Z == 1 ? 2 : 1;   // rows per warp
+    const int R = (long long)n * Z >= (Z == 1 ? 16384 : 148 * 64) ? 2 : 1;   // rows per warp: two where one each would be more warps than the chip holds at a time
     const dim3 grid((unsigned)std::max(1, std::min((n + 8 * R - 1) / (8 * R), 148 * 8)), (unsigned)Z);
 #define DSK_GEMV1(E) do { if (R == 2) launch_next(gemv_one<WT, E, 2>, grid, 256, 0, st)(P); else launch_next(gemv_one<WT, E, 1>, grid, 256, 0, st)(P); } while (0)
     switch (epi) {
@@ -1786,16 +1787,22 @@ static void portion_attn(State* S, const PattnSize& z, PackP K, PattnP A, cudaSt
   A.kb = S->k16; A.vb = S->v16; A.G = z.G; A.D = z.D; A.Dp = z.Dp; A.V = z.V; A.Vp = z.Vp; A.Lk = K.Lk; A.nk = K.nk; A.first = K.first; A.mods.keep = K.keep;
   if (z.parts == 1) launch_next(pattn_pack<1>, K.Lk, 256, 0, st)(K);
   else launch_next(pattn_pack<3>, K.Lk, 256, 0, st)(K);
-  // 16 query rows per warp: as many warps as shared memory holds, fewer where that leaves SMs idle (a warp's share of a tile's copy grows)
+  // 16 query rows per warp: eight warps, with tiles of 16 keys where 32 do not fit (deep heads: a head of 192 leaves room for four warps with
+  // 32 keys or eight with 16), fewer where that leaves SMs idle (a warp's share of a tile's copy grows)
   const int zc = z.Vp / (z.VN * 8);
-  int w = 8;
-  while (w > 2 && (pattn_smem(z.parts, w, z.Dp, z.VN) > (size_t)kPattnSmemMax || (long long)((A.T + 16 * w - 1) / (16 * w)) * A.H * zc < 148)) w /= 2;
-  const dim3 grid((unsigned)((A.T + 16 * w - 1) / (16 * w)), (unsigned)A.H, (unsigned)zc);
-  const size_t smem = pattn_smem(z.parts, w, z.Dp, z.VN);
-  if (z.parts == 1 && z.VN == 8) launch_next(pattn<1, 8>, grid, 32 * w, smem, st)(A);
-  else if (z.parts == 1) launch_next(pattn<1, 16>, grid, 32 * w, smem, st)(A);
-  else if (z.VN == 8) launch_next(pattn<3, 8>, grid, 32 * w, smem, st)(A);
-  else launch_next(pattn<3, 16>, grid, 32 * w, smem, st)(A);
+  int w = 8, nk = 4;
+  auto fits = [&] { return pattn_smem(z.parts, w, z.Dp, z.VN, nk) <= (size_t)kPattnSmemMax; };
+  if (!fits()) nk = 2;
+  while (w > 2 && (!fits() || (long long)((A.T + 16 * w - 1) / (16 * w)) * A.H * zc < 148)) w /= 2;
+  if (nk == 2) { nk = 4; if (!fits()) nk = 2; }
+  const dim3 grid((unsigned)A.H, (unsigned)((A.T + 16 * w - 1) / (16 * w)), (unsigned)zc);
+  const size_t smem = pattn_smem(z.parts, w, z.Dp, z.VN, nk);
+#define DSK_PATTN(A_, B_) do { if (nk == 4) launch_next(pattn<A_, B_, 4>, grid, 32 * w, smem, st)(A); else launch_next(pattn<A_, B_, 2>, grid, 32 * w, smem, st)(A); } while (0)
+  if (z.parts == 1 && z.VN == 8) DSK_PATTN(1, 8);
+  else if (z.parts == 1) DSK_PATTN(1, 16);
+  else if (z.VN == 8) DSK_PATTN(3, 8);
+  else DSK_PATTN(3, 16);
+#undef DSK_PATTN
   S->launches += 2;
 }
 

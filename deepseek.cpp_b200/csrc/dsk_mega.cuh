@@ -31,6 +31,7 @@ constexpr int kMegaThreads = 288;          // + producer warp 8
 constexpr int kSlotScale = 2048;           // bytes reserved per ring slot for f8 scale rows
 constexpr int kSlotData = 32 * 1024;       // weight bytes per ring slot
 constexpr int kSlotBytes = kSlotScale + kSlotData;
+constexpr int kKvPrefetch = 512;           // cached positions whose keys and values are fetched ahead of the attention stage
 constexpr int kRingEntries = 16;          // tiles in flight per CTA (mbarrier pairs); their bytes come out of one circular buffer
 constexpr int kMaxPieces = 24;
 constexpr int kMegaHdr = 8192;             // barriers, scratch, partial results, smem copies of Program + 2 Stage descriptors
@@ -1674,27 +1675,29 @@ __device__ __forceinline__ float kq_quarter(uint32_t row, int qb, int nqb, const
     const float o = (yr.d * h2f((uint16_t)(dm & 0xffff))) * (float)isum - (yr.d * h2f((uint16_t)(dm >> 16))) * (float)summs;
     out = act ? o : 0.f;
   } else {
-    int isum = 0;
+    // weight = q + 4 hbit - 4 (q: 2-bit field, hbit: its bit in the high-bit mask), scale = 6 bits - 32.  As with Q2_K nothing is shifted into
+    // place: dp4a of the masked words gives 4^s x and 2^bit x the sums over the sub-block, exact multiples that are shifted back once per
+    // sub-block, and the sixteen 6-bit scales' four of this lane come out of three PRMTs (the shift-and-or form took about 144 integer
+    // instructions a quarter block, this one about 95).
     const uint32_t blk = row + (uint32_t)b * kQ3Bytes;
     const uint4 hm = lds128(blk + 16 * c);
     const uint4 qq = lds128(blk + 32 + 32 * h + 16 * c);
     const uint32_t s0 = lds32(blk + 96), s1 = lds32(blk + 100), s2 = lds32(blk + 104);
     const uint32_t dw = lds32(blk + 108);
+    const uint32_t lo4 = (__byte_perm(s0, s1, c ? 0x7531u : 0x6420u) >> (4 * h)) & 0x0F0F0F0Fu;   // bytes of sub-blocks s = 0..3
+    const uint32_t hb = __byte_perm(s2, 0u, c ? 0x3131u : 0x2020u) >> (4 * h);
+    const uint32_t sc6 = lo4 | (((hb & 0x00000303u) | ((hb >> 2) & 0x03030000u)) << 4);
+    const uint32_t hmask = h ? 0x10101010u : 0x01010101u;
+    int isum = 0;
 #pragma unroll
     for (int s = 0; s < 4; s++) {
-      const int bit = 4 * h + s;
-      int dp = __dp4a((int)(((qq.x >> (2 * s)) & 0x03030303u) | (((hm.x >> bit) & 0x01010101u) << 2)), yr.y[s].x, 0);
-      dp = __dp4a((int)(((qq.y >> (2 * s)) & 0x03030303u) | (((hm.y >> bit) & 0x01010101u) << 2)), yr.y[s].y, dp);
-      dp = __dp4a((int)(((qq.z >> (2 * s)) & 0x03030303u) | (((hm.z >> bit) & 0x01010101u) << 2)), yr.y[s].z, dp);
-      dp = __dp4a((int)(((qq.w >> (2 * s)) & 0x03030303u) | (((hm.w >> bit) & 0x01010101u) << 2)), yr.y[s].w, dp);
-      dp -= 4 * yr.bs[s];
-      const int t = 2 * s + c;
-      const uint32_t lw = (t < 4) ? s0 : s1;
-      const int lob = (lw >> (8 * (t & 3))) & 0xff;
-      const int lo4 = h ? (lob >> 4) : (lob & 0xF);
-      const int hib = (s2 >> (8 * (t & 3))) & 0xff;
-      const int hi2 = (hib >> (2 * (2 * h + (t >> 2)))) & 3;
-      isum += ((lo4 | (hi2 << 4)) - 32) * dp;
+      const uint32_t mk = 0x03030303u << (2 * s), hk = hmask << s;
+      int dp = dp4a_us(qq.x & mk, yr.y[s].x, 0), dh = dp4a_us(hm.x & hk, yr.y[s].x, 0);
+      dp = dp4a_us(qq.y & mk, yr.y[s].y, dp); dh = dp4a_us(hm.y & hk, yr.y[s].y, dh);
+      dp = dp4a_us(qq.z & mk, yr.y[s].z, dp); dh = dp4a_us(hm.z & hk, yr.y[s].z, dh);
+      dp = dp4a_us(qq.w & mk, yr.y[s].w, dp); dh = dp4a_us(hm.w & hk, yr.y[s].w, dh);
+      const int v = (dp >> (2 * s)) + 4 * ((dh >> (4 * h + s)) - yr.bs[s]);
+      isum += ((int)__byte_perm(sc6, 0u, 0x4440u + s) - 32) * v;
     }
     const float o = (h2f((uint16_t)(dw & 0xffff)) * yr.d) * (float)isum;
     out = act ? o : 0.f;
@@ -2666,6 +2669,18 @@ __global__ void __launch_bounds__(kMegaThreads, 1) decode_kernel(const Program* 
     const Stage& st = *sm.st_c;
     if (st.kind == ST_GEMV && st.norm_w && (int)blockIdx.x < st.ntiles) {
       for (int i = tid * 32; i < st.n; i += kConsumers * 32) asm volatile("prefetch.global.L1 [%0];" ::"l"(st.norm_w + i));
+    }
+    // the stage that writes this token's keys and values runs ahead of the attention stage: while it waits, the older rows of the heads this
+    // CTA will attend to come into L2 (up to kKvPrefetch positions; beyond that they are a stream of their own)
+    if (st.kind == ST_GEMV && st.epi == EPI_KVB && (int)blockIdx.x < P.n_heads && P.ctrl->kv_len <= kKvPrefetch) {
+      const int len = P.ctrl->kv_len, kl = (P.hd * 2 + 127) / 128, vl = (P.vh * 2 + 127) / 128;
+      for (int h = blockIdx.x; h < P.n_heads; h += gridDim.x)
+        for (int i = tid; i < len * (kl + vl); i += kConsumers) {
+          const int t = i / (kl + vl), c = i - t * (kl + vl);
+          const char* p = c < kl ? reinterpret_cast<const char*>(st.kcache + ((size_t)t * P.n_heads + h) * P.hd) + c * 128
+                                 : reinterpret_cast<const char*>(st.vcache + ((size_t)t * P.n_heads + h) * P.vh) + (c - kl) * 128;
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+        }
     }
     if (nstage_seen > 0) {         // grid barrier: every CTA has finished (and released) the previous stage
       if (tid == 0) grid_wait(P.sync_counter, base + (unsigned int)nstage_seen * G);

@@ -7,8 +7,8 @@
 // registers (rounded to nearest), so that a sum of n elements sees n / 16 roundings where a chain of FMAs sees n: the error against 64 bits is not
 // larger than that of the fp32 products it replaces.  PARTS = 1: operands rounded to bf16 (latent attention of bf16 models, whose products
 // always took them so).
-// pattn_pack splits the visible keys and values once per step; a CTA (16 query rows per warp) streams them in tiles of 32 through two buffers
-// (cp.async).  Bound: the tensor pipe at six products per element, then shared-memory reads of the query fragments.  Before, a block of 256
+// pattn_pack splits the visible keys and values once per step; a CTA (16 query rows per warp) streams them in tiles of 32 or 16 through two
+// buffers (cp.async).  Bound: issue slots - six products per element, their operands from shared memory, softmax.  Before, a block of 256
 // queries wrote its scores, read them for the softmax and again for the values, all three in kernels of their own on the fp32 pipe.
 #pragma once
 
@@ -73,9 +73,9 @@ struct PattnP {
   ScoreMods mods;
 };
 
-constexpr int kPattnKeys = 32;
-__host__ __device__ inline size_t pattn_smem(int parts, int warps, int Dp, int VN) {
-  return (size_t)parts * 2 * ((size_t)warps * 16 * (Dp + 8) + 2 * kPattnKeys * ((Dp + 8) + (VN * 8 + 8)));
+// NK: 8-key groups of a tile
+__host__ __device__ inline size_t pattn_smem(int parts, int warps, int Dp, int VN, int NK) {
+  return (size_t)parts * 2 * ((size_t)warps * 16 * (Dp + 8) + 2 * NK * 8 * ((Dp + 8) + (VN * 8 + 8)));
 }
 
 __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr) {
@@ -84,34 +84,64 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t add
 __device__ __forceinline__ void ldmatrix_x4_at(uint32_t (&r)[4], uint32_t addr) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
 }
-// acc += sum over 16 elements of a b: the six leading pairs of the operands' parts, small ones first, joined in the tensor core
+__device__ __forceinline__ void mma_bf16_first(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {   // c = a b
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+               : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "f"(0.f));
+}
+// two fp32 values as PARTS pairs of bf16, for finite values
 template <int PARTS>
-__device__ __forceinline__ void mma_parts(float (&acc)[4], const uint32_t (&a)[PARTS][4], const uint32_t (&b)[PARTS][2]) {
-  if constexpr (PARTS == 1) {
-    mma_bf16_16816(acc, a[0][0], a[0][1], a[0][2], a[0][3], b[0][0], b[0][1]);
-  } else {
-    float t[4] = {0.f, 0.f, 0.f, 0.f};
-    mma_bf16_16816(t, a[2][0], a[2][1], a[2][2], a[2][3], b[0][0], b[0][1]);
-    mma_bf16_16816(t, a[0][0], a[0][1], a[0][2], a[0][3], b[2][0], b[2][1]);
-    mma_bf16_16816(t, a[1][0], a[1][1], a[1][2], a[1][3], b[1][0], b[1][1]);
-    mma_bf16_16816(t, a[1][0], a[1][1], a[1][2], a[1][3], b[0][0], b[0][1]);
-    mma_bf16_16816(t, a[0][0], a[0][1], a[0][2], a[0][3], b[1][0], b[1][1]);
-    mma_bf16_16816(t, a[0][0], a[0][1], a[0][2], a[0][3], b[0][0], b[0][1]);
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t (&o)[PARTS]) {
 #pragma unroll
-    for (int i = 0; i < 4; i++) acc[i] += t[i];
+  for (int i = 0; i < PARTS; i++) {
+    const __nv_bfloat162 p = __floats2bfloat162_rn(x, y);
+    o[i] = *reinterpret_cast<const uint32_t*>(&p);
+    if (i + 1 < PARTS) { x -= __uint_as_float(o[i] << 16); y -= __uint_as_float(o[i] & 0xffff0000u); }
+  }
+}
+// acc[n] += sum over 16 elements of a b[n] for N tiles: the six leading pairs of the operands' parts, joined in the tensor core and then added.  A
+// step of all N sums comes before the next step of any: a sum's products wait for one another (some 24 cycles each), the N sums do not.
+// load(part, b) brings the tiles' b operands of a part.
+template <int PARTS, int N, typename Load>
+__device__ __forceinline__ void mma_parts(float (*acc)[4], const uint32_t (&a)[PARTS][4], Load load) {
+  uint32_t b[N][2];
+  auto step = [&](float (*t)[4], const uint32_t (&x)[4]) {
+#pragma unroll
+    for (int n = 0; n < N; n++) mma_bf16_16816(t[n], x[0], x[1], x[2], x[3], b[n][0], b[n][1]);
+  };
+  if constexpr (PARTS == 1) {
+    load(0, b);
+    step(acc, a[0]);
+  } else {
+    float t[N][4];
+    load(2, b);
+#pragma unroll
+    for (int n = 0; n < N; n++) mma_bf16_first(t[n], a[0], b[n]);
+    load(1, b);
+    step(t, a[1]);
+    step(t, a[0]);
+    load(0, b);
+    step(t, a[2]);
+    step(t, a[1]);
+    step(t, a[0]);
+#pragma unroll
+    for (int n = 0; n < N; n++)
+#pragma unroll
+      for (int i = 0; i < 4; i++) acc[n][i] += t[n][i];
   }
 }
 
-template <int PARTS, int VN>   // VN: 8-column groups of values in a CTA (blockIdx.z picks the columns)
+template <int PARTS, int VN, int NK>   // VN: 8-column groups of values in a CTA (blockIdx.z picks the columns)
 __global__ void __launch_bounds__(256, 1) pattn(const PattnP P) {
+  constexpr int KT = NK * 8;                                           // keys of a tile
   extern __shared__ __align__(16) unsigned char pa_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nthr = blockDim.x, BM = nthr / 2;
-  const int Dp = P.Dp, pq = Dp + 8, pvt = VN * 8 + 8;                 // row pitches (ldmatrix rows on distinct banks)
+  const int Dp = P.Dp, pq = Dp + 8;
+  constexpr int pvt = VN * 8 + 8;                                      // row pitches (ldmatrix rows on distinct banks)
   const uint32_t qs = smem_u32(pa_raw), qpart = (uint32_t)(BM * pq * 2);
-  const uint32_t kpart = (uint32_t)(kPattnKeys * pq * 2), vpart = (uint32_t)(kPattnKeys * pvt * 2), buf = PARTS * (kpart + vpart);
+  const uint32_t kpart = (uint32_t)(KT * pq * 2), vpart = (uint32_t)(KT * pvt * 2), buf = PARTS * (kpart + vpart);
   const uint32_t ks0 = qs + PARTS * qpart;
-  const int qb = (int)gridDim.x - 1 - (int)blockIdx.x, q0 = qb * BM;   // late queries, which see most keys, first
-  const int h = blockIdx.y, g = h / (P.H / P.G), v0 = (int)blockIdx.z * VN * 8;
+  const int qb = (int)gridDim.y - 1 - (int)blockIdx.y, q0 = qb * BM;   // late queries, which see most keys, first for every head
+  const int h = blockIdx.x, g = h / (P.H / P.G), v0 = (int)blockIdx.z * VN * 8;
   grid_enter();
   // query rows, split
   for (int e = threadIdx.x; e < BM * (Dp / 4); e += nthr) {
@@ -130,27 +160,33 @@ __global__ void __launch_bounds__(256, 1) pattn(const PattnP P) {
   const int last = min(P.T, q0 + BM) - 1;
   const int lo_v = P.nk + mask_first(P.mask, P.span, P.pos0 + q0) - P.first, hi_v = P.nk + P.pos0 + last - P.first;
   // (kept positions are keys 0 .. keep - 1 whether or not they lie in the range)
-  const int kept = (min(P.mods.keep, hi_v + 1) + kPattnKeys - 1) / kPattnKeys, t0 = max(kept, lo_v / kPattnKeys), n_tiles = kept + max(0, hi_v / kPattnKeys - t0 + 1);
-  auto tile_key = [&](int i) { return (i < kept ? i : t0 + i - kept) * kPattnKeys; };
-  auto fetch = [&](int i) {
+  const int kept = (min(P.mods.keep, hi_v + 1) + KT - 1) / KT, t0 = max(kept, lo_v / KT), n_tiles = kept + max(0, hi_v / KT - t0 + 1);
+  auto tile_key = [&](int i) { return (i < kept ? i : t0 + i - kept) * KT; };
+  const int chunks = Dp / 8 + VN;
+  auto fetch = [&](int i) {   // a warp copies rows (part, key) warp, warp + warps, ..: a lane per 16 bytes of the key row and the value row
     const int key0 = tile_key(i);
     const uint32_t kd = ks0 + (uint32_t)(i & 1) * buf, vd = kd + PARTS * kpart;
-    const int kc = Dp / 8;
-    for (int e = threadIdx.x; e < PARTS * kPattnKeys * (kc + VN); e += nthr) {
-      const bool key = e < PARTS * kPattnKeys * kc;
-      const int q = key ? e : e - PARTS * kPattnKeys * kc, per = key ? kc : VN, r = q / per, c = (q - r * per) * 8, part = r / kPattnKeys, j = r - part * kPattnKeys;
-      const int v = key0 + j;
+    for (int r = warp; r < PARTS * KT; r += nthr >> 5) {
+      const int part = r / KT, j = r - part * KT, v = key0 + j;
       const bool in = v < P.Lk;
       const size_t row = ((size_t)part * P.G + g) * P.Lk + (in ? v : 0);
-      const __nv_bfloat16* src = key ? P.kb + row * Dp + c : P.vb + row * P.Vp + v0 + c;
-      const uint32_t dst = key ? kd + part * kpart + (uint32_t)(j * pq + c) * 2 : vd + part * vpart + (uint32_t)(j * pvt + c) * 2;
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+      for (int c = lane; c < chunks; c += 32) {
+        const bool key = c < chunks - VN;
+        const int cc = (key ? c : c - (chunks - VN)) * 8;
+        const __nv_bfloat16* src = key ? P.kb + row * Dp + cc : P.vb + row * P.Vp + v0 + cc;
+        const uint32_t dst = key ? kd + part * kpart + (uint32_t)(j * pq + cc) * 2 : vd + part * vpart + (uint32_t)(j * pvt + cc) * 2;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+      }
     }
     cp_async_commit();
   };
   if (n_tiles > 0) fetch(0);
   const int row_lo = q0 + warp * 16 + (lane >> 2);                      // this thread's query rows: row_lo and row_lo + 8
   const int first_lo[2] = {mask_first(P.mask, P.span, P.pos0 + row_lo), mask_first(P.mask, P.span, P.pos0 + row_lo + 8)};
+  // a tile whose keys every query of the warp sees needs no mask
+  const int w_pos = P.pos0 + q0 + warp * 16, w_lo = mask_first(P.mask, P.span, w_pos + 15);
+  const bool capped = P.mods.cap > 0.f;
+  const float s_mul = capped ? P.scale / P.mods.cap : P.scale;
   float o[VN][4], m[2] = {-1e30f, -1e30f}, l[2] = {0.f, 0.f};
 #pragma unroll
   for (int n = 0; n < VN; n++)
@@ -162,53 +198,64 @@ __global__ void __launch_bounds__(256, 1) pattn(const PattnP P) {
     __syncthreads();                                                     // tile it is there; everyone is through tile it - 1
     if (it + 1 < n_tiles) fetch(it + 1);
     const uint32_t kt = ks0 + (uint32_t)(it & 1) * buf, vt = kt + PARTS * kpart;
-    float s[4][4];
+    float s[NK][4];
 #pragma unroll
-    for (int n = 0; n < 4; n++)
+    for (int n = 0; n < NK; n++)
 #pragma unroll
       for (int i = 0; i < 4; i++) s[n][i] = 0.f;
     const uint32_t kaddr = kt + (uint32_t)(((lane & 7) + (lane >> 4) * 8) * pq + ((lane >> 3) & 1) * 8) * 2;
+#pragma unroll 2
     for (int k = 0; k < Dp; k += 16) {
       uint32_t a[PARTS][4];
 #pragma unroll
       for (int i = 0; i < PARTS; i++) ldmatrix_x4_at(a[i], qa + i * qpart + k * 2);
+      mma_parts<PARTS, NK>(s, a, [&](int part, uint32_t (&bb)[NK][2]) {
 #pragma unroll
-      for (int np = 0; np < 2; np++) {
-        uint32_t b0[PARTS][2], b1[PARTS][2];
-#pragma unroll
-        for (int i = 0; i < PARTS; i++) {
+        for (int np = 0; np < NK / 2; np++) {
           uint32_t r[4];
-          ldmatrix_x4_at(r, kaddr + i * kpart + (uint32_t)(np * 16 * pq + k) * 2);
-          b0[i][0] = r[0]; b0[i][1] = r[1]; b1[i][0] = r[2]; b1[i][1] = r[3];
+          ldmatrix_x4_at(r, kaddr + part * kpart + (uint32_t)(np * 16 * pq + k) * 2);
+          bb[2 * np][0] = r[0]; bb[2 * np][1] = r[1]; bb[2 * np + 1][0] = r[2]; bb[2 * np + 1][1] = r[3];
         }
-        mma_parts<PARTS>(s[2 * np], a, b0);
-        mma_parts<PARTS>(s[2 * np + 1], a, b1);
-      }
+      });
     }
-    // mask and softmax: rows row_lo (entries 0, 1) and row_lo + 8 (entries 2, 3); keys n * 8 + (lane & 3) * 2 + {0, 1}
+    // scale, cap, bias and mask: rows row_lo (entries 0, 1) and row_lo + 8 (entries 2, 3); keys n * 8 + (lane & 3) * 2 + {0, 1}
     const int key0 = tile_key(it);
-    float mx[2] = {-1e30f, -1e30f};
 #pragma unroll
-    for (int n = 0; n < 4; n++)
+    for (int n = 0; n < NK; n++)
 #pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const int t = row_lo + (i >> 1) * 8, pos = P.pos0 + t, v = key0 + n * 8 + (lane & 3) * 2 + (i & 1), p = v < P.nk ? v : P.first + v - P.nk;
-        const bool ok = v < P.Lk && p <= pos && (p < P.mods.keep || p >= first_lo[i >> 1]);
-        s[n][i] = ok ? mod_score(P.mods, s[n][i] * P.scale, pos - p, h, P.H) : -INFINITY;
-        mx[i >> 1] = fmaxf(mx[i >> 1], s[n][i]);
-      }
-    float c[2];
+      for (int i = 0; i < 4; i++) s[n][i] *= s_mul;
+    if (capped) {
+#pragma unroll
+      for (int n = 0; n < NK; n++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) s[n][i] = P.mods.cap * tanhf(s[n][i]);
+    }
+    const int p_lo = P.first + key0 - P.nk, p_hi = p_lo + KT - 1;        // positions of a tile behind the kept rows
+    if (P.mods.rel || key0 < P.nk || p_hi > w_pos || p_lo < w_lo || key0 + KT > P.Lk) {
+#pragma unroll
+      for (int n = 0; n < NK; n++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const int pos = P.pos0 + row_lo + (i >> 1) * 8, v = key0 + n * 8 + (lane & 3) * 2 + (i & 1), p = v < P.nk ? v : P.first + v - P.nk;
+          const bool ok = v < P.Lk && p <= pos && (p < P.mods.keep || p >= first_lo[i >> 1]);
+          if (ok && P.mods.rel) s[n][i] += P.mods.rel[(size_t)P.mods.bucket[min(pos - p, P.mods.rel_max)] * P.H + h];
+          if (!ok) s[n][i] = -INFINITY;
+        }
+    }
+    float c[2], sum[2] = {0.f, 0.f};
 #pragma unroll
     for (int r = 0; r < 2; r++) {
-      mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
-      mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
-      const float m_new = fmaxf(m[r], mx[r]);
+      float mx = fmaxf(s[0][2 * r], s[0][2 * r + 1]);
+#pragma unroll
+      for (int n = 1; n < NK; n++) mx = fmaxf(mx, fmaxf(s[n][2 * r], s[n][2 * r + 1]));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+      const float m_new = fmaxf(m[r], mx);
       c[r] = expf(m[r] - m_new);
       m[r] = m_new;
     }
-    float sum[2] = {0.f, 0.f};
 #pragma unroll
-    for (int n = 0; n < 4; n++)
+    for (int n = 0; n < NK; n++)
 #pragma unroll
       for (int i = 0; i < 4; i++) { s[n][i] = expf(s[n][i] - m[i >> 1]); sum[i >> 1] += s[n][i]; }   // (a key out of sight: e^-inf = 0)
 #pragma unroll
@@ -217,33 +264,32 @@ __global__ void __launch_bounds__(256, 1) pattn(const PattnP P) {
       sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 2);
       l[r] = fmaf(l[r], c[r], sum[r]);
     }
+    if (__any_sync(0xffffffffu, c[0] != 1.f || c[1] != 1.f)) {
 #pragma unroll
-    for (int n = 0; n < VN; n++) { o[n][0] *= c[0]; o[n][1] *= c[0]; o[n][2] *= c[1]; o[n][3] *= c[1]; }
+      for (int n = 0; n < VN; n++) { o[n][0] *= c[0]; o[n][1] *= c[0]; o[n][2] *= c[1]; o[n][3] *= c[1]; }
+    }
     const uint32_t vaddr = vt + (uint32_t)(((lane & 7) + ((lane >> 3) & 1) * 8) * pvt + (lane >> 4) * 8) * 2;
 #pragma unroll
-    for (int kk = 0; kk < 2; kk++) {
+    for (int kk = 0; kk < NK / 2; kk++) {
       uint32_t a[PARTS][4];
 #pragma unroll
       for (int q = 0; q < 4; q++) {   // fragment registers: {row, keys 0-7}, {row + 8, keys 0-7}, {row, keys 8-15}, {row + 8, keys 8-15}
         const int n = 2 * kk + (q >> 1), i0 = (q & 1) * 2;
-        __nv_bfloat16 x0[PARTS], x1[PARTS];
-        split_bf16<PARTS>(s[n][i0], x0);
-        split_bf16<PARTS>(s[n][i0 + 1], x1);
+        uint32_t x[PARTS];
+        split_pair<PARTS>(s[n][i0], s[n][i0 + 1], x);
 #pragma unroll
-        for (int i = 0; i < PARTS; i++) { __nv_bfloat162 pr; pr.x = x0[i]; pr.y = x1[i]; a[i][q] = *reinterpret_cast<const uint32_t*>(&pr); }
+        for (int i = 0; i < PARTS; i++) a[i][q] = x[i];
       }
 #pragma unroll
-      for (int n = 0; n < VN; n += 2) {
-        uint32_t b0[PARTS][2], b1[PARTS][2];
+      for (int n = 0; n < VN; n += 4)
+        mma_parts<PARTS, 4>(o + n, a, [&](int part, uint32_t (&bb)[4][2]) {
 #pragma unroll
-        for (int i = 0; i < PARTS; i++) {
-          uint32_t r[4];
-          ldmatrix_x4_trans(r, vaddr + i * vpart + (uint32_t)(kk * 16 * pvt + n * 8) * 2);
-          b0[i][0] = r[0]; b0[i][1] = r[1]; b1[i][0] = r[2]; b1[i][1] = r[3];
-        }
-        mma_parts<PARTS>(o[n], a, b0);
-        mma_parts<PARTS>(o[n + 1], a, b1);
-      }
+          for (int np = 0; np < 2; np++) {
+            uint32_t r[4];
+            ldmatrix_x4_trans(r, vaddr + part * vpart + (uint32_t)(kk * 16 * pvt + (n + 2 * np) * 8) * 2);
+            bb[2 * np][0] = r[0]; bb[2 * np][1] = r[1]; bb[2 * np + 1][0] = r[2]; bb[2 * np + 1][1] = r[3];
+          }
+        });
     }
   }
 #pragma unroll
