@@ -449,6 +449,105 @@ __global__ void __launch_bounds__(256) gemm_tiled(const GemmP P) {
   }
 }
 
+template <typename WT> struct WVec;
+template <> struct WVec<float> {
+  static constexpr int N = 4;
+  static __device__ __forceinline__ void load(const float* p, float (&o)[4]) { const float4 v = *reinterpret_cast<const float4*>(p); o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w; }
+  static __device__ __forceinline__ void decode(const uint4& v, float (&o)[4]) { o[0] = __uint_as_float(v.x); o[1] = __uint_as_float(v.y); o[2] = __uint_as_float(v.z); o[3] = __uint_as_float(v.w); }
+};
+template <> struct WVec<__nv_bfloat16> {
+  static constexpr int N = 8;
+  static __device__ __forceinline__ void load(const __nv_bfloat16* p, float (&o)[8]) {
+    decode(*reinterpret_cast<const uint4*>(p), o);
+  }
+  static __device__ __forceinline__ void decode(const uint4& v, float (&o)[8]) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; i++) { o[2 * i] = __uint_as_float(w[i] << 16); o[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
+  }
+};
+
+// Narrow outputs over many rows (a router, a token-input gate: N <= 96 columns): fp32 activations, plain FMA.  A CTA takes 16 rows and all columns,
+// 32 columns at a time; its 8 warps share the depth (warp w takes every eighth slice of 16) and their sums are joined in shared memory.  A lane holds
+// 4 rows x 4 columns, so 32 bytes from shared memory feed 16 FMAs, and every weight is read once per 16 rows, where a warp per weight row
+// over 4 rows read the activations once per column.
+constexpr int kNarrowRows = 16;
+template <typename WT, int EPI>
+__global__ void __launch_bounds__(256) gemm_narrow(const GemmP P) {
+  __shared__ __align__(16) float As[8][16][kNarrowRows + 4], Ws[8][16][32 + 4];   // [warp][k][row], [warp][k][column]
+  float* red = &As[0][0][0];                                                      // [8 warps][16 rows][32 columns], over both at the end
+  static_assert(sizeof(As) + sizeof(Ws) >= 8 * 16 * 32 * 4, "the sums of 8 warps fit");
+  grid_enter();
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, row0 = blockIdx.x * kNarrowRows, n0 = blockIdx.y * 32;
+  const WT* __restrict__ W = reinterpret_cast<const WT*>(P.W);
+  const int tr = (lane >> 3) * 4, tc = (lane & 7) * 4;                             // this lane's rows and columns
+  float acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+  // staging: lane -> half of a row's slice of 16: 8 consecutive k of 16 activation rows; a whole slice of a weight row
+  const int ar = lane >> 1, ak = (lane & 1) * 8, m = row0 + ar;
+  const float* arow = m < P.M ? P.A + (size_t)(P.a_map ? P.a_map[m] / P.a_div : m) * P.lda : nullptr;
+  const WT* wrow = n0 + lane < P.N ? W + (size_t)(n0 + lane) * P.ldw : nullptr;
+  const bool va = (P.lda & 3) == 0 && (reinterpret_cast<uintptr_t>(P.A) & 15) == 0;
+  const bool vw = P.ldw % WVec<WT>::N == 0 && (reinterpret_cast<uintptr_t>(P.W) & 15) == 0;
+  float a[8], b[16];
+  auto fetch = [&](int k0) {
+    if (arow && va && k0 + ak + 8 <= P.K) {
+      const float4 x = *reinterpret_cast<const float4*>(arow + k0 + ak), y = *reinterpret_cast<const float4*>(arow + k0 + ak + 4);
+      a[0] = x.x; a[1] = x.y; a[2] = x.z; a[3] = x.w; a[4] = y.x; a[5] = y.y; a[6] = y.z; a[7] = y.w;
+    } else {
+#pragma unroll
+      for (int q = 0; q < 8; q++) a[q] = arow && k0 + ak + q < P.K ? arow[k0 + ak + q] : 0.f;
+    }
+    if (wrow && vw && k0 + 16 <= P.K) {
+#pragma unroll
+      for (int q = 0; q < 16; q += WVec<WT>::N) {
+        float v[WVec<WT>::N];
+        WVec<WT>::load(wrow + k0 + q, v);
+#pragma unroll
+        for (int u = 0; u < WVec<WT>::N; u++) b[q + u] = v[u];
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < 16; q++) b[q] = wrow && k0 + q < P.K ? to_f<WT>(wrow[k0 + q]) : 0.f;
+    }
+  };
+  if (w * 16 < P.K) fetch(w * 16);
+  for (int k0 = w * 16; k0 < P.K; k0 += 128) {
+#pragma unroll
+    for (int q = 0; q < 8; q++) As[w][ak + q][ar] = a[q];
+#pragma unroll
+    for (int q = 0; q < 16; q++) Ws[w][q][lane] = b[q];
+    __syncwarp();
+    if (k0 + 128 < P.K) fetch(k0 + 128);   // in flight during this slice's FMAs
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+      const float4 x = *reinterpret_cast<const float4*>(&As[w][k][tr]), y = *reinterpret_cast<const float4*>(&Ws[w][k][tc]);
+      const float xr[4] = {x.x, x.y, x.z, x.w}, yc[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = fmaf(xr[i], yc[j], acc[i][j]);
+    }
+    __syncwarp();
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; i++) *reinterpret_cast<float4*>(red + ((w * 16 + tr + i) * 32 + tc)) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+  __syncthreads();
+  for (int e = tid; e < 16 * 32; e += 256) {
+    const int r = e >> 5, n = n0 + (e & 31), mm = row0 + r;
+    if (mm >= P.M || n >= P.N) continue;
+    float v = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; k++) v += red[(k * 16 + r) * 32 + (e & 31)];
+    const int cr = P.c_map ? P.c_map[mm] : mm;
+    gemm_epilogue<WT, EPI>(P, P.C + (size_t)cr * P.ldc, cr, n, v, 0.f);
+  }
+}
+
 // Tensor-core variant for bf16 weights and more than a handful of rows: 128 x 128 tile of A W^T per CTA (K in steps of 32), the
 // fp32 activations rounded to bf16 while they are staged, mma.sync m16n8k16 bf16 x bf16 -> fp32.  8 warps as 2 (rows) x 4
 // (columns), a 64 x 32 warp tile.  Same row maps, expert tiles, batches and epilogues as gemm_tiled.  For the GLU epilogue the
@@ -731,23 +830,6 @@ __global__ void __launch_bounds__(128) rms_add_shift_small(const float* __restri
   if (mu) carry[c] = prev;
 }
 
-template <typename WT> struct WVec;
-template <> struct WVec<float> {
-  static constexpr int N = 4;
-  static __device__ __forceinline__ void load(const float* p, float (&o)[4]) { const float4 v = *reinterpret_cast<const float4*>(p); o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w; }
-  static __device__ __forceinline__ void decode(const uint4& v, float (&o)[4]) { o[0] = __uint_as_float(v.x); o[1] = __uint_as_float(v.y); o[2] = __uint_as_float(v.z); o[3] = __uint_as_float(v.w); }
-};
-template <> struct WVec<__nv_bfloat16> {
-  static constexpr int N = 8;
-  static __device__ __forceinline__ void load(const __nv_bfloat16* p, float (&o)[8]) {
-    decode(*reinterpret_cast<const uint4*>(p), o);
-  }
-  static __device__ __forceinline__ void decode(const uint4& v, float (&o)[8]) {
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int i = 0; i < 4; i++) { o[2 * i] = __uint_as_float(w[i] << 16); o[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u); }
-  }
-};
 __device__ __forceinline__ uint4 ldg_stream(const void* p) {   // 16 read-only bytes that are used once
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
@@ -2305,8 +2387,23 @@ __global__ void __launch_bounds__(1024) moe_plan(const int* __restrict__ idx, in
 __global__ void moe_combine(float* __restrict__ x, int ldx, const float* __restrict__ y, const float* __restrict__ wgt, int top,
                             int width, float alpha, int add, const float* __restrict__ ysh = nullptr, const float* __restrict__ wsh = nullptr) {
   grid_enter();
-  const int t = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;   // a column per thread: the rows' loads are in flight together
+  // four columns per thread where rows start on 16-byte boundaries, all rows' loads in flight together
+  const int t = blockIdx.x, V = (width & 3) == 0 && (ldx & 3) == 0 ? 4 : 1, c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
   if (c >= width) return;
+  if (V == 4) {
+    const float4 old = add ? *reinterpret_cast<const float4*>(x + (size_t)t * ldx + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto more = [&](float w, const float* row) {
+      const float4 r = *reinterpret_cast<const float4*>(row + c);
+      s.x = fmaf(w, r.x, s.x); s.y = fmaf(w, r.y, s.y); s.z = fmaf(w, r.z, s.z); s.w = fmaf(w, r.w, s.w);
+    };
+#pragma unroll 8
+    for (int k = 0; k < top; k++) more(wgt[(size_t)t * top + k], y + ((size_t)t * top + k) * width);
+    if (ysh) more(wsh[t], ysh + (size_t)t * width);
+    *reinterpret_cast<float4*>(x + (size_t)t * ldx + c) = add ? make_float4(old.x + alpha * s.x, old.y + alpha * s.y, old.z + alpha * s.z, old.w + alpha * s.w)
+                                                              : make_float4(alpha * s.x, alpha * s.y, alpha * s.z, alpha * s.w);
+    return;
+  }
   const float old = add ? x[(size_t)t * ldx + c] : 0.f;
   float s = 0.f;
 #pragma unroll 8

@@ -409,6 +409,7 @@ static void set_kernel_attrs() {
   cudaFuncSetAttribute(decode_attn<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big); cudaFuncSetAttribute(decode_attn<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(decode_attn<true, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big); cudaFuncSetAttribute(decode_attn<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(decode_attn<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big); cudaFuncSetAttribute(decode_attn<false, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(ssd_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(gqa_attn, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(mix_heads, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   done = true;
@@ -1247,6 +1248,7 @@ static dsk_state* state_create(dsk_model* m) {
       if (salloc(S, (void**)&ls.ssm, ls.ssm_bytes) || salloc(S, (void**)&ls.hist, ls.hist_bytes)) return nullptr;
       mx0 = std::max<size_t>(mx0, ssd_proj(sp)); mx1 = std::max<size_t>(mx1, ssd_channels(sp));
       mx2 = std::max<size_t>(mx2, ssd_inner(sp)); mx3 = std::max<size_t>(mx3, ssd_inner(sp));
+      mxLH = std::max<size_t>(mxLH, sp.ssm_heads);
     } else {
       if (M->runs[r].owner_run == (int)r) {
         ls.cache_bytes = (size_t)L.ring * sp.att_kv_rank * 4;
@@ -1578,10 +1580,25 @@ static void launch_gemm_t(int epi, const GemmP& P, int Z, bool small, int tile_c
     }
   }
 }
+// many rows, few columns (gemm_narrow); the epilogues such products have
+static void launch_narrow(bool bf16, int epi, const GemmP& P, cudaStream_t st) {
+  const dim3 grid((unsigned)((P.M + kNarrowRows - 1) / kNarrowRows), (unsigned)((P.N + 31) / 32));
+#define DSK_NARROW(E) case E: if (bf16) launch_next(gemm_narrow<__nv_bfloat16, E>, grid, 256, 0, st)(P); else launch_next(gemm_narrow<float, E>, grid, 256, 0, st)(P); break
+  switch (epi) {
+    DSK_NARROW(HEPI_STORE); DSK_NARROW(HEPI_ADD); DSK_NARROW(HEPI_XIELU); DSK_NARROW(HEPI_RELU2); DSK_NARROW(HEPI_LINGATE); DSK_NARROW(HEPI_SILU_SIG);
+    DSK_NARROW(HEPI_SOFTCAP); DSK_NARROW(HEPI_GELU_MUL);
+  }
+#undef DSK_NARROW
+}
 // C = A W^T (+ epilogue).  Z > 1: per-head batches or (gemv) one batch per routed (token, slot) pair.
 static void linear(State* S, bool bf16, int epi, const GemmP& P, int Z, cudaStream_t st, int tile_cap = 0) {
   const bool small = P.z_expert != nullptr || (!P.tiles && P.M <= 4);
   if (!small && !P.tiles && Z == 1 && P.N <= 96) {   // narrow output (router, token-input gate): warp-per-row products over batches of 4 rows
+    if (epi != HEPI_SIGMUL && P.M > 32 && !epi_dual(epi)) {
+      launch_narrow(bf16, epi, P, st);
+      S->launches++;
+      return;
+    }
     GemmP Q = P;
     Q.z_rows = P.M;
     const int zb = (P.M + 3) / 4;
@@ -1654,8 +1671,12 @@ static void launch_hgrn2(const dsk_layer_spec& sp, const float* proj, int ld, fl
 }
 
 // the walk over the blocks of a step (lin_scan): lanes per channel group by the key size, warps per CTA by how many CTAs there are
+static size_t ssd_gram_smem(const dsk_layer_spec& s) {
+  return ((size_t)2 * kLinBlk * (((s.ssm_state + 3) & ~3) + 4) + (size_t)2 * kLinBlk * (s.ssm_heads / s.ssm_groups)) * 4;
+}
 static void launch_lin_scan(bool delta, const float* q, const float* k, int ldq, int hs, int rep, const float* v, int ldv, const float* rec, float* state,
-                            float* out, int ldo, int T, int H, int N, int P, cudaStream_t st, float* nst = nullptr, float* den = nullptr) {
+                            float* out, int ldo, int T, int H, int N, int P, cudaStream_t st, float* nst = nullptr, float* den = nullptr, int sn = 0, int sp = 1) {
+  if (!sn) sn = P;                    // state rows [N][P] of a head, unless said otherwise
   const int TPC = N <= 32 ? 8 : N <= 64 ? 16 : 32, RQ = N <= 128 ? 1 : 2;
   int CPT = N > 128 ? 4 : 2;          // value channels per lane
   if (const char* e = getenv("DSK_LIN_CPT")) CPT = atoi(e) == 4 || N > 128 ? 4 : 2;   // A/B switch
@@ -1666,7 +1687,7 @@ static void launch_lin_scan(bool delta, const float* q, const float* k, int ldq,
   const int PB = warps * CW;
   const dim3 grid((unsigned)H, (unsigned)((P + (nst ? 1 : 0) + PB - 1) / PB));
   const size_t smem = lin_scan_smem(4 * TPC * RQ, PB, warps, CW);
-#define DSK_LSCAN(D, A, B, C) launch_next(lin_scan<D, A, B, C>, grid, 32 * (warps + kLinStage), smem, st)(q, k, ldq, hs, rep, v, ldv, rec, state, out, ldo, T, H, N, P, PB, nst, den)
+#define DSK_LSCAN(D, A, B, C) launch_next(lin_scan<D, A, B, C>, grid, 32 * (warps + kLinStage), smem, st)(q, k, ldq, hs, rep, v, ldv, rec, state, out, ldo, T, H, N, P, PB, nst, den, sn, sp)
 #define DSK_LSCANS(D) do { if (N > 128) DSK_LSCAN(D, 32, 2, 4); else if (CPT == 2) { if (N <= 32) DSK_LSCAN(D, 8, 1, 2); else if (N <= 64) DSK_LSCAN(D, 16, 1, 2); else DSK_LSCAN(D, 32, 1, 2); } \
   else { if (N <= 32) DSK_LSCAN(D, 8, 1, 4); else if (N <= 64) DSK_LSCAN(D, 16, 1, 4); else DSK_LSCAN(D, 32, 1, 4); } } while (0)
   if (delta) DSK_LSCANS(true); else DSK_LSCANS(false);
@@ -2244,7 +2265,16 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         if (sp.ssm_conv > 1) launch_next(conv_history_update, (ch + 127) / 128, 128, 0, st)(S->b0 + inner, pw, ls.hist, T, ch, sp.ssm_conv);
       }
       MK("ssd.conv");
-      launch_scan(sp, S->b0, pw, S->b1, ch, L, ls.ssm, S->b2, T, st);
+      if (T > kLinDecodeTokens && ssd_gram_smem(sp) <= 200 * 1024) {   // blocks of 16 tokens at once (ssd_scan: a chain over single tokens, 0.47 us each)
+        const int H = sp.ssm_heads, N = sp.ssm_state, P = sp.ssm_vdim, G = sp.ssm_groups;
+        launch_next(ssd_gram, dim3((unsigned)((T + kLinBlk - 1) / kLinBlk), (unsigned)G), 256, ssd_gram_smem(sp), st)(
+            S->b1 + inner + G * N, S->b1 + inner, ch, S->b0 + inner + ch, pw, L.dt_bias, L.A_log, T, H, N, H / G, S->lrec);
+        launch_lin_scan(false, S->b1 + inner + G * N, S->b1 + inner, ch, N, H / G, S->b1, ch, S->lrec, ls.ssm, S->b2, inner, T, H, N, P, st, nullptr, nullptr, 1, N);
+        if (inner % 4 == 0 && ch % 4 == 0 && pw % 4 == 0 && P % 4 == 0)
+          launch_next(ssd_gate<4>, dim3((unsigned)T, (unsigned)((inner + 1023) / 1024)), 256, 0, st)(S->b2, S->b1, ch, S->b0, pw, L.D, inner, P);
+        else launch_next(ssd_gate<1>, dim3((unsigned)T, (unsigned)((inner + 255) / 256)), 256, 0, st)(S->b2, S->b1, ch, S->b0, pw, L.D, inner, P);
+        S->launches += 2;
+      } else launch_scan(sp, S->b0, pw, S->b1, ch, L, ls.ssm, S->b2, T, st);
       MK("ssd.scan");
       launch_next(group_rmsnorm<float>, dim3((unsigned)T, (unsigned)sp.ssm_norm_groups), 256, 0, st)(S->b2, inner, L.mnorm, S->b3, inner, inner, sp.ssm_norm_groups, c.norm_eps, 0, 0.f, nullptr, 0, nullptr, 0);
       S->launches += 4;
@@ -2448,7 +2478,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         launch_next(layer_norm, T, 256, 0, st)(S->b3, W, L.close2, L.norm2_bias, S->x, W, W, c.norm_eps, 1, mult, S->wgt, top);
         S->launches++;
       } else if (!frms) {   // (sandwich blocks of RMS norms combine as they close)
-        launch_next(moe_combine, dim3((unsigned)T, (unsigned)((W + 255) / 256)), 256, 0, st)(sink.C, W, S->b3, S->wgt, top, W, sink.alpha, sink.epi == HEPI_ADD ? 1 : 0, shared ? ysh : nullptr, S->wsh);
+        launch_next(moe_combine, dim3((unsigned)T, (unsigned)((W + (W % 4 ? 255 : 1023)) / (W % 4 ? 256 : 1024))), 256, 0, st)(sink.C, W, S->b3, S->wgt, top, W, sink.alpha, sink.epi == HEPI_ADD ? 1 : 0, shared ? ysh : nullptr, S->wsh);
         S->launches++;
       }
       MK("moe.combine");

@@ -263,6 +263,69 @@ __global__ void __launch_bounds__(256) mlstm_gram(const float* __restrict__ q, c
   }
 }
 
+// The state-space recurrence S <- e^(a dt) S + dt B x^T, y = S^T C as the same walk (k = B, q = C, v = x, one key group per `rep` heads): records
+// with the weights e^(sum of a dt between two tokens) dt.  Grid (blocks, groups): the group's Gram products serve its heads.
+__global__ void __launch_bounds__(256) ssd_gram(const float* __restrict__ q, const float* __restrict__ k, int ld, const float* __restrict__ dt_raw, int ld_dt,
+                                                const float* __restrict__ dt_bias, const float* __restrict__ A_log, int T, int H, int N, int rep, float* __restrict__ rec) {
+  grid_enter();
+  extern __shared__ __align__(16) float sm[];
+  const int pitch = ((N + 3) & ~3) + 4, tid = threadIdx.x, t0 = blockIdx.x * kLinBlk, nt = min(kLinBlk, T - t0), g = blockIdx.y;
+  float* sq = sm;
+  float* sk = sq + kLinBlk * pitch;
+  float* sd = sk + kLinBlk * pitch;       // [rep][16] dt, then a dt
+  float* sf = sd + rep * kLinBlk;
+  for (int e = tid; e < kLinBlk * pitch; e += 256) {
+    const int t = e / pitch, n = e - t * pitch;
+    const bool ok = t < nt && n < N;
+    sq[e] = ok ? q[(size_t)(t0 + t) * ld + g * N + n] : 0.f;
+    sk[e] = ok ? k[(size_t)(t0 + t) * ld + g * N + n] : 0.f;
+  }
+  for (int e = tid; e < rep * kLinBlk; e += 256) {
+    const int h = g * rep + e / kLinBlk, t = e & (kLinBlk - 1);
+    const float dt = t < nt ? softplus_f(dt_raw[(size_t)(t0 + t) * ld_dt + h] + dt_bias[h]) : 0.f;
+    sd[e] = dt;
+    sf[e] = -expf(A_log[h]) * dt;
+  }
+  __syncthreads();
+  float kk, qk;
+  block_gram(sq, sk, pitch, (N + 3) >> 2, kk, qk);
+  const int j = tid >> 4, i = tid & 15;
+  for (int hh = 0; hh < rep; hh++) {
+    const float *d = sd + hh * kLinBlk, *f = sf + hh * kLinBlk;
+    float* R = rec + ((size_t)blockIdx.x * H + g * rep + hh) * kRecFloats;
+    float lr = 0.f;
+    for (int l = i + 1; l <= j; l++) lr += f[l];
+    R[kRecM + tid] = i <= j && j < nt ? expf(lr) * d[i] * qk : 0.f;
+    if (tid < kLinBlk) {
+      float lg = 0.f, le = 0.f;
+      for (int l = 0; l <= tid; l++) lg += f[l];
+      for (int l = tid + 1; l < nt; l++) le += f[l];
+      R[kRecG + tid] = tid < nt ? expf(lg) : 0.f;
+      R[kRecB + tid] = 1.f;
+      R[kRecE + tid] = tid < nt ? expf(le) * d[tid] : 0.f;
+      if (tid == nt - 1) R[kRecEnd] = expf(lg);
+    }
+  }
+}
+// y = (y + D x) silu(z) over the rows of a step, four channels per thread where they are aligned (V: channels per thread)
+template <int V>
+__global__ void __launch_bounds__(256) ssd_gate(float* __restrict__ y, const float* __restrict__ x, int ld_x, const float* __restrict__ z, int ld_z,
+                                                const float* __restrict__ Dskip, int inner, int P) {
+  grid_enter();
+  const int t = blockIdx.x, c = (blockIdx.y * 256 + threadIdx.x) * V;
+  if (c >= inner) return;
+  float *yr = y + (size_t)t * inner + c, yv[V], xv[V], zv[V];
+  const float *xr = x + (size_t)t * ld_x + c, *zr = z + (size_t)t * ld_z + c;
+  if constexpr (V == 4) {
+    const float4 a = *reinterpret_cast<const float4*>(yr), b = *reinterpret_cast<const float4*>(xr), d = *reinterpret_cast<const float4*>(zr);
+    yv[0] = a.x; yv[1] = a.y; yv[2] = a.z; yv[3] = a.w; xv[0] = b.x; xv[1] = b.y; xv[2] = b.z; xv[3] = b.w; zv[0] = d.x; zv[1] = d.y; zv[2] = d.z; zv[3] = d.w;
+  } else { yv[0] = yr[0]; xv[0] = xr[0]; zv[0] = zr[0]; }
+#pragma unroll
+  for (int u = 0; u < V; u++) yv[u] = fmaf(Dskip[(c + u) / P], xv[u], yv[u]) * silu_f(zv[u]);
+  if constexpr (V == 4) *reinterpret_cast<float4*>(yr) = make_float4(yv[0], yv[1], yv[2], yv[3]);
+  else yr[0] = yv[0];
+}
+
 // sums of 32 accumulators over TPC neighbouring lanes, scattered: afterwards a[0 .. 32 / TPC - 1] of a lane hold the totals of
 // the entries red_index(..) .. + 32 / TPC - 1
 template <int TPC>
@@ -293,13 +356,14 @@ __device__ __forceinline__ int reduce_index(int s) {
 // they bring the blocks' q, k, v and records through three buffers, two blocks ahead (16-byte asynchronous copies where the rows
 // allow it, plain loads otherwise), so a block costs the computing warps one barrier.
 // q, k: head stride hs (rows of N entries), v: head stride P; head h reads q / k head h / rep.
+// state: entry (n, p) of head h at h N P + n sn + p sp.
 // nst non-null: one more value channel (index P) whose value is 1 for every token, with its state in nst [H][N] and its output in den [T][H].
 // ---------------------------------------------------------------------------------------------------------------------
 constexpr int kLinStage = 2;           // staging warps of a CTA
 template <bool DELTA, int TPC, int RQ, int CPT>
 __global__ void __launch_bounds__(320) lin_scan(const float* __restrict__ q, const float* __restrict__ k, int ldq, int hs, int rep,
                                                 const float* __restrict__ v, int ldv, const float* __restrict__ rec, float* __restrict__ state,
-                                                float* __restrict__ out, int ldo, int T, int H, int N, int P, int PB, float* __restrict__ nst, float* __restrict__ den) {
+                                                float* __restrict__ out, int ldo, int T, int H, int N, int P, int PB, float* __restrict__ nst, float* __restrict__ den, int sn, int sp) {
   grid_enter();
   extern __shared__ __align__(16) float sm[];
   constexpr int C = kLinBlk, PITCH = 4 * TPC * RQ, CW = CPT * (32 / TPC), VB = 32 / CPT;
@@ -318,7 +382,7 @@ __global__ void __launch_bounds__(320) lin_scan(const float* __restrict__ q, con
       const int n = 4 * (s + TPC * r) + i;
 #pragma unroll
       for (int c = 0; c < CPT; c++) {
-        S[r][i][c] = (n < N && pc + c < P && cw + grp * CPT + c < PB) ? state[((size_t)h * N + n) * P + pc + c] : 0.f;
+        S[r][i][c] = (n < N && pc + c < P && cw + grp * CPT + c < PB) ? state[(size_t)h * N * P + (size_t)n * sn + (size_t)(pc + c) * sp] : 0.f;
         if (nst && n < N && pc + c == P && cw + grp * CPT + c < PB) S[r][i][c] = nst[(size_t)h * N + n];
       }
     }
@@ -491,7 +555,7 @@ __global__ void __launch_bounds__(320) lin_scan(const float* __restrict__ q, con
       const int n = 4 * (s + TPC * r) + i;
 #pragma unroll
       for (int c = 0; c < CPT; c++) {
-        if (n < N && pc + c < P && cw + grp * CPT + c < PB) state[((size_t)h * N + n) * P + pc + c] = S[r][i][c];
+        if (n < N && pc + c < P && cw + grp * CPT + c < PB) state[(size_t)h * N * P + (size_t)n * sn + (size_t)(pc + c) * sp] = S[r][i][c];
         if (nst && n < N && pc + c == P && cw + grp * CPT + c < PB) nst[(size_t)h * N + n] = S[r][i][c];
       }
     }

@@ -150,6 +150,21 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc5(const GemmP P, const T
       const int mine = min(32, nrows - quad * 32);            // rows of this warp
       int cr_lane = row0 + quad * 32 + lane;
       if (!T.C16 && P.c_map && lane < mine) cr_lane = P.c_map[cr_lane];
+      // epilogues on top of what C holds read it a 32 x 32 block ahead (the first under the products): a block's rows one after the other behind
+      // the accumulator cost a tile 26 us of waiting, more than its products
+      constexpr bool ON_C = EPI == HEPI_ADD || EPI == HEPI_SIGMUL;
+      float held[ON_C ? 32 : 1];
+      auto fetch_c = [&](int c0) {
+        if constexpr (ON_C) {
+          const int n = n0 + c0 + lane;
+#pragma unroll
+          for (int i = 0; i < 32; i++) {
+            const int cr = __shfl_sync(0xffffffffu, cr_lane, i);
+            held[i] = i < mine && n < P.N ? P.C[(size_t)cr * P.ldc + n] : 0.f;
+          }
+        }
+      };
+      fetch_c(0);
       const bool ok = tc_wait(done0 + 8 * buf, (nth >> 1) & 1, T.err);   // (every lane polls: the loads below are warp-wide)
       if (!__all_sync(0xffffffffu, ok)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -175,6 +190,19 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc5(const GemmP P, const T
         }
         __syncwarp();
         const int n = n0 + c0 + lane;
+        if constexpr (ON_C) {
+          float old[32];
+#pragma unroll
+          for (int i = 0; i < 32; i++) old[i] = held[i];
+          if (c0 + 32 < cols) fetch_c(c0 + 32);
+          const float bias = P.bias && n < P.N ? P.bias[n] : 0.f;
+#pragma unroll
+          for (int i = 0; i < 32; i++) {
+            const int cr = __shfl_sync(0xffffffffu, cr_lane, i);
+            const float v = turn[i * 33 + lane] + bias;
+            if (i < mine && n < P.N) P.C[(size_t)cr * P.ldc + n] = EPI == HEPI_ADD ? old[i] + P.alpha * v : old[i] * sigmoid_f(v);
+          }
+        } else
 #pragma unroll 8
         for (int i = 0; i < 32; i++) {
           const int cr = __shfl_sync(0xffffffffu, cr_lane, i);

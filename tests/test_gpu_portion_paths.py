@@ -1,0 +1,31 @@
+"""Paths that only portions take, at their edges, against the float64 statement: the state-space recurrence in blocks of 16 tokens (ragged last
+block, state sizes around the kernel's groups, heads sharing a group, a walk that continues a decoded state and is continued by one), narrow
+products over many rows (router and token-input gate: 16 rows, 32 columns, slices of 16), and products on top of what they add to."""
+import pytest
+
+from test_gpu_hybrid import F32_TOL, ho, in_portions, mk, rel, tokens_for  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+def ssd(heads, vdim, state, groups, conv=3):
+    return {"type": "mamba2", "mixer": {"heads": heads, "vdim": vdim, "state": state, "groups": groups, "conv": conv, "norm_groups": 1}, "mlp": None}
+
+
+@pytest.mark.parametrize("heads,vdim,state,groups", [(3, 5, 3, 1), (4, 12, 33, 2), (6, 8, 130, 3), (2, 65, 256, 1), (9, 4, 16, 3)])
+def test_recurrence_in_blocks(mk, ho, heads, vdim, state, groups):  # noqa: F811
+    cfg = ho.small_config(layers=[ssd(heads, vdim, state, groups)] * 2, width=36, norm={"eps": 1e-5, "groups": 1})
+    m, W = mk(cfg, seed=state, chunk=64)
+    toks = tokens_for(cfg, 90, 11)
+    exp = ho.run(cfg, W, toks)[0]
+    for sizes in ([64, 26], [5, 17, 1, 1, 33], [4, 16, 32], [15, 49]):
+        assert rel(in_portions(m, toks, sizes), exp) < F32_TOL
+
+
+@pytest.mark.parametrize("experts,side,width,tokens", [(5, 3, 36, 33), (33, 32, 40, 48), (96, 90, 72, 65), (7, 64, 130, 100)])
+def test_narrow_products(mk, ho, experts, side, width, tokens):  # noqa: F811
+    moe = {"kind": "moe", "router": {"experts": experts, "top": 2, "scale": 1.0}, "expert": {"ff": 12, "limit": 3.0}}
+    cfg = ho.small_config(layers=[dict(ssd(2, 6, 4, 1), mlp=moe)], width=width, norm={"eps": 1e-5, "groups": 1}, token_side={"dim": side})
+    m, W = mk(cfg, seed=experts, chunk=128)
+    toks = tokens_for(cfg, tokens, 12)
+    assert rel(m.forward_chunk(toks, 0, range(tokens)), ho.run(cfg, W, toks)[0]) < F32_TOL
