@@ -3,7 +3,8 @@ block, state sizes around the kernel's groups, heads sharing a group, a walk tha
 products over many rows (router and token-input gate: 16 rows, 32 columns, slices of 16), and products on top of what they add to."""
 import pytest
 
-from test_gpu_hybrid import F32_TOL, ho, in_portions, mk, rel, tokens_for  # noqa: F401
+from test_gpu_hybrid import F32_TOL, ho, mk, rel, tokens_for  # noqa: F401
+from test_gpu_netusun import in_portions
 
 pytestmark = pytest.mark.gpu
 
