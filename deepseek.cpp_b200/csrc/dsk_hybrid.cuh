@@ -308,9 +308,9 @@ struct GemmP {
   const void *sW1, *sW2;   // [sN][sK], packed
   const float* As;
   float* Cs;
-  // gemm_tc5 only.  n_expert: experts behind W (tile lists);  A16: the activations as packed bf16 rows in the product's row order (null: rounded
+  // n_expert: experts behind W, tile_rows: rows a tile may have (tile lists).  gemm_tc5 only:  A16: the activations as packed bf16 rows in the product's row order (null: rounded
   // from A by a pass of its own);  C16: results go there as packed bf16 rows in the product's row order instead of to C
-  int n_expert;
+  int n_expert, tile_rows;
   const __nv_bfloat16* A16;
   __nv_bfloat16* C16;
 };

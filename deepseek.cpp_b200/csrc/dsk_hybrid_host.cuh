@@ -178,6 +178,7 @@ struct State {
   long long launches = 0;
 };
 
+static constexpr int kSplitMinRows = 64;   // fp32 products of more rows run on gemm_split (at most half of its first 128-row tile is padding)
 static constexpr int kPrefillQ = 256, kPrefillMin = 32;   // prefill attention: queries per block / smallest portion that takes the matrix path
 static constexpr int kAttnSplitMax = 64, kAttnSplitTokens = 4;   // decode-sized chunks split a window over up to 64 CTAs
 
@@ -402,6 +403,10 @@ static void set_kernel_attrs() {
 #define DSK_PATTN_ATTR(A, B) cudaFuncSetAttribute(pattn<A, B, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax); cudaFuncSetAttribute(pattn<A, B, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax)
   DSK_PATTN_ATTR(1, 8); DSK_PATTN_ATTR(1, 16); DSK_PATTN_ATTR(3, 8); DSK_PATTN_ATTR(3, 16);
 #undef DSK_PATTN_ATTR
+#define DSK_SPLIT_ATTR(E) cudaFuncSetAttribute(gemm_split<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem)
+  DSK_SPLIT_ATTR(HEPI_STORE); DSK_SPLIT_ATTR(HEPI_ADD); DSK_SPLIT_ATTR(HEPI_GLU); DSK_SPLIT_ATTR(HEPI_XIELU); DSK_SPLIT_ATTR(HEPI_GEGLU); DSK_SPLIT_ATTR(HEPI_SIGMUL);
+  DSK_SPLIT_ATTR(HEPI_RELU2); DSK_SPLIT_ATTR(HEPI_LINGATE); DSK_SPLIT_ATTR(HEPI_SILU_SIG); DSK_SPLIT_ATTR(HEPI_SOFTCAP); DSK_SPLIT_ATTR(HEPI_SWIGLU); DSK_SPLIT_ATTR(HEPI_GELU_MUL);
+#undef DSK_SPLIT_ATTR
 #define DSK_TC5_ATTR(E) cudaFuncSetAttribute(gemm_tc5<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem)
   DSK_TC5_ATTR(HEPI_STORE); DSK_TC5_ATTR(HEPI_ADD); DSK_TC5_ATTR(HEPI_GLU); DSK_TC5_ATTR(HEPI_XIELU); DSK_TC5_ATTR(HEPI_GEGLU); DSK_TC5_ATTR(HEPI_SIGMUL);
   DSK_TC5_ATTR(HEPI_RELU2); DSK_TC5_ATTR(HEPI_LINGATE); DSK_TC5_ATTR(HEPI_SILU_SIG); DSK_TC5_ATTR(HEPI_SOFTCAP); DSK_TC5_ATTR(HEPI_SWIGLU); DSK_TC5_ATTR(HEPI_GELU_MUL);
@@ -1580,6 +1585,17 @@ static void launch_gemm_t(int epi, const GemmP& P, int Z, bool small, int tile_c
     }
   }
 }
+// fp32 products of more than 64 rows (gemm_split)
+static void launch_split(int epi, const GemmP& P, int Z, int tile_cap, cudaStream_t st) {
+  const int bn = epi_dual(epi) ? 32 : 64;
+  const dim3 grid((unsigned)((P.N + bn - 1) / bn), (unsigned)(P.tiles ? tile_cap : (P.M + 127) / 128), (unsigned)Z);
+#define DSK_SPLIT(E) case E: launch_next(gemm_split<E>, grid, 256, kSplitSmem, st)(P); break
+  switch (epi) {
+    DSK_SPLIT(HEPI_STORE); DSK_SPLIT(HEPI_ADD); DSK_SPLIT(HEPI_GLU); DSK_SPLIT(HEPI_XIELU); DSK_SPLIT(HEPI_GEGLU); DSK_SPLIT(HEPI_SIGMUL);
+    DSK_SPLIT(HEPI_RELU2); DSK_SPLIT(HEPI_LINGATE); DSK_SPLIT(HEPI_SILU_SIG); DSK_SPLIT(HEPI_SOFTCAP); DSK_SPLIT(HEPI_SWIGLU); DSK_SPLIT(HEPI_GELU_MUL);
+  }
+#undef DSK_SPLIT
+}
 // many rows, few columns (gemm_narrow); the epilogues such products have
 static void launch_narrow(bool bf16, int epi, const GemmP& P, cudaStream_t st) {
   const dim3 grid((unsigned)((P.M + kNarrowRows - 1) / kNarrowRows), (unsigned)((P.N + 31) / 32));
@@ -1610,6 +1626,7 @@ static void linear(State* S, bool bf16, int epi, const GemmP& P, int Z, cudaStre
   if (tc_ok(S, bf16, epi, P, Z)) launch_tc5(S, epi, P, tile_cap, st);
   else if (bf16 && !small) launch_gemm_mma(epi, P, Z, tile_cap, st);
   else if (bf16) launch_gemm_t<__nv_bfloat16>(epi, P, Z, small, tile_cap, st);
+  else if (!small && P.M > kSplitMinRows && (!P.tiles || P.tile_rows == 128)) launch_split(epi, P, Z, tile_cap, st);
   else launch_gemm_t<float>(epi, P, Z, small, tile_cap, st);
   S->launches++;
 }
@@ -2451,13 +2468,14 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         linear(S, bf, HEPI_STORE, Dn, pairs + (shared ? T : 0), st);
         MK("moe.down");
       } else {
-        const int bm = bf ? 128 : 64;   // rows per tile of the product kernel that follows (gemm_mma / gemm_tiled)
+        // rows per tile of the product kernel that follows (gemm_tc5, gemm_mma and gemm_split, or gemm_tiled: few rows per expert)
+        const int bm = bf || pairs >= 64 * E ? 128 : 64;
         launch_next(moe_plan, 1, 1024, (size_t)2 * E * 4, st)(S->d_idx, pairs, E, bm, S->d_perm, S->d_tiles, S->d_ntiles);
         S->launches++;
         G.tiles = S->d_tiles; G.n_tiles = S->d_ntiles; G.a_map = S->d_perm; G.a_div = top; G.c_map = S->d_perm;
         Dn.tiles = S->d_tiles; Dn.n_tiles = S->d_ntiles; Dn.a_map = S->d_perm; Dn.a_div = 1; Dn.c_map = S->d_perm;
         const int cap = std::min(S->max_tiles, pairs / bm + E + 1);
-        G.n_expert = Dn.n_expert = E;
+        G.n_expert = Dn.n_expert = E; G.tile_rows = Dn.tile_rows = bm;
         hidden16(S, bf, epi_up, G, HEPI_STORE, Dn, S->hid16);
         MK("moe.plan");
         linear(S, bf, epi_up, G, 1, st, cap);
