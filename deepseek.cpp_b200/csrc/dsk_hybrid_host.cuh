@@ -1168,7 +1168,7 @@ static dsk_state* state_create(dsk_model* m) {
   const size_t Tc = c.chunk;
   // the pieces the shared sampling / arg-max code reads
   cudaMalloc((void**)&s->ctrl, sizeof(Ctrl)); cudaMemset(s->ctrl, 0, sizeof(Ctrl));
-  cudaMallocHost((void**)&s->h_ctrl, sizeof(Ctrl)); memset(s->h_ctrl, 0, sizeof(Ctrl));
+  if (alloc_host_side(s)) return nullptr;
   s->token_log_cap = 1 << 16;
   cudaMalloc((void**)&s->token_log, s->token_log_cap * sizeof(int));
   cudaMalloc((void**)&s->step, sizeof(int));
@@ -2574,12 +2574,13 @@ static int forward_chunk(dsk_model* m, dsk_state* s, const int32_t* tokens, int 
     for (int g0 = 0; g0 < nw; g0 += S->head_rows) {   // the LM head in groups of head_rows wanted rows
       const int gn = std::min(S->head_rows, nw - g0);
       if (g0 > 0) enqueue_head(m, s, g0, gn, S->logits, s->stream);
-      if (host_logits) CK(cudaMemcpyAsync(host_logits + (size_t)(wi + g0) * c.vocab_size, S->logits, (size_t)gn * c.vocab_size * 4, cudaMemcpyDeviceToHost, s->stream));
-    }
-    if (nw) {   // the last wanted row stays in the state for the samplers
-      CK(cudaMemcpyAsync(s->logits, S->logits + (size_t)((nw - 1) % S->head_rows) * c.vocab_size, (size_t)c.vocab_size * 4, cudaMemcpyDeviceToDevice, s->stream));
-      CK(cudaMemsetAsync(&s->ctrl->argmax_key, 0, sizeof(s->ctrl->argmax_key), s->stream));
-      launch_argmax(s, c.vocab_size);
+      if (g0 + gn == nw) {   // the last wanted row stays in the state for the samplers
+        CK(cudaMemcpyAsync(s->logits, S->logits + (size_t)(gn - 1) * c.vocab_size, (size_t)c.vocab_size * 4, cudaMemcpyDeviceToDevice, s->stream));
+        CK(cudaMemsetAsync(&s->ctrl->argmax_key, 0, sizeof(s->ctrl->argmax_key), s->stream));
+        launch_argmax(s, c.vocab_size);
+        CK(cudaMemcpyAsync(s->h_ctrl, s->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, s->stream));
+      }
+      if (host_logits && copy_to_host(s, host_logits + (size_t)(wi + g0) * c.vocab_size, S->logits, (size_t)gn * c.vocab_size * 4)) return -2;
     }
     timeline_report(S, T);
     if (host_layers) {
