@@ -315,7 +315,7 @@ struct GemmP {
   __nv_bfloat16* C16;
 };
 
-// the epilogues that join two matrices' results, and those that are a function of one result and its column
+// the epilogues that join two matrices' results
 template <int EPI>
 __device__ __forceinline__ float dual_value(const GemmP& P, float v, float v2) {
   if (EPI == HEPI_GEGLU) return gelu_tanh_f(v) * v2;
@@ -323,33 +323,34 @@ __device__ __forceinline__ float dual_value(const GemmP& P, float v, float v2) {
   const float g = fminf(v, P.lim), u = fminf(fmaxf(v2, -P.lim), P.lim);   // HEPI_GLU
   return g * sigmoid_f(1.702f * g) * (u + 1.f);
 }
-template <int EPI>
-__device__ __forceinline__ float epi_value(const GemmP& P, int n, float v) {   // (joined results come as they are)
-  if (epi_dual(EPI)) return v;
+// what C[row cr][n] becomes, from the result v of a single product and, for the epilogues on top of it, what C holds
+template <typename WT, int EPI>
+__device__ __forceinline__ float final_value(const GemmP& P, int cr, int n, float v, float old) {
   if (P.bias) v += P.bias[n];
+  if (EPI == HEPI_STORE) return P.alpha * v;
+  if (EPI == HEPI_ADD) return old + P.alpha * v;
   if (EPI == HEPI_XIELU) return v > 0.f ? fmaf(P.act_a * v, v, 0.5f * v) : fmaf(P.act_b, expm1f(v) - v, 0.5f * v);
   if (EPI == HEPI_RELU2) { const float r = fmaxf(v, 0.f); return r * r; }
-  return P.alpha * v;
+  if (EPI == HEPI_SIGMUL) return old * sigmoid_f(v);
+  if (EPI == HEPI_SILU_SIG) return n < P.aux_off ? silu_f(v) : sigmoid_f(v);
+  if (EPI == HEPI_SOFTCAP) return P.lim * tanhf(P.alpha * v / P.lim);
+  if (EPI == HEPI_LINGATE) {
+    const int hn = P.aux_off;
+    if (n < hn) return silu_f(v);
+    if (n >= 2 * hn) return v;
+    const float lo = reinterpret_cast<const float*>(P.aux)[n - hn];
+    return fmaf(1.f - lo, sigmoid_f(v), lo);
+  }
+  const WT* aux = reinterpret_cast<const WT*>(P.aux);   // HEPI_GELU_MUL
+  return gelu_tanh_f(v) * to_f<WT>(aux[(size_t)P.aux_row[cr] * P.aux_ld + P.aux_off + n]);
 }
-
 template <typename WT, int EPI>
 __device__ __forceinline__ void gemm_epilogue(const GemmP& P, float* __restrict__ crow, int cr, int n, float v, float v2) {
-  if (EPI == HEPI_STORE || EPI == HEPI_XIELU || EPI == HEPI_RELU2) { crow[n] = epi_value<EPI>(P, n, v); return; }
-  if (P.bias) v += P.bias[n];
-  if (EPI == HEPI_ADD) crow[n] += P.alpha * v;
-  else if (epi_dual(EPI)) crow[n] = dual_value<EPI>(P, v, v2);
-  else if (EPI == HEPI_SIGMUL) crow[n] *= sigmoid_f(v);
-  else if (EPI == HEPI_SILU_SIG) crow[n] = n < P.aux_off ? silu_f(v) : sigmoid_f(v);
-  else if (EPI == HEPI_SOFTCAP) crow[n] = P.lim * tanhf(P.alpha * v / P.lim);
-  else if (EPI == HEPI_LINGATE) {
-    const int hn = P.aux_off;
-    if (n < hn) crow[n] = silu_f(v);
-    else if (n < 2 * hn) { const float lo = reinterpret_cast<const float*>(P.aux)[n - hn]; crow[n] = fmaf(1.f - lo, sigmoid_f(v), lo); }
-    else crow[n] = v;
-  }
-  else {
-    const WT* aux = reinterpret_cast<const WT*>(P.aux);
-    crow[n] = gelu_tanh_f(v) * to_f<WT>(aux[(size_t)P.aux_row[cr] * P.aux_ld + P.aux_off + n]);
+  if constexpr (epi_dual(EPI)) {
+    if (P.bias) v += P.bias[n];
+    crow[n] = dual_value<EPI>(P, v, v2);
+  } else {
+    crow[n] = final_value<WT, EPI>(P, cr, n, v, EPI == HEPI_ADD || EPI == HEPI_SIGMUL ? crow[n] : 0.f);
   }
 }
 

@@ -28,6 +28,7 @@ struct TcP {
   int bn, stages, n_mt, rows_per_expert;   // column tile, ring stages, row tiles (no tile list), weight rows between experts
   __nv_bfloat16* C16;                      // non-null: results go here as bf16, row = position in the product (no c_map), pitch ldc16
   int ldc16;
+  int wide;                                // rows of C (C16) take 32-byte (16-byte) accesses at columns that are multiples of eight
   int* err;                                // host-visible word: set when a wait gave up
 };
 
@@ -64,6 +65,14 @@ __device__ __forceinline__ void tc_load32(uint32_t addr, uint32_t (&r)[32]) {
         "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
         "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(addr));
+}
+
+__device__ __forceinline__ void store8(float* p, const float* v) {   // 32 bytes
+  asm volatile("st.global.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]) : "memory");
+}
+__device__ __forceinline__ void load8(const float* p, float* v) {
+  asm volatile("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]) : "l"(p) : "memory");
 }
 
 template <int EPI>
@@ -150,17 +159,19 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc5(const GemmP P, const T
       const int mine = min(32, nrows - quad * 32);            // rows of this warp
       int cr_lane = row0 + quad * 32 + lane;
       if (!T.C16 && P.c_map && lane < mine) cr_lane = P.c_map[cr_lane];
-      // epilogues on top of what C holds read it a 32 x 32 block ahead (the first under the products): a block's rows one after the other behind
-      // the accumulator cost a tile 26 us of waiting, more than its products
+      // A lane has one row of the accumulator.  Where rows of C take 32-byte stores it writes its 32 columns of a block by itself; ragged blocks and
+      // odd pitches are turned through shared memory so that a warp stores along rows (turning every block and storing 64 or 128 bytes at a time was what
+      // bound a tile: the expert products of 2048 tokens took 240 + 150 us a layer, now 225 + 115).  Epilogues on top of what C holds read it a block ahead
+      // (the first under the products; a 2048 x 2048 product of 2048 tokens onto the stream: 50 -> 38 us).
+      float* crow = P.C + (lane < mine ? (size_t)cr_lane * P.ldc : 0) + n0;
+      __nv_bfloat16* crow16 = T.C16 + (lane < mine ? (size_t)cr_lane * T.ldc16 : 0) + n0;
       constexpr bool ON_C = EPI == HEPI_ADD || EPI == HEPI_SIGMUL;
       float held[ON_C ? 32 : 1];
       auto fetch_c = [&](int c0) {
         if constexpr (ON_C) {
-          const int n = n0 + c0 + lane;
+          if (T.wide && n0 + c0 + 32 <= P.N && lane < mine) {
 #pragma unroll
-          for (int i = 0; i < 32; i++) {
-            const int cr = __shfl_sync(0xffffffffu, cr_lane, i);
-            held[i] = i < mine && n < P.N ? P.C[(size_t)cr * P.ldc + n] : 0.f;
+            for (int q = 0; q < 32; q += 8) load8(crow + c0 + q, held + q);
           }
         }
       };
@@ -172,48 +183,62 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc5(const GemmP P, const T
         uint32_t r[32];
         const uint32_t at = tmem + ((uint32_t)(quad * 32) << 16) + buf * 256 + c0;
         tc_load32(at, r);
-        if (DUAL) {
-          uint32_t r2[32];
-          tc_load32(at + cols, r2);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-          for (int c = 0; c < 32; c++) turn[lane * 33 + c] = dual_value<EPI>(P, __uint_as_float(r[c]), __uint_as_float(r2[c]));
-        } else {
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-          for (int c = 0; c < 32; c++) turn[lane * 33 + c] = __uint_as_float(r[c]);
-        }
+        uint32_t r2[DUAL ? 32 : 1];
+        if constexpr (DUAL) tc_load32(at + cols, r2);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         if (c0 + 32 >= cols) {                               // the accumulator is read: the next tile but one may have it
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
           if (lane == 0) tc_arrive(drained0 + 8 * buf);
         }
-        __syncwarp();
-        const int n = n0 + c0 + lane;
-        if constexpr (ON_C) {
-          float old[32];
+        float v[32];
 #pragma unroll
-          for (int i = 0; i < 32; i++) old[i] = held[i];
-          if (c0 + 32 < cols) fetch_c(c0 + 32);
-          const float bias = P.bias && n < P.N ? P.bias[n] : 0.f;
+        for (int c = 0; c < 32; c++) v[c] = __uint_as_float(r[c]);
+        if constexpr (DUAL) {
 #pragma unroll
+          for (int c = 0; c < 32; c++) v[c] = dual_value<EPI>(P, v[c], __uint_as_float(r2[c]));
+        }
+        if (T.wide && n0 + c0 + 32 <= P.N) {
+          if (lane < mine) {
+            if constexpr (!DUAL) {
+#pragma unroll
+              for (int c = 0; c < 32; c++) v[c] = final_value<__nv_bfloat16, EPI>(P, cr_lane, n0 + c0 + c, v[c], ON_C ? held[ON_C ? c : 0] : 0.f);
+            }
+            if (T.C16) {
+#pragma unroll
+              for (int q = 0; q < 32; q += 8) {
+                uint4 o;
+                uint32_t* w = reinterpret_cast<uint32_t*>(&o);
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                  const __nv_bfloat162 pr = __floats2bfloat162_rn(v[q + 2 * u], v[q + 2 * u + 1]);
+                  w[u] = *reinterpret_cast<const uint32_t*>(&pr);
+                }
+                *reinterpret_cast<uint4*>(crow16 + c0 + q) = o;
+              }
+            } else {
+              if (c0 + 32 < cols) fetch_c(c0 + 32);
+#pragma unroll
+              for (int q = 0; q < 32; q += 8) store8(crow + c0 + q, v + q);
+            }
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < 32; c++) turn[lane * 33 + c] = v[c];
+          __syncwarp();
+          const int n = n0 + c0 + lane;
+#pragma unroll 4
           for (int i = 0; i < 32; i++) {
             const int cr = __shfl_sync(0xffffffffu, cr_lane, i);
-            const float v = turn[i * 33 + lane] + bias;
-            if (i < mine && n < P.N) P.C[(size_t)cr * P.ldc + n] = EPI == HEPI_ADD ? old[i] + P.alpha * v : old[i] * sigmoid_f(v);
+            if (i < mine && n < P.N) {
+              float* c = P.C + (size_t)cr * P.ldc + n;
+              const float old = ON_C ? *c : 0.f, x = DUAL ? turn[i * 33 + lane] : final_value<__nv_bfloat16, EPI>(P, cr, n, turn[i * 33 + lane], old);
+              if (T.C16) T.C16[(size_t)cr * T.ldc16 + n] = __float2bfloat16_rn(x);
+              else *c = x;
+            }
           }
-        } else
-#pragma unroll 8
-        for (int i = 0; i < 32; i++) {
-          const int cr = __shfl_sync(0xffffffffu, cr_lane, i);
-          if (i < mine && n < P.N) {
-            const float v = turn[i * 33 + lane];
-            if (T.C16) T.C16[(size_t)cr * T.ldc16 + n] = __float2bfloat16_rn(epi_value<EPI>(P, n, v));
-            else if (DUAL) P.C[(size_t)cr * P.ldc + n] = v;
-            else gemm_epilogue<__nv_bfloat16, EPI>(P, P.C + (size_t)cr * P.ldc, cr, n, v, 0.f);
-          }
+          __syncwarp();
         }
-        __syncwarp();
       }
     }
   }

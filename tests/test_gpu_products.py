@@ -26,6 +26,17 @@ def test_routed_edges(mk, no, experts, top, ff, tokens):  # noqa: F811
     assert close_bf16(m.forward_chunk(toks, 0, range(tokens)), no.run(cfg, W, toks)[0], no.rounding_noise(cfg, W, toks))
 
 
+# results stored by rows (32 bytes a lane) and turned through shared memory: rows of C that are no multiple of eight columns (84), blocks of 32
+# columns that end inside the matrix (72, 136, 264), whole ones (256); additions into the residual rows, gated pairs, scattered expert rows
+@pytest.mark.parametrize("width,experts,top,ff,tokens", [(84, 2, 1, 104, 60), (136, 2, 2, 264, 256), (256, 3, 2, 128, 300), (100, 1, 1, 72, 129)])
+def test_stores(mk, no, width, experts, top, ff, tokens):  # noqa: F811
+    cfg = no.model_config([no.att(heads=4, dim=32, vdim=24, size=40, mlp=no.moe(experts=experts, top=top, ff=ff, shared=2 * ff)), no.lat(mlp=no.dense(ff))],
+                          width=width, vocab=131)
+    m, W = mk(cfg, seed=tokens, quant="bf16", chunk=512)
+    toks = tokens_for(cfg, tokens, 6)
+    assert close_bf16(m.forward_chunk(toks, 0, range(tokens)), no.run(cfg, W, toks)[0], no.rounding_noise(cfg, W, toks))
+
+
 def test_unaligned_depth_and_short_steps(mk, no):  # noqa: F811
     """Depths that TMA cannot address (not a multiple of 8) and the steps of up to four rows keep their own kernels."""
     cfg = no.model_config([no.att(heads=3, dim=10, vdim=6, mlp=no.dense(98))], width=84, vocab=61)
