@@ -178,7 +178,6 @@ struct State {
   long long launches = 0;
 };
 
-static constexpr int kSplitMinRows = 64;   // fp32 products of more rows run on gemm_split (at most half of its first 128-row tile is padding)
 static constexpr int kPrefillQ = 256, kPrefillMin = 32;   // prefill attention: queries per block / smallest portion that takes the matrix path
 static constexpr int kAttnSplitMax = 64, kAttnSplitTokens = 4;   // decode-sized chunks split a window over up to 64 CTAs
 
@@ -1586,7 +1585,7 @@ static void launch_gemm_t(int epi, const GemmP& P, int Z, bool small, int tile_c
     }
   }
 }
-// fp32 products of more than 64 rows (gemm_split)
+// fp32 products of more than four rows, routed ones in tiles of 128 (gemm_split)
 static void launch_split(int epi, const GemmP& P, int Z, int tile_cap, cudaStream_t st) {
   const int bn = epi_dual(epi) ? 32 : 64;
   const dim3 grid((unsigned)((P.N + bn - 1) / bn), (unsigned)(P.tiles ? tile_cap : (P.M + 127) / 128), (unsigned)Z);
@@ -1627,7 +1626,7 @@ static void linear(State* S, bool bf16, int epi, const GemmP& P, int Z, cudaStre
   if (tc_ok(S, bf16, epi, P, Z)) launch_tc5(S, epi, P, tile_cap, st);
   else if (bf16 && !small) launch_gemm_mma(epi, P, Z, tile_cap, st);
   else if (bf16) launch_gemm_t<__nv_bfloat16>(epi, P, Z, small, tile_cap, st);
-  else if (!small && P.M > kSplitMinRows && (!P.tiles || P.tile_rows == 128)) launch_split(epi, P, Z, tile_cap, st);
+  else if (!small && (!P.tiles || P.tile_rows == 128)) launch_split(epi, P, Z, tile_cap, st);
   else launch_gemm_t<float>(epi, P, Z, small, tile_cap, st);
   S->launches++;
 }
@@ -2470,6 +2469,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         MK("moe.down");
       } else {
         // rows per tile of the product kernel that follows (gemm_tc5, gemm_mma and gemm_split, or gemm_tiled: few rows per expert)
+        // (fp32, under 64 rows per expert: gemm_tiled's FMA on 64 rows are fewer cycles than six tensor-core products on 128)
         const int bm = bf || pairs >= 64 * E ? 128 : 64;
         launch_next(moe_plan, 1, 1024, (size_t)2 * E * 4, st)(S->d_idx, pairs, E, bm, S->d_perm, S->d_tiles, S->d_ntiles);
         S->launches++;
