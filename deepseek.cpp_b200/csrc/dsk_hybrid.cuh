@@ -20,7 +20,7 @@
 //                     keys and values written into their ring caches
 //   gqa_attn          softmax attention of grouped query heads over ring caches of keys and values with a window or chunk mask
 //                     and optional mixing of the heads' scores before the softmax (decode-sized steps)
-//   pack_ring_kv, mix_heads, softmax_band   the same attention for portions, between three matrix products
+//   pack_ring_kv, mix_softmax, softmax_band   the same attention for portions, between three matrix products
 //   token_shift       h_t + (h_(t-1) - h_t) * mu in front of a mixer, the last row carried from step to step
 //   rms_add_shift_small   decode-sized steps: an RMS-normed addition into the stream and the next layer's token shift in one launch
 //   rms_open          opening of a pre-norm sublayer: additions of a loop pass and the RMS norm in one launch
@@ -313,7 +313,12 @@ struct GemmP {
   int n_expert, tile_rows;
   const __nv_bfloat16* A16;
   __nv_bfloat16* C16;
+  // gemm_split only: scores of queries at positions band_pos + row against keys at positions band_first + column (BAND_COLS: tiles that no query of
+  // theirs sees are left out) and the product of such rows with the values (BAND_DEPTH: the depth that a row tile sees; the rows hold 0
+  // elsewhere).  band_keep: the first columns are kept first positions, which all queries see
+  int band, band_first, band_pos, band_mask, band_window, band_keep;
 };
+enum { BAND_NONE, BAND_COLS, BAND_DEPTH };
 
 // the epilogues that join two matrices' results
 template <int EPI>
@@ -2184,7 +2189,7 @@ __global__ void __launch_bounds__(256) gqa_attn(const float* __restrict__ q, con
 
 // Portions run the same attention as matrix products per block of queries (like the latent attention above).  pack_ring_kv
 // gathers the visible positions first .. first + Lk - 1 from the ring caches into per-group operands: keys [G][Lk][D], values
-// transposed [G][Dv][Lk].  mix_heads applies the heads' score mixing to a [H][Tq][Lk] score array (out of place).
+// transposed [G][Dv][Lk].  mix_softmax mixes the heads' scores in a [H][Tq][Lk] score array.
 // The first nk operand rows are the kept first positions 0 .. nk - 1 (cache rows of their own, see cache_row).
 template <typename WT>
 __global__ void pack_ring_kv(const float* __restrict__ kc, const float* __restrict__ vc, WT* __restrict__ kb, WT* __restrict__ vt,
@@ -2269,22 +2274,66 @@ __global__ void pack_mla_kv(const float* __restrict__ kf, const float* __restric
   }
 }
 
-// out[h][e] = sum_g talk[h][g] in[g][e] for the n = Tq * Lk entries of every head; a CTA takes 128 consecutive entries
-__global__ void __launch_bounds__(128) mix_heads(const float* __restrict__ in, float* __restrict__ out, const float* __restrict__ talk,
-                                                 int H, long long n) {
+// One CTA per query, in place on S [H][Tq][Lk]: the heads' scores of a key mixed, s'_h = sum_g talk[h][g] s_g, masked, and the softmax over a
+// head's keys (hidden keys get 0 and are not read).  HR > 0: a thread has the HR >= H scores of a key in registers; 0 (more than 32 heads):
+// in shared memory.  The mixed scores stay in shared memory between the two parts where H x Lk floats fit (staged), else in S.
+// Bound: the scores' way in and out of L2.  Mixing and softmax as kernels of their own, with an array between them, took 39 us per 256 queries
+// of 16 heads behind 1023 keys.
+template <int HR>
+__global__ void __launch_bounds__(HR ? 512 : 128) mix_softmax(float* __restrict__ S, const float* __restrict__ talk, int H, int Tq, int Lk, int first, int qpos0,
+                                                              int mask, int window, int nk, ScoreMods sm, int staged) {
   grid_enter();
-  extern __shared__ float sm[];
-  float* tk = sm;              // [H][H]
-  float* col = sm + H * H;     // [H][128]
-  const long long e = (long long)blockIdx.x * 128 + threadIdx.x;
-  for (int k = threadIdx.x; k < H * H; k += blockDim.x) tk[k] = talk[k];
-  if (e < n) for (int g = 0; g < H; g++) col[g * 128 + threadIdx.x] = in[(size_t)g * n + e];
+  extern __shared__ __align__(16) float sh[];
+  constexpr int TP = HR ? HR : 1;
+  const int tp = HR ? TP : H, t = blockIdx.x, i = qpos0 + t, j_lo = mask_first(mask, window, i), nt = blockDim.x;
+  float* tk = sh;                                            // [H][tp]
+  float* col = sh + (H * tp + 3) / 4 * 4;                    // HR 0: [H][nt]
+  float* row = S + (size_t)t * Lk;                           // head g: + g Tq Lk
+  const size_t hs = (size_t)Tq * Lk;
+  float* mixed = staged ? col + (HR ? 0 : H * nt) : row;
+  const size_t ms = staged ? (size_t)Lk : hs;
+  for (int k = threadIdx.x; k < H * tp; k += nt) tk[k] = k % tp < H ? talk[k / tp * H + k % tp] : 0.f;
   __syncthreads();
-  if (e >= n) return;
-  for (int h = 0; h < H; h++) {
-    float s = 0.f;
-    for (int g = 0; g < H; g++) s = fmaf(tk[h * H + g], col[g * 128 + threadIdx.x], s);
-    out[(size_t)h * n + e] = s;
+  auto visible = [&](int c) { const int j = c < nk ? c : first + c - nk; return j <= i && (j >= j_lo || j < sm.keep); };
+  for (int c = threadIdx.x; c < Lk; c += nt) {
+    if (!visible(c)) continue;
+    const int dist = i - (c < nk ? c : first + c - nk);
+    if constexpr (HR > 0) {
+      float v[HR];
+#pragma unroll
+      for (int g = 0; g < HR; g++) v[g] = g < H ? row[g * hs + c] : 0.f;
+      for (int h = 0; h < H; h++) {
+        float x = 0.f;
+#pragma unroll
+        for (int g = 0; g < HR; g += 4) {
+          const float4 w = *reinterpret_cast<const float4*>(tk + h * HR + g);
+          x = fmaf(w.x, v[g], x); x = fmaf(w.y, v[g + 1], x); x = fmaf(w.z, v[g + 2], x); x = fmaf(w.w, v[g + 3], x);
+        }
+        mixed[h * ms + c] = mod_score(sm, x, dist, h, H);
+      }
+    } else {
+      for (int g = 0; g < H; g++) col[g * nt + threadIdx.x] = row[g * hs + c];
+      for (int h = 0; h < H; h++) {
+        float x = 0.f;
+        for (int g = 0; g < H; g++) x = fmaf(tk[h * H + g], col[g * nt + threadIdx.x], x);
+        mixed[h * ms + c] = mod_score(sm, x, dist, h, H);
+      }
+    }
+  }
+  __syncthreads();
+  for (int h = threadIdx.x >> 5; h < H; h += nt >> 5) {      // a warp per head
+    const int lane = threadIdx.x & 31;
+    float* m = mixed + h * ms;
+    float* out = row + h * hs;
+    const float sink = sm.sink ? sm.sink[h] : -1e30f;
+    float mx = sink, sum = 0.f;
+    for (int c = lane; c < Lk; c += 32) if (visible(c)) mx = fmaxf(mx, m[c]);
+    mx = warp_max(mx);
+    for (int c = lane; c < Lk; c += 32) if (visible(c)) { const float p = expf(m[c] - mx); m[c] = p; sum += p; }
+    sum = warp_sum(sum);
+    if (sm.sink) sum += expf(sink - mx);
+    const float inv = 1.f / sum;
+    for (int c = lane; c < Lk; c += 32) out[c] = visible(c) ? m[c] * inv : 0.f;
   }
 }
 

@@ -141,7 +141,8 @@ struct State {
   int head_rows = 0;                         // rows of the logits buffer: the LM head runs over the wanted rows in groups of this size
   float* part = nullptr;                     // partial softmax results of key-split attention (decode-sized chunks)
   // prefill attention as matrix products (blocks of kPrefillQ queries): up-projected keys / values, their per-head packing, scores
-  float *kf = nullptr, *vf = nullptr, *sc = nullptr, *sc2 = nullptr;   // sc2: scores after the heads were mixed
+  float *kf = nullptr, *vf = nullptr, *sc = nullptr;
+  int talk_q = 0;   // queries per block of layers that mix heads
   void *kb = nullptr, *vt = nullptr;
   int* d_rows = nullptr;
   int prefill_keys = 0;                      // keys a block of queries can see at most; 0: the matrix path is off
@@ -415,7 +416,8 @@ static void set_kernel_attrs() {
   cudaFuncSetAttribute(decode_attn<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big); cudaFuncSetAttribute(decode_attn<false, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(ssd_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(gqa_attn, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(mix_heads, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(mix_softmax<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, big); cudaFuncSetAttribute(mix_softmax<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+  cudaFuncSetAttribute(mix_softmax<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   done = true;
 }
 
@@ -1288,22 +1290,27 @@ static dsk_state* state_create(dsk_model* m) {
   rc |= salloc(S, (void**)&S->part, mxPart * 4);
   if ((int)Tc >= kPrefillMin) {   // buffers of the matrix-product attention path, unless a window is too long for them
     // latent attention up-projects keys and values of all heads (fp32, then packed in the matrix type); grouped-query
-    // attention packs its cached key / value heads in fp32 (kf / vf) and needs a second score array when it mixes heads
+    // attention packs its cached key / value heads in fp32 (kf / vf)
     // (latent attention with a rotated key part packs in fp32: its scores are 32-bit products)
-    size_t keys = 0, hd = 0, hv = 0, heads = 0, pack_es = 0;
+    size_t keys = 0, hd = 0, hv = 0, heads = 0, pack_es = 0, bytes = 0;
     bool latent = false;
-    for (const HLayer& L : M->L) {
-      if (!has_attn(L.sp)) continue;
-      const size_t kh = L.sp.mixer == DSK_MIX_GQA ? L.sp.att_kv_heads : L.sp.att_heads;
-      latent |= L.sp.mixer == DSK_MIX_LATENT_SWA || L.sp.mixer == DSK_MIX_MLA;
-      if (L.sp.mixer == DSK_MIX_LATENT_SWA) pack_es = std::max(pack_es, M->wsize);
-      if (L.sp.mixer == DSK_MIX_MLA) pack_es = 4;
-      keys = std::max<size_t>(keys, (size_t)std::min<long long>((long long)L.sp.att_window - 1, (long long)c.max_seq_len) + std::min<size_t>(Tc, kPrefillQ) +
-                                        (L.sp.mixer == DSK_MIX_GQA ? L.sp.att_keep_first : 0));
-      hd = std::max<size_t>(hd, kh * (L.sp.att_dim + (L.sp.mixer == DSK_MIX_MLA ? L.sp.att_rot_dim : 0))); hv = std::max<size_t>(hv, kh * L.sp.att_vdim);
-      heads = std::max<size_t>(heads, L.sp.att_heads);
+    // (layers that mix heads take 512 queries at a time, where their scores fit: a head's product with the values is then 8 tiles)
+    for (S->talk_q = any_talk ? 2 * kPrefillQ : kPrefillQ;; S->talk_q = kPrefillQ) {
+      keys = 0;
+      for (const HLayer& L : M->L) {
+        if (!has_attn(L.sp)) continue;
+        const size_t kh = L.sp.mixer == DSK_MIX_GQA ? L.sp.att_kv_heads : L.sp.att_heads;
+        latent |= L.sp.mixer == DSK_MIX_LATENT_SWA || L.sp.mixer == DSK_MIX_MLA;
+        if (L.sp.mixer == DSK_MIX_LATENT_SWA) pack_es = std::max(pack_es, M->wsize);
+        if (L.sp.mixer == DSK_MIX_MLA) pack_es = 4;
+        keys = std::max<size_t>(keys, (size_t)std::min<long long>((long long)L.sp.att_window - 1, (long long)c.max_seq_len) + std::min<size_t>(Tc, S->talk_q) +
+                                          (L.sp.mixer == DSK_MIX_GQA ? L.sp.att_keep_first : 0));
+        hd = std::max<size_t>(hd, kh * (L.sp.att_dim + (L.sp.mixer == DSK_MIX_MLA ? L.sp.att_rot_dim : 0))); hv = std::max<size_t>(hv, kh * L.sp.att_vdim);
+        heads = std::max<size_t>(heads, L.sp.att_heads);
+      }
+      bytes = keys * (hd + hv) * (4 + (latent ? pack_es : 0)) + heads * S->talk_q * keys * 4;
+      if (bytes <= ((size_t)4 << 30) || S->talk_q == kPrefillQ) break;
     }
-    const size_t bytes = keys * (hd + hv) * (4 + (latent ? pack_es : 0)) + heads * kPrefillQ * keys * 4 * (any_talk ? 2 : 1);
     if (keys > 0 && bytes <= ((size_t)4 << 30)) {
       // layers that run pattn: the visible keys of a whole step split into bf16 parts, behind the up-projected fp32 rows of latent layers (blocks of
       // kPrefillQ queries where a step's keys would take over 4 GB)
@@ -1330,8 +1337,7 @@ static dsk_state* state_create(dsk_model* m) {
       rc |= salloc(S, (void**)&S->d_rows, rows * 4);
       if (old) {
         if (latent) rc |= salloc(S, &S->kb, keys * hd * pack_es) | salloc(S, &S->vt, keys * hv * pack_es);
-        rc |= salloc(S, (void**)&S->sc, heads * kPrefillQ * keys * 4);
-        if (any_talk) rc |= salloc(S, (void**)&S->sc2, heads * kPrefillQ * keys * 4);
+        rc |= salloc(S, (void**)&S->sc, heads * S->talk_q * keys * 4);
       }
     }
   }
@@ -2072,29 +2078,33 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
           }
           MK("att.fused");
         } else {
-        // a portion: blocks of kPrefillQ queries, each as  scores = q k^T per head (fp32);  mixing of the heads;  masked softmax;  o = P v
-        for (int t0 = 0; t0 < T; t0 += kPrefillQ) {
-          const int Tq = std::min(kPrefillQ, T - t0), qpos0 = pos0 + t0;
+        // a portion: blocks of queries, each as  scores = q k^T per head (fp32);  mixing of the heads and masked softmax;  o = P v
+        const int block_q = sp.att_talk ? S->talk_q : kPrefillQ;
+        for (int t0 = 0; t0 < T; t0 += block_q) {
+          const int Tq = std::min(block_q, T - t0), qpos0 = pos0 + t0;
           const int first = mask_first(sp.att_mask, sp.att_window, qpos0), nk = std::min(keep, first), Lk = nk + qpos0 + Tq - first;
           launch_next(pack_ring_kv<float>, Lk, 256, 0, st)(kc, vc, S->kf, S->vf, first, Lk, ring, G, D, V, nk, keep);
           S->launches++;
           MK("att.pack");
           GemmP Sc = gp(S->b2 + (size_t)t0 * HD, HD, S->kf, D, S->sc, Lk, Tq, Lk, D);
           Sc.sA = D; Sc.sW = (long long)Lk * D; Sc.z_wdiv = rep; Sc.sC = (long long)Tq * Lk; Sc.alpha = sp.att_scale;
+          Sc.band = BAND_COLS; Sc.band_first = first - nk; Sc.band_pos = qpos0; Sc.band_mask = sp.att_mask; Sc.band_window = sp.att_window; Sc.band_keep = nk > 0;
           linear(S, false, HEPI_STORE, Sc, H, st);
           MK("att.scores");
-          float* pr = S->sc;
           if (sp.att_talk) {
-            const long long n = (long long)Tq * Lk;
-            launch_next(mix_heads, (unsigned)((n + 127) / 128), 128, (size_t)(H * H + H * 128) * 4, st)(S->sc, S->sc2, L.talk, H, n);
-            S->launches++;
-            pr = S->sc2;
+            const int hr = H <= 16 ? 16 : H <= 32 ? 32 : 0, nt = hr ? 512 : 128;
+            const size_t base = ((size_t)(H * (hr ? hr : H) + 3) / 4 * 4 + (hr ? 0 : (size_t)H * nt)) * 4, all = base + (size_t)H * Lk * 4;
+            const int staged = all <= (size_t)200 * 1024;
+            auto* kernel = hr == 16 ? mix_softmax<16> : hr == 32 ? mix_softmax<32> : mix_softmax<0>;
+            launch_next(kernel, (unsigned)Tq, (unsigned)nt, staged ? all : base, st)(S->sc, L.talk, H, Tq, Lk, first, qpos0, sp.att_mask, sp.att_window, nk, sm, staged);
+          } else {
+            launch_next(softmax_band, dim3((unsigned)Tq, (unsigned)H), 128, 0, st)(S->sc, Tq, Lk, first, qpos0, sp.att_mask, sp.att_window, nk, sm);
           }
-          launch_next(softmax_band, dim3((unsigned)Tq, (unsigned)H), 128, 0, st)(pr, Tq, Lk, first, qpos0, sp.att_mask, sp.att_window, nk, sm);
           S->launches++;
           MK("att.softmax");
-          GemmP Ov = gp(pr, Lk, S->vf, Lk, S->b3 + (size_t)t0 * ldo, ldo, Tq, V, Lk);
+          GemmP Ov = gp(S->sc, Lk, S->vf, Lk, S->b3 + (size_t)t0 * ldo, ldo, Tq, V, Lk);
           Ov.sA = (long long)Tq * Lk; Ov.sW = (long long)V * Lk; Ov.z_wdiv = rep; Ov.sC = V; Ov.alpha = lscale;
+          Ov.band = BAND_DEPTH; Ov.band_first = Sc.band_first; Ov.band_pos = qpos0; Ov.band_mask = sp.att_mask; Ov.band_window = sp.att_window; Ov.band_keep = Sc.band_keep;
           linear(S, false, HEPI_STORE, Ov, H, st);
           MK("att.pv");
         }

@@ -355,6 +355,12 @@ __global__ void __launch_bounds__(256, 2) gemm_split(const GemmP P) {
   }
   __syncthreads();
   const int n0 = blockIdx.x * BN;
+  int k_lo = 0, k_hi = P.K;
+  if (P.band) {
+    const int i0 = P.band_pos + row0, lo = P.band_keep ? 0 : max(0, mask_first(P.band_mask, P.band_window, i0) - P.band_first), hi = i0 + nrows - P.band_first;
+    if (P.band == BAND_DEPTH) { k_lo = lo / BK * BK; k_hi = min(P.K, hi); }
+    else if (n0 >= hi || n0 + BN <= lo) return;
+  }
   const float* __restrict__ A = P.A + aoff;
   // staging: thread -> 16 consecutive k of an activation row, 8 of a weight row
   const int lr = tid >> 1, lk = (tid & 1) * 16, ar = rowsA[lr];
@@ -413,12 +419,12 @@ __global__ void __launch_bounds__(256, 2) gemm_split(const GemmP P) {
     for (int j = 0; j < 4; j++)
 #pragma unroll
       for (int q = 0; q < 4; q++) acc[i][j][q] = 0.f;
-  const int nk = (P.K + BK - 1) / BK;
-  fetch(0);
+  const int nk = (k_hi - k_lo + BK - 1) / BK;
+  fetch(k_lo);
   put(0);
   __syncthreads();
   for (int kt = 0; kt < nk; kt++) {
-    if (kt + 1 < nk) fetch((kt + 1) * BK);
+    if (kt + 1 < nk) fetch(k_lo + (kt + 1) * BK);
     const uint32_t sa = sm0 + (uint32_t)((kt & 1) * kSplitStage) * 2, sw = sa + 3 * BM * PITCH * 2;
     const uint32_t aaddr = sa + (uint32_t)((wm * 32 + (lane & 7) + ((lane >> 3) & 1) * 8) * PITCH + (lane >> 4) * 8) * 2;
     const uint32_t waddr = sw + (uint32_t)((wn * 32 + (lane & 7) + (lane >> 4) * 8) * PITCH + ((lane >> 3) & 1) * 8) * 2;
