@@ -9,12 +9,17 @@
 //                     scaled, into the residual, or write its rows into a ring cache
 //   gemm_tiled        C = A W^T for T > 4 rows (fp32 activations, fp32 or bf16 weights, fp32 accumulate) with fused
 //                     epilogues (residual add, clamped GLU, GELU x per-token embedding) and row gather / scatter / expert tiles
-//   gemm_mma          the same interface on the tensor cores for bf16 weights (activations rounded to bf16 as they are staged)
+//   gemm_tc5          the same for bf16 weights that TMA can address, on the 5th-generation tensor cores (dsk_tc5.cuh)
+//   gemm_mma          the same for the other bf16 weights on mma.sync (activations rounded to bf16 as they are staged)
+//   gemm_split        the same for fp32 weights, operands as three bf16 parts (dsk_pattn.cuh);  gemm_tiled keeps routed products of few rows
+//   gemm_narrow       up to 96 columns over more than 32 rows
 //   gemv_rows         the same interface for T <= 4 rows: one warp per weight row, 16-byte loads
 //   gemv_one          the same for one row (a decoded token): eight 16-byte weight loads in flight per lane
 //   causal_conv_silu  depthwise causal convolution over the chunk continuing from the carried (taps - 1) inputs, + SiLU
 //   ssd_scan          the state-space recurrence S <- exp(-exp(A_log) dt) S + dt B x^T, y = S^T C + D x, gated by silu(z)
+//   ssd_gram, lin_scan, ssd_gate   the same recurrence over a portion in blocks of 16 tokens (lin_scan: dsk_linattn.cuh)
 //   decode_attn       softmax attention of decode-sized steps over cached keys and values, or cached latents with absorbed key up-projection
+//   pattn             softmax attention of portions in one kernel (dsk_pattn.cuh)
 //   layer_norm        (x - mean) / sqrt(var + eps) * w, stored or added into the residual
 //   qk_norm_rope      RMS norm over a whole query / key projection, partial interleaved rotary positions from a frequency table,
 //                     keys and values written into their ring caches
@@ -37,7 +42,7 @@
 // Numerics: the residual stream, norms, router, softmax, recurrent state, decays, step sizes and gates are fp32 in every mode;
 // DSK_BF16 models keep their matrices in bfloat16 and accumulate in fp32: decode-sized products multiply them with the fp32
 // activations, larger ones round the activations to bfloat16 on their way into the tensor cores.  DSK_F32 models are fp32
-// throughout (plain FMA, no reduced-precision matrix mode).
+// throughout (plain FMA, or tensor-core products of operands in three bf16 parts, whose error is no larger).
 #pragma once
 
 #include <cuda_bf16.h>
@@ -234,7 +239,7 @@ __global__ void __launch_bounds__(256) group_rmsnorm(const float* __restrict__ i
     return;
   }
   // a CTA per group, everything it reads in flight ahead of the sum (a decoded token's 4 groups one after the other, each with two waits for
-  // memory, took 12 to 20 us; side by side 5)
+  // memory, took 12 to 20 us; side by side 4)
   const int c0 = (int)blockIdx.y * gs;
   constexpr int NV = 4;
   float v[NV], wt[NV], old[NV], ss = 0.f;
