@@ -2671,7 +2671,7 @@ __global__ void __launch_bounds__(kMegaThreads, 1) decode_kernel(const Program* 
       for (int i = tid * 32; i < st.n; i += kConsumers * 32) asm volatile("prefetch.global.L1 [%0];" ::"l"(st.norm_w + i));
     }
     // the stage that writes this token's keys and values runs ahead of the attention stage: while it waits, the older rows of the heads this
-    // CTA will attend to come into L2 (up to kKvPrefetch positions; beyond that they are a stream of their own; two V2 layers behind 145 positions:
+    // CTA will attend to come into L2 (up to kKvPrefetch positions; beyond that they are a stream of their own; three V2 layers behind 144 positions:
     // attention stage 17 -> 14.5 us, token 474 -> 469 us)
     if (st.kind == ST_GEMV && st.epi == EPI_KVB && (int)blockIdx.x < P.n_heads && P.ctrl->kv_len <= kKvPrefetch) {
       const int len = P.ctrl->kv_len, kl = (P.hd * 2 + 127) / 128, vl = (P.vh * 2 + 127) / 128;
