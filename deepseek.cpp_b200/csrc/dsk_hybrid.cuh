@@ -320,7 +320,8 @@ struct GemmP {
   __nv_bfloat16* C16;
   // gemm_split only: scores of queries at positions band_pos + row against keys at positions band_first + column (BAND_COLS: tiles that no query of
   // theirs sees are left out) and the product of such rows with the values (BAND_DEPTH: the depth that a row tile sees; the rows hold 0
-  // elsewhere).  band_keep: the first columns are kept first positions, which all queries see
+  // elsewhere).  band_keep: the first band_keep columns are kept first positions, which all queries behind them see (whether they lie ahead of
+  // the step's range or are its start)
   int band, band_first, band_pos, band_mask, band_window, band_keep;
 };
 enum { BAND_NONE, BAND_COLS, BAND_DEPTH };

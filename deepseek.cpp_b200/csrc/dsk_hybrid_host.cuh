@@ -2088,7 +2088,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
           MK("att.pack");
           GemmP Sc = gp(S->b2 + (size_t)t0 * HD, HD, S->kf, D, S->sc, Lk, Tq, Lk, D);
           Sc.sA = D; Sc.sW = (long long)Lk * D; Sc.z_wdiv = rep; Sc.sC = (long long)Tq * Lk; Sc.alpha = sp.att_scale;
-          Sc.band = BAND_COLS; Sc.band_first = first - nk; Sc.band_pos = qpos0; Sc.band_mask = sp.att_mask; Sc.band_window = sp.att_window; Sc.band_keep = nk > 0;
+          Sc.band = BAND_COLS; Sc.band_first = first - nk; Sc.band_pos = qpos0; Sc.band_mask = sp.att_mask; Sc.band_window = sp.att_window; Sc.band_keep = keep;
           linear(S, false, HEPI_STORE, Sc, H, st);
           MK("att.scores");
           if (sp.att_talk) {

@@ -357,9 +357,9 @@ __global__ void __launch_bounds__(256, 2) gemm_split(const GemmP P) {
   const int n0 = blockIdx.x * BN;
   int k_lo = 0, k_hi = P.K;
   if (P.band) {
-    const int i0 = P.band_pos + row0, lo = P.band_keep ? 0 : max(0, mask_first(P.band_mask, P.band_window, i0) - P.band_first), hi = i0 + nrows - P.band_first;
-    if (P.band == BAND_DEPTH) { k_lo = lo / BK * BK; k_hi = min(P.K, hi); }
-    else if (n0 >= hi || n0 + BN <= lo) return;
+    const int i0 = P.band_pos + row0, lo = max(0, mask_first(P.band_mask, P.band_window, i0) - P.band_first), hi = i0 + nrows - P.band_first;
+    if (P.band == BAND_DEPTH) { k_lo = P.band_keep ? 0 : lo / BK * BK; k_hi = min(P.K, hi); }
+    else if (n0 >= hi || (n0 + BN <= lo && n0 >= P.band_keep)) return;
   }
   const float* __restrict__ A = P.A + aoff;
   // staging: thread -> 16 consecutive k of an activation row, 8 of a weight row

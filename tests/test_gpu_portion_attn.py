@@ -3,6 +3,8 @@ or 128), against the float64 statement: steps that continue a sequence inside a 
 import pytest
 
 from test_gpu_netusun import F32_TOL, close_bf16, in_portions, mk, no, rel, tokens_for  # noqa: F401
+from test_gpu_sakusun import mk as mk_sakusun  # noqa: F401
+from test_gpu_sakusun import so  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -28,3 +30,15 @@ def test_latents(mk, no, heads, dim, rot_dim, vdim):  # noqa: F811
         for sizes in ([128, 72], [33, 95, 65]):
             got = in_portions(m, toks, sizes)
             assert rel(got, exp) < F32_TOL if quant == "fp32" else close_bf16(got, exp, noise)
+
+
+@pytest.mark.parametrize("size,keep", [(20, 3), (70, 40), (1, 1), (20, 0)])
+def test_kept_positions_of_deep_heads(mk_sakusun, so, size, keep):  # noqa: F811
+    """Heads too deep for the one kernel (335 is the deepest): score and value products that leave out what a block of queries does not see.  Kept
+    first positions stay visible to queries whose window has left them behind, also where the step's range starts with them."""
+    cfg = so.model_config([so.att(heads=2, kv_heads=1, dim=352, vdim=20, size=size, keep_first=keep, scale=0.05, ff=None)], width=48, vocab=97)
+    m, W = mk_sakusun(cfg, seed=size, chunk=300)
+    toks = tokens_for(cfg, 360, 8)
+    exp = so.run(cfg, W, toks)[0]
+    for sizes in ([300, 60], [33, 40, 287]):
+        assert rel(in_portions(m, toks, sizes), exp) < F32_TOL
