@@ -88,7 +88,7 @@ __device__ __forceinline__ void mma_bf16_first(float (&c)[4], const uint32_t (&a
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
                : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "f"(0.f));
 }
-// two fp32 values as PARTS pairs of bf16, for finite values
+// two fp32 values as PARTS pairs of bf16, for finite values (see plain_dot for the others)
 template <int PARTS>
 __device__ __forceinline__ void split_pair(float x, float y, uint32_t (&o)[PARTS]) {
 #pragma unroll
@@ -323,6 +323,15 @@ __global__ void __launch_bounds__(256, 1) pattn(const PattnP P) {
 // bound by the fp32 pipe: a step in fp32 at width 1024 went from 1.85 to 1.22 ms (600 tokens), from 0.95 to 0.67 (64 tokens) and from 0.89 to 0.64
 // (5 tokens), a 1500-token prompt with mixed heads from 2.98 to 2.67 ms; the error against 64 bits of the first from 1.0e-6 to 5e-7.
 // ---------------------------------------------------------------------------------------------------------------------
+// The same sum as a chain of FMAs over the numbers themselves, for a result that is not finite: an infinite operand has no three parts (what is left
+// of it is inf - inf), nor has a finite one that rounds to an infinity in bf16 (from 2^128 - 2^119).  Such operands make every result that they enter
+// NaN, so that looking at the results is enough.  weights: A holds softmax weights, 0 for keys out of sight, which do not enter.
+__device__ __noinline__ float plain_dot(const float* a, const float* w, int k_lo, int k_hi, bool weights) {
+  float s = 0.f;
+  for (int k = k_lo; k < k_hi && !isnan(s); k++)
+    if (!weights || a[k] != 0.f) s = fmaf(a[k], w[k], s);
+  return s;
+}
 constexpr int kSplitPitch = 40;                                      // bf16 per staged row: 32 + 8
 constexpr int kSplitStage = 3 * (128 + 64) * kSplitPitch;            // bf16 of one stage: A parts, then W parts
 constexpr int kSplitSmem = 2 * kSplitStage * 2;
@@ -451,7 +460,7 @@ __global__ void __launch_bounds__(256, 2) gemm_split(const GemmP P) {
   for (int mi = 0; mi < 2; mi++)
 #pragma unroll
     for (int half = 0; half < 2; half++) {
-      const int cr = rowsC[wm * 32 + mi * 16 + (lane >> 2) + half * 8];
+      const int r = wm * 32 + mi * 16 + (lane >> 2) + half * 8, cr = rowsC[r];
       if (cr < 0) continue;
       float* crow = P.C + coff + (size_t)cr * P.ldc;
 #pragma unroll
@@ -460,7 +469,11 @@ __global__ void __launch_bounds__(256, 2) gemm_split(const GemmP P) {
         for (int q = 0; q < 2; q++) {
           const int g = wn * 4 + ni;   // granule of 8 staged rows
           const int n = DUAL ? n0 + (g >> 1) * 8 + (lane & 3) * 2 + q : n0 + g * 8 + (lane & 3) * 2 + q;
-          if (n < P.N) gemm_epilogue<float, EPI>(P, crow, cr, n, acc[mi][ni][half * 2 + q], DUAL ? acc[mi][ni + 1][half * 2 + q] : 0.f);
+          if (n >= P.N) continue;
+          float v = acc[mi][ni][half * 2 + q], v2 = DUAL ? acc[mi][ni + 1][half * 2 + q] : 0.f;
+          if (!isfinite(v)) v = plain_dot(A + (size_t)rowsA[r] * P.lda, reinterpret_cast<const float*>(P.W) + woff + (size_t)n * P.ldw, k_lo, k_hi, P.band == BAND_DEPTH);
+          if (DUAL && !isfinite(v2)) v2 = plain_dot(A + (size_t)rowsA[r] * P.lda, reinterpret_cast<const float*>(P.W2) + woff + (size_t)n * P.ldw, k_lo, k_hi, false);
+          gemm_epilogue<float, EPI>(P, crow, cr, n, v, v2);
         }
     }
 }
