@@ -29,7 +29,10 @@ __device__ __forceinline__ void split_bf16(float x, __nv_bfloat16 (&o)[PARTS]) {
 #pragma unroll
   for (int i = 0; i < PARTS; i++) {
     o[i] = __float2bfloat16_rn(x);
-    if (i + 1 < PARTS) x = isfinite(x) ? x - __bfloat162float(o[i]) : 0.f;   // exact: the rest has fewer bits (an infinity stays in the first part)
+    if (i + 1 < PARTS) {   // exact: the rest has fewer bits (an infinity stays in the first part; a finite number has finite parts)
+      if (isinf(__bfloat162float(o[i])) && isfinite(x)) o[i] = __ushort_as_bfloat16(x > 0.f ? 0x7F7F : 0xFF7F);
+      x = isfinite(x) ? x - __bfloat162float(o[i]) : 0.f;
+    }
   }
 }
 
@@ -130,8 +133,66 @@ __device__ __forceinline__ void mma_parts(float (*acc)[4], const uint32_t (&a)[P
   }
 }
 
+template <int PARTS>
+__device__ __forceinline__ float joined(const __nv_bfloat16* x, size_t part) {   // the number whose parts lie `part` apart
+  float v = __bfloat162float(x[(PARTS - 1) * part]);
+#pragma unroll
+  for (int i = PARTS - 2; i >= 0; i--) v += __bfloat162float(x[i * part]);
+  return v;
+}
+// Query t of head h again, by one warp and from its visible keys alone, into columns v0 .. v0 + VN * 8 - 1 of the output: for rows whose result is not
+// finite.  In the products of a tile a key out of sight has the weight 0, and 0 x Inf is NaN; an infinity times the parts of a number is NaN.
+template <int PARTS, int VN>
+__device__ __noinline__ void pattn_row(const PattnP& P, int t, int h, int v0) {
+  constexpr int CL = VN / 4;           // columns per lane
+  const int lane = threadIdx.x & 31, g = h / (P.H / P.G), pos = P.pos0 + t, lo = mask_first(P.mask, P.span, pos), last = P.nk + pos - P.first;
+  const float* q = P.q + (size_t)t * P.ldq + (size_t)h * P.D;
+  const size_t kpart = (size_t)P.G * P.Lk * P.Dp, vpart = (size_t)P.G * P.Lk * P.Vp;
+  float m = -1e30f, l = 0.f, acc[CL];
+#pragma unroll
+  for (int k = 0; k < CL; k++) acc[k] = 0.f;
+  for (int j0 = 0; j0 <= last && !isnan(l); j0 += 32) {
+    const int v = j0 + lane, p = v < P.nk ? v : P.first + v - P.nk;
+    const bool ok = v <= last && (p < P.mods.keep || p >= lo);
+    if (!__any_sync(0xffffffffu, ok)) continue;
+    float s = 0.f;
+    if (ok) {
+      const __nv_bfloat16* kr = P.kb + ((size_t)g * P.Lk + v) * P.Dp;
+      for (int d = 0; d < P.D; d++) s = fmaf(PARTS == 1 ? __bfloat162float(__float2bfloat16_rn(q[d])) : q[d], joined<PARTS>(kr + d, kpart), s);
+      s = mod_score(P.mods, s * P.scale, pos - p, h, P.H);
+    }
+    s = ok ? s : -1e30f;
+    const float m_new = fmaxf(m, warp_max(s)), c = expf(m - m_new), pr = ok ? expf(s - m_new) : 0.f;
+    l = l * c + warp_sum(pr);
+    m = m_new;
+#pragma unroll
+    for (int k = 0; k < CL; k++) acc[k] *= c;
+    for (int jj = 0; jj < 32; jj++) {
+      const float pj = __shfl_sync(0xffffffffu, pr, jj);
+      if (pj == 0.f) continue;
+      const __nv_bfloat16* vr = P.vb + ((size_t)g * P.Lk + j0 + jj) * P.Vp + v0 + lane;
+#pragma unroll
+      for (int k = 0; k < CL; k++) acc[k] = fmaf(pj, joined<PARTS>(vr + 32 * k, vpart), acc[k]);
+    }
+  }
+  float f = 1.f;
+  if (P.mods.sink) {
+    const float sk = P.mods.sink[h], m_new = fmaxf(m, sk);
+    f = expf(m - m_new);
+    l = l * f + expf(sk - m_new);
+  }
+  const float inv = f / l * P.alpha;
+#pragma unroll
+  for (int k = 0; k < CL; k++) {
+    const int c = v0 + lane + 32 * k;
+    if (c >= P.V) continue;
+    const float gt = P.gate ? sigmoid_f(P.gate[(size_t)t * P.ld_gate + (P.gate_head ? (size_t)h : (size_t)h * P.V + c)]) : 1.f;
+    P.out[(size_t)t * P.ld_out + (size_t)h * P.V + c] = acc[k] * inv * gt;
+  }
+}
+
 template <int PARTS, int VN, int NK>   // VN: 8-column groups of values in a CTA (blockIdx.z picks the columns)
-__global__ void __launch_bounds__(256, 1) pattn(const PattnP P) {
+__global__ void __launch_bounds__(256, 1) pattn(const __grid_constant__ PattnP P) {
   constexpr int KT = NK * 8;                                           // keys of a tile
   extern __shared__ __align__(16) unsigned char pa_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nthr = blockDim.x, BM = nthr / 2;
@@ -292,10 +353,21 @@ __global__ void __launch_bounds__(256, 1) pattn(const PattnP P) {
         });
     }
   }
+  uint32_t again = 0;   // rows of the warp whose result is not finite
+#pragma unroll
+  for (int r = 0; r < 2; r++) {
+    float any = l[r];   // (finite as long as everything is)
+#pragma unroll
+    for (int n = 0; n < VN; n++) any = fmaf(0.f, o[n][2 * r], fmaf(0.f, o[n][2 * r + 1], any));
+    uint32_t lanes = __ballot_sync(0xffffffffu, !isfinite(any));
+    lanes |= lanes >> 1; lanes |= lanes >> 2;
+#pragma unroll
+    for (int i = 0; i < 8; i++) again |= ((lanes >> (4 * i)) & 1u) << (i + 8 * r);
+  }
 #pragma unroll
   for (int r = 0; r < 2; r++) {
     const int t = row_lo + r * 8;
-    if (t >= P.T) continue;
+    if (t >= P.T || ((again >> ((lane >> 2) + 8 * r)) & 1u)) continue;
     float f = 1.f;
     if (P.mods.sink) {   // a key with a zero value vector
       const float sk = P.mods.sink[h], m_new = fmaxf(m[r], sk);
@@ -312,6 +384,10 @@ __global__ void __launch_bounds__(256, 1) pattn(const PattnP P) {
         const float gt = P.gate ? sigmoid_f(P.gate[(size_t)t * P.ld_gate + (P.gate_head ? (size_t)h : (size_t)h * P.V + c)]) : 1.f;
         P.out[(size_t)t * P.ld_out + (size_t)h * P.V + c] = o[n][r * 2 + i] * inv * gt;
       }
+  }
+  for (; again; again &= again - 1) {
+    const int t = q0 + warp * 16 + __ffs(again) - 1;
+    if (t < P.T) pattn_row<PARTS, VN>(P, t, h, v0);
   }
 }
 

@@ -3,7 +3,9 @@ of it.  Expected values: the float64 statements, over the tokens ahead where a t
 import numpy as np
 import pytest
 
-from test_gpu_netusun import F32_TOL, no, rel, tokens_for  # noqa: F401
+from test_gpu_hybrid import ho  # noqa: F401
+from test_gpu_hybrid import mk as mk_hybrid  # noqa: F401
+from test_gpu_netusun import F32_TOL, in_portions, mk, no, rel, tokens_for  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -45,3 +47,61 @@ def test_products(no, value, tokens):  # noqa: F811
     assert np.array_equal(got[~fin & ~near, 77], exp[~fin & ~near, 77], equal_nan=True)
     if np.any(fin & ~near):
         assert np.all(np.abs(got[fin & ~near, 77] - exp[fin & ~near, 77]) <= 1e-4 * np.abs(value))
+
+
+def poisoned(W, value, row):
+    W["embed"][row, 1] = value
+
+
+def ahead_of_the_poison(m, run, cfg, W, toks, at, sizes):
+    """Largest error of the tokens ahead of token `at` (the head is the embedding: the poisoned row's own logits are left out)."""
+    others = np.arange(cfg["vocab"]) != toks[at]
+    with np.errstate(invalid="ignore"):
+        got, exp = in_portions(m, toks, sizes)[:at, others], run(cfg, W, toks[:at])[0][:, others]
+    return rel(got, exp) if np.all(np.isfinite(got)) else np.inf
+
+
+def attention_model(mk, no, kind, value):  # noqa: F811
+    layer = {"grouped": lambda: no.att(heads=6, kv_heads=2, dim=12, vdim=10, size=25), "own_keys": lambda: no.att(heads=3, kv_heads=3, dim=16, vdim=70, size=None, conv=1),
+             "latent": lambda: no.lat(heads=3), "deep_latent": lambda: no.lat(heads=9, kv_rank=300, rot_dim=6)}[kind]
+    cfg = no.model_config([layer(), layer()], width=48, vocab=97)
+    return (cfg,) + mk(cfg, seed=4, chunk=64, edit=lambda W: poisoned(W, value, 90))
+
+
+def check_steps(mk, no, kind, value, steps):  # noqa: F811
+    """A step whose token `at` has keys and values that are not finite: its earlier tokens share CTAs and key tiles with it."""
+    cfg, m, W = attention_model(mk, no, kind, value)
+    for sizes in steps:
+        n = sum(sizes)
+        toks = tokens_for(cfg, n, 5)
+        toks[toks == 90] = 7
+        for at in (1, 6, 15, n - 1):
+            t = toks.copy()
+            t[at] = 90
+            m.reset()
+            assert ahead_of_the_poison(m, no.run, cfg, W, t, at, sizes) < F32_TOL
+
+
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+@pytest.mark.parametrize("kind", ["grouped", "own_keys", "latent", "deep_latent"])
+def test_attention_of_portions(mk, no, kind, value):  # noqa: F811
+    check_steps(mk, no, kind, value, [[40], [64], [33, 32]])
+
+
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+def test_latents_in_bf16(mk_hybrid, ho, value):  # noqa: F811
+    """Latent attention of bf16 models (one bf16 part an operand) against the same portion without the token."""
+    att = {"type": "latent_attention", "mixer": {"heads": 3, "dim": 12, "vdim": 20, "kv_rank": 40, "mask": {"size": 30}, "scale": 0.3}, "mlp": None}
+    cfg = ho.small_config(layers=[att] * 2, width=36, norm={"eps": 1e-5, "groups": 1})
+    m, W = mk_hybrid(cfg, seed=4, quant="bf16", chunk=64, edit=lambda W: poisoned(W, value, 50))
+    toks = tokens_for(cfg, 64, 5)
+    toks[toks == 50] = 7
+    base = m.forward_chunk(toks, 0, range(64))
+    for at in (1, 16, 33, 63):
+        t = toks.copy()
+        t[at] = 50
+        m.reset()
+        got = m.forward_chunk(t, 0, range(64))
+        others = np.arange(cfg["vocab"]) != 50
+        assert np.all(np.isfinite(got[:at, others])) and rel(got[:at, others], base[:at, others]) < 2e-2   # (rows that are summed again: weights not rounded)
+    m.reset()
