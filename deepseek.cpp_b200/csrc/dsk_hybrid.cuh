@@ -1454,7 +1454,11 @@ __global__ void __launch_bounds__(256) decode_attn(const DecodeAttn P) {
   if (D & 3) for (int jj = tid; jj < 32; jj += 256) for (int e = D; e < 4 * d4; e++) ks[jj * pd + e] = 0.f;   // (a depth that ends inside a group of four)
   const bool mine = live(w);
   const int i_w = pos0 + row_t(w), lo_w = mask_first(P.mask, P.span, i_w), h_w = g * rep + row_h(w);
-  float m = -1e30f, l = 0.f, acc[8][CV];
+  float m, l, acc[8][CV];
+  // A key that a row does not see has the weight 0 in that row's sums, and 0 x Inf is NaN: where a sum is not finite, the share is gone through again
+  // with weights of 0 left out (a product with a predicate per row, which the first walk is spared).
+  for (bool careful = false;; careful = true) {
+  m = -1e30f; l = 0.f;
 #pragma unroll
   for (int r = 0; r < 8; r++)
 #pragma unroll
@@ -1507,6 +1511,17 @@ __global__ void __launch_bounds__(256) decode_attn(const DecodeAttn P) {
 #pragma unroll
       for (int k = 0; k < CV; k++) acc[r][k] *= c;
     }
+    if (careful) {
+      for (int jj = 0; jj < 32; jj++)
+#pragma unroll
+        for (int k = 0; k < CV; k++) {
+          const int c = tid + 256 * k;
+          const float v = c < Dv ? vs[jj * pv + c] : 0.f;
+#pragma unroll
+          for (int r = 0; r < 8; r++) { const float pr = pt[jj * 8 + r]; if (pr != 0.f) acc[r][k] = fmaf(pr, v, acc[r][k]); }
+        }
+      continue;
+    }
 #pragma unroll 4
     for (int jj = 0; jj < 32; jj++) {
       const float4 p0 = *reinterpret_cast<const float4*>(pt + jj * 8), p1 = *reinterpret_cast<const float4*>(pt + jj * 8 + 4);
@@ -1518,6 +1533,14 @@ __global__ void __launch_bounds__(256) decode_attn(const DecodeAttn P) {
         acc[4][k] = fmaf(p1.x, v, acc[4][k]); acc[5][k] = fmaf(p1.y, v, acc[5][k]); acc[6][k] = fmaf(p1.z, v, acc[6][k]); acc[7][k] = fmaf(p1.w, v, acc[7][k]);
       }
     }
+  }
+  if (careful) break;
+  float any = 0.f;   // (stays 0 as long as every sum is finite)
+#pragma unroll
+  for (int r = 0; r < 8; r++)
+#pragma unroll
+    for (int k = 0; k < CV; k++) any = fmaf(0.f, acc[r][k], any);
+  if (!__syncthreads_or(any != 0.f)) break;
   }
   float c_end = 1.f;
   if (P.mods.sink && blockIdx.z == 0 && mine) {   // the sink joins the first share like a key with a zero value vector

@@ -89,6 +89,12 @@ def test_attention_of_portions(mk, no, kind, value):  # noqa: F811
 
 
 @pytest.mark.parametrize("value", [np.inf, np.nan])
+@pytest.mark.parametrize("kind", ["grouped", "own_keys", "latent", "deep_latent"])
+def test_attention_of_short_steps(mk, no, kind, value):  # noqa: F811
+    check_steps(mk, no, kind, value, [[2] * 20, [3] * 13, [5] * 8, [8] * 5, [13] * 3, [31, 9]])
+
+
+@pytest.mark.parametrize("value", [np.inf, np.nan])
 def test_latents_in_bf16(mk_hybrid, ho, value):  # noqa: F811
     """Latent attention of bf16 models (one bf16 part an operand) against the same portion without the token."""
     att = {"type": "latent_attention", "mixer": {"heads": 3, "dim": 12, "vdim": 20, "kv_rank": 40, "mask": {"size": 30}, "scale": 0.3}, "mlp": None}
