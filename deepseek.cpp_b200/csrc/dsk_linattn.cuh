@@ -520,8 +520,13 @@ __global__ void __launch_bounds__(320) lin_scan(const float* __restrict__ q, con
         s0 = fmaf(mm.x, Xw[i * CW + c], s0); s1 = fmaf(mm.y, Xw[(i + 1) * CW + c], s1);
         s0 = fmaf(mm.z, Xw[(i + 2) * CW + c], s0); s1 = fmaf(mm.w, Xw[(i + 3) * CW + c], s1);
       }
-      if (j < nt && cw + c < PB && p0 + cw + c < P) out[(size_t)(t0 + j) * ldo + (size_t)h * P + p0 + cw + c] = s0 + s1;
-      else if (nst && j < nt && cw + c < PB && p0 + cw + c == P) den[(size_t)(t0 + j) * H + h] = s0 + s1;
+      float y = s0 + s1;
+      if (!isfinite(y)) {   // the weights of later tokens are 0, and 0 x Inf is NaN: the tokens up to this one alone
+        y = br[kRecG + j] * Rw[C * CW + e];
+        for (int i = 0; i <= j; i++) y = fmaf(br[kRecM + j * C + i], Xw[i * CW + c], y);
+      }
+      if (j < nt && cw + c < PB && p0 + cw + c < P) out[(size_t)(t0 + j) * ldo + (size_t)h * P + p0 + cw + c] = y;
+      else if (nst && j < nt && cw + c < PB && p0 + cw + c == P) den[(size_t)(t0 + j) * H + h] = y;
     }
     __syncwarp();
     const float ge = br[kRecEnd];

@@ -111,3 +111,19 @@ def test_latents_in_bf16(mk_hybrid, ho, value):  # noqa: F811
         others = np.arange(cfg["vocab"]) != 50
         assert np.all(np.isfinite(got[:at, others])) and rel(got[:at, others], base[:at, others]) < 2e-2   # (rows that are summed again: weights not rounded)
     m.reset()
+
+
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+def test_recurrence_in_blocks(mk_hybrid, ho, value):  # noqa: F811
+    ssd = {"type": "mamba2", "mixer": {"heads": 4, "vdim": 12, "state": 33, "groups": 2, "conv": 3, "norm_groups": 1}, "mlp": None}
+    cfg = ho.small_config(layers=[ssd] * 2, width=36, norm={"eps": 1e-5, "groups": 1})
+    m, W = mk_hybrid(cfg, seed=4, chunk=64, edit=lambda W: poisoned(W, value, 50))
+    toks = tokens_for(cfg, 40, 5)
+    toks[toks == 50] = 7
+    for sizes in ([40], [17, 23], [5] * 8):
+        for at in (1, 9, 20, 39):
+            t = toks.copy()
+            t[at] = 50
+            m.reset()
+            assert ahead_of_the_poison(m, ho.run, cfg, W, t, at, sizes) < F32_TOL
+    m.reset()
