@@ -486,9 +486,12 @@ template <> struct WVec<__nv_bfloat16> {
 constexpr int kNarrowRows = 16;
 template <typename WT, int EPI>
 __global__ void __launch_bounds__(256) gemm_narrow(const GemmP P) {
-  __shared__ __align__(16) float As[8][16][kNarrowRows + 4], Ws[8][16][32 + 4];   // [warp][k][row], [warp][k][column]
-  float* red = &As[0][0][0];                                                      // [8 warps][16 rows][32 columns], over both at the end
-  static_assert(sizeof(As) + sizeof(Ws) >= 8 * 16 * 32 * 4, "the sums of 8 warps fit");
+  struct Slices { float a[8][16][kNarrowRows + 4], w[8][16][32 + 4]; };            // [warp][k][row], [warp][k][column]
+  __shared__ __align__(16) union { Slices s; float red[8 * kNarrowRows * 32]; } u;   // red: [8 warps][16 rows][32 columns], over the slices at the end
+  auto& As = u.s.a;
+  auto& Ws = u.s.w;
+  float* red = u.red;
+  static_assert(kNarrowRows == 16 && sizeof(Slices::a) % 16 == 0, "a lane's 4 rows, and weights on a 16-byte boundary");
   grid_enter();
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, row0 = blockIdx.x * kNarrowRows, n0 = blockIdx.y * 32;
   const WT* __restrict__ W = reinterpret_cast<const WT*>(P.W);
