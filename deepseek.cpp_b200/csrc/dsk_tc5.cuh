@@ -22,7 +22,7 @@ constexpr int kTcRows = 128, kTcDepth = 64, kTcThreads = 192, kTcMaxStages = 10;
 constexpr int kTcRing = 192 * 1024;                                  // operand ring
 constexpr int kTcTurn = 4 * 32 * 33 * 4;                             // epilogue: a 32 x 32 block per warp
 constexpr int kTcSmem = 1024 + kTcRing + kTcTurn + 256;              // (+ alignment, + barriers)
-constexpr int kTcWaitLimit = 1 << 24;                                // polls of a barrier before a wait gives up (seconds)
+constexpr long long kTcWaitCycles = 1ll << 32;                       // how long a wait polls a barrier before it gives up (two seconds)
 
 struct TcP {
   int bn, stages, n_mt, rows_per_expert;   // column tile, ring stages, row tiles (no tile list), weight rows between experts
@@ -32,13 +32,18 @@ struct TcP {
   int* err;                                // host-visible word: set when a wait gave up
 };
 
+__device__ __forceinline__ bool tc_poll(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+               : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
 __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, int* err) {
-  for (int i = 0; i < kTcWaitLimit; i++) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    if (ok) return true;
-  }
+  if (tc_poll(bar, parity)) return true;
+  const long long from = clock64();
+  do {
+    if (tc_poll(bar, parity)) return true;
+  } while (clock64() - from < kTcWaitCycles);
   *reinterpret_cast<volatile int*>(err) = 1;
   return false;
 }
@@ -83,12 +88,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc5(const GemmP P, const T
   const uint32_t base = (smem_u32(tc_raw) + 1023u) & ~1023u;
   unsigned char* gbase = tc_raw + (base - smem_u32(tc_raw));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t bars = base + kTcRing + kTcTurn;            // full[stages], empty[stages], done[2], drained[2], then the TMEM address
-  const uint32_t full0 = bars, empty0 = bars + 8 * kTcMaxStages, done0 = bars + 16 * kTcMaxStages, drained0 = done0 + 16;
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gbase + kTcRing + kTcTurn + 16 * kTcMaxStages + 32);
+  const uint32_t bars = base + kTcRing + kTcTurn;            // full[stages], empty[stages], done[2], drained[2], flushed, then the TMEM address
+  const uint32_t full0 = bars, empty0 = bars + 8 * kTcMaxStages, done0 = bars + 16 * kTcMaxStages, drained0 = done0 + 16, flushed0 = done0 + 32;
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gbase + kTcRing + kTcTurn + 16 * kTcMaxStages + 40);
   if (threadIdx.x == 0) {
     for (int s = 0; s < T.stages; s++) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
     for (int b = 0; b < 2; b++) { mbar_init(done0 + 8 * b, 1); mbar_init(drained0 + 8 * b, 4); }
+    mbar_init(flushed0, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) {
@@ -122,6 +128,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc5(const GemmP P, const T
           if (DUAL) tma_tile(b + (uint32_t)cols * kTcDepth * 2, &mapB2, kb * kTcDepth, rowB, bar);
         }
       }
+      // no copy of this CTA is under way when it leaves, also where a wait gave up (else the products have waited for all of them already)
+      for (int i = max(0, it - T.stages); i < it; i++) tc_wait(full0 + 8 * (i % T.stages), (i / T.stages) & 1, T.err);
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -146,6 +154,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc5(const GemmP P, const T
         }
         if (alive) tc_commit(done0 + 8 * buf);
       }
+      tc_commit(flushed0);                                   // nor a product, ahead of giving TMEM back
+      tc_wait(flushed0, 0, T.err);
     }
     __syncwarp();
   } else {

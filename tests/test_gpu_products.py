@@ -4,6 +4,8 @@ import numpy as np
 import pytest
 
 from test_gpu_netusun import close_bf16, mk, no, tokens_for  # noqa: F401
+from test_gpu_zetivik import mk as mk_zetivik  # noqa: F401
+from test_gpu_zetivik import zo  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -46,3 +48,25 @@ def test_unaligned_depth_and_short_steps(mk, no):  # noqa: F811
     assert close_bf16(m.forward_chunk(toks, 0, range(40)), exp, noise)
     rows = np.concatenate([m.forward_chunk(toks[p:p + 4], p, range(4)) for p in range(0, 40, 4)])
     assert close_bf16(rows, exp, noise)
+
+
+# More than three tiles of 128 x 256 per CTA (148 of them), so that both accumulators go round, the ring's indices run on over tiles and what a tile adds to is
+# fetched under the products of the one ahead.  1024 rows are 8 row tiles.  Stored: 57 column tiles; added: the same onto the stream; gated: tiles of
+# 128 columns, 57 of them; routed: some 18 row tiles by 29 column tiles
+@pytest.mark.parametrize("kind", ["stored", "gated", "routed"])
+def test_many_tiles_per_cta(mk, no, kind):  # noqa: F811
+    wide, att = 14344, dict(heads=2, dim=16, vdim=8, size=9)
+    if kind == "stored":
+        cfg = no.model_config([no.att(**att)], width=wide, vocab=131)
+    else:
+        cfg = no.model_config([no.att(mlp=no.dense(7208) if kind == "gated" else no.moe(experts=3, top=2, ff=3656, shared=None), **att)], width=104, vocab=131)
+    m, W = mk(cfg, seed=len(kind), quant="bf16", chunk=1024, context=1100)
+    toks = tokens_for(cfg, 1024, 7)
+    assert close_bf16(m.forward_chunk(toks, 0, range(1024)), no.run(cfg, W, toks)[0], no.rounding_noise(cfg, W, toks))
+
+
+def test_many_tiles_added(mk_zetivik, zo):  # noqa: F811
+    cfg = zo.model_config([zo.light(heads=3, dim=8, vdim=8, ff=16)], width=14344, vocab=131)
+    m, W = mk_zetivik(cfg, seed=5, quant="bf16", chunk=1024, context=1100)
+    toks = tokens_for(cfg, 1024, 7)
+    assert close_bf16(m.forward_chunk(toks, 0, range(1024)), zo.run(cfg, W, toks)[0], zo.rounding_noise(cfg, W, toks))
