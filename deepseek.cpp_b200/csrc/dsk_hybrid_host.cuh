@@ -180,6 +180,9 @@ struct State {
 };
 
 static constexpr int kPrefillQ = 256, kPrefillMin = 32;   // prefill attention: queries per block / smallest portion that takes the matrix path
+// Buffers of the attention of portions: a state takes them up to this size (blocks of kPrefillQ queries of the fused kernel, the smallest there are: up to
+// half as much again).  Heads x keys decide: 16 key heads of 64 + 64 entries take 25 KB a key.
+static constexpr size_t kPortionBytes = (size_t)4 << 30;
 static constexpr int kAttnSplitMax = 64, kAttnSplitTokens = 4;   // decode-sized chunks split a window over up to 64 CTAs
 
 static bool is_ssd(const dsk_layer_spec& s) { return s.mixer == DSK_MIX_SSD; }
@@ -1288,57 +1291,56 @@ static dsk_state* state_create(dsk_model* m) {
     if (L.sp.mixer == DSK_MIX_MLA) mxPart = std::max(mxPart, (size_t)kAttnSplitTokens * L.sp.att_heads * kAttnSplitMax * (L.sp.att_kv_rank + L.sp.att_rot_dim + 2));
   }
   rc |= salloc(S, (void**)&S->part, mxPart * 4);
-  if ((int)Tc >= kPrefillMin) {   // buffers of the matrix-product attention path, unless a window is too long for them
-    // latent attention up-projects keys and values of all heads (fp32, then packed in the matrix type); grouped-query
-    // attention packs its cached key / value heads in fp32 (kf / vf)
-    // (latent attention with a rotated key part packs in fp32: its scores are 32-bit products)
-    size_t keys = 0, hd = 0, hv = 0, heads = 0, pack_es = 0, bytes = 0;
-    bool latent = false;
-    // (layers that mix heads take 512 queries at a time, where their scores fit: a head's product with the values is then 8 tiles)
-    for (S->talk_q = any_talk ? 2 * kPrefillQ : kPrefillQ;; S->talk_q = kPrefillQ) {
+  if ((int)Tc >= kPrefillMin) {   // buffers of the attention of portions, counted for the layers that use them; without them portions run like short steps
+    const bool bf16 = c.quant == DSK_BF16;
+    auto visible = [&](const dsk_layer_spec& sp, int q) {   // keys that a block of q queries can see
+      return (size_t)std::min<long long>((long long)sp.att_window - 1, (long long)c.max_seq_len) + std::min<size_t>(Tc, q) + (sp.mixer == DSK_MIX_GQA ? sp.att_keep_first : 0);
+    };
+    // layers that run pattn: the visible keys and values split into bf16 parts, behind the up-projected fp32 rows of latent layers
+    size_t k16 = 0, v16 = 0, kup = 0, vup = 0, rows = 0;
+    auto fused_bytes = [&](int q) {
+      k16 = v16 = kup = vup = 0;
+      for (const HLayer& L : M->L) {
+        if (!takes_pattn(L.sp, bf16)) continue;
+        const PattnSize z = pattn_size(L.sp, bf16);
+        const size_t n = visible(L.sp, q);
+        k16 = std::max(k16, n * z.G * z.Dp * z.parts); v16 = std::max(v16, n * z.G * z.Vp * z.parts);
+        if (L.sp.mixer != DSK_MIX_GQA) { kup = std::max(kup, n * z.G * L.sp.att_dim); vup = std::max(vup, n * z.G * z.V); }
+      }
+      return 2 * (k16 + v16) + 4 * (kup + vup);
+    };
+    // the others, as matrix products between which the scores lie in memory: latent attention up-projects keys and values of all heads (fp32, then packed in
+    // the matrix type; with a rotated key part in fp32: its scores are 32-bit products), grouped-query attention packs its cached key / value heads in fp32
+    size_t keys = 0, hd = 0, hv = 0, heads = 0, pack_es = 0;
+    auto plain_bytes = [&](int q) {
       keys = 0;
       for (const HLayer& L : M->L) {
-        if (!has_attn(L.sp)) continue;
+        if (!has_attn(L.sp) || takes_pattn(L.sp, bf16)) continue;
         const size_t kh = L.sp.mixer == DSK_MIX_GQA ? L.sp.att_kv_heads : L.sp.att_heads;
-        latent |= L.sp.mixer == DSK_MIX_LATENT_SWA || L.sp.mixer == DSK_MIX_MLA;
         if (L.sp.mixer == DSK_MIX_LATENT_SWA) pack_es = std::max(pack_es, M->wsize);
         if (L.sp.mixer == DSK_MIX_MLA) pack_es = 4;
-        keys = std::max<size_t>(keys, (size_t)std::min<long long>((long long)L.sp.att_window - 1, (long long)c.max_seq_len) + std::min<size_t>(Tc, S->talk_q) +
-                                          (L.sp.mixer == DSK_MIX_GQA ? L.sp.att_keep_first : 0));
+        keys = std::max(keys, visible(L.sp, q));
         hd = std::max<size_t>(hd, kh * (L.sp.att_dim + (L.sp.mixer == DSK_MIX_MLA ? L.sp.att_rot_dim : 0))); hv = std::max<size_t>(hv, kh * L.sp.att_vdim);
         heads = std::max<size_t>(heads, L.sp.att_heads);
       }
-      bytes = keys * (hd + hv) * (4 + (latent ? pack_es : 0)) + heads * S->talk_q * keys * 4;
-      if (bytes <= ((size_t)4 << 30) || S->talk_q == kPrefillQ) break;
-    }
-    if (keys > 0 && bytes <= ((size_t)4 << 30)) {
-      // layers that run pattn: the visible keys of a whole step split into bf16 parts, behind the up-projected fp32 rows of latent layers (blocks of
-      // kPrefillQ queries where a step's keys would take over 4 GB)
-      const bool bf16 = c.quant == DSK_BF16;
-      size_t k16 = 0, v16 = 0, kup = 0, vup = 0, rows = keys;
-      bool old = false;
-      for (S->pattn_q = (int)Tc;; S->pattn_q = kPrefillQ) {
-        k16 = v16 = kup = vup = 0; rows = keys; old = false;
-        for (const HLayer& L : M->L) {
-          if (!has_attn(L.sp)) continue;
-          if (!takes_pattn(L.sp, bf16)) { old = true; continue; }
-          const PattnSize z = pattn_size(L.sp, bf16);
-          const size_t n = (size_t)std::min<long long>((long long)L.sp.att_window - 1, (long long)c.max_seq_len) + std::min<size_t>(Tc, S->pattn_q) +
-                           (L.sp.mixer == DSK_MIX_GQA ? L.sp.att_keep_first : 0);
-          k16 = std::max(k16, n * z.G * z.Dp * z.parts); v16 = std::max(v16, n * z.G * z.Vp * z.parts);
-          if (L.sp.mixer != DSK_MIX_GQA) { kup = std::max(kup, n * z.G * L.sp.att_dim); vup = std::max(vup, n * z.G * z.V); }
-          rows = std::max(rows, n);
-        }
-        if (2 * (k16 + v16) + 4 * (kup + vup) <= ((size_t)4 << 30) || S->pattn_q <= kPrefillQ) break;
-      }
+      return keys * (hd + hv) * (4 + pack_es) + heads * q * keys * 4;
+    };
+    // a whole step at a time where its keys take up to 4 GB, else blocks of kPrefillQ queries; layers that mix heads 512 queries at a time where
+    // their scores fit (a head's product with the values is then 8 tiles)
+    S->pattn_q = (int)Tc;
+    size_t fused = fused_bytes(S->pattn_q);
+    if (fused > kPortionBytes && S->pattn_q > kPrefillQ) fused = fused_bytes(S->pattn_q = kPrefillQ);
+    S->talk_q = any_talk ? 2 * kPrefillQ : kPrefillQ;
+    size_t plain = plain_bytes(S->talk_q);
+    if (plain > kPortionBytes && any_talk) plain = plain_bytes(S->talk_q = kPrefillQ);
+    for (const HLayer& L : M->L) if (has_attn(L.sp)) rows = std::max(rows, visible(L.sp, takes_pattn(L.sp, bf16) ? S->pattn_q : S->talk_q));
+    if (rows > 0 && fused <= kPortionBytes + kPortionBytes / 2 && plain <= kPortionBytes) {
       S->prefill_keys = (int)rows;
       if (k16) rc |= salloc(S, (void**)&S->k16, k16 * 2) | salloc(S, (void**)&S->v16, v16 * 2);
-      rc |= salloc(S, (void**)&S->kf, std::max(kup, old ? keys * hd : 0) * 4) | salloc(S, (void**)&S->vf, std::max(vup, old ? keys * hv : 0) * 4);
+      rc |= salloc(S, (void**)&S->kf, std::max(kup, keys * hd) * 4) | salloc(S, (void**)&S->vf, std::max(vup, keys * hv) * 4);
       rc |= salloc(S, (void**)&S->d_rows, rows * 4);
-      if (old) {
-        if (latent) rc |= salloc(S, &S->kb, keys * hd * pack_es) | salloc(S, &S->vt, keys * hv * pack_es);
-        rc |= salloc(S, (void**)&S->sc, heads * S->talk_q * keys * 4);
-      }
+      if (pack_es) rc |= salloc(S, &S->kb, keys * hd * pack_es) | salloc(S, &S->vt, keys * hv * pack_es);
+      if (keys) rc |= salloc(S, (void**)&S->sc, heads * S->talk_q * keys * 4);
     }
   }
   rc |= salloc(S, (void**)&S->x, Tc * c.dim * 4) | salloc(S, (void**)&S->h, Tc * c.dim * 4);

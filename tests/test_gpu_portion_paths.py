@@ -5,6 +5,8 @@ import pytest
 
 from test_gpu_hybrid import F32_TOL, ho, mk, rel, tokens_for  # noqa: F401
 from test_gpu_netusun import in_portions
+from test_gpu_netusun import mk as mk_netusun  # noqa: F401
+from test_gpu_netusun import no  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -30,3 +32,15 @@ def test_narrow_products(mk, ho, experts, side, width, tokens):  # noqa: F811
     m, W = mk(cfg, seed=experts, chunk=128)
     toks = tokens_for(cfg, tokens, 12)
     assert rel(m.forward_chunk(toks, 0, range(tokens)), ho.run(cfg, W, toks)[0]) < F32_TOL
+
+
+def test_large_windows_take_the_fused_kernel(mk_netusun, no, monkeypatch, capfd):  # noqa: F811
+    """What switches the attention of portions on is the memory of the layers that use it: 64 heads x 256 queries x 70000 keys are 4.6 GB of scores, which
+    only the products between which scores lie in memory would have."""
+    monkeypatch.setenv("DSK_HY_TIMELINE", "1")
+    cfg = no.model_config([no.att(heads=64, kv_heads=1, dim=8, vdim=8, size=None)], width=40, vocab=97)
+    m, W = mk_netusun(cfg, seed=3, chunk=64, context=70000)
+    toks = tokens_for(cfg, 100, 9)
+    got = in_portions(m, toks, [60, 40])
+    assert rel(got, no.run(cfg, W, toks)[0]) < F32_TOL
+    assert capfd.readouterr().err.count("att.fused") == 2
