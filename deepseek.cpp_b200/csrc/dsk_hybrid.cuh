@@ -323,6 +323,7 @@ struct GemmP {
   // elsewhere).  band_keep: the first band_keep columns are kept first positions, which all queries behind them see (whether they lie ahead of
   // the step's range or are its start)
   int band, band_first, band_pos, band_mask, band_window, band_keep;
+  int w_made;   // W is written by kernels of the step (packed keys and values), not a matrix of the model: not to be read ahead of grid_wait
 };
 enum { BAND_NONE, BAND_COLS, BAND_DEPTH };
 
@@ -959,8 +960,9 @@ __global__ void __launch_bounds__(256) gemv_one(const GemmP P) {
   const WT *W, *W2 = nullptr;
   const float* A = nullptr;
   float* C = nullptr;
-  // the first weights of a product whose matrix is known are asked for while the kernel ahead still runs; a routed one has to wait for its router
-  bool ready = P.z_expert != nullptr;
+  // the first weights of a product whose matrix is known are asked for while the kernel ahead still runs; a routed one has to wait for its router,
+  // and one by keys or values for the kernel that makes them
+  bool ready = P.z_expert != nullptr || P.w_made;
   if (ready) grid_enter();
   const bool shared = P.z_expert && P.n_shared > 0 && z >= P.z_shared;
   if (shared) {

@@ -2089,6 +2089,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
           S->launches++;
           MK("att.pack");
           GemmP Sc = gp(S->b2 + (size_t)t0 * HD, HD, S->kf, D, S->sc, Lk, Tq, Lk, D);
+          Sc.w_made = 1;
           Sc.sA = D; Sc.sW = (long long)Lk * D; Sc.z_wdiv = rep; Sc.sC = (long long)Tq * Lk; Sc.alpha = sp.att_scale;
           Sc.band = BAND_COLS; Sc.band_first = first - nk; Sc.band_pos = qpos0; Sc.band_mask = sp.att_mask; Sc.band_window = sp.att_window; Sc.band_keep = keep;
           linear(S, false, HEPI_STORE, Sc, H, st);
@@ -2105,6 +2106,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
           S->launches++;
           MK("att.softmax");
           GemmP Ov = gp(S->sc, Lk, S->vf, Lk, S->b3 + (size_t)t0 * ldo, ldo, Tq, V, Lk);
+          Ov.w_made = 1;
           Ov.sA = (long long)Tq * Lk; Ov.sW = (long long)V * Lk; Ov.z_wdiv = rep; Ov.sC = V; Ov.alpha = lscale;
           Ov.band = BAND_DEPTH; Ov.band_first = Sc.band_first; Ov.band_pos = qpos0; Ov.band_mask = sp.att_mask; Ov.band_window = sp.att_window; Ov.band_keep = Sc.band_keep;
           linear(S, false, HEPI_STORE, Ov, H, st);
@@ -2194,12 +2196,14 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
           launch_next(pack_mla_kv, Lk, 256, 0, st)(S->kf, S->vf, cache, S->d_rows, (float*)S->kb, (float*)S->vt, Lk, H, D, Rd, R, V);
           MK("att.pack");
           GemmP Sc = gp(S->b0 + (size_t)t0 * H * DK, H * DK, S->kb, DK, S->sc, Lk, Tq, Lk, DK);
+          Sc.w_made = 1;
           Sc.sA = DK; Sc.sW = (long long)Lk * DK; Sc.sC = (long long)Tq * Lk; Sc.alpha = sp.att_scale;
           linear(S, false, HEPI_STORE, Sc, H, st);
           MK("att.scores");
           launch_next(softmax_band, dim3((unsigned)Tq, (unsigned)H), 128, 0, st)(S->sc, Tq, Lk, first, qpos0, sp.att_mask, sp.att_window, 0, sm);
           MK("att.softmax");
           GemmP Ov = gp(S->sc, Lk, S->vt, Lk, S->b3 + (size_t)t0 * H * V, H * V, Tq, V, Lk);
+          Ov.w_made = 1;
           Ov.sA = (long long)Tq * Lk; Ov.sW = (long long)V * Lk; Ov.sC = V;
           linear(S, false, HEPI_STORE, Ov, H, st);
           MK("att.pv");
@@ -2365,12 +2369,14 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
           if (bf) launch_next(pack_keys_values<__nv_bfloat16>, Lk, 256, 0, st)(S->kf, S->vf, (__nv_bfloat16*)S->kb, (__nv_bfloat16*)S->vt, Lk, H, D, V);
           else launch_next(pack_keys_values<float>, Lk, 256, 0, st)(S->kf, S->vf, (float*)S->kb, (float*)S->vt, Lk, H, D, V);
           GemmP Sc = gp(S->b0 + (size_t)t0 * H * D, H * D, S->kb, D, S->sc, Lk, Tq, Lk, D);
+          Sc.w_made = 1;
           Sc.sA = D; Sc.sW = (long long)Lk * D; Sc.sC = (long long)Tq * Lk; Sc.alpha = sp.att_scale;
           MK("att.pack");
           linear(S, bf, HEPI_STORE, Sc, H, st);
           MK("att.scores");
           launch_next(softmax_band, dim3((unsigned)Tq, (unsigned)H), 128, 0, st)(S->sc, Tq, Lk, first, qpos0, sp.att_mask, sp.att_window, 0, ScoreMods{});
           GemmP Ov = gp(S->sc, Lk, S->vt, Lk, S->b3 + (size_t)t0 * H * V, H * V, Tq, V, Lk);
+          Ov.w_made = 1;
           Ov.sA = (long long)Tq * Lk; Ov.sW = (long long)V * Lk; Ov.sC = V;
           MK("att.softmax");
           linear(S, bf, HEPI_STORE, Ov, H, st);

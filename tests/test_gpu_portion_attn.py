@@ -42,3 +42,11 @@ def test_kept_positions_of_deep_heads(mk_sakusun, so, size, keep):  # noqa: F811
     exp = so.run(cfg, W, toks)[0]
     for sizes in ([300, 60], [33, 40, 287]):
         assert rel(in_portions(m, toks, sizes), exp) < F32_TOL
+
+
+def test_last_block_of_one_query(mk_sakusun, so):  # noqa: F811
+    """Blocks of 256 queries whose last one is a single row: its products read keys and values that were packed a launch ahead."""
+    cfg = so.model_config([so.att(heads=2, kv_heads=1, dim=352, vdim=20, size=150, keep_first=2, scale=0.05, ff=None)], width=48, vocab=97)
+    m, W = mk_sakusun(cfg, seed=2, chunk=300)
+    toks = tokens_for(cfg, 290, 8)
+    assert rel(in_portions(m, toks, [257, 33]), so.run(cfg, W, toks)[0]) < F32_TOL
