@@ -785,11 +785,12 @@ static int alloc_host_side(dsk_state* s) {
   return 0;
 }
 // device -> pageable host memory through two pinned pieces, one landing while the other is copied on (the driver's own staging of such a
-// copy takes them one after the other: 410 KB of logits behind a token cost 12 us more, 2.4 MB behind a portion 150 us).  Returns when the bytes are there; pinned destinations are written directly.
+// copy takes them one after the other: 410 KB of logits behind a token cost 12 us more, 2.4 MB behind a portion 150 us).  Returns when the bytes are there; destinations
+// that the driver knows (pinned, managed) are written directly.
 static int copy_to_host(dsk_state* s, void* dst, const void* src, size_t bytes) {
   cudaPointerAttributes at{};
-  const bool pinned = cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type == cudaMemoryTypeHost;
-  if (pinned || bytes <= ((size_t)16 << 10)) {
+  const bool pageable = cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
+  if (!pageable || bytes <= ((size_t)16 << 10)) {   // (a device address is the copy's to refuse)
     CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     return 0;
