@@ -775,12 +775,12 @@ extern "C" double dsk_model_active_bytes_per_token(const dsk_model* m) {
 // ---------------------------------------------------------------------------------------------------
 static int build_program(dsk_model* m, dsk_state* s);
 
-// the control words and the pieces of copy_to_host in one pinned allocation
+// the pieces of copy_to_host, the control words and `more` zeroed bytes behind them in one pinned allocation
 static constexpr size_t kBouncePiece = (size_t)256 << 10;
-static int alloc_host_side(dsk_state* s) {
-  CK(cudaMallocHost((void**)&s->bounce, 2 * kBouncePiece + sizeof(Ctrl)));
+static int alloc_host_side(dsk_state* s, size_t more = 0) {
+  CK(cudaMallocHost((void**)&s->bounce, 2 * kBouncePiece + sizeof(Ctrl) + more));
   s->h_ctrl = (Ctrl*)(s->bounce + 2 * kBouncePiece);
-  memset(s->h_ctrl, 0, sizeof(Ctrl));
+  memset(s->h_ctrl, 0, sizeof(Ctrl) + more);
   for (cudaEvent_t& e : s->bounce_ev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   return 0;
 }

@@ -157,7 +157,7 @@ struct State {
   float* vfirst = nullptr;                   // [chunk][kv_heads * vdim] values of the step's tokens in the first value-mixing layer
   int* d_prev = nullptr;                     // the sequence's last token (bigram embedding)
   float *x = nullptr, *h = nullptr, *b0 = nullptr, *b1 = nullptr, *b2 = nullptr, *b3 = nullptr, *wgt = nullptr, *logits = nullptr;
-  int *h_tok = nullptr, *h_want = nullptr;   // pinned staging of a chunk's token ids / wanted rows (one allocation, with h_err)
+  int *h_tok = nullptr, *h_want = nullptr;   // pinned staging of a chunk's token ids / wanted rows (behind dsk_state::h_ctrl, with h_err)
   // attention of portions in one kernel (pattn): split keys and values of the visible positions, queries it takes at a time
   __nv_bfloat16 *k16 = nullptr, *v16 = nullptr;
   int pattn_q = 0;
@@ -166,7 +166,10 @@ struct State {
   __nv_bfloat16 *a16 = nullptr, *hid16 = nullptr;
   size_t a16_elems = 0, hid16_elems = 0;
   int* h_err = nullptr;
-  std::vector<void*> allocs;
+  // device memory of the state: one allocation, cut into the pieces that salloc was asked for (portion: one that only the attention of portions needs)
+  struct Piece { void** at; size_t bytes; bool portion; };
+  std::vector<Piece> pieces;
+  char* arena = nullptr;
   // side-by-side mixers run on two streams, forked and joined by events
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -1136,11 +1139,24 @@ static int launches_per_token(const dsk_model* m) {
 // ---------------------------------------------------------------------------------------------------------------------
 // state
 // ---------------------------------------------------------------------------------------------------------------------
-static int salloc(State* S, void** p, size_t bytes) {
-  CK(cudaMalloc(p, bytes ? bytes : 16));
-  CK(cudaMemset(*p, 0, bytes ? bytes : 16));
-  S->allocs.push_back(*p);
+// Asks for a piece of the state's memory; *p is set by salloc_all.
+static int salloc(State* S, void** p, size_t bytes, bool portion = false) {
+  S->pieces.push_back({p, (std::max<size_t>(bytes, 16) + 511) / 512 * 512, portion});
   return 0;
+}
+// All pieces in one allocation (an allocation and a zeroing for each of 30 to 50 pieces were most of the time that a state took to make and to free), zeroed.
+// Where it does not fit with the buffers of the attention of portions, without them.
+static int salloc_all(State* S, cudaStream_t st) {
+  auto total = [&] { size_t n = 0; for (const State::Piece& q : S->pieces) n += q.bytes; return n; };
+  if (cudaMalloc((void**)&S->arena, total()) != cudaSuccess) {
+    cudaGetLastError();
+    for (State::Piece& q : S->pieces) if (q.portion) { q.bytes = 0; S->prefill_keys = 0; }
+    CK(cudaMalloc((void**)&S->arena, total()));
+  }
+  CK(cudaMemsetAsync(S->arena, 0, total(), st));
+  char* at = S->arena;
+  for (const State::Piece& q : S->pieces) { *q.at = q.bytes ? at : nullptr; at += q.bytes; }
+  return cudaStreamSynchronize(st) == cudaSuccess ? 0 : -2;
 }
 
 static int state_reset(dsk_state* s) {
@@ -1171,14 +1187,14 @@ static dsk_state* state_create(dsk_model* m) {
   S->timeline = getenv("DSK_HY_TIMELINE") != nullptr;
   const size_t Tc = c.chunk;
   // the pieces the shared sampling / arg-max code reads
-  cudaMalloc((void**)&s->ctrl, sizeof(Ctrl)); cudaMemset(s->ctrl, 0, sizeof(Ctrl));
-  if (alloc_host_side(s)) return nullptr;
+  salloc(S, (void**)&s->ctrl, sizeof(Ctrl));
+  if (alloc_host_side(s, (2 * Tc + 1) * 4)) return nullptr;
+  S->h_tok = (int*)(s->h_ctrl + 1); S->h_want = S->h_tok + Tc; S->h_err = S->h_tok + 2 * Tc;   // (zeroed)
   s->token_log_cap = 1 << 16;
-  cudaMalloc((void**)&s->token_log, s->token_log_cap * sizeof(int));
-  cudaMalloc((void**)&s->step, sizeof(int));
-  cudaMalloc((void**)&s->sample_out, 4 * sizeof(float)); cudaMemset(s->sample_out, 0, 4 * sizeof(float));
-  cudaMalloc((void**)&s->logits, (size_t)c.vocab_size * 4); cudaMemset(s->logits, 0, (size_t)c.vocab_size * 4);
-  s->logits_src = s->logits;
+  salloc(S, (void**)&s->token_log, s->token_log_cap * sizeof(int));
+  salloc(S, (void**)&s->step, sizeof(int));
+  salloc(S, (void**)&s->sample_out, 4 * sizeof(float));
+  salloc(S, (void**)&s->logits, (size_t)c.vocab_size * 4);
   cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
   cudaEventCreate(&s->ev0); cudaEventCreate(&s->ev1);
   if (cudaGetLastError() != cudaSuccess) { fail(-2, "state allocation failed"); return nullptr; }
@@ -1336,11 +1352,11 @@ static dsk_state* state_create(dsk_model* m) {
     for (const HLayer& L : M->L) if (has_attn(L.sp)) rows = std::max(rows, visible(L.sp, takes_pattn(L.sp, bf16) ? S->pattn_q : S->talk_q));
     if (rows > 0 && fused <= kPortionBytes + kPortionBytes / 2 && plain <= kPortionBytes) {
       S->prefill_keys = (int)rows;
-      if (k16) rc |= salloc(S, (void**)&S->k16, k16 * 2) | salloc(S, (void**)&S->v16, v16 * 2);
-      rc |= salloc(S, (void**)&S->kf, std::max(kup, keys * hd) * 4) | salloc(S, (void**)&S->vf, std::max(vup, keys * hv) * 4);
-      rc |= salloc(S, (void**)&S->d_rows, rows * 4);
-      if (pack_es) rc |= salloc(S, &S->kb, keys * hd * pack_es) | salloc(S, &S->vt, keys * hv * pack_es);
-      if (keys) rc |= salloc(S, (void**)&S->sc, heads * S->talk_q * keys * 4);
+      if (k16) rc |= salloc(S, (void**)&S->k16, k16 * 2, true) | salloc(S, (void**)&S->v16, v16 * 2, true);
+      rc |= salloc(S, (void**)&S->kf, std::max(kup, keys * hd) * 4, true) | salloc(S, (void**)&S->vf, std::max(vup, keys * hv) * 4, true);
+      rc |= salloc(S, (void**)&S->d_rows, rows * 4, true);
+      if (pack_es) rc |= salloc(S, &S->kb, keys * hd * pack_es, true) | salloc(S, &S->vt, keys * hv * pack_es, true);
+      if (keys) rc |= salloc(S, (void**)&S->sc, heads * S->talk_q * keys * 4, true);
     }
   }
   rc |= salloc(S, (void**)&S->x, Tc * c.dim * 4) | salloc(S, (void**)&S->h, Tc * c.dim * 4);
@@ -1371,10 +1387,8 @@ static dsk_state* state_create(dsk_model* m) {
     rc |= salloc(S, (void**)&S->a16, S->a16_elems * 2) | salloc(S, (void**)&S->hid16, S->hid16_elems * 2);
   }
   rc |= salloc(S, (void**)&S->logits, (size_t)S->head_rows * c.vocab_size * 4);
-  if (rc) { fail(-2, "state allocation failed"); return nullptr; }
-  if (cudaMallocHost((void**)&S->h_tok, (2 * Tc + 1) * 4) != cudaSuccess) { fail(-2, "pinned allocation failed"); return nullptr; }
-  S->h_want = S->h_tok + Tc; S->h_err = S->h_tok + 2 * Tc;
-  *S->h_err = 0;
+  if (rc || salloc_all(S, s->stream)) { fail(-2, "state allocation failed"); return nullptr; }
+  s->logits_src = s->logits;
   m->n_states++;
   return s;
 }
@@ -1385,8 +1399,8 @@ static void state_free(dsk_state* s) {
   if (S->step_graph) cudaGraphExecDestroy(S->step_graph);
   if (S->side) { cudaStreamSynchronize(S->side); cudaStreamDestroy(S->side); cudaEventDestroy(S->ev_fork); cudaEventDestroy(S->ev_join); }
   for (cudaEvent_t e : S->tl_events) cudaEventDestroy(e);
-  for (void* p : S->allocs) cudaFree(p);
-  cudaFreeHost(S->h_tok);
+  cudaFree(S->arena);
+  s->ctrl = nullptr; s->token_log = s->step = nullptr; s->sample_out = s->logits = nullptr;   // (pieces of it)
   delete S;
   s->hy = nullptr;
 }
