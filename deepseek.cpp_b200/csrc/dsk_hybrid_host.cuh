@@ -1810,7 +1810,11 @@ static void launch_decode_attn(State* S, DecodeAttn P, bool latent, cudaStream_t
   P.NS = 1;
   if (T <= kAttnSplitTokens) {   // the widest key range a CTA can meet is span + kept + TQ - 1 keys
     const int tiles = (std::min(P.span, P.ring) + P.mods.keep + P.TQ - 1 + 31) / 32;
-    P.NS = std::max(1, std::min(tiles, kAttnSplitMax));
+    // Shares of the keys: one a tile, but no more CTAs than run at a time (three an SM).  With a CTA per tile and key head, 16 key heads behind a window of 4096
+    // were 1024 CTAs, waiting for a place and mostly without a key of theirs: two such layers (width 1024) and their head took 120 us a token behind 30 keys and
+    // 150 behind 2000, gqa_attn with its four key heads a CTA 117 and 139, this 109 and 135.
+    const int rows = (T + P.TQ - 1) / P.TQ * P.G * ((rep + P.HB - 1) / P.HB), most = std::max(1, std::min(kAttnSplitMax, 3 * 148 / rows)), per = (tiles + most - 1) / most;
+    P.NS = (tiles + per - 1) / per;
   }
   P.part = S->part;
   const dim3 grid((unsigned)((T + P.TQ - 1) / P.TQ), (unsigned)(P.G * ((rep + P.HB - 1) / P.HB)), (unsigned)P.NS);

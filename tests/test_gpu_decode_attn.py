@@ -28,3 +28,14 @@ def test_latents(mk, no, heads, kv_rank, rot_dim):  # noqa: F811
     exp = no.run(cfg, W, toks)[0]
     for sizes in PORTIONS:
         assert rel(in_portions(m, toks, sizes), exp) < F32_TOL
+
+
+@pytest.mark.parametrize("heads,kv_heads", [(16, 16), (8, 4), (5, 5)])
+def test_shares_of_several_tiles(mk, no, heads, kv_heads):  # noqa: F811
+    """Windows so wide, over so many key heads, that a CTA's share of the keys is more than a tile: 74 tiles in shares of 3, 1 and 1."""
+    cfg = no.model_config([no.att(heads=heads, kv_heads=kv_heads, dim=16, vdim=12, size=None)] * 2, width=48, vocab=97)
+    m, W = mk(cfg, seed=heads, chunk=200, context=2300)
+    toks = tokens_for(cfg, 240, 6)
+    exp = no.run(cfg, W, toks)[0]
+    for sizes in ([], [200, 2, 2, 3, 3, 4, 4], [90, 1, 4, 3, 2, 100]):
+        assert rel(in_portions(m, toks, sizes), exp) < F32_TOL
