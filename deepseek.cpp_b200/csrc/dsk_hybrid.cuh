@@ -12,7 +12,7 @@
 //   gemm_tc5          the same for bf16 weights that TMA can address, on the 5th-generation tensor cores (dsk_tc5.cuh)
 //   gemm_mma          the same for the other bf16 weights on mma.sync (activations rounded to bf16 as they are staged)
 //   gemm_split        the same for fp32 weights, operands as three bf16 parts (dsk_pattn.cuh);  gemm_tiled keeps routed products of few rows
-//   gemm_narrow       up to 96 columns over more than 32 rows
+//   gemm_narrow       up to 96 columns over 448 rows and more
 //   gemv_rows         the same interface for T <= 4 rows: one warp per weight row, 16-byte loads
 //   gemv_one          the same for one row (a decoded token): eight 16-byte weight loads in flight per lane
 //   causal_conv_silu  depthwise causal convolution over the chunk continuing from the carried (taps - 1) inputs, + SiLU

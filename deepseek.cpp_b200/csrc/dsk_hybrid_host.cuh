@@ -186,6 +186,7 @@ static constexpr int kPrefillQ = 256, kPrefillMin = 32;   // prefill attention: 
 // Buffers of the attention of portions: a state takes them up to this size (blocks of kPrefillQ queries of the fused kernel, the smallest there are: up to
 // half as much again).  Heads x keys decide: 16 key heads of 64 + 64 entries take 25 KB a key.
 static constexpr size_t kPortionBytes = (size_t)4 << 30;
+static constexpr int kNarrowMin = 448;                           // rows from which a product of up to 96 columns runs on gemm_narrow
 static constexpr int kAttnSplitMax = 64, kAttnSplitTokens = 4;   // decode-sized chunks split a window over up to 64 CTAs
 
 static bool is_ssd(const dsk_layer_spec& s) { return s.mixer == DSK_MIX_SSD; }
@@ -1632,7 +1633,9 @@ static void launch_narrow(bool bf16, int epi, const GemmP& P, cudaStream_t st) {
 static void linear(State* S, bool bf16, int epi, const GemmP& P, int Z, cudaStream_t st, int tile_cap = 0) {
   const bool small = P.z_expert != nullptr || (!P.tiles && P.M <= 4);
   if (!small && !P.tiles && Z == 1 && P.N <= 96) {   // narrow output (router, token-input gate): warp-per-row products over batches of 4 rows
-    if (epi != HEPI_SIGMUL && P.M > 32 && !epi_dual(epi)) {
+    // (a CTA of gemm_narrow has 16 rows: under 448 they are too few.  Steps of 256 / 384 / 512 / 1024 tokens, two layers with 64 experts and a token input of
+    // 32, width 2048: 714 / 819 / 873 / 1126 us with it, 650 / 806 / 895 / 1221 with the products of warps; width 1024: 519 / 669 / 738 / 786 and 506 / 654 / 749 / 832)
+    if (epi != HEPI_SIGMUL && P.M >= kNarrowMin && !epi_dual(epi)) {
       launch_narrow(bf16, epi, P, st);
       S->launches++;
       return;

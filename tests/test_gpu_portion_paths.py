@@ -34,6 +34,15 @@ def test_narrow_products(mk, ho, experts, side, width, tokens):  # noqa: F811
     assert rel(m.forward_chunk(toks, 0, range(tokens)), ho.run(cfg, W, toks)[0]) < F32_TOL
 
 
+@pytest.mark.parametrize("experts,side,width,tokens", [(5, 3, 36, 448), (33, 32, 40, 449), (96, 90, 72, 513), (7, 64, 130, 463)])
+def test_narrow_products_of_many_rows(mk, ho, experts, side, width, tokens):  # noqa: F811
+    moe = {"kind": "moe", "router": {"experts": experts, "top": 2, "scale": 1.0}, "expert": {"ff": 12, "limit": 3.0}}
+    cfg = ho.small_config(layers=[dict(ssd(2, 6, 4, 1), mlp=moe)], width=width, norm={"eps": 1e-5, "groups": 1}, token_side={"dim": side})
+    m, W = mk(cfg, seed=experts, chunk=600)
+    toks = tokens_for(cfg, tokens, 12)
+    assert rel(m.forward_chunk(toks, 0, range(tokens)), ho.run(cfg, W, toks)[0]) < F32_TOL
+
+
 def test_large_windows_take_the_fused_kernel(mk_netusun, no, monkeypatch, capfd):  # noqa: F811
     """What switches the attention of portions on is the memory of the layers that use it: 64 heads x 256 queries x 70000 keys are 4.6 GB of scores, which
     only the products between which scores lie in memory would have."""
