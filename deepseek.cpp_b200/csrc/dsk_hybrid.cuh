@@ -7,11 +7,10 @@
 //   embed_rows        token ids -> fp32 residual rows
 //   group_rmsnorm     RMS norm in `groups` equal consecutive parts (groups = 1: plain RMSNorm); can also add its result,
 //                     scaled, into the residual, or write its rows into a ring cache
-//   gemm_tiled        C = A W^T for T > 4 rows (fp32 activations, fp32 or bf16 weights, fp32 accumulate) with fused
+//   gemm_tc5          C = A W^T for T > 4 rows and bf16 weights that TMA can address, on the 5th-generation tensor cores (dsk_tc5.cuh), with fused
 //                     epilogues (residual add, clamped GLU, GELU x per-token embedding) and row gather / scatter / expert tiles
-//   gemm_tc5          the same for bf16 weights that TMA can address, on the 5th-generation tensor cores (dsk_tc5.cuh)
 //   gemm_mma          the same for the other bf16 weights on mma.sync (activations rounded to bf16 as they are staged)
-//   gemm_split        the same for fp32 weights, operands as three bf16 parts (dsk_pattn.cuh);  gemm_tiled keeps routed products of few rows
+//   gemm_split        the same for fp32 weights, operands as three bf16 parts (dsk_pattn.cuh)
 //   gemm_narrow       up to 96 columns over 448 rows and more
 //   gemv_rows         the same interface for T <= 4 rows: one warp per weight row, 16-byte loads
 //   gemv_one          the same for one row (a decoded token): eight 16-byte weight loads in flight per lane
@@ -36,7 +35,7 @@
 //   hgrn2_scan        the gated linear recurrence S <- diag(f) S + (1 - f) v^T, o = S^T silu(q), f = l + (1 - l) sigmoid(.)
 //   moe_route         sigmoid scores, selection by score + correction, weights = normalised scores x scale; or the largest
 //                     logits with a softmax over the chosen ones; or a softmax over all experts, limited to the best groups
-//   moe_plan          groups the (token, slot) pairs of a chunk by expert into row tiles for gemm_tiled
+//   moe_plan          groups the (token, slot) pairs of a chunk by expert into row tiles for those products
 //   moe_combine       residual += alpha * sum_k w_k y_k (or stored, when a norm follows), a shared expert's row included
 //
 // Numerics: the residual stream, norms, router, softmax, recurrent state, decays, step sizes and gates are fp32 in every mode;
@@ -294,7 +293,7 @@ struct GemmP {
   const int* z_expert;     // gemv_rows only: batch z uses expert z_expert[z], A row z / z_adiv, C row z (one row per batch)
   int z_adiv;
   int z_rows;              // gemv_rows only, > 0: batch z takes rows 4z .. 4z + 3 of z_rows rows (narrow outputs over many rows)
-  const int4* tiles;       // gemm_tiled only: row tiles grouped by expert {expert, first logical row, rows, -}
+  const int4* tiles;       // more than four rows only: row tiles grouped by expert {expert, first logical row, rows, -}
   const int* n_tiles;
   float alpha;             // STORE: C = alpha acc; ADD: C += alpha acc
   float lim;               // GLU: g = min(gate, lim), u = clamp(up, -lim, lim), C = g sigmoid(1.702 g) (u + 1)
@@ -313,9 +312,9 @@ struct GemmP {
   const void *sW1, *sW2;   // [sN][sK], packed
   const float* As;
   float* Cs;
-  // n_expert: experts behind W, tile_rows: rows a tile may have (tile lists).  gemm_tc5 only:  A16: the activations as packed bf16 rows in the product's row order (null: rounded
+  // n_expert: experts behind W (tile lists).  gemm_tc5 only:  A16: the activations as packed bf16 rows in the product's row order (null: rounded
   // from A by a pass of its own);  C16: results go there as packed bf16 rows in the product's row order instead of to C
-  int n_expert, tile_rows;
+  int n_expert;
   const __nv_bfloat16* A16;
   __nv_bfloat16* C16;
   // gemm_split only: scores of queries at positions band_pos + row against keys at positions band_first + column (BAND_COLS: tiles that no query of
@@ -363,102 +362,6 @@ __device__ __forceinline__ void gemm_epilogue(const GemmP& P, float* __restrict_
     crow[n] = dual_value<EPI>(P, v, v2);
   } else {
     crow[n] = final_value<WT, EPI>(P, cr, n, v, EPI == HEPI_ADD || EPI == HEPI_SIGMUL ? crow[n] : 0.f);
-  }
-}
-
-// 64 x 64 output tile, K in steps of 16, 256 threads with a 4 x 4 micro-tile each; plain fp32 FMA on fp32 activations.
-template <typename WT, int EPI>
-__global__ void __launch_bounds__(256) gemm_tiled(const GemmP P) {
-  grid_enter();
-  constexpr int BM = 64, BN = 64, BK = 16;
-  constexpr bool DUAL = epi_dual(EPI);
-  __shared__ __align__(16) float As[BK][BM + 4];
-  __shared__ __align__(16) float Bs[DUAL ? 2 : 1][BK][BN + 4];
-  __shared__ int rowsA[BM], rowsC[BM];
-  const int tid = threadIdx.x;
-  long long aoff = (long long)blockIdx.z * P.sA, woff = (long long)((int)blockIdx.z / P.z_wdiv) * P.sW, coff = (long long)blockIdx.z * P.sC;
-  int row0, nrows;
-  if (P.tiles) {
-    if ((int)blockIdx.y >= *P.n_tiles) return;
-    const int4 t = P.tiles[blockIdx.y];
-    woff = (long long)t.x * P.sW;
-    row0 = t.y;
-    nrows = t.z;
-  } else {
-    row0 = blockIdx.y * BM;
-    nrows = min(BM, P.M - row0);
-  }
-  if (tid < BM) {
-    const int i = row0 + tid;
-    const bool ok = tid < nrows;
-    rowsA[tid] = ok ? (P.a_map ? P.a_map[i] / P.a_div : i) : -1;
-    rowsC[tid] = ok ? (P.c_map ? P.c_map[i] : i) : -1;
-  }
-  __syncthreads();
-  const int n0 = blockIdx.x * BN;
-  const WT* __restrict__ W = reinterpret_cast<const WT*>(P.W) + woff;
-  const WT* __restrict__ W2 = DUAL ? reinterpret_cast<const WT*>(P.W2) + woff : nullptr;
-  const float* __restrict__ A = P.A + aoff;
-  const int lr = tid >> 2, lk = (tid & 3) * 4;
-  const int tx = tid & 15, ty = tid >> 4;
-  float acc[4][4], acc2[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) { acc[i][j] = 0.f; acc2[i][j] = 0.f; }
-  const int ar = rowsA[lr];
-  const int wn = n0 + lr;
-  float ra[4], rb[4], rb2[4];
-  auto fetch = [&](int k0) {
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int k = k0 + lk + j;
-      ra[j] = (ar >= 0 && k < P.K) ? A[(size_t)ar * P.lda + k] : 0.f;
-      const bool wok = wn < P.N && k < P.K;
-      rb[j] = wok ? to_f<WT>(W[(size_t)wn * P.ldw + k]) : 0.f;
-      rb2[j] = (DUAL && wok) ? to_f<WT>(W2[(size_t)wn * P.ldw + k]) : 0.f;
-    }
-  };
-  fetch(0);
-  for (int k0 = 0; k0 < P.K; k0 += BK) {
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      As[lk + j][lr] = ra[j];
-      Bs[0][lk + j][lr] = rb[j];
-      if (DUAL) Bs[DUAL ? 1 : 0][lk + j][lr] = rb2[j];
-    }
-    __syncthreads();
-    if (k0 + BK < P.K) fetch(k0 + BK);   // in flight during this step's FMAs
-#pragma unroll
-    for (int kk = 0; kk < BK; kk++) {
-      const float4 a4 = *reinterpret_cast<const float4*>(&As[kk][ty * 4]);
-      const float4 b4 = *reinterpret_cast<const float4*>(&Bs[0][kk][tx * 4]);
-      const float a[4] = {a4.x, a4.y, a4.z, a4.w}, b[4] = {b4.x, b4.y, b4.z, b4.w};
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-      if (DUAL) {
-        const float4 c4 = *reinterpret_cast<const float4*>(&Bs[DUAL ? 1 : 0][kk][tx * 4]);
-        const float c[4] = {c4.x, c4.y, c4.z, c4.w};
-#pragma unroll
-        for (int i = 0; i < 4; i++)
-#pragma unroll
-          for (int j = 0; j < 4; j++) acc2[i][j] = fmaf(a[i], c[j], acc2[i][j]);
-      }
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int cr = rowsC[ty * 4 + i];
-    if (cr < 0) continue;
-    float* crow = P.C + coff + (size_t)cr * P.ldc;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int n = n0 + tx * 4 + j;
-      if (n < P.N) gemm_epilogue<WT, EPI>(P, crow, cr, n, acc[i][j], acc2[i][j]);
-    }
   }
 }
 
@@ -566,7 +469,7 @@ __global__ void __launch_bounds__(256) gemm_narrow(const GemmP P) {
 
 // Tensor-core variant for bf16 weights and more than a handful of rows: 128 x 128 tile of A W^T per CTA (K in steps of 32), the
 // fp32 activations rounded to bf16 while they are staged, mma.sync m16n8k16 bf16 x bf16 -> fp32.  8 warps as 2 (rows) x 4
-// (columns), a 64 x 32 warp tile.  Same row maps, expert tiles, batches and epilogues as gemm_tiled.  For the GLU epilogue the
+// (columns), a 64 x 32 warp tile.  Row maps, expert tiles, batches and epilogues of GemmP.  For the GLU epilogue the
 // 128 staged weight rows alternate, in granules of 8, between the gate and the up matrix, so a thread holds both values of an
 // output element in neighbouring accumulators and a CTA produces 64 output columns.
 __device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {

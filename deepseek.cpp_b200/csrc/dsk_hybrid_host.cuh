@@ -1553,8 +1553,9 @@ static void launch_tc5(State* S, int epi, const GemmP& P, int tile_cap, cudaStre
 }
 
 template <typename WT>
-static void launch_gemm_t(int epi, const GemmP& P, int Z, bool small, int tile_cap, cudaStream_t st) {
-  if (small && gemv_one_ok<WT>(P)) {
+// products of up to four rows
+static void launch_gemv(int epi, const GemmP& P, int Z, cudaStream_t st) {
+  if (gemv_one_ok<WT>(P)) {
     const int n = std::max(P.N, P.n_shared > 0 ? P.sN : 0);
     const int R = (long long)n * Z >= (Z == 1 ? 16384 : 148 * 64) ? 2 : 1;   // rows per warp: two where one each would be more warps than the chip holds at a time
     const dim3 grid((unsigned)std::max(1, std::min((n + 8 * R - 1) / (8 * R), 148 * 8)), (unsigned)Z);
@@ -1574,7 +1575,7 @@ static void launch_gemm_t(int epi, const GemmP& P, int Z, bool small, int tile_c
       default: DSK_GEMV1(HEPI_GELU_MUL); break;
     }
 #undef DSK_GEMV1
-  } else if (small) {
+  } else {
     const dim3 grid((unsigned)std::max(1, std::min((std::max(P.N, P.n_shared > 0 ? P.sN : 0) + 7) / 8, 148 * 8)), (unsigned)Z);
     switch (epi) {
       case HEPI_STORE: launch_next(gemv_rows<WT, HEPI_STORE>, grid, 256, 0, st)(P); break;
@@ -1589,22 +1590,6 @@ static void launch_gemm_t(int epi, const GemmP& P, int Z, bool small, int tile_c
       case HEPI_SOFTCAP: launch_next(gemv_rows<WT, HEPI_SOFTCAP>, grid, 256, 0, st)(P); break;
       case HEPI_SWIGLU: launch_next(gemv_rows<WT, HEPI_SWIGLU>, grid, 256, 0, st)(P); break;
       default: launch_next(gemv_rows<WT, HEPI_GELU_MUL>, grid, 256, 0, st)(P); break;
-    }
-  } else {
-    const dim3 grid((unsigned)((P.N + 63) / 64), (unsigned)(P.tiles ? tile_cap : (P.M + 63) / 64), (unsigned)Z);
-    switch (epi) {
-      case HEPI_STORE: launch_next(gemm_tiled<WT, HEPI_STORE>, grid, 256, 0, st)(P); break;
-      case HEPI_ADD: launch_next(gemm_tiled<WT, HEPI_ADD>, grid, 256, 0, st)(P); break;
-      case HEPI_GLU: launch_next(gemm_tiled<WT, HEPI_GLU>, grid, 256, 0, st)(P); break;
-      case HEPI_XIELU: launch_next(gemm_tiled<WT, HEPI_XIELU>, grid, 256, 0, st)(P); break;
-      case HEPI_GEGLU: launch_next(gemm_tiled<WT, HEPI_GEGLU>, grid, 256, 0, st)(P); break;
-      case HEPI_SIGMUL: launch_next(gemm_tiled<WT, HEPI_SIGMUL>, grid, 256, 0, st)(P); break;
-      case HEPI_RELU2: launch_next(gemm_tiled<WT, HEPI_RELU2>, grid, 256, 0, st)(P); break;
-      case HEPI_LINGATE: launch_next(gemm_tiled<WT, HEPI_LINGATE>, grid, 256, 0, st)(P); break;
-      case HEPI_SILU_SIG: launch_next(gemm_tiled<WT, HEPI_SILU_SIG>, grid, 256, 0, st)(P); break;
-      case HEPI_SOFTCAP: launch_next(gemm_tiled<WT, HEPI_SOFTCAP>, grid, 256, 0, st)(P); break;
-      case HEPI_SWIGLU: launch_next(gemm_tiled<WT, HEPI_SWIGLU>, grid, 256, 0, st)(P); break;
-      default: launch_next(gemm_tiled<WT, HEPI_GELU_MUL>, grid, 256, 0, st)(P); break;
     }
   }
 }
@@ -1643,16 +1628,16 @@ static void linear(State* S, bool bf16, int epi, const GemmP& P, int Z, cudaStre
     GemmP Q = P;
     Q.z_rows = P.M;
     const int zb = (P.M + 3) / 4;
-    if (bf16) launch_gemm_t<__nv_bfloat16>(epi, Q, zb, true, 0, st);
-    else launch_gemm_t<float>(epi, Q, zb, true, 0, st);
+    if (bf16) launch_gemv<__nv_bfloat16>(epi, Q, zb, st);
+    else launch_gemv<float>(epi, Q, zb, st);
     S->launches++;
     return;
   }
   if (tc_ok(S, bf16, epi, P, Z)) launch_tc5(S, epi, P, tile_cap, st);
   else if (bf16 && !small) launch_gemm_mma(epi, P, Z, tile_cap, st);
-  else if (bf16) launch_gemm_t<__nv_bfloat16>(epi, P, Z, small, tile_cap, st);
-  else if (!small && (!P.tiles || P.tile_rows == 128)) launch_split(epi, P, Z, tile_cap, st);
-  else launch_gemm_t<float>(epi, P, Z, small, tile_cap, st);
+  else if (!small) launch_split(epi, P, Z, tile_cap, st);
+  else if (bf16) launch_gemv<__nv_bfloat16>(epi, P, Z, st);
+  else launch_gemv<float>(epi, P, Z, st);
   S->launches++;
 }
 
@@ -2507,15 +2492,13 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         linear(S, bf, HEPI_STORE, Dn, pairs + (shared ? T : 0), st);
         MK("moe.down");
       } else {
-        // rows per tile of the product kernel that follows (gemm_tc5, gemm_mma and gemm_split, or gemm_tiled: few rows per expert)
-        // (fp32, under 64 rows per expert: gemm_tiled's FMA on 64 rows are fewer cycles than six tensor-core products on 128)
-        const int bm = bf || pairs >= 64 * E ? 128 : 64;
+        constexpr int bm = 128;   // rows per tile of the product kernels that follow (gemm_tc5, gemm_mma, gemm_split)
         launch_next(moe_plan, 1, 1024, (size_t)2 * E * 4, st)(S->d_idx, pairs, E, bm, S->d_perm, S->d_tiles, S->d_ntiles);
         S->launches++;
         G.tiles = S->d_tiles; G.n_tiles = S->d_ntiles; G.a_map = S->d_perm; G.a_div = top; G.c_map = S->d_perm;
         Dn.tiles = S->d_tiles; Dn.n_tiles = S->d_ntiles; Dn.a_map = S->d_perm; Dn.a_div = 1; Dn.c_map = S->d_perm;
         const int cap = std::min(S->max_tiles, pairs / bm + E + 1);
-        G.n_expert = Dn.n_expert = E; G.tile_rows = Dn.tile_rows = bm;
+        G.n_expert = Dn.n_expert = E;
         hidden16(S, bf, epi_up, G, HEPI_STORE, Dn, S->hid16);
         MK("moe.plan");
         linear(S, bf, epi_up, G, 1, st, cap);

@@ -395,8 +395,8 @@ __global__ void __launch_bounds__(256, 1) pattn(const __grid_constant__ PattnP P
 // fp32 products of many rows (fp32 models; the score and value products of attention with mixed heads) on the tensor cores: both operands split
 // into three bf16 parts on their way into shared memory, six products per element as in pattn.  128 x 64 tile, 32 deep; 8 warps as 4 (rows) x 2
 // (columns), a 32 x 32 warp tile; the next slice's fp32 values are in registers during this one's products.  Interface, row maps, expert tiles,
-// batches and epilogues as gemm_tiled, which keeps routed products of few rows per expert.  Bound: the six mma.sync per element.  gemm_tiled was
-// bound by the fp32 pipe: a step in fp32 at width 1024 went from 1.85 to 1.22 ms (600 tokens), from 0.95 to 0.67 (64 tokens) and from 0.89 to 0.64
+// batches and epilogues of GemmP.  Bound: the six mma.sync per element.  A kernel of 64 x 64 tiles was bound by the fp32 pipe, with routed products of four
+// rows per expert too (1.58 ms a step of 33 tokens with it, 1.57 with this; 16 rows: 1.17 and 1.10): a step in fp32 at width 1024 went from 1.85 to 1.22 ms (600 tokens), from 0.95 to 0.67 (64 tokens) and from 0.89 to 0.64
 // (5 tokens), a 1500-token prompt with mixed heads from 2.98 to 2.67 ms; the error against 64 bits of the first from 1.0e-6 to 5e-7.
 // ---------------------------------------------------------------------------------------------------------------------
 // The same sum as a chain of FMAs over the numbers themselves, for a result that is not finite: an infinite operand has no three parts (what is left
