@@ -2297,7 +2297,8 @@ __global__ void moe_route(const float* __restrict__ logits, int ldz, const float
   for (int e = threadIdx.x; e < E; e += blockDim.x) {
     const float s = mode == 0 ? sigmoid_f(z[e]) : z[e];
     sc[e] = s;
-    ch[e] = s + (correction ? correction[e] : 0.f);
+    const float c = s + (correction ? correction[e] : 0.f);
+    ch[e] = isnan(c) ? -INFINITY : c;   // (a rank of its own for every expert, so that every slot gets one: the row's results are NaN by its weights)
   }
   __syncthreads();
   float zmax = 0.f, zsum = 1.f;

@@ -127,3 +127,25 @@ def test_recurrence_in_blocks(mk_hybrid, ho, value):  # noqa: F811
             m.reset()
             assert ahead_of_the_poison(m, ho.run, cfg, W, t, at, sizes) < F32_TOL
     m.reset()
+
+
+@pytest.mark.parametrize("router", ["sigmoid", "groups"])
+def test_routed_rows(mk, mk_hybrid, no, ho, router):  # noqa: F811
+    """A token whose router scores are NaN gets experts that exist, and the others theirs: in short steps, and in portions, where rows are put into
+    expert order."""
+    if router == "groups":
+        cfg, run = no.model_config([no.att(mlp=no.moe(experts=12, top=4, count=3, keep=2))], width=40, vocab=97), no.run
+        m, W = mk(cfg, seed=4, chunk=64, edit=lambda W: poisoned(W, np.nan, 50))
+    else:
+        moe = {"kind": "moe", "router": {"experts": 7, "top": 3, "scale": 1.0}, "expert": {"ff": 12, "limit": 3.0}}
+        att = {"type": "latent_attention", "mixer": {"heads": 3, "dim": 12, "vdim": 20, "kv_rank": 40, "mask": {"size": 30}, "scale": 0.3}, "mlp": moe}
+        cfg, run = ho.small_config(layers=[att], width=36, norm={"eps": 1e-5, "groups": 1}), ho.run
+        m, W = mk_hybrid(cfg, seed=4, chunk=64, edit=lambda W: poisoned(W, np.nan, 50))
+    toks = tokens_for(cfg, 60, 5)
+    toks[toks == 50] = 7
+    for sizes in ([60], [4] * 15, [9, 51]):
+        for at in (1, 20, 59):
+            t = toks.copy()
+            t[at] = 50
+            m.reset()
+            assert ahead_of_the_poison(m, run, cfg, W, t, at, sizes) < F32_TOL
