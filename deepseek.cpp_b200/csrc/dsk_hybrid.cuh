@@ -46,6 +46,8 @@
 
 #include <cuda_bf16.h>
 
+#include <type_traits>
+
 #include "dsk_kernels.cuh"
 
 namespace dsk {
@@ -1317,7 +1319,7 @@ __host__ __device__ inline int attn_pitch(int n) { return ((n + 3) & ~3) + 4; }
 __host__ __device__ inline size_t decode_attn_floats(int D, int Dv, bool kv) {
   return (size_t)40 * attn_pitch(D) + (kv ? 0 : (size_t)32 * attn_pitch(Dv)) + 8 * 8 * 32 + 32 * 8 + 3 * 8;
 }
-template <bool KV, int CV>   // CV: value columns per thread (CV * 256 >= Dv)
+template <bool KV, int CV, bool MULTI>   // CV: value columns per thread (CV * 256 >= Dv); MULTI: rows of several tokens
 __global__ void __launch_bounds__(256) decode_attn(const DecodeAttn P) {
   extern __shared__ __align__(16) float sm[];
   const int D = P.D, Dv = P.Dv, pd = attn_pitch(D), pv = KV ? pd : attn_pitch(Dv), rep = P.H / P.G, hblocks = (rep + P.HB - 1) / P.HB;
@@ -1364,91 +1366,93 @@ __global__ void __launch_bounds__(256) decode_attn(const DecodeAttn P) {
   const int i_w = pos0 + row_t(w), lo_w = mask_first(P.mask, P.span, i_w), h_w = g * rep + row_h(w);
   float m, l, acc[8][CV];
   // A key that a row does not see has the weight 0 in that row's sums, and 0 x Inf is NaN: where a sum is not finite, the share is gone through again
-  // with weights of 0 left out (a product with a predicate per row, which the first walk is spared).
-  for (bool careful = false;; careful = true) {
-  m = -1e30f; l = 0.f;
+  // with weights of 0 left out (a predicate per row and product, which the first walk is spared).
+  auto walk = [&](auto careful) {
+    m = -1e30f; l = 0.f;
 #pragma unroll
-  for (int r = 0; r < 8; r++)
+    for (int r = 0; r < 8; r++)
 #pragma unroll
-    for (int k = 0; k < CV; k++) acc[r][k] = 0.f;
-  for (int j0 = lo; j0 <= hi; j0 += 32) {
-    __syncthreads();
-    stage(ks, P.kc, P.ldk, g * D, D, pd, vk, j0);
-    cp_async_commit();
-    if (!KV) stage(vs, P.vc, P.ldv, g * Dv, Dv, pv, vv, j0);
-    cp_async_commit();
-    cp_async_wait<KV ? 0 : 1>();
-    __syncthreads();
-    {   // this warp's share of the depth for all 8 rows
-      float s[8];
+      for (int k = 0; k < CV; k++) acc[r][k] = 0.f;
+    for (int j0 = lo; j0 <= hi; j0 += 32) {
+      __syncthreads();
+      stage(ks, P.kc, P.ldk, g * D, D, pd, vk, j0);
+      cp_async_commit();
+      if (!KV) stage(vs, P.vc, P.ldv, g * Dv, Dv, pv, vv, j0);
+      cp_async_commit();
+      cp_async_wait<KV ? 0 : 1>();
+      __syncthreads();
+      {   // this warp's share of the depth for all 8 rows
+        float s[8];
 #pragma unroll
-      for (int r = 0; r < 8; r++) s[r] = 0.f;
-      const float4* k4 = reinterpret_cast<const float4*>(ks + lane * pd);
+        for (int r = 0; r < 8; r++) s[r] = 0.f;
+        const float4* k4 = reinterpret_cast<const float4*>(ks + lane * pd);
 #pragma unroll 2
-      for (int u = w; u < d4; u += 8) {
-        const float4 kv = k4[u];
+        for (int u = w; u < d4; u += 8) {
+          const float4 kv = k4[u];
 #pragma unroll
-        for (int r = 0; r < 8; r++) {
-          const float4 qv = reinterpret_cast<const float4*>(qs + r * pd)[u];
-          s[r] = fmaf(qv.x, kv.x, s[r]); s[r] = fmaf(qv.y, kv.y, s[r]); s[r] = fmaf(qv.z, kv.z, s[r]); s[r] = fmaf(qv.w, kv.w, s[r]);
+          for (int r = 0; r < 8; r++) {
+            const float4 qv = reinterpret_cast<const float4*>(qs + r * pd)[u];
+            s[r] = fmaf(qv.x, kv.x, s[r]); s[r] = fmaf(qv.y, kv.y, s[r]); s[r] = fmaf(qv.z, kv.z, s[r]); s[r] = fmaf(qv.w, kv.w, s[r]);
+          }
         }
+#pragma unroll
+        for (int r = 0; r < 8; r++) red[(w * 8 + r) * 32 + lane] = s[r];
       }
+      __syncthreads();
+      {
+        float s = 0.f;
 #pragma unroll
-      for (int r = 0; r < 8; r++) red[(w * 8 + r) * 32 + lane] = s[r];
-    }
-    __syncthreads();
-    {
-      float s = 0.f;
+        for (int k = 0; k < 8; k++) s += red[(k * 8 + w) * 32 + lane];
+        const int v = j0 + lane, p = v < nk ? v : j_lo + v - nk;
+        const bool ok = mine && v <= hi && p <= i_w && (p >= lo_w || p < keep);
+        s = ok ? mod_score(P.mods, s, i_w - p, h_w, P.H) : -1e30f;
+        const float m_new = fmaxf(m, warp_max(s));
+        const float c = expf(m - m_new), pr = ok ? expf(s - m_new) : 0.f;
+        l = l * c + warp_sum(pr);
+        m = m_new;
+        pt[lane * 8 + w] = pr;
+        if (lane == 0) corr[w] = c;
+      }
+      cp_async_wait<0>();
+      __syncthreads();
 #pragma unroll
-      for (int k = 0; k < 8; k++) s += red[(k * 8 + w) * 32 + lane];
-      const int v = j0 + lane, p = v < nk ? v : j_lo + v - nk;
-      const bool ok = mine && v <= hi && p <= i_w && (p >= lo_w || p < keep);
-      s = ok ? mod_score(P.mods, s, i_w - p, h_w, P.H) : -1e30f;
-      const float m_new = fmaxf(m, warp_max(s));
-      const float c = expf(m - m_new), pr = ok ? expf(s - m_new) : 0.f;
-      l = l * c + warp_sum(pr);
-      m = m_new;
-      pt[lane * 8 + w] = pr;
-      if (lane == 0) corr[w] = c;
-    }
-    cp_async_wait<0>();
-    __syncthreads();
+      for (int r = 0; r < 8; r++) {
+        const float c = corr[r];
 #pragma unroll
-    for (int r = 0; r < 8; r++) {
-      const float c = corr[r];
+        for (int k = 0; k < CV; k++) acc[r][k] *= c;
+      }
+      if constexpr (decltype(careful)::value) {
+        for (int jj = 0; jj < 32; jj++)
 #pragma unroll
-      for (int k = 0; k < CV; k++) acc[r][k] *= c;
-    }
-    if (careful) {
-      for (int jj = 0; jj < 32; jj++)
+          for (int k = 0; k < CV; k++) {
+            const int c = tid + 256 * k;
+            const float v = c < Dv ? vs[jj * pv + c] : 0.f;
 #pragma unroll
-        for (int k = 0; k < CV; k++) {
-          const int c = tid + 256 * k;
-          const float v = c < Dv ? vs[jj * pv + c] : 0.f;
-#pragma unroll
-          for (int r = 0; r < 8; r++) { const float pr = pt[jj * 8 + r]; if (pr != 0.f) acc[r][k] = fmaf(pr, v, acc[r][k]); }
-        }
-      continue;
-    }
+            for (int r = 0; r < 8; r++) { const float pr = pt[jj * 8 + r]; if (pr != 0.f) acc[r][k] = fmaf(pr, v, acc[r][k]); }
+          }
+      } else {
 #pragma unroll 4
-    for (int jj = 0; jj < 32; jj++) {
-      const float4 p0 = *reinterpret_cast<const float4*>(pt + jj * 8), p1 = *reinterpret_cast<const float4*>(pt + jj * 8 + 4);
+        for (int jj = 0; jj < 32; jj++) {
+          const float4 p0 = *reinterpret_cast<const float4*>(pt + jj * 8), p1 = *reinterpret_cast<const float4*>(pt + jj * 8 + 4);
 #pragma unroll
-      for (int k = 0; k < CV; k++) {
-        const int c = tid + 256 * k;
-        const float v = c < Dv ? vs[jj * pv + c] : 0.f;
-        acc[0][k] = fmaf(p0.x, v, acc[0][k]); acc[1][k] = fmaf(p0.y, v, acc[1][k]); acc[2][k] = fmaf(p0.z, v, acc[2][k]); acc[3][k] = fmaf(p0.w, v, acc[3][k]);
-        acc[4][k] = fmaf(p1.x, v, acc[4][k]); acc[5][k] = fmaf(p1.y, v, acc[5][k]); acc[6][k] = fmaf(p1.z, v, acc[6][k]); acc[7][k] = fmaf(p1.w, v, acc[7][k]);
+          for (int k = 0; k < CV; k++) {
+            const int c = tid + 256 * k;
+            const float v = c < Dv ? vs[jj * pv + c] : 0.f;
+            acc[0][k] = fmaf(p0.x, v, acc[0][k]); acc[1][k] = fmaf(p0.y, v, acc[1][k]); acc[2][k] = fmaf(p0.z, v, acc[2][k]); acc[3][k] = fmaf(p0.w, v, acc[3][k]);
+            acc[4][k] = fmaf(p1.x, v, acc[4][k]); acc[5][k] = fmaf(p1.y, v, acc[5][k]); acc[6][k] = fmaf(p1.z, v, acc[6][k]); acc[7][k] = fmaf(p1.w, v, acc[7][k]);
+          }
+        }
       }
     }
-  }
-  if (careful) break;
-  float any = 0.f;   // (stays 0 as long as every sum is finite)
+  };
+  walk(std::false_type{});
+  if constexpr (MULTI) {   // (the rows of one token see the same keys)
+    float any = 0.f;       // (stays 0 as long as every sum is finite)
 #pragma unroll
-  for (int r = 0; r < 8; r++)
+    for (int r = 0; r < 8; r++)
 #pragma unroll
-    for (int k = 0; k < CV; k++) any = fmaf(0.f, acc[r][k], any);
-  if (!__syncthreads_or(any != 0.f)) break;
+      for (int k = 0; k < CV; k++) any = fmaf(0.f, acc[r][k], any);
+    if (__syncthreads_or(any != 0.f)) walk(std::true_type{});
   }
   float c_end = 1.f;
   if (P.mods.sink && blockIdx.z == 0 && mine) {   // the sink joins the first share like a key with a zero value vector

@@ -418,9 +418,9 @@ static void set_kernel_attrs() {
   DSK_TC5_ATTR(HEPI_STORE); DSK_TC5_ATTR(HEPI_ADD); DSK_TC5_ATTR(HEPI_GLU); DSK_TC5_ATTR(HEPI_XIELU); DSK_TC5_ATTR(HEPI_GEGLU); DSK_TC5_ATTR(HEPI_SIGMUL);
   DSK_TC5_ATTR(HEPI_RELU2); DSK_TC5_ATTR(HEPI_LINGATE); DSK_TC5_ATTR(HEPI_SILU_SIG); DSK_TC5_ATTR(HEPI_SOFTCAP); DSK_TC5_ATTR(HEPI_SWIGLU); DSK_TC5_ATTR(HEPI_GELU_MUL);
 #undef DSK_TC5_ATTR
-  cudaFuncSetAttribute(decode_attn<true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big); cudaFuncSetAttribute(decode_attn<true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(decode_attn<true, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big); cudaFuncSetAttribute(decode_attn<false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
-  cudaFuncSetAttribute(decode_attn<false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, big); cudaFuncSetAttribute(decode_attn<false, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
+#define DSK_DECODE_ATTR(KV, CV) cudaFuncSetAttribute(decode_attn<KV, CV, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, big); cudaFuncSetAttribute(decode_attn<KV, CV, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, big)
+  DSK_DECODE_ATTR(true, 1); DSK_DECODE_ATTR(true, 2); DSK_DECODE_ATTR(true, 4); DSK_DECODE_ATTR(false, 1); DSK_DECODE_ATTR(false, 2); DSK_DECODE_ATTR(false, 4);
+#undef DSK_DECODE_ATTR
   cudaFuncSetAttribute(ssd_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(gqa_attn, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(mix_softmax<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, big); cudaFuncSetAttribute(mix_softmax<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
@@ -1808,15 +1808,15 @@ static void launch_decode_attn(State* S, DecodeAttn P, bool latent, cudaStream_t
   const dim3 grid((unsigned)((T + P.TQ - 1) / P.TQ), (unsigned)(P.G * ((rep + P.HB - 1) / P.HB)), (unsigned)P.NS);
   const size_t smem = decode_attn_floats(P.D, P.Dv, latent) * 4;
   const int cv = P.Dv <= 256 ? 1 : P.Dv <= 512 ? 2 : 4;
+#define DSK_DECODE_ATTN(KV, CV) do { if (P.TQ > 1) launch_next(decode_attn<KV, CV, true>, grid, 256, smem, st)(P); else launch_next(decode_attn<KV, CV, false>, grid, 256, smem, st)(P); } while (0)
   if (latent) {
-    if (cv == 1) launch_next(decode_attn<true, 1>, grid, 256, smem, st)(P);
-    else if (cv == 2) launch_next(decode_attn<true, 2>, grid, 256, smem, st)(P);
-    else launch_next(decode_attn<true, 4>, grid, 256, smem, st)(P);
-  } else {
-    if (cv == 1) launch_next(decode_attn<false, 1>, grid, 256, smem, st)(P);
-    else if (cv == 2) launch_next(decode_attn<false, 2>, grid, 256, smem, st)(P);
-    else launch_next(decode_attn<false, 4>, grid, 256, smem, st)(P);
-  }
+    if (cv == 1) DSK_DECODE_ATTN(true, 1);
+    else if (cv == 2) DSK_DECODE_ATTN(true, 2);
+    else DSK_DECODE_ATTN(true, 4);
+  } else if (cv == 1) DSK_DECODE_ATTN(false, 1);
+  else if (cv == 2) DSK_DECODE_ATTN(false, 2);
+  else DSK_DECODE_ATTN(false, 4);
+#undef DSK_DECODE_ATTN
   S->launches++;
   if (P.NS > 1) {
     launch_next(latent_swa_merge, dim3((unsigned)(T * P.H), (unsigned)((P.Dv + 127) / 128)), 128, 0, st)(S->part, P.out, P.Dv, P.NS, P.gate, P.ld_gate, P.H, P.gate_head,

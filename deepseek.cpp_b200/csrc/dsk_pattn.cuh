@@ -532,11 +532,30 @@ __global__ void __launch_bounds__(256, 2) gemm_split(const GemmP P) {
     if (kt + 1 < nk) put((kt + 1) & 1);   // the other buffer: everyone was through it at the last barrier
     __syncthreads();
   }
+  float any = 0.f;   // (stays 0 as long as every sum is finite)
+#pragma unroll
+  for (int mi = 0; mi < 2; mi++)
+#pragma unroll
+    for (int ni = 0; ni < 4; ni++)
+#pragma unroll
+      for (int q = 0; q < 4; q++) any = fmaf(0.f, acc[mi][ni][q], any);
+  if (any != 0.f) {   // all of this lane's results as plain sums (in code of its own: calls beside the sums above cost a step 2 %)
+#pragma unroll 1
+    for (int e = 0; e < (DUAL ? 16 : 32); e++) {   // e: row (mi, half) x granule x column
+      const int r = wm * 32 + (e & 1) * 8 + ((e >> 1) & 1) * 16 + (lane >> 2), g = wn * (DUAL ? 2 : 4) + (e >> 3), n = n0 + g * 8 + (lane & 3) * 2 + ((e >> 2) & 1), cr = rowsC[r];
+      if (cr < 0 || n >= P.N) continue;
+      const float* a = A + (size_t)rowsA[r] * P.lda;
+      const float v = plain_dot(a, reinterpret_cast<const float*>(P.W) + woff + (size_t)n * P.ldw, k_lo, k_hi, P.band == BAND_DEPTH);
+      const float v2 = DUAL ? plain_dot(a, reinterpret_cast<const float*>(P.W2) + woff + (size_t)n * P.ldw, k_lo, k_hi, false) : 0.f;
+      gemm_epilogue<float, EPI>(P, P.C + coff + (size_t)cr * P.ldc, cr, n, v, v2);
+    }
+    return;
+  }
 #pragma unroll
   for (int mi = 0; mi < 2; mi++)
 #pragma unroll
     for (int half = 0; half < 2; half++) {
-      const int r = wm * 32 + mi * 16 + (lane >> 2) + half * 8, cr = rowsC[r];
+      const int cr = rowsC[wm * 32 + mi * 16 + (lane >> 2) + half * 8];
       if (cr < 0) continue;
       float* crow = P.C + coff + (size_t)cr * P.ldc;
 #pragma unroll
@@ -545,11 +564,7 @@ __global__ void __launch_bounds__(256, 2) gemm_split(const GemmP P) {
         for (int q = 0; q < 2; q++) {
           const int g = wn * 4 + ni;   // granule of 8 staged rows
           const int n = DUAL ? n0 + (g >> 1) * 8 + (lane & 3) * 2 + q : n0 + g * 8 + (lane & 3) * 2 + q;
-          if (n >= P.N) continue;
-          float v = acc[mi][ni][half * 2 + q], v2 = DUAL ? acc[mi][ni + 1][half * 2 + q] : 0.f;
-          if (!isfinite(v)) v = plain_dot(A + (size_t)rowsA[r] * P.lda, reinterpret_cast<const float*>(P.W) + woff + (size_t)n * P.ldw, k_lo, k_hi, P.band == BAND_DEPTH);
-          if (DUAL && !isfinite(v2)) v2 = plain_dot(A + (size_t)rowsA[r] * P.lda, reinterpret_cast<const float*>(P.W2) + woff + (size_t)n * P.ldw, k_lo, k_hi, false);
-          gemm_epilogue<float, EPI>(P, crow, cr, n, v, v2);
+          if (n < P.N) gemm_epilogue<float, EPI>(P, crow, cr, n, acc[mi][ni][half * 2 + q], DUAL ? acc[mi][ni + 1][half * 2 + q] : 0.f);
         }
     }
 }

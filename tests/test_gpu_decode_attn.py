@@ -32,7 +32,7 @@ def test_latents(mk, no, heads, kv_rank, rot_dim):  # noqa: F811
 
 @pytest.mark.parametrize("heads,kv_heads", [(16, 16), (8, 4), (5, 5)])
 def test_shares_of_several_tiles(mk, no, heads, kv_heads):  # noqa: F811
-    """Windows so wide, over so many key heads, that a CTA's share of the keys is more than a tile: 74 tiles in shares of 3, 1 and 1."""
+    """Windows so wide, over so many key heads, that a CTA's share of the keys is more than a tile: 72 tiles and more in shares of up to 3, 2 and 2."""
     cfg = no.model_config([no.att(heads=heads, kv_heads=kv_heads, dim=16, vdim=12, size=None)] * 2, width=48, vocab=97)
     m, W = mk(cfg, seed=heads, chunk=200, context=2300)
     toks = tokens_for(cfg, 240, 6)
