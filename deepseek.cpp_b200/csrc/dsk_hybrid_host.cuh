@@ -1140,9 +1140,12 @@ static int launches_per_token(const dsk_model* m) {
 // ---------------------------------------------------------------------------------------------------------------------
 // state
 // ---------------------------------------------------------------------------------------------------------------------
-// Asks for a piece of the state's memory; *p is set by salloc_all.
+// Asks for a piece of the state's memory; *p is set by salloc_all.  A piece of 1 MB and more takes whole pages of 2 MB, as an allocation of its own does: with all pieces
+// packed at 512 bytes, decoded tokens of two designs took 0.6 and 1.7 % longer (where caches, states and rows lie, not what is done with them).
+constexpr size_t kStatePage = (size_t)2 << 20;
 static int salloc(State* S, void** p, size_t bytes, bool portion = false) {
-  S->pieces.push_back({p, (std::max<size_t>(bytes, 16) + 511) / 512 * 512, portion});
+  const size_t unit = bytes >= kStatePage / 2 ? kStatePage : 512;
+  S->pieces.push_back({p, (std::max<size_t>(bytes, 16) + unit - 1) / unit * unit, portion});
   return 0;
 }
 // All pieces in one allocation (an allocation and a zeroing for each of 30 to 50 pieces were most of the time that a state took to make and to free), zeroed.
@@ -1155,6 +1158,7 @@ static int salloc_all(State* S, cudaStream_t st) {
     CK(cudaMalloc((void**)&S->arena, total()));
   }
   CK(cudaMemsetAsync(S->arena, 0, total(), st));
+  std::stable_partition(S->pieces.begin(), S->pieces.end(), [](const State::Piece& q) { return q.bytes % kStatePage == 0; });   // pages first
   char* at = S->arena;
   for (const State::Piece& q : S->pieces) { *q.at = q.bytes ? at : nullptr; at += q.bytes; }
   return cudaStreamSynchronize(st) == cudaSuccess ? 0 : -2;
