@@ -1,13 +1,13 @@
 #!/usr/bin/env python
-"""bench.py — single-batch DeepSeek decode throughput on B200 (BASELINE.json metric).
+"""bench.py — single-batch DeepSeek decode throughput on B200.
 
   python bench.py --gpus N --steps K --warmup W            # this engine (libdsk.so), one rank per GPU
   python bench.py --impl reference --gpus N --steps K ...   # the reference's own CPU path (oracle/_ref)
 
-Workload (every N): DeepSeek-V2 236B shapes, Q2_K, all 60 layers (BASELINE.json configs[3]; 77 GB of weights — fits ONE
-B200, so N = 1, 2, 4, 8 is a legitimate strong-scaling curve of the model north_star says to shard).  The V2-Lite
-configs[1] / configs[2] numbers of round 1 are measured in the same run at N = 1 and reported under `secondary`.
-`--workload v3 --quant q2_k --gpus 8` times the north-star target (220 GB, needs >= 2 GPUs).
+Workload (every N): DeepSeek-V2 236B shapes, Q2_K, all 60 layers (77 GB of weights — fits ONE
+B200, so N = 1, 2, 4, 8 is a legitimate strong-scaling curve of a model to shard).  The V2-Lite
+numbers (F8 and K-quants) are measured in the same run at N = 1 and reported under `secondary`.
+`--workload v3 --quant q2_k --gpus 8` times the largest model (220 GB, needs >= 2 GPUs).
 
 A "step" is one fixed 128-token greedy completion (the reference's `-n 128 -t 0`, src/main.cpp:324-335) after a
 16-token prompt has hydrated the KV cache.  `value` is decode-only tok/s with everything resident in HBM (the token loop
@@ -35,7 +35,7 @@ sys.path.insert(0, os.path.join(REPO, "deepseek.cpp_b200"))
 GEN_TOKENS = 128
 PROMPT_LEN = 16
 
-# shapes: HF configs of the DeepSeek family; K-quants need 256-multiples
+# shapes: HF configs of the DeepSeek family ; K-quants need 256-multiples
 WORKLOADS = {
     "v2lite": dict(arch="DeepseekV2ForCausalLM", dim=2048, hidden_dim=10944, n_layers=27, n_heads=16, vocab_size=102400,
                    qk_nope_head_dim=128, qk_rope_head_dim=64, v_head_dim=128, kv_lora_rank=512, q_lora_rank=0,
@@ -126,7 +126,7 @@ def make_config(dsk, w):
 
 
 def mint_on_gpu(dsk, w, rank, n_ranks, device):
-    """Random-init weights of the named architecture, generated on the GPU (SURVEY §8(d) / N1)."""
+    """Random-init weights of the named architecture, generated on the GPU."""
     import zlib
 
     import torch
@@ -721,7 +721,7 @@ def main():
                                      "completion (the e2e region launches it once per token: steps x 128)",
                 "roofline": roof, "clocks": R["clocks"], "sharded_check": R["sharded_check"], "resident_gb": R["resident_gb"],
                 "sample_tokens": R["tokens"]})
-    # ---- secondary: the V2-Lite configs of BASELINE.json (round-1 headline), same run, N = 1 only ---------------------
+    # ---- secondary: the V2-Lite models, same run, N = 1 only ---------------------
     if world == 1 and not a.no_secondary and a.workload != "v2lite" and not a.n_layers:
         sec = {}
         for sq in ("f8e5m2", "q2_k"):

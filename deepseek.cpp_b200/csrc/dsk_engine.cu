@@ -117,7 +117,7 @@ struct Layer {
   __half *kcache = nullptr, *vcache = nullptr;
 };
 
-// Host->device weight upload pipeline (SURVEY N1): the .dseek payload is an mmap of pageable memory, so a plain cudaMemcpy
+// Host->device weight upload pipeline: the .dseek payload is an mmap of pageable memory, so a plain cudaMemcpy
 // stages every tensor synchronously through the driver's bounce buffer.  Here two pinned staging buffers alternate: while
 // chunk i travels over PCIe (cudaMemcpy2DAsync on the upload stream, which also re-pitches rows), the host thread copies
 // chunk i+1 out of the page cache.  dsk_model_finalize() joins the stream.
@@ -730,7 +730,7 @@ extern "C" int dsk_model_sharding(const dsk_model* m, int* tensor_parallel, int*
   return 0;
 }
 
-// Algorithmic weight bytes per decoded token (SURVEY §8(d)): sum over executed GEMVs of rows*cols*bpw,
+// Algorithmic weight bytes per decoded token: sum over executed GEMVs of rows*cols*bpw,
 // bpw = 4 / 2 / 1+4/(bs0*bs1) / 84/256 / 110/256, plus the F32 gate, gate bias and norm weights.
 extern "C" double dsk_model_active_bytes_per_token(const dsk_model* m) {
   if (!m) return 0;

@@ -1437,9 +1437,11 @@ static void timeline_report(State* S, int T) {
 }
 
 // Launches a kernel as a programmatic dependent of the one ahead of it in the stream: it is set up, and runs up to its grid_wait, while
-// that one still runs.  Only in short steps (chain_step): their kernels take a few microseconds, about what a launch takes (a decoded token 10 -
-// 15 % less, 45 tokens 436 -> 359 us).  In long ones the waiting CTAs take the places that the running kernel leaves, not one per SM: a
-// 600-token step in fp32, whose products are about one CTA per SM, went from 1.88 to 2.56 ms.  plain_next: the coming launch waits
+// that one still runs.  Only in short steps (chain_step): their kernels take a few microseconds, about what a launch takes.  bf16, six models of two or three
+// layers (widths 1024 and 2048), with against without: 5 tokens 15 - 18 % less, 45 tokens 11 - 17, 100 tokens 11 - 17, 256 tokens 6 - 13, and from
+// there on not in all of them (400 and 512 tokens 0 to 14 % less, 1024 tokens 10 % less to 5 % more): 256 is the line.  fp32: up to 4 tokens 10 - 15 %
+// less; 5 to 45 tokens 3 - 7 % less, 100 tokens 5 % less to 8 % more, 600 tokens 36 % more (1.88 to 2.56 ms: its products are about one CTA per SM, and waiting
+// CTAs take the places that the running kernel leaves): 4 is the line.  plain_next: the coming launch waits
 // as usual (it joins another stream).
 static thread_local bool chain_step = false, plain_next = false;
 template <typename... KA> struct Launch {

@@ -1,7 +1,6 @@
 // dsk_kernels.cuh — shared device helpers of the sm_100a decode path (async-copy / mbarrier wrappers, quant traits,
 // activation layouts) plus the two upload/fallback utility kernels.  The decode path itself is the persistent interpreter
-// in dsk_mega.cuh; the first-generation per-stage kernels that used to live here were removed in round 2 so that every
-// C-ABI test hook exercises the code that produces the benchmark numbers.
+// in dsk_mega.cuh; every C-ABI test hook runs it too, the code that produces the benchmark numbers.
 #pragma once
 
 #include <cuda_fp16.h>

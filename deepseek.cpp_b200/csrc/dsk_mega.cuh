@@ -95,7 +95,7 @@ struct Program {
   // multi-GPU, peer-memory mode: every rank stores its MoE partial sums straight into every peer's exchange buffer over
   // NVLink (plain stores to IPC-mapped memory), then raises a flag there; an ST_XCHG stage waits for the N flags and adds the
   // N partials in rank order — no kernel boundary, no NCCL call on the token path
-  int n_ranks, rank, n_xchg, tp;           // tp: tensor-parallel program (heads / FFN slices / LM-head rows sharded, see DESIGN §7)
+  int n_ranks, rank, n_xchg, tp;           // tp: tensor-parallel program (heads / FFN slices / LM-head rows sharded)
   float* xchg_peer[kMaxRanks];             // [2][n_ranks][dim] buffer of rank q (q == rank: the local one)
   unsigned* xflag_peer[kMaxRanks];         // n_ranks flags of rank q: flag[r] = sequence number of rank r's last finished store
   float* logits_peer[kMaxRanks];           // tp: full-vocabulary logits of rank q (every rank stores its rows into every copy)
@@ -238,7 +238,7 @@ __device__ __noinline__ void q8_block_nf(float4 va, float4 vb, int b, int8_t* q_
   const uint32_t p1 = (qv[4] & 0xff) | ((qv[5] & 0xff) << 8) | ((qv[6] & 0xff) << 16) | ((uint32_t)(qv[7] & 0xff) << 24);
   *reinterpret_cast<uint2*>(q.qs + (b << 8) + lane * 8) = make_uint2(p0, p1);
 }
-// out-of-line on purpose: one copy for every staging site (instruction-cache footprint; see DESIGN.md)
+// out-of-line on purpose: one copy for every staging site (instruction-cache footprint)
 __device__ __forceinline__ void q8_block(const float (&v)[8], int b, int lane, const Q8Smem& q) {
   (void)lane;
   q8_block_nf(make_float4(v[0], v[1], v[2], v[3]), make_float4(v[4], v[5], v[6], v[7]), b, q.qs, q.d, q.bsums);
@@ -650,7 +650,7 @@ __device__ __forceinline__ int my_tile_count(int n) { return (int)blockIdx.x < n
 //   * the reference's K x "arg-max with strict >, lowest index wins ties" selection picks, in order, the experts of RANK
 //     0..K-1 where rank(j) = #{j' selectable : x[j'] > x[j] or (x[j'] == x[j] and j' < j)} — every thread counts its own rank;
 //   * GROUP_LIMITED_GREEDY first keeps, inside each group, the topk_group best experts with x > 0 (the reference compares
-//     the first candidate against x[-1], which is 0.0f in its heap layout: SURVEY §8 A7) — the same rank inside the group;
+//     the first candidate against x[-1], which is 0.0f in its heap layout) — the same rank inside the group;
 //   * wsum is accumulated in selection order like the reference (only when norm_topk_prob).
 // `publish` (CTA 0) also writes the state buffers.  A slot with no selectable expert left (the reference then indexes
 // x[-1] / mask[-1]: UB) gets expert -1 and weight 0.

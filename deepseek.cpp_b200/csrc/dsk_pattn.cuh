@@ -395,9 +395,10 @@ __global__ void __launch_bounds__(256, 1) pattn(const __grid_constant__ PattnP P
 // fp32 products of many rows (fp32 models; the score and value products of attention with mixed heads) on the tensor cores: both operands split
 // into three bf16 parts on their way into shared memory, six products per element as in pattn.  128 x 64 tile, 32 deep; 8 warps as 4 (rows) x 2
 // (columns), a 32 x 32 warp tile; the next slice's fp32 values are in registers during this one's products.  Interface, row maps, expert tiles,
-// batches and epilogues of GemmP.  Bound: the six mma.sync per element.  A kernel of 64 x 64 tiles was bound by the fp32 pipe, with routed products of four
-// rows per expert too (1.58 ms a step of 33 tokens with it, 1.57 with this; 16 rows: 1.17 and 1.10): a step in fp32 at width 1024 went from 1.85 to 1.22 ms (600 tokens), from 0.95 to 0.67 (64 tokens) and from 0.89 to 0.64
-// (5 tokens), a 1500-token prompt with mixed heads from 2.98 to 2.67 ms; the error against 64 bits of the first from 1.0e-6 to 5e-7.
+// batches and epilogues of GemmP.  Bound: the six mma.sync per element.  FMA on 64 x 64 tiles, before, was bound by the fp32 pipe: a step in fp32 at
+// width 1024 went from 1.85 to 1.22 ms (600 tokens), from 0.95 to 0.67 (64 tokens) and from 0.89 to 0.64 (5 tokens), a 1500-token prompt with mixed
+// heads from 2.98 to 2.67 ms, fp32 routed products of two layers with 16 experts of which 2 from 1.17 to 1.10 (33 tokens, 4 rows an expert) and from 1.40 to 1.28
+// (340, 42 rows).  Error of the first against 64 bits, attention in three parts included: 1.0e-6 before, 3.1e-7.
 // ---------------------------------------------------------------------------------------------------------------------
 // The same sum as a chain of FMAs over the numbers themselves, for a result that is not finite: an infinite operand has no three parts (what is left
 // of it is inf - inf), nor has a finite one that rounds to an infinity in bf16 (from 2^128 - 2^119).  Such operands make every result that they enter

@@ -3,12 +3,13 @@
 //
 // One CTA per SM walks output tiles of 128 rows x bn columns (bn = 32 .. 256, picked by the host for the grid it gives).  Warp 0 copies
 // 64-deep slices of both operands into a ring of shared memory (128-byte swizzle), one thread of warp 1 issues the products, warps 2 - 5 read
-// the finished accumulators (two in TMEM: a tile's epilogue runs under the next tile's products), turn them through shared memory so
-// that a warp stores whole 128-byte lines, and apply the epilogue.
+// the finished accumulators (two in TMEM: a tile's epilogue runs under the next tile's products), apply the epilogue and store: a lane its own
+// row in 32-byte pieces, ragged blocks turned through shared memory.
 // The activations are rounded to bf16 (as gemm_mma rounds them while staging) and, in routed products, put into expert order by one
 // pass ahead of the product (bf16_rows), or by the epilogue of the product that made them (TcP::C16): every column tile then reads half
 // the bytes, by TMA, instead of gathering and converting fp32 rows again.
-// Bound: the 48 KB per 64-deep slice that a 128 x 256 tile takes from L2.
+// Bound: not established.  A 64-deep slice of a 128 x 256 tile takes about 1250 cycles, of which the tensor pipe is busy 570; L2 runs at 8 to 17 % of its
+// rate, and two thirds of the bytes a slice (pairs of CTAs on a tile) took the same time.
 #pragma once
 
 #include <cuda.h>   // CUtensorMap

@@ -236,7 +236,7 @@ int dsk_device_info(char* name128, int* sm_count, size_t* hbm_bytes);
 
 /* ---- model: replaces Model::Model weight binding (src/model.cpp:756-871) + device upload -------- */
 /* rank/n_ranks: shard placement, decided here so that dsk_upload_tensor() can keep only this rank's slices.
- * Routed expert e lives on rank e / ceil(E/n_ranks) (SURVEY §8(e)).  With n_ranks > 1 and peer memory (default; DSK_TP=0 or
+ * Routed expert e lives on rank e / ceil(E/n_ranks).  With n_ranks > 1 and peer memory (default; DSK_TP=0 or
  * DSK_P2P=0 switch it off) the model is also TENSOR PARALLEL: attention heads (wq/wq_b/wkv_b rows, wo columns, KV cache),
  * the hidden units of the shared experts and of the dense FFN layers (256-blocks) and the LM-head rows are split across
  * the ranks; wq_a / wkv_a / the gate / norms / embedding stay replicated.  Requires n_heads % n_ranks == 0 and
@@ -255,13 +255,13 @@ void dsk_model_destroy(dsk_model* m);
  * checked by byte count, everything else by the exact 4-slot shape (unused slots 0).  Host payloads travel
  * through a pinned double buffer with asynchronous copies (the call returns once the last chunk is staged;
  * dsk_model_finalize() joins the pipeline).  `src_on_device` != 0 means `data` is already a device pointer
- * (GPU-side minting, SURVEY N1). */
+ * (GPU-side minting). */
 int dsk_upload_tensor(dsk_model* m, const char* name, int dtype, const int64_t shape[4], const void* data,
                       size_t nbytes, int src_on_device);
 /* Checks every tensor the config requires is present (check_tensor, src/model.cpp:129-136). */
 int dsk_model_finalize(dsk_model* m);
 /* Bytes of weights resident on this GPU / algorithmic weight bytes streamed per decoded token
- * (SURVEY §8(d); replaces Model::active_bytes, src/model.cpp:885-901, which under-counts). */
+ * (replaces Model::active_bytes, src/model.cpp:885-901, which under-counts). */
 size_t dsk_model_resident_bytes(const dsk_model* m);
 double dsk_model_active_bytes_per_token(const dsk_model* m);
 
@@ -322,7 +322,7 @@ int dsk_launches_per_forward(const dsk_model* m, int mode);
 int dsk_sample(dsk_model* m, dsk_state* s, float temperature, float top_p, float coin, int* token);
 int dsk_sample_prob(dsk_model* m, dsk_state* s, int index, float* prob);
 
-/* ---- multi-GPU (SURVEY §8(e)) ---------------------------------------------------------------------------
+/* ---- multi-GPU ---------------------------------------------------------------------------
  * The reference has no distributed path.  Expert-only sharding has one real exchange step per MoE layer (the MoE partial
  * sum); the tensor-parallel model adds one after the wo projection of every layer (partial sums of the column-sharded wo),
  * one after the dense FFN layers, and one arg-max / logits exchange per token.  All of them run INSIDE the persistent

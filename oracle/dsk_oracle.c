@@ -361,7 +361,7 @@ static float sigmoidf(float x) { return 1.0f / (1.0f + expf(-x)); } /* src/infer
 
 /* moe_gate: src/infer.cpp:493-599.
  * GROUP_LIMITED_GREEDY first pass (551-566): `best` starts at -1 and the test is `x[j] > x[best]`, i.e. it reads
- * x[-1] (UB).  For the reference's `new float[]` buffer that word is 0.0f (SURVEY §8 A7), so the rule is
+ * x[-1] (UB).  For the reference's `new float[]` buffer that word is 0.0f, so the rule is
  * "the first unmasked j is accepted iff x[j] > 0".  Restated with an explicit 0.0f; if no candidate is found
  * (all remaining scores <= 0) nothing is marked for that (group, k) — the reference would index mask[-1]. */
 void ork_moe_gate(float* moe_weights, const float* bias, int* active_experts, float* x, int n_routed, int n_active,

@@ -2,7 +2,7 @@
 
 TEST INFRASTRUCTURE.  No real DeepSeek weights exist in this environment (no network), so every
 checkpoint is synthetic: weights N(0,1)/sqrt(fan_in), embedding N(0,1), norm weights 1+0.1 N(0,1),
-gate N(0,1)/sqrt(dim)*gate_gain, V3 gate bias 0.01 N(0,1), quantised exactly the way
+gate N(0,1)/sqrt(dim)*gate_gain, V3 gate bias 0.01 N(0,1) quantised exactly the way
 /root/reference/convert.py does:
   * fp16: cast;  * f8e5m2: per 128x128 block scale=57344/amax, RNE cast, stored scale=1/scale
     (convert.py:216-275);  * q2_k/q3_k: the reference's own quantize_row_q{2,3}_K_ref through
@@ -43,7 +43,7 @@ PRESETS = {
                     n_routed_experts=16, n_active_routed=4, moe_intermediate_size=256, routed_scaling_factor=2.5,
                     n_group=4, topk_group=2, norm_topk_prob=True, scoring_func="sigmoid",
                     topk_method="group_limited_greedy"),
-    # the real V2-Lite shapes (K-quants need the 1408->1536 / 10944->11008 zero padding, SURVEY §0.2)
+    # the real V2-Lite shapes (K-quants need the 1408->1536 / 10944->11008 zero padding)
     "v2lite": dict(arch="DeepseekV2ForCausalLM", dim=2048, hidden_dim=10944, n_layers=27, n_heads=16,
                    vocab_size=102400, max_seq_len=1024, qk_nope_head_dim=128, qk_rope_head_dim=64, v_head_dim=128,
                    kv_lora_rank=512, q_lora_rank=0, first_k_dense_replace=1, n_shared_experts=2,
@@ -86,7 +86,7 @@ def kquant_rows(w: np.ndarray, quant: str, fast: bool, rng: np.random.Generator)
         w = np.ascontiguousarray(w, dtype=np.float32)
         L.ref_quantize_rows(O._fp(w), O._vp(out), rows, cols, 1 if quant == "q3_k" else 0)
         return out
-    # random valid blocks: any byte pattern with finite fp16 d/dmin is a valid block (SURVEY §7)
+    # random valid blocks: any byte pattern with finite fp16 d/dmin is a valid block
     out[:] = rng.integers(0, 256, size=out.shape, dtype=np.uint8)
     blk = out.reshape(rows, cols // 256, bb)
     scale = np.float16(1.0 / np.sqrt(cols) / 6.0)

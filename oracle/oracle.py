@@ -6,8 +6,7 @@ never from the product (deepseek.cpp_b200/).
   RefLib   -> oracle/_ref/libdsref.so : the UNMODIFIED reference compiled from /root/reference (ref_shim.cpp)
   PortLib  -> oracle/libdsk_oracle.so : the plain-C restatement (dsk_oracle.c)
 
-`/root/reference` is never read at run time: libdsref.so is prebuilt in the build container and
-travels to the GPU box with the repo snapshot.
+`/root/reference` is never read at run time: libdsref.so is built ahead of it.
 """
 from __future__ import annotations
 

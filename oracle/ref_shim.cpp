@@ -4,8 +4,7 @@
 // /root/reference/src.  It textually includes the reference's infer.cpp so that its
 // file-static kernels (matmul, moe_gate, rmsnorm, rope, ...) are reachable, and is
 // compiled with -fno-access-control so Model::_copy_embedding (private) can be driven.
-// Built by oracle/Makefile into oracle/_ref/libdsref.so (git-ignored; travels to the
-// GPU box with gpurun).  No reference source is copied into this repository.
+// Built by oracle/Makefile into oracle/_ref/libdsref.so (git-ignored).  No reference source is copied into this repository.
 //
 // Every wrapper names the reference symbol (file:line @ 8db9e56) it forwards to.
 
@@ -77,7 +76,7 @@ void ref_softmax(float* o, float* x, int size) { softmax(o, x, size); }
 // moe_gate src/infer.cpp:493-599.  `x` (E floats) is modified in place like the reference.
 // The GROUP_LIMITED_GREEDY branch reads x[-1] (infer.cpp:558, UB); callers must pass a
 // pointer whose preceding float is 0.0f to reproduce the value the reference sees for
-// its `new float[]` buffer (SURVEY §8 A7) — ref_moe_gate_padded below does that.
+// its `new float[]` buffer — ref_moe_gate_padded below does that.
 void ref_moe_gate(float* moe_weights, float* bias, int* active_experts, float* x, int n_routed, int n_active,
                   int norm_topk_prob, float routed_scaling_factor, int scoring_sigmoid, int topk_method,
                   int n_group, int topk_group) {
