@@ -160,6 +160,7 @@ struct State {
   int *h_tok = nullptr, *h_want = nullptr;   // pinned staging of a chunk's token ids / wanted rows (behind dsk_state::h_ctrl, with h_err)
   // attention of portions in one kernel (pattn): split keys and values of the visible positions, queries it takes at a time
   __nv_bfloat16 *k16 = nullptr, *v16 = nullptr;
+  float* ppart = nullptr;                    // partial softmax results of shares of the keys: up to 148 CTAs of 128 rows (launches that fill the chip are not split)
   int pattn_q = 0;
   // bf16 products of portions: activations rounded for the product that follows, hidden rows of a feed-forward, and a host word that a wait
   // which gave up sets
@@ -1318,13 +1319,14 @@ static dsk_state* state_create(dsk_model* m) {
       return (size_t)std::min<long long>((long long)sp.att_window - 1, (long long)c.max_seq_len) + std::min<size_t>(Tc, q) + (sp.mixer == DSK_MIX_GQA ? sp.att_keep_first : 0);
     };
     // layers that run pattn: the visible keys and values split into bf16 parts, behind the up-projected fp32 rows of latent layers
-    size_t k16 = 0, v16 = 0, kup = 0, vup = 0, rows = 0;
+    size_t k16 = 0, v16 = 0, kup = 0, vup = 0, rows = 0, shares = 0;
     auto fused_bytes = [&](int q) {
       k16 = v16 = kup = vup = 0;
       for (const HLayer& L : M->L) {
         if (!takes_pattn(L.sp, bf16)) continue;
         const PattnSize z = pattn_size(L.sp, bf16);
         const size_t n = visible(L.sp, q);
+        shares = std::max<size_t>(shares, (size_t)148 * 128 * (z.V + 2) / (z.Vp / (z.VN * 8)));
         k16 = std::max(k16, n * z.G * z.Dp * z.parts); v16 = std::max(v16, n * z.G * z.Vp * z.parts);
         if (L.sp.mixer != DSK_MIX_GQA) { kup = std::max(kup, n * z.G * L.sp.att_dim); vup = std::max(vup, n * z.G * z.V); }
       }
@@ -1357,7 +1359,7 @@ static dsk_state* state_create(dsk_model* m) {
     for (const HLayer& L : M->L) if (has_attn(L.sp)) rows = std::max(rows, visible(L.sp, takes_pattn(L.sp, bf16) ? S->pattn_q : S->talk_q));
     if (rows > 0 && fused <= kPortionBytes + kPortionBytes / 2 && plain <= kPortionBytes) {
       S->prefill_keys = (int)rows;
-      if (k16) rc |= salloc(S, (void**)&S->k16, k16 * 2, true) | salloc(S, (void**)&S->v16, v16 * 2, true);
+      if (k16) rc |= salloc(S, (void**)&S->ppart, shares * 4, true) | salloc(S, (void**)&S->k16, k16 * 2, true) | salloc(S, (void**)&S->v16, v16 * 2, true);
       rc |= salloc(S, (void**)&S->kf, std::max(kup, keys * hd) * 4, true) | salloc(S, (void**)&S->vf, std::max(vup, keys * hv) * 4, true);
       rc |= salloc(S, (void**)&S->d_rows, rows * 4, true);
       if (pack_es) rc |= salloc(S, &S->kb, keys * hd * pack_es, true) | salloc(S, &S->vt, keys * hv * pack_es, true);
@@ -1845,15 +1847,27 @@ static void portion_attn(State* S, const PattnSize& z, PackP K, PattnP A, cudaSt
   A.kb = S->k16; A.vb = S->v16; A.G = z.G; A.D = z.D; A.Dp = z.Dp; A.V = z.V; A.Vp = z.Vp; A.Lk = K.Lk; A.nk = K.nk; A.first = K.first; A.mods.keep = K.keep;
   if (z.parts == 1) launch_next(pattn_pack<1>, K.Lk, 256, 0, st)(K);
   else launch_next(pattn_pack<3>, K.Lk, 256, 0, st)(K);
-  // 16 query rows per warp: eight warps, with tiles of 16 keys where 32 do not fit (deep heads: a head of 192 leaves room for four warps with
-  // 32 keys or eight with 16), fewer where that leaves SMs idle (a warp's share of a tile's copy grows)
+  // 16 query rows per warp, a CTA an SM, tiles of 16 keys where 32 do not fit.  Four warps are one on each of an SM's tensor cores: a tile of keys takes them as long as it takes two, and
+  // eight twice as long.  Where that leaves SMs idle, the keys are cut into shares of at least four tiles, one CTA each, and latent_swa_merge joins them.  What costs
+  // least rounds x warps x tiles is taken (8 warps and few shares where even: half the copying per row).  Two layers of width 2048, 16 heads of 128, behind 8000 keys, steps of
+  // 32 / 128 / 256 / 512 tokens take 0.68 / 0.84 / 2.4 / 5.1 ms; with warps halved until the SMs had a CTA each they took 4.3 / 5.0 / 6.1 / 13.4, as products between which scores lie in
+  // memory 2.2 / 3.1 / 4.5 / 9.3
   const int zc = z.Vp / (z.VN * 8);
-  int w = 8, nk = 4;
-  auto fits = [&] { return pattn_smem(z.parts, w, z.Dp, z.VN, nk) <= (size_t)kPattnSmemMax; };
-  if (!fits()) nk = 2;
-  while (w > 2 && (!fits() || (long long)((A.T + 16 * w - 1) / (16 * w)) * A.H * zc < 148)) w /= 2;
-  if (nk == 2) { nk = 4; if (!fits()) nk = 2; }
-  const dim3 grid((unsigned)A.H, (unsigned)((A.T + 16 * w - 1) / (16 * w)), (unsigned)zc);
+  int w = 0, nk = 0;
+  A.NS = 1;
+  long long best = 0;
+  for (int cw = 8; cw >= 2; cw /= 2) {
+    const int ck = pattn_smem(z.parts, cw, z.Dp, z.VN, 4) <= (size_t)kPattnSmemMax ? 4 : 2;
+    if (pattn_smem(z.parts, cw, z.Dp, z.VN, ck) > (size_t)kPattnSmemMax) continue;
+    const long long ctas = (long long)((A.T + 16 * cw - 1) / (16 * cw)) * A.H * zc, tiles = (std::min<long long>(K.Lk, (long long)A.span + 16 * cw) + 8 * ck - 1) / (8 * ck);
+    const long long most = std::max<long long>(1, std::min({148 / ctas, tiles / 4, (long long)kAttnSplitMax}));
+    for (long long ns = 1; ns <= most; ns += std::max<long long>(1, most - 1)) {   // (joining shares takes about as long as a tile)
+      const long long cost = (ctas * ns + 147) / 148 * std::max(cw, 4) * ((tiles + ns - 1) / ns + (ns > 1)) * ck;
+      if (!w || cost < best) { best = cost; w = cw; nk = ck; A.NS = (int)ns; }
+    }
+  }
+  A.part = S->ppart;
+  const dim3 grid((unsigned)A.H, (unsigned)((A.T + 16 * w - 1) / (16 * w)), (unsigned)(zc * A.NS));
   const size_t smem = pattn_smem(z.parts, w, z.Dp, z.VN, nk);
 #define DSK_PATTN(A_, B_) do { if (nk == 4) launch_next(pattn<A_, B_, 4>, grid, 32 * w, smem, st)(A); else launch_next(pattn<A_, B_, 2>, grid, 32 * w, smem, st)(A); } while (0)
   if (z.parts == 1 && z.VN == 8) DSK_PATTN(1, 8);
@@ -1861,6 +1875,10 @@ static void portion_attn(State* S, const PattnSize& z, PackP K, PattnP A, cudaSt
   else if (z.VN == 8) DSK_PATTN(3, 8);
   else DSK_PATTN(3, 16);
 #undef DSK_PATTN
+  if (A.NS > 1) {
+    launch_next(latent_swa_merge, dim3((unsigned)(A.T * A.H), (unsigned)((A.V + 127) / 128)), 128, 0, st)(S->ppart, A.out, A.V, A.NS, A.gate, A.ld_gate, A.H, A.gate_head, A.ld_out, A.alpha);
+    S->launches++;
+  }
   S->launches += 2;
 }
 

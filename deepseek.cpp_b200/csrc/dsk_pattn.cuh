@@ -8,7 +8,7 @@
 // larger than that of the fp32 products it replaces.  PARTS = 1: operands rounded to bf16 (latent attention of bf16 models, whose products
 // always took them so).
 // pattn_pack splits the visible keys and values once per step; a CTA (16 query rows per warp) streams them in tiles of 32 or 16 through two
-// buffers (cp.async).  Bound: issue slots - six products per element, their operands from shared memory, softmax.  Before, a block of 256
+// buffers (cp.async); where the query blocks of all heads are fewer than the SMs, shares of the keys are CTAs of their own.  Bound: issue slots - six products per element, their operands from shared memory, softmax.  Before, a block of 256
 // queries wrote its scores, read them for the softmax and again for the values, all three in kernels of their own on the fp32 pipe.
 #pragma once
 
@@ -71,7 +71,8 @@ struct PattnP {
   const __nv_bfloat16 *kb, *vb;  // (pattn_pack)
   float* out;                    // token t, head h at out + t * ld_out + h * V
   const float* gate;             // (see gqa_attn)
-  int T, H, G, D, Dp, V, Vp, ldq, ld_out, ld_gate, gate_head, Lk, nk, first, pos0, mask, span;
+  float* part;                   // NS > 1: results of a share of the keys (see latent_swa_merge)
+  int T, H, G, D, Dp, V, Vp, ldq, ld_out, ld_gate, gate_head, Lk, nk, first, pos0, mask, span, NS;
   float scale, alpha;
   ScoreMods mods;
 };
@@ -140,10 +141,25 @@ __device__ __forceinline__ float joined(const __nv_bfloat16* x, size_t part) {  
   for (int i = PARTS - 2; i >= 0; i--) v += __bfloat162float(x[i * part]);
   return v;
 }
+// The key tiles (KT keys) that a CTA with queries q0 .. q0 + BM - 1 meets: those of the kept keys, then from the first key of its first query to its last query.  Share `s` of
+// NS has the tiles begin .. end - 1 of them.
+struct KeyTiles { int kept, t0, begin, end; };
+__device__ __forceinline__ KeyTiles key_tiles(const PattnP& P, int q0, int BM, int KT, int s) {
+  const int last = min(P.T, q0 + BM) - 1;
+  const int lo_v = P.nk + mask_first(P.mask, P.span, P.pos0 + q0) - P.first, hi_v = P.nk + P.pos0 + last - P.first;
+  KeyTiles k;
+  k.kept = (min(P.mods.keep, hi_v + 1) + KT - 1) / KT;   // (kept positions are keys 0 .. keep - 1 whether or not they lie in the range)
+  k.t0 = max(k.kept, lo_v / KT);
+  const int n = k.kept + max(0, hi_v / KT - k.t0 + 1), per = (n + P.NS - 1) / P.NS;
+  k.begin = s * per;
+  k.end = min(n, k.begin + per);
+  return k;
+}
+__device__ __forceinline__ int tile_key(const KeyTiles& k, int i, int KT) { return (i < k.kept ? i : k.t0 + i - k.kept) * KT; }
 // Query t of head h again, by one warp and from its visible keys alone, into columns v0 .. v0 + VN * 8 - 1 of the output: for rows whose result is not
 // finite.  In the products of a tile a key out of sight has the weight 0, and 0 x Inf is NaN; an infinity times the parts of a number is NaN.
-template <int PARTS, int VN>
-__device__ __noinline__ void pattn_row(const PattnP& P, int t, int h, int v0) {
+template <int PARTS, int VN, int KT>
+__device__ __noinline__ void pattn_row(const PattnP& P, int t, int h, int v0, KeyTiles tiles, int share) {
   constexpr int CL = VN / 4;           // columns per lane
   const int lane = threadIdx.x & 31, g = h / (P.H / P.G), pos = P.pos0 + t, lo = mask_first(P.mask, P.span, pos), last = P.nk + pos - P.first;
   const float* q = P.q + (size_t)t * P.ldq + (size_t)h * P.D;
@@ -151,9 +167,9 @@ __device__ __noinline__ void pattn_row(const PattnP& P, int t, int h, int v0) {
   float m = -1e30f, l = 0.f, acc[CL];
 #pragma unroll
   for (int k = 0; k < CL; k++) acc[k] = 0.f;
-  for (int j0 = 0; j0 <= last && !isnan(l); j0 += 32) {
-    const int v = j0 + lane, p = v < P.nk ? v : P.first + v - P.nk;
-    const bool ok = v <= last && (p < P.mods.keep || p >= lo);
+  for (int i = tiles.begin; i < tiles.end && !isnan(l); i++) {
+    const int j0 = tile_key(tiles, i, KT), v = j0 + lane, p = v < P.nk ? v : P.first + v - P.nk;
+    const bool ok = lane < KT && v <= last && (p < P.mods.keep || p >= lo);
     if (!__any_sync(0xffffffffu, ok)) continue;
     float s = 0.f;
     if (ok) {
@@ -167,7 +183,7 @@ __device__ __noinline__ void pattn_row(const PattnP& P, int t, int h, int v0) {
     m = m_new;
 #pragma unroll
     for (int k = 0; k < CL; k++) acc[k] *= c;
-    for (int jj = 0; jj < 32; jj++) {
+    for (int jj = 0; jj < KT; jj++) {
       const float pj = __shfl_sync(0xffffffffu, pr, jj);
       if (pj == 0.f) continue;
       const __nv_bfloat16* vr = P.vb + ((size_t)g * P.Lk + j0 + jj) * P.Vp + v0 + lane;
@@ -176,22 +192,26 @@ __device__ __noinline__ void pattn_row(const PattnP& P, int t, int h, int v0) {
     }
   }
   float f = 1.f;
-  if (P.mods.sink) {
+  if (P.mods.sink && share == 0) {
     const float sk = P.mods.sink[h], m_new = fmaxf(m, sk);
     f = expf(m - m_new);
     l = l * f + expf(sk - m_new);
+    m = m_new;
   }
   const float inv = f / l * P.alpha;
+  float* pp = P.part + (((size_t)t * P.H + h) * P.NS + share) * (P.V + 2);
+  if (P.NS > 1 && v0 == 0 && lane == 0) { pp[0] = m; pp[1] = l; }
 #pragma unroll
   for (int k = 0; k < CL; k++) {
     const int c = v0 + lane + 32 * k;
     if (c >= P.V) continue;
+    if (P.NS > 1) { pp[2 + c] = acc[k] * f; continue; }
     const float gt = P.gate ? sigmoid_f(P.gate[(size_t)t * P.ld_gate + (P.gate_head ? (size_t)h : (size_t)h * P.V + c)]) : 1.f;
     P.out[(size_t)t * P.ld_out + (size_t)h * P.V + c] = acc[k] * inv * gt;
   }
 }
 
-template <int PARTS, int VN, int NK>   // VN: 8-column groups of values in a CTA (blockIdx.z picks the columns)
+template <int PARTS, int VN, int NK>   // VN: 8-column groups of values in a CTA (blockIdx.z picks the columns and the share of the keys)
 __global__ void __launch_bounds__(256, 1) pattn(const __grid_constant__ PattnP P) {
   constexpr int KT = NK * 8;                                           // keys of a tile
   extern __shared__ __align__(16) unsigned char pa_raw[];
@@ -202,7 +222,8 @@ __global__ void __launch_bounds__(256, 1) pattn(const __grid_constant__ PattnP P
   const uint32_t kpart = (uint32_t)(KT * pq * 2), vpart = (uint32_t)(KT * pvt * 2), buf = PARTS * (kpart + vpart);
   const uint32_t ks0 = qs + PARTS * qpart;
   const int qb = (int)gridDim.y - 1 - (int)blockIdx.y, q0 = qb * BM;   // late queries, which see most keys, first for every head
-  const int h = blockIdx.x, g = h / (P.H / P.G), v0 = (int)blockIdx.z * VN * 8;
+  const int zc = (int)gridDim.z / P.NS, share = (int)blockIdx.z / zc;
+  const int h = blockIdx.x, g = h / (P.H / P.G), v0 = ((int)blockIdx.z - share * zc) * VN * 8;
   grid_enter();
   // query rows, split
   for (int e = threadIdx.x; e < BM * (Dp / 4); e += nthr) {
@@ -217,15 +238,10 @@ __global__ void __launch_bounds__(256, 1) pattn(const __grid_constant__ PattnP P
       *reinterpret_cast<uint2*>(pa_raw + i * qpart + (size_t)(r * pq + c) * 2) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
     }
   }
-  // tiles this CTA meets: those of the kept keys, then from the first key of its first query to its last query
-  const int last = min(P.T, q0 + BM) - 1;
-  const int lo_v = P.nk + mask_first(P.mask, P.span, P.pos0 + q0) - P.first, hi_v = P.nk + P.pos0 + last - P.first;
-  // (kept positions are keys 0 .. keep - 1 whether or not they lie in the range)
-  const int kept = (min(P.mods.keep, hi_v + 1) + KT - 1) / KT, t0 = max(kept, lo_v / KT), n_tiles = kept + max(0, hi_v / KT - t0 + 1);
-  auto tile_key = [&](int i) { return (i < kept ? i : t0 + i - kept) * KT; };
+  const KeyTiles tiles = key_tiles(P, q0, BM, KT, share);
   const int chunks = Dp / 8 + VN;
   auto fetch = [&](int i) {   // a warp copies rows (part, key) warp, warp + warps, ..: a lane per 16 bytes of the key row and the value row
-    const int key0 = tile_key(i);
+    const int key0 = tile_key(tiles, i, KT);
     const uint32_t kd = ks0 + (uint32_t)(i & 1) * buf, vd = kd + PARTS * kpart;
     for (int r = warp; r < PARTS * KT; r += nthr >> 5) {
       const int part = r / KT, j = r - part * KT, v = key0 + j;
@@ -241,7 +257,7 @@ __global__ void __launch_bounds__(256, 1) pattn(const __grid_constant__ PattnP P
     }
     cp_async_commit();
   };
-  if (n_tiles > 0) fetch(0);
+  if (tiles.begin < tiles.end) fetch(tiles.begin);
   const int row_lo = q0 + warp * 16 + (lane >> 2);                      // this thread's query rows: row_lo and row_lo + 8
   const int first_lo[2] = {mask_first(P.mask, P.span, P.pos0 + row_lo), mask_first(P.mask, P.span, P.pos0 + row_lo + 8)};
   // a tile whose keys every query of the warp sees needs no mask
@@ -254,10 +270,10 @@ __global__ void __launch_bounds__(256, 1) pattn(const __grid_constant__ PattnP P
 #pragma unroll
     for (int i = 0; i < 4; i++) o[n][i] = 0.f;
   const uint32_t qa = qs + (uint32_t)((warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * pq + (lane >> 4) * 8) * 2;
-  for (int it = 0; it < n_tiles; it++) {
+  for (int it = tiles.begin; it < tiles.end; it++) {
     cp_async_wait<0>();
     __syncthreads();                                                     // tile it is there; everyone is through tile it - 1
-    if (it + 1 < n_tiles) fetch(it + 1);
+    if (it + 1 < tiles.end) fetch(it + 1);
     const uint32_t kt = ks0 + (uint32_t)(it & 1) * buf, vt = kt + PARTS * kpart;
     float s[NK][4];
 #pragma unroll
@@ -280,7 +296,7 @@ __global__ void __launch_bounds__(256, 1) pattn(const __grid_constant__ PattnP P
       });
     }
     // scale, cap, bias and mask: rows row_lo (entries 0, 1) and row_lo + 8 (entries 2, 3); keys n * 8 + (lane & 3) * 2 + {0, 1}
-    const int key0 = tile_key(it);
+    const int key0 = tile_key(tiles, it, KT);
 #pragma unroll
     for (int n = 0; n < NK; n++)
 #pragma unroll
@@ -369,25 +385,29 @@ __global__ void __launch_bounds__(256, 1) pattn(const __grid_constant__ PattnP P
     const int t = row_lo + r * 8;
     if (t >= P.T || ((again >> ((lane >> 2) + 8 * r)) & 1u)) continue;
     float f = 1.f;
-    if (P.mods.sink) {   // a key with a zero value vector
+    if (P.mods.sink && share == 0) {   // a key with a zero value vector
       const float sk = P.mods.sink[h], m_new = fmaxf(m[r], sk);
       f = expf(m[r] - m_new);
       l[r] = l[r] * f + expf(sk - m_new);
+      m[r] = m_new;
     }
     const float inv = f / l[r] * P.alpha;
+    float* pp = P.part + (((size_t)t * P.H + h) * P.NS + share) * (P.V + 2);
+    if (P.NS > 1 && v0 == 0 && (lane & 3) == 0) { pp[0] = m[r]; pp[1] = l[r]; }
 #pragma unroll
     for (int n = 0; n < VN; n++)
 #pragma unroll
       for (int i = 0; i < 2; i++) {
         const int c = v0 + n * 8 + (lane & 3) * 2 + i;
         if (c >= P.V) continue;
+        if (P.NS > 1) { pp[2 + c] = o[n][r * 2 + i] * f; continue; }
         const float gt = P.gate ? sigmoid_f(P.gate[(size_t)t * P.ld_gate + (P.gate_head ? (size_t)h : (size_t)h * P.V + c)]) : 1.f;
         P.out[(size_t)t * P.ld_out + (size_t)h * P.V + c] = o[n][r * 2 + i] * inv * gt;
       }
   }
   for (; again; again &= again - 1) {
     const int t = q0 + warp * 16 + __ffs(again) - 1;
-    if (t < P.T) pattn_row<PARTS, VN>(P, t, h, v0);
+    if (t < P.T) pattn_row<PARTS, VN, KT>(P, t, h, v0, tiles, share);
   }
 }
 

@@ -149,3 +149,20 @@ def test_routed_rows(mk, mk_hybrid, no, ho, router):  # noqa: F811
             t[at] = 50
             m.reset()
             assert ahead_of_the_poison(m, run, cfg, W, t, at, sizes) < F32_TOL
+
+
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+@pytest.mark.parametrize("kind", ["grouped", "own_keys", "deep_latent"])
+def test_shares_of_the_keys(mk, no, kind, value):  # noqa: F811
+    """The same where a portion's keys are cut into shares: rows ahead of the token take part in its share too."""
+    layer = {"grouped": lambda: no.att(heads=4, kv_heads=2, dim=12, vdim=10, size=None), "own_keys": lambda: no.att(heads=2, kv_heads=2, dim=16, vdim=70, size=200, conv=1),
+             "deep_latent": lambda: no.lat(heads=2, kv_rank=30, rot_dim=6)}[kind]
+    cfg = no.model_config([layer(), layer()], width=48, vocab=97)
+    m, W = mk(cfg, seed=4, chunk=300, context=700, edit=lambda W: poisoned(W, value, 90))
+    toks = tokens_for(cfg, 560, 5)
+    toks[toks == 90] = 7
+    for at in (420, 500, 558):
+        t = toks.copy()
+        t[at] = 90
+        m.reset()
+        assert ahead_of_the_poison(m, no.run, cfg, W, t, at, [300, 100, 160]) < F32_TOL

@@ -50,3 +50,35 @@ def test_last_block_of_one_query(mk_sakusun, so):  # noqa: F811
     m, W = mk_sakusun(cfg, seed=2, chunk=300)
     toks = tokens_for(cfg, 290, 8)
     assert rel(in_portions(m, toks, [257, 33]), so.run(cfg, W, toks)[0]) < F32_TOL
+
+
+# Steps whose query blocks are fewer than the SMs: the keys behind them in shares (of at least four tiles of 32 or 16), joined afterwards; windows that
+# cut the shares, several column groups, a depth that takes tiles of 16, kept positions, sinks, a cap and distance biases, gates
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,size", [(2, 1, 12, 10, None), (3, 3, 64, 150, 300), (1, 1, 320, 24, None), (5, 5, 16, 64, 130)])
+def test_shares_of_the_keys(mk, no, heads, kv_heads, dim, vdim, size):  # noqa: F811
+    cfg = no.model_config([no.att(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, size=size)] * 2, width=48, vocab=97)
+    m, W = mk(cfg, seed=heads + dim, chunk=400, context=1200)
+    toks = tokens_for(cfg, 1000, 8)
+    exp = no.run(cfg, W, toks)[0]
+    for sizes in ([400, 400, 200], [399, 33, 100, 32, 130, 306]):
+        assert rel(in_portions(m, toks, sizes), exp) < F32_TOL
+
+
+def test_shares_of_latents(mk, no):  # noqa: F811
+    cfg = no.model_config([no.lat(heads=3, dim=40, rot_dim=8, vdim=129), no.lat(heads=2, dim=16, vdim=16)], width=40, vocab=97)
+    toks = tokens_for(cfg, 800, 9)
+    for quant in ("fp32", "bf16"):
+        m, W = mk(cfg, seed=3, chunk=400, quant=quant, context=900)
+        exp = no.run(cfg, W, toks)[0]
+        got = in_portions(m, toks, [350, 40, 400, 10])
+        assert rel(got, exp) < F32_TOL if quant == "fp32" else close_bf16(got, exp, no.rounding_noise(cfg, W, toks))
+
+
+def test_shares_with_kept_positions(mk_sakusun, so):  # noqa: F811
+    cfg = so.model_config([so.att(heads=4, kv_heads=2, dim=8, vdim=8, size=450, keep_first=70, bias_max=200, rel_rows=12, ff=12),
+                           so.att(heads=2, dim=8, vdim=70, size=None, softcap=None, v_mix=False, ff=None)], width=40, vocab=97)
+    m, W = mk_sakusun(cfg, seed=3, chunk=256, context=1000)
+    toks = tokens_for(cfg, 900, 8)
+    exp = so.run(cfg, W, toks)[0]
+    for sizes in ([256, 256, 256, 132], [250, 250, 40, 33, 256]):
+        assert rel(in_portions(m, toks, sizes), exp) < F32_TOL
