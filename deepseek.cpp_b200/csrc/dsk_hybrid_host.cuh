@@ -2640,7 +2640,8 @@ static int forward_chunk(dsk_model* m, dsk_state* s, const int32_t* tokens, int 
   }
   CK(cudaStreamSynchronize(s->stream));
   CK(cudaGetLastError());
-  if (*(volatile int*)S->h_err) { const int e = *S->h_err; *S->h_err = 0; return fail(-2, e == 2 ? "a product's tensor map was refused" : "a wait inside a matrix product gave up"); }
+  // (a step that lacks a product has gone into caches and recurrences: the sequence is not to be continued)
+  if (*(volatile int*)S->h_err) { const int e = *S->h_err; *S->h_err = 0; S->next_pos = -1; return fail(-2, e == 2 ? "a product's tensor map was refused" : "a wait inside a matrix product gave up"); }
   S->next_pos = pos0 + n;
   s->last_pos = pos0 + n - 1;
   s->have_logits = n_want > 0 && want[n_want - 1] == n - 1;
