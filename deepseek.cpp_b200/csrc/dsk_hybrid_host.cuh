@@ -2599,7 +2599,7 @@ static int forward_chunk(dsk_model* m, dsk_state* s, const int32_t* tokens, int 
   const dsk_hybrid_config& c = M->c;
   if (n <= 0) return fail(-4, "empty chunk");
   if (pos0 == 0) { if (state_reset(s)) return -2; }
-  else if (pos0 != S->next_pos) return fail(-4, "chunk starts at position %d but the state's sequence is at %d (recurrent state cannot be rewound; position 0 starts a new sequence)", pos0, S->next_pos);
+  else if (pos0 < 0 || pos0 != S->next_pos) return fail(-4, "chunk starts at position %d but the state's sequence is at %d (recurrent state cannot be rewound; position 0 starts a new sequence)", pos0, S->next_pos);
   for (int i = 0; i < n; i++) if (tokens[i] < 0 || tokens[i] >= c.vocab_size) return fail(-4, "token %d out of range", tokens[i]);
   for (int i = 0; i < n_want; i++) if (want[i] < 0 || want[i] >= n || (i && want[i] <= want[i - 1])) return fail(-4, "wanted rows must be ascending indices into the chunk");
   for (const HLayer& L : M->L)   // a ring cache shortened to max_seq_len holds no position beyond it
@@ -2654,7 +2654,7 @@ static int decode_greedy(dsk_model* m, dsk_state* s, int start_pos, int n_steps,
   Model* M = m->hy;
   State* S = s->hy;
   const dsk_hybrid_config& c = M->c;
-  if (start_pos != S->next_pos) return fail(-4, "dsk_decode_greedy: start_pos %d must follow the state's sequence (at %d)", start_pos, S->next_pos);
+  if (start_pos < 0 || start_pos != S->next_pos) return fail(-4, "dsk_decode_greedy: start_pos %d must follow the state's sequence (at %d)", start_pos, S->next_pos);
   const int one = 0;
   CK(cudaMemcpyAsync(S->d_want, &one, 4, cudaMemcpyHostToDevice, s->stream));
   launch_next(set_ctl, 1, 1, 0, s->stream)(S->d_ctl, start_pos);
