@@ -408,7 +408,8 @@ static void set_kernel_attrs() {
   DSK_LSCAN_ATTR(8, 1, 2); DSK_LSCAN_ATTR(16, 1, 2); DSK_LSCAN_ATTR(32, 1, 2); DSK_LSCAN_ATTR(8, 1, 4); DSK_LSCAN_ATTR(16, 1, 4); DSK_LSCAN_ATTR(32, 1, 4); DSK_LSCAN_ATTR(32, 2, 4);
 #undef DSK_LSCAN_ATTR
   cudaFuncSetAttribute(gemm_mma<HEPI_SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMmaSmem);
-#define DSK_PATTN_ATTR(A, B) cudaFuncSetAttribute(pattn<A, B, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax); cudaFuncSetAttribute(pattn<A, B, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax)
+#define DSK_PATTN_ATTR(A, B) cudaFuncSetAttribute(pattn<A, B, 4, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax); cudaFuncSetAttribute(pattn<A, B, 2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax); \
+  cudaFuncSetAttribute(pattn<A, B, 4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax); cudaFuncSetAttribute(pattn<A, B, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax)
   DSK_PATTN_ATTR(1, 8); DSK_PATTN_ATTR(1, 16); DSK_PATTN_ATTR(3, 8); DSK_PATTN_ATTR(3, 16);
 #undef DSK_PATTN_ATTR
 #define DSK_SPLIT_ATTR(E) cudaFuncSetAttribute(gemm_split<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem)
@@ -1847,11 +1848,11 @@ static void portion_attn(State* S, const PattnSize& z, PackP K, PattnP A, cudaSt
   A.kb = S->k16; A.vb = S->v16; A.G = z.G; A.D = z.D; A.Dp = z.Dp; A.V = z.V; A.Vp = z.Vp; A.Lk = K.Lk; A.nk = K.nk; A.first = K.first; A.mods.keep = K.keep;
   if (z.parts == 1) launch_next(pattn_pack<1>, K.Lk, 256, 0, st)(K);
   else launch_next(pattn_pack<3>, K.Lk, 256, 0, st)(K);
-  // 16 query rows per warp, a CTA an SM, tiles of 16 keys where 32 do not fit.  Four warps are one on each of an SM's tensor cores: a tile of keys takes them as long as it takes two, and
-  // eight twice as long.  Where that leaves SMs idle, the keys are cut into shares of at least four tiles, one CTA each, and latent_swa_merge joins them.  What costs
-  // least rounds x warps x tiles is taken (8 warps and few shares where even: half the copying per row).  Two layers of width 2048, 16 heads of 128, behind 8000 keys, steps of
-  // 32 / 128 / 256 / 512 tokens take 0.68 / 0.84 / 2.4 / 5.1 ms; with warps halved until the SMs had a CTA each they took 4.3 / 5.0 / 6.1 / 13.4, as products between which scores lie in
-  // memory 2.2 / 3.1 / 4.5 / 9.3
+  // 16 query rows per warp, a CTA an SM, tiles of 16 keys where 32 do not fit.  Four warps are one on each of an SM's tensor cores; with eight a tile of keys takes about 1.2 times
+  // as long (two a core hide one another's waits, and more threads copy the tile), with two 1.4 times.  Where the query blocks leave SMs idle, the keys are cut into shares of
+  // at least four tiles, one CTA each, and latent_swa_merge joins them.  What costs least, rounds of CTAs x time of a tile x tiles, is taken.  Two layers of width 2048, 16 heads of 128, behind
+  // 8000 keys, steps of 32 / 128 / 256 / 512 tokens take 0.68 / 0.83 / 1.6 / 3.3 ms; with warps halved until the SMs had a CTA each they took 4.3 / 5.0 / 6.1 / 13.4, as products between
+  // which scores lie in memory 2.2 / 3.1 / 4.5 / 9.3
   const int zc = z.Vp / (z.VN * 8);
   int w = 0, nk = 0;
   A.NS = 1;
@@ -1862,14 +1863,15 @@ static void portion_attn(State* S, const PattnSize& z, PackP K, PattnP A, cudaSt
     const long long ctas = (long long)((A.T + 16 * cw - 1) / (16 * cw)) * A.H * zc, tiles = (std::min<long long>(K.Lk, (long long)A.span + 16 * cw) + 8 * ck - 1) / (8 * ck);
     const long long most = std::max<long long>(1, std::min({148 / ctas, tiles / 4, (long long)kAttnSplitMax}));
     for (long long ns = 1; ns <= most; ns += std::max<long long>(1, most - 1)) {   // (joining shares takes about as long as a tile)
-      const long long cost = (ctas * ns + 147) / 148 * std::max(cw, 4) * ((tiles + ns - 1) / ns + (ns > 1)) * ck;
+      const long long cost = (ctas * ns + 147) / 148 * (cw == 8 ? 6 : cw == 4 ? 5 : 7) * ((tiles + ns - 1) / ns + (ns > 1)) * ck;
       if (!w || cost < best) { best = cost; w = cw; nk = ck; A.NS = (int)ns; }
     }
   }
   A.part = S->ppart;
   const dim3 grid((unsigned)A.H, (unsigned)((A.T + 16 * w - 1) / (16 * w)), (unsigned)(zc * A.NS));
   const size_t smem = pattn_smem(z.parts, w, z.Dp, z.VN, nk);
-#define DSK_PATTN(A_, B_) do { if (nk == 4) launch_next(pattn<A_, B_, 4>, grid, 32 * w, smem, st)(A); else launch_next(pattn<A_, B_, 2>, grid, 32 * w, smem, st)(A); } while (0)
+  auto run = [&](auto* k4, auto* k2) { launch_next(nk == 4 ? k4 : k2, grid, 32 * w, smem, st)(A); };
+#define DSK_PATTN(A_, B_) do { if (A.NS > 1) run(pattn<A_, B_, 4, true>, pattn<A_, B_, 2, true>); else run(pattn<A_, B_, 4, false>, pattn<A_, B_, 2, false>); } while (0)
   if (z.parts == 1 && z.VN == 8) DSK_PATTN(1, 8);
   else if (z.parts == 1) DSK_PATTN(1, 16);
   else if (z.VN == 8) DSK_PATTN(3, 8);

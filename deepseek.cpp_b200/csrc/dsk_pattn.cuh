@@ -144,13 +144,13 @@ __device__ __forceinline__ float joined(const __nv_bfloat16* x, size_t part) {  
 // The key tiles (KT keys) that a CTA with queries q0 .. q0 + BM - 1 meets: those of the kept keys, then from the first key of its first query to its last query.  Share `s` of
 // NS has the tiles begin .. end - 1 of them.
 struct KeyTiles { int kept, t0, begin, end; };
-__device__ __forceinline__ KeyTiles key_tiles(const PattnP& P, int q0, int BM, int KT, int s) {
+__device__ __forceinline__ KeyTiles key_tiles(const PattnP& P, int q0, int BM, int KT, int s, int NS) {
   const int last = min(P.T, q0 + BM) - 1;
   const int lo_v = P.nk + mask_first(P.mask, P.span, P.pos0 + q0) - P.first, hi_v = P.nk + P.pos0 + last - P.first;
   KeyTiles k;
   k.kept = (min(P.mods.keep, hi_v + 1) + KT - 1) / KT;   // (kept positions are keys 0 .. keep - 1 whether or not they lie in the range)
   k.t0 = max(k.kept, lo_v / KT);
-  const int n = k.kept + max(0, hi_v / KT - k.t0 + 1), per = (n + P.NS - 1) / P.NS;
+  const int n = k.kept + max(0, hi_v / KT - k.t0 + 1), per = (n + NS - 1) / NS;
   k.begin = s * per;
   k.end = min(n, k.begin + per);
   return k;
@@ -158,7 +158,7 @@ __device__ __forceinline__ KeyTiles key_tiles(const PattnP& P, int q0, int BM, i
 __device__ __forceinline__ int tile_key(const KeyTiles& k, int i, int KT) { return (i < k.kept ? i : k.t0 + i - k.kept) * KT; }
 // Query t of head h again, by one warp and from its visible keys alone, into columns v0 .. v0 + VN * 8 - 1 of the output: for rows whose result is not
 // finite.  In the products of a tile a key out of sight has the weight 0, and 0 x Inf is NaN; an infinity times the parts of a number is NaN.
-template <int PARTS, int VN, int KT>
+template <int PARTS, int VN, int KT, bool SHARES>
 __device__ __noinline__ void pattn_row(const PattnP& P, int t, int h, int v0, KeyTiles tiles, int share) {
   constexpr int CL = VN / 4;           // columns per lane
   const int lane = threadIdx.x & 31, g = h / (P.H / P.G), pos = P.pos0 + t, lo = mask_first(P.mask, P.span, pos), last = P.nk + pos - P.first;
@@ -199,19 +199,20 @@ __device__ __noinline__ void pattn_row(const PattnP& P, int t, int h, int v0, Ke
     m = m_new;
   }
   const float inv = f / l * P.alpha;
-  float* pp = P.part + (((size_t)t * P.H + h) * P.NS + share) * (P.V + 2);
-  if (P.NS > 1 && v0 == 0 && lane == 0) { pp[0] = m; pp[1] = l; }
+  float* pp = SHARES ? P.part + (((size_t)t * P.H + h) * P.NS + share) * (P.V + 2) : nullptr;
+  if (SHARES && v0 == 0 && lane == 0) { pp[0] = m; pp[1] = l; }
 #pragma unroll
   for (int k = 0; k < CL; k++) {
     const int c = v0 + lane + 32 * k;
     if (c >= P.V) continue;
-    if (P.NS > 1) { pp[2 + c] = acc[k] * f; continue; }
+    if (SHARES) { pp[2 + c] = acc[k] * f; continue; }
     const float gt = P.gate ? sigmoid_f(P.gate[(size_t)t * P.ld_gate + (P.gate_head ? (size_t)h : (size_t)h * P.V + c)]) : 1.f;
     P.out[(size_t)t * P.ld_out + (size_t)h * P.V + c] = acc[k] * inv * gt;
   }
 }
 
-template <int PARTS, int VN, int NK>   // VN: 8-column groups of values in a CTA (blockIdx.z picks the columns and the share of the keys)
+// VN: 8-column groups of values in a CTA (blockIdx.z picks the columns and, with SHARES, the share of the keys: a form of its own, prompts that fill the chip ran 3 % longer on one for both)
+template <int PARTS, int VN, int NK, bool SHARES>
 __global__ void __launch_bounds__(256, 1) pattn(const __grid_constant__ PattnP P) {
   constexpr int KT = NK * 8;                                           // keys of a tile
   extern __shared__ __align__(16) unsigned char pa_raw[];
@@ -222,7 +223,7 @@ __global__ void __launch_bounds__(256, 1) pattn(const __grid_constant__ PattnP P
   const uint32_t kpart = (uint32_t)(KT * pq * 2), vpart = (uint32_t)(KT * pvt * 2), buf = PARTS * (kpart + vpart);
   const uint32_t ks0 = qs + PARTS * qpart;
   const int qb = (int)gridDim.y - 1 - (int)blockIdx.y, q0 = qb * BM;   // late queries, which see most keys, first for every head
-  const int zc = (int)gridDim.z / P.NS, share = (int)blockIdx.z / zc;
+  const int zc = SHARES ? (int)gridDim.z / P.NS : 1, share = SHARES ? (int)blockIdx.z / zc : 0;
   const int h = blockIdx.x, g = h / (P.H / P.G), v0 = ((int)blockIdx.z - share * zc) * VN * 8;
   grid_enter();
   // query rows, split
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(256, 1) pattn(const __grid_constant__ PattnP P
       *reinterpret_cast<uint2*>(pa_raw + i * qpart + (size_t)(r * pq + c) * 2) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
     }
   }
-  const KeyTiles tiles = key_tiles(P, q0, BM, KT, share);
+  const KeyTiles tiles = key_tiles(P, q0, BM, KT, share, SHARES ? P.NS : 1);
   const int chunks = Dp / 8 + VN;
   auto fetch = [&](int i) {   // a warp copies rows (part, key) warp, warp + warps, ..: a lane per 16 bytes of the key row and the value row
     const int key0 = tile_key(tiles, i, KT);
@@ -392,22 +393,22 @@ __global__ void __launch_bounds__(256, 1) pattn(const __grid_constant__ PattnP P
       m[r] = m_new;
     }
     const float inv = f / l[r] * P.alpha;
-    float* pp = P.part + (((size_t)t * P.H + h) * P.NS + share) * (P.V + 2);
-    if (P.NS > 1 && v0 == 0 && (lane & 3) == 0) { pp[0] = m[r]; pp[1] = l[r]; }
+    float* pp = SHARES ? P.part + (((size_t)t * P.H + h) * P.NS + share) * (P.V + 2) : nullptr;
+    if (SHARES && v0 == 0 && (lane & 3) == 0) { pp[0] = m[r]; pp[1] = l[r]; }
 #pragma unroll
     for (int n = 0; n < VN; n++)
 #pragma unroll
       for (int i = 0; i < 2; i++) {
         const int c = v0 + n * 8 + (lane & 3) * 2 + i;
         if (c >= P.V) continue;
-        if (P.NS > 1) { pp[2 + c] = o[n][r * 2 + i] * f; continue; }
+        if (SHARES) { pp[2 + c] = o[n][r * 2 + i] * f; continue; }
         const float gt = P.gate ? sigmoid_f(P.gate[(size_t)t * P.ld_gate + (P.gate_head ? (size_t)h : (size_t)h * P.V + c)]) : 1.f;
         P.out[(size_t)t * P.ld_out + (size_t)h * P.V + c] = o[n][r * 2 + i] * inv * gt;
       }
   }
   for (; again; again &= again - 1) {
     const int t = q0 + warp * 16 + __ffs(again) - 1;
-    if (t < P.T) pattn_row<PARTS, VN, KT>(P, t, h, v0, tiles, share);
+    if (t < P.T) pattn_row<PARTS, VN, KT, SHARES>(P, t, h, v0, tiles, share);
   }
 }
 
