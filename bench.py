@@ -11,7 +11,8 @@ numbers (F8 and K-quants) are measured in the same run at N = 1 and reported und
 
 A "step" is one fixed 128-token greedy completion (the reference's `-n 128 -t 0`, src/main.cpp:324-335) after a
 16-token prompt has hydrated the KV cache.  `value` is decode-only tok/s with everything resident in HBM (the token loop
-runs inside ONE persistent kernel launch per completion, device arg-max feeding the next token, CUDA-event timed); `e2e`
+is one captured graph a token, or ONE persistent kernel launch per completion on several GPUs; device arg-max feeding the next
+token, CUDA-event timed); `e2e`
 is the same completion driven through the reference-shaped host call `dsk_forward(token, pos, OUTPUT_LOGITS, host_logits)`
 per token: control words go host->device, the vocab-sized logits come device->host, and the host samples (argmax) — copies
 inside the timed region.  Weights are synthetic (no checkpoints exist offline): N(0,1)/sqrt(fan_in) quantised like
@@ -521,7 +522,7 @@ def measure(dsk, torch, dist, w, rank, world, local_rank, steps, warmup, want_e2
         if rank == 0:
             print(timeline, file=sys.stderr, flush=True)
 
-    # ---- value: device-resident decode, CUDA events inside dsk_decode_greedy (one persistent launch per completion) ----
+    # ---- value: device-resident decode, CUDA events inside dsk_decode_greedy ----
     for _ in range(warmup):
         hydrate()
         m.decode_greedy(PROMPT_LEN, GEN_TOKENS)
@@ -705,19 +706,21 @@ def main():
         kern["note"] = "ONE interpreter GEMV stage per launch (decode_kernel<Q>, production tile plan); launch overhead included"
     except Exception as e:
         kern = {"error": str(e)[:120]}
-    traffic, capture = committed_traffic(a.workload, a.quant) if world == 1 and not a.n_layers and not a.mla else (None, None)
+    chain = R["launches_per_forward"] > 1 and world == 1   # a token as launches, or a completion as one
+    traffic, capture = (None, None) if chain else committed_traffic(a.workload, a.quant) if world == 1 and not a.n_layers and not a.mla else (None, None)
     roof = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
             "traffic_unit": "bytes per token (= per launch / tokens per launch), ncu capture in profiles/", "traffic_capture": capture,
-            "kernel": "decode_kernel<Q> (a whole completion is one launch; achieved = algorithmic bytes/token x tok/s / N_gpus, i.e. every "
-                      "barrier, staging phase and attention is charged to the GEMV stream)",
+            "kernel": ("dk_gemv and the other launches of a token" if chain else "decode_kernel<Q> (a whole completion is one launch)") +
+                      ": achieved = algorithmic bytes/token x tok/s / N_gpus, i.e. every barrier or launch, staging phase and attention is charged to the GEMV stream",
             "algorithmic_bytes_per_token": abytes, "peak_source": peak_src, "isolated_stages": kern}
 
     out = dict(base)
     vocab = w["vocab_size"]
     out.update({"value": value, "ms_per_step": R["dev_ms"] / a.steps, "wall_s": R["wall"],
                 "e2e": {"value": R["e2e"], "unit": "tok/s", "h2d_bytes_per_step": GEN_TOKENS * 48, "d2h_bytes_per_step": GEN_TOKENS * vocab * 4},
-                "gpu_launches": a.steps * R["launches_per_forward"],
-                "gpu_launches_note": "decode_kernel launches inside the timed region of `value`: one persistent cooperative launch per 128-token "
+                "gpu_launches": a.steps * R["launches_per_forward"] * (GEN_TOKENS if chain else 1),
+                "gpu_launches_note": "dk_* launches inside the timed region of `value` (a captured chain a token)" if chain else
+                                     "decode_kernel launches inside the timed region of `value`: one persistent cooperative launch per 128-token "
                                      "completion (the e2e region launches it once per token: steps x 128)",
                 "roofline": roof, "clocks": R["clocks"], "sharded_check": R["sharded_check"], "resident_gb": R["resident_gb"],
                 "sample_tokens": R["tokens"]})

@@ -26,8 +26,10 @@
 #include <vector>
 
 #include <algorithm>
+#include <array>
 #include "dsk_kernels.cuh"
 #include "dsk_mega.cuh"
+#include "dsk_decode.cuh"
 #include "dsk_hybrid.cuh"
 #include "dsk_linattn.cuh"
 #include "dsk_tc5.cuh"
@@ -113,7 +115,7 @@ struct Layer {
   DTensor wq, wq_a, wq_b, wkv_a, wkv_b, wo, w1, w2, w3, sw1, sw2, sw3;
   DTensor wc, wq_rope_b, wv_b;   // true-MLA blocks (use_mla): absorbed query projection, rope query projection, per-head value up-projection
   float *gate = nullptr, *gate_bias = nullptr;
-  bool is_moe = false;
+  bool is_moe = false, gate_tiled = false;
   __half *kcache = nullptr, *vcache = nullptr;
 };
 
@@ -128,17 +130,27 @@ struct Uploader {
   cudaStream_t st = nullptr;
   int cur = 0;
   std::vector<void*> staging;   // device staging buffers (Q3_K repack), freed at finalize
+  void* raw = nullptr;          // rows as the file has them, on their way into tiles (reused: copies and kernels of the stream follow one another)
+  size_t raw_cap = 0;
   size_t bytes = 0;
   double seconds = 0;
 };
 
 namespace hyb { struct Model; struct State; }   // layer-list model family (dsk_hybrid_host.cuh)
+namespace dk {                                  // token chain of one GPU (dsk_decode_host.cuh)
+struct Plan;
+static bool fits(const dsk_config& c, int n_ranks);
+static int set_attributes();
+static int tile(int quant, const unsigned char* src, uint8_t* dst, int rows, int cols, int count, cudaStream_t st, bool wait);
+static int tile_router(dsk_model* m, const float* src, float** dst);
+}
 
 struct dsk_model {
   dsk_config c;
   hyb::Model* hy = nullptr;    // set: a layer-list model; the DeepSeek fields below are unused
   int head_dim = 0;
   int rank = 0, n_ranks = 1;
+  bool chain = false;          // tokens run as the launches of dsk_decode.cuh; matrices lie in its tiles
   int expert_first = 0, expert_count = 0;
   std::vector<Layer> layers;
   DTensor embed, wcls;
@@ -202,6 +214,7 @@ struct dsk_state {
   int n_xchg = 0;                       // in-kernel exchanges per token (peer-memory mode)
   std::vector<int> xchg_before;         // exchanges preceding stage i within a token (size n_stages + 1)
   int n_tail = 1;                       // stages after the last layer (LM head [+ arg-max exchange]): skipped by HYDRATE_KV_CACHE
+  dk::Plan* chain = nullptr;            // set: what runs the tokens; the program above is planned (its limits hold) but not run
   float* logits_src = nullptr;          // where the full logits of the last forward live (tp: the exchange allocation)
 };
 
@@ -246,8 +259,8 @@ static bool g_coop_small = false, g_kq_small = true;   // DSK_COOP_SMALL=1 / DSK
 // (cooperative tiles for one-tile-per-CTA F8 stages won 2 us per stage in isolation but lose overall: their code is one more
 //  cold path per layer — 393 vs 408 tok/s)
 static bool g_use_mma = true;   // F8E5M2 tiles through mma.sync (DSK_NO_MMA=1: CUDA-core dequant path)
-enum { ENG_MEGA = 0, ENG_STAGE = 1 };
-static int g_engine = ENG_MEGA;
+enum { ENG_CHAIN = 0, ENG_MEGA = 1, ENG_STAGE = 2 };   // DSK_ENGINE=mega / stage: the interpreter also for models that the chain fits
+static int g_engine = ENG_CHAIN;
 
 typedef void (*DecodeKernel)(const Program*, int, int, int, int);
 static DecodeKernel decode_kernel_for(int quant) {
@@ -281,9 +294,10 @@ extern "C" int dsk_init(int device) {
     g_use_mma = getenv("DSK_NO_MMA") == nullptr;
     if (const char* e = getenv("DSK_COOP_SMALL")) g_coop_small = atoi(e) != 0;
     if (const char* e = getenv("DSK_KQ_SMALL")) g_kq_small = atoi(e) != 0;
-    if (const char* en = getenv("DSK_ENGINE")) g_engine = !strcmp(en, "stage") ? ENG_STAGE : ENG_MEGA;
+    if (const char* en = getenv("DSK_ENGINE")) g_engine = !strcmp(en, "stage") ? ENG_STAGE : !strcmp(en, "mega") ? ENG_MEGA : ENG_CHAIN;
     for (int q = DSK_F32; q <= DSK_Q3_K; q++)
       CK(cudaFuncSetAttribute(decode_kernel_for(q), cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax - 1024));
+    if (dk::set_attributes()) return -2;
     g_attrs_set = true;
   }
   return 0;
@@ -369,6 +383,7 @@ extern "C" dsk_model* dsk_model_create(const dsk_config* cfg, int rank, int n_ra
   m->head_dim = cfg->qk_nope_head_dim + cfg->qk_rope_head_dim;
   m->rank = rank;
   m->n_ranks = n_ranks;
+  m->chain = g_engine == ENG_CHAIN && (g_use_mma || cfg->quant != DSK_F8E5M2) && dk::fits(*cfg, n_ranks);
   const int E = cfg->n_routed_experts;
   const int per = E > 0 ? cdiv(E, n_ranks) : 0;
   m->expert_first = std::min(E, rank * per);
@@ -425,6 +440,8 @@ static void uploader_release(Uploader& u) {
   if (u.st) cudaStreamSynchronize(u.st);
   for (void* p : u.staging) cudaFree(p);
   u.staging.clear();
+  cudaFree(u.raw);
+  u.raw = nullptr; u.raw_cap = 0;
   for (int i = 0; i < 2; i++) {
     if (u.pin[i]) { cudaFreeHost(u.pin[i]); u.pin[i] = nullptr; }
     if (u.ev[i]) { cudaEventDestroy(u.ev[i]); u.ev[i] = nullptr; }
@@ -584,6 +601,23 @@ static int upload_weight(dsk_model* m, DTensor& t, int rows, int cols, bool expe
   t.cols = cc;
   t.row_bytes = vrb;
   t.expert_bytes = vrb * rc;
+  if (m->chain) {   // rows as the file has them -> tiles (dsk_decode.cuh); one GPU: the whole tensor
+    t.expert_bytes = dk_matrix_bytes(q, rc, cc);
+    if (dmalloc(m, (void**)&t.w, t.expert_bytes * count)) return -2;
+    const unsigned char* dsrc = (const unsigned char*)data;
+    if (!on_dev || (uintptr_t)data % 16) {
+      if (m->up.raw_cap < tot) {
+        if (m->up.st) CK(cudaStreamSynchronize(m->up.st));
+        cudaFree(m->up.raw);
+        m->up.raw = nullptr; m->up.raw_cap = 0;
+        CK(cudaMalloc(&m->up.raw, tot));
+        m->up.raw_cap = tot;
+      }
+      if (copy_rows(m, m->up.raw, tot, data, tot, tot, 1, on_dev)) return -2;
+      dsrc = (const unsigned char*)m->up.raw;
+    }
+    return dk::tile(q, dsrc, t.w, rc, cc, count, on_dev ? nullptr : m->up.st, on_dev);
+  }
   const size_t nrows_loc = (size_t)rc * count;
   const size_t local_disk = drb_loc * nrows_loc, local_dev = vrb * nrows_loc;
   if (dmalloc(m, (void**)&t.w, local_dev + 16)) return -2;
@@ -711,6 +745,16 @@ extern "C" int dsk_model_finalize(dsk_model* m) {
         return -5;
     }
   }
+  if (m->chain)   // the router's rows into tiles
+    for (Layer& L : m->layers) {
+      if (!L.is_moe || L.gate_tiled) continue;
+      if (m->up.st) CK(cudaStreamSynchronize(m->up.st));
+      float* tiles = nullptr;
+      if (dk::tile_router(m, L.gate, &tiles)) return -2;
+      m->allocs.erase(std::find(m->allocs.begin(), m->allocs.end(), (void*)L.gate));
+      cudaFree(L.gate);
+      L.gate = tiles; L.gate_tiled = true;
+    }
   // join the upload pipeline and give its pinned staging buffers back
   if (m->up.st) {
     cudaError_t e = cudaStreamSynchronize(m->up.st);
@@ -774,6 +818,8 @@ extern "C" double dsk_model_active_bytes_per_token(const dsk_model* m) {
 // state
 // ---------------------------------------------------------------------------------------------------
 static int build_program(dsk_model* m, dsk_state* s);
+static int build_chain(dsk_model* m, dsk_state* s);
+static void drop_chain(dsk_state* s);
 
 // the pieces of copy_to_host, the control words and `more` zeroed bytes behind them in one pinned allocation
 static constexpr size_t kBouncePiece = (size_t)256 << 10;
@@ -849,6 +895,7 @@ extern "C" dsk_state* dsk_state_create(dsk_model* m) {
   cudaEventCreate(&s->ev1);
   if (cudaGetLastError() != cudaSuccess) { fail(-2, "state allocation failed"); return nullptr; }
   if (build_program(m, s)) { return nullptr; }
+  if (m->chain && build_chain(m, s)) { return nullptr; }
   m->n_states++;
   return s;
 }
@@ -857,6 +904,7 @@ extern "C" void dsk_state_destroy(dsk_state* s) {
   if (!s) return;
   if (s->m) s->m->n_states--;
   if (s->hy) hyb::state_free(s);
+  drop_chain(s);
   float* bufs[] = {s->x, s->xb2, s->hbk, s->hbs, s->q_a, s->q, s->q_c, s->kv_a, s->kv_b, s->moe_logits, s->moe_scores, s->act_w, s->logits, s->partial};
   for (float* b : bufs) cudaFree(b);
   cudaFree(s->prog); cudaFree(s->att_scratch); cudaFree(s->sync_words); cudaFree(s->tstamp);
@@ -1507,6 +1555,17 @@ static int run_stages(dsk_model* m, dsk_state* s, int b, int e, int from_argmax,
   return flush(e);
 }
 
+#include "dsk_decode_host.cuh"
+
+static int build_chain(dsk_model* m, dsk_state* s) {
+  s->chain = new dk::Plan();
+  return dk::build(m, s, s->chain);
+}
+static void drop_chain(dsk_state* s) {
+  delete s->chain;
+  s->chain = nullptr;
+}
+
 static void fill_ctrl(Ctrl* h, const dsk_config& c, int token, int pos) {
   // src/infer.cpp:1274-1277
   const int omp = c.original_max_position;
@@ -1541,7 +1600,8 @@ extern "C" int dsk_forward(dsk_model* m, dsk_state* s, int token, int pos, int m
   const int e = mode == DSK_HYDRATE_KV_CACHE ? s->n_stages - s->n_tail : s->n_stages;
   set_xchg_base(m, s, 0, e);
   CK(cudaMemcpyAsync(s->ctrl, s->h_ctrl, sizeof(Ctrl), cudaMemcpyHostToDevice, s->stream));
-  if (run_stages(m, s, 0, e, 0, s->stream)) return -2;
+  if (s->chain) { if (dk::token(*s->chain, mode == DSK_HYDRATE_KV_CACHE ? dk::HOST_HYDRATE : dk::HOST_LOGITS, s->stream)) return -2; }
+  else if (run_stages(m, s, 0, e, 0, s->stream)) return -2;
   if (mode && argmax) CK(cudaMemcpyAsync(s->h_ctrl, s->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, s->stream));
   if (mode && host_logits) { if (copy_to_host(s, host_logits, s->logits_src, (size_t)c.vocab_size * 4)) return -2; }
   else CK(cudaStreamSynchronize(s->stream));
@@ -1560,7 +1620,8 @@ extern "C" int dsk_copy_embedding(dsk_model* m, dsk_state* s, int token) {
   fill_ctrl(s->h_ctrl, m->c, token, 0);
   set_xchg_base(m, s, 0, 1);
   CK(cudaMemcpyAsync(s->ctrl, s->h_ctrl, sizeof(Ctrl), cudaMemcpyHostToDevice, s->stream));
-  if (run_stages(m, s, 0, 1, 0, s->stream)) return -2;
+  if (s->chain) { if (dk::run(*s->chain, 0, 1, 0, s->stream)) return -2; }
+  else if (run_stages(m, s, 0, 1, 0, s->stream)) return -2;
   CK(cudaStreamSynchronize(s->stream));
   s->have_logits = false;
   return 0;
@@ -1580,7 +1641,11 @@ extern "C" int dsk_block_forward(dsk_model* m, dsk_state* s, int layer, int pos,
   h->token = 0; h->pos = pos; h->kv_sink = kv_sink; h->kv_pos = kv_pos; h->kv_len = kv_len; h->argmax_key = 0;
   set_xchg_base(m, s, s->layer_begin[layer], s->layer_end[layer]);
   CK(cudaMemcpyAsync(s->ctrl, h, sizeof(Ctrl), cudaMemcpyHostToDevice, s->stream));
-  if (run_stages(m, s, s->layer_begin[layer], s->layer_end[layer], 0, s->stream)) return -2;
+  if (s->chain) {
+    int b = 0, e = 0;
+    dk::layer_range(*s->chain, layer, &b, &e);
+    if (dk::run(*s->chain, b, e, 0, s->stream)) return -2;
+  } else if (run_stages(m, s, s->layer_begin[layer], s->layer_end[layer], 0, s->stream)) return -2;
   CK(cudaStreamSynchronize(s->stream));
   s->have_logits = false;
   return 0;
@@ -1611,7 +1676,9 @@ extern "C" int dsk_decode_greedy(dsk_model* m, dsk_state* s, int start_pos, int 
   }
   CK(cudaMemsetAsync(s->step, 0, sizeof(int), s->stream));
   CK(cudaEventRecord(s->ev0, s->stream));
-  if (g_engine == ENG_MEGA && s->cut_after.empty()) {
+  if (s->chain) {
+    for (int i = 0; i < n_steps; i++) if (dk::token(*s->chain, dk::GREEDY, s->stream)) return -2;
+  } else if (g_engine != ENG_STAGE && s->cut_after.empty()) {
     CKL(launch_decode(m, s, 0, s->n_stages, 1, n_steps, s->stream));   // the token loop runs inside the persistent kernel
   } else {
     for (int i = 0; i < n_steps; i++) if (run_stages(m, s, 0, s->n_stages, 1, s->stream)) return -2;
@@ -1731,9 +1798,13 @@ extern "C" int dsk_sample_prob(dsk_model* m, dsk_state* s, int index, float* pro
 
 extern "C" int dsk_launches_per_forward(const dsk_model* m, int mode) {
   if (!m) return 0;
-  (void)mode;
   if (m->hy) return hyb::launches_per_token(m);
   const dsk_config& c = m->c;
+  if (m->chain) {   // embedding, six launches a dense layer and seven a routed one, LM head
+    int n = 2;
+    for (const Layer& L : m->layers) n += L.is_moe ? 7 : 6;
+    return mode ? n : n - 1;
+  }
   int cuts = 0;
   if (m->n_ranks > 1 && !m->p2p) for (int l = 0; l < c.n_layers; l++) cuts += m->layers[l].is_moe ? 1 : 0;   // peer-memory mode: one kernel
   return 1 + cuts * 3;
@@ -2181,10 +2252,45 @@ extern "C" int dsk_bench_gemv(int quant, int d, int n, int n_mats, int warmup, i
 // ---------------------------------------------------------------------------------------------------
 // stage-level timeline of one token from the interpreter's own globaltimer stamps (CTA 0)
 // ---------------------------------------------------------------------------------------------------
+// the chain's launches one by one, an event behind each: what a launch takes by itself, start and end included (they overlap in a token)
+static int profile_chain(dsk_model* m, dsk_state* s, int token, int pos, char* out, size_t cap) {
+  if (dsk_forward(m, s, token, pos, 1, nullptr, nullptr)) return -2;
+  const dk::Plan& P = *s->chain;
+  std::vector<cudaEvent_t> ev(P.L.size() + 1);
+  for (cudaEvent_t& e : ev) CK(cudaEventCreate(&e));
+  CK(cudaEventRecord(ev[0], s->stream));
+  for (size_t i = 0; i < P.L.size(); i++) {
+    if (dk::run(P, (int)i, (int)i + 1, 0, s->stream)) return -2;
+    CK(cudaEventRecord(ev[i + 1], s->stream));
+  }
+  CK(cudaStreamSynchronize(s->stream));
+  struct Agg { int n = 0; float us = 0; };
+  std::map<std::string, Agg> agg;
+  float total = 0;
+  for (size_t i = 0; i < P.L.size(); i++) {
+    float ms = 0;
+    CK(cudaEventElapsedTime(&ms, ev[i], ev[i + 1]));
+    char nm[64];
+    snprintf(nm, sizeof(nm), "%-12s smem %6d", P.L[i].name, P.L[i].smem);
+    Agg& a = agg[nm];
+    a.n++; a.us += ms * 1e3f; total += ms * 1e3f;
+  }
+  for (cudaEvent_t e : ev) cudaEventDestroy(e);
+  size_t off = 0;
+  for (auto& kv : agg) {
+    const int n = snprintf(out + off, cap - off, "%s x%3d  %7.2f us a launch | sum %8.1f us\n", kv.first.c_str(), kv.second.n, kv.second.us / kv.second.n, kv.second.us);
+    if (n < 0 || (size_t)n >= cap - off) break;
+    off += n;
+  }
+  snprintf(out + off, cap - off, "token total %.1f us over %zu launches, one at a time\n", total, P.L.size());
+  return 0;
+}
+
 extern "C" int dsk_profile_token(dsk_model* m, dsk_state* s, int token, int pos, char* out, size_t cap) {
   if (m && m->hy) return fail(-4, "dsk_profile_token: the stage timeline belongs to the persistent interpreter");
   if (need_device()) return -1;
   if (!m || !s || !out) return fail(-1, "bad arguments");
+  if (s->chain) return profile_chain(m, s, token, pos, out, cap);
   if (ensure_program(m, s)) return -2;
   {  // switch the stamps on for this token only (they cost a few globaltimer reads per stage)
     unsigned long long* on = s->tstamp;

@@ -1,6 +1,6 @@
 // dsk_kernels.cuh — shared device helpers of the sm_100a decode path (async-copy / mbarrier wrappers, quant traits,
-// activation layouts) plus the two upload/fallback utility kernels.  The decode path itself is the persistent interpreter
-// in dsk_mega.cuh; every C-ABI test hook runs it too, the code that produces the benchmark numbers.
+// activation layouts) plus the two upload/fallback utility kernels.  The decode path itself is dsk_decode.cuh (one GPU, MHA
+// blocks) and the persistent interpreter in dsk_mega.cuh (the rest, and every C-ABI test hook); K-quants are equal bit for bit in both.
 #pragma once
 
 #include <cuda_fp16.h>

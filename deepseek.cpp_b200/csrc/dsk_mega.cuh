@@ -5,6 +5,7 @@
 // (/root/reference/src/infer.cpp:810-1049, 1265-1317):
 //     EMBED | per layer: S1 q(+q_a)+kv_a | [S1b wq_b] | S2 kv_b->KV cache | S3 rope+attention | S4 wo+residual |
 //     S5 gate logits | S56 routing + shared/routed w1,w3 with act(h1)*h3 | S7 w2 + weighted accumulate | LM head+argmax
+// It runs models on several GPUs, true-MLA blocks, shapes that the launches of dsk_decode.cuh refuse, and every test hook.
 // decode_kernel<Q> executes stages [s_begin, s_end) with ONE CTA per SM:
 //   * warp 8 is the TMA producer: it walks this CTA's tiles of the current stage — and runs ahead into the NEXT
 //     stage's static weights — issuing cp.async.bulk copies (weight rows + their f8 scale row) into a ring of

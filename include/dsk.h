@@ -303,12 +303,12 @@ int dsk_block_forward(dsk_model* m, dsk_state* s, int layer, int pos, int kv_sin
 /* Device-resident greedy decode (run_completion's sample->forward loop, src/main.cpp:324-335, -t 0):
  * starting from the logits already in `s` (the previous call must have been dsk_forward(..., DSK_OUTPUT_LOGITS)
  * or dsk_decode_greedy — anything else is rejected), generates n_steps tokens with on-device argmax feeding
- * the next forward.  The token loop runs INSIDE one persistent kernel launch: no host round trip and no
- * launch per token.  out_tokens (n_steps ints, nullable).  Returns the device time of the loop in milliseconds
+ * the next forward.  No host round trip: one captured graph a token (one GPU, MHA blocks), or the token loop
+ * INSIDE one persistent kernel launch.  out_tokens (n_steps ints, nullable).  Returns the device time of the loop in milliseconds
  * through *elapsed_ms (CUDA events), nullable. */
 int dsk_decode_greedy(dsk_model* m, dsk_state* s, int start_pos, int n_steps, int32_t* out_tokens,
                       float* elapsed_ms);
-/* Number of kernels one forward launches (for bench.py's gpu_launches) */
+/* Number of kernels one forward launches */
 int dsk_launches_per_forward(const dsk_model* m, int mode);
 
 /* ---- on-device sampling: Sampler (src/sampler.cpp), reading the logits left in `s` by the last forward ----
@@ -374,8 +374,8 @@ int dsk_attn(const float* q, const uint16_t* kcache, const uint16_t* vcache, int
  * (launch overhead included) and the algorithmic bytes per launch. */
 int dsk_bench_gemv(int quant, int d, int n, int n_mats, int warmup, int iters, float* avg_ms, double* bytes_per_launch);
 
-/* Stage-level timeline of one token from the decode kernel's own globaltimer stamps (CTA 0): a text table (stage kind,
- * count, barrier / staging / tiles / arrive microseconds) written into `out`. */
+/* Timeline of one token as a text table written into `out`: the launches of a token one by one (one GPU, MHA blocks), or the
+ * interpreter's stages from its own globaltimer stamps (CTA 0: barrier / staging / tiles / arrive microseconds). */
 int dsk_profile_token(dsk_model* m, dsk_state* s, int token, int pos, char* out, size_t cap);
 
 #ifdef __cplusplus
