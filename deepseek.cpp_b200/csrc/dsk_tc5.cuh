@@ -8,8 +8,10 @@
 // The activations are rounded to bf16 (as gemm_mma rounds them while staging) and, in routed products, put into expert order by one
 // pass ahead of the product (bf16_rows), or by the epilogue of the product that made them (TcP::C16): every column tile then reads half
 // the bytes, by TMA, instead of gathering and converting fp32 rows again.
-// Bound: not established.  A 64-deep slice of a 128 x 256 tile takes about 1250 cycles, of which the tensor pipe is busy 570; L2 runs at 8 to 17 % of its
-// rate, and two thirds of the bytes a slice (pairs of CTAs on a tile) took the same time.
+// Bound: large products by the tensor pipe (2048 x 8192 x 8192: 1325 TFLOP/s, a 64-deep slice 640 cycles); one-tile grids by what is not under the products
+// (ring fill 1300 to 3000 cycles, 36 cycles a column to store); narrow tiles by the two issuing threads.  Those are elected lanes that count stages and parities:
+// lanes picked by number, which divided by the number of stages, took 650 cycles a slice at any width, now 535 at 256 columns, 340 at 128, 285 at 64, 270 at 32
+// (512 x 2048 x 2048: 21 -> 14.5 us, 45 x 1024 x 4096: 29 -> 17 us).
 #pragma once
 
 #include <cuda.h>   // CUtensorMap
@@ -47,6 +49,12 @@ __device__ __forceinline__ bool tc_wait(uint32_t bar, uint32_t parity, int* err)
   } while (clock64() - from < kTcWaitCycles);
   *reinterpret_cast<volatile int*>(err) = 1;
   return false;
+}
+// one lane of a whole warp
+__device__ __forceinline__ bool tc_elect() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
 }
 __device__ __forceinline__ void tc_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ void tma_tile(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
@@ -111,22 +119,27 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc5(const GemmP P, const T
   const int cols = DUAL ? T.bn / 2 : T.bn;                   // output columns of a tile
   const int n_nt = (P.N + cols - 1) / cols, total = n_mt * n_nt, nk = (P.K + kTcDepth - 1) / kTcDepth;
   const uint32_t stage_bytes = (uint32_t)(kTcRows + T.bn) * kTcDepth * 2;
+  // Row tiles first: neighbours share a slice of the weights.  Routed products have a matrix for every other row tile: columns first, so that the tiles of an
+  // expert run at a time and its weights, and the rows that all columns read again, cross from HBM once.
+  auto row_tile = [&](int tile) { return P.tiles ? tile / n_nt : tile % n_mt; };
+  auto column = [&](int tile) { return (P.tiles ? tile % n_nt : tile / n_mt) * cols; };
   if (warp == 0) {
-    if (lane == 0) {
-      int it = 0;
+    if (tc_elect()) {
+      int it = 0, s = 0;
+      uint32_t turn = 1;                                     // parity that a stage's barrier has next
       bool alive = true;
-      for (int tile = blockIdx.x; tile < total && alive; tile += gridDim.x) {   // row tiles first: neighbours share a slice of the weights
-        const int mt = tile % n_mt, n0 = (tile / n_mt) * cols;
+      for (int tile = blockIdx.x; tile < total && alive; tile += gridDim.x) {
+        const int mt = row_tile(tile), n0 = column(tile);
         int rowA = mt * kTcRows, rowB = n0;
         if (P.tiles) { const int4 t = P.tiles[mt]; rowA = t.y; rowB += t.x * T.rows_per_expert; }
         for (int kb = 0; kb < nk; kb++, it++) {
-          const int s = it % T.stages;
-          if (!tc_wait(empty0 + 8 * s, ((it / T.stages) & 1) ^ 1, T.err)) { alive = false; break; }
+          if (!tc_wait(empty0 + 8 * s, turn, T.err)) { alive = false; break; }
           const uint32_t a = base + (uint32_t)s * stage_bytes, b = a + kTcRows * kTcDepth * 2, bar = full0 + 8 * s;
           mbar_expect_tx(bar, stage_bytes);
           tma_tile(a, &mapA, kb * kTcDepth, rowA, bar);
           tma_tile(b, &mapB, kb * kTcDepth, rowB, bar);
           if (DUAL) tma_tile(b + (uint32_t)cols * kTcDepth * 2, &mapB2, kb * kTcDepth, rowB, bar);
+          if (++s == T.stages) { s = 0; turn ^= 1; }
         }
       }
       // no copy of this CTA is under way when it leaves, also where a wait gave up (else the products have waited for all of them already)
@@ -134,24 +147,25 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc5(const GemmP P, const T
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (tc_elect()) {
       // fp32 accumulate, bf16 x bf16, both K-major
       const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(T.bn / 8) << 17) | ((uint32_t)(kTcRows / 16) << 24);
-      int it = 0, nth = 0;
+      int s = 0, nth = 0;
+      uint32_t turn = 0;
       bool alive = true;
       for (int tile = blockIdx.x; tile < total && alive; tile += gridDim.x, nth++) {
         const int buf = nth & 1;
         if (!tc_wait(drained0 + 8 * buf, ((nth >> 1) & 1) ^ 1, T.err)) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        for (int kb = 0; kb < nk; kb++, it++) {
-          const int s = it % T.stages;
-          if (!tc_wait(full0 + 8 * s, (it / T.stages) & 1, T.err)) { alive = false; break; }
+        for (int kb = 0; kb < nk; kb++) {
+          if (!tc_wait(full0 + 8 * s, turn, T.err)) { alive = false; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint32_t a = base + (uint32_t)s * stage_bytes;
           const uint64_t da = tc_desc(a), db = tc_desc(a + kTcRows * kTcDepth * 2);
 #pragma unroll
           for (int k = 0; k < kTcDepth / 16; k++) tc_mma(tmem + buf * 256, da + 2 * k, db + 2 * k, idesc, kb > 0 || k > 0);
           tc_commit(empty0 + 8 * s);
+          if (++s == T.stages) { s = 0; turn ^= 1; }
         }
         if (alive) tc_commit(done0 + 8 * buf);
       }
@@ -164,7 +178,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc5(const GemmP P, const T
     float* turn = reinterpret_cast<float*>(gbase + kTcRing) + (warp - 2) * 32 * 33;
     int nth = 0;
     for (int tile = blockIdx.x; tile < total; tile += gridDim.x, nth++) {
-      const int buf = nth & 1, mt = tile % n_mt, n0 = (tile / n_mt) * cols;
+      const int buf = nth & 1, mt = row_tile(tile), n0 = column(tile);
       int row0 = mt * kTcRows, nrows = min(kTcRows, P.M - row0);
       if (P.tiles) { const int4 t = P.tiles[mt]; row0 = t.y; nrows = t.z; }
       const int mine = min(32, nrows - quad * 32);            // rows of this warp
