@@ -66,19 +66,13 @@ __device__ __forceinline__ float gelu_tanh_f(float z) { return 0.5f * z * (1.f +
 // log(1 + e^v) without a clamp: beyond 20 the correction term is below half an ulp of v
 __device__ __forceinline__ float softplus_f(float v) { return v > 20.f ? v : log1pf(expf(v)); }
 
-__device__ __forceinline__ float block_sum(float v, float* red) {   // red: 33 floats of shared memory; every thread gets the sum
+__device__ __forceinline__ float block_sum(float v, float* red) {   // red: 32 floats of shared memory, free until the next barrier but one; every thread gets the sum
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
   v = warp_sum(v);
   __syncthreads();
   if (lane == 0) red[warp] = v;
   __syncthreads();
-  if (warp == 0) {
-    float t = lane < nw ? red[lane] : 0.f;
-    t = warp_sum(t);
-    if (lane == 0) red[32] = t;
-  }
-  __syncthreads();
-  return red[32];
+  return warp_sum(lane < nw ? red[lane] : 0.f);   // every warp for itself: the same sum without a third barrier
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -242,7 +236,7 @@ __global__ void __launch_bounds__(256) group_rmsnorm(const float* __restrict__ i
   // a CTA per group, everything it reads in flight ahead of the sum (a decoded token's 4 groups one after the other, each with two waits for
   // memory, took 12 to 20 us; side by side 4)
   const int c0 = (int)blockIdx.y * gs;
-  constexpr int NV = 4;
+  constexpr int NV = 8;
   float v[NV], wt[NV], old[NV], ss = 0.f;
   const bool cached = gs <= 256 * NV;
   if (cached) {
@@ -271,6 +265,40 @@ __global__ void __launch_bounds__(256) group_rmsnorm(const float* __restrict__ i
   } else {
 #pragma unroll 4
     for (int i = threadIdx.x; i < gs; i += 256) put(i, x[c0 + i], w[c0 + i], mode != 0 ? to_f<OT>(o[c0 + i]) : 0.f);
+  }
+}
+
+// The same for many rows of groups of up to 1024 values (mode 0, fp32, no ring): a warp a group, its values in registers.  Lane l holds what threads l, l + 32, ..
+// of group_rmsnorm's 256 hold and adds it up in their order, so that both give the same bits.  (A CTA a group, two values a thread and three barriers: 2048 rows of
+// four groups of 512 took 25.7 us.)
+__global__ void __launch_bounds__(256) group_rmsnorm_rows(const float* __restrict__ in, int ld_in, const float* __restrict__ w, float* __restrict__ out, int ld_out,
+                                                          int rows, int n, int groups, float eps) {
+  grid_enter();
+  const int lane = threadIdx.x & 31, gs = n / groups;
+  const long long id = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (id >= (long long)rows * groups) return;
+  const int t = (int)(id / groups), c0 = (int)(id - (long long)t * groups) * gs;
+  const float* x = in + (size_t)t * ld_in + c0;
+  float* o = out + (size_t)t * ld_out + c0;
+  float v[32], s[8];
+#pragma unroll
+  for (int k = 0; k < 32; k++) v[k] = lane + 32 * k < gs ? x[lane + 32 * k] : 0.f;
+#pragma unroll
+  for (int j = 0; j < 8; j++) {   // warp j's thread of this lane
+    s[j] = 0.f;
+#pragma unroll
+    for (int k = j; k < 32; k += 8) s[j] = fmaf(v[k], v[k], s[j]);
+  }
+#pragma unroll
+  for (int d = 16; d; d >>= 1)
+#pragma unroll
+    for (int j = 0; j < 8; j++) s[j] += __shfl_xor_sync(0xffffffffu, s[j], d);
+  const float ss = ((s[0] + s[4]) + (s[2] + s[6])) + ((s[1] + s[5]) + (s[3] + s[7]));   // the butterfly over eight warps
+  const float sc = 1.f / sqrtf(ss / (float)gs + eps);
+#pragma unroll
+  for (int k = 0; k < 32; k++) {
+    const int i = lane + 32 * k;
+    if (i < gs) o[i] = v[k] * sc * w[c0 + i];
   }
 }
 
@@ -407,40 +435,55 @@ __global__ void __launch_bounds__(256) gemm_narrow(const GemmP P) {
   for (int i = 0; i < 4; i++)
 #pragma unroll
     for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
-  // staging: lane -> half of a row's slice of 16: 8 consecutive k of 16 activation rows; a whole slice of a weight row
-  const int ar = lane >> 1, ak = (lane & 1) * 8, m = row0 + ar;
-  const float* arow = m < P.M ? P.A + (size_t)(P.a_map ? P.a_map[m] / P.a_div : m) * P.lda : nullptr;
-  const WT* wrow = n0 + lane < P.N ? W + (size_t)(n0 + lane) * P.ldw : nullptr;
+  // staging: the lanes of a load have whole slices of 64 (bf16 weights: 32) bytes of neighbouring rows.  (A lane a row of its own, 16 values each, made every
+  // load 32 lines: 2048 rows x 64 columns x 2048 took 44 us.)
+  constexpr int V = WVec<WT>::N, LW = 16 / V, NW = LW;                             // lanes of a weight row's slice, loads of 32 / LW rows
+  const int ak = (lane & 3) * 4, wk = (lane & (LW - 1)) * V;
+  const float* arow[2];
+  const WT* wrow[NW];
+#pragma unroll
+  for (int i = 0; i < 2; i++) {
+    const int m = row0 + (lane >> 2) + 8 * i;
+    arow[i] = m < P.M ? P.A + (size_t)(P.a_map ? P.a_map[m] / P.a_div : m) * P.lda : nullptr;
+  }
+#pragma unroll
+  for (int i = 0; i < NW; i++) {
+    const int n = n0 + lane / LW + 32 / LW * i;
+    wrow[i] = n < P.N ? W + (size_t)n * P.ldw : nullptr;
+  }
   const bool va = (P.lda & 3) == 0 && (reinterpret_cast<uintptr_t>(P.A) & 15) == 0;
-  const bool vw = P.ldw % WVec<WT>::N == 0 && (reinterpret_cast<uintptr_t>(P.W) & 15) == 0;
-  float a[8], b[16];
+  const bool vw = P.ldw % V == 0 && (reinterpret_cast<uintptr_t>(P.W) & 15) == 0;
+  float a[2][4], b[NW][V];
   auto fetch = [&](int k0) {
-    if (arow && va && k0 + ak + 8 <= P.K) {
-      const float4 x = *reinterpret_cast<const float4*>(arow + k0 + ak), y = *reinterpret_cast<const float4*>(arow + k0 + ak + 4);
-      a[0] = x.x; a[1] = x.y; a[2] = x.z; a[3] = x.w; a[4] = y.x; a[5] = y.y; a[6] = y.z; a[7] = y.w;
-    } else {
 #pragma unroll
-      for (int q = 0; q < 8; q++) a[q] = arow && k0 + ak + q < P.K ? arow[k0 + ak + q] : 0.f;
-    }
-    if (wrow && vw && k0 + 16 <= P.K) {
+    for (int i = 0; i < 2; i++) {
+      if (arow[i] && va && k0 + ak + 4 <= P.K) {
+        const float4 x = *reinterpret_cast<const float4*>(arow[i] + k0 + ak);
+        a[i][0] = x.x; a[i][1] = x.y; a[i][2] = x.z; a[i][3] = x.w;
+      } else {
 #pragma unroll
-      for (int q = 0; q < 16; q += WVec<WT>::N) {
-        float v[WVec<WT>::N];
-        WVec<WT>::load(wrow + k0 + q, v);
-#pragma unroll
-        for (int u = 0; u < WVec<WT>::N; u++) b[q + u] = v[u];
+        for (int q = 0; q < 4; q++) a[i][q] = arow[i] && k0 + ak + q < P.K ? arow[i][k0 + ak + q] : 0.f;
       }
-    } else {
+    }
 #pragma unroll
-      for (int q = 0; q < 16; q++) b[q] = wrow && k0 + q < P.K ? to_f<WT>(wrow[k0 + q]) : 0.f;
+    for (int i = 0; i < NW; i++) {
+      if (wrow[i] && vw && k0 + wk + V <= P.K) WVec<WT>::load(wrow[i] + k0 + wk, b[i]);
+      else {
+#pragma unroll
+        for (int q = 0; q < V; q++) b[i][q] = wrow[i] && k0 + wk + q < P.K ? to_f<WT>(wrow[i][k0 + wk + q]) : 0.f;
+      }
     }
   };
   if (w * 16 < P.K) fetch(w * 16);
   for (int k0 = w * 16; k0 < P.K; k0 += 128) {
 #pragma unroll
-    for (int q = 0; q < 8; q++) As[w][ak + q][ar] = a[q];
+    for (int i = 0; i < 2; i++)
 #pragma unroll
-    for (int q = 0; q < 16; q++) Ws[w][q][lane] = b[q];
+      for (int q = 0; q < 4; q++) As[w][ak + q][(lane >> 2) + 8 * i] = a[i][q];
+#pragma unroll
+    for (int i = 0; i < NW; i++)
+#pragma unroll
+      for (int q = 0; q < V; q++) Ws[w][wk + q][lane / LW + 32 / LW * i] = b[i][q];
     __syncwarp();
     if (k0 + 128 < P.K) fetch(k0 + 128);   // in flight during this slice's FMAs
 #pragma unroll
@@ -957,18 +1000,27 @@ inline bool gemv_one_ok(const GemmP& P) {
 // on the current token; `hist` [taps - 1][ch] holds the inputs of the taps - 1 tokens before the chunk (zeros at the start of a
 // sequence).  conv_history_update then replaces `hist` with the last taps - 1 inputs seen (it runs after the convolution).
 // ---------------------------------------------------------------------------------------------------------------------
-__global__ void causal_conv_silu(const float* __restrict__ in, int ld_in, const float* __restrict__ w, const float* __restrict__ b,
-                                 const float* __restrict__ hist, float* __restrict__ out, int ld_out, int T, int ch, int taps) {
+// A thread takes kConvTokens tokens of a channel, their loads of a tap in flight together.  (A token a thread was 82 000 CTAs for 2048 tokens of 5120
+// channels, and bound by their number: 86 us.)
+constexpr int kConvTokens = 8;
+__global__ void __launch_bounds__(128) causal_conv_silu(const float* __restrict__ in, int ld_in, const float* __restrict__ w, const float* __restrict__ b,
+                                                        const float* __restrict__ hist, float* __restrict__ out, int ld_out, int T, int ch, int taps) {
   grid_enter();
-  const int t = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t0 = blockIdx.y * kConvTokens, c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ch) return;
-  float acc = b[c];
+  float acc[kConvTokens];
+#pragma unroll
+  for (int u = 0; u < kConvTokens; u++) acc[u] = b[c];
   for (int k = 0; k < taps; k++) {
-    const int tau = t - (taps - 1) + k;
-    const float v = tau >= 0 ? in[(size_t)tau * ld_in + c] : hist[(size_t)(taps - 1 + tau) * ch + c];
-    acc = fmaf(w[(size_t)c * taps + k], v, acc);
+    const float wk = w[(size_t)c * taps + k];
+#pragma unroll
+    for (int u = 0; u < kConvTokens; u++) {
+      const int tau = min(t0 + u, T - 1) - (taps - 1) + k;
+      acc[u] = fmaf(wk, tau >= 0 ? in[(size_t)tau * ld_in + c] : hist[(size_t)(taps - 1 + tau) * ch + c], acc[u]);
+    }
   }
-  out[(size_t)t * ld_out + c] = silu_f(acc);
+#pragma unroll
+  for (int u = 0; u < kConvTokens; u++) if (t0 + u < T) out[(size_t)(t0 + u) * ld_out + c] = silu_f(acc[u]);
 }
 // The same for steps of at most kConvShort tokens, history included: thread = channel
 constexpr int kConvShort = 4;
@@ -1721,8 +1773,9 @@ __global__ void __launch_bounds__(256) rms_open(float* __restrict__ x, const flo
 //   x' = x + alpha rms(y) wy  -> xo (row pitch ldxo; the stream itself, or the input rows of the product that opens a loop pass);
 //   h = rms(x') wh            (wh nullable: no norm follows here).
 // wgt non-null: y_t = sum_k wgt[t][k] y[t * top + k] (+ wsh[t] ysh[t], nullable): routed experts' outputs and the shared one's.
-// NT threads per row: 256, or 1024 when a step has so few rows that the latency of one row counts.
-template <int NT>
+// NT threads per row: 256, or 1024 when a step has so few rows that the latency of one row counts.  KR values a thread: as few as the rows need, for more rows
+// on an SM and more of a sum's rows in flight (2048 rows of 2048 values, KR = 16 and 8: see launch_rms_add_norm).
+template <int NT, int KR>
 __global__ void __launch_bounds__(NT) rms_add_norm(const float* __restrict__ y, const float* __restrict__ wgt, int top, const float* __restrict__ ysh,
                                                     const float* __restrict__ wsh, const float* __restrict__ wy, const float* x, float* xo, int ldxo,
                                                     const float* __restrict__ wh, float* __restrict__ h, int n,
@@ -1730,7 +1783,6 @@ __global__ void __launch_bounds__(NT) rms_add_norm(const float* __restrict__ y, 
   grid_enter();
   __shared__ float red[33];
   const size_t t = blockIdx.x;
-  constexpr int KR = 256 * kLnRegs / NT;
   float v[KR], u[KR], ss = 0.f;
 #pragma unroll
   for (int k = 0; k < KR; k++) {
@@ -1739,7 +1791,7 @@ __global__ void __launch_bounds__(NT) rms_add_norm(const float* __restrict__ y, 
     u[k] = i < n ? x[t * n + i] : 0.f;
   }
   if (wgt) {
-    constexpr int EB = KR >= 16 ? 2 : 32 / KR;   // rows whose loads are in flight together
+    constexpr int EB = KR >= 16 ? 2 : KR == 8 ? 3 : 32 / KR;   // rows whose loads are in flight together
     for (int e0 = 0; e0 < top; e0 += EB) {
       float r[EB][KR];
 #pragma unroll
@@ -2351,28 +2403,54 @@ __global__ void moe_route(const float* __restrict__ logits, int ldz, const float
 
 // Groups the `pairs` (token, slot) pairs of a chunk by expert: perm lists the pairs expert by expert (in no particular order
 // inside an expert: every row is computed on its own), tiles cuts every expert's run into row tiles of at most `bm` rows
-// {expert, first index into perm, rows}.  One CTA: histogram, serial scan over the experts, placement.
+// {expert, first index into perm, rows}.  One CTA.  A pair's place among its expert's is what the histogram's addition returned; a thread keeps the
+// experts and places of its first kPlanHeld pairs, all read ahead of the first addition.  Experts are scanned a warp of 32 at a time, and a lane writes its expert's tiles.
+// (A thread that scanned the experts alone, and a second pass of additions: 12 288 pairs of 64 experts took 20.5 us.)
+constexpr int kPlanHeld = 16;
 __global__ void __launch_bounds__(1024) moe_plan(const int* __restrict__ idx, int pairs, int E, int bm, int* __restrict__ perm,
                                                  int4* __restrict__ tiles, int* __restrict__ n_tiles) {
   grid_enter();
   extern __shared__ int smi[];
-  int* cnt = smi;            // [E]
-  int* off = smi + E;        // [E]
-  for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
+  int* cnt = smi;            // [E] pairs of an expert
+  int* off = smi + E;        // [E] its first place
+  int* next = smi + 2 * E;   // [E] place of its next pair that no thread holds
+  const int tid = threadIdx.x, lane = tid & 31;
+  int e_held[kPlanHeld], at[kPlanHeld];
+#pragma unroll
+  for (int k = 0; k < kPlanHeld; k++) e_held[k] = tid + 1024 * k < pairs ? idx[tid + 1024 * k] : -1;
+  for (int e = tid; e < E; e += 1024) cnt[e] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x) atomicAdd(&cnt[idx[i]], 1);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int o = 0, nt = 0;
-    for (int e = 0; e < E; e++) {
-      off[e] = o;
-      for (int r = 0; r < cnt[e]; r += bm) tiles[nt++] = make_int4(e, o + r, min(bm, cnt[e] - r), 0);
-      o += cnt[e];
-    }
-    *n_tiles = nt;
+#pragma unroll
+  for (int k = 0; k < kPlanHeld; k++) at[k] = e_held[k] >= 0 ? atomicAdd(&cnt[e_held[k]], 1) : 0;
+  if (pairs > 1024 * kPlanHeld) {
+    __syncthreads();
+    for (int e = tid; e < E; e += 1024) next[e] = cnt[e];
+    __syncthreads();
+    for (int i = tid + 1024 * kPlanHeld; i < pairs; i += 1024) atomicAdd(&cnt[idx[i]], 1);
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x) perm[atomicAdd(&off[idx[i]], 1)] = i;
+  if (tid < 32) {
+    int o = 0, nt = 0;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int e = e0 + lane, n = e < E ? cnt[e] : 0, m = (n + bm - 1) / bm;
+      int so = n, sm = m;
+#pragma unroll
+      for (int d = 1; d < 32; d *= 2) {
+        const int po = __shfl_up_sync(0xffffffffu, so, d), pm = __shfl_up_sync(0xffffffffu, sm, d);
+        if (lane >= d) { so += po; sm += pm; }
+      }
+      const int first = o + so - n;
+      if (e < E) off[e] = first;
+      for (int r = 0; r < m; r++) tiles[nt + sm - m + r] = make_int4(e, first + r * bm, min(bm, n - r * bm), 0);
+      o += __shfl_sync(0xffffffffu, so, 31);
+      nt += __shfl_sync(0xffffffffu, sm, 31);
+    }
+    if (lane == 0) *n_tiles = nt;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kPlanHeld; k++) if (e_held[k] >= 0) perm[off[e_held[k]] + at[k]] = tid + 1024 * k;
+  for (int i = tid + 1024 * kPlanHeld; i < pairs; i += 1024) { const int e = idx[i]; perm[off[e] + atomicAdd(&next[e], 1)] = i; }
 }
 
 // ysh (nullable, [T][width]): a shared expert's output, added with the weight wsh[t]

@@ -1894,18 +1894,26 @@ static void enqueue_head(dsk_model* m, dsk_state* s, int first, int count, float
   linear(S, c.quant == DSK_BF16, c.logit_softcap > 0.f ? HEPI_SOFTCAP : HEPI_STORE, P, 1, st);
 }
 
+// RMS norm in groups, stored.  A warp a group where the groups are more than the CTAs that the chip holds at a time (eight of 256 threads an SM).
+static void rms_groups(const float* in, int ld_in, const float* w, float* out, int ld_out, int T, int n, int groups, float eps, cudaStream_t st) {
+  if (n / groups <= 1024 && (long long)T * groups > 148 * 8)
+    launch_next(group_rmsnorm_rows, (unsigned)(((long long)T * groups + 7) / 8), 256, 0, st)(in, ld_in, w, out, ld_out, T, n, groups, eps);
+  else launch_next(group_rmsnorm<float>, dim3((unsigned)T, (unsigned)groups), 256, 0, st)(in, ld_in, w, out, ld_out, n, groups, eps, 0, 0.f, nullptr, 0, nullptr, 0);
+}
 // the model's norm over the T rows of `in` (width values each): stored into `out`, or added into it times alpha (mode 1)
 static void norm_rows(const dsk_hybrid_config& c, State* S, const float* in, const float* w, const float* b, float* out, int T, int mode, float alpha, cudaStream_t st) {
   if (c.norm_kind == DSK_NORM_LAYER) launch_next(layer_norm, T, 256, 0, st)(in, c.dim, w, b, out, c.dim, c.dim, c.norm_eps, mode, alpha, nullptr, 0);
   else if (mode == 0 && c.norm_groups == 1) launch_next(rms_open, T, 256, 0, st)(const_cast<float*>(in), nullptr, nullptr, w, out, c.dim, c.norm_eps);   // (adds nothing: the row is only read)
+  else if (mode == 0) rms_groups(in, c.dim, w, out, c.dim, T, c.dim, c.norm_groups, c.norm_eps, st);
   else launch_next(group_rmsnorm<float>, dim3((unsigned)T, (unsigned)c.norm_groups), 256, 0, st)(in, c.dim, w, out, c.dim, c.dim, c.norm_groups, c.norm_eps, mode, alpha, nullptr, 0, nullptr, 0);
   S->launches++;
 }
 
 template <typename... A>
-static void launch_rms_add_norm(int T, cudaStream_t st, A... a) {
-  if (T <= kAttnSplitTokens) launch_next(rms_add_norm<1024>, T, 1024, 0, st)(a...);
-  else launch_next(rms_add_norm<256>, T, 256, 0, st)(a...);
+static void launch_rms_add_norm(int T, int n, cudaStream_t st, A... a) {
+  if (T <= kAttnSplitTokens) launch_next(rms_add_norm<1024, kLnRegs / 4>, T, 1024, 0, st)(a...);
+  else if (n <= 256 * 8) launch_next(rms_add_norm<256, 8>, T, 256, 0, st)(a...);
+  else launch_next(rms_add_norm<256, kLnRegs>, T, 256, 0, st)(a...);
 }
 
 static bool fused_norms(const dsk_hybrid_config& c) {
@@ -2027,7 +2035,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         const bool to_xin = next && next->pass >= 0;   // the pass opens with a product: its norm follows that
         const bool product = to_xin && c.loop_in;
         const bool shared = routed && sp.ff_shared > 0;
-        launch_rms_add_norm(T, st, routed ? S->b3 : S->y, routed ? S->wgt : nullptr, routed, shared ? S->b3 + (size_t)T * routed * W : nullptr, S->wsh, wb, S->x,
+        launch_rms_add_norm(T, W, st, routed ? S->b3 : S->y, routed ? S->wgt : nullptr, routed, shared ? S->b3 + (size_t)T * routed * W : nullptr, S->wsh, wb, S->x,
                                         product ? S->xin : S->x, product ? 2 * W : W, to_xin ? nullptr : next ? M->L[next->layer].norm1 : M->final_norm, S->h, W, c.norm_eps, mult);
         S->launches++;
         xin_ready = product;
@@ -2178,7 +2186,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       const int ldi = Q + RW;
       MK("norm");
       linear(S, bf, HEPI_STORE, gp(hin, W, L.in2.p, W, S->b1, ldi, T, ldi, W), 1, st);              // [query latent | key / value latent | rotated key part]
-      launch_next(group_rmsnorm<float>, T, 256, 0, st)(S->b1, ldi, L.dq_norm, S->b2, Q, Q, 1, c.norm_eps, 0, 0.f, nullptr, 0, nullptr, 0);
+      rms_groups(S->b1, ldi, L.dq_norm, S->b2, Q, T, Q, 1, c.norm_eps, st);
       S->launches++;
       linear(S, bf, HEPI_STORE, gp(S->b2, Q, L.uq.p, Q, S->b0, H * DK, T, H * DK, Q), 1, st);       // q [T][H][D | Rd]
       const bool portion = pos0 >= 0 && T >= kPrefillMin && S->prefill_keys > 0;
@@ -2326,7 +2334,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       MK("ssd.in");
       if (T <= kConvShort) launch_next(causal_conv_silu_short, (ch + 127) / 128, 128, 0, st)(S->b0 + inner, pw, L.conv_w, L.conv_b, ls.hist, S->b1, ch, T, ch, sp.ssm_conv);
       else {
-        launch_next(causal_conv_silu, dim3((unsigned)((ch + 127) / 128), (unsigned)T), 128, 0, st)(S->b0 + inner, pw, L.conv_w, L.conv_b, ls.hist, S->b1, ch, T, ch, sp.ssm_conv);
+        launch_next(causal_conv_silu, dim3((unsigned)((ch + 127) / 128), (unsigned)((T + kConvTokens - 1) / kConvTokens)), 128, 0, st)(S->b0 + inner, pw, L.conv_w, L.conv_b, ls.hist, S->b1, ch, T, ch, sp.ssm_conv);
         if (sp.ssm_conv > 1) launch_next(conv_history_update, (ch + 127) / 128, 128, 0, st)(S->b0 + inner, pw, ls.hist, T, ch, sp.ssm_conv);
       }
       MK("ssd.conv");
@@ -2341,7 +2349,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         S->launches += 2;
       } else launch_scan(sp, S->b0, pw, S->b1, ch, L, ls.ssm, S->b2, T, st);
       MK("ssd.scan");
-      launch_next(group_rmsnorm<float>, dim3((unsigned)T, (unsigned)sp.ssm_norm_groups), 256, 0, st)(S->b2, inner, L.mnorm, S->b3, inner, inner, sp.ssm_norm_groups, c.norm_eps, 0, 0.f, nullptr, 0, nullptr, 0);
+      rms_groups(S->b2, inner, L.mnorm, S->b3, inner, T, inner, sp.ssm_norm_groups, c.norm_eps, st);
       S->launches += 4;
       MK("ssd.norm");
       GemmP P = gp(S->b3, inner, L.o.p, inner, sink.C, W, T, W, inner);
@@ -2447,7 +2455,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
     if (sandwich) {   // x += norm1b(mixer output); the feed-forward then reads norm2 of the new x
       if (sp.ff_kind == DSK_FF_NONE) close_run(L.close1);
       else if (frms) {
-        launch_rms_add_norm(T, st, S->y, nullptr, 0, nullptr, nullptr, L.close1, S->x, S->x, W, L.norm2, S->h, W, c.norm_eps, mult);
+        launch_rms_add_norm(T, W, st, S->y, nullptr, 0, nullptr, nullptr, L.close1, S->x, S->x, W, L.norm2, S->h, W, c.norm_eps, mult);
         S->launches++;
       } else if (fuse) {
         launch_next(layer_norm_add_norm, T, 256, 0, st)(S->y, L.close1, S->x, nullptr, L.norm2, S->h, W, c.norm_eps, mult);
@@ -2519,7 +2527,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         MK("moe.down");
       } else {
         constexpr int bm = 128;   // rows per tile of the product kernels that follow (gemm_tc5, gemm_mma, gemm_split)
-        launch_next(moe_plan, 1, 1024, (size_t)2 * E * 4, st)(S->d_idx, pairs, E, bm, S->d_perm, S->d_tiles, S->d_ntiles);
+        launch_next(moe_plan, 1, 1024, (size_t)3 * E * 4, st)(S->d_idx, pairs, E, bm, S->d_perm, S->d_tiles, S->d_ntiles);
         S->launches++;
         G.tiles = S->d_tiles; G.n_tiles = S->d_ntiles; G.a_map = S->d_perm; G.a_div = top; G.c_map = S->d_perm;
         Dn.tiles = S->d_tiles; Dn.n_tiles = S->d_ntiles; Dn.a_map = S->d_perm; Dn.a_div = 1; Dn.c_map = S->d_perm;
