@@ -2667,16 +2667,15 @@ static int decode_greedy(dsk_model* m, dsk_state* s, int start_pos, int n_steps,
   if (start_pos < 0 || start_pos != S->next_pos) return fail(-4, "dsk_decode_greedy: start_pos %d must follow the state's sequence (at %d)", start_pos, S->next_pos);
   const int one = 0;
   CK(cudaMemcpyAsync(S->d_want, &one, 4, cudaMemcpyHostToDevice, s->stream));
-  launch_next(set_ctl, 1, 1, 0, s->stream)(S->d_ctl, start_pos);
+  launch_next(set_ctl, 1, 1, 0, s->stream)(S->d_ctl, start_pos - 1);   // (greedy_feed moves on)
   CK(cudaMemsetAsync(s->step, 0, sizeof(int), s->stream));
   CK(cudaStreamSynchronize(s->stream));
   if (!S->step_graph) {
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal));
-    launch_next(greedy_feed, 1, 1, 0, s->stream)(s->ctrl, S->d_tok, s->token_log, s->step);
+    launch_next(greedy_feed, 1, 1, 0, s->stream)(s->ctrl, S->d_tok, s->token_log, s->step, S->d_ctl);
     int rc = enqueue_chunk(m, s, 1, 1, nullptr, s->stream);
     launch_argmax(s, c.vocab_size);
-    launch_next(advance_ctl, 1, 1, 0, s->stream)(S->d_ctl, 1);
     cudaError_t e = cudaStreamEndCapture(s->stream, &g);
     if (rc || e != cudaSuccess) return fail(-2, "capturing the decode step failed: %s", cudaGetErrorString(e));
     CK(cudaGraphInstantiate(&S->step_graph, g, 0));
