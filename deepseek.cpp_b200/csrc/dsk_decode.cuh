@@ -296,7 +296,7 @@ __device__ __forceinline__ void q8_half_block(const float4 (&x)[4], bool on, uin
     f = __shfl_sync(0xffffffffu, f, hb + (who ? __ffs(who) - 1 : 0));
     if (hi == -lo) mx = f;
   }
-  const bool zero = mx == 0.f;
+  const bool zero = !(fabsf(mx) > 0.f);   // (also a block of NaN alone: the reference's scan finds no largest value in it)
   const float iscale = zero ? 0.f : __fdiv_rn(-127.f, mx);
   uint32_t w[4];
 #pragma unroll

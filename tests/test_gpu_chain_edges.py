@@ -1,0 +1,103 @@
+"""The token chain (csrc/dsk_decode.cuh) against the interpreter that runs the models it refuses, where a call leaves the ordinary: values that are not finite.
+
+K-quants have one order of sums in both and are equal bit for bit; of the other formats the places that are not finite are equal, and the rest within 2^-11 (a cached
+key or value that rounds to fp16 the other way)."""
+import os
+import pickle
+import subprocess
+import sys
+import tempfile
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+sys.path[:0] = [os.path.join(HERE, "..", "deepseek.cpp_b200"), os.path.join(HERE, "..", "oracle")]
+pytestmark = pytest.mark.gpu
+
+PRESET = {"q2_k": "tiny_v2", "q3_k": "tiny_v3", "f8e5m2": "tiny_v2", "fp16": "tiny_v3", "fp32": "tiny_v2"}
+NAN = {"q2_k": (slice(84 + 80, 84 + 82), (0, 0x7E)), "q3_k": (slice(110 + 108, 110 + 110), (0, 0x7E)), "f8e5m2": (300, 0x7F), "fp16": (300, np.nan), "fp32": (300, np.nan)}
+INF = {"q2_k": (slice(84 + 80, 84 + 82), (0, 0x7C)), "q3_k": (slice(110 + 108, 110 + 110), (0, 0x7C)), "f8e5m2": (300, 0x7C), "fp16": (300, np.inf), "fp32": (300, np.inf)}
+
+
+def load(quant, edit=None, seed=5, **sizes):
+    """A small model; `edit` changes copies of its tensors."""
+    import dseek
+    import dsk
+    import mint
+    with tempfile.TemporaryDirectory() as d:
+        mint.mint(d, PRESET[quant], quant, fast=True, seed=seed, **sizes)
+        md, tensors = dseek.read_dir(d)
+        m = dsk.Model(dsk.Config.from_metadata(md, 0))
+        for name, t in tensors.items():
+            data = np.array(t.data)
+            if edit:
+                edit(name, data)
+            m.upload(name, t.dtype, t.shape, data)
+        m.finalize()
+    return m
+
+
+def not_finite(quant):
+    """Embedding rows with a block (K-quants) or a value that is NaN, infinite; then cached values that are, which attention hands on to a product without a norm."""
+    def edit(name, data):
+        if name == "model.embed.weight":
+            for row, (at, v) in ((7, NAN[quant]), (9, INF[quant])):
+                data.reshape(1024, -1)[row, at] = v
+    m = load(quant, edit)
+    got = {}
+    for pos, token in enumerate((3, 7, 9, 4)):
+        logits, best = m.forward(token, pos)
+        got[f"token {token}"] = [np.array(logits), np.array([best])]
+    for pos in range(4):
+        m.forward(3 + 2 * pos + (pos > 1), pos)   # (finite rows again)
+    clean = m.kv_cache(0, 1).copy()
+    c = m.cfg
+    for name, heads, value in (("NaN", 1, np.nan), ("inf", 1, np.inf), ("-inf", 1, -np.inf), ("NaN heads", 4, np.nan)):
+        kv = clean.view(np.float16).reshape(-1, c.n_heads, c.v_head_dim).copy()
+        kv[1, :heads, 5 if heads == 1 else slice(None)] = value
+        m.set_kv_cache(0, 1, kv.view(np.uint16).reshape(-1))
+        m.copy_embedding(3)
+        m.block(0, 3, 0, 3, 4)
+        got["cached " + name] = [m.buffer("x")]
+    m.close()
+    return got
+
+
+SCENARIOS = {("not finite", q): (not_finite, q) for q in PRESET}
+
+
+def _run(out):
+    import dsk
+    dsk.init(0)
+    with open(out, "wb") as f:
+        pickle.dump({k: fn(*args) for k, (fn, *args) in SCENARIOS.items()}, f)
+
+
+@pytest.fixture(scope="module")
+def both(tmp_path_factory):
+    out = []
+    for engine in ("chain", "mega"):
+        p = str(tmp_path_factory.mktemp(engine) / "out")
+        subprocess.run([sys.executable, __file__, p], env={**os.environ, "DSK_ENGINE": engine}, check=True, timeout=300)
+        with open(p, "rb") as f:
+            out.append(pickle.load(f))
+    return out
+
+
+@pytest.mark.parametrize("scenario", SCENARIOS, ids=str)
+def test_chain_against_interpreter(both, scenario):
+    chain, mega = (b[scenario] for b in both)
+    assert chain.keys() == mega.keys()
+    for what in chain:
+        for a, b in zip(chain[what], mega[what]):
+            if scenario[1] in ("q2_k", "q3_k") or a.dtype.kind == "i":
+                assert np.array_equal(a, b, equal_nan=a.dtype.kind == "f"), what
+            else:
+                f = np.isfinite(b)
+                assert np.array_equal(np.isfinite(a), f) and np.array_equal(np.isnan(a), np.isnan(b)), what
+                assert np.linalg.norm((a - b)[f]) <= 2.0 ** -11 * np.linalg.norm(b[f]), what
+
+
+if __name__ == "__main__":
+    _run(sys.argv[1])
