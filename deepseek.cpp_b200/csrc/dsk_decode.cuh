@@ -1032,8 +1032,8 @@ __global__ void __maxnreg__(80) dk_gemv(const DkGemv* __restrict__ told, const _
 // ---- rope + attention of one head (src/infer.cpp:648-762, 956-1045): one CTA a head ------------------------------------------------------
 // The head's older keys and values come into shared memory ahead of the wait: they were written launches ago (a launch begins when the one ahead of it
 // is past its own wait, so only the one ahead may still run, and that writes row kv_pos).  What is left behind the wait is the new row, one pass over
-// shared memory for the scores and one for the values.  Contexts that do not fit (157 or 180 positions of 192 + 128 halves), and those whose first rows
-// turn in place (sinks), are read from global memory in the same passes.
+// shared memory for the scores and one for the values.  Contexts that do not fit (157 or 180 positions of 192 + 128 halves), those whose first rows
+// turn in place (sinks) and those that the new row lies behind are read from global memory in the same passes.
 // Shared memory: query | scores of `hold` positions | their keys (later partial sums of the values) | their values; or query | partial sums | scores
 __host__ __device__ inline int dk_attn_parts(int vh) { return (vh <= 256 ? 256 / vh : 1) * vh; }
 template <int NW>
@@ -1048,7 +1048,7 @@ __global__ void __maxnreg__(80) dk_attn(const __grid_constant__ DkAttn P) {
   const volatile int* cw = reinterpret_cast<const volatile int*>(P.ctrl);   // (set launches ago; not out of L1)
   const int pos = cw[offsetof(Ctrl, pos) / 4], kv_pos = cw[offsetof(Ctrl, kv_pos) / 4], kv_len = cw[offsetof(Ctrl, kv_len) / 4], kv_sink = cw[offsetof(Ctrl, kv_sink) / 4];
   const int nc = P.hd >> 3, nv = P.vh >> 3, half_r = P.rope >> 1;   // (16-byte words of a row)
-  const bool held = kv_len <= P.hold && kv_sink == 0;
+  const bool held = kv_len <= P.hold && kv_pos < kv_len && kv_sink == 0;   // (a block call may put its row behind those that it reads)
   float* att = qs + P.hd;
   __half *ks = reinterpret_cast<__half*>(att + P.hold), *vs = ks + (size_t)P.hold * P.hd;
   float* part = held ? reinterpret_cast<float*>(ks) : att;

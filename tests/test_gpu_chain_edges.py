@@ -1,4 +1,5 @@
-"""The token chain (csrc/dsk_decode.cuh) against the interpreter that runs the models it refuses, where a call leaves the ordinary: values that are not finite.
+"""The token chain (csrc/dsk_decode.cuh) against the interpreter that runs the models it refuses, where a call leaves the ordinary: values that are not finite, cache rows behind
+those that are read.
 
 K-quants have one order of sums in both and are equal bit for bit; of the other formats the places that are not finite are equal, and the rest within 2^-11 (a cached
 key or value that rounds to fp16 the other way)."""
@@ -64,7 +65,22 @@ def not_finite(quant):
     return got
 
 
-SCENARIOS = {("not finite", q): (not_finite, q) for q in PRESET}
+def row_behind(quant):
+    """Block calls whose new row lies behind the rows that are read: inside and outside of what the attention holds in shared memory (about 90 rows of these heads)."""
+    m = load(quant, qk_nope_head_dim=256, qk_rope_head_dim=64, v_head_dim=256)
+    for pos in range(10):
+        m.forward(5 + 31 * pos, pos)
+    got = {}
+    for kv_pos in (9, 10, 60, 89, 130, 255):
+        for layer in (0, 1):
+            m.copy_embedding(40 + kv_pos)
+            m.block(layer, kv_pos, 0, kv_pos, 10)
+            got[f"row {kv_pos}, layer {layer}"] = [m.buffer("x")] + [m.kv_cache(layer, which).view(np.float16).astype(np.float32) for which in (0, 1)]
+    m.close()
+    return got
+
+
+SCENARIOS = {(n, q): (f, q) for n, f in (("not finite", not_finite), ("row behind", row_behind)) for q in PRESET}
 
 
 def _run(out):
