@@ -1081,6 +1081,7 @@ __global__ void __maxnreg__(80) dk_attn(const __grid_constant__ DkAttn P) {
     if (P.is_v3) { kr[2 * t] = r0h; kr[2 * t + 1] = r1h; }
     else { kr[t] = r0h; kr[t + half_r] = r1h; }
   }
+  if (kv_pos < kv_sink) __syncthreads();   // (a block call whose new row is a sink: it turns too)
   const int rows_at_once = NT / half_r;   // sink rows turn by one position, in place: read, then write
   for (int r0 = 0; r0 < kv_sink; r0 += rows_at_once) {
     const int r = r0 + tid / half_r, t = tid - (tid / half_r) * half_r;

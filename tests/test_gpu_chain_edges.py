@@ -115,5 +115,30 @@ def test_chain_against_interpreter(both, scenario):
                 assert np.linalg.norm((a - b)[f]) <= 2.0 ** -11 * np.linalg.norm(b[f]), what
 
 
+@pytest.mark.parametrize("row", [0, 1])
+def test_new_row_is_a_sink(row):
+    """A block call whose new row is one of the rows that turn: it is rotated, written and then turned with them.  Against the oracle (fp32; a cached value may round
+    to fp16 the other way)."""
+    import dsk
+    import mint
+    import oracle
+    with tempfile.TemporaryDirectory() as d:
+        mint.mint(d, "tiny_v2", "fp32", fast=True, seed=5)
+        m, o = dsk.Model.from_dir(d), oracle.open_session(d)
+        for pos in range(6):
+            m.forward(5 + 31 * pos, pos)
+        for which in (0, 1):
+            o.kv_cache(0, which)[:] = m.kv_cache(0, which)
+        for s in (m, o):
+            s.copy_embedding(40)
+            s.block(0, 9, 2, row, 6)
+        exp = o.buffer("x")
+        assert np.linalg.norm(m.buffer("x") - exp) <= 2.0 ** -11 * np.linalg.norm(exp)
+        a, b = (s.kv_cache(0, 0)[:6 * 4 * 96].view(np.float16).astype(np.float32) for s in (m, o))
+        assert np.abs(a - b).max() <= 2.0 ** -10 * np.abs(b).max()
+        m.close()
+        o.close()
+
+
 if __name__ == "__main__":
     _run(sys.argv[1])
