@@ -606,8 +606,9 @@ static int upload_weight(dsk_model* m, DTensor& t, int rows, int cols, bool expe
     if (dmalloc(m, (void**)&t.w, t.expert_bytes * count)) return -2;
     const unsigned char* dsrc = (const unsigned char*)data;
     if (!on_dev || (uintptr_t)data % 16) {
+      // (a device source is copied on the legacy stream, which the upload stream does not wait for nor keep waiting)
+      if (m->up.st && (on_dev || m->up.raw_cap < tot)) CK(cudaStreamSynchronize(m->up.st));
       if (m->up.raw_cap < tot) {
-        if (m->up.st) CK(cudaStreamSynchronize(m->up.st));
         cudaFree(m->up.raw);
         m->up.raw = nullptr; m->up.raw_cap = 0;
         CK(cudaMalloc(&m->up.raw, tot));

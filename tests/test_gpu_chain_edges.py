@@ -140,5 +140,39 @@ def test_new_row_is_a_sink(row):
         o.close()
 
 
+@pytest.mark.parametrize("quant", PRESET)
+def test_tensors_from_host_and_device(quant):
+    """A model whose tensors come by turns from the host, each a larger one, and from device addresses that no vector load may take, each a smaller one."""
+    import dseek
+    import dsk
+    import mint
+    import torch
+    logits = []
+    with tempfile.TemporaryDirectory() as d:
+        mint.mint(d, PRESET[quant], quant, fast=True, seed=5, hidden_dim=8192)
+        md, tensors = dseek.read_dir(d)
+        names = sorted((n for n in tensors if n != "tokenizer.tokens"), key=lambda n: tensors[n].data.nbytes)
+        big, small = names[len(names) // 2:][::-1], names[:len(names) // 2]
+        turns = [n for pair in zip(big, small + [None]) for n in pair if n]
+        assert sorted(turns) == sorted(names)
+        for mixed in (False, True):
+            m = dsk.Model(dsk.Config.from_metadata(md, 0))
+            for i, name in enumerate(turns):
+                t = tensors[name]
+                data = np.ascontiguousarray(t.data)
+                if mixed and name in small:
+                    buf = torch.zeros(data.nbytes + 16, dtype=torch.uint8, device="cuda")
+                    at = 2 if data.dtype.itemsize <= 2 else 4
+                    buf[at:at + data.nbytes] = torch.from_numpy(data.reshape(-1).view(np.uint8).copy()).cuda()
+                    torch.cuda.synchronize()
+                    m.upload_device(name, t.dtype, t.shape, buf.data_ptr() + at, data.nbytes)
+                else:
+                    m.upload(name, t.dtype, t.shape, data)
+            m.finalize()
+            logits.append(np.stack([np.array(m.forward(5 + 31 * pos, pos)[0]) for pos in range(4)]))
+            m.close()
+    assert np.array_equal(*logits)
+
+
 if __name__ == "__main__":
     _run(sys.argv[1])
