@@ -341,7 +341,8 @@ static int build(dsk_model* m, dsk_state* s, Plan* out) {
   auto expert = [&](DkSeg& S, const DTensor& t, int k) { S.slot = k; S.w_stride = (long long)t.expert_bytes; S.s_stride = (long long)t.scale_expert; };
   std::map<std::vector<int>, Lists> seen;   // layers are alike: a plan is made once per shape
   auto key_of = [&](const Draft& D, int form) {
-    std::vector<int> key{form, D.g.nsegs, D.g.nin, D.g.in[0].n, D.g.in[1].n, D.g.in[0].seg, D.even};
+    std::vector<int> key{form, D.g.nsegs, D.g.nin, D.even};   // (all that plan() reads)
+    for (const DkInput& I : D.g.in) { key.push_back(I.n); key.push_back(I.seg); key.push_back(I.norm != nullptr); }
     for (int j = 0; j < D.g.nsegs; j++) { key.push_back(D.g.seg[j].rows); key.push_back(D.g.seg[j].nb); key.push_back((D.g.seg[j].f32 << 1) | D.g.seg[j].pair); }
     return key;
   };

@@ -1,5 +1,5 @@
 """The token chain (csrc/dsk_decode.cuh) against the interpreter that runs the models it refuses, where a call leaves the ordinary: values that are not finite, cache rows behind
-those that are read.
+those that are read, launches of like sizes.
 
 K-quants have one order of sums in both and are equal bit for bit; of the other formats the places that are not finite are equal, and the rest within 2^-11 (a cached
 key or value that rounds to fp16 the other way)."""
@@ -80,7 +80,15 @@ def row_behind(quant):
     return got
 
 
-SCENARIOS = {(n, q): (f, q) for n, f in (("not finite", not_finite), ("row behind", row_behind)) for q in PRESET}
+def like_sizes(quant):
+    """The output projection of attention and the LM head have the same sizes; only the second one's input has a norm (they run in launches of the same form)."""
+    m = load(quant, dim=512, vocab_size=512, n_heads=4, v_head_dim=128, n_layers=1, first_k_dense_replace=0)
+    got = {f"position {pos}": [np.array(m.forward(5 + 31 * pos, pos)[0])] for pos in range(4)}
+    m.close()
+    return got
+
+
+SCENARIOS = {(n, q): (f, q) for n, f in (("not finite", not_finite), ("row behind", row_behind), ("like sizes", like_sizes)) for q in PRESET}
 
 
 def _run(out):
