@@ -57,15 +57,18 @@ static int tile(int quant, const unsigned char* src, uint8_t* dst, int rows, int
   if (wait) CK(cudaDeviceSynchronize());
   return 0;
 }
-static int tile_router(dsk_model* m, const float* src, float** dst) {
-  const int E = m->c.n_routed_experts, n = m->c.dim;
-  const bool plain = m->c.quant == DSK_F32;
-  const size_t units = plain ? dk_matrix_bytes(DSK_F32, E, n) / (size_t)dk_unit_bytes(DSK_F32) : (size_t)cdiv(E, kDkF32Rows) * cdiv(n, kDkF32Cols);
-  if (dmalloc(m, (void**)dst, units * (plain ? dk_unit_bytes(DSK_F32) : kDkF32Unit))) return -2;
-  if (plain) return tile(DSK_F32, (const unsigned char*)src, (uint8_t*)*dst, E, n, 1, nullptr, true);
-  dk_tile_router<<<(unsigned)((units + 7) / 8), 256>>>(src, (unsigned char*)*dst, E, n, (int)units);
+// the router: tiles of its own in a quantised model
+static size_t router_bytes(const dsk_config& c) {
+  const int E = c.n_routed_experts;
+  return c.quant == DSK_F32 ? dk_matrix_bytes(DSK_F32, E, c.dim) : (size_t)cdiv(E, kDkF32Rows) * cdiv(c.dim, kDkF32Cols) * kDkF32Unit;
+}
+static int tile_router(const dsk_config& c, const float* src, float* dst, cudaStream_t st, bool wait) {
+  const int E = c.n_routed_experts, n = c.dim;
+  if (c.quant == DSK_F32) return tile(DSK_F32, (const unsigned char*)src, (uint8_t*)dst, E, n, 1, st, wait);
+  const int units = (int)(router_bytes(c) / kDkF32Unit);
+  if (units > 0) dk_tile_router<<<(unsigned)((units + 7) / 8), 256, 0, st>>>(src, (unsigned char*)dst, E, n, units);
   CK(cudaGetLastError());
-  CK(cudaDeviceSynchronize());
+  if (wait) CK(cudaDeviceSynchronize());
   return 0;
 }
 

@@ -26,7 +26,6 @@
 #include <vector>
 
 #include <algorithm>
-#include <array>
 #include "dsk_kernels.cuh"
 #include "dsk_mega.cuh"
 #include "dsk_decode.cuh"
@@ -115,7 +114,7 @@ struct Layer {
   DTensor wq, wq_a, wq_b, wkv_a, wkv_b, wo, w1, w2, w3, sw1, sw2, sw3;
   DTensor wc, wq_rope_b, wv_b;   // true-MLA blocks (use_mla): absorbed query projection, rope query projection, per-head value up-projection
   float *gate = nullptr, *gate_bias = nullptr;
-  bool is_moe = false, gate_tiled = false;
+  bool is_moe = false;
   __half *kcache = nullptr, *vcache = nullptr;
 };
 
@@ -142,7 +141,8 @@ struct Plan;
 static bool fits(const dsk_config& c, int n_ranks);
 static int set_attributes();
 static int tile(int quant, const unsigned char* src, uint8_t* dst, int rows, int cols, int count, cudaStream_t st, bool wait);
-static int tile_router(dsk_model* m, const float* src, float** dst);
+static size_t router_bytes(const dsk_config& c);
+static int tile_router(const dsk_config& c, const float* src, float* dst, cudaStream_t st, bool wait);
 }
 
 struct dsk_model {
@@ -549,6 +549,34 @@ static int upload_f32(dsk_model* m, float** dst, int64_t d0, int64_t d1, int dty
   return copy_rows(m, *dst, nbytes, data, nbytes, nbytes, 1, on_dev);
 }
 
+// `bytes` of rows as the file has them, at an aligned device address: where they are, or in the upload's own buffer
+static int rows_on_device(dsk_model* m, const void* data, size_t bytes, int on_dev, const void** out) {
+  *out = data;
+  if (on_dev && (uintptr_t)data % 16 == 0) return 0;
+  Uploader& u = m->up;
+  // (a device source is copied on the legacy stream, which the upload stream does not wait for nor keep waiting)
+  if (u.st && (on_dev || u.raw_cap < bytes)) CK(cudaStreamSynchronize(u.st));
+  if (u.raw_cap < bytes) {
+    cudaFree(u.raw);
+    u.raw = nullptr; u.raw_cap = 0;
+    CK(cudaMalloc(&u.raw, bytes));
+    u.raw_cap = bytes;
+  }
+  *out = u.raw;
+  return copy_rows(m, u.raw, bytes, data, bytes, bytes, 1, on_dev);
+}
+// The router's rows into the tiles of the token chain (here and not when the model is finished: a state may be made before that)
+static int upload_router(dsk_model* m, float** dst, int dtype, const int64_t shape[4], const void* data, size_t nbytes, int on_dev, const char* name) {
+  const dsk_config& c = m->c;
+  const int64_t want[4] = {c.n_routed_experts, c.dim, 0, 0};
+  if (check_tensor(name, dtype, shape, nbytes, DSK_DT_F32, false, want, (size_t)c.n_routed_experts * c.dim * 4)) return -4;
+  if (*dst) return fail(-4, "tensor %s uploaded twice", name);
+  if (dmalloc(m, (void**)dst, dk::router_bytes(c))) return -2;
+  const void* src = nullptr;
+  if (rows_on_device(m, data, nbytes, on_dev, &src)) return -2;
+  return dk::tile_router(c, (const float*)src, *dst, on_dev ? nullptr : m->up.st, on_dev);
+}
+
 // bytes of `cols` consecutive columns of a disk row (cols: a multiple of the quant's block width)
 static size_t disk_col_bytes(int quant, int cols) { return disk_row_bytes(quant, cols); }
 
@@ -604,20 +632,9 @@ static int upload_weight(dsk_model* m, DTensor& t, int rows, int cols, bool expe
   if (m->chain) {   // rows as the file has them -> tiles (dsk_decode.cuh); one GPU: the whole tensor
     t.expert_bytes = dk_matrix_bytes(q, rc, cc);
     if (dmalloc(m, (void**)&t.w, t.expert_bytes * count)) return -2;
-    const unsigned char* dsrc = (const unsigned char*)data;
-    if (!on_dev || (uintptr_t)data % 16) {
-      // (a device source is copied on the legacy stream, which the upload stream does not wait for nor keep waiting)
-      if (m->up.st && (on_dev || m->up.raw_cap < tot)) CK(cudaStreamSynchronize(m->up.st));
-      if (m->up.raw_cap < tot) {
-        cudaFree(m->up.raw);
-        m->up.raw = nullptr; m->up.raw_cap = 0;
-        CK(cudaMalloc(&m->up.raw, tot));
-        m->up.raw_cap = tot;
-      }
-      if (copy_rows(m, m->up.raw, tot, data, tot, tot, 1, on_dev)) return -2;
-      dsrc = (const unsigned char*)m->up.raw;
-    }
-    return dk::tile(q, dsrc, t.w, rc, cc, count, on_dev ? nullptr : m->up.st, on_dev);
+    const void* dsrc = nullptr;
+    if (rows_on_device(m, data, tot, on_dev, &dsrc)) return -2;
+    return dk::tile(q, (const unsigned char*)dsrc, t.w, rc, cc, count, on_dev ? nullptr : m->up.st, on_dev);
   }
   const size_t nrows_loc = (size_t)rc * count;
   const size_t local_disk = drb_loc * nrows_loc, local_dev = vrb * nrows_loc;
@@ -674,7 +691,10 @@ extern "C" int dsk_upload_tensor(dsk_model* m, const char* name, int dtype, cons
   if (rest == "mlp.norm.weight") return F(&L.rms_ffn, c.dim, 0);
   if (rest == "attn.kv_a_norm.weight") return F(&L.rms_kv_a, c.kv_lora_rank, 0);
   if (rest == "attn.q_a_norm.weight") return F(&L.rms_q_a, c.q_lora_rank, 0);
-  if (rest == "moegate.weight") return F(&L.gate, c.n_routed_experts, c.dim);
+  if (rest == "moegate.weight") {
+    if (m->chain) return upload_router(m, &L.gate, dtype, shape, data, nbytes, src_on_device, name);
+    return F(&L.gate, c.n_routed_experts, c.dim);
+  }
   if (rest == "moegate.bias") return F(&L.gate_bias, c.n_routed_experts, 0);
   const size_t dot = rest.rfind('.');
   if (dot == std::string::npos) return fail(-4, "unknown tensor name %s", name);
@@ -746,16 +766,6 @@ extern "C" int dsk_model_finalize(dsk_model* m) {
         return -5;
     }
   }
-  if (m->chain)   // the router's rows into tiles
-    for (Layer& L : m->layers) {
-      if (!L.is_moe || L.gate_tiled) continue;
-      if (m->up.st) CK(cudaStreamSynchronize(m->up.st));
-      float* tiles = nullptr;
-      if (dk::tile_router(m, L.gate, &tiles)) return -2;
-      m->allocs.erase(std::find(m->allocs.begin(), m->allocs.end(), (void*)L.gate));
-      cudaFree(L.gate);
-      L.gate = tiles; L.gate_tiled = true;
-    }
   // join the upload pipeline and give its pinned staging buffers back
   if (m->up.st) {
     cudaError_t e = cudaStreamSynchronize(m->up.st);

@@ -182,5 +182,28 @@ def test_tensors_from_host_and_device(quant):
     assert np.array_equal(*logits)
 
 
+@pytest.mark.parametrize("quant", PRESET)
+def test_state_before_finalize(quant):
+    """A state that is made when all tensors have come, but before the model is finished."""
+    import dseek
+    import dsk
+    import mint
+    logits = []
+    with tempfile.TemporaryDirectory() as d:
+        mint.mint(d, PRESET[quant], quant, fast=True, seed=5)
+        md, tensors = dseek.read_dir(d)
+    for early in (False, True):
+        m = dsk.Model(dsk.Config.from_metadata(md, 0))
+        for name, t in tensors.items():
+            m.upload(name, t.dtype, t.shape, t.data)
+        state = m.new_state() if early else None
+        m.finalize()
+        if early:
+            m.s, m._extra_states = state, [m.s]
+        logits.append(np.stack([np.array(m.forward(5 + 31 * pos, pos)[0]) for pos in range(4)]))
+        m.close()
+    assert np.array_equal(*logits)
+
+
 if __name__ == "__main__":
     _run(sys.argv[1])
