@@ -19,7 +19,6 @@ struct Plan {
   std::vector<Launch> L;
   std::vector<DkGemv> gemv;
   DkGemv* told = nullptr;                // the same on the device
-  std::vector<void*> lists;              // their runs
   unsigned char* staged = nullptr;       // a feed-forward's staged input, for the launch of its routed experts
   std::vector<DkAttn> attn;
   DkEmbed embed{};
@@ -27,7 +26,6 @@ struct Plan {
   bool ran[3] = {false, false, false};   // a variant is captured when it comes a second time: its first pass is plain launches
   ~Plan() {
     for (cudaGraphExec_t g : graph) if (g) cudaGraphExecDestroy(g);
-    for (void* l : lists) cudaFree(l);
     cudaFree(told);
     cudaFree(staged);
   }
@@ -72,9 +70,9 @@ static int tile_router(const dsk_config& c, const float* src, float* dst, cudaSt
   return 0;
 }
 
-// Whether the chain runs a model of these shapes (decided when the model is made: K-quant matrices are laid out for it)
-static bool fits(const dsk_config& c, int n_ranks) {
-  if (n_ranks != 1 || c.use_mla) return false;
+// Whether the kernels take a model of these shapes
+static bool takes(const dsk_config& c) {
+  if (c.use_mla) return false;
   const int hd = c.qk_nope_head_dim + c.qk_rope_head_dim, sh = c.n_shared_experts * c.moe_intermediate_size, att = c.n_heads * c.v_head_dim;
   if ((c.quant == DSK_Q2_K || c.quant == DSK_Q3_K) && (c.dim > 8192 || c.q_lora_rank > 8192 || c.kv_lora_rank > 8192)) return false;   // (one pass of the norm)
   if (hd % 8 || c.v_head_dim % 8 || c.v_head_dim > 8 * 32 * kDkWarpsB || hd > 4096) return false;
@@ -84,13 +82,14 @@ static bool fits(const dsk_config& c, int n_ranks) {
   for (int n : {c.dim, c.q_lora_rank, c.kv_lora_rank, att, mi, moe ? sh : 0, c.hidden_dim}) if (n % unit) return false;
   auto pow2 = [](int v) { return v > 0 && (v & (v - 1)) == 0; };
   if (c.quant == DSK_F8E5M2 && (c.bs1 < 64 || !pow2(c.bs1) || !pow2(c.bs0))) return false;   // a group of 64 columns has one scale
+  if (c.hidden_dim <= 0 && !(moe && c.first_k_dense_replace <= 0)) return false;
   if (moe && (c.n_active_routed < 1 || c.n_active_routed > 8 || mi <= 0)) return false;
   for (int n : {c.dim, c.q_lora_rank, c.kv_lora_rank, att, mi, moe ? sh : 0, c.hidden_dim}) if (dk_units(c.quant, n) > 255) return false;
   if (dk_whole(DSK_F32, c.dim) / kDkF32Cols > 255) return false;
   auto bytes = [&](int n, int times) { return dk_x_bytes(c.quant, times * dk_whole(c.quant, n)); };
   const int most = std::max(std::max(bytes(c.dim, 1) + dk_whole(DSK_F32, c.dim) * 4, bytes(att, 1)),
                             std::max(bytes(c.q_lora_rank, 1) + bytes(c.kv_lora_rank, 1), std::max(bytes(mi, K) + bytes(moe ? sh : 0, 1), bytes(c.hidden_dim, 1))));
-  return most <= 96 * 1024;   // leaves room for the shallowest rings and the partial sums (at most 24 KB)
+  return most <= 96 * 1024;   // (whether sums and rings fit beside the staged inputs, arrange() says launch by launch)
 }
 
 // A launch in the making: matrices in order, each with the row tiles it has
@@ -100,7 +99,22 @@ struct Draft {
   bool even = false;        // every matrix is cut at the same rows (down projection)
 };
 // what a shape's plan consists of
-struct Lists { DkLists d; void* mem; int part_at, raw_at, ring_at, depth, smem; DkInput in[2]; std::vector<int> kind; };
+struct Arranged {
+  std::vector<DkRun> runs;
+  std::vector<DkWarp> warps;
+  std::vector<DkItem> items;
+  std::vector<int> first, even, kind;   // kind: of a matrix
+  std::vector<unsigned short> units;
+  int max_runs, part_at, raw_at, ring_at, depth, smem;
+  DkInput in[2];
+  DkLists lists;                        // the above on the device (then they are empty here)
+};
+// The plans of a model, worked out and placed when it is made (layers are alike: one a shape); its states only read them
+struct Shapes {
+  std::map<std::vector<int>, Arranged> of;
+  void* mem = nullptr;
+  ~Shapes() { cudaFree(mem); }
+};
 
 // Row tiles to CTAs: by bytes, a tile to the CTA in whose share of the whole it begins; a pair's halves alike.
 static void deal(const Draft& D, int q, int G, std::vector<std::vector<DkRun>>* out) {
@@ -166,16 +180,17 @@ static void share(const std::vector<int>& piece, int NW, std::vector<int>* first
     if (w + 1 == busy) p = n;
   }
 }
-// Lists of a shape, and shared memory: staged inputs | sums of pieces, ahead of them x as it comes | rings as deep as leaves room for a CTA of the other form
-static int plan(const Draft& D, int q, int G, int form, Lists* out) {
+// The plan of a shape, and shared memory: staged inputs | sums of pieces, ahead of them x as it comes | rings as deep as leaves room for a CTA of the other form.
+// false: it does not fit
+static bool arrange(const Draft& D, int q, int G, int form, Arranged* out) {
   const DkGemv& g = D.g;
   const int NW = form ? kDkWarpsB : kDkWarpsA, TR = dk_rows(q), PS = dk_part(q);
   std::vector<std::vector<DkRun>> runs;
-  Lists& L = *out;
+  Arranged& L = *out;
   deal(D, q, G, &runs);
-  int max_runs = 1;
-  for (auto& r : runs) max_runs = std::max(max_runs, (int)r.size());
-  // kinds of matrices (columns, router) and the pieces of their tiles: the choice with the least loaded busiest warp; a piece costs about a unit more than it has
+  L.max_runs = 1;
+  for (auto& r : runs) L.max_runs = std::max(L.max_runs, (int)r.size());
+  // kinds of matrices (columns, router), and for each the ways to cut a tile into pieces
   std::vector<std::pair<int, int>> kinds;
   L.kind.clear();
   for (int j = 0; j < g.nsegs; j++) {
@@ -184,78 +199,79 @@ static int plan(const Draft& D, int q, int G, int form, Lists* out) {
     L.kind.push_back((int)(it - kinds.begin()));
     if (it == kinds.end()) kinds.push_back(k);
   }
-  if (kinds.size() > 3) return fail(-4, "token chain: more than three kinds of matrices in a launch");
-  std::vector<unsigned short> units(3 * 256, 0);
-  std::vector<std::vector<int>> shapes;   // tiles of each kind of a CTA, in order: (kind, tiles)
+  if (kinds.size() > 3) return false;
+  struct Cut { int pieces = 1; std::vector<unsigned short> units; std::vector<int> len; };   // len: units of its pieces
+  std::vector<Cut> cuts[3];
+  const int nk = (int)kinds.size();
+  for (int k = 0; k < nk; k++) {
+    std::vector<int> ways{1, 2, 3, 4, 5, 6, 8, 11, 12, 16};
+    if (kinds[k].second) ways = {std::min(8, kinds[k].first)};   // (the router has no choice)
+    for (int n : ways) {
+      Cut c;
+      c.pieces = n; c.units.assign(256, 0);
+      if (!places(q, kinds[k].second, kinds[k].first, n, c.units.data())) continue;
+      for (int u = 0, len = 1; u < kinds[k].first; u++, len++) if (c.units[u] & kDkPieceEnds) { c.len.push_back(len); len = 0; }
+      cuts[k].push_back(c);
+    }
+  }
+  for (int k = nk; k < 3; k++) cuts[k].resize(1);
+  std::vector<std::vector<int>> shapes;   // of CTAs: (kind, tiles) in order
   for (auto& R : runs) {
     std::vector<int> v;
     for (auto& r : R) { v.push_back(L.kind[r.seg]); v.push_back(r.tiles); }
     if (std::find(shapes.begin(), shapes.end(), v) == shapes.end()) shapes.push_back(v);
   }
-  static const int kPieces[] = {1, 2, 3, 4, 5, 6, 8, 11, 12, 16};
-  const int nk = (int)kinds.size();
-  std::vector<int> pick(3, 0), c(3, 0);
+  // the choice with the least loaded busiest warp; a piece costs about a unit more than it has
+  const Cut* pick[3] = {};
   long long best = 1ll << 60;
   int most_pieces = 0;
   std::vector<int> ends, fp;
-  for (int a : kPieces)
-    for (int b : kPieces)
-      for (int d : kPieces) {
-        c = {a, b, d};
-        if ((nk < 2 && b > 1) || (nk < 3 && d > 1)) continue;
-        bool ok = true;
-        std::vector<unsigned short> tab[3];
-        for (int k = 0; k < nk && ok; k++) {
-          if (kinds[k].second) { if (c[k] != 1) { ok = false; break; } c[k] = std::min(8, kinds[k].first); }   // (the router has no choice)
-          tab[k].resize(256);
-          ok = places(q, kinds[k].second, kinds[k].first, c[k], tab[k].data());
-        }
-        if (!ok) continue;
+  auto add_tiles = [&](const Cut& c, int tiles) { for (int t = 0; t < tiles; t++) for (int n : c.len) ends.push_back(ends.back() + n); };
+  for (const Cut& a : cuts[0])
+    for (const Cut& b : cuts[1])
+      for (const Cut& d : cuts[2]) {
+        const Cut* c[3] = {&a, &b, &d};
         long long worst = 0;
         int pieces = 0;
         for (auto& v : shapes) {
           ends.assign(1, 0);
-          for (size_t i = 0; i < v.size(); i += 2)
-            for (int t = 0; t < v[i + 1]; t++)
-              for (int u = 0, n = 0; u < kinds[v[i]].first; u++) { n++; if (tab[v[i]][u] & kDkPieceEnds) { ends.push_back(ends.back() + n); n = 0; } }
+          for (size_t i = 0; i < v.size(); i += 2) add_tiles(*c[v[i]], v[i + 1]);
           pieces = std::max(pieces, (int)ends.size() - 1);
           share(ends, NW, &fp);
           for (int w = 0; w < NW; w++) worst = std::max(worst, (long long)(ends[fp[w + 1]] - ends[fp[w]]) * 2 + (fp[w + 1] - fp[w]));
         }
-        if (pieces * PS * 4 > 32 * 1024 && best < 1ll << 60) continue;
-        if (worst < best) { best = worst; pick = c; most_pieces = pieces; for (int k = 0; k < nk; k++) std::copy(tab[k].begin(), tab[k].end(), units.begin() + 256 * k); }
+        if (pieces * PS * 4 > 32 * 1024 && best < 1ll << 60) continue;   // (the first choice, uncut tiles, is there for shapes that need more)
+        if (worst < best) { best = worst; most_pieces = pieces; std::copy(c, c + 3, pick); }
       }
-  if (best == 1ll << 60 || most_pieces * PS > 65535) return fail(-4, "token chain: sums of a launch do not fit shared memory");
-  std::vector<DkRun> flat((size_t)G * max_runs, DkRun{-1, 0, 0, 0});
-  std::vector<DkWarp> warps((size_t)G * NW, DkWarp{});
-  std::vector<DkItem> items;
-  std::vector<int> first, even;
+  if (best == 1ll << 60 || most_pieces * PS > 65535) return false;   // (DkItem::parts)
+  L.units.assign(3 * 256, 0);
+  for (int k = 0; k < nk; k++) std::copy(pick[k]->units.begin(), pick[k]->units.end(), L.units.begin() + 256 * k);
+  L.runs.assign((size_t)G * L.max_runs, DkRun{-1, 0, 0, 0});
+  L.warps.assign((size_t)G * NW, DkWarp{});
   for (int cta = 0; cta < G; cta++) {
     auto& R = runs[cta];
     std::vector<int> start(R.size() + 1, 0), piece0(R.size() + 1, 0);   // first units, first pieces of the runs
     ends.assign(1, 0);
     for (size_t i = 0; i < R.size(); i++) {
-      const int nb = g.seg[R[i].seg].nb;
-      for (int t = 0; t < R[i].tiles; t++)
-        for (int u = 0, n = 0; u < nb; u++) { n++; if (units[256 * L.kind[R[i].seg] + u] & kDkPieceEnds) { ends.push_back(ends.back() + n); n = 0; } }
-      start[i + 1] = start[i] + R[i].tiles * nb; piece0[i + 1] = (int)ends.size() - 1;
+      add_tiles(*pick[L.kind[R[i].seg]], R[i].tiles);
+      start[i + 1] = start[i] + R[i].tiles * g.seg[R[i].seg].nb; piece0[i + 1] = (int)ends.size() - 1;
       R[i].piece = piece0[i];
     }
-    std::copy(R.begin(), R.end(), flat.begin() + (size_t)cta * max_runs);
+    std::copy(R.begin(), R.end(), L.runs.begin() + (size_t)cta * L.max_runs);
     share(ends, NW, &fp);
     for (int w = 0; w < NW; w++) {
-      DkWarp& W = warps[(size_t)cta * NW + w];
+      DkWarp& W = L.warps[(size_t)cta * NW + w];
       W.u0 = ends[fp[w]]; W.u1 = ends[fp[w + 1]]; W.piece = fp[w];
       if (W.u0 >= W.u1) { W.u0 = W.u1 = 0; continue; }
       while (W.u0 >= start[W.run + 1]) W.run++;
       const int nb = g.seg[R[W.run].seg].nb;
       W.start = start[W.run]; W.tile = (W.u0 - W.start) / nb; W.kb = W.u0 - W.start - W.tile * nb;
     }
-    first.push_back((int)items.size());
+    L.first.push_back((int)L.items.size());
     for (size_t i = 0; i < R.size(); i++) {
       const DkSeg& S = g.seg[R[i].seg];
       const bool router = S.f32 && q != DSK_F32;
-      const int tr = router ? kDkF32Rows : TR, n = pick[L.kind[R[i].seg]];
+      const int tr = router ? kDkF32Rows : TR, n = pick[L.kind[R[i].seg]]->pieces;
       auto at = [&](size_t run, int k) {   // a row's place in the sums of its tile's first piece
         const int r = k % tr;
         return (unsigned short)((piece0[run] + k / tr * n) * PS + (dk_kq(q) && !router ? (r >> 3) * 32 + (r & 7) * 4 : r));
@@ -267,26 +283,13 @@ static int plan(const Draft& D, int q, int G, int form, Lists* out) {
         I.n = (short)n;
         I.parts = at(i, k);
         if (S.pair) I.parts2 = at(i + 1, k);
-        items.push_back(I);
+        L.items.push_back(I);
       }
       if (S.pair) i++;
     }
   }
-  first.push_back((int)items.size());
-  if (D.even) for (int cta = 0; cta <= G; cta++) even.push_back((int)((long long)D.tiles[0] * cta / G));
-  {
-    const void* src[] = {flat.data(), warps.data(), items.data(), first.data(), units.data(), even.data()};
-    const size_t len[] = {flat.size() * sizeof(DkRun), warps.size() * sizeof(DkWarp), items.size() * sizeof(DkItem), first.size() * 4, units.size() * 2, even.size() * 4};
-    size_t at[7] = {0};
-    for (int i = 0; i < 6; i++) at[i + 1] = align_up(at[i] + len[i], 128);
-    std::vector<char> all(at[6]);
-    for (int i = 0; i < 6; i++) if (len[i]) memcpy(all.data() + at[i], src[i], len[i]);
-    char* d = nullptr;
-    CK(cudaMalloc((void**)&d, all.size()));
-    CK(cudaMemcpy(d, all.data(), all.size(), cudaMemcpyHostToDevice));
-    L.mem = d;
-    L.d = DkLists{(const DkRun*)d, (const DkWarp*)(d + at[1]), (const DkItem*)(d + at[2]), (const int*)(d + at[3]), (const unsigned short*)(d + at[4]), (const int*)(d + at[5]), max_runs};
-  }
+  L.first.push_back((int)L.items.size());
+  if (D.even) for (int cta = 0; cta <= G; cta++) L.even.push_back((int)((long long)D.tiles[0] * cta / G));
   int off = 0;
   for (int i = 0; i < g.nin; i++) {
     DkInput& I = L.in[i] = g.in[i];
@@ -311,13 +314,38 @@ static int plan(const Draft& D, int q, int G, int form, Lists* out) {
   while (L.depth < 4 && off + (L.depth + 1) * ring <= room) L.depth++;
   L.smem = off + L.depth * ring;
   if (form) L.smem = std::max(L.smem, kSmemB);
-  return L.smem <= kSmemLimit ? 0 : fail(-4, "token chain: %d bytes of shared memory", L.smem);
+  return L.smem <= kSmemLimit;
+}
+// all lists on the device, one behind another
+static int place(Shapes& S) {
+  std::vector<char> all;
+  auto put = [&](const auto& v) {
+    const size_t at = all.size(), n = v.size() * sizeof(v[0]);
+    all.resize(align_up(at + n, 128));
+    if (n) memcpy(all.data() + at, v.data(), n);
+    return at;
+  };
+  std::vector<std::array<size_t, 6>> at;
+  for (auto& s : S.of) { Arranged& A = s.second; at.push_back({put(A.runs), put(A.warps), put(A.items), put(A.first), put(A.units), put(A.even)}); }
+  CK(cudaMalloc(&S.mem, all.size()));
+  CK(cudaMemcpy(S.mem, all.data(), all.size(), cudaMemcpyHostToDevice));
+  const char* d = (const char*)S.mem;
+  size_t i = 0;
+  for (auto& s : S.of) {
+    Arranged& A = s.second;
+    const std::array<size_t, 6>& o = at[i++];
+    A.lists = DkLists{(const DkRun*)(d + o[0]), (const DkWarp*)(d + o[1]), (const DkItem*)(d + o[2]), (const int*)(d + o[3]), (const unsigned short*)(d + o[4]), (const int*)(d + o[5]), A.max_runs};
+    A.runs = {}; A.warps = {}; A.items = {}; A.first = {}; A.units = {}; A.even = {};
+  }
+  return 0;
 }
 
-static int build(dsk_model* m, dsk_state* s, Plan* out) {
+// The launches of a token.  Without `out` only their shapes are worked out, into `shapes`; -1 there: one does not fit
+static int build(const dsk_model* m, const dsk_state* s, Shapes& shapes, Plan* out) {
   const dsk_config& c = m->c;
   const int q = c.quant, G = g_sm_count, mi = c.moe_intermediate_size, hd = m->head_dim;
-  Plan& P = *out;
+  Plan none;
+  Plan& P = out ? *out : none;
   P.quant = q;
   auto log2i = [](int v) { int sh = 0; while ((1 << sh) < v) sh++; return sh; };
   auto draft = [&] {
@@ -342,26 +370,22 @@ static int build(dsk_model* m, dsk_state* s, Plan* out) {
   };
   auto tensor = [&](Draft& D, const DTensor& t, float* o, int in, int segment = 0) -> DkSeg& { return matrix(D, t.w, t.scale, t.rows, t.cols, o, in, segment); };
   auto expert = [&](DkSeg& S, const DTensor& t, int k) { S.slot = k; S.w_stride = (long long)t.expert_bytes; S.s_stride = (long long)t.scale_expert; };
-  std::map<std::vector<int>, Lists> seen;   // layers are alike: a plan is made once per shape
-  auto key_of = [&](const Draft& D, int form) {
-    std::vector<int> key{form, D.g.nsegs, D.g.nin, D.even};   // (all that plan() reads)
+  auto planned = [&](const Draft& D, int form) -> const Arranged* {
+    std::vector<int> key{form, D.g.nsegs, D.g.nin, D.even};   // (all that arrange() reads)
     for (const DkInput& I : D.g.in) { key.push_back(I.n); key.push_back(I.seg); key.push_back(I.norm != nullptr); }
     for (int j = 0; j < D.g.nsegs; j++) { key.push_back(D.g.seg[j].rows); key.push_back(D.g.seg[j].nb); key.push_back((D.g.seg[j].f32 << 1) | D.g.seg[j].pair); }
-    return key;
-  };
-  auto planned = [&](const Draft& D, int form) -> const Lists* {
-    auto it = seen.find(key_of(D, form));
-    if (it != seen.end()) return &it->second;
-    Lists L{};
-    if (plan(D, q, G, form, &L)) return nullptr;
-    P.lists.push_back(L.mem);
-    return &(seen[key_of(D, form)] = L);
+    auto it = shapes.of.find(key);
+    if (it != shapes.of.end()) return &it->second;
+    if (out) { fail(-4, "dsk_state_create: tensors of the model are missing"); return nullptr; }
+    Arranged& A = shapes.of[key];
+    return arrange(D, q, G, form, &A) ? &A : nullptr;
   };
   int form = 0;
   auto add = [&](Draft& D, int layer, const char* name, const int* down_tiles = nullptr) -> int {
     form ^= 1;
-    const Lists* L = planned(D, form);
-    if (!L) return -4;
+    const Arranged* L = planned(D, form);
+    if (!L) return -1;
+    if (!out) return 0;
     DkGemv& g = D.g;
     g.part_at = L->part_at; g.raw_at = L->raw_at; g.ring_at = L->ring_at; g.depth = L->depth;
     for (int i = 0; i < g.nin; i++) { const DkInput o = g.in[i]; g.in[i] = L->in[i]; g.in[i].x = o.x; g.in[i].norm = o.norm; g.in[i].ready = o.ready; }
@@ -375,12 +399,12 @@ static int build(dsk_model* m, dsk_state* s, Plan* out) {
       else { S.xa = I.at + col * 4; S.xb = 0; }
       if (S.f32 && I.f32_at >= 0) S.xa = I.f32_at;
     }
-    P.L.push_back(Launch{GEMV, layer, G, L->smem, (int)P.gemv.size(), form, name, L->d});
+    P.L.push_back(Launch{GEMV, layer, G, L->smem, (int)P.gemv.size(), form, name, L->lists});
     P.L.back().lists.down_tiles = down_tiles;
     P.gemv.push_back(g);
     return 0;
   };
-  CK(cudaMalloc((void**)&P.staged, (size_t)dk_x_bytes(q, dk_whole(q, c.dim)) + 16));   // (and the norm's factor)
+  if (out) CK(cudaMalloc((void**)&P.staged, (size_t)dk_x_bytes(q, dk_whole(q, c.dim)) + 16));   // (and the norm's factor)
   {
     DkEmbed& e = P.embed;
     e.table = m->embed.w; e.scale = m->embed.scale; e.x = s->x; e.ctrl = s->ctrl; e.log = s->token_log; e.step = s->step;
@@ -388,7 +412,7 @@ static int build(dsk_model* m, dsk_state* s, Plan* out) {
     P.L.push_back(Launch{EMBED, -1, cdiv(c.dim, 256), 0, 0, 0, "embed", DkLists{}});
   }
   for (int l = 0; l < c.n_layers; l++) {
-    Layer& L = m->layers[l];
+    const Layer& L = m->layers[l];
     {
       Draft D = draft();
       input(D, s->x, L.rms_att, c.dim);
@@ -396,7 +420,7 @@ static int build(dsk_model* m, dsk_state* s, Plan* out) {
       tensor(D, L.wkv_a, s->kv_a, 0);
       D.g.epi = EPI_STORE;
       if (l == 0) D.g.reset = &s->ctrl->argmax_key;
-      if (add(D, l, "proj")) return -4;
+      if (add(D, l, "proj")) return -1;
     }
     {   // query up-projection beside keys and values: both wait for the same launch
       Draft D = draft();
@@ -404,7 +428,7 @@ static int build(dsk_model* m, dsk_state* s, Plan* out) {
       input(D, s->kv_a, L.rms_kv_a, c.kv_lora_rank);
       tensor(D, L.wkv_b, s->kv_b, D.g.nin - 1);
       D.g.epi = EPI_KVB; D.g.kcache = L.kcache; D.g.vcache = L.vcache;
-      if (add(D, l, "q_b+kv_b")) return -4;
+      if (add(D, l, "q_b+kv_b")) return -1;
     }
     {
       DkAttn a{};
@@ -426,7 +450,7 @@ static int build(dsk_model* m, dsk_state* s, Plan* out) {
       input(D, s->xb2, nullptr, c.n_heads * c.v_head_dim);
       tensor(D, L.wo, s->x, 0);
       D.g.epi = EPI_RESID;
-      if (add(D, l, "wo")) return -4;
+      if (add(D, l, "wo")) return -1;
     }
     const int sh = L.is_moe ? c.n_shared_experts * mi : c.hidden_dim, K = L.is_moe ? c.n_active_routed : 0;
     {   // router logits and the feed-forward that every token takes (shared experts, or the dense layer)
@@ -439,7 +463,7 @@ static int build(dsk_model* m, dsk_state* s, Plan* out) {
       }
       if (sh > 0) { tensor(D, L.is_moe ? L.sw1 : L.w1, s->hbs, 0).pair = 1; tensor(D, L.is_moe ? L.sw3 : L.w3, nullptr, 0); }
       D.g.epi = EPI_STORE;
-      if (D.g.nsegs > 0 && add(D, l, L.is_moe ? "gate+shared" : "glu")) return -4;
+      if (D.g.nsegs > 0 && add(D, l, L.is_moe ? "gate+shared" : "glu")) return -1;
     }
     DkRoute r{};
     r.logits = s->moe_logits; r.bias = L.gate_bias; r.scores = s->moe_scores; r.act_w = s->act_w; r.act = s->act;
@@ -453,8 +477,8 @@ static int build(dsk_model* m, dsk_state* s, Plan* out) {
     for (int k = 0; k < K; k++) expert(tensor(down, L.w2, s->x, 0, k), L.w2, k);
     down.g.epi = EPI_DOWN; down.even = true; down.g.route = K ? ROUTE_READ : ROUTE_NONE; down.g.r = r;
     if (K) {   // routing + routed experts
-      const Lists* dl = planned(down, form);   // (the form after next)
-      if (!dl) return -4;
+      const Arranged* dl = planned(down, form);   // (the form after next)
+      if (!dl) return -1;
       Draft D = draft();
       input(D, nullptr, nullptr, c.dim);
       D.g.in[0].ready = P.staged;
@@ -466,20 +490,49 @@ static int build(dsk_model* m, dsk_state* s, Plan* out) {
       }
       D.g.epi = EPI_STORE; D.g.route = ROUTE_MAKE; D.g.r = r;
       D.g.r.w2 = L.w2.w; D.g.r.w2_stride = (long long)L.w2.expert_bytes; D.g.r.w2_tile = (long long)dk_units(q, mi) * dk_unit_bytes(q);
-      if (add(D, l, "glu", dl->d.down_tiles)) return -4;
+      if (add(D, l, "glu", dl->lists.down_tiles)) return -1;
     }
-    if (add(down, l, "down")) return -4;
+    if (add(down, l, "down")) return -1;
   }
   {
     Draft D = draft();
     input(D, s->x, m->rms_final, c.dim);
     tensor(D, m->wcls, s->logits, 0);
     D.g.epi = EPI_LOGITS; D.g.argmax = &s->ctrl->argmax_key;
-    if (add(D, -1, "lm_head")) return -4;
+    if (add(D, -1, "lm_head")) return -1;
   }
+  if (!out) return 0;
   CK(cudaMalloc((void**)&P.told, P.gemv.size() * sizeof(DkGemv)));
   CK(cudaMemcpy(P.told, P.gemv.data(), P.gemv.size() * sizeof(DkGemv), cudaMemcpyHostToDevice));
   return 0;
+}
+
+// The plans of a model of these shapes, or null: the interpreter runs it (decided when the model is made, since matrices are laid out for the chain)
+static std::shared_ptr<Shapes> fits(const dsk_config& c, int n_ranks) {
+  if (n_ranks != 1 || !takes(c)) return nullptr;
+  // a model of these sizes and a state, neither with any memory
+  static float there;   // (a norm)
+  const int hd = c.qk_nope_head_dim + c.qk_rope_head_dim, mi = c.moe_intermediate_size, sh = c.n_shared_experts * mi;
+  auto sized = [](int rows, int cols) { DTensor t; t.rows = rows; t.cols = cols; return t; };
+  dsk_model m;
+  m.c = c; m.head_dim = hd; m.rms_final = &there; m.wcls = sized(c.vocab_size, c.dim);
+  m.layers.resize(c.n_layers);
+  for (int l = 0; l < c.n_layers; l++) {
+    Layer& L = m.layers[l];
+    L.is_moe = c.n_routed_experts > 0 && l >= c.first_k_dense_replace;
+    L.rms_att = L.rms_ffn = L.rms_q_a = L.rms_kv_a = &there;
+    const int ff = L.is_moe ? mi : c.hidden_dim;
+    L.wq = sized(c.n_heads * hd, c.dim); L.wq_a = sized(c.q_lora_rank, c.dim); L.wq_b = sized(c.n_heads * hd, c.q_lora_rank);
+    L.wkv_a = sized(c.kv_lora_rank + c.qk_rope_head_dim, c.dim); L.wkv_b = sized(c.n_heads * (c.qk_nope_head_dim + c.v_head_dim), c.kv_lora_rank);
+    L.wo = sized(c.dim, c.n_heads * c.v_head_dim);
+    L.w1 = L.w3 = sized(ff, c.dim); L.w2 = sized(c.dim, ff);
+    L.sw1 = L.sw3 = sized(sh, c.dim); L.sw2 = sized(c.dim, sh);
+  }
+  dsk_state s;
+  Ctrl ctrl;
+  s.ctrl = &ctrl;
+  auto shapes = std::make_shared<Shapes>();
+  return build(&m, &s, *shapes, nullptr) ? nullptr : shapes;
 }
 
 template <int Q>

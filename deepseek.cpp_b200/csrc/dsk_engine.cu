@@ -22,10 +22,12 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <string>
 #include <vector>
 
 #include <algorithm>
+#include <array>
 #include "dsk_kernels.cuh"
 #include "dsk_mega.cuh"
 #include "dsk_decode.cuh"
@@ -138,7 +140,9 @@ struct Uploader {
 namespace hyb { struct Model; struct State; }   // layer-list model family (dsk_hybrid_host.cuh)
 namespace dk {                                  // token chain of one GPU (dsk_decode_host.cuh)
 struct Plan;
-static bool fits(const dsk_config& c, int n_ranks);
+struct Shapes;
+static std::shared_ptr<Shapes> fits(const dsk_config& c, int n_ranks);
+static int place(Shapes& S);
 static int set_attributes();
 static int tile(int quant, const unsigned char* src, uint8_t* dst, int rows, int cols, int count, cudaStream_t st, bool wait);
 static size_t router_bytes(const dsk_config& c);
@@ -151,6 +155,7 @@ struct dsk_model {
   int head_dim = 0;
   int rank = 0, n_ranks = 1;
   bool chain = false;          // tokens run as the launches of dsk_decode.cuh; matrices lie in its tiles
+  std::shared_ptr<dk::Shapes> shapes;   // their plans
   int expert_first = 0, expert_count = 0;
   std::vector<Layer> layers;
   DTensor embed, wcls;
@@ -383,7 +388,9 @@ extern "C" dsk_model* dsk_model_create(const dsk_config* cfg, int rank, int n_ra
   m->head_dim = cfg->qk_nope_head_dim + cfg->qk_rope_head_dim;
   m->rank = rank;
   m->n_ranks = n_ranks;
-  m->chain = g_engine == ENG_CHAIN && (g_use_mma || cfg->quant != DSK_F8E5M2) && dk::fits(*cfg, n_ranks);
+  if (g_engine == ENG_CHAIN && (g_use_mma || cfg->quant != DSK_F8E5M2)) m->shapes = dk::fits(*cfg, n_ranks);
+  m->chain = m->shapes != nullptr;
+  if (m->chain && dk::place(*m->shapes)) { delete m; return nullptr; }
   const int E = cfg->n_routed_experts;
   const int per = E > 0 ? cdiv(E, n_ranks) : 0;
   m->expert_first = std::min(E, rank * per);
@@ -1570,7 +1577,7 @@ static int run_stages(dsk_model* m, dsk_state* s, int b, int e, int from_argmax,
 
 static int build_chain(dsk_model* m, dsk_state* s) {
   s->chain = new dk::Plan();
-  return dk::build(m, s, s->chain);
+  return dk::build(m, s, *m->shapes, s->chain);
 }
 static void drop_chain(dsk_state* s) {
   delete s->chain;

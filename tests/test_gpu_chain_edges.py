@@ -205,5 +205,35 @@ def test_state_before_finalize(quant):
     assert np.array_equal(*logits)
 
 
+@pytest.mark.parametrize("vocab,chain", [(1000003, True), (2000003, False)])
+def test_large_vocabulary(vocab, chain):
+    """The sums of an LM head's rows (64 floats a tile of 16 rows) fit a CTA's shared memory up to about 1.5 million rows; the interpreter runs what does not."""
+    import dseek
+    import dsk
+    import mint
+    import torch
+    logits = []
+    with tempfile.TemporaryDirectory() as d:
+        mint.mint(d, "tiny_v2", "q2_k", fast=True, seed=5, dim=256)
+        md, tensors = dseek.read_dir(d)
+    for rows in (1024, vocab):
+        cfg = dsk.Config.from_metadata(md, 0)
+        cfg.vocab_size = rows
+        m = dsk.Model(cfg)
+        for name, t in tensors.items():
+            if name in ("model.embed.weight", "model.output.weight"):
+                q = torch.from_numpy(np.array(t.data)).cuda()
+                q = q.repeat(-(-rows // 1024), 1)[:rows].contiguous()
+                torch.cuda.synchronize()
+                m.upload_device(name, t.dtype, q.shape, q.data_ptr(), q.numel())
+            else:
+                m.upload(name, t.dtype, t.shape, t.data)
+        m.finalize()
+        assert (m.launches_per_forward() > 1) == (chain or rows == 1024)
+        logits.append(np.stack([np.array(m.forward(5 + 31 * pos, pos)[0]) for pos in range(3)]))
+        m.close()
+    assert np.array_equal(logits[1], np.tile(logits[0], (1, -(-vocab // 1024)))[:, :vocab])
+
+
 if __name__ == "__main__":
     _run(sys.argv[1])
