@@ -76,68 +76,120 @@ __host__ __device__ inline int dk_place_of(bool pairs, int nb, int unit) {
   return at;
 }
 
-// rows as the file has them -> tiles, a warp a unit.  src: matrices of `rows` rows of n values, one behind another
+// rows as the file has them -> tiles.  src: `bytes` on a 16-byte boundary, matrices of `rows` rows of n values, one behind another; `tiles`: row tiles of all of them.
+// K-quants: a CTA takes eight blocks side by side of a tile's 16 rows.  Blocks of 110 bytes begin on any even address, so the rows come as whole words into shared
+// memory, every block there on a boundary of four bytes, and a warp makes a unit with word operations.  Bound by memory: 1.61 GB of Q3_K from the device,
+// allocation of the tiles included, 2.2 ms (a lane that gathered its unit byte by byte 5.0; laid out as before the chain 2.4).
+template <int Q>
+__global__ void __launch_bounds__(256) dk_tile_kq(const unsigned char* __restrict__ src, unsigned char* __restrict__ dst, int rows, int n, long long tiles, size_t bytes) {
+  constexpr int BB = Q == Q_Q2K ? kQ2Bytes : kQ3Disk, SB = (BB + 3) / 4 * 4, RW = (8 * BB + 5) / 4;   // words that hold eight blocks at any even address
+  __shared__ __align__(16) unsigned char blk[16][8][SB];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3, h = t >> 1, c = t & 1;   // (h, c: the lane's quarter)
+  const int nb = n >> 8, per = (rows + 15) / 16, chunks = (nb + 7) / 8;
+  for (long long job = blockIdx.x; job < tiles * chunks; job += gridDim.x) {
+    const long long rt = job / chunks, mat = rt / per;
+    const int b0 = (int)(job - rt * chunks) * 8, blocks = min(8, nb - b0), r0 = (int)(rt - mat * per) * 16, nr = min(16, rows - r0);
+    __syncthreads();
+    const long long base = ((mat * rows + r0) * nb + b0) * BB;   // the first row's blocks; row r's `pitch` bytes further on
+    const int pitch = nb * BB, len = blocks * BB;
+    for (int i0 = tid; i0 < nr * RW; i0 += 256 * 4) {   // (four loads under way)
+      uint32_t v[4];
+      int row[4], p[4];   // of a word: its row, the place in it that the word begins at (-2 where that is a boundary ahead of it)
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const int i = i0 + 256 * j;
+        row[j] = i / RW;
+        const long long from = base + (long long)row[j] * pitch, at = (from & ~3ll) + 4 * (i - row[j] * RW);
+        p[j] = i < nr * RW && at < from + len ? (int)(at - from) : len;
+        v[j] = 0u;
+        if (p[j] < len) v[j] = at + 4 <= (long long)bytes ? *reinterpret_cast<const uint32_t*>(src + at) : *reinterpret_cast<const unsigned short*>(src + at);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        if constexpr (BB % 4 == 0) { if (p[j] < len) *reinterpret_cast<uint32_t*>(&blk[row[j]][p[j] / BB][p[j] % BB]) = v[j]; }
+        else {
+#pragma unroll
+          for (int k = 0; k < 2; k++) {
+            const int at = p[j] + 2 * k;
+            if (at >= 0 && at < len) *reinterpret_cast<unsigned short*>(&blk[row[j]][at / BB][at % BB]) = (unsigned short)(v[j] >> (16 * k));
+          }
+        }
+      }
+    }
+    __syncthreads();
+    if (warp >= blocks) continue;
+    unsigned char* o = dst + (size_t)(rt * nb + dk_place_of(true, nb, b0 + warp)) * DkTraits<Q>::unit;
+    auto word = [&](int half, int at) { return g + 8 * half < nr ? *reinterpret_cast<const uint32_t*>(&blk[g + 8 * half][warp][at]) : 0u; };   // of row g, g + 8
+    const int pick = c ? 0x7531 : 0x6420;   // bytes c, c + 2, c + 4, c + 6 of eight
+    if constexpr (Q == Q_Q2K) {
+#pragma unroll
+      for (int hh = 0; hh < 2; hh++) {
+        const int at = 16 + 32 * hh + 4 * t;
+        *reinterpret_cast<uint4*>(o + 512 * hh + 16 * lane) = make_uint4(word(0, at), word(1, at), word(0, at + 16), word(1, at + 16));
+      }
+      *reinterpret_cast<uint2*>(o + 1024 + 8 * lane) = make_uint2(__byte_perm(word(0, 8 * h), word(0, 8 * h + 4), pick), __byte_perm(word(1, 8 * h), word(1, 8 * h + 4), pick));
+      if (t < 2) *reinterpret_cast<uint32_t*>(o + 1280 + 8 * g + 4 * t) = word(t, 80);
+    } else {
+      uint32_t nib[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+      for (int hh = 0; hh < 2; hh++) {
+        uint32_t b[4];
+#pragma unroll
+        for (int w = 0; w < 4; w++) {   // row g + 8 (w & 1), columns 4t + 16 (w >> 1)
+          const int at = 4 * t + 16 * (w >> 1);
+          const uint32_t q = word(w & 1, 32 + 32 * hh + at), hm = word(w & 1, at) >> (4 * hh);
+          uint32_t u[4];
+#pragma unroll
+          for (int s = 0; s < 4; s++) u[s] = ((q >> (2 * s)) & 0x03030303u) | (((hm >> s) & 0x01010101u) << 2);
+          b[w] = u[0] | (u[1] << 3) | ((u[2] & 0x06060606u) << 5);
+          nib[w] |= ((u[2] & 0x01010101u) | (u[3] << 1)) << (4 * hh);
+        }
+        *reinterpret_cast<uint4*>(o + 512 * hh + 16 * lane) = make_uint4(b[0], b[1], b[2], b[3]);
+      }
+      *reinterpret_cast<uint4*>(o + 1024 + 16 * lane) = make_uint4(nib[0], nib[1], nib[2], nib[3]);
+      unsigned long long sc = 0;
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const uint32_t lo = (__byte_perm(word(i, 96), word(i, 100), pick) >> (4 * h)) & 0x0F0F0F0Fu, hi = word(i, 104);
+#pragma unroll
+        for (int k = 0; k < 4; k++)   // sub-block 8h + 2k + c
+          sc |= (unsigned long long)(((lo >> (8 * k)) & 15u) | (((hi >> (8 * ((2 * k + c) & 3) + 4 * h + 2 * (k >> 1))) & 3u) << 4)) << (24 * i + 6 * k);
+      }
+      *reinterpret_cast<uint32_t*>(o + 1536 + 4 * lane) = (uint32_t)sc;
+      *reinterpret_cast<unsigned short*>(o + 1664 + 2 * lane) = (unsigned short)(sc >> 32);
+      if (t < 2) *reinterpret_cast<unsigned short*>(o + 1728 + 4 * g + 2 * t) = (unsigned short)word(t, 108);
+    }
+  }
+}
+// the rest, 16-byte words (n is a multiple of 16, 16 or 4 values: whole words), a warp a unit
 template <int Q>
 __global__ void __launch_bounds__(256) dk_tile_kernel(const unsigned char* __restrict__ src, unsigned char* __restrict__ dst, int rows, int n, long long units) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  constexpr int R = DkTraits<Q>::rows;
+  constexpr int R = DkTraits<Q>::rows, ES = Q == Q_F8 ? 1 : Q == Q_F16 ? 2 : 4;
   const int nb = (n + DkTraits<Q>::cols - 1) / DkTraits<Q>::cols, per = (rows + R - 1) / R;
-  for (long long unit = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); unit < units; unit += (long long)gridDim.x * 8) {
-    const long long rt = unit / nb, mat = rt / per;
-    const int r0 = (int)(rt - mat * per) * R;
-    int b = (int)(unit - rt * nb);
-    unsigned char* o = dst + (size_t)unit * DkTraits<Q>::unit;
-    if constexpr (QTraits<Q>::kq) {
-      b = dk_unit_at(true, nb, b);
-      constexpr int BB = Q == Q_Q2K ? kQ2Bytes : kQ3Disk;
-      const unsigned char* blk[2];
-      for (int i = 0; i < 2; i++) blk[i] = r0 + g + 8 * i < rows ? src + ((size_t)(mat * rows + r0 + g + 8 * i) * nb + b) * BB : nullptr;
-      const int h = t >> 1, c = t & 1;   // the lane's quarter
-      if constexpr (Q == Q_Q2K) {
-        for (int hh = 0; hh < 2; hh++)
-          for (int i = 0; i < 16; i++) {   // word i / 4: row g + 8 (word & 1), columns + 16 (word >> 1)
-            const unsigned char* p = blk[(i >> 2) & 1];
-            o[512 * hh + 16 * lane + i] = p ? p[16 + 32 * hh + 4 * t + 16 * (i >> 3) + (i & 3)] : 0;
-          }
-        for (int i = 0; i < 8; i++) {
-          const unsigned char* p = blk[i >> 2];
-          o[1024 + 8 * lane + i] = p ? p[8 * h + 2 * (i & 3) + c] : 0;
-        }
-        if (t < 2) for (int i = 0; i < 4; i++) o[1280 + 8 * g + 4 * t + i] = blk[t] ? blk[t][80 + i] : 0;
-      } else {
-        unsigned char nib[16];
-        for (int i = 0; i < 16; i++) nib[i] = 0;
-        for (int hh = 0; hh < 2; hh++)
-          for (int i = 0; i < 16; i++) {
-            const unsigned char* p = blk[(i >> 2) & 1];
-            const int l = 4 * t + 16 * (i >> 3) + (i & 3);
-            int u[4];
-            for (int s = 0; s < 4; s++) u[s] = p ? ((p[32 + 32 * hh + l] >> (2 * s)) & 3) + 4 * ((p[l] >> (4 * hh + s)) & 1) : 0;
-            o[512 * hh + 16 * lane + i] = (unsigned char)(u[0] | (u[1] << 3) | ((u[2] >> 1) << 6));
-            nib[i] |= (unsigned char)(((u[2] & 1) | (u[3] << 1)) << (4 * hh));
-          }
-        for (int i = 0; i < 16; i++) o[1024 + 16 * lane + i] = nib[i];
-        unsigned long long sc = 0;
-        for (int i = 0; i < 8; i++) {   // row g + 8 (i >> 2), sub-block 8h + 2s + c
-          const unsigned char* p = blk[i >> 2];
-          const int j = 8 * h + 2 * (i & 3) + c;
-          const int lob = p ? p[96 + (j & 7)] : 0, lo4 = j < 8 ? lob & 0xF : lob >> 4;
-          const int hi2 = p ? (p[104 + (j & 3)] >> (2 * (j >> 2))) & 3 : 0;
-          sc |= (unsigned long long)(lo4 | (hi2 << 4)) << (6 * i);
-        }
-        for (int i = 0; i < 4; i++) o[1536 + 4 * lane + i] = (unsigned char)(sc >> (8 * i));
-        for (int i = 0; i < 2; i++) o[1664 + 2 * lane + i] = (unsigned char)(sc >> (32 + 8 * i));
-        if (t < 2) for (int i = 0; i < 2; i++) o[1728 + 4 * g + 2 * t + i] = blk[t] ? blk[t][108 + i] : 0;
-      }
-    } else {   // 16-byte words (n is a multiple of 16, 16 or 4 values: whole words)
-      constexpr int ES = Q == Q_F8 ? 1 : Q == Q_F16 ? 2 : 4;
+  // (four units side by side a warp: one division for them, sixteen loads under way)
+  for (long long u0 = 4 * ((long long)blockIdx.x * 8 + (threadIdx.x >> 5)); u0 < units; u0 += (long long)gridDim.x * 32) {
+    long long rt = u0 / nb;
+    int b = (int)(u0 - rt * nb), tile = (int)(rt % per);
+    long long row0 = rt / per * rows;   // the matrix's first row
+    uint4 v[4][4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+#pragma unroll
       for (int k = 0; k < 4; k++) {
-        const int r = r0 + (Q == Q_F8 ? g + 8 * (k & 1) : k), col = b * DkTraits<Q>::cols + (Q == Q_F8 ? 64 * (k >> 1) + 16 * t : lane * (16 / ES));
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (r < rows && col < n) v = *reinterpret_cast<const uint4*>(src + ((size_t)(mat * rows + r) * n + col) * ES);
-        *reinterpret_cast<uint4*>(o + 512 * k + 16 * lane) = v;
+        const int r = tile * R + (Q == Q_F8 ? g + 8 * (k & 1) : k), col = b * DkTraits<Q>::cols + (Q == Q_F8 ? 64 * (k >> 1) + 16 * t : lane * (16 / ES));
+        v[j][k] = make_uint4(0u, 0u, 0u, 0u);
+        if (u0 + j < units && r < rows && col < n) v[j][k] = *reinterpret_cast<const uint4*>(src + ((size_t)(row0 + r) * n + col) * ES);
       }
+      if (++b == nb) { b = 0; if (++tile == per) { tile = 0; row0 += rows; } }
     }
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+      if (u0 + j < units) {
+        unsigned char* o = dst + (size_t)(u0 + j) * DkTraits<Q>::unit;
+#pragma unroll
+        for (int k = 0; k < 4; k++) *reinterpret_cast<uint4*>(o + 512 * k + 16 * lane) = v[j][k];
+      }
   }
 }
 __global__ void __launch_bounds__(256) dk_tile_router(const float* __restrict__ src, unsigned char* __restrict__ dst, int rows, int n, int units) {

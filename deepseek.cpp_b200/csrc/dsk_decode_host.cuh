@@ -40,8 +40,12 @@ static int slot_bytes(int q) { return q == DSK_Q2_K ? DkTraits<Q_Q2K>::slot : Dk
 // `count` matrices as the file has them -> tiles
 template <int Q>
 static void tile_q(const unsigned char* src, uint8_t* dst, int rows, int cols, int count, cudaStream_t st) {
-  const long long units = (long long)(dk_matrix_bytes(Q, rows, cols) / (size_t)dk_unit_bytes(Q)) * count;
-  if (units > 0) dk_tile_kernel<Q><<<(unsigned)std::min<long long>((units + 7) / 8, 1 << 16), 256, 0, st>>>(src, dst, rows, cols, units);
+  const long long tiles = (long long)cdiv(rows, DkTraits<Q>::rows) * count, units = tiles * dk_units(Q, cols);
+  if (units == 0) return;
+  if constexpr (DkTraits<Q>::kq)
+    dk_tile_kq<Q><<<(unsigned)std::min<long long>(tiles * cdiv(cols, 2048), 1 << 16), 256, 0, st>>>(src, dst, rows, cols, tiles, disk_row_bytes(Q, cols) * rows * count);
+  else
+    dk_tile_kernel<Q><<<(unsigned)std::min<long long>((units + 31) / 32, 1 << 16), 256, 0, st>>>(src, dst, rows, cols, units);
 }
 static int tile(int quant, const unsigned char* src, uint8_t* dst, int rows, int cols, int count, cudaStream_t st, bool wait) {
   switch (quant) {
@@ -248,6 +252,9 @@ static bool arrange(const Draft& D, int q, int G, int form, Arranged* out) {
   for (int k = 0; k < nk; k++) std::copy(pick[k]->units.begin(), pick[k]->units.end(), L.units.begin() + 256 * k);
   L.runs.assign((size_t)G * L.max_runs, DkRun{-1, 0, 0, 0});
   L.warps.assign((size_t)G * NW, DkWarp{});
+  size_t rows = 0;
+  for (int j = 0; j < g.nsegs; j++) rows += (size_t)D.tiles[j] * TR;
+  L.items.reserve(rows);
   for (int cta = 0; cta < G; cta++) {
     auto& R = runs[cta];
     std::vector<int> start(R.size() + 1, 0), piece0(R.size() + 1, 0);   // first units, first pieces of the runs
@@ -272,19 +279,17 @@ static bool arrange(const Draft& D, int q, int G, int form, Arranged* out) {
       const DkSeg& S = g.seg[R[i].seg];
       const bool router = S.f32 && q != DSK_F32;
       const int tr = router ? kDkF32Rows : TR, n = pick[L.kind[R[i].seg]]->pieces;
-      auto at = [&](size_t run, int k) {   // a row's place in the sums of its tile's first piece
-        const int r = k % tr;
-        return (unsigned short)((piece0[run] + k / tr * n) * PS + (dk_kq(q) && !router ? (r >> 3) * 32 + (r & 7) * 4 : r));
-      };
-      for (int k = 0; k < R[i].tiles * tr; k++) {
-        DkItem I{};
-        I.r = R[i].tile0 * tr + k;
-        I.seg = (short)(I.r < S.rows ? R[i].seg : -1);
-        I.n = (short)n;
-        I.parts = at(i, k);
-        if (S.pair) I.parts2 = at(i + 1, k);
-        L.items.push_back(I);
-      }
+      for (int t = 0; t < R[i].tiles; t++)
+        for (int r = 0; r < tr; r++) {   // a row's place in the sums of its tile's first piece
+          const int place = t * n * PS + (dk_kq(q) && !router ? (r >> 3) * 32 + (r & 7) * 4 : r);
+          DkItem I{};
+          I.r = (R[i].tile0 + t) * tr + r;
+          I.seg = (short)(I.r < S.rows ? R[i].seg : -1);
+          I.n = (short)n;
+          I.parts = (unsigned short)(piece0[i] * PS + place);
+          if (S.pair) I.parts2 = (unsigned short)(piece0[i + 1] * PS + place);
+          L.items.push_back(I);
+        }
       if (S.pair) i++;
     }
   }

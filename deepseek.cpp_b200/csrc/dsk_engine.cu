@@ -125,13 +125,13 @@ struct Layer {
 // chunk i travels over PCIe (cudaMemcpy2DAsync on the upload stream, which also re-pitches rows), the host thread copies
 // chunk i+1 out of the page cache.  dsk_model_finalize() joins the stream.
 struct Uploader {
-  static constexpr size_t kChunk = 32u << 20;
+  static constexpr size_t kChunk = 32u << 20, kRaw = 256u << 20;
   void* pin[2] = {nullptr, nullptr};
   cudaEvent_t ev[2] = {nullptr, nullptr};
   cudaStream_t st = nullptr;
   int cur = 0;
   std::vector<void*> staging;   // device staging buffers (Q3_K repack), freed at finalize
-  void* raw = nullptr;          // rows as the file has them, on their way into tiles (reused: copies and kernels of the stream follow one another)
+  void* raw = nullptr;          // up to kRaw bytes of rows as the file has them, on their way into tiles (reused: copies and kernels of the stream follow one another)
   size_t raw_cap = 0;
   size_t bytes = 0;
   double seconds = 0;
@@ -572,6 +572,23 @@ static int rows_on_device(dsk_model* m, const void* data, size_t bytes, int on_d
   *out = u.raw;
   return copy_rows(m, u.raw, bytes, data, bytes, bytes, 1, on_dev);
 }
+// `count` matrices -> the tiles of the token chain.  What passes through the upload's buffer does so in pieces of whole matrices or whole row tiles, so that a large
+// tensor does not lie on the device twice (pieces of 64 MB: some sizes took a tenth longer from the host than in one piece)
+static int tile_rows(dsk_model* m, int q, const void* data, uint8_t* dst, int rows, int cols, int count, int on_dev) {
+  const size_t rb = disk_row_bytes(q, cols), tiled = dk_matrix_bytes(q, rows, cols);
+  const bool whole = on_dev && (uintptr_t)data % 16 == 0;
+  const int R = dk_rows(q), mats = whole ? count : (int)std::max<size_t>(1, std::min<size_t>(count, Uploader::kRaw / std::max<size_t>(1, rb * rows)));
+  const int step = whole || rb * rows <= Uploader::kRaw ? rows : std::max(R, (int)(Uploader::kRaw / rb) / R * R);
+  for (int e = 0; e < count; e += mats)
+    for (int r = 0; r < rows; r += step) {
+      const int n = std::min(mats, count - e), nr = std::min(step, rows - r);
+      const void* src = nullptr;
+      if (rows_on_device(m, (const char*)data + ((size_t)e * rows + r) * rb, (size_t)n * nr * rb, on_dev, &src)) return -2;
+      const size_t o = (size_t)e * tiled + (size_t)(r / R) * dk_units(q, cols) * dk_unit_bytes(q);
+      if (dk::tile(q, (const unsigned char*)src, dst + o, nr, cols, n, on_dev ? nullptr : m->up.st, on_dev)) return -2;
+    }
+  return 0;
+}
 // The router's rows into the tiles of the token chain (here and not when the model is finished: a state may be made before that)
 static int upload_router(dsk_model* m, float** dst, int dtype, const int64_t shape[4], const void* data, size_t nbytes, int on_dev, const char* name) {
   const dsk_config& c = m->c;
@@ -639,9 +656,7 @@ static int upload_weight(dsk_model* m, DTensor& t, int rows, int cols, bool expe
   if (m->chain) {   // rows as the file has them -> tiles (dsk_decode.cuh); one GPU: the whole tensor
     t.expert_bytes = dk_matrix_bytes(q, rc, cc);
     if (dmalloc(m, (void**)&t.w, t.expert_bytes * count)) return -2;
-    const void* dsrc = nullptr;
-    if (rows_on_device(m, data, tot, on_dev, &dsrc)) return -2;
-    return dk::tile(q, (const unsigned char*)dsrc, t.w, rc, cc, count, on_dev ? nullptr : m->up.st, on_dev);
+    return tile_rows(m, q, data, t.w, rc, cc, count, on_dev);
   }
   const size_t nrows_loc = (size_t)rc * count;
   const size_t local_disk = drb_loc * nrows_loc, local_dev = vrb * nrows_loc;

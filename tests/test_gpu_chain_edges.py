@@ -235,5 +235,33 @@ def test_large_vocabulary(vocab, chain):
     assert np.array_equal(logits[1], np.tile(logits[0], (1, -(-vocab // 1024)))[:, :vocab])
 
 
+@pytest.mark.parametrize("quant,sizes", [("q3_k", dict(moe_intermediate_size=5120, n_routed_experts=256, n_layers=2)),   # 288 MB a stack of experts
+                                         ("fp32", dict(dim=1036, n_heads=5, v_head_dim=64, vocab_size=66003, n_layers=2))])   # 274 MB of vocabulary, the last piece ragged
+def test_uploads_in_pieces(quant, sizes):
+    """Tensors from the host pass through a buffer of 256 MB: stacks of experts in whole matrices, one large matrix in whole row tiles.  Against one copy on the device."""
+    import dseek
+    import dsk
+    import mint
+    import torch
+    logits = []
+    with tempfile.TemporaryDirectory() as d:
+        mint.mint(d, PRESET[quant], quant, fast=True, seed=5, **sizes)
+        md, tensors = dseek.read_dir(d)
+        for host in (True, False):
+            m = dsk.Model(dsk.Config.from_metadata(md, 0))
+            assert m.launches_per_forward() > 1
+            for name, t in tensors.items():
+                if host or name == "tokenizer.tokens":
+                    m.upload(name, t.dtype, t.shape, t.data)
+                else:
+                    q = torch.from_numpy(np.array(t.data).reshape(-1).view(np.uint8)).cuda()
+                    torch.cuda.synchronize()
+                    m.upload_device(name, t.dtype, t.shape, q.data_ptr(), q.numel())
+            m.finalize()
+            logits.append(np.stack([np.array(m.forward(5 + 31 * pos, pos)[0]) for pos in range(3)] + [np.array(m.forward(m.cfg.vocab_size - 1, 3)[0])]))
+            m.close()
+    assert np.array_equal(*logits)
+
+
 if __name__ == "__main__":
     _run(sys.argv[1])
