@@ -1084,7 +1084,7 @@ __global__ void __maxnreg__(80) dk_gemv(const DkGemv* __restrict__ told, const _
 // ---- rope + attention of one head (src/infer.cpp:648-762, 956-1045): one CTA a head ------------------------------------------------------
 // The head's older keys and values come into shared memory ahead of the wait: they were written launches ago (a launch begins when the one ahead of it
 // is past its own wait, so only the one ahead may still run, and that writes row kv_pos).  What is left behind the wait is the new row, one pass over
-// shared memory for the scores and one for the values.  Contexts that do not fit (157 or 180 positions of 192 + 128 halves), those whose first rows
+// shared memory for the scores and one for the values.  Contexts that do not fit (156 or 180 positions of 192 + 128 halves), those whose first rows
 // turn in place (sinks) and those that the new row lies behind are read from global memory in the same passes.
 // Shared memory: query | scores of `hold` positions | their keys (later partial sums of the values) | their values; or query | partial sums | scores
 __host__ __device__ inline int dk_attn_parts(int vh) { return (vh <= 256 ? 256 / vh : 1) * vh; }

@@ -32,8 +32,12 @@ struct Plan {
 };
 
 static constexpr int kSmemLimit = 200 * 1024;
-// dynamic shared memory of the two forms (beside 7 KB each that are not): together within an SM, the second not twice; rings are as deep as that allows
-static constexpr int kSmemA = 100 * 1024, kSmemB = 109 * 1024, kSmemAttnB = 114 * 1024;
+// dynamic shared memory of the two forms: together within an SM's 228 KB, the second not twice; rings are as deep as that allows.  A dk_gemv has kSmemFixed beside it
+// (its static variables and the kilobyte that a CTA costs).  A launch whose inputs and shallowest rings take more than kSmemA comes to its SMs when the one ahead has gone.
+static constexpr int kSmemFixed = 9344 + 1024;
+static constexpr int kSmemB = 108 * 1024, kSmemA = 228 * 1024 - kSmemB - 2 * kSmemFixed, kSmemAttnB = 114 * 1024;
+static_assert(sizeof(DkGemv) + (kDkSegs + 1) * sizeof(DkRun) + 3 * 256 * 2 + 32 * 4 + sizeof(DkRouteSmem) + 8 + 1024 <= kSmemFixed, "dk_gemv's static variables");
+static_assert(2 * (kSmemB + kSmemFixed) > 228 * 1024 && 2 * (kSmemAttnB + 1024) > 228 * 1024 && kSmemA + kSmemAttnB + kSmemFixed + 2048 <= 228 * 1024, "two forms beside one another, the second not twice");
 
 static int slot_bytes(int q) { return q == DSK_Q2_K ? DkTraits<Q_Q2K>::slot : DkTraits<Q_F32>::slot; }
 
