@@ -1896,7 +1896,7 @@ static void enqueue_head(dsk_model* m, dsk_state* s, int first, int count, float
 
 // RMS norm in groups, stored.  A warp a group where the groups are more than the CTAs that the chip holds at a time (eight of 256 threads an SM).
 static void rms_groups(const float* in, int ld_in, const float* w, float* out, int ld_out, int T, int n, int groups, float eps, cudaStream_t st) {
-  if (n / groups <= 1024 && (long long)T * groups > 148 * 8)
+  if (n / groups <= 1024 && (long long)T * groups > 8ll * g_sm_count)
     launch_next(group_rmsnorm_rows, (unsigned)(((long long)T * groups + 7) / 8), 256, 0, st)(in, ld_in, w, out, ld_out, T, n, groups, eps);
   else launch_next(group_rmsnorm<float>, dim3((unsigned)T, (unsigned)groups), 256, 0, st)(in, ld_in, w, out, ld_out, n, groups, eps, 0, 0.f, nullptr, 0, nullptr, 0);
 }
