@@ -1,7 +1,7 @@
 // dsk_engine.cu — C-ABI (include/dsk.h) over the sm_100a kernels: device model, state, the per-token
 // launch sequence (one CUDA graph per token), expert-shard placement and the NCCL partial-sum all-reduce.
 //
-// Replaces, behind the reference's call surface (all /root/reference @ 8db9e56):
+// Replaces, behind the reference's call surface (files at commit 8db9e56):
 //   Model::forward -> _forward_cpu        src/model.cpp:874-883, src/infer.cpp:1265-1317   dsk_forward
 //   Block::block   -> _block_cpu          src/model.cpp:290-322, src/infer.cpp:810-932     dsk_block_forward
 //   BlockMHA::_attention_impl             src/infer.cpp:934-1049                           enqueue_layer (attention part)

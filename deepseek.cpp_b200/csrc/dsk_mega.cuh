@@ -2,7 +2,7 @@
 //
 // A token is a PROGRAM: an array of Stage descriptors in device memory (built once per dsk_state).  Stages are the
 // dependent phases of Model::_forward_cpu / Block::_block_cpu / BlockMHA::_attention_impl
-// (/root/reference/src/infer.cpp:810-1049, 1265-1317):
+// (src/infer.cpp:810-1049, 1265-1317):
 //     EMBED | per layer: S1 q(+q_a)+kv_a | [S1b wq_b] | S2 kv_b->KV cache | S3 rope+attention | S4 wo+residual |
 //     S5 gate logits | S56 routing + shared/routed w1,w3 with act(h1)*h3 | S7 w2 + weighted accumulate | LM head+argmax
 // It runs models on several GPUs, true-MLA blocks, shapes that the launches of dsk_decode.cuh refuse, and every test hook.

@@ -2,7 +2,7 @@
 
 Byte-compatible with the reference's format: a checkpoint is a DIRECTORY whose every entry is a
 safetensors-layout shard `u64 LE header_len | JSON header | raw tensor bytes`
-(reader: /root/reference/src/codec.cpp:262-377, writer: convert.py:582-588).  `__metadata__` (flat
+(reader: src/codec.cpp:262-377, writer: convert.py:582-588).  `__metadata__` (flat
 str->str map, convert.py:123-170) is taken from the first shard in sorted order; tensors are merged
 from all shards.  K-quant tensors are stored as U8 with shape (rows, cols/256*block_bytes)
 (quantizer.cpp:19); f8e5m2 weights carry an F32 `.scale` sibling of shape ceil(rows/128) x ceil(cols/128).

@@ -4,11 +4,11 @@
  * library.  The product (deepseek.cpp_b200/) never links or calls it.
  *
  * Parity pinning: every function here is checked against oracle/_ref/libdsref.so (the UNMODIFIED
- * reference compiled from /root/reference, see oracle/Makefile) by tests/test_oracle_vs_ref.py and
+ * reference compiled, see oracle/Makefile) by tests/test_oracle_vs_ref.py and
  * against the committed golden vectors in tests/golden/ (generated by tests/golden/make_golden.py
  * from that same library, plus the known answers of the reference's own src/test.cpp:128-186).
  *
- * All file:line citations are relative to /root/reference at commit 8db9e56.
+ * All file:line citations are relative to the reference at commit 8db9e56.
  */
 #ifndef DSK_ORACLE_H
 #define DSK_ORACLE_H

@@ -3,7 +3,7 @@
 TEST INFRASTRUCTURE.  No real DeepSeek weights exist in this environment (no network), so every
 checkpoint is synthetic: weights N(0,1)/sqrt(fan_in), embedding N(0,1), norm weights 1+0.1 N(0,1),
 gate N(0,1)/sqrt(dim)*gate_gain, V3 gate bias 0.01 N(0,1) quantised exactly the way
-/root/reference/convert.py does:
+convert.py does:
   * fp16: cast;  * f8e5m2: per 128x128 block scale=57344/amax, RNE cast, stored scale=1/scale
     (convert.py:216-275);  * q2_k/q3_k: the reference's own quantize_row_q{2,3}_K_ref through
     oracle/_ref/libdsref.so (quantizer.cpp:4-66) — or, with fast=True / no _ref, random *valid* blocks.

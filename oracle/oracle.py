@@ -60,7 +60,7 @@ def build_port(force: bool = False) -> str:
 
 
 def build_ref() -> Optional[str]:
-    """Builds oracle/_ref when /root/reference is present (build container); else keeps the prebuilt files."""
+    """Builds oracle/_ref where the reference's sources are present; else keeps the prebuilt files."""
     subprocess.check_call(["make", "-C", HERE, "ref"], stdout=subprocess.DEVNULL)
     so = os.path.join(HERE, "_ref", "libdsref.so")
     return so if os.path.exists(so) else None

@@ -1,14 +1,13 @@
 // oracle/ref_shim.cpp — TEST INFRASTRUCTURE ONLY (never linked into the product).
 //
-// A thin extern "C" harness around the UNMODIFIED reference sources under
-// /root/reference/src.  It textually includes the reference's infer.cpp so that its
+// A thin extern "C" harness around the UNMODIFIED reference sources (found by the Makefile).  It textually includes the reference's infer.cpp so that its
 // file-static kernels (matmul, moe_gate, rmsnorm, rope, ...) are reachable, and is
 // compiled with -fno-access-control so Model::_copy_embedding (private) can be driven.
 // Built by oracle/Makefile into oracle/_ref/libdsref.so (git-ignored).  No reference source is copied into this repository.
 //
 // Every wrapper names the reference symbol (file:line @ 8db9e56) it forwards to.
 
-#include "infer.cpp"  // /root/reference/src/infer.cpp (via -I)
+#include "infer.cpp"  // the reference's src/infer.cpp (via -I)
 
 #include <cstdlib>
 #include <cstring>

@@ -1,6 +1,6 @@
 """Generates tests/golden/*.npz|json from the UNMODIFIED reference (oracle/_ref/libdsref.so).
 
-Run in the build container (needs oracle/_ref, i.e. `make -C oracle ref` with /root/reference present):
+Run where the sources are (needs oracle/_ref, i.e. `make -C oracle ref` with the reference present):
     python tests/golden/make_golden.py
 The fixtures are committed; they pin the oracle port (CPU tests) and the CUDA kernels (GPU tests) on
 machines where the reference cannot be run.  Inputs are seeded; nothing here reads real model weights.
@@ -36,7 +36,7 @@ kat = {
     "testcpp_ref_f32": R.matmul(x16, w16, "fp32", 2, 16).tolist(),
     "testcpp_ref_f16": R.matmul(x16, w16_f16, "fp16", 2, 16).tolist(),
     "testcpp_ref_f8": R.matmul(x16, w16_f8, "f8e5m2", 2, 16).tolist(),
-    # SURVEY §8(c) known answers produced from the reference's static functions
+    # known answers produced from the reference's static functions
     "rmsnorm_in": [1, -2, 3, -4, 5, -6, 7, -8], "rmsnorm_w": [1, 1, 1, 1, 2, 2, 2, 2], "rmsnorm_eps": 1e-6,
     "rope_in": [1, 2, 3, 4, 5, 6, 7, 8], "rope_pos": 3, "rope_theta": 1e4,
     "gate_logits": [0.1, 2, -1, 2, 0.5, 1.5, -0.3, 0],

@@ -1,4 +1,4 @@
-"""GPU parity, tiers T2/T3 (SURVEY §8(c)): per-layer with re-synchronised inputs, and end-to-end teacher-forced,
+"""GPU parity, tiers T2/T3: per-layer with re-synchronised inputs, and end-to-end teacher-forced,
 through the reference-shaped call surface of the C-ABI (dsk_forward / dsk_block_forward / dsk_copy_embedding)."""
 import os
 
@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 PRESETS = ["tiny_v2lite", "tiny_v2", "tiny_v3"]
 # end-to-end tolerance on logits rel-L2: fp32 summation order for the dense quants; the K-quant bound is the
-# reference-vs-reference floor (SURVEY §0.4: a single Q8_K rounding flip moves the residual stream by ~1e-2)
+# reference-vs-reference floor (a single Q8_K rounding flip moves the residual stream by ~1e-2)
 E2E_TOL = {"fp32": 2e-4, "fp16": 2e-4, "f8e5m2": 5e-4, "q2_k": 8e-2, "q3_k": 8e-2}
 TOKENS = [0, 9, 400, 33, 1001, 77, 5, 640]
 

@@ -1,4 +1,4 @@
-"""Sharded decode on >= 2 GPUs of one node (SURVEY §8e): every rank loads the same checkpoint and keeps its slices —
+"""Sharded decode on >= 2 GPUs of one node: every rank loads the same checkpoint and keeps its slices —
 routed experts always; with peer memory (DSK_P2P=1, the default) and head dims that allow it also the attention heads, wo
 columns, shared-expert / dense-FFN hidden units and LM-head rows (tensor parallel).  Partial sums, logits and arg-max keys
 are exchanged inside the persistent kernel over CUDA-IPC-mapped peer memory; DSK_P2P=0 = expert-only sharding with
@@ -7,7 +7,7 @@ the reference (or its C restatement) on the full checkpoint; the "_tp" cases use
 two heads fill a 256-column K-quant block and assert that the tensor-parallel plan is actually active; the "_mla" case runs a
 true-MLA checkpoint (experts sharded, attention replicated).
 
-Skipped on a single-GPU box (the round-end driver); run it with `gpurun --gpus 2 -- python -m pytest tests/test_gpu_multigpu.py`.
+Skipped on a single GPU.
 """
 import os
 import subprocess
@@ -104,7 +104,7 @@ def test_sharded_decode_matches_reference(repo, ckpt, tmp_path, p2p, preset, qua
         assert res["dev"] == res["host"], res      # greedy tokens identical to the reference for the dense quants
     else:
         # K-quants: the sharded sum order differs from the CPU's expert loop, so a Q8_K rounding may flip downstream
-        # (SURVEY §0.4); the bound is the reference-vs-reference floor and the median must sit far below it
+        # (the reference does the same against itself); the bound is the reference-vs-reference floor and the median must sit far below it
         import numpy as np
         assert np.median(res["errs"]) < 2e-2, res
     assert res["launches"] == (1 if p2p == "1" else res["launches"])   # peer-memory mode: one kernel per token

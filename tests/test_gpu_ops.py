@@ -1,4 +1,4 @@
-"""GPU parity, tier T1 (SURVEY §8(c)): every kernel fed the oracle's exact inputs, through the C-ABI hooks.
+"""GPU parity, tier T1: every kernel fed the oracle's exact inputs, through the C-ABI hooks.
 Checker = the unmodified reference (oracle/_ref) when present, else the plain-C port; plus committed goldens.
 
 Every hook runs a one-stage program through the persistent decode kernel itself (decode_kernel<quant>: stage_q8 /
@@ -105,7 +105,7 @@ def test_gate_logits_stage(dsk, chk, mq, E, n):
     exp = chk.matmul(xn, gw, "fp32", E, n)
     got, got_xn = dsk.gate_logits(mq, gw, x, w, 1e-6)
     assert rel_l2(got_xn, xn) < 1e-6
-    assert rel_l2(got, exp) < 1e-5          # the reference's scalar F32 loop is re-associated by -ffast-math (DESIGN §2)
+    assert rel_l2(got, exp) < 1e-5          # the reference's scalar F32 loop is re-associated by -ffast-math
 
 
 @pytest.mark.parametrize("quant,d,n,tol", [

@@ -83,7 +83,7 @@ def test_real_dims_layers_and_logits(dsk, workload, quant, mla):
         print(f"real-dims {workload}/{quant} T2: median {np.median(errs):.2e} max {errs.max():.2e} spikes {spikes}/{errs.size}")
         if kq:
             # At these widths a layer quantises ~50 k activations to Q8_K: a 1-ulp difference in one of them flips a rounding
-            # in a sizeable fraction of (layer, token) pairs and moves the output by ~3e-3 (SURVEY §0.4 — the reference
+            # in a sizeable fraction of (layer, token) pairs and moves the output by ~3e-3 (the reference
             # does the same against itself).  The clean pairs prove the arithmetic (fp32 re-association only); the flipped
             # ones must stay at the single-flip magnitude.
             if errs.max() >= 5e-2 and O.ref_lib() is None:

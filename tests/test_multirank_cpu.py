@@ -1,5 +1,4 @@
-"""N>1 host logic on CPU (gloo, world_size 2): expert-shard placement and the per-layer partial-sum all-reduce
-(SURVEY §8(e)).  Each rank evaluates only its own experts of one MoE layer with the oracle port, rank 0 adds the
+"""N>1 host logic on CPU (gloo, world_size 2): expert-shard placement and the per-layer partial-sum all-reduce.  Each rank evaluates only its own experts of one MoE layer with the oracle port, rank 0 adds the
 shared expert, the partials are all-reduced and must equal the single-rank layer update."""
 import os
 import socket
@@ -93,7 +92,7 @@ def test_sharded_moe_partial_allreduce_equals_full(ckpt, tmp_path):
     assert np.allclose(got, full, rtol=1e-5, atol=1e-6)   # summation order differs across ranks (fp32 re-association)
 
 
-# ---- tensor-parallel shards (round 2): the rules of dsk_model_create and the identities the in-kernel exchanges rely on ----------
+# ---- tensor-parallel shards: the rules of dsk_model_create and the identities the in-kernel exchanges rely on ----------
 
 def tp_shard(cfg, rank, n_ranks):
     """Same arithmetic as dsk_model_create (csrc/dsk_engine.cu): block splits [r B / N, (r + 1) B / N)."""
