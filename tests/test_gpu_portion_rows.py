@@ -1,9 +1,14 @@
 """Kernels of long portions that share out rows: token tiles of the causal convolution with a remainder, norms of a warp a group, narrow products of ragged
-sizes, and the grouping of more (token, expert) pairs than its threads hold, over several scans of 32 experts."""
+sizes, the grouping of more (token, expert) pairs than its threads hold, over several scans of 32 experts, and norms of rows and groups on both sides of what a warp, a
+thread's eight values and a CTA's registers hold."""
 import numpy as np
 import pytest
 
-from test_gpu_hybrid import F32_TOL, ho, mk, rel, tokens_for  # noqa: F401
+import test_gpu_netusun as netusun
+from test_gpu_hybrid import F32_TOL, att_layer, ho, mk, model_cfg, rel, ssd_layer, tokens_for  # noqa: F401
+from test_gpu_netusun import no  # noqa: F401
+
+mk_netusun = netusun.mk
 
 pytestmark = pytest.mark.gpu
 
@@ -19,3 +24,24 @@ def test_long_portion(mk, ho, tokens, top, seed):  # noqa: F811
     got, got_layers = m.forward_chunk(toks, 0, range(tokens), layers=True)
     assert rel(got_layers, exp_layers) < F32_TOL
     assert rel(got, exp) < F32_TOL
+
+
+# groups of 1000 and 1024 values, more than the CTAs that the device holds: a warp each; of 1026 and 2048: a CTA each, in registers; of 2050: read twice
+@pytest.mark.parametrize("width,groups,tokens", [(3000, 3, 500), (2048, 2, 700), (2052, 2, 620), (4096, 2, 5), (4100, 2, 5)])
+def test_norm_groups(mk, ho, width, groups, tokens):  # noqa: F811
+    cfg = model_cfg([ssd_layer(heads=2, vdim=6, state=4, groups=1, conv=2, ng=2), att_layer(heads=1, dim=4, vdim=3, rank=5, win=9)], width=width, groups=groups)
+    m, W = mk(cfg, seed=7, chunk=tokens)
+    toks = tokens_for(cfg, tokens, 4)
+    exp, exp_layers = ho.run(cfg, W, toks)
+    got, got_layers = m.forward_chunk(toks, 0, range(tokens), layers=True)
+    assert rel(got_layers, exp_layers) < F32_TOL
+    assert rel(got, exp) < F32_TOL
+
+
+@pytest.mark.parametrize("width", [2048, 2056, 4096, 4100])   # eight values a thread up to 2048, sixteen up to 4096, norms by themselves behind that
+def test_norms_of_closing_blocks(mk_netusun, no, width):  # noqa: F811
+    cfg = no.model_config([no.att(heads=2, dim=8, vdim=6, mlp=no.moe(6, 3, 8, 2, 1, 1.0, 11)), no.mem(heads=2, dim=4, vdim=5, mlp=no.dense(12))], width=width, vocab=61)
+    m, W = mk_netusun(cfg, seed=3, chunk=24)
+    toks = tokens_for(cfg, 21, 5)
+    exp = no.run(cfg, W, toks)
+    assert rel(m.forward_chunk(toks, 0, range(21)), exp[0] if isinstance(exp, tuple) else exp) < F32_TOL
