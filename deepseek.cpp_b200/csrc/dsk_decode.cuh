@@ -636,8 +636,8 @@ __device__ __forceinline__ void dk_issue(const uint8_t* p, uint32_t place, bool 
 
 // What unit u adds to the sums of a piece; acc: K-quant: quarter t of rows g, g + 8; f8: rows g, g + 8, high and low halves; else one a row.
 // K-quants: the instructions' columns 2t and 2t + 1 are quarter t's sub-blocks s = 0, 1 in one set of sums and s = 2, 3 in another.  About 105 instructions for the 1344 bytes
-// of a Q2_K unit (13 bytes each; a lane a quarter block with dp4a, as in the interpreter, 5.3), 8 of them mma at 8 cycles of a sub-partition; at 6.5 TB/s that is
-// half the issue slots.
+// of a Q2_K unit (13 bytes each; a lane a quarter block with dp4a, as in the interpreter, 5.3), 8 of them mma at 8 cycles of a sub-partition.  In a launch
+// they are a third of what a warp issues (ncu, V2's routed w1 and w3: 3740 instructions for 12 units, 34 % of the issue slots; staging and routing have the rest).
 template <int Q>
 __device__ __forceinline__ void dk_unit(float (&acc)[4], uint32_t src, uint32_t xa, uint32_t xb, uint32_t xc, int u, float f0, float f1) {
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
