@@ -385,7 +385,7 @@ static int build(const dsk_model* m, const dsk_state* s, Shapes& shapes, Plan* o
     for (int j = 0; j < D.g.nsegs; j++) { key.push_back(D.g.seg[j].rows); key.push_back(D.g.seg[j].nb); key.push_back((D.g.seg[j].f32 << 1) | D.g.seg[j].pair); }
     auto it = shapes.of.find(key);
     if (it != shapes.of.end()) return &it->second;
-    if (out) { fail(-4, "dsk_state_create: tensors of the model are missing"); return nullptr; }
+    if (out) { fail(-4, "token chain: a launch without a plan"); return nullptr; }
     Arranged& A = shapes.of[key];
     return arrange(D, q, G, form, &A) ? &A : nullptr;
   };

@@ -755,10 +755,8 @@ extern "C" int dsk_upload_tensor(dsk_model* m, const char* name, int dtype, cons
   return fail(-4, "unknown tensor name %s (MLA-mode tensors are not part of this path)", name);
 }
 
-extern "C" int dsk_model_finalize(dsk_model* m) {
-  if (need_device()) return -1;
-  if (!m) return fail(-1, "null model");
-  if (m->hy) return hyb::finalize(m);
+// Whether all tensors of a model have come (kernels read what is missing at address 0)
+static int check_complete(const dsk_model* m) {
   const dsk_config& c = m->c;
   const bool f8 = c.quant == DSK_F8E5M2;
   auto need = [&](const DTensor& t, const char* what, int l) -> int {
@@ -768,9 +766,9 @@ extern "C" int dsk_model_finalize(dsk_model* m) {
   };
   if (need(m->embed, "model.embed", -1)) return -5;
   if (!m->rms_final) return fail(-5, "missing model.norm.weight");
-  if (!m->has_wcls) m->wcls = m->embed;  // tied embeddings (src/model.cpp:852-855)
+  if (m->has_wcls && need(m->wcls, "model.output", -1)) return -5;
   for (int l = 0; l < c.n_layers; l++) {
-    Layer& L = m->layers[l];
+    const Layer& L = m->layers[l];
     if (!L.rms_att || !L.rms_ffn || !L.rms_kv_a) return fail(-5, "missing norm weights (layer %d)", l);
     if (c.use_mla) {
       if (!L.rms_q_a) return fail(-5, "missing q_a_norm (layer %d)", l);
@@ -788,6 +786,15 @@ extern "C" int dsk_model_finalize(dsk_model* m) {
         return -5;
     }
   }
+  return 0;
+}
+
+extern "C" int dsk_model_finalize(dsk_model* m) {
+  if (need_device()) return -1;
+  if (!m) return fail(-1, "null model");
+  if (m->hy) return hyb::finalize(m);
+  if (check_complete(m)) return -5;
+  if (!m->has_wcls) m->wcls = m->embed;  // tied embeddings (src/model.cpp:852-855)
   // join the upload pipeline and give its pinned staging buffers back
   if (m->up.st) {
     cudaError_t e = cudaStreamSynchronize(m->up.st);
@@ -894,6 +901,8 @@ extern "C" dsk_state* dsk_state_create(dsk_model* m) {
   if (need_device() || !m) return nullptr;
   if (m->hy) return hyb::state_create(m);
   const dsk_config& c = m->c;
+  if (check_complete(m)) return nullptr;
+  if (!m->wcls.present) { fail(-5, "dsk_state_create: the model is not finished (tied embeddings)"); return nullptr; }
   dsk_state* s = new dsk_state();
   s->m = m;
   auto fa = [&](float** p, size_t n) { cudaMalloc((void**)p, std::max<size_t>(n, 4) * 4); cudaMemset(*p, 0, std::max<size_t>(n, 4) * 4); };

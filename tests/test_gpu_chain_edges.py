@@ -205,6 +205,30 @@ def test_state_before_finalize(quant):
     assert np.array_equal(*logits)
 
 
+@pytest.mark.parametrize("missing", ["model.output.scale", "model.output.weight", "model.embed.scale", "model.layers.1.moegate.weight", "model.layers.1.mlp.w2.scale",
+                                     "model.layers.0.attn.norm.weight", "model.layers.2.shared_mlp.w1.weight"])
+def test_state_of_an_incomplete_model_is_refused(missing):
+    import dseek
+    import dsk
+    import mint
+    with tempfile.TemporaryDirectory() as d:
+        mint.mint(d, "tiny_v2", "f8e5m2", fast=True, seed=5)
+        md, tensors = dseek.read_dir(d)
+    m = dsk.Model(dsk.Config.from_metadata(md, 0))
+    for name, t in tensors.items():
+        if name != missing and not (missing == "model.output.weight" and name == "model.output.scale"):
+            m.upload(name, t.dtype, t.shape, t.data)
+    with pytest.raises(dsk.DskError):
+        m.new_state()
+    if missing == "model.output.weight":   # (tied embeddings: once the model is finished)
+        m.finalize()
+        assert np.isfinite(m.forward(3, 0)[0]).all()
+    else:
+        with pytest.raises(dsk.DskError):
+            m.finalize()
+    m.close()
+
+
 @pytest.mark.parametrize("vocab,chain", [(1000003, True), (2000003, False)])
 def test_large_vocabulary(vocab, chain):
     """The sums of an LM head's rows (64 floats a tile of 16 rows) fit a CTA's shared memory up to about 1.5 million rows; the interpreter runs what does not."""
