@@ -10,7 +10,7 @@
 //   gemm_tc5          C = A W^T for T > 4 rows and bf16 weights that TMA can address, on the 5th-generation tensor cores (dsk_tc5.cuh), with fused
 //                     epilogues (residual add, clamped GLU, GELU x per-token embedding) and row gather / scatter / expert tiles
 //   gemm_mma          the same for the other bf16 weights on mma.sync (activations rounded to bf16 as they are staged)
-//   gemm_split        the same for fp32 weights, operands as three bf16 parts (dsk_pattn.cuh)
+//   gemm_split        the same for fp32 weights, operands as three bf16 parts (dsk_split.cuh)
 //   gemm_narrow       up to 96 columns over 448 rows and more
 //   gemv_rows         the same interface for T <= 4 rows: one warp per weight row, 16-byte loads
 //   gemv_one          the same for one row (a decoded token): eight 16-byte weight loads in flight per lane

@@ -412,7 +412,7 @@ static void set_kernel_attrs() {
   cudaFuncSetAttribute(pattn<A, B, 4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax); cudaFuncSetAttribute(pattn<A, B, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax)
   DSK_PATTN_ATTR(1, 8); DSK_PATTN_ATTR(1, 16); DSK_PATTN_ATTR(3, 8); DSK_PATTN_ATTR(3, 16);
 #undef DSK_PATTN_ATTR
-#define DSK_SPLIT_ATTR(E) cudaFuncSetAttribute(gemm_split<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSmem)
+#define DSK_SPLIT_ATTR(E) cudaFuncSetAttribute(gemm_split<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, split_smem(kSplitStages))
   DSK_SPLIT_ATTR(HEPI_STORE); DSK_SPLIT_ATTR(HEPI_ADD); DSK_SPLIT_ATTR(HEPI_GLU); DSK_SPLIT_ATTR(HEPI_XIELU); DSK_SPLIT_ATTR(HEPI_GEGLU); DSK_SPLIT_ATTR(HEPI_SIGMUL);
   DSK_SPLIT_ATTR(HEPI_RELU2); DSK_SPLIT_ATTR(HEPI_LINGATE); DSK_SPLIT_ATTR(HEPI_SILU_SIG); DSK_SPLIT_ATTR(HEPI_SOFTCAP); DSK_SPLIT_ATTR(HEPI_SWIGLU); DSK_SPLIT_ATTR(HEPI_GELU_MUL);
 #undef DSK_SPLIT_ATTR
@@ -1603,10 +1603,12 @@ static void launch_gemv(int epi, const GemmP& P, int Z, cudaStream_t st) {
   }
 }
 // fp32 products of more than four rows, routed ones in tiles of 128 (gemm_split)
-static void launch_split(int epi, const GemmP& P, int Z, int tile_cap, cudaStream_t st) {
-  const int bn = epi_dual(epi) ? 32 : 64;
-  const dim3 grid((unsigned)((P.N + bn - 1) / bn), (unsigned)(P.tiles ? tile_cap : (P.M + 127) / 128), (unsigned)Z);
-#define DSK_SPLIT(E) case E: launch_next(gemm_split<E>, grid, 256, kSplitSmem, st)(P); break
+static void launch_split(State* S, int epi, const GemmP& P, int Z, int tile_cap, cudaStream_t st) {
+  const int bn = epi_dual(epi) ? kSplitN / 2 : kSplitN;
+  const dim3 grid((unsigned)((P.N + bn - 1) / bn), (unsigned)(P.tiles ? tile_cap : (P.M + kTcRows - 1) / kTcRows), (unsigned)Z);
+  // (a short depth takes no more of an SM than it has slices: short steps' next kernels start beside it)
+  const int stages = std::max(1, std::min(kSplitStages, (P.K + kSplitDepth - 1) / kSplitDepth));
+#define DSK_SPLIT(E) case E: launch_next(gemm_split<E>, grid, kSplitThreads, split_smem(stages), st)(P, stages, S->h_err); break
   switch (epi) {
     DSK_SPLIT(HEPI_STORE); DSK_SPLIT(HEPI_ADD); DSK_SPLIT(HEPI_GLU); DSK_SPLIT(HEPI_XIELU); DSK_SPLIT(HEPI_GEGLU); DSK_SPLIT(HEPI_SIGMUL);
     DSK_SPLIT(HEPI_RELU2); DSK_SPLIT(HEPI_LINGATE); DSK_SPLIT(HEPI_SILU_SIG); DSK_SPLIT(HEPI_SOFTCAP); DSK_SPLIT(HEPI_SWIGLU); DSK_SPLIT(HEPI_GELU_MUL);
@@ -1644,7 +1646,7 @@ static void linear(State* S, bool bf16, int epi, const GemmP& P, int Z, cudaStre
   }
   if (tc_ok(S, bf16, epi, P, Z)) launch_tc5(S, epi, P, tile_cap, st);
   else if (bf16 && !small) launch_gemm_mma(epi, P, Z, tile_cap, st);
-  else if (!small) launch_split(epi, P, Z, tile_cap, st);
+  else if (!small) launch_split(S, epi, P, Z, tile_cap, st);
   else if (bf16) launch_gemv<__nv_bfloat16>(epi, P, Z, st);
   else launch_gemv<float>(epi, P, Z, st);
   S->launches++;

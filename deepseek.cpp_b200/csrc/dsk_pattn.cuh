@@ -412,184 +412,5 @@ __global__ void __launch_bounds__(256, 1) pattn(const __grid_constant__ PattnP P
   }
 }
 
-// ---------------------------------------------------------------------------------------------------------------------
-// fp32 products of many rows (fp32 models; the score and value products of attention with mixed heads) on the tensor cores: both operands split
-// into three bf16 parts on their way into shared memory, six products per element as in pattn.  128 x 64 tile, 32 deep; 8 warps as 4 (rows) x 2
-// (columns), a 32 x 32 warp tile; the next slice's fp32 values are in registers during this one's products.  Interface, row maps, expert tiles,
-// batches and epilogues of GemmP.  Bound: the six mma.sync per element.  FMA on 64 x 64 tiles, before, was bound by the fp32 pipe: a step in fp32 at
-// width 1024 went from 1.85 to 1.22 ms (600 tokens), from 0.95 to 0.67 (64 tokens) and from 0.89 to 0.64 (5 tokens), a 1500-token prompt with mixed
-// heads from 2.98 to 2.67 ms, fp32 routed products of two layers with 16 experts of which 2 from 1.17 to 1.10 (33 tokens, 4 rows an expert) and from 1.40 to 1.28
-// (340, 42 rows).  Error of the first against 64 bits, attention in three parts included: 1.0e-6 before, 3.1e-7.
-// ---------------------------------------------------------------------------------------------------------------------
-// The same sum as a chain of FMAs over the numbers themselves, for a result that is not finite: an infinite operand has no three parts (what is left
-// of it is inf - inf), nor has a finite one that rounds to an infinity in bf16 (from 2^128 - 2^119).  Such operands make every result that they enter
-// NaN, so that looking at the results is enough.  weights: A holds softmax weights, 0 for keys out of sight, which do not enter.
-__device__ __noinline__ float plain_dot(const float* a, const float* w, int k_lo, int k_hi, bool weights) {
-  float s = 0.f;
-  for (int k = k_lo; k < k_hi && !isnan(s); k++)
-    if (!weights || a[k] != 0.f) s = fmaf(a[k], w[k], s);
-  return s;
-}
-constexpr int kSplitPitch = 40;                                      // bf16 per staged row: 32 + 8
-constexpr int kSplitStage = 3 * (128 + 64) * kSplitPitch;            // bf16 of one stage: A parts, then W parts
-constexpr int kSplitSmem = 2 * kSplitStage * 2;
-template <int EPI>
-__global__ void __launch_bounds__(256, 2) gemm_split(const GemmP P) {
-  constexpr int BM = 128, BT = 64, BK = 32, PITCH = kSplitPitch;
-  constexpr bool DUAL = epi_dual(EPI);
-  constexpr int BN = DUAL ? 32 : 64;
-  extern __shared__ __align__(16) unsigned char gs_raw[];
-  __shared__ int rowsA[BM], rowsC[BM];
-  grid_enter();
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  long long aoff = (long long)blockIdx.z * P.sA, woff = (long long)((int)blockIdx.z / P.z_wdiv) * P.sW, coff = (long long)blockIdx.z * P.sC;
-  int row0, nrows;
-  if (P.tiles) {
-    if ((int)blockIdx.y >= *P.n_tiles) return;
-    const int4 t = P.tiles[blockIdx.y];
-    woff = (long long)t.x * P.sW;
-    row0 = t.y;
-    nrows = t.z;
-  } else {
-    row0 = blockIdx.y * BM;
-    nrows = min(BM, P.M - row0);
-  }
-  if (tid < BM) {
-    const int i = row0 + tid;
-    const bool ok = tid < nrows;
-    rowsA[tid] = ok ? (P.a_map ? P.a_map[i] / P.a_div : i) : -1;
-    rowsC[tid] = ok ? (P.c_map ? P.c_map[i] : i) : -1;
-  }
-  __syncthreads();
-  const int n0 = blockIdx.x * BN;
-  int k_lo = 0, k_hi = P.K;
-  if (P.band) {
-    const int i0 = P.band_pos + row0, lo = max(0, mask_first(P.band_mask, P.band_window, i0) - P.band_first), hi = i0 + nrows - P.band_first;
-    if (P.band == BAND_DEPTH) { k_lo = P.band_keep ? 0 : lo / BK * BK; k_hi = min(P.K, hi); }
-    else if (n0 >= hi || (n0 + BN <= lo && n0 >= P.band_keep)) return;
-  }
-  const float* __restrict__ A = P.A + aoff;
-  // staging: thread -> 16 consecutive k of an activation row, 8 of a weight row
-  const int lr = tid >> 1, lk = (tid & 1) * 16, ar = rowsA[lr];
-  const int wl = tid >> 2, wk = (tid & 3) * 8;
-  int wrow;
-  const float* wsrc = reinterpret_cast<const float*>(P.W) + woff;
-  if (DUAL) { const int g = wl >> 3; wrow = n0 + (g >> 1) * 8 + (wl & 7); if (g & 1) wsrc = reinterpret_cast<const float*>(P.W2) + woff; }
-  else wrow = n0 + wl;
-  const bool wok = wrow < P.N;
-  const float* arow = A + (size_t)(ar < 0 ? 0 : ar) * P.lda;
-  const float* wr = wsrc + (size_t)(wok ? wrow : 0) * P.ldw;
-  const bool va = (reinterpret_cast<uintptr_t>(arow) & 15) == 0, vw = (reinterpret_cast<uintptr_t>(wr) & 15) == 0;
-  float xa[16], xw[8];
-  auto fetch = [&](int k0) {
-    if (ar >= 0 && va && k0 + lk + 16 <= P.K) {
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const float4 v = reinterpret_cast<const float4*>(arow + k0 + lk)[q];
-        xa[4 * q] = v.x; xa[4 * q + 1] = v.y; xa[4 * q + 2] = v.z; xa[4 * q + 3] = v.w;
-      }
-    } else {
-#pragma unroll
-      for (int q = 0; q < 16; q++) xa[q] = ar >= 0 && k0 + lk + q < P.K ? arow[k0 + lk + q] : 0.f;
-    }
-    if (wok && vw && k0 + wk + 8 <= P.K) {
-#pragma unroll
-      for (int q = 0; q < 2; q++) {
-        const float4 v = reinterpret_cast<const float4*>(wr + k0 + wk)[q];
-        xw[4 * q] = v.x; xw[4 * q + 1] = v.y; xw[4 * q + 2] = v.z; xw[4 * q + 3] = v.w;
-      }
-    } else {
-#pragma unroll
-      for (int q = 0; q < 8; q++) xw[q] = wok && k0 + wk + q < P.K ? wr[k0 + wk + q] : 0.f;
-    }
-  };
-  const uint32_t sm0 = smem_u32(gs_raw);
-  auto put = [&](int buf) {
-    unsigned char* base = gs_raw + (size_t)buf * kSplitStage * 2;
-    uint32_t pa[3][8], pw[3][4];
-#pragma unroll
-    for (int q = 0; q < 8; q++) { uint32_t x[3]; split_pair<3>(xa[2 * q], xa[2 * q + 1], x); pa[0][q] = x[0]; pa[1][q] = x[1]; pa[2][q] = x[2]; }
-#pragma unroll
-    for (int q = 0; q < 4; q++) { uint32_t x[3]; split_pair<3>(xw[2 * q], xw[2 * q + 1], x); pw[0][q] = x[0]; pw[1][q] = x[1]; pw[2][q] = x[2]; }
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-      uint4* da = reinterpret_cast<uint4*>(base + ((size_t)i * BM * PITCH + lr * PITCH + lk) * 2);
-      da[0] = make_uint4(pa[i][0], pa[i][1], pa[i][2], pa[i][3]); da[1] = make_uint4(pa[i][4], pa[i][5], pa[i][6], pa[i][7]);
-      *reinterpret_cast<uint4*>(base + ((size_t)3 * BM * PITCH + (size_t)i * BT * PITCH + wl * PITCH + wk) * 2) = make_uint4(pw[i][0], pw[i][1], pw[i][2], pw[i][3]);
-    }
-  };
-  const int wm = warp & 3, wn = warp >> 2;
-  float acc[2][4][4];
-#pragma unroll
-  for (int i = 0; i < 2; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++)
-#pragma unroll
-      for (int q = 0; q < 4; q++) acc[i][j][q] = 0.f;
-  const int nk = (k_hi - k_lo + BK - 1) / BK;
-  fetch(k_lo);
-  put(0);
-  __syncthreads();
-  for (int kt = 0; kt < nk; kt++) {
-    if (kt + 1 < nk) fetch(k_lo + (kt + 1) * BK);
-    const uint32_t sa = sm0 + (uint32_t)((kt & 1) * kSplitStage) * 2, sw = sa + 3 * BM * PITCH * 2;
-    const uint32_t aaddr = sa + (uint32_t)((wm * 32 + (lane & 7) + ((lane >> 3) & 1) * 8) * PITCH + (lane >> 4) * 8) * 2;
-    const uint32_t waddr = sw + (uint32_t)((wn * 32 + (lane & 7) + (lane >> 4) * 8) * PITCH + ((lane >> 3) & 1) * 8) * 2;
-#pragma unroll
-    for (int k = 0; k < BK; k += 16)
-#pragma unroll
-      for (int mi = 0; mi < 2; mi++) {
-        uint32_t a[3][4];
-#pragma unroll
-        for (int i = 0; i < 3; i++) ldmatrix_x4_at(a[i], aaddr + (uint32_t)(i * BM * PITCH + mi * 16 * PITCH + k) * 2);
-        mma_parts<3, 4>(acc[mi], a, [&](int part, uint32_t (&bb)[4][2]) {
-#pragma unroll
-          for (int np = 0; np < 2; np++) {
-            uint32_t r[4];
-            ldmatrix_x4_at(r, waddr + (uint32_t)(part * BT * PITCH + np * 16 * PITCH + k) * 2);
-            bb[2 * np][0] = r[0]; bb[2 * np][1] = r[1]; bb[2 * np + 1][0] = r[2]; bb[2 * np + 1][1] = r[3];
-          }
-        });
-      }
-    if (kt + 1 < nk) put((kt + 1) & 1);   // the other buffer: everyone was through it at the last barrier
-    __syncthreads();
-  }
-  float any = 0.f;   // (stays 0 as long as every sum is finite)
-#pragma unroll
-  for (int mi = 0; mi < 2; mi++)
-#pragma unroll
-    for (int ni = 0; ni < 4; ni++)
-#pragma unroll
-      for (int q = 0; q < 4; q++) any = fmaf(0.f, acc[mi][ni][q], any);
-  if (any != 0.f) {   // all of this lane's results as plain sums (in code of its own: calls beside the sums above cost a step 2 %)
-#pragma unroll 1
-    for (int e = 0; e < (DUAL ? 16 : 32); e++) {   // e: row (mi, half) x granule x column
-      const int r = wm * 32 + (e & 1) * 8 + ((e >> 1) & 1) * 16 + (lane >> 2), g = wn * (DUAL ? 2 : 4) + (e >> 3), n = n0 + g * 8 + (lane & 3) * 2 + ((e >> 2) & 1), cr = rowsC[r];
-      if (cr < 0 || n >= P.N) continue;
-      const float* a = A + (size_t)rowsA[r] * P.lda;
-      const float v = plain_dot(a, reinterpret_cast<const float*>(P.W) + woff + (size_t)n * P.ldw, k_lo, k_hi, P.band == BAND_DEPTH);
-      const float v2 = DUAL ? plain_dot(a, reinterpret_cast<const float*>(P.W2) + woff + (size_t)n * P.ldw, k_lo, k_hi, false) : 0.f;
-      gemm_epilogue<float, EPI>(P, P.C + coff + (size_t)cr * P.ldc, cr, n, v, v2);
-    }
-    return;
-  }
-#pragma unroll
-  for (int mi = 0; mi < 2; mi++)
-#pragma unroll
-    for (int half = 0; half < 2; half++) {
-      const int cr = rowsC[wm * 32 + mi * 16 + (lane >> 2) + half * 8];
-      if (cr < 0) continue;
-      float* crow = P.C + coff + (size_t)cr * P.ldc;
-#pragma unroll
-      for (int ni = 0; ni < 4; ni += (DUAL ? 2 : 1))
-#pragma unroll
-        for (int q = 0; q < 2; q++) {
-          const int g = wn * 4 + ni;   // granule of 8 staged rows
-          const int n = DUAL ? n0 + (g >> 1) * 8 + (lane & 3) * 2 + q : n0 + g * 8 + (lane & 3) * 2 + q;
-          if (n < P.N) gemm_epilogue<float, EPI>(P, crow, cr, n, acc[mi][ni][half * 2 + q], DUAL ? acc[mi][ni + 1][half * 2 + q] : 0.f);
-        }
-    }
-}
-
 }  // namespace hy
 }  // namespace dsk
