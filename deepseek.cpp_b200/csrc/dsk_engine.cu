@@ -312,6 +312,13 @@ static int need_device() {
   if (g_device < 0) return fail(-1, "dsk_init() has not bound a CUDA device — libdsk has no CPU fallback");
   return 0;
 }
+extern "C" void* dsk_host_alloc(size_t bytes) {
+  void* p = nullptr;
+  if (need_device()) return nullptr;
+  if (!bytes || cudaMallocHost(&p, bytes) != cudaSuccess) { cudaGetLastError(); fail(-2, "dsk_host_alloc: %zu bytes of pinned memory are not to be had", bytes); return nullptr; }
+  return p;
+}
+extern "C" void dsk_host_free(void* p) { if (p) cudaFreeHost(p); }
 extern "C" int dsk_sync(void) {
   if (need_device()) return -1;
   CK(cudaDeviceSynchronize());
@@ -873,13 +880,13 @@ static int alloc_host_side(dsk_state* s, size_t more = 0) {
 }
 // device -> pageable host memory through two pinned pieces, one landing while the other is copied on (the driver's own staging of such a
 // copy takes them one after the other: 410 KB of logits behind a token cost 12 us more, 2.4 MB behind a portion 150 us).  Returns when the bytes are there; destinations
-// that the driver knows (pinned, managed) are written directly.
-static int copy_to_host(dsk_state* s, void* dst, const void* src, size_t bytes) {
+// that the driver knows (pinned, managed) are written directly, and the call need not wait where more follows on the stream (last).
+static int copy_to_host(dsk_state* s, void* dst, const void* src, size_t bytes, bool last = true) {
   cudaPointerAttributes at{};
   const bool pageable = cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
   if (!pageable || bytes <= ((size_t)16 << 10)) {   // (a device address is the copy's to refuse)
     CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s->stream));
-    CK(cudaStreamSynchronize(s->stream));
+    if (last) CK(cudaStreamSynchronize(s->stream));
     return 0;
   }
   const size_t n = (bytes + kBouncePiece - 1) / kBouncePiece;

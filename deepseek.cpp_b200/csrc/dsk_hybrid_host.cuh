@@ -157,7 +157,10 @@ struct State {
   float* vfirst = nullptr;                   // [chunk][kv_heads * vdim] values of the step's tokens in the first value-mixing layer
   int* d_prev = nullptr;                     // the sequence's last token (bigram embedding)
   float *x = nullptr, *h = nullptr, *b0 = nullptr, *b1 = nullptr, *b2 = nullptr, *b3 = nullptr, *wgt = nullptr, *logits = nullptr;
-  int *h_tok = nullptr, *h_want = nullptr;   // pinned staging of a chunk's token ids / wanted rows (behind dsk_state::h_ctrl, with h_err)
+  // pinned staging of a chunk's first position, token ids and wanted rows (behind dsk_state::h_ctrl, with h_err), two of them: [4] [chunk] [chunk], on the
+  // device d_ctl, d_tok and d_want
+  int* h_in[2] = {nullptr, nullptr};
+  cudaEvent_t in_ev[2] = {nullptr, nullptr};   // its copy is through
   // attention of portions in one kernel (pattn): split keys and values of the visible positions, queries it takes at a time
   __nv_bfloat16 *k16 = nullptr, *v16 = nullptr;
   float* ppart = nullptr;                    // partial softmax results of shares of the keys: up to 148 CTAs of 128 rows (launches that fill the chip are not split)
@@ -167,10 +170,12 @@ struct State {
   __nv_bfloat16 *a16 = nullptr, *hid16 = nullptr;
   size_t a16_elems = 0, hid16_elems = 0;
   int* h_err = nullptr;
-  // device memory of the state: one allocation, cut into the pieces that salloc was asked for (portion: one that only the attention of portions needs)
-  struct Piece { void** at; size_t bytes; bool portion; };
+  // device memory of the state: one allocation, cut into the pieces that salloc was asked for (portion: one that only the attention of portions needs; seq: caches and carried
+  // states of the sequence)
+  struct Piece { void** at; size_t bytes; bool portion, seq; };
   std::vector<Piece> pieces;
-  char* arena = nullptr;
+  char *arena = nullptr, *seq = nullptr;     // seq: what a new sequence finds zeroed (Piece::seq), in one run
+  size_t seq_bytes = 0;
   // side-by-side mixers run on two streams, forked and joined by events
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -1145,9 +1150,9 @@ static int launches_per_token(const dsk_model* m) {
 // Asks for a piece of the state's memory; *p is set by salloc_all.  A piece of 1 MB and more takes whole pages of 2 MB, as an allocation of its own does: with all pieces
 // packed at 512 bytes, decoded tokens of two designs took 0.6 and 1.7 % longer (where caches, states and rows lie, not what is done with them).
 constexpr size_t kStatePage = (size_t)2 << 20;
-static int salloc(State* S, void** p, size_t bytes, bool portion = false) {
+static int salloc(State* S, void** p, size_t bytes, bool portion = false, bool seq = false) {
   const size_t unit = bytes >= kStatePage / 2 ? kStatePage : 512;
-  S->pieces.push_back({p, (std::max<size_t>(bytes, 16) + unit - 1) / unit * unit, portion});
+  S->pieces.push_back({p, (std::max<size_t>(bytes, 16) + unit - 1) / unit * unit, portion, seq});
   return 0;
 }
 // All pieces in one allocation (an allocation and a zeroing for each of 30 to 50 pieces were most of the time that a state took to make and to free), zeroed.
@@ -1160,23 +1165,21 @@ static int salloc_all(State* S, cudaStream_t st) {
     CK(cudaMalloc((void**)&S->arena, total()));
   }
   CK(cudaMemsetAsync(S->arena, 0, total(), st));
-  std::stable_partition(S->pieces.begin(), S->pieces.end(), [](const State::Piece& q) { return q.bytes % kStatePage == 0; });   // pages first
+  // pages first; what a new sequence finds zeroed stands together, on the pages and behind them (a memset for every piece kept a short prompt waiting for 2 to 4 us each)
+  auto place = [](const State::Piece& q) { return q.bytes % kStatePage == 0 ? (q.seq ? 1 : 0) : q.seq ? 2 : 3; };
+  std::stable_sort(S->pieces.begin(), S->pieces.end(), [&](const State::Piece& a, const State::Piece& b) { return place(a) < place(b); });
   char* at = S->arena;
-  for (const State::Piece& q : S->pieces) { *q.at = q.bytes ? at : nullptr; at += q.bytes; }
+  for (const State::Piece& q : S->pieces) {
+    *q.at = q.bytes ? at : nullptr;
+    if (q.seq) { if (!S->seq) S->seq = at; S->seq_bytes = at + q.bytes - S->seq; }
+    at += q.bytes;
+  }
   return cudaStreamSynchronize(st) == cudaSuccess ? 0 : -2;
 }
 
 static int state_reset(dsk_state* s) {
   State* S = s->hy;
-  for (LayerState& l : S->L) {
-    if (l.ssm) CK(cudaMemsetAsync(l.ssm, 0, l.ssm_bytes, s->stream));
-    if (l.hist) CK(cudaMemsetAsync(l.hist, 0, l.hist_bytes, s->stream));
-    if (l.cache) CK(cudaMemsetAsync(l.cache, 0, l.cache_bytes, s->stream));
-    if (l.vcache) CK(cudaMemsetAsync(l.vcache, 0, l.vcache_bytes, s->stream));
-    if (l.canon) CK(cudaMemsetAsync(l.canon, 0, l.canon_bytes, s->stream));
-    if (l.shift) CK(cudaMemsetAsync(l.shift, 0, l.shift_bytes, s->stream));
-    if (l.lin) CK(cudaMemsetAsync(l.lin, 0, l.lin_bytes, s->stream));
-  }
+  if (S->seq_bytes) CK(cudaMemsetAsync(S->seq, 0, S->seq_bytes, s->stream));
   S->next_pos = 0;
   s->last_pos = -1;
   s->have_logits = false;
@@ -1195,8 +1198,8 @@ static dsk_state* state_create(dsk_model* m) {
   const size_t Tc = c.chunk;
   // the pieces the shared sampling / arg-max code reads
   salloc(S, (void**)&s->ctrl, sizeof(Ctrl));
-  if (alloc_host_side(s, (2 * Tc + 1) * 4)) return nullptr;
-  S->h_tok = (int*)(s->h_ctrl + 1); S->h_want = S->h_tok + Tc; S->h_err = S->h_tok + 2 * Tc;   // (zeroed)
+  if (alloc_host_side(s, (2 * (2 * Tc + 4) + 1) * 4)) return nullptr;
+  S->h_in[0] = (int*)(s->h_ctrl + 1); S->h_in[1] = S->h_in[0] + 2 * Tc + 4; S->h_err = S->h_in[1] + 2 * Tc + 4;   // (zeroed)
   s->token_log_cap = 1 << 16;
   salloc(S, (void**)&s->token_log, s->token_log_cap * sizeof(int));
   salloc(S, (void**)&s->step, sizeof(int));
@@ -1204,6 +1207,7 @@ static dsk_state* state_create(dsk_model* m) {
   salloc(S, (void**)&s->logits, (size_t)c.vocab_size * 4);
   cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
   cudaEventCreate(&s->ev0); cudaEventCreate(&s->ev1);
+  for (cudaEvent_t& e : S->in_ev) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
   if (cudaGetLastError() != cudaSuccess) { fail(-2, "state allocation failed"); return nullptr; }
   size_t mx0 = c.dim, mx1 = c.dim, mx2 = c.dim, mx3 = c.dim, mxE = 1, mxTop = 1;
   S->L.resize(M->runs.size());   // one state per layer run
@@ -1217,17 +1221,17 @@ static dsk_state* state_create(dsk_model* m) {
     LayerState& ls = S->L[r];
     if (c.block == DSK_BLOCK_POST && c.canon_taps > 1) {
       ls.canon_bytes = (size_t)2 * (c.canon_taps - 1) * c.dim * 4;
-      if (salloc(S, (void**)&ls.canon, ls.canon_bytes)) return nullptr;
+      if (salloc(S, (void**)&ls.canon, ls.canon_bytes, false, true)) return nullptr;
     }
     if (c.token_shift) {
       ls.shift_bytes = (size_t)c.dim * 4;
-      if (salloc(S, (void**)&ls.shift, ls.shift_bytes)) return nullptr;
+      if (salloc(S, (void**)&ls.shift, ls.shift_bytes, false, true)) return nullptr;
     }
     if (has_gdn(sp)) {
       const size_t KD = gdn_qk(sp), RV = gdn_v(sp), NP = (size_t)sp.gdn_kv_heads * ((sp.gdn_dim + 3) & ~3);
       ls.lin_bytes = (size_t)sp.gdn_heads * sp.gdn_dim * sp.gdn_vdim * 4;
       ls.hist_bytes = (size_t)(sp.gdn_conv - 1 + kConvSpare) * (2 * KD + RV) * 4;
-      if (salloc(S, (void**)&ls.lin, ls.lin_bytes) || salloc(S, (void**)&ls.hist, ls.hist_bytes)) return nullptr;
+      if (salloc(S, (void**)&ls.lin, ls.lin_bytes, false, true) || salloc(S, (void**)&ls.hist, ls.hist_bytes, false, true)) return nullptr;
       mxLQ = std::max(mxLQ, NP); mxLV = std::max(mxLV, RV); mxLH = std::max<size_t>(mxLH, sp.gdn_heads);
       mx0 = std::max<size_t>(mx0, att_layout(sp).total);
       mx3 = std::max<size_t>(mx3, RV + (sp.mixer2 ? (size_t)sp.att_heads * sp.att_vdim : 0));
@@ -1236,19 +1240,19 @@ static dsk_state* state_create(dsk_model* m) {
     } else if (sp.mixer == DSK_MIX_MLSTM) {
       const size_t H = sp.lin_heads, HN = H * sp.lin_dim, HP = H * sp.lin_vdim;
       ls.lin_bytes = (HN * sp.lin_vdim + HN + H) * 4;   // S, n, m
-      if (salloc(S, (void**)&ls.lin, ls.lin_bytes)) return nullptr;
+      if (salloc(S, (void**)&ls.lin, ls.lin_bytes, false, true)) return nullptr;
       mx0 = std::max<size_t>(mx0, mlstm_layout(sp).total); mx3 = std::max<size_t>(mx3, HP);
       mxLV = std::max(mxLV, HP); mxLH = std::max(mxLH, H); mxMH = std::max(mxMH, H);
     } else if (sp.mixer == DSK_MIX_LIGHTNING) {
       const size_t HN = (size_t)sp.lin_heads * sp.lin_dim, HP = (size_t)sp.lin_heads * sp.lin_vdim;
       ls.lin_bytes = HN * sp.lin_vdim * 4;
-      if (salloc(S, (void**)&ls.lin, ls.lin_bytes)) return nullptr;
+      if (salloc(S, (void**)&ls.lin, ls.lin_bytes, false, true)) return nullptr;
       mx0 = std::max<size_t>(mx0, 2 * HN + 2 * HP); mx3 = std::max<size_t>(mx3, HP);
       mxLV = std::max(mxLV, HP); mxLH = std::max<size_t>(mxLH, sp.lin_heads);
     } else if (sp.mixer == DSK_MIX_HGRN2) {
       const size_t HN = (size_t)sp.lin_heads * sp.lin_dim, HP = (size_t)sp.lin_heads * sp.lin_vdim;
       ls.lin_bytes = HN * sp.lin_vdim * 4;
-      if (salloc(S, (void**)&ls.lin, ls.lin_bytes)) return nullptr;
+      if (salloc(S, (void**)&ls.lin, ls.lin_bytes, false, true)) return nullptr;
       mx0 = std::max<size_t>(mx0, 2 * HN + HP); mx2 = std::max<size_t>(mx2, HP); mx3 = std::max<size_t>(mx3, HP);
     } else if (sp.mixer == DSK_MIX_GQA) {
       const size_t HD = (size_t)sp.att_heads * sp.att_dim, GD = (size_t)sp.att_kv_heads * sp.att_dim, GV = (size_t)sp.att_kv_heads * sp.att_vdim;
@@ -1256,20 +1260,20 @@ static dsk_state* state_create(dsk_model* m) {
         const size_t rows = (size_t)sp.att_keep_first + L.ring;   // the kept first positions have rows of their own in front of the ring
         ls.cache_bytes = rows * GD * 4;
         ls.vcache_bytes = rows * GV * 4;
-        if (salloc(S, &ls.cache, ls.cache_bytes) || salloc(S, &ls.vcache, ls.vcache_bytes)) return nullptr;
+        if (salloc(S, &ls.cache, ls.cache_bytes, false, true) || salloc(S, &ls.vcache, ls.vcache_bytes, false, true)) return nullptr;
       }
       mx0 = std::max<size_t>(mx0, (sp.att_value_proj ? HD + GD + GV : HD) + (sp.att_out_gate ? (size_t)sp.att_heads * sp.att_vdim : 0)); mx1 = std::max<size_t>(mx1, GD); mx2 = std::max<size_t>(mx2, HD);
       mx3 = std::max<size_t>(mx3, (size_t)sp.att_heads * sp.att_vdim);
       any_talk |= sp.att_talk != 0;
       if (sp.att_conv > 1) {
         ls.hist_bytes = (size_t)(sp.att_conv - 1 + kConvSpare) * (HD + GD + GV) * 4;
-        if (salloc(S, (void**)&ls.hist, ls.hist_bytes)) return nullptr;
+        if (salloc(S, (void**)&ls.hist, ls.hist_bytes, false, true)) return nullptr;
       }
       if (sp.att_vmix) mxGV = std::max(mxGV, GV);
     } else if (sp.mixer == DSK_MIX_MLA) {
       const size_t H = sp.att_heads, RW = (size_t)sp.att_kv_rank + sp.att_rot_dim;
       ls.cache_bytes = (size_t)L.ring * RW * 4;
-      if (salloc(S, &ls.cache, ls.cache_bytes)) return nullptr;
+      if (salloc(S, &ls.cache, ls.cache_bytes, false, true)) return nullptr;
       mx0 = std::max<size_t>(mx0, std::max(H * (sp.att_dim + sp.att_rot_dim), H * sp.att_vdim));
       mx1 = std::max<size_t>(mx1, sp.att_q_rank + RW);
       mx2 = std::max<size_t>(mx2, std::max<size_t>(sp.att_q_rank, H * RW));
@@ -1277,14 +1281,14 @@ static dsk_state* state_create(dsk_model* m) {
     } else if (is_ssd(sp)) {
       ls.ssm_bytes = (size_t)sp.ssm_heads * sp.ssm_vdim * sp.ssm_state * 4;
       ls.hist_bytes = (size_t)std::max(1, sp.ssm_conv - 1) * ssd_channels(sp) * 4;
-      if (salloc(S, (void**)&ls.ssm, ls.ssm_bytes) || salloc(S, (void**)&ls.hist, ls.hist_bytes)) return nullptr;
+      if (salloc(S, (void**)&ls.ssm, ls.ssm_bytes, false, true) || salloc(S, (void**)&ls.hist, ls.hist_bytes, false, true)) return nullptr;
       mx0 = std::max<size_t>(mx0, ssd_proj(sp)); mx1 = std::max<size_t>(mx1, ssd_channels(sp));
       mx2 = std::max<size_t>(mx2, ssd_inner(sp)); mx3 = std::max<size_t>(mx3, ssd_inner(sp));
       mxLH = std::max<size_t>(mxLH, sp.ssm_heads);
     } else {
       if (M->runs[r].owner_run == (int)r) {
         ls.cache_bytes = (size_t)L.ring * sp.att_kv_rank * 4;
-        if (salloc(S, &ls.cache, ls.cache_bytes)) return nullptr;
+        if (salloc(S, &ls.cache, ls.cache_bytes, false, true)) return nullptr;
       }
       mx0 = std::max<size_t>(mx0, std::max((size_t)sp.att_heads * sp.att_dim, (size_t)sp.att_heads * sp.att_vdim));
       mx1 = std::max<size_t>(mx1, sp.att_kv_rank);
@@ -1384,7 +1388,7 @@ static dsk_state* state_create(dsk_model* m) {
   rc |= salloc(S, (void**)&S->b0, Tc * mx0 * 4) | salloc(S, (void**)&S->b1, Tc * mx1 * 4) | salloc(S, (void**)&S->b2, Tc * mx2 * 4) | salloc(S, (void**)&S->b3, Tc * mx3 * 4);
   rc |= salloc(S, (void**)&S->wgt, Tc * mxTop * 4) | salloc(S, (void**)&S->d_idx, Tc * mxTop * 4) | salloc(S, (void**)&S->d_perm, Tc * mxTop * 4);
   rc |= salloc(S, (void**)&S->d_tiles, (size_t)S->max_tiles * sizeof(int4)) | salloc(S, (void**)&S->d_ntiles, 16);
-  rc |= salloc(S, (void**)&S->d_tok, Tc * 4) | salloc(S, (void**)&S->d_want, Tc * 4) | salloc(S, (void**)&S->d_ctl, 16);
+  rc |= salloc(S, (void**)&S->d_ctl, (2 * Tc + 4) * 4);
   S->head_rows = (int)std::min<size_t>(Tc, 256);
   if (c.quant == DSK_BF16 && Tc > 4) {
     // a product's input is one of b0 .. b3, a row of 2 x width values (loop products), or latents of the visible keys
@@ -1396,6 +1400,7 @@ static dsk_state* state_create(dsk_model* m) {
   }
   rc |= salloc(S, (void**)&S->logits, (size_t)S->head_rows * c.vocab_size * 4);
   if (rc || salloc_all(S, s->stream)) { fail(-2, "state allocation failed"); return nullptr; }
+  S->d_tok = S->d_ctl + 4; S->d_want = S->d_tok + Tc;
   s->logits_src = s->logits;
   m->n_states++;
   return s;
@@ -1407,6 +1412,7 @@ static void state_free(dsk_state* s) {
   if (S->step_graph) cudaGraphExecDestroy(S->step_graph);
   if (S->side) { cudaStreamSynchronize(S->side); cudaStreamDestroy(S->side); cudaEventDestroy(S->ev_fork); cudaEventDestroy(S->ev_join); }
   for (cudaEvent_t e : S->tl_events) cudaEventDestroy(e);
+  for (cudaEvent_t e : S->in_ev) if (e) cudaEventDestroy(e);
   cudaFree(S->arena);
   s->ctrl = nullptr; s->token_log = s->step = nullptr; s->sample_out = s->logits = nullptr;   // (pieces of it)
   delete S;
@@ -2604,8 +2610,7 @@ static void launch_argmax(dsk_state* s, int vocab) {
 
 // tokens [n] at positions pos0.. of the state's sequence; want: ascending indices into tokens whose logits go to host_logits
 // [n_want][vocab]; host_layers (nullable): [layers][n][width] residual stream after every layer.
-static int forward_chunk(dsk_model* m, dsk_state* s, const int32_t* tokens, int n, int pos0, const int32_t* want, int n_want,
-                         float* host_logits, float* host_layers) {
+static int run_chunks(dsk_model* m, dsk_state* s, const int32_t* tokens, int n, int pos0, const int32_t* want, int n_want, float* host_logits, float* host_layers) {
   Model* M = m->hy;
   State* S = s->hy;
   const dsk_hybrid_config& c = M->c;
@@ -2621,13 +2626,18 @@ static int forward_chunk(dsk_model* m, dsk_state* s, const int32_t* tokens, int 
   int wi = 0;
   for (int o = 0; o < n; o += S->chunk) {
     const int T = std::min(S->chunk, n - o);
-    CK(cudaStreamSynchronize(s->stream));   // the pinned staging buffers are reused
-    memcpy(S->h_tok, tokens + o, (size_t)T * 4);
+    // one copy brings the chunk in (position, tokens and rows apart, behind a wait for the chunk ahead, kept the GPU idle for some 15 us a chunk)
+    const int slot = (o / S->chunk) & 1;
+    int *in = S->h_in[slot], *in_want = in + 4 + S->chunk;
+    CK(cudaEventSynchronize(S->in_ev[slot]));   // the copy that had this staging buffer before
+    in[0] = pos0 + o;
+    memcpy(in + 4, tokens + o, (size_t)T * 4);
     int nw = 0;
-    while (wi + nw < n_want && want[wi + nw] < o + T) { S->h_want[nw] = want[wi + nw] - o; nw++; }
-    CK(cudaMemcpyAsync(S->d_tok, S->h_tok, (size_t)T * 4, cudaMemcpyHostToDevice, s->stream));
-    if (nw) CK(cudaMemcpyAsync(S->d_want, S->h_want, (size_t)nw * 4, cudaMemcpyHostToDevice, s->stream));
-    launch_next(set_ctl, 1, 1, 0, s->stream)(S->d_ctl, pos0 + o);
+    while (wi + nw < n_want && want[wi + nw] < o + T) { in_want[nw] = want[wi + nw] - o; nw++; }
+    const bool apart = S->chunk - T > 4096;     // (rows far behind the tokens of a short chunk)
+    CK(cudaMemcpyAsync(S->d_ctl, in, (size_t)(nw && !apart ? 4 + S->chunk + nw : 4 + T) * 4, cudaMemcpyHostToDevice, s->stream));
+    if (nw && apart) CK(cudaMemcpyAsync(S->d_want, in_want, (size_t)nw * 4, cudaMemcpyHostToDevice, s->stream));
+    CK(cudaEventRecord(S->in_ev[slot], s->stream));
     if (host_layers) { CK(cudaMalloc((void**)&d_trace, M->runs.size() * (size_t)T * c.dim * 4)); }
     if (enqueue_chunk(m, s, T, nw, d_trace, s->stream, pos0 + o)) { if (d_trace) cudaFree(d_trace); return -2; }
     for (int g0 = 0; g0 < nw; g0 += S->head_rows) {   // the LM head in groups of head_rows wanted rows
@@ -2639,7 +2649,7 @@ static int forward_chunk(dsk_model* m, dsk_state* s, const int32_t* tokens, int 
         launch_argmax(s, c.vocab_size);
         CK(cudaMemcpyAsync(s->h_ctrl, s->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, s->stream));
       }
-      if (host_logits && copy_to_host(s, host_logits + (size_t)(wi + g0) * c.vocab_size, S->logits, (size_t)gn * c.vocab_size * 4)) return -2;
+      if (host_logits && copy_to_host(s, host_logits + (size_t)(wi + g0) * c.vocab_size, S->logits, (size_t)gn * c.vocab_size * 4, false)) return -2;   // (the call waits at its end)
     }
     timeline_report(S, T);
     if (host_layers) {
@@ -2658,6 +2668,12 @@ static int forward_chunk(dsk_model* m, dsk_state* s, const int32_t* tokens, int 
   s->last_pos = pos0 + n - 1;
   s->have_logits = n_want > 0 && want[n_want - 1] == n - 1;
   return 0;
+}
+
+static int forward_chunk(dsk_model* m, dsk_state* s, const int32_t* tokens, int n, int pos0, const int32_t* want, int n_want, float* host_logits, float* host_layers) {
+  const int rc = run_chunks(m, s, tokens, n, pos0, want, n_want, host_logits, host_layers);
+  if (rc) cudaStreamSynchronize(s->stream);   // nothing is on its way into the caller's memory, nor out of the staging buffers
+  return rc;
 }
 
 // greedy loop on the device: arg-max of the logits in the state -> next token -> one-token chunk -> logits, n_steps times,

@@ -231,6 +231,9 @@ const char* dsk_last_error(void);
 /* Binds the calling process to CUDA device `device` (one process per GPU). */
 int dsk_init(int device);
 int dsk_sync(void);
+/* Pinned host memory for results: calls that return logits write into it directly, where pageable memory takes a second copy on the host. */
+void* dsk_host_alloc(size_t bytes);
+void dsk_host_free(void* p);
 /* Device facts for logs/bench: name (<=128 chars), SM count, HBM bytes. */
 int dsk_device_info(char* name128, int* sm_count, size_t* hbm_bytes);
 
