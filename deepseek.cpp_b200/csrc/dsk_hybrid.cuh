@@ -1075,7 +1075,6 @@ __global__ void __launch_bounds__(512) ssd_scan(const float* __restrict__ proj, 
                                                 const float* __restrict__ dt_bias, const float* __restrict__ A_log,
                                                 const float* __restrict__ Dskip, float* __restrict__ state,
                                                 float* __restrict__ out, int ld_out, int T, int H, int P, int N, int G, int PB, int TB) {
-  grid_enter();
   extern __shared__ __align__(16) float sm[];
   const int NP = (N + 3) & ~3;      // staged B / C rows are padded to whole float4s
   float* s_B = sm;                  // [TB][NP]
@@ -1094,9 +1093,10 @@ __global__ void __launch_bounds__(512) ssd_scan(const float* __restrict__ proj, 
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       const int n = 4 * (s + 8 * j) + q;
-      S[j][q] = (pok && n < N) ? state[((size_t)h * P + p) * N + n] : 0.f;
+      S[j][q] = (pok && n < N) ? __ldcg(state + ((size_t)h * P + p) * N + n) : 0.f;   // (carried from an earlier step: asked for under the kernel ahead)
     }
   const float a = -expf(A_log[h]), dsk = Dskip[h], dtb = dt_bias[h];
+  grid_enter();
   for (int t0 = 0; t0 < T; t0 += TB) {
     const int nt = min(TB, T - t0);
     __syncthreads();
@@ -1383,11 +1383,13 @@ __global__ void __launch_bounds__(256) decode_attn(const DecodeAttn P) {
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int g = (int)blockIdx.y / hblocks, hb = (int)blockIdx.y % hblocks, tq0 = (int)blockIdx.x * P.TQ;
   // query row r of the CTA: token tq0 + r % TQ, head hb * HB + r / TQ of the group
-  auto row_t = [&](int r) { return tq0 + r % P.TQ; };
-  auto row_h = [&](int r) { return hb * P.HB + r / P.TQ; };
-  auto live = [&](int r) { return r < P.TQ * P.HB && row_t(r) < P.T && row_h(r) < rep; };
-  grid_enter();
-  const int pos0 = P.ctl[0], keep = P.mods.keep;
+  const int TQ = MULTI ? P.TQ : 1, lq = MULTI ? 31 - __clz(P.TQ) : 0;   // (1, 2, 4 or 8)
+  auto row_t = [&](int r) { return tq0 + (r & (TQ - 1)); };
+  auto row_h = [&](int r) { return hb * P.HB + (r >> lq); };
+  auto live = [&](int r) { return r < TQ * P.HB && row_t(r) < P.T && row_h(r) < rep; };
+  // The position and the rows of earlier tokens are there before the kernel ahead is through (it is the one that may write the new tokens' rows): the first tile's
+  // rows are asked for under it.
+  const int pos0 = __ldcg(P.ctl), keep = P.mods.keep;
   const int j_lo = mask_first(P.mask, P.span, pos0 + tq0), nk = min(keep, j_lo);
   int lo = 0, hi = nk + pos0 + min(P.T, tq0 + P.TQ) - 1 - j_lo;   // visible keys of all rows in one index space: kept ones, then the range
   if (P.NS > 1) {
@@ -1396,25 +1398,47 @@ __global__ void __launch_bounds__(256) decode_attn(const DecodeAttn P) {
     hi = min(hi, lo + per * 32 - 1);
   }
   const bool vk = (D & 3) == 0 && (P.ldk & 3) == 0, vv = (Dv & 3) == 0 && (P.ldv & 3) == 0;   // cudaMalloc'd caches: rows on 16-byte boundaries
-  auto stage = [&](float* dst, const float* src, int ld, int off, int n, int pitch, bool vec, int j0) {
+  enum { ALL, EARLIER, NEW };   // rows of which tokens
+  auto stage = [&](float* dst, const float* src, int ld, int off, int n, int pitch, bool vec, int j0, int which) {
     for (int jj = w; jj < 32; jj += 8) {
       const int v = j0 + jj;
       float* d = dst + jj * pitch;
-      if (v > hi) { for (int r = lane; r < n; r += 32) d[r] = 0.f; continue; }
+      if (which != ALL && (v <= hi && (v < nk ? v : j_lo + v - nk) >= pos0) != (which == NEW)) continue;
+      if (v > hi) {                                  // (the values' products take four keys at a time)
+        if (j0 + (jj & ~3) <= hi) for (int r = lane; r < n; r += 32) d[r] = 0.f;
+        continue;
+      }
       const float* s = src + (size_t)cache_row(v < nk ? v : j_lo + v - nk, keep, P.ring) * ld + off;
       if (vec) { for (int r = lane * 4; r < n; r += 128) cp_async_16(d + r, s + r, 16); }
       else for (int r = lane; r < n; r += 32) d[r] = s[r];
     }
   };
   const int d4 = (D + 3) >> 2;
-  for (int r = 0; r < 8; r++) {
-    const bool on = live(r);
-    const float* src = P.q + ((size_t)row_t(r) * P.H + g * rep + row_h(r)) * D;
-    for (int e = tid; e < 4 * d4; e += 256) qs[r * pd + e] = on && e < D ? src[e] * P.scale : 0.f;
+  bool first = vk && vv && lo <= hi;   // the first tile's earlier rows are on their way
+  if (first) {
+    stage(ks, P.kc, P.ldk, g * D, D, pd, vk, lo, EARLIER);
+    cp_async_commit();
+    if (!KV) stage(vs, P.vc, P.ldv, g * Dv, Dv, pv, vv, lo, EARLIER);
+    cp_async_commit();
   }
-  if (D & 3) for (int jj = tid; jj < 32; jj += 256) for (int e = D; e < 4 * d4; e++) ks[jj * pd + e] = 0.f;   // (a depth that ends inside a group of four)
+  grid_enter();
+  // query rows, a warp a row and all of its loads in flight (row after row, each a wait for memory, took 9 us of a token's latent attention with 8 rows of 576)
   const bool mine = live(w);
   const int i_w = pos0 + row_t(w), lo_w = mask_first(P.mask, P.span, i_w), h_w = g * rep + row_h(w);
+  {
+    const float* src = P.q + ((size_t)row_t(w) * P.H + h_w) * D;
+    float* dst = qs + w * pd;
+    if ((D & 3) == 0 && D <= 1024) {
+      float4 x[8];
+#pragma unroll
+      for (int u = 0; u < 8; u++) x[u] = mine && lane + 32 * u < d4 ? reinterpret_cast<const float4*>(src)[lane + 32 * u] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int u = 0; u < 8; u++)
+        if (lane + 32 * u < d4) reinterpret_cast<float4*>(dst)[lane + 32 * u] = make_float4(x[u].x * P.scale, x[u].y * P.scale, x[u].z * P.scale, x[u].w * P.scale);
+    } else
+      for (int e = lane; e < 4 * d4; e += 32) dst[e] = mine && e < D ? src[e] * P.scale : 0.f;
+  }
+  if (D & 3) for (int jj = tid; jj < 32; jj += 256) for (int e = D; e < 4 * d4; e++) ks[jj * pd + e] = 0.f;   // (a depth that ends inside a group of four)
   float m, l, acc[8][CV];
   // A key that a row does not see has the weight 0 in that row's sums, and 0 x Inf is NaN: where a sum is not finite, the share is gone through again
   // with weights of 0 left out (a predicate per row and product, which the first walk is spared).
@@ -1425,10 +1449,12 @@ __global__ void __launch_bounds__(256) decode_attn(const DecodeAttn P) {
 #pragma unroll
       for (int k = 0; k < CV; k++) acc[r][k] = 0.f;
     for (int j0 = lo; j0 <= hi; j0 += 32) {
+      const int which = first ? NEW : ALL, nj = min(32, (hi - j0 + 4) & ~3);   // (a few keys are not 32)
+      first = false;
       __syncthreads();
-      stage(ks, P.kc, P.ldk, g * D, D, pd, vk, j0);
+      stage(ks, P.kc, P.ldk, g * D, D, pd, vk, j0, which);
       cp_async_commit();
-      if (!KV) stage(vs, P.vc, P.ldv, g * Dv, Dv, pv, vv, j0);
+      if (!KV) stage(vs, P.vc, P.ldv, g * Dv, Dv, pv, vv, j0, which);
       cp_async_commit();
       cp_async_wait<KV ? 0 : 1>();
       __syncthreads();
@@ -1473,7 +1499,7 @@ __global__ void __launch_bounds__(256) decode_attn(const DecodeAttn P) {
         for (int k = 0; k < CV; k++) acc[r][k] *= c;
       }
       if constexpr (decltype(careful)::value) {
-        for (int jj = 0; jj < 32; jj++)
+        for (int jj = 0; jj < nj; jj++)
 #pragma unroll
           for (int k = 0; k < CV; k++) {
             const int c = tid + 256 * k;
@@ -1483,7 +1509,7 @@ __global__ void __launch_bounds__(256) decode_attn(const DecodeAttn P) {
           }
       } else {
 #pragma unroll 4
-        for (int jj = 0; jj < 32; jj++) {
+        for (int jj = 0; jj < nj; jj++) {
           const float4 p0 = *reinterpret_cast<const float4*>(pt + jj * 8), p1 = *reinterpret_cast<const float4*>(pt + jj * 8 + 4);
 #pragma unroll
           for (int k = 0; k < CV; k++) {
@@ -1538,38 +1564,40 @@ __global__ void __launch_bounds__(256) decode_attn(const DecodeAttn P) {
 }
 
 // merges the NS partial softmax results of one (token, head): out = sum_s e^(m_s - m) acc_s / sum_s e^(m_s - m) l_s.
-// Grid (token x head, blocks of 128 columns): a thread owns one column and reads its NS partial values with independent loads.
+// Grid (token x head, blocks of 128 columns): a thread owns one column and reads its NS partial values with independent loads, 16 at a time.
 __global__ void __launch_bounds__(128) latent_swa_merge(const float* __restrict__ part, float* __restrict__ out, int R, int NS,
                                                         const float* __restrict__ gate = nullptr, int ld_gate = 0, int H = 1,
                                                         int gate_head = 0, int ld_out = 0, float alpha = 1.f) {
   grid_enter();
-  __shared__ float wts[64], ms[64], ls[64];   // NS <= 64 (kAttnSplitMax)
+  __shared__ float wts[64];   // NS <= 64 (kAttnSplitMax)
   const size_t th = blockIdx.x;
   const float* pp = part + th * NS * (R + 2);
-  if ((int)threadIdx.x < NS) { ms[threadIdx.x] = pp[(size_t)threadIdx.x * (R + 2)]; ls[threadIdx.x] = pp[(size_t)threadIdx.x * (R + 2) + 1]; }
+  const int r = blockIdx.y * 128 + threadIdx.x, lane = threadIdx.x & 31;
+  // the shares' maxima and sums, two a lane, and the first values of this thread's column: all loads ahead of the first use
+  constexpr int AHEAD = 16;
+  float m0 = -1e30f, l0 = 0.f, m1 = -1e30f, l1 = 0.f, v[AHEAD];
+  if (lane < NS) { m0 = pp[(size_t)lane * (R + 2)]; l0 = pp[(size_t)lane * (R + 2) + 1]; }
+  if (lane + 32 < NS) { m1 = pp[(size_t)(lane + 32) * (R + 2)]; l1 = pp[(size_t)(lane + 32) * (R + 2) + 1]; }
+#pragma unroll
+  for (int s = 0; s < AHEAD; s++) v[s] = s < NS && r < R ? pp[(size_t)s * (R + 2) + 2 + r] : 0.f;
+  const float m = warp_max(fmaxf(m0, m1)), w0 = expf(m0 - m), w1 = expf(m1 - m);
+  const float inv = 1.f / warp_sum(fmaf(w0, l0, w1 * l1));
+  if (threadIdx.x < 32) { wts[lane] = w0; wts[lane + 32] = w1; }
   __syncthreads();
-  float m = -1e30f;
-  for (int s = 0; s < NS; s++) m = fmaxf(m, ms[s]);
-  if ((int)threadIdx.x < NS) wts[threadIdx.x] = expf(ms[threadIdx.x] - m);
-  __syncthreads();
-  float l = 0.f;
-  for (int s = 0; s < NS; s++) l = fmaf(wts[s], ls[s], l);
-  const float inv = 1.f / l;
-  const int r = blockIdx.y * 128 + threadIdx.x;
   if (r >= R) return;
-  float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
-  int s = 0;
-#pragma unroll 4
-  for (; s + 4 <= NS; s += 4) {
-    const float v0 = pp[(size_t)s * (R + 2) + 2 + r], v1 = pp[(size_t)(s + 1) * (R + 2) + 2 + r];
-    const float v2 = pp[(size_t)(s + 2) * (R + 2) + 2 + r], v3 = pp[(size_t)(s + 3) * (R + 2) + 2 + r];
-    a0 = fmaf(wts[s], v0, a0); a1 = fmaf(wts[s + 1], v1, a1); a2 = fmaf(wts[s + 2], v2, a2); a3 = fmaf(wts[s + 3], v3, a3);
+  float a[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int s = 0; s < AHEAD; s++) if (s < NS) a[s & 3] = fmaf(wts[s], v[s], a[s & 3]);
+  for (int s0 = AHEAD; s0 < NS; s0 += AHEAD) {
+#pragma unroll
+    for (int s = 0; s < AHEAD; s++) v[s] = s0 + s < NS ? pp[(size_t)(s0 + s) * (R + 2) + 2 + r] : 0.f;
+#pragma unroll
+    for (int s = 0; s < AHEAD; s++) if (s0 + s < NS) a[s & 3] = fmaf(wts[s0 + s], v[s], a[s & 3]);
   }
-  for (; s < NS; s++) a0 = fmaf(wts[s], pp[(size_t)s * (R + 2) + 2 + r], a0);
   // gate (nullable): row th = token * H + head is multiplied by sigmoid(gate[token][head * R + r]), with gate_head by sigmoid(gate[token][head]);
   // ld_out > 0: pitch of a token's output row (otherwise H * R); every result is multiplied by alpha
   const float gt = gate ? sigmoid_f(gate[(th / H) * (size_t)ld_gate + (gate_head ? th % H : (th % H) * (size_t)R + r)]) : 1.f;
-  out[(ld_out > 0 ? (th / H) * (size_t)ld_out + (th % H) * (size_t)R : th * R) + r] = ((a0 + a1) + (a2 + a3)) * inv * gt * alpha;
+  out[(ld_out > 0 ? (th / H) * (size_t)ld_out + (th % H) * (size_t)R : th * R) + r] = ((a[0] + a[1]) + (a[2] + a[3])) * inv * gt * alpha;
 }
 
 // out[t][c] *= sigmoid(gate[t][c / per]) for the n columns of T rows (an output gate whose raw values came out of a stacked
@@ -1740,8 +1768,11 @@ __global__ void __launch_bounds__(256) layer_norm_add_norm(const float* __restri
 // h = x / sqrt(mean(x^2) + eps) * w.  The row stays in registers up to 256 * kLnRegs values.
 __global__ void __launch_bounds__(256) rms_open(float* __restrict__ x, const float* __restrict__ e, const float* __restrict__ row,
                                                 const float* __restrict__ w, float* __restrict__ h, int n, float eps) {
-  grid_enter();
   __shared__ float red[33];
+  float wt[kLnRegs];   // (the model's: under the kernel ahead, not behind the sum)
+#pragma unroll
+  for (int k = 0; k < kLnRegs; k++) { const int i = threadIdx.x + 256 * k; wt[k] = i < n ? w[i] : 0.f; }
+  grid_enter();
   float* xr = x + (size_t)blockIdx.x * n;
   const float* er = e ? e + (size_t)blockIdx.x * n : nullptr;
   float* hr = h + (size_t)blockIdx.x * n;
@@ -1764,7 +1795,7 @@ __global__ void __launch_bounds__(256) rms_open(float* __restrict__ x, const flo
   }
   const float sc = 1.f / sqrtf(block_sum(ss, red) / (float)n + eps);
 #pragma unroll
-  for (int k = 0; k < kLnRegs; k++) { const int i = threadIdx.x + 256 * k; if (i < n) hr[i] = v[k] * sc * w[i]; }
+  for (int k = 0; k < kLnRegs; k++) { const int i = threadIdx.x + 256 * k; if (i < n) hr[i] = v[k] * sc * wt[k]; }
   for (int i = threadIdx.x + 256 * kLnRegs; i < n; i += 256) hr[i] = xr[i] * sc * w[i];
 }
 
@@ -1779,8 +1810,15 @@ __global__ void __launch_bounds__(NT) rms_add_norm(const float* __restrict__ y, 
                                                     const float* __restrict__ wsh, const float* __restrict__ wy, const float* x, float* xo, int ldxo,
                                                     const float* __restrict__ wh, float* __restrict__ h, int n,
                                                     float eps, float alpha) {
-  grid_enter();
   __shared__ float red[33];
+  // a decoded token's row: the model's weights under the kernel ahead, not each behind its sum
+  constexpr bool EARLY = NT == 1024;
+  float a_w[EARLY ? KR : 1], b_w[EARLY ? KR : 1];
+  if constexpr (EARLY) {
+#pragma unroll
+    for (int k = 0; k < KR; k++) { const int i = threadIdx.x + NT * k; a_w[k] = i < n ? wy[i] : 0.f; b_w[k] = wh && i < n ? wh[i] : 0.f; }
+  }
+  grid_enter();
   const size_t t = blockIdx.x;
   float v[KR], u[KR], ss = 0.f;
 #pragma unroll
@@ -1817,12 +1855,12 @@ __global__ void __launch_bounds__(NT) rms_add_norm(const float* __restrict__ y, 
 #pragma unroll
   for (int k = 0; k < KR; k++) {
     const int i = threadIdx.x + NT * k;
-    if (i < n) { u[k] = fmaf(v[k] * sc, wy[i], u[k]); xo[t * ldxo + i] = u[k]; ss = fmaf(u[k], u[k], ss); }
+    if (i < n) { u[k] = fmaf(v[k] * sc, EARLY ? a_w[EARLY ? k : 0] : wy[i], u[k]); xo[t * ldxo + i] = u[k]; ss = fmaf(u[k], u[k], ss); }
   }
   if (!wh) return;
   sc = 1.f / sqrtf(block_sum(ss, red) / (float)n + eps);
 #pragma unroll
-  for (int k = 0; k < KR; k++) { const int i = threadIdx.x + NT * k; if (i < n) h[t * n + i] = u[k] * sc * wh[i]; }
+  for (int k = 0; k < KR; k++) { const int i = threadIdx.x + NT * k; if (i < n) h[t * n + i] = u[k] * sc * (EARLY ? b_w[EARLY ? k : 0] : wh[i]); }
 }
 
 // the T rows of a step (pitch ls) copied to rows of pitch ld

@@ -585,7 +585,6 @@ template <int MODE, int RN>
 __global__ void __launch_bounds__(kLinDecodeThreads) lin_decode(const GdnP D, const float* __restrict__ decay, float* __restrict__ state,
                                                                 const float* __restrict__ norm_w, float eps, int gate_off, float alpha,
                                                                 float* __restrict__ out, int ldo, const MlstmP X) {
-  grid_enter();
   constexpr bool DELTA = MODE == LIN_DELTA, MLSTM = MODE == LIN_MLSTM;
   extern __shared__ __align__(16) float sm[];
   __shared__ float red[33], gb[5];
@@ -601,20 +600,21 @@ __global__ void __launch_bounds__(kLinDecodeThreads) lin_decode(const GdnP D, co
   float* sn = part + 2 * (size_t)NG * 4 * PL;   // [N]  (mLSTM)
   const bool vec = (P & 3) == 0;
   if (MLSTM) {
-    for (int n = tid; n < N; n += kLinDecodeThreads) sn[n] = X.n[(size_t)h * N + n];
-    if (tid == 0) gb[3] = X.m[h];
+    for (int n = tid; n < N; n += kLinDecodeThreads) sn[n] = __ldcg(X.n + (size_t)h * N + n);
+    if (tid == 0) gb[3] = __ldcg(X.m + h);
   }
 #pragma unroll
   for (int r = 0; r < RN; r++) {
     const int n = ng + NG * r;
     const float* src = state + ((size_t)h * N + n) * P + 4 * pl;
     if (on && n < N && vec) {
-      const float4 v = *reinterpret_cast<const float4*>(src);
+      const float4 v = __ldcg(reinterpret_cast<const float4*>(src));
       S[r][0] = v.x; S[r][1] = v.y; S[r][2] = v.z; S[r][3] = v.w;
     } else
 #pragma unroll
-      for (int c = 0; c < 4; c++) S[r][c] = on && n < N && 4 * pl + c < P ? src[c] : 0.f;
+      for (int c = 0; c < 4; c++) S[r][c] = on && n < N && 4 * pl + c < P ? __ldcg(src + c) : 0.f;
   }
+  grid_enter();   // (what the sequence carries comes from an earlier step: asked for under the kernel ahead)
   const int KD = D.G * N, CH = 2 * KD + D.H * P, pos0 = D.ctl[0];
   for (int t = 0; t < D.T; t++) {
     const float* pr = D.proj + (size_t)t * D.ld;
