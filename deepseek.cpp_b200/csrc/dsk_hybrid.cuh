@@ -1637,15 +1637,15 @@ __global__ void pack_keys_values(const float* __restrict__ kf, const float* __re
   }
 }
 
-// S [H][Tq][Lk] in place: the first nk columns are positions 0 .. nk - 1 (kept first positions that lie before `first`), column
+// S [H][Tq][Lk] (row pitch ld) in place: the first nk columns are positions 0 .. nk - 1 (kept first positions that lie before `first`), column
 // c >= nk is position first + c - nk; row t is position qpos0 + t and sees j <= i inside its mask or among the kept first
 // positions.  Visible scores are modified (ScoreMods) and normalised, hidden entries become 0.
-__global__ void __launch_bounds__(128) softmax_band(float* __restrict__ S, int Tq, int Lk, int first, int qpos0, int mask, int window,
+__global__ void __launch_bounds__(128) softmax_band(float* __restrict__ S, int Tq, int Lk, int ld, int first, int qpos0, int mask, int window,
                                                     int nk, ScoreMods sm) {
   grid_enter();
   __shared__ float red[33];
   const int t = blockIdx.x, h = blockIdx.y, H = gridDim.y;
-  float* row = S + ((size_t)h * Tq + t) * Lk;
+  float* row = S + ((size_t)h * Tq + t) * ld;
   const int i = qpos0 + t, j_lo = mask_first(mask, window, i);
   float mx = -1e30f;
   for (int c = threadIdx.x; c < Lk; c += blockDim.x) {
@@ -2219,11 +2219,11 @@ __global__ void __launch_bounds__(256) gqa_attn(const float* __restrict__ q, con
 
 // Portions run the same attention as matrix products per block of queries (like the latent attention above).  pack_ring_kv
 // gathers the visible positions first .. first + Lk - 1 from the ring caches into per-group operands: keys [G][Lk][D], values
-// transposed [G][Dv][Lk].  mix_softmax mixes the heads' scores in a [H][Tq][Lk] score array.
+// transposed [G][Dv][Lk] (row pitch ld_vt).  mix_softmax mixes the heads' scores in a [H][Tq][Lk] score array.
 // The first nk operand rows are the kept first positions 0 .. nk - 1 (cache rows of their own, see cache_row).
 template <typename WT>
 __global__ void pack_ring_kv(const float* __restrict__ kc, const float* __restrict__ vc, WT* __restrict__ kb, WT* __restrict__ vt,
-                             int first, int Lk, int ring, int G, int D, int Dv, int nk, int keep) {
+                             int first, int Lk, int ld_vt, int ring, int G, int D, int Dv, int nk, int keep) {
   grid_enter();
   const int j = blockIdx.x;
   const size_t row = (size_t)cache_row(j < nk ? j : first + j - nk, keep, ring);
@@ -2233,7 +2233,7 @@ __global__ void pack_ring_kv(const float* __restrict__ kc, const float* __restri
   }
   for (int e = threadIdx.x; e < G * Dv; e += blockDim.x) {
     const int g = e / Dv, v = e - g * Dv;
-    vt[((size_t)g * Dv + v) * Lk + j] = from_f<WT>(vc[row * G * Dv + e]);
+    vt[((size_t)g * Dv + v) * ld_vt + j] = from_f<WT>(vc[row * G * Dv + e]);
   }
 }
 
@@ -2304,13 +2304,13 @@ __global__ void pack_mla_kv(const float* __restrict__ kf, const float* __restric
   }
 }
 
-// One CTA per query, in place on S [H][Tq][Lk]: the heads' scores of a key mixed, s'_h = sum_g talk[h][g] s_g, masked, and the softmax over a
+// One CTA per query, in place on S [H][Tq][Lk] (row pitch ld): the heads' scores of a key mixed, s'_h = sum_g talk[h][g] s_g, masked, and the softmax over a
 // head's keys (hidden keys get 0 and are not read).  HR > 0: a thread has the HR >= H scores of a key in registers; 0 (more than 32 heads):
 // in shared memory.  The mixed scores stay in shared memory between the two parts where H x Lk floats fit (staged), else in S.
 // Bound: the scores' way in and out of L2.  Mixing and softmax as kernels of their own, with an array between them, took 39 us per 256 queries
 // of 16 heads behind 1023 keys.
 template <int HR>
-__global__ void __launch_bounds__(HR ? 512 : 128) mix_softmax(float* __restrict__ S, const float* __restrict__ talk, int H, int Tq, int Lk, int first, int qpos0,
+__global__ void __launch_bounds__(HR ? 512 : 128) mix_softmax(float* __restrict__ S, const float* __restrict__ talk, int H, int Tq, int Lk, int ld, int first, int qpos0,
                                                               int mask, int window, int nk, ScoreMods sm, int staged) {
   grid_enter();
   extern __shared__ __align__(16) float sh[];
@@ -2318,8 +2318,8 @@ __global__ void __launch_bounds__(HR ? 512 : 128) mix_softmax(float* __restrict_
   const int tp = HR ? TP : H, t = blockIdx.x, i = qpos0 + t, j_lo = mask_first(mask, window, i), nt = blockDim.x;
   float* tk = sh;                                            // [H][tp]
   float* col = sh + (H * tp + 3) / 4 * 4;                    // HR 0: [H][nt]
-  float* row = S + (size_t)t * Lk;                           // head g: + g Tq Lk
-  const size_t hs = (size_t)Tq * Lk;
+  float* row = S + (size_t)t * ld;                           // head g: + g Tq ld
+  const size_t hs = (size_t)Tq * ld;
   float* mixed = staged ? col + (HR ? 0 : H * nt) : row;
   const size_t ms = staged ? (size_t)Lk : hs;
   for (int k = threadIdx.x; k < H * tp; k += nt) tk[k] = k % tp < H ? talk[k / tp * H + k % tp] : 0.f;

@@ -417,7 +417,8 @@ static void set_kernel_attrs() {
   cudaFuncSetAttribute(pattn<A, B, 4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax); cudaFuncSetAttribute(pattn<A, B, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax)
   DSK_PATTN_ATTR(1, 8); DSK_PATTN_ATTR(1, 16); DSK_PATTN_ATTR(3, 8); DSK_PATTN_ATTR(3, 16);
 #undef DSK_PATTN_ATTR
-#define DSK_SPLIT_ATTR(E) cudaFuncSetAttribute(gemm_split<E>, cudaFuncAttributeMaxDynamicSharedMemorySize, split_smem(kSplitStages))
+#define DSK_SPLIT_ATTR(E) cudaFuncSetAttribute(gemm_split<E, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, split_smem(kSplitStages)); \
+  cudaFuncSetAttribute(gemm_split<E, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, split_smem(kSplitStages))
   DSK_SPLIT_ATTR(HEPI_STORE); DSK_SPLIT_ATTR(HEPI_ADD); DSK_SPLIT_ATTR(HEPI_GLU); DSK_SPLIT_ATTR(HEPI_XIELU); DSK_SPLIT_ATTR(HEPI_GEGLU); DSK_SPLIT_ATTR(HEPI_SIGMUL);
   DSK_SPLIT_ATTR(HEPI_RELU2); DSK_SPLIT_ATTR(HEPI_LINGATE); DSK_SPLIT_ATTR(HEPI_SILU_SIG); DSK_SPLIT_ATTR(HEPI_SOFTCAP); DSK_SPLIT_ATTR(HEPI_SWIGLU); DSK_SPLIT_ATTR(HEPI_GELU_MUL);
 #undef DSK_SPLIT_ATTR
@@ -1365,10 +1366,10 @@ static dsk_state* state_create(dsk_model* m) {
     if (rows > 0 && fused <= kPortionBytes + kPortionBytes / 2 && plain <= kPortionBytes) {
       S->prefill_keys = (int)rows;
       if (k16) rc |= salloc(S, (void**)&S->ppart, shares * 4, true) | salloc(S, (void**)&S->k16, k16 * 2, true) | salloc(S, (void**)&S->v16, v16 * 2, true);
-      rc |= salloc(S, (void**)&S->kf, std::max(kup, keys * hd) * 4, true) | salloc(S, (void**)&S->vf, std::max(vup, keys * hv) * 4, true);
+      rc |= salloc(S, (void**)&S->kf, std::max(kup, keys * hd) * 4, true) | salloc(S, (void**)&S->vf, std::max(vup, (keys + 3) * hv) * 4, true);
       rc |= salloc(S, (void**)&S->d_rows, rows * 4, true);
       if (pack_es) rc |= salloc(S, &S->kb, keys * hd * pack_es, true) | salloc(S, &S->vt, keys * hv * pack_es, true);
-      if (keys) rc |= salloc(S, (void**)&S->sc, heads * S->talk_q * keys * 4, true);
+      if (keys) rc |= salloc(S, (void**)&S->sc, heads * S->talk_q * (keys + 3) * 4, true);   // (rows of whole quads)
     }
   }
   rc |= salloc(S, (void**)&S->x, Tc * c.dim * 4) | salloc(S, (void**)&S->h, Tc * c.dim * 4);
@@ -1456,22 +1457,30 @@ static thread_local bool chain_step = false, plain_next = false;
 template <typename... KA> struct Launch {
   void (*kernel)(KA...);
   cudaLaunchConfig_t cfg;
+  unsigned cluster;   // CTAs of a cluster, along x
   template <typename... A> void operator()(A&&... a) const {
     static_assert(sizeof...(A) == sizeof...(KA), "every argument of a kernel is given");
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute at[2]{};
     cudaLaunchConfig_t c = cfg;
-    if (chain_step && !plain_next) { c.attrs = &at; c.numAttrs = 1; }
+    c.attrs = at;
+    c.numAttrs = 0;
+    if (chain_step && !plain_next) {
+      at[c.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      at[c.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+      at[c.numAttrs].id = cudaLaunchAttributeClusterDimension;
+      at[c.numAttrs].val.clusterDim.x = cluster; at[c.numAttrs].val.clusterDim.y = 1; at[c.numAttrs++].val.clusterDim.z = 1;
+    }
     plain_next = false;
     cudaLaunchKernelEx(&c, kernel, static_cast<KA>(a)...);
   }
 };
 template <typename... KA>
-static Launch<KA...> launch_next(void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t st) {
+static Launch<KA...> launch_next(void (*kernel)(KA...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, unsigned cluster = 1) {
   cudaLaunchConfig_t c{};
   c.gridDim = grid; c.blockDim = block; c.dynamicSmemBytes = smem; c.stream = st;
-  return {kernel, c};
+  return {kernel, c, cluster};
 }
 
 static GemmP gp(const float* A, int lda, const void* W, int ldw, float* C, int ldc, int M, int N, int K) {
@@ -1609,12 +1618,37 @@ static void launch_gemv(int epi, const GemmP& P, int Z, cudaStream_t st) {
   }
 }
 // fp32 products of more than four rows, routed ones in tiles of 128 (gemm_split)
-static void launch_split(State* S, int epi, const GemmP& P, int Z, int tile_cap, cudaStream_t st) {
+static void launch_split(State* state, int epi, const GemmP& P, int Z, int tile_cap, cudaStream_t st) {
   const int bn = epi_dual(epi) ? kSplitN / 2 : kSplitN;
-  const dim3 grid((unsigned)((P.N + bn - 1) / bn), (unsigned)(P.tiles ? tile_cap : (P.M + kTcRows - 1) / kTcRows), (unsigned)Z);
+  const int mt = P.tiles ? tile_cap : (P.M + kTcRows - 1) / kTcRows, nt = (P.N + bn - 1) / bn, slices = (P.K + kSplitDepth - 1) / kSplitDepth;
+  // Shares of the depth, a cluster of CTAs a tile: rounds of CTAs x (slices of 2000 cycles + what a tile takes besides, joining included).  45 x 1024 x 4096: 59 us by tiles
+  // alone, 27 with four CTAs a tile; 37 x 130 x 8192 108 and 26 with eight; 600 x 1024 x 2816, 80 tiles, 56 and 70 with two.
+  static const std::array<int, 9> room = [] {   // CTAs of clusters of c that run at a time (not all SMs are in a group of eight)
+    std::array<int, 9> r{};
+    for (int c = 2; c <= 8; c *= 2) {
+      cudaLaunchConfig_t cfg{};
+      cudaLaunchAttribute at{};
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim.x = (unsigned)c; at.val.clusterDim.y = at.val.clusterDim.z = 1;
+      cfg.gridDim = dim3((unsigned)c * 32); cfg.blockDim = dim3(kSplitThreads); cfg.dynamicSmemBytes = split_smem(kSplitStages); cfg.attrs = &at; cfg.numAttrs = 1;
+      int n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, gemm_split<HEPI_STORE, true>, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+      r[c] = n * c;
+    }
+    return r;
+  }();
+  int S = 1;
+  long long best = 0;
+  for (int c = 1; c <= 8 && c <= slices && (c == 1 || (!P.band && room[c])); c *= 2) {
+    const long long ctas = (long long)mt * nt * Z * c, at_once = c == 1 ? g_sm_count : room[c];
+    const long long cost = (ctas + at_once - 1) / at_once * ((slices + c - 1) / c * 2000LL + (c > 1 ? 8000 : 5500));
+    if (c == 1 || cost < best) { best = cost; S = c; }
+  }
+  const dim3 grid((unsigned)(nt * S), (unsigned)mt, (unsigned)Z);
   // (a short depth takes no more of an SM than it has slices: short steps' next kernels start beside it)
-  const int stages = std::max(1, std::min(kSplitStages, (P.K + kSplitDepth - 1) / kSplitDepth));
-#define DSK_SPLIT(E) case E: launch_next(gemm_split<E>, grid, kSplitThreads, split_smem(stages), st)(P, stages, S->h_err); break
+  const int stages = std::max(1, std::min(kSplitStages, (slices + S - 1) / S));
+#define DSK_SPLIT(E) case E: if (S > 1) launch_next(gemm_split<E, true>, grid, kSplitThreads, split_smem(stages), st, (unsigned)S)(P, stages, S, state->h_err); \
+    else launch_next(gemm_split<E, false>, grid, kSplitThreads, split_smem(stages), st)(P, stages, 1, state->h_err); break
   switch (epi) {
     DSK_SPLIT(HEPI_STORE); DSK_SPLIT(HEPI_ADD); DSK_SPLIT(HEPI_GLU); DSK_SPLIT(HEPI_XIELU); DSK_SPLIT(HEPI_GEGLU); DSK_SPLIT(HEPI_SIGMUL);
     DSK_SPLIT(HEPI_RELU2); DSK_SPLIT(HEPI_LINGATE); DSK_SPLIT(HEPI_SILU_SIG); DSK_SPLIT(HEPI_SOFTCAP); DSK_SPLIT(HEPI_SWIGLU); DSK_SPLIT(HEPI_GELU_MUL);
@@ -1637,6 +1671,13 @@ static void linear(State* S, bool bf16, int epi, const GemmP& P, int Z, cudaStre
   if (!small && !P.tiles && Z == 1 && P.N <= 96) {   // narrow output (router, token-input gate): warp-per-row products over batches of 4 rows
     // (a CTA of gemm_narrow has 16 rows: under 448 they are too few.  Steps of 256 / 384 / 512 / 1024 tokens, two layers with 64 experts and a token input of
     // 32, width 2048: 714 / 819 / 873 / 1126 us with it, 650 / 806 / 895 / 1221 with the products of warps; width 1024: 519 / 669 / 738 / 786 and 506 / 654 / 749 / 832)
+    // (fp32 ones of some more are faster in three parts, their depth shared by a cluster.  64 columns, us, gemm_narrow and gemm_split: 2048 rows 2048 deep 31 and 19, 448 rows
+    // 2048 deep 21 and 14, 777 rows 1024 deep 12 and 12)
+    if (!bf16 && P.M >= kNarrowMin && (long long)P.M * P.K >= 900000) {
+      launch_split(S, epi, P, 1, 0, st);
+      S->launches++;
+      return;
+    }
     if (epi != HEPI_SIGMUL && P.M >= kNarrowMin && !epi_dual(epi)) {
       launch_narrow(bf16, epi, P, st);
       S->launches++;
@@ -2133,12 +2174,13 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         for (int t0 = 0; t0 < T; t0 += block_q) {
           const int Tq = std::min(block_q, T - t0), qpos0 = pos0 + t0;
           const int first = mask_first(sp.att_mask, sp.att_window, qpos0), nk = std::min(keep, first), Lk = nk + qpos0 + Tq - first;
-          launch_next(pack_ring_kv<float>, Lk, 256, 0, st)(kc, vc, S->kf, S->vf, first, Lk, ring, G, D, V, nk, keep);
+          const int LP = (Lk + 3) & ~3;   // rows of scores and of transposed values take 16-byte loads
+          launch_next(pack_ring_kv<float>, Lk, 256, 0, st)(kc, vc, S->kf, S->vf, first, Lk, LP, ring, G, D, V, nk, keep);
           S->launches++;
           MK("att.pack");
-          GemmP Sc = gp(S->b2 + (size_t)t0 * HD, HD, S->kf, D, S->sc, Lk, Tq, Lk, D);
+          GemmP Sc = gp(S->b2 + (size_t)t0 * HD, HD, S->kf, D, S->sc, LP, Tq, Lk, D);
           Sc.w_made = 1;
-          Sc.sA = D; Sc.sW = (long long)Lk * D; Sc.z_wdiv = rep; Sc.sC = (long long)Tq * Lk; Sc.alpha = sp.att_scale;
+          Sc.sA = D; Sc.sW = (long long)Lk * D; Sc.z_wdiv = rep; Sc.sC = (long long)Tq * LP; Sc.alpha = sp.att_scale;
           Sc.band = BAND_COLS; Sc.band_first = first - nk; Sc.band_pos = qpos0; Sc.band_mask = sp.att_mask; Sc.band_window = sp.att_window; Sc.band_keep = keep;
           linear(S, false, HEPI_STORE, Sc, H, st);
           MK("att.scores");
@@ -2147,15 +2189,15 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
             const size_t base = ((size_t)(H * (hr ? hr : H) + 3) / 4 * 4 + (hr ? 0 : (size_t)H * nt)) * 4, all = base + (size_t)H * Lk * 4;
             const int staged = all <= (size_t)200 * 1024;
             auto* kernel = hr == 16 ? mix_softmax<16> : hr == 32 ? mix_softmax<32> : mix_softmax<0>;
-            launch_next(kernel, (unsigned)Tq, (unsigned)nt, staged ? all : base, st)(S->sc, L.talk, H, Tq, Lk, first, qpos0, sp.att_mask, sp.att_window, nk, sm, staged);
+            launch_next(kernel, (unsigned)Tq, (unsigned)nt, staged ? all : base, st)(S->sc, L.talk, H, Tq, Lk, LP, first, qpos0, sp.att_mask, sp.att_window, nk, sm, staged);
           } else {
-            launch_next(softmax_band, dim3((unsigned)Tq, (unsigned)H), 128, 0, st)(S->sc, Tq, Lk, first, qpos0, sp.att_mask, sp.att_window, nk, sm);
+            launch_next(softmax_band, dim3((unsigned)Tq, (unsigned)H), 128, 0, st)(S->sc, Tq, Lk, LP, first, qpos0, sp.att_mask, sp.att_window, nk, sm);
           }
           S->launches++;
           MK("att.softmax");
-          GemmP Ov = gp(S->sc, Lk, S->vf, Lk, S->b3 + (size_t)t0 * ldo, ldo, Tq, V, Lk);
+          GemmP Ov = gp(S->sc, LP, S->vf, LP, S->b3 + (size_t)t0 * ldo, ldo, Tq, V, Lk);
           Ov.w_made = 1;
-          Ov.sA = (long long)Tq * Lk; Ov.sW = (long long)V * Lk; Ov.z_wdiv = rep; Ov.sC = V; Ov.alpha = lscale;
+          Ov.sA = (long long)Tq * LP; Ov.sW = (long long)V * LP; Ov.z_wdiv = rep; Ov.sC = V; Ov.alpha = lscale;
           Ov.band = BAND_DEPTH; Ov.band_first = Sc.band_first; Ov.band_pos = qpos0; Ov.band_mask = sp.att_mask; Ov.band_window = sp.att_window; Ov.band_keep = Sc.band_keep;
           linear(S, false, HEPI_STORE, Ov, H, st);
           MK("att.pv");
@@ -2248,7 +2290,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
           Sc.sA = DK; Sc.sW = (long long)Lk * DK; Sc.sC = (long long)Tq * Lk; Sc.alpha = sp.att_scale;
           linear(S, false, HEPI_STORE, Sc, H, st);
           MK("att.scores");
-          launch_next(softmax_band, dim3((unsigned)Tq, (unsigned)H), 128, 0, st)(S->sc, Tq, Lk, first, qpos0, sp.att_mask, sp.att_window, 0, sm);
+          launch_next(softmax_band, dim3((unsigned)Tq, (unsigned)H), 128, 0, st)(S->sc, Tq, Lk, Lk, first, qpos0, sp.att_mask, sp.att_window, 0, sm);
           MK("att.softmax");
           GemmP Ov = gp(S->sc, Lk, S->vt, Lk, S->b3 + (size_t)t0 * H * V, H * V, Tq, V, Lk);
           Ov.w_made = 1;
@@ -2422,7 +2464,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
           MK("att.pack");
           linear(S, bf, HEPI_STORE, Sc, H, st);
           MK("att.scores");
-          launch_next(softmax_band, dim3((unsigned)Tq, (unsigned)H), 128, 0, st)(S->sc, Tq, Lk, first, qpos0, sp.att_mask, sp.att_window, 0, ScoreMods{});
+          launch_next(softmax_band, dim3((unsigned)Tq, (unsigned)H), 128, 0, st)(S->sc, Tq, Lk, Lk, first, qpos0, sp.att_mask, sp.att_window, 0, ScoreMods{});
           GemmP Ov = gp(S->sc, Lk, S->vt, Lk, S->b3 + (size_t)t0 * H * V, H * V, Tq, V, Lk);
           Ov.w_made = 1;
           Ov.sA = (long long)Tq * Lk; Ov.sW = (long long)V * Lk; Ov.sC = V;

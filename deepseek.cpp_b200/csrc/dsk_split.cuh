@@ -11,9 +11,10 @@
 // inside of 64 elements the leading products are four additions of the tensor core.
 // Bound: the banks of shared memory, some 2000 cycles a slice: 768 for the operands of the products (which take 890 by themselves), 576 for the parts, 384 for the numbers
 // on their way through L1, the rest for rows' addresses and results.  Measured, us, before (the same six products on mma.sync, two CTAs of 128 x 64 an SM) and now, rows x columns x
-// depth: 600 x 4160 x 1024 139 and 68, 600 x 1024 x 2816 140 and 55, 45 x 1024 x 4096 203 and 59, 5 x 1024 x 1024 53 and 19, 1024 x 128 x 512 30 and 17; 64 x 100 x 36 8.3 and
-// 8.5.  Error against 64 bits, normal operands, depth 1024 / 2816 / 4096: 1.5, 2.4, 2.9e-7 before, 1.0, 1.4, 1.6e-7 now; positive ones, depth 512 / 1000: 1.0 and 1.3e-7 before, 0.9
-// and 1.0e-7 now.  Tried: numbers past L1 (3 to 10 % longer), rows' addresses in registers (they spill), eight or twelve splitting warps (84 and 60 instead of 55 us).
+// depth: 600 x 4160 x 1024 139 and 72, 600 x 1024 x 2816 140 and 57, 45 x 1024 x 4096 203 and 27 (four CTAs share a tile's depth, 61 by one), 5 x 1024 x 1024 53 and 12, 1024 x 128 x
+// 512 30 and 13; 64 x 100 x 36 8 and 9.  Error against 64 bits, normal operands, depth 1024 / 2816 / 4096: 1.5, 2.4, 2.9e-7 before, 1.0, 1.4, 1.6e-7 now; positive ones, depth 512 /
+// 1000: 1.0 and 1.3e-7 before, 0.9 and 1.0e-7 now.  Tried: numbers past L1 (3 to 10 % longer), rows' addresses in registers (they spill), eight or twelve splitting warps (84 and 60
+// instead of 55 us).
 // The products that the three parts leave out are below an fp32 rounding.
 #pragma once
 
@@ -74,49 +75,52 @@ __device__ __forceinline__ void tc_load16(uint32_t addr, uint32_t (&r)[16]) {
 // A splitting warp's way through the half slices of its group: group g has half slices g, g + 4, ..  Eight lanes have the 32 values of a row, a load four rows: w + 4 q of every
 // 16 (rows 4 apart are on different banks behind the swizzle, whose phase is one for all rows of a lane).  The numbers of a group's next half slice are asked for as soon as
 // the registers of this one's are free: 48 KB a slice cross from L2 at some 64 bytes a clock, which is as long as the products of a slice take.
+// VEC: rows on 16-byte boundaries with whole quads behind their last numbers; the others are read number by number when they are needed.
 template <bool VEC>
 __device__ __forceinline__ void split_walk(const float* const* rows, unsigned char* gbase, uint32_t full0, uint32_t empty0, int k_lo, int K, int nk, int nrows, int stages, int* err) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r0 = (warp & 3) + 4 * (lane >> 3), kk = (lane & 7) * 4, n4 = (nrows + 63) / 64;   // (64 rows at a time)
   const float* const* row = rows + r0;
-  float4 x[3][4];                                            // rows 0 - 63 and 64 - 127 of A, rows of W
+  float4 x[VEC ? 3 : 1][4];                                  // rows 0 - 63 and 64 - 127 of A, rows of W
   auto fetch = [&](int j, int k) {
     if (VEC && k >= K) return;
 #pragma unroll
     for (int i = 0; i < 4; i++) {
       const float* p = row[64 * j + 16 * i] + k;
-      if (VEC) x[j][i] = *reinterpret_cast<const float4*>(p);
-      else {
-        x[j][i].x = k < K ? p[0] : 0.f;
-        x[j][i].y = k + 1 < K ? p[1] : 0.f;
-        x[j][i].z = k + 2 < K ? p[2] : 0.f;
-        x[j][i].w = k + 3 < K ? p[3] : 0.f;
-      }
+      float4& v = x[VEC ? j : 0][i];
+      if (VEC) v = *reinterpret_cast<const float4*>(p);
+      else v = make_float4(k < K ? p[0] : 0.f, k + 1 < K ? p[1] : 0.f, k + 2 < K ? p[2] : 0.f, k + 3 < K ? p[3] : 0.f);
     }
   };
   int k = k_lo + (warp >> 2) * 32 + kk;
-  if ((warp >> 2) < 2 * nk) {
+  if (VEC && (warp >> 2) < 2 * nk) {
     fetch(0, k);
     if (n4 > 1) fetch(1, k);
     fetch(2, k);
   }
   for (int u = warp >> 2; u < 2 * nk; u += kSplitGroups) {
     const int kb = u >> 1, s = kb % stages, kn = k + kSplitGroups * 32;
-    const bool more = u + kSplitGroups < 2 * nk;
-    if (VEC && k >= K) {                                     // the end of the last slice
+    const bool more = VEC && u + kSplitGroups < 2 * nk;
+    if (VEC && k + 4 > K) {                                  // the end of the last slice
 #pragma unroll
       for (int j = 0; j < 3; j++)
 #pragma unroll
-        for (int i = 0; i < 4; i++) x[j][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int i = 0; i < 4; i++) {
+          float4& v = x[VEC ? j : 0][i];
+          v = make_float4(k < K ? v.x : 0.f, k + 1 < K ? v.y : 0.f, k + 2 < K ? v.z : 0.f, 0.f);
+        }
     }
     if (!__all_sync(0xffffffffu, tc_wait(empty0 + 8 * s, ((kb / stages) & 1) ^ 1, err))) break;
     unsigned char* dst = gbase + s * kSplitStage + r0 * 128 + ((((u & 1) * 4 + (kk >> 3)) ^ (r0 & 7)) << 4) + (kk & 4) * 2;
+    if (!VEC) fetch(0, k);
     split_rows(x[0], dst, kSplitPartA);
     if (more) fetch(0, kn);
     if (n4 > 1) {
-      split_rows(x[1], dst + 64 * 128, kSplitPartA);
+      if (!VEC) fetch(1, k);
+      split_rows(x[VEC ? 1 : 0], dst + 64 * 128, kSplitPartA);
       if (more) fetch(1, kn);
     }
-    split_rows(x[2], dst + 3 * kSplitPartA, kSplitPartW);
+    if (!VEC) fetch(2, k);
+    split_rows(x[VEC ? 2 : 0], dst + 3 * kSplitPartA, kSplitPartW);
     if (more) fetch(2, kn);
     k = kn;
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -125,15 +129,28 @@ __device__ __forceinline__ void split_walk(const float* const* rows, unsigned ch
   }
 }
 
-template <int EPI>
-__global__ void __launch_bounds__(kSplitThreads, 1) gemm_split(const GemmP P, int stages, int* err) {
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ float load_of_rank(uint32_t addr, int rank) {   // shared memory of a CTA of the cluster
+  uint32_t at;
+  float v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at) : "memory");
+  return v;
+}
+
+// SHARES: a cluster of S CTAs shares a tile's depth; each joins the sums of 128 / S rows, in the order of the shares (a form of its own: on one for both the splitting warps
+// spill, and products that take no shares ran 10 % longer).
+template <int EPI, bool SHARES>
+__global__ void __launch_bounds__(kSplitThreads, 1) gemm_split(const GemmP P, int stages, int S_, int* err) {
+  const int S = SHARES ? S_ : 1;
   constexpr bool DUAL = epi_dual(EPI);
   constexpr int BN = DUAL ? kSplitN / 2 : kSplitN;                                  // output columns (DUAL: rows 0 - 31 of a slice of W, 32 - 63 of W2)
   extern __shared__ unsigned char sp_raw[];
   __shared__ int rowsC[kTcRows];
   __shared__ const float* rows[kTcRows + kSplitN];           // of A and of W; those out of the product are another row of theirs, no result reads them
   __shared__ uint32_t tmem_slot;
-  const int n0 = blockIdx.x * BN;
+  const int share = SHARES ? (int)blockIdx.x % S : 0, n0 = (int)blockIdx.x / S * BN;
   if (P.band == BAND_COLS) {                                 // a tile that no query of its rows sees
     const int i0 = P.band_pos + (int)blockIdx.y * kTcRows, lo = max(0, mask_first(P.band_mask, P.band_window, i0) - P.band_first);
     if (n0 >= i0 + min(kTcRows, P.M - (int)blockIdx.y * kTcRows) - P.band_first || (n0 + BN <= lo && n0 >= P.band_keep)) { grid_enter(); return; }
@@ -178,7 +195,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split(const GemmP P, in
     rows[threadIdx.x] = (DUAL && r >= 32 ? W2 : W) + (size_t)n * P.ldw;
   }
   auto al = [](const float* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-  const bool vec = P.K % 4 == 0 && P.lda % 4 == 0 && P.ldw % 4 == 0 && al(A) && al(W) && (!DUAL || al(W2));   // rows take 16-byte loads
+  const bool vec = P.lda % 4 == 0 && P.ldw % 4 == 0 && al(A) && al(W) && (!DUAL || al(W2)) && P.sA % 4 == 0 && P.sW % 4 == 0 && P.ldw >= P.K && P.lda >= P.K;   // rows take 16-byte loads (K may end inside the last)
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -189,10 +206,12 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split(const GemmP P, in
     k_lo = P.band_keep ? 0 : lo / kSplitDepth * kSplitDepth;
     k_hi = min(P.K, i0 + nrows - P.band_first);
   }
-  const int nk = nrows > 0 ? (k_hi - k_lo + kSplitDepth - 1) / kSplitDepth : 0;
+  const int all = nrows > 0 ? (k_hi - k_lo + kSplitDepth - 1) / kSplitDepth : 0, per = (all + S - 1) / S;   // slices of the tile, of a share
+  const int nk = max(0, min(per, all - share * per)), k_from = k_lo + share * per * kSplitDepth;
   if (warp < kSplitWarps) {
-    if (vec) split_walk<true>(rows, gbase, full0, empty0, k_lo, P.K, nk, nrows, stages, err);
-    else split_walk<false>(rows, gbase, full0, empty0, k_lo, P.K, nk, nrows, stages, err);
+    if (vec) split_walk<true>(rows, gbase, full0, empty0, k_from, P.K, nk, nrows, stages, err);
+    else split_walk<false>(rows, gbase, full0, empty0, k_from, P.K, nk, nrows, stages, err);
+    if (SHARES) { cluster_arrive(); cluster_wait(); cluster_arrive(); cluster_wait(); }
   } else if (warp >= kSplitWarps + 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
     if (warp == kSplitWarps + 4 && tc_elect()) {
@@ -220,6 +239,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split(const GemmP P, in
       tc_wait(flushed0, 0, err);
     }
     __syncwarp();
+    if (SHARES) { cluster_arrive(); cluster_wait(); cluster_arrive(); cluster_wait(); }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 120;");    // (with the others' 4 x 80 and 32: 472 of the 480 that the CTA has)
     const int quad = warp & 3;                               // a warp reads the TMEM lanes of its place in a group of four
@@ -248,39 +268,62 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split(const GemmP P, in
       if (lane == 0) tc_arrive(drained0 + 8 * buf);
     }
     // results, turned so that a warp stores along rows (the ring is free: all products are through it)
-    if (ok && nrows > 0) {
-      float* turn = reinterpret_cast<float*>(gbase) + quad * 32 * 65;
+    float* turn = reinterpret_cast<float*>(gbase);           // [row][65]
+    auto again = [&](int row, int c) { return plain_dot(rows[row], rows[kTcRows + c], k_lo, k_hi, P.band == BAND_DEPTH); };
+    auto store = [&](int row, float v, float v2) {
+      const int cr = rowsC[row], n = n0 + lane;
+      if (cr < 0) return;
+      float* crow = P.C + coff + (size_t)cr * P.ldc;
+      if (n < P.N) gemm_epilogue<float, EPI>(P, crow, cr, n, v, v2);
+      if (!DUAL && n + 32 < P.N) gemm_epilogue<float, EPI>(P, crow, cr, n + 32, v2, 0.f);
+    };
+    if constexpr (!SHARES) {
+      const int row = quad * 32 + lane, count = min(32, nrows - quad * 32);
       float any = 0.f;                                       // (stays 0 as long as every sum is finite)
-      const int row = quad * 32 + lane;
 #pragma unroll
-      for (int c = 0; c < kSplitN; c++) { any = fmaf(0.f, acc[c], any); turn[lane * 65 + c] = acc[c]; }
+      for (int c = 0; c < kSplitN; c++) { any = fmaf(0.f, acc[c], any); turn[row * 65 + c] = acc[c]; }
       if (any != 0.f && row < nrows) {
-        const float* a = rows[row];
 #pragma unroll 1
-        for (int c = 0; c < kSplitN; c++) {
-          const int n = n0 + (DUAL ? c & 31 : c);
-          if (n < P.N && !isfinite(turn[lane * 65 + c])) turn[lane * 65 + c] = plain_dot(a, rows[kTcRows + c], k_lo, k_hi, P.band == BAND_DEPTH);
-        }
+        for (int c = 0; c < kSplitN; c++) if (!isfinite(turn[row * 65 + c])) turn[row * 65 + c] = again(row, c);
       }
       __syncwarp();
-      const int mine = min(32, nrows - quad * 32);
-      for (int i0 = 0; i0 < mine; i0 += 8) {                 // (eight rows' values ahead of their stores, which may not pass one another)
-        float v[8][2];
-        int cr[8];
+      if (ok)
+        for (int i0 = 0; i0 < count; i0 += 8) {              // (eight rows' values ahead of their stores, which may not pass one another)
+          float v[8][2];
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-          cr[i] = rowsC[quad * 32 + i0 + i];
-          v[i][0] = turn[(i0 + i) * 65 + lane];
-          v[i][1] = turn[(i0 + i) * 65 + 32 + lane];
-        }
+          for (int i = 0; i < 8; i++) { v[i][0] = turn[(quad * 32 + i0 + i) * 65 + lane]; v[i][1] = turn[(quad * 32 + i0 + i) * 65 + 32 + lane]; }
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-          if (cr[i] < 0) break;                              // (rows of a tile are its first ones)
-          float* crow = P.C + coff + (size_t)cr[i] * P.ldc;
-          if (n0 + lane < P.N) gemm_epilogue<float, EPI>(P, crow, cr[i], n0 + lane, v[i][0], v[i][1]);
-          if (!DUAL && n0 + 32 + lane < P.N) gemm_epilogue<float, EPI>(P, crow, cr[i], n0 + 32 + lane, v[i][1], 0.f);
+          for (int i = 0; i < 8; i++) store(quad * 32 + i0 + i, v[i][0], v[i][1]);
         }
-      }
+    } else {
+#pragma unroll
+      for (int c = 0; c < kSplitN; c++) turn[(quad * 32 + lane) * 65 + c] = acc[c];
+      cluster_arrive();
+      cluster_wait();
+      const int mine = kTcRows / S / 4, from = share * (kTcRows / S) + quad * mine;   // this warp's rows, two at a time
+      if (ok)
+#pragma unroll 1
+        for (int i = 0; i < min(mine, nrows - from); i += 2) {
+          float v[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+          const uint32_t at = base + (uint32_t)((from + i) * 65 + lane) * 4;
+#pragma unroll
+          for (int q = 0; q < 8; q++)
+            if (q < S) {
+#pragma unroll
+              for (int u = 0; u < 2; u++) { v[u][0] += load_of_rank(at + u * 260, q); v[u][1] += load_of_rank(at + u * 260 + 128, q); }
+            }
+          if (__any_sync(0xffffffffu, !isfinite(v[0][0] + v[0][1] + v[1][0] + v[1][1]))) {   // (a sum of finite ones may be infinite too: looked at one by one)
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+              if (!isfinite(v[u][0])) v[u][0] = again(from + i + u, lane);
+              if (!isfinite(v[u][1])) v[u][1] = again(from + i + u, 32 + lane);
+            }
+          }
+          store(from + i, v[0][0], v[0][1]);
+          store(from + i + 1, v[1][0], v[1][1]);
+        }
+      cluster_arrive();                                      // (no CTA leaves while another reads its sums)
+      cluster_wait();
     }
   }
   __syncthreads();

@@ -24,3 +24,12 @@ def test_routed_edges(mk, no, experts, top, ff, sizes):  # noqa: F811
     m, W = mk(cfg, seed=experts, chunk=256)
     toks = tokens_for(cfg, sum(sizes), 4)
     assert rel(in_portions(m, toks, sizes), no.run(cfg, W, toks)[0]) < F32_TOL
+
+
+# tiles whose depth two, four or eight CTAs share: ragged last slices, shares without a slice (17 slices over 8 CTAs: the last one has two, 9 over 8: three have none), narrow router products
+@pytest.mark.parametrize("width,ff,tokens", [(520, 40, 40), (1100, 36, 70), (2060, 24, 5), (2048, 16, 460), (600, 700, 130)])
+def test_shared_depth(mk, no, width, ff, tokens):  # noqa: F811
+    cfg = no.model_config([no.att(heads=2, dim=16, vdim=16, mlp=no.moe(experts=6, top=2, ff=ff, shared=ff))], width=width, vocab=67)
+    m, W = mk(cfg, seed=width, chunk=512)
+    toks = tokens_for(cfg, tokens, 4)
+    assert rel(m.forward_chunk(toks, 0, range(tokens)), no.run(cfg, W, toks)[0]) < F32_TOL
