@@ -35,6 +35,7 @@
 #include "dsk_linattn.cuh"
 #include "dsk_tc5.cuh"
 #include "dsk_pattn.cuh"
+#include "dsk_pattn5.cuh"
 #include "dsk_split.cuh"
 
 using namespace dsk;

@@ -366,7 +366,7 @@ static int validate(const dsk_hybrid_config& c, const dsk_layer_spec* L) {
 }
 
 // attention of portions in one kernel: sizes and the layers that take it (no mixing of the heads' scores, a tile of keys that fits)
-static constexpr int kPattnSmemMax = 220 * 1024;
+static constexpr int kPattnSmemMax = 220 * 1024, kPattn5SmemMax = 226 * 1024;
 struct PattnSize { int parts, G, D, V, Dp, Vp, VN; };
 static PattnSize pattn_size(const dsk_layer_spec& s, bool bf16) {
   PattnSize z;
@@ -417,6 +417,9 @@ static void set_kernel_attrs() {
   cudaFuncSetAttribute(pattn<A, B, 4, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax); cudaFuncSetAttribute(pattn<A, B, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattnSmemMax)
   DSK_PATTN_ATTR(1, 8); DSK_PATTN_ATTR(1, 16); DSK_PATTN_ATTR(3, 8); DSK_PATTN_ATTR(3, 16);
 #undef DSK_PATTN_ATTR
+#define DSK_PATTN5_ATTR(A, B) cudaFuncSetAttribute(pattn5<A, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPattn5SmemMax)
+  DSK_PATTN5_ATTR(1, 1); DSK_PATTN5_ATTR(1, 2); DSK_PATTN5_ATTR(3, 1); DSK_PATTN5_ATTR(3, 2);
+#undef DSK_PATTN5_ATTR
 #define DSK_SPLIT_ATTR(E) cudaFuncSetAttribute(gemm_split<E, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, split_smem(kSplitStages)); \
   cudaFuncSetAttribute(gemm_split<E, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, split_smem(kSplitStages))
   DSK_SPLIT_ATTR(HEPI_STORE); DSK_SPLIT_ATTR(HEPI_ADD); DSK_SPLIT_ATTR(HEPI_GLU); DSK_SPLIT_ATTR(HEPI_XIELU); DSK_SPLIT_ATTR(HEPI_GEGLU); DSK_SPLIT_ATTR(HEPI_SIGMUL);
@@ -1891,12 +1894,36 @@ static void launch_latent_attn(State* S, const float* qa, const float* cache, fl
   launch_decode_attn(S, P, true, st);
 }
 
-// Attention of Tq queries in one kernel: K (keys, values and the visible range given) is split into bf16 parts, then A runs over it.
-static void portion_attn(State* S, const PattnSize& z, PackP K, PattnP A, cudaStream_t st) {
-  K.V = z.V; K.Dp = z.Dp; K.Vp = z.Vp; K.G = z.G; K.kb = S->k16; K.vb = S->v16;
-  A.kb = S->k16; A.vb = S->v16; A.G = z.G; A.D = z.D; A.Dp = z.Dp; A.V = z.V; A.Vp = z.Vp; A.Lk = K.Lk; A.nk = K.nk; A.first = K.first; A.mods.keep = K.keep;
-  if (z.parts == 1) launch_next(pattn_pack<1>, K.Lk, 256, 0, st)(K);
-  else launch_next(pattn_pack<3>, K.Lk, 256, 0, st)(K);
+// rows x cols bf16 matrices, `count` of them behind one another, copied in boxes of 32 rows x 64 columns (rows past a matrix read as zeros)
+static bool box_map(CUtensorMap* m, const void* p, long long cols, long long rows, long long count) {
+  const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)count}, strides[2] = {(cuuint64_t)cols * 2, (cuuint64_t)rows * cols * 2};
+  const cuuint32_t box[3] = {64, (cuuint32_t)kP5Keys, 1}, one[3] = {1, 1, 1};
+  return encode_tiled()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(p), dims, strides, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// Heads that pattn5 takes: queries and two pieces of keys in shared memory, whole 64-entry rows (smaller heads would be half padding), scores' accumulators in TMEM
+static bool pattn5_takes(const PattnSize& z) {
+  const int nch = (z.Dp + 63) / 64;
+  return encode_tiled() && z.Dp >= 64 && nch <= kP5MaxChunks && p5_smem(z.parts, nch, z.VN / 8, 2, 1) <= kPattn5SmemMax;
+}
+static void launch_pattn5(State* S, const PattnSize& z, PattnP& A, cudaStream_t st) {
+  const int nch = (z.Dp + 63) / 64, vb = z.VN / 8, vst = p5_smem(z.parts, nch, vb, 4, 2) <= kPattn5SmemMax ? 2 : 1;
+  int kst = 2;
+  while (kst < std::min(kP5MaxK, 3 * nch) && p5_smem(z.parts, nch, vb, kst + 1, vst) <= kPattn5SmemMax) kst++;
+  const int smem = p5_smem(z.parts, nch, vb, kst, vst), qb = (A.T + kP5Rows - 1) / kP5Rows, zc = z.Vp / (vb * 64);
+  // shares of the keys where the query blocks leave SMs idle, of at least four tiles (joining them takes about as long as three)
+  const long long ctas = (long long)qb * A.H * zc, tiles = (std::min<long long>(A.Lk, (long long)A.span + kP5Rows) + kP5Keys - 1) / kP5Keys;
+  const long long most = std::min({148 / ctas, tiles / 4, (long long)kAttnSplitMax});
+  A.NS = most > 1 && (tiles + most - 1) / most + 3 < tiles ? (int)most : 1;
+  A.part = S->ppart;
+  CUtensorMap mK, mV;
+  if (!box_map(&mK, A.kb, z.Dp, A.Lk, (long long)z.parts * z.G) || !box_map(&mV, A.vb, z.Vp, A.Lk, (long long)z.parts * z.G)) { *S->h_err = 2; return; }
+  const dim3 grid((unsigned)A.H, (unsigned)qb, (unsigned)(zc * A.NS));
+  auto* kernel = z.parts == 1 ? (vb == 1 ? pattn5<1, 1> : pattn5<1, 2>) : vb == 1 ? pattn5<3, 1> : pattn5<3, 2>;
+  launch_next(kernel, grid, kP5Threads, smem, st)(A, mK, mV, kst, vst, S->h_err);
+}
+
+static void launch_pattn(State* S, const PattnSize& z, const PackP& K, PattnP& A, cudaStream_t st) {
   // 16 query rows per warp, a CTA an SM, tiles of 16 keys where 32 do not fit.  Four warps are one on each of an SM's tensor cores; with eight a tile of keys takes about 1.2 times
   // as long (two a core hide one another's waits, and more threads copy the tile), with two 1.4 times.  Where the query blocks leave SMs idle, the keys are cut into shares of
   // at least four tiles, one CTA each, and latent_swa_merge joins them.  What costs least, rounds of CTAs x time of a tile x tiles, is taken.  Two layers of width 2048, 16 heads of 128, behind
@@ -1926,6 +1953,16 @@ static void portion_attn(State* S, const PattnSize& z, PackP K, PattnP A, cudaSt
   else if (z.VN == 8) DSK_PATTN(3, 8);
   else DSK_PATTN(3, 16);
 #undef DSK_PATTN
+}
+
+// Attention of Tq queries in one kernel: K (keys, values and the visible range given) is split into bf16 parts, then A runs over it.
+static void portion_attn(State* S, const PattnSize& z, PackP K, PattnP A, cudaStream_t st) {
+  K.V = z.V; K.Dp = z.Dp; K.Vp = z.Vp; K.G = z.G; K.kb = S->k16; K.vb = S->v16;
+  A.kb = S->k16; A.vb = S->v16; A.G = z.G; A.D = z.D; A.Dp = z.Dp; A.V = z.V; A.Vp = z.Vp; A.Lk = K.Lk; A.nk = K.nk; A.first = K.first; A.mods.keep = K.keep;
+  if (z.parts == 1) launch_next(pattn_pack<1>, K.Lk, 256, 0, st)(K);
+  else launch_next(pattn_pack<3>, K.Lk, 256, 0, st)(K);
+  if (pattn5_takes(z)) launch_pattn5(S, z, A, st);
+  else launch_pattn(S, z, K, A, st);
   if (A.NS > 1) {
     launch_next(latent_swa_merge, dim3((unsigned)(A.T * A.H), (unsigned)((A.V + 127) / 128)), 128, 0, st)(S->ppart, A.out, A.V, A.NS, A.gate, A.ld_gate, A.H, A.gate_head, A.ld_out, A.alpha);
     S->launches++;

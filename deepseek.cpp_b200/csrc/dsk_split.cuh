@@ -65,13 +65,6 @@ __device__ __forceinline__ void split_rows(const float4 (&x)[4], unsigned char* 
     }
   }
 }
-__device__ __forceinline__ void tc_load16(uint32_t addr, uint32_t (&r)[16]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]),
-                 "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-               : "r"(addr));
-}
-
 // A splitting warp's way through the half slices of its group: group g has half slices g, g + 4, ..  Eight lanes have the 32 values of a row, a load four rows: w + 4 q of every
 // 16 (rows 4 apart are on different banks behind the swizzle, whose phase is one for all rows of a lane).  The numbers of a group's next half slice are asked for as soon as
 // the registers of this one's are free: 48 KB a slice cross from L2 at some 64 bytes a clock, which is as long as the products of a slice take.

@@ -82,3 +82,22 @@ def test_shares_with_kept_positions(mk_sakusun, so):  # noqa: F811
     exp = so.run(cfg, W, toks)[0]
     for sizes in ([256, 256, 256, 132], [250, 250, 40, 33, 256]):
         assert rel(in_portions(m, toks, sizes), exp) < F32_TOL
+
+
+# heads of 64 entries and more: blocks of 128 queries, tiles of 32 keys, depth in pieces of 64 (65 and 100 end inside one), columns of values in blocks of 64 and 128 (150: two CTAs),
+# windows that begin inside a tile, more tiles than a turn of the ring, and shares of the keys (one block of queries behind many keys)
+@pytest.mark.parametrize("heads,kv_heads,dim,vdim,size,sizes", [(2, 1, 64, 64, 50, [127, 33]), (3, 3, 65, 70, None, [128, 129]), (4, 2, 128, 128, 200, [300]), (2, 2, 100, 150, 33, [257]),
+                                                               (2, 1, 192, 128, None, [130, 126]), (1, 1, 180, 20, 150, [600, 40]), (1, 1, 64, 128, None, [900, 35, 33])])
+def test_blocks_of_128_queries(mk, no, heads, kv_heads, dim, vdim, size, sizes):  # noqa: F811
+    cfg = no.model_config([no.att(heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, size=size)] * 2, width=48, vocab=97)
+    m, W = mk(cfg, seed=dim, chunk=1024, context=1100)
+    toks = tokens_for(cfg, sum(sizes), 5)
+    assert rel(in_portions(m, toks, sizes), no.run(cfg, W, toks)[0]) < F32_TOL
+
+
+@pytest.mark.parametrize("dim,rot_dim,vdim,tokens", [(64, 64, 64, 150), (128, 64, 128, 260), (72, 8, 129, 140)])
+def test_blocks_of_128_queries_with_a_rotated_part(mk, no, dim, rot_dim, vdim, tokens):  # noqa: F811
+    cfg = no.model_config([no.lat(heads=2, dim=dim, rot_dim=rot_dim, vdim=vdim)], width=40, vocab=97)
+    m, W = mk(cfg, seed=dim, chunk=512, context=600)
+    toks = tokens_for(cfg, tokens, 6)
+    assert rel(m.forward_chunk(toks, 0, range(tokens)), no.run(cfg, W, toks)[0]) < F32_TOL
