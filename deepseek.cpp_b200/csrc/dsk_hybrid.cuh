@@ -199,13 +199,13 @@ __global__ void __launch_bounds__(128) canon_conv(const float* __restrict__ x, i
 // RMS norm in groups, grid (rows, groups).  Row t of `in` (n values) is cut into `groups` equal consecutive parts; each part is divided by
 // sqrt(mean(part^2) + eps) and the row is multiplied by w.  mode 0: out[row] = result, where row = (ctl ? ctl[0] : 0) + t,
 // taken modulo `ring` (a ring cache of latents; ring = 0 means rows are not wrapped).  mode 1: out[t] += alpha * result.
-// gate (nullable, row pitch ld_gate): the result is multiplied by it entry by entry.
+// gate (nullable, row pitch ld_gate): the result is multiplied by it entry by entry.  o16 (nullable, mode 0): the result goes there instead, as packed bf16 rows.
 // ---------------------------------------------------------------------------------------------------------------------
 template <typename OT>
 __global__ void __launch_bounds__(256) group_rmsnorm(const float* __restrict__ in, int ld_in, const float* __restrict__ w,
                                                      OT* __restrict__ out, int ld_out, int n, int groups, float eps, int mode,
                                                      float alpha, const int* __restrict__ ctl, int ring,
-                                                     const float* __restrict__ gate = nullptr, int ld_gate = 0) {
+                                                     const float* __restrict__ gate = nullptr, int ld_gate = 0, __nv_bfloat16* __restrict__ o16 = nullptr) {
   grid_enter();
   __shared__ float red[33];
   const int t = blockIdx.x;
@@ -228,7 +228,10 @@ __global__ void __launch_bounds__(256) group_rmsnorm(const float* __restrict__ i
 #pragma unroll
     for (int k = 0; k < 16; k++) {
       const int i = threadIdx.x + 256 * k;
-      if (i < n) o[i] = from_f<OT>(mode == 0 ? v[k] * sc * gt[k] : to_f<OT>(o[i]) + alpha * (v[k] * sc * gt[k]));
+      if (i < n) {
+        if (o16) o16[(size_t)t * n + i] = __float2bfloat16_rn(v[k] * sc * gt[k]);
+        else o[i] = from_f<OT>(mode == 0 ? v[k] * sc * gt[k] : to_f<OT>(o[i]) + alpha * (v[k] * sc * gt[k]));
+      }
     }
     return;
   }
@@ -256,7 +259,8 @@ __global__ void __launch_bounds__(256) group_rmsnorm(const float* __restrict__ i
   auto put = [&](int i, float xv, float wv, float ov) {
     float r = xv * sc * wv;
     if (gate) r *= gate[(size_t)t * ld_gate + c0 + i];
-    o[c0 + i] = from_f<OT>(mode == 0 ? r : ov + alpha * r);
+    if (o16) o16[(size_t)t * n + c0 + i] = __float2bfloat16_rn(r);
+    else o[c0 + i] = from_f<OT>(mode == 0 ? r : ov + alpha * r);
   };
   if (cached) {
 #pragma unroll
@@ -271,7 +275,7 @@ __global__ void __launch_bounds__(256) group_rmsnorm(const float* __restrict__ i
 // of group_rmsnorm's 256 hold and adds it up in their order, so that both give the same bits.  (A CTA a group, two values a thread and three barriers: 2048 rows of
 // four groups of 512 took 25.7 us.)
 __global__ void __launch_bounds__(256) group_rmsnorm_rows(const float* __restrict__ in, int ld_in, const float* __restrict__ w, float* __restrict__ out, int ld_out,
-                                                          int rows, int n, int groups, float eps) {
+                                                          int rows, int n, int groups, float eps, __nv_bfloat16* __restrict__ o16) {
   grid_enter();
   const int lane = threadIdx.x & 31, gs = n / groups;
   const long long id = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -279,9 +283,9 @@ __global__ void __launch_bounds__(256) group_rmsnorm_rows(const float* __restric
   const int t = (int)(id / groups), c0 = (int)(id - (long long)t * groups) * gs;
   const float* x = in + (size_t)t * ld_in + c0;
   float* o = out + (size_t)t * ld_out + c0;
-  float v[32], s[8];
+  float v[32], wv[32], s[8];
 #pragma unroll
-  for (int k = 0; k < 32; k++) v[k] = lane + 32 * k < gs ? x[lane + 32 * k] : 0.f;
+  for (int k = 0; k < 32; k++) { v[k] = lane + 32 * k < gs ? x[lane + 32 * k] : 0.f; wv[k] = lane + 32 * k < gs ? w[c0 + lane + 32 * k] : 0.f; }
 #pragma unroll
   for (int j = 0; j < 8; j++) {   // warp j's thread of this lane
     s[j] = 0.f;
@@ -296,8 +300,24 @@ __global__ void __launch_bounds__(256) group_rmsnorm_rows(const float* __restric
   const float sc = 1.f / sqrtf(ss / (float)gs + eps);
 #pragma unroll
   for (int k = 0; k < 32; k++) {
-    const int i = lane + 32 * k;
-    if (i < gs) o[i] = v[k] * sc * w[c0 + i];
+    v[k] = v[k] * sc * wv[k];
+    if (out && lane + 32 * k < gs) o[lane + 32 * k] = v[k];
+  }
+  if (!o16) return;
+  // packed bf16 rows, beside the others or instead of them (out may be null): lanes trade a value, so that even ones have a pair of columns of round k and odd ones of round k + 1
+  __nv_bfloat16* ob = o16 + (size_t)t * n + c0;
+  const int odd = lane & 1;
+  const bool pairs = ((n | c0) & 1) == 0;
+#pragma unroll
+  for (int k = 0; k < 32; k += 2) {
+    const float other = __shfl_xor_sync(0xffffffffu, odd ? v[k] : v[k + 1], 1);
+    const int i = (lane & ~1) + 32 * (k + odd);
+    const __nv_bfloat162 p = odd ? __floats2bfloat162_rn(other, v[k + 1]) : __floats2bfloat162_rn(v[k], other);
+    if (pairs && i + 1 < gs) *reinterpret_cast<__nv_bfloat162*>(ob + i) = p;
+    else {
+      if (i < gs) ob[i] = p.x;
+      if (i + 1 < gs) ob[i + 1] = p.y;
+    }
   }
 }
 
@@ -1182,17 +1202,25 @@ __global__ void __launch_bounds__(512) ssd_scan(const float* __restrict__ proj, 
 // after its own read; longer steps run shift_carry afterwards, because their first CTA reads what the last one would write.
 // ---------------------------------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(128) token_shift(const float* __restrict__ x, int ld, const float* __restrict__ mu, float* __restrict__ carry,
-                                                   float* __restrict__ h, int ldh, int T, int ch, const int* __restrict__ ctl) {
+                                                   float* __restrict__ h, int ldh, int T, int ch, const int* __restrict__ ctl, __nv_bfloat16* __restrict__ h16) {
   grid_enter();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ch) return;
   const int t0 = blockIdx.y * kCanonTokens, t1 = min(T, t0 + kCanonTokens);
   float prev = t0 > 0 ? x[(size_t)(t0 - 1) * ld + c] : (ctl[0] > 0 ? carry[c] : 0.f);
   const float m = mu[c];
-  for (int t = t0; t < t1; t++) {
-    const float cur = x[(size_t)t * ld + c];
-    h[(size_t)t * ldh + c] = fmaf(prev - cur, m, cur);
-    prev = cur;
+  for (int tb = t0; tb < t1; tb += 8) {   // eight rows' loads ahead of their stores
+    float cur[8];
+#pragma unroll
+    for (int u = 0; u < 8; u++) cur[u] = tb + u < t1 ? x[(size_t)(tb + u) * ld + c] : 0.f;
+#pragma unroll
+    for (int u = 0; u < 8; u++)
+      if (tb + u < t1) {
+        const float r = fmaf(prev - cur[u], m, cur[u]);
+        h[(size_t)(tb + u) * ldh + c] = r;
+        if (h16) h16[(size_t)(tb + u) * ch + c] = __float2bfloat16_rn(r);
+        prev = cur[u];
+      }
   }
   if (gridDim.y == 1) carry[c] = prev;
 }
@@ -1696,7 +1724,7 @@ __device__ __forceinline__ void ln_stats(const float (&v)[kLnRegs], const float*
 
 __global__ void __launch_bounds__(256) layer_norm(const float* __restrict__ in, int ld_in, const float* __restrict__ w, const float* __restrict__ b,
                                                   float* __restrict__ out, int ld_out, int n, float eps, int mode, float alpha,
-                                                  const float* __restrict__ wgt, int top) {
+                                                  const float* __restrict__ wgt, int top, __nv_bfloat16* __restrict__ o16) {
   grid_enter();
   __shared__ float red[33];
   const int t = blockIdx.x;
@@ -1725,10 +1753,20 @@ __global__ void __launch_bounds__(256) layer_norm(const float* __restrict__ in, 
 #pragma unroll
     for (int k = 0; k < kLnRegs; k++) {
       const int i = threadIdx.x + 256 * k;
-      if (i < n) { const float r = (v[k] - mean) * sc * w[i] + (b ? b[i] : 0.f); o[i] = mode == 0 ? r : o[i] + alpha * r; }
+      if (i < n) {
+        float r = (v[k] - mean) * sc * w[i] + (b ? b[i] : 0.f);
+        if (mode != 0) r = o[i] + alpha * r;
+        o[i] = r;
+        if (o16) o16[(size_t)t * n + i] = __float2bfloat16_rn(r);
+      }
     }
   } else {
-    for (int i = threadIdx.x; i < n; i += 256) { const float r = (x[i] - mean) * sc * w[i] + (b ? b[i] : 0.f); o[i] = mode == 0 ? r : o[i] + alpha * r; }
+    for (int i = threadIdx.x; i < n; i += 256) {
+      float r = (x[i] - mean) * sc * w[i] + (b ? b[i] : 0.f);
+      if (mode != 0) r = o[i] + alpha * r;
+      o[i] = r;
+      if (o16) o16[(size_t)t * n + i] = __float2bfloat16_rn(r);
+    }
   }
 }
 
@@ -1736,7 +1774,7 @@ __global__ void __launch_bounds__(256) layer_norm(const float* __restrict__ in, 
 //   x += alpha * ln(y) * wy  (+ row, the vector of a loop pass that opens next);   h = ln(x) * wh
 __global__ void __launch_bounds__(256) layer_norm_add_norm(const float* __restrict__ y, const float* __restrict__ wy, float* __restrict__ x,
                                                            const float* __restrict__ row, const float* __restrict__ wh,
-                                                           float* __restrict__ h, int n, float eps, float alpha) {
+                                                           float* __restrict__ h, int n, float eps, float alpha, __nv_bfloat16* __restrict__ h16) {
   grid_enter();
   __shared__ float red[33];
   const size_t t = blockIdx.x;
@@ -1760,14 +1798,18 @@ __global__ void __launch_bounds__(256) layer_norm_add_norm(const float* __restri
 #pragma unroll
   for (int k = 0; k < kLnRegs; k++) {
     const int i = threadIdx.x + 256 * k;
-    if (i < n) h[t * n + i] = (v[k] - mean) * sc * wh[i];
+    if (i < n) {
+      const float r = (v[k] - mean) * sc * wh[i];
+      h[t * n + i] = r;
+      if (h16) h16[t * n + i] = __float2bfloat16_rn(r);
+    }
   }
 }
 
 // Opening of a pre-norm sublayer:  x += e + row (both nullable: the embedding and the vector of a loop pass that starts here);
 // h = x / sqrt(mean(x^2) + eps) * w.  The row stays in registers up to 256 * kLnRegs values.
 __global__ void __launch_bounds__(256) rms_open(float* __restrict__ x, const float* __restrict__ e, const float* __restrict__ row,
-                                                const float* __restrict__ w, float* __restrict__ h, int n, float eps) {
+                                                const float* __restrict__ w, float* __restrict__ h, int n, float eps, __nv_bfloat16* __restrict__ h16) {
   __shared__ float red[33];
   float wt[kLnRegs];   // (the model's: under the kernel ahead, not behind the sum)
 #pragma unroll
@@ -1795,8 +1837,8 @@ __global__ void __launch_bounds__(256) rms_open(float* __restrict__ x, const flo
   }
   const float sc = 1.f / sqrtf(block_sum(ss, red) / (float)n + eps);
 #pragma unroll
-  for (int k = 0; k < kLnRegs; k++) { const int i = threadIdx.x + 256 * k; if (i < n) hr[i] = v[k] * sc * wt[k]; }
-  for (int i = threadIdx.x + 256 * kLnRegs; i < n; i += 256) hr[i] = xr[i] * sc * w[i];
+  for (int k = 0; k < kLnRegs; k++) { const int i = threadIdx.x + 256 * k; if (i < n) { hr[i] = v[k] * sc * wt[k]; if (h16) h16[(size_t)blockIdx.x * n + i] = __float2bfloat16_rn(v[k] * sc * wt[k]); } }
+  for (int i = threadIdx.x + 256 * kLnRegs; i < n; i += 256) { hr[i] = xr[i] * sc * w[i]; if (h16) h16[(size_t)blockIdx.x * n + i] = __float2bfloat16_rn(xr[i] * sc * w[i]); }
 }
 
 // Sandwich blocks of RMS norms (rows of up to 256 * kLnRegs values): the end of one sublayer and the start of the next in one pass,
@@ -1809,7 +1851,7 @@ template <int NT, int KR>
 __global__ void __launch_bounds__(NT) rms_add_norm(const float* __restrict__ y, const float* __restrict__ wgt, int top, const float* __restrict__ ysh,
                                                     const float* __restrict__ wsh, const float* __restrict__ wy, const float* x, float* xo, int ldxo,
                                                     const float* __restrict__ wh, float* __restrict__ h, int n,
-                                                    float eps, float alpha) {
+                                                    float eps, float alpha, __nv_bfloat16* __restrict__ h16) {
   __shared__ float red[33];
   // a decoded token's row: the model's weights under the kernel ahead, not each behind its sum
   constexpr bool EARLY = NT == 1024;
@@ -1860,7 +1902,7 @@ __global__ void __launch_bounds__(NT) rms_add_norm(const float* __restrict__ y, 
   if (!wh) return;
   sc = 1.f / sqrtf(block_sum(ss, red) / (float)n + eps);
 #pragma unroll
-  for (int k = 0; k < KR; k++) { const int i = threadIdx.x + NT * k; if (i < n) h[t * n + i] = u[k] * sc * (EARLY ? b_w[EARLY ? k : 0] : wh[i]); }
+  for (int k = 0; k < KR; k++) { const int i = threadIdx.x + NT * k; if (i < n) { const float r = u[k] * sc * (EARLY ? b_w[EARLY ? k : 0] : wh[i]); h[t * n + i] = r; if (h16) h16[t * n + i] = __float2bfloat16_rn(r); } }
 }
 
 // the T rows of a step (pitch ls) copied to rows of pitch ld
@@ -1876,7 +1918,7 @@ __global__ void copy_rows(const float* __restrict__ src, int ls, float* __restri
 __global__ void __launch_bounds__(256) head_rmsnorm(const float* __restrict__ in, int ld_in, const float* __restrict__ w, float* __restrict__ out,
                                                     int ld_out, int T, int H, int P, float eps, const float* __restrict__ gate = nullptr,
                                                     int ld_gate = 0, float alpha = 1.f, int w_stride = 0, int gate_sig = 0,
-                                                    const float* __restrict__ den = nullptr, const float* __restrict__ mrow = nullptr) {
+                                                    const float* __restrict__ den = nullptr, const float* __restrict__ mrow = nullptr, __nv_bfloat16* __restrict__ o16 = nullptr) {
   grid_enter();
   const int lane = threadIdx.x & 31;
   const long long id = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -1891,9 +1933,17 @@ __global__ void __launch_bounds__(256) head_rmsnorm(const float* __restrict__ in
   const float sc = pre / sqrtf(warp_sum(ss) / (float)P + eps);
   if (gate) {
     const float* g = gate + (size_t)t * ld_gate + (size_t)h * P;
-    for (int i = lane; i < P; i += 32) o[i] = x[i] * sc * w[i] * (alpha * (gate_sig ? sigmoid_f(g[i]) : silu_f(g[i])));
+    for (int i = lane; i < P; i += 32) {
+      const float r = x[i] * sc * w[i] * (alpha * (gate_sig ? sigmoid_f(g[i]) : silu_f(g[i])));
+      if (o16) o16[((size_t)t * H + h) * P + i] = __float2bfloat16_rn(r);   // (packed bf16 rows instead)
+      else o[i] = r;
+    }
   } else
-    for (int i = lane; i < P; i += 32) o[i] = x[i] * sc * w[i];
+    for (int i = lane; i < P; i += 32) {
+      const float r = x[i] * sc * w[i];
+      if (o16) o16[((size_t)t * H + h) * P + i] = __float2bfloat16_rn(r);
+      else o[i] = r;
+    }
 }
 
 // x[t][:] += row[:] for the T rows of a step (the per-pass vector of a layer loop)

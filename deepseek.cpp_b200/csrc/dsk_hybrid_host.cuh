@@ -133,7 +133,7 @@ struct LayerState {
 
 struct State {
   std::vector<LayerState> L;
-  int chunk = 0;
+  int chunk = 0, width = 0;
   int next_pos = 0;
   int *d_tok = nullptr, *d_want = nullptr, *d_ctl = nullptr, *d_idx = nullptr, *d_perm = nullptr, *d_ntiles = nullptr;
   int4* d_tiles = nullptr;
@@ -168,6 +168,9 @@ struct State {
   // bf16 products of portions: activations rounded for the product that follows, hidden rows of a feed-forward, and a host word that a wait
   // which gave up sets
   __nv_bfloat16 *a16 = nullptr, *hid16 = nullptr;
+  // rows of the width that products read, rounded by the kernel that made them (h, hs or x: `mirror`, until something else writes it)
+  __nv_bfloat16* h16 = nullptr;
+  const float* mirror = nullptr;
   size_t a16_elems = 0, hid16_elems = 0;
   int* h_err = nullptr;
   // device memory of the state: one allocation, cut into the pieces that salloc was asked for (portion: one that only the attention of portions needs; seq: caches and carried
@@ -1198,6 +1201,7 @@ static dsk_state* state_create(dsk_model* m) {
   s->m = m;
   s->hy = S;
   S->chunk = c.chunk;
+  S->width = c.dim;
   S->timeline = getenv("DSK_HY_TIMELINE") != nullptr;
   const size_t Tc = c.chunk;
   // the pieces the shared sampling / arg-max code reads
@@ -1400,7 +1404,7 @@ static dsk_state* state_create(dsk_model* m) {
     for (const HLayer& L : M->L) rank = std::max<size_t>(rank, has_attn(L.sp) && L.sp.mixer != DSK_MIX_GQA ? L.sp.att_kv_rank : 0);
     S->a16_elems = std::max(Tc * std::max({mx0, mx1, mx2, mx3, (size_t)2 * c.dim, mxRouted}), (size_t)S->prefill_keys * rank);
     S->hid16_elems = Tc * mxHid;
-    rc |= salloc(S, (void**)&S->a16, S->a16_elems * 2) | salloc(S, (void**)&S->hid16, S->hid16_elems * 2);
+    rc |= salloc(S, (void**)&S->a16, S->a16_elems * 2) | salloc(S, (void**)&S->hid16, S->hid16_elems * 2) | salloc(S, (void**)&S->h16, Tc * c.dim * 2);
   }
   rc |= salloc(S, (void**)&S->logits, (size_t)S->head_rows * c.vocab_size * 4);
   if (rc || salloc_all(S, s->stream)) { fail(-2, "state allocation failed"); return nullptr; }
@@ -1542,6 +1546,14 @@ static bool tc_ok(const State* S, bool bf16, int epi, const GemmP& P, int Z) {
 }
 static void launch_tc5(State* S, int epi, const GemmP& P, int tile_cap, cudaStream_t st) {
   const __nv_bfloat16* A16 = P.A16;
+  if (!A16 && P.A == S->mirror && P.lda == S->width && P.K == S->width) {
+    A16 = S->h16;
+    if (P.a_map) {
+      launch_next(gather_rows16, (unsigned)std::min<long long>(((long long)P.M * (P.K / 8) + 255) / 256, 148 * 8), 256, 0, st)(S->h16, P.a_map, P.a_div, S->a16, P.M, P.K);
+      S->launches++;
+      A16 = S->a16;
+    }
+  }
   if (!A16) {
     const int vec = P.lda % 4 == 0 && (reinterpret_cast<uintptr_t>(P.A) & 15) == 0;
     const long long n = (long long)P.M * (P.K / 8);
@@ -1670,6 +1682,7 @@ static void launch_narrow(bool bf16, int epi, const GemmP& P, cudaStream_t st) {
 }
 // C = A W^T (+ epilogue).  Z > 1: per-head batches or (gemv) one batch per routed (token, slot) pair.
 static void linear(State* S, bool bf16, int epi, const GemmP& P, int Z, cudaStream_t st, int tile_cap = 0) {
+  struct Over { State* S; const float* C; ~Over() { if (C == S->mirror) S->mirror = nullptr; } } over{S, P.C};   // (its operand may be the mirror until then)
   const bool small = P.z_expert != nullptr || (!P.tiles && P.M <= 4);
   if (!small && !P.tiles && Z == 1 && P.N <= 96) {   // narrow output (router, token-input gate): warp-per-row products over batches of 4 rows
     // (a CTA of gemm_narrow has 16 rows: under 448 they are too few.  Steps of 256 / 384 / 512 / 1024 tokens, two layers with 64 experts and a token input of
@@ -1795,7 +1808,7 @@ static void launch_lin_decode(int mode, const GdnP& D, const float* decay, float
 }
 
 // gated delta rule of T tokens from the raw projections in S->b0 (columns of att_layout) -> out rows (pitch ldo), times alpha
-static void gdn_forward(State* S, const HLayer& L, LayerState& ls, int ldp, const AttLayout& a, float* out, int ldo, float alpha, float eps, int T, cudaStream_t st) {
+static void gdn_forward(State* S, const HLayer& L, LayerState& ls, int ldp, const AttLayout& a, float* out, int ldo, float alpha, float eps, int T, cudaStream_t st, __nv_bfloat16* out16 = nullptr) {
   const dsk_layer_spec& sp = L.sp;
   const int H = sp.gdn_heads, G = sp.gdn_kv_heads, N = sp.gdn_dim, P = sp.gdn_vdim, RV = H * P, NP = (N + 3) & ~3, CH = 2 * G * N + RV;
   const GdnP D{S->b0, ldp, (int)a.dq, (int)a.db, (int)a.da, L.gdn_conv_w, L.A_log, L.dt_bias, ls.hist, sp.gdn_conv - 1 + kConvSpare, sp.gdn_conv, T, H, G, N, P, S->d_ctl};
@@ -1809,7 +1822,7 @@ static void gdn_forward(State* S, const HLayer& L, LayerState& ls, int ldp, cons
   launch_next(gdn_prepare, dim3((unsigned)nb, (unsigned)(G + (RV + 255) / 256)), 256, smem, st)(D, S->lq, S->lk, S->lv, NP, S->lrec);
   launch_lin_scan(true, S->lq, S->lk, G * NP, NP, H / G, S->lv, RV, S->lrec, ls.lin, S->lout, RV, T, H, N, P, st);
   if (sp.gdn_conv > 1) { launch_next(conv_ring_store, (CH + 127) / 128, 128, 0, st)(S->b0, ldp, (int)a.dq, ls.hist, D.ring, T, CH, sp.gdn_conv, S->d_ctl); S->launches++; }
-  launch_next(head_rmsnorm, (unsigned)(((long long)T * H + 7) / 8), 256, 0, st)(S->lout, RV, L.lin_norm, out, ldo, T, H, P, eps, S->b0 + a.dg, ldp, alpha, 0, 0, nullptr, nullptr);
+  launch_next(head_rmsnorm, (unsigned)(((long long)T * H + 7) / 8), 256, 0, st)(S->lout, RV, L.lin_norm, out, ldo, T, H, P, eps, S->b0 + a.dg, ldp, alpha, 0, 0, nullptr, nullptr, out16);
   S->launches += 3;
 }
 
@@ -1829,7 +1842,7 @@ static void lightning_forward(State* S, const HLayer& L, LayerState& ls, int ldp
 }
 
 // mLSTM of T tokens from the stacked projection in S->b0 (columns of mlstm_layout) -> normed and gated heads in out [T][H P]
-static void mlstm_forward(State* S, const HLayer& L, LayerState& ls, int ldp, const MlstmLayout& a, float* out, float eps, int T, cudaStream_t st) {
+static void mlstm_forward(State* S, const HLayer& L, LayerState& ls, int ldp, const MlstmLayout& a, float* out, float eps, int T, cudaStream_t st, __nv_bfloat16* out16) {
   const dsk_layer_spec& sp = L.sp;
   const int H = sp.lin_heads, N = sp.lin_dim, P = sp.lin_vdim, HN = H * N, HP = H * P;
   float *nst = ls.lin + (size_t)HN * P, *mst = nst + HN;
@@ -1843,7 +1856,7 @@ static void mlstm_forward(State* S, const HLayer& L, LayerState& ls, int ldp, co
   launch_next(mlstm_gates, H, 256, 0, st)(S->b0, ldp, (int)a.i, (int)a.f, sp.lin_gate_cap, T, H, gi, gf, gm, mst);
   launch_next(mlstm_gram, dim3((unsigned)((T + kLinBlk - 1) / kLinBlk), (unsigned)H), 256, (size_t)2 * kLinBlk * (((N + 3) & ~3) + 4) * 4, st)(S->b0, S->b0 + HN, ldp, gi, gf, gm, T, H, N, S->lrec);
   launch_lin_scan(false, S->b0, S->b0 + HN, ldp, N, 1, S->b0 + 2 * HN, ldp, S->lrec, ls.lin, S->lout, HP, T, H, N, P, st, nst, S->lden);
-  launch_next(head_rmsnorm, (unsigned)(((long long)T * H + 7) / 8), 256, 0, st)(S->lout, HP, L.mnorm, out, HP, T, H, P, eps, S->b0 + a.g, ldp, 1.f, P, 1, S->lden, gm);
+  launch_next(head_rmsnorm, (unsigned)(((long long)T * H + 7) / 8), 256, 0, st)(S->lout, HP, L.mnorm, out, HP, T, H, P, eps, S->b0 + a.g, ldp, 1.f, P, 1, S->lden, gm, out16);
   S->launches += 4;
 }
 
@@ -1980,18 +1993,28 @@ static void enqueue_head(dsk_model* m, dsk_state* s, int first, int count, float
   linear(S, c.quant == DSK_BF16, c.logit_softcap > 0.f ? HEPI_SOFTCAP : HEPI_STORE, P, 1, st);
 }
 
+// where a kernel that makes rows of the width for the products of a portion puts them rounded (those products read bf16 rows; short steps' read fp32)
+static __nv_bfloat16* mirror16(State* S, int T) { return T > 4 ? S->h16 : nullptr; }
 // RMS norm in groups, stored.  A warp a group where the groups are more than the CTAs that the chip holds at a time (eight of 256 threads an SM).
-static void rms_groups(const float* in, int ld_in, const float* w, float* out, int ld_out, int T, int n, int groups, float eps, cudaStream_t st) {
-  if (n / groups <= 1024 && (long long)T * groups > 8ll * g_sm_count)
-    launch_next(group_rmsnorm_rows, (unsigned)(((long long)T * groups + 7) / 8), 256, 0, st)(in, ld_in, w, out, ld_out, T, n, groups, eps);
-  else launch_next(group_rmsnorm<float>, dim3((unsigned)T, (unsigned)groups), 256, 0, st)(in, ld_in, w, out, ld_out, n, groups, eps, 0, 0.f, nullptr, 0, nullptr, 0);
+// out16 (nullable): packed bf16 rows, with the warps' form beside the others (out may be null), else instead of them.  Returns whether both were written.
+static bool rms_groups(const float* in, int ld_in, const float* w, float* out, int ld_out, int T, int n, int groups, float eps, cudaStream_t st, __nv_bfloat16* out16 = nullptr) {
+  const bool rows = n / groups <= 1024 && (long long)T * groups > 8ll * g_sm_count;
+  if (rows)
+    launch_next(group_rmsnorm_rows, (unsigned)(((long long)T * groups + 7) / 8), 256, 0, st)(in, ld_in, w, out, ld_out, T, n, groups, eps, out16);
+  else launch_next(group_rmsnorm<float>, dim3((unsigned)T, (unsigned)groups), 256, 0, st)(in, ld_in, w, out, ld_out, n, groups, eps, 0, 0.f, nullptr, 0, nullptr, 0, out ? nullptr : out16);
+  return rows;
 }
 // the model's norm over the T rows of `in` (width values each): stored into `out`, or added into it times alpha (mode 1)
 static void norm_rows(const dsk_hybrid_config& c, State* S, const float* in, const float* w, const float* b, float* out, int T, int mode, float alpha, cudaStream_t st) {
-  if (c.norm_kind == DSK_NORM_LAYER) launch_next(layer_norm, T, 256, 0, st)(in, c.dim, w, b, out, c.dim, c.dim, c.norm_eps, mode, alpha, nullptr, 0);
-  else if (mode == 0 && c.norm_groups == 1) launch_next(rms_open, T, 256, 0, st)(const_cast<float*>(in), nullptr, nullptr, w, out, c.dim, c.norm_eps);   // (adds nothing: the row is only read)
-  else if (mode == 0) rms_groups(in, c.dim, w, out, c.dim, T, c.dim, c.norm_groups, c.norm_eps, st);
-  else launch_next(group_rmsnorm<float>, dim3((unsigned)T, (unsigned)c.norm_groups), 256, 0, st)(in, c.dim, w, out, c.dim, c.dim, c.norm_groups, c.norm_eps, mode, alpha, nullptr, 0, nullptr, 0);
+  __nv_bfloat16* m16 = mirror16(S, T);
+  S->mirror = m16 ? out : nullptr;
+  if (c.norm_kind == DSK_NORM_LAYER) launch_next(layer_norm, T, 256, 0, st)(in, c.dim, w, b, out, c.dim, c.dim, c.norm_eps, mode, alpha, nullptr, 0, m16);
+  else if (mode == 0 && c.norm_groups == 1) launch_next(rms_open, T, 256, 0, st)(const_cast<float*>(in), nullptr, nullptr, w, out, c.dim, c.norm_eps, m16);   // (adds nothing: the row is only read)
+  else if (mode == 0) { if (!rms_groups(in, c.dim, w, out, c.dim, T, c.dim, c.norm_groups, c.norm_eps, st, m16)) S->mirror = nullptr; }
+  else {
+    S->mirror = nullptr;
+    launch_next(group_rmsnorm<float>, dim3((unsigned)T, (unsigned)c.norm_groups), 256, 0, st)(in, c.dim, w, out, c.dim, c.dim, c.norm_groups, c.norm_eps, mode, alpha, nullptr, 0, nullptr, 0, nullptr);
+  }
   S->launches++;
 }
 
@@ -2028,6 +2051,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
   const int nb = c.bigram_buckets;
   float* keep_emb = S->xin ? S->xin + W : S->emb;   // the embedding output again, for a layer loop
   const int ld_keep = S->xin ? 2 * W : W;
+  S->mirror = nullptr;
   if (bf) launch_next(embed_rows<__nv_bfloat16>, T, 256, 0, st)(S->d_tok, (const __nv_bfloat16*)M->embed.p, W, S->x, es, nb > 0 ? (const __nv_bfloat16*)M->bigram.p : nullptr,
                                                        nb, c.bigram_mul_prev, c.bigram_mul_cur, S->d_ctl, S->d_prev, keep_emb, ld_keep);
   else launch_next(embed_rows<float>, T, 256, 0, st)(S->d_tok, (const float*)M->embed.p, W, S->x, es, nb > 0 ? (const float*)M->bigram.p : nullptr, nb, c.bigram_mul_prev,
@@ -2038,6 +2062,8 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
   const bool tl = S->timeline && pos0 >= 0;
   auto MK = [&](const char* label) { if (tl) mark(S, label, st); };
   MK("embed");
+  // a product whose input the kernel ahead of it may write rounded: where to
+  auto rounded = [&](int epi, GemmP& P) -> __nv_bfloat16* { return T > 4 && bf && tc_ok(S, bf, epi, P, 1) ? const_cast<__nv_bfloat16*>(P.A16 = S->a16) : nullptr; };
   const Sink to_x{HEPI_ADD, S->x, mult}, to_y{HEPI_STORE, S->y, 1.f};
   // sandwich blocks: "x += norm(y); h = norm(x)" runs as one kernel (not while the residual stream is being recorded)
   const bool fuse = fused_norms(c) && !trace, frms = fuse && rms_fused(c);
@@ -2056,6 +2082,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       if (c.canon_taps <= 0) return S->x;
       float* ring = ls.canon ? ls.canon + (size_t)which * (c.canon_taps - 1) * W : nullptr;
       const int ty = (T + kCanonTokens - 1) / kCanonTokens;
+      S->mirror = nullptr;
       launch_next(canon_conv, dim3((unsigned)((W + 127) / 128), (unsigned)ty), 128, 0, st)(S->x, W, taps, ring, S->h, W, T, W, c.canon_taps, S->d_ctl);
       S->launches++;
       if (ty > 1 && c.canon_taps > 1) { launch_next(canon_history, (W + 127) / 128, 128, 0, st)(S->x, W, ring, T, W, c.canon_taps, S->d_ctl); S->launches++; }
@@ -2078,6 +2105,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         G.bias = rg_b;
         linear(S, bf, HEPI_SIGMUL, G, 1, st);
       }
+      S->mirror = nullptr;
       launch_next(close_open_small, (W + 127) / 128, 128, 0, st)(S->y, close_w, mult, c.norm_eps, S->x, W, next_taps, next_ring, S->h, T, W, c.canon_taps, S->d_ctl);
       S->launches++;
     };
@@ -2087,7 +2115,8 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
     if (post) { if (!h_ready) hin = open_post(L.canon1, 0); }
     else if (pre) {   // a pass of the layer loop opens with its vector (and, but for the first, the embedding) added to the stream
       const bool again = c.loop_embed && run.pass > 0;
-      launch_next(rms_open, T, 256, 0, st)(S->x, again ? S->emb : nullptr, run.pass >= 0 ? M->loop_step + (size_t)run.pass * W : nullptr, L.norm1, S->h, W, c.norm_eps);
+      launch_next(rms_open, T, 256, 0, st)(S->x, again ? S->emb : nullptr, run.pass >= 0 ? M->loop_step + (size_t)run.pass * W : nullptr, L.norm1, S->h, W, c.norm_eps, mirror16(S, T));
+      S->mirror = mirror16(S, T) ? S->h : nullptr;
       S->launches++;
     } else if (!h_ready) {
       if (run.pass >= 0 && c.loop_in) {   // a pass of the layer loop opens with a product over [stream | embedding], its vector as the bias
@@ -2098,6 +2127,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         linear(S, bf, HEPI_STORE, In, 1, st);
         MK("loop.in");
       } else if (run.pass >= 0) {   // a pass of the layer loop opens with its own vector added to the residual stream
+        if (S->mirror == S->x) S->mirror = nullptr;
         launch_next(add_row, T, 256, 0, st)(S->x, W, M->loop_step + (size_t)run.pass * W, W);
         S->launches++;
       }
@@ -2108,7 +2138,8 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
     if (c.token_shift && hs_ready) { hin = S->hs; hs_ready = false; }   // the previous run's last kernel shifted already
     else if (c.token_shift) {      // the mixer reads its input blended with the previous token's; the step's last row is carried on
       const int ty = (T + kCanonTokens - 1) / kCanonTokens;
-      launch_next(token_shift, dim3((unsigned)((W + 127) / 128), (unsigned)ty), 128, 0, st)(hin, W, L.shift, ls.shift, S->hs, W, T, W, S->d_ctl);
+      launch_next(token_shift, dim3((unsigned)((W + 127) / 128), (unsigned)ty), 128, 0, st)(hin, W, L.shift, ls.shift, S->hs, W, T, W, S->d_ctl, mirror16(S, T));
+      S->mirror = mirror16(S, T) ? S->hs : nullptr;
       S->launches++;
       if (ty > 1) { launch_next(shift_carry, (W + 127) / 128, 128, 0, st)(hin, W, ls.shift, T, W); S->launches++; }
       hin = S->hs;
@@ -2116,20 +2147,23 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
     // the closing norm of this run's last sublayer, fused with what opens the next run (its pass vector and first norm) or the head
     auto close_run = [&](const float* wb, int routed = 0) {   // routed > 0: the sublayer's output is the weighted sum of the routed rows in S->b3
       if (!fuse) { norm_rows(c, S, S->y, wb, nullptr, S->x, T, 1, mult, st); return; }
+      __nv_bfloat16* m16 = mirror16(S, T);
       const Run* next = ri + 1 < M->runs.size() ? &M->runs[ri + 1] : nullptr;
       if (frms) {
         const bool to_xin = next && next->pass >= 0;   // the pass opens with a product: its norm follows that
         const bool product = to_xin && c.loop_in;
         const bool shared = routed && sp.ff_shared > 0;
         launch_rms_add_norm(T, W, st, routed ? S->b3 : S->y, routed ? S->wgt : nullptr, routed, shared ? S->b3 + (size_t)T * routed * W : nullptr, S->wsh, wb, S->x,
-                                        product ? S->xin : S->x, product ? 2 * W : W, to_xin ? nullptr : next ? M->L[next->layer].norm1 : M->final_norm, S->h, W, c.norm_eps, mult);
+                                        product ? S->xin : S->x, product ? 2 * W : W, to_xin ? nullptr : next ? M->L[next->layer].norm1 : M->final_norm, S->h, W, c.norm_eps, mult, m16);
+        S->mirror = !to_xin && m16 ? S->h : nullptr;
         S->launches++;
         xin_ready = product;
         h_ready = !to_xin;
         return;
       }
       const float* row = next && next->pass >= 0 ? M->loop_step + (size_t)next->pass * W : nullptr;
-      launch_next(layer_norm_add_norm, T, 256, 0, st)(S->y, wb, S->x, row, next ? M->L[next->layer].norm1 : M->final_norm, S->h, W, c.norm_eps, mult);
+      launch_next(layer_norm_add_norm, T, 256, 0, st)(S->y, wb, S->x, row, next ? M->L[next->layer].norm1 : M->final_norm, S->h, W, c.norm_eps, mult, m16);
+      S->mirror = m16 ? S->h : nullptr;
       S->launches++;
       h_ready = true;
     };
@@ -2273,9 +2307,11 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       const int ldi = Q + RW;
       MK("norm");
       linear(S, bf, HEPI_STORE, gp(hin, W, L.in2.p, W, S->b1, ldi, T, ldi, W), 1, st);              // [query latent | key / value latent | rotated key part]
-      rms_groups(S->b1, ldi, L.dq_norm, S->b2, Q, T, Q, 1, c.norm_eps, st);
+      GemmP Uq = gp(S->b2, Q, L.uq.p, Q, S->b0, H * DK, T, H * DK, Q);                             // q [T][H][D | Rd]
+      __nv_bfloat16* q16 = rounded(HEPI_STORE, Uq);
+      rms_groups(S->b1, ldi, L.dq_norm, q16 ? nullptr : S->b2, Q, T, Q, 1, c.norm_eps, st, q16);
       S->launches++;
-      linear(S, bf, HEPI_STORE, gp(S->b2, Q, L.uq.p, Q, S->b0, H * DK, T, H * DK, Q), 1, st);       // q [T][H][D | Rd]
+      linear(S, bf, HEPI_STORE, Uq, 1, st);
       const bool portion = pos0 >= 0 && T >= kPrefillMin && S->prefill_keys > 0;
       launch_next(mla_prepare, T, 256, 0, st)(S->b1 + Q, ldi, L.dkv_norm, c.norm_eps, S->b0, portion ? nullptr : S->b2, H, D, Rd, R, sp.rot_dims, L.rot_freq,
                                      L.rot_mag, sp.rot_layout, S->d_ctl, cache, L.ring);
@@ -2362,10 +2398,10 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       MK("norm");
       linear(S, bf, HEPI_STORE, gp(hin, W, L.qkv.p, W, S->b0, ldp, T, ldp, W), 1, st);
       MK("gdn.in");
-      gdn_forward(S, L, ls, ldp, lay, S->b3, RV, 1.f, c.norm_eps, T, st);
-      MK("gdn");
       GemmP P = gp(S->b3, RV, L.o.p, RV, sink.C, W, T, W, RV);
       P.alpha = sink.alpha;
+      gdn_forward(S, L, ls, ldp, lay, S->b3, RV, 1.f, c.norm_eps, T, st, rounded(sink.epi, P));
+      MK("gdn");
       linear(S, bf, sink.epi, P, 1, st);
       MK("gdn.o");
     } else if (sp.mixer == DSK_MIX_MLSTM) {
@@ -2376,10 +2412,10 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       In.bias = L.lin_bias;
       linear(S, bf, HEPI_STORE, In, 1, st);
       MK("lin.in");
-      mlstm_forward(S, L, ls, pw, lay, S->b3, c.norm_eps, T, st);
-      MK("lin.scan");
       GemmP P = gp(S->b3, HP, L.o.p, HP, sink.C, W, T, W, HP);
       P.alpha = sink.alpha;
+      mlstm_forward(S, L, ls, pw, lay, S->b3, c.norm_eps, T, st, rounded(sink.epi, P));
+      MK("lin.scan");
       linear(S, bf, sink.epi, P, 1, st);
       MK("lin.o");
     } else if (sp.mixer == DSK_MIX_LIGHTNING) {
@@ -2391,11 +2427,11 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       MK("lin.in");
       lightning_forward(S, L, ls, pw, T, st);
       MK("lin.scan");
-      launch_next(group_rmsnorm<float>, T, 256, 0, st)(S->lout, HP, L.mnorm, S->b3, HP, HP, 1, c.norm_eps, 0, 0.f, nullptr, 0, S->b0 + 2 * HN + HP, pw);
-      S->launches++;
-      MK("lin.norm");
       GemmP P = gp(S->b3, HP, L.o.p, HP, sink.C, W, T, W, HP);
       P.alpha = sink.alpha;
+      launch_next(group_rmsnorm<float>, T, 256, 0, st)(S->lout, HP, L.mnorm, S->b3, HP, HP, 1, c.norm_eps, 0, 0.f, nullptr, 0, S->b0 + 2 * HN + HP, pw, rounded(sink.epi, P));
+      S->launches++;
+      MK("lin.norm");
       linear(S, bf, sink.epi, P, 1, st);
       MK("lin.o");
     } else if (sp.mixer == DSK_MIX_HGRN2) {
@@ -2407,11 +2443,12 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       MK("lin.in");
       launch_hgrn2(sp, S->b0, pw, ls.lin, S->b2, T, st);
       MK("lin.scan");
-      launch_next(head_rmsnorm, (unsigned)(((long long)T * H + 7) / 8), 256, 0, st)(S->b2, HP, L.lin_norm, S->b3, HP, T, H, sp.lin_vdim, c.norm_eps, nullptr, 0, 1.f, 0, 0, nullptr, nullptr);
-      S->launches += 2;
-      MK("lin.norm");
       GemmP P = gp(S->b3, HP, L.o.p, HP, sink.C, W, T, W, HP);
       P.alpha = sink.alpha;
+      launch_next(head_rmsnorm, (unsigned)(((long long)T * H + 7) / 8), 256, 0, st)(S->b2, HP, L.lin_norm, S->b3, HP, T, H, sp.lin_vdim, c.norm_eps, nullptr, 0, 1.f, 0, 0, nullptr, nullptr,
+                                                                                    rounded(sink.epi, P));
+      S->launches += 2;
+      MK("lin.norm");
       linear(S, bf, sink.epi, P, 1, st);
       MK("lin.o");
     } else if (is_ssd(sp)) {
@@ -2436,11 +2473,12 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         S->launches += 2;
       } else launch_scan(sp, S->b0, pw, S->b1, ch, L, ls.ssm, S->b2, T, st);
       MK("ssd.scan");
-      rms_groups(S->b2, inner, L.mnorm, S->b3, inner, T, inner, sp.ssm_norm_groups, c.norm_eps, st);
-      S->launches += 4;
-      MK("ssd.norm");
       GemmP P = gp(S->b3, inner, L.o.p, inner, sink.C, W, T, W, inner);
       P.alpha = sink.alpha;
+      __nv_bfloat16* o16 = rounded(sink.epi, P);
+      rms_groups(S->b2, inner, L.mnorm, o16 ? nullptr : S->b3, inner, T, inner, sp.ssm_norm_groups, c.norm_eps, st, o16);
+      S->launches += 4;
+      MK("ssd.norm");
       linear(S, bf, sink.epi, P, 1, st);
       MK("ssd.o");
     } else {
@@ -2451,7 +2489,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       linear(S, bf, HEPI_STORE, gp(hin, W, L.q.p, W, S->b0, H * D, T, H * D, W), 1, st);
       if (L.owner == li) {
         linear(S, bf, HEPI_STORE, gp(hin, W, L.dkv.p, W, S->b1, R, T, R, W), 1, st);
-        launch_next(group_rmsnorm<float>, T, 256, 0, st)(S->b1, R, L.dkv_norm, cache, R, R, 1, c.norm_eps, 0, 0.f, S->d_ctl, O.ring, nullptr, 0);
+        launch_next(group_rmsnorm<float>, T, 256, 0, st)(S->b1, R, L.dkv_norm, cache, R, R, 1, c.norm_eps, 0, 0.f, S->d_ctl, O.ring, nullptr, 0, nullptr);
         S->launches++;
       }
       MK("att.q+latent");
@@ -2542,10 +2580,12 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
     if (sandwich) {   // x += norm1b(mixer output); the feed-forward then reads norm2 of the new x
       if (sp.ff_kind == DSK_FF_NONE) close_run(L.close1);
       else if (frms) {
-        launch_rms_add_norm(T, W, st, S->y, nullptr, 0, nullptr, nullptr, L.close1, S->x, S->x, W, L.norm2, S->h, W, c.norm_eps, mult);
+        launch_rms_add_norm(T, W, st, S->y, nullptr, 0, nullptr, nullptr, L.close1, S->x, S->x, W, L.norm2, S->h, W, c.norm_eps, mult, mirror16(S, T));
+        S->mirror = mirror16(S, T) ? S->h : nullptr;
         S->launches++;
       } else if (fuse) {
-        launch_next(layer_norm_add_norm, T, 256, 0, st)(S->y, L.close1, S->x, nullptr, L.norm2, S->h, W, c.norm_eps, mult);
+        launch_next(layer_norm_add_norm, T, 256, 0, st)(S->y, L.close1, S->x, nullptr, L.norm2, S->h, W, c.norm_eps, mult, mirror16(S, T));
+        S->mirror = mirror16(S, T) ? S->h : nullptr;
         S->launches++;
       } else {
         norm_rows(c, S, S->y, L.close1, nullptr, S->x, T, 1, mult, st);
@@ -2554,7 +2594,8 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       MK("norm");
     }
     if (pre && sp.ff_kind != DSK_FF_NONE) {
-      launch_next(rms_open, T, 256, 0, st)(S->x, nullptr, nullptr, L.norm2, S->h, W, c.norm_eps);
+      launch_next(rms_open, T, 256, 0, st)(S->x, nullptr, nullptr, L.norm2, S->h, W, c.norm_eps, mirror16(S, T));
+      S->mirror = mirror16(S, T) ? S->h : nullptr;
       S->launches++;
       hin = S->h;
       MK("norm");
@@ -2637,9 +2678,11 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         }
       }
       if (combine_in_norm) {   // x += ln(sum_k w_k y_k): the weighted sum of the experts' outputs is taken by the closing layer norm as it reads its row
-        launch_next(layer_norm, T, 256, 0, st)(S->b3, W, L.close2, L.norm2_bias, S->x, W, W, c.norm_eps, 1, mult, S->wgt, top);
+        launch_next(layer_norm, T, 256, 0, st)(S->b3, W, L.close2, L.norm2_bias, S->x, W, W, c.norm_eps, 1, mult, S->wgt, top, mirror16(S, T));
+        S->mirror = mirror16(S, T) ? S->x : nullptr;
         S->launches++;
       } else if (!frms) {   // (sandwich blocks of RMS norms combine as they close)
+        if (S->mirror == sink.C) S->mirror = nullptr;
         launch_next(moe_combine, dim3((unsigned)T, (unsigned)((W + (W % 4 ? 255 : 1023)) / (W % 4 ? 256 : 1024))), 256, 0, st)(sink.C, W, S->b3, S->wgt, top, W, sink.alpha, sink.epi == HEPI_ADD ? 1 : 0, shared ? ysh : nullptr, S->wsh);
         S->launches++;
       }
@@ -2663,17 +2706,21 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
       // decode-sized steps of post-norm blocks: the normed addition and the next layer's token shift in one launch over 128-channel CTAs
       if (post && c.canon_taps <= 0 && T <= kCloseOpenTokens && !trace) {
         const bool next_shift = c.token_shift && has_next;
+        S->mirror = nullptr;
         launch_next(rms_add_shift_small, (W + 127) / 128, 128, 0, st)(S->h, L.snorm, mult, c.norm_eps, S->x, W, next_shift ? M->L[M->runs[ri + 1].layer].shift : nullptr,
                                                              next_shift ? S->L[ri + 1].shift : nullptr, S->hs, T, W, S->d_ctl);
         hs_ready = next_shift;
-      } else launch_next(group_rmsnorm<float>, T, 256, 0, st)(S->h, W, L.snorm, S->x, W, W, 1, c.norm_eps, 1, mult, nullptr, 0, nullptr, 0);
+      } else {
+        if (S->mirror == S->x) S->mirror = nullptr;
+        launch_next(group_rmsnorm<float>, T, 256, 0, st)(S->h, W, L.snorm, S->x, W, W, 1, c.norm_eps, 1, mult, nullptr, 0, nullptr, 0, nullptr);
+      }
       S->launches++;
       MK("side");
     }
     if (trace) CKL(cudaMemcpyAsync(trace + ri * (size_t)T * W, S->x, (size_t)T * W * 4, cudaMemcpyDeviceToDevice, st));
   }
   if (n_want > 0) {   // final norm of every row, LM head on the first group of wanted rows (enqueue_head does the others)
-    if (pre) { launch_next(rms_open, T, 256, 0, st)(S->x, nullptr, nullptr, M->final_norm, S->h, W, c.norm_eps); S->launches++; }
+    if (pre) { launch_next(rms_open, T, 256, 0, st)(S->x, nullptr, nullptr, M->final_norm, S->h, W, c.norm_eps, mirror16(S, T)); S->mirror = mirror16(S, T) ? S->h : nullptr; S->launches++; }
     else if (!h_ready) norm_rows(c, S, S->x, M->final_norm, M->final_norm_b, S->h, T, 0, 0.f, st);
     enqueue_head(m, s, 0, std::min(n_want, S->head_rows), pos0 < 0 ? s->logits : S->logits, st);   // a captured step leaves its one row in the state
     MK("head");

@@ -309,5 +309,16 @@ __global__ void __launch_bounds__(256) bf16_rows(const float* __restrict__ A, in
   }
 }
 
+// out[i] = in[a_map[i] / a_div], rows of K bf16 values (K a multiple of 8)
+__global__ void __launch_bounds__(256) gather_rows16(const __nv_bfloat16* __restrict__ in, const int* __restrict__ a_map, int a_div, __nv_bfloat16* __restrict__ out, int rows, int K) {
+  grid_enter();
+  const int per = K / 8;
+  const long long n = (long long)rows * per;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    const int row = (int)(i / per), k = (int)(i - (long long)row * per);
+    reinterpret_cast<uint4*>(out + (size_t)row * K)[k] = reinterpret_cast<const uint4*>(in + (size_t)(a_map[row] / a_div) * K)[k];
+  }
+}
+
 }  // namespace hy
 }  // namespace dsk
