@@ -37,6 +37,7 @@
 #include "dsk_pattn.cuh"
 #include "dsk_pattn5.cuh"
 #include "dsk_split.cuh"
+#include "dsk_linmma.cuh"
 
 using namespace dsk;
 

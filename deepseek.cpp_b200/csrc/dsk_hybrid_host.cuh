@@ -153,6 +153,7 @@ struct State {
   float* wsh = nullptr;                      // [chunk] weights of the shared expert
   // linear attention: prepared q, k and v rows, per-block records, outputs ahead of their norm
   float *lq = nullptr, *lk = nullptr, *lv = nullptr, *lrec = nullptr, *lout = nullptr;
+  float* lseg = nullptr;                     // lin_mma: states between the segments of a step
   float* hs = nullptr;                       // the token-shifted mixer input of the step
   float* vfirst = nullptr;                   // [chunk][kv_heads * vdim] values of the step's tokens in the first value-mixing layer
   int* d_prev = nullptr;                     // the sequence's last token (bigram embedding)
@@ -410,6 +411,7 @@ static void set_kernel_attrs() {
   cudaFuncSetAttribute(hgrn2_scan<1, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, big); cudaFuncSetAttribute(hgrn2_scan<2, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, big);
   cudaFuncSetAttribute(gemm_mma<HEPI_SILU_SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMmaSmem);
   cudaFuncSetAttribute(gemm_mma<HEPI_SOFTCAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMmaSmem);
+  cudaFuncSetAttribute(lin_mma<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, LinMma<8>::SMEM); cudaFuncSetAttribute(lin_mma<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, LinMma<16>::SMEM);
 #define DSK_LSCAN_ATTR(A, B, C) \
   cudaFuncSetAttribute(lin_scan<true, A, B, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, big); \
   cudaFuncSetAttribute(lin_scan<false, A, B, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, big)
@@ -1220,7 +1222,7 @@ static dsk_state* state_create(dsk_model* m) {
   size_t mx0 = c.dim, mx1 = c.dim, mx2 = c.dim, mx3 = c.dim, mxE = 1, mxTop = 1;
   S->L.resize(M->runs.size());   // one state per layer run
   bool any_talk = false;
-  size_t mxLQ = 0, mxLV = 0, mxLH = 0, mxMH = 0, mxShared = 0;
+  size_t mxLQ = 0, mxLV = 0, mxLH = 0, mxMH = 0, mxShared = 0, mxSeg = 0;
   size_t mxGV = 0;
   for (size_t r = 0; r < M->runs.size(); r++) {
     const int i = M->runs[r].layer;
@@ -1251,12 +1253,14 @@ static dsk_state* state_create(dsk_model* m) {
       if (salloc(S, (void**)&ls.lin, ls.lin_bytes, false, true)) return nullptr;
       mx0 = std::max<size_t>(mx0, mlstm_layout(sp).total); mx3 = std::max<size_t>(mx3, HP);
       mxLV = std::max(mxLV, HP); mxLH = std::max(mxLH, H); mxMH = std::max(mxMH, H);
+      mxSeg = std::max(mxSeg, lin_mma_floats((int)H, sp.lin_vdim / 16 + 1, sp.lin_dim, kLmSegs));
     } else if (sp.mixer == DSK_MIX_LIGHTNING) {
       const size_t HN = (size_t)sp.lin_heads * sp.lin_dim, HP = (size_t)sp.lin_heads * sp.lin_vdim;
       ls.lin_bytes = HN * sp.lin_vdim * 4;
       if (salloc(S, (void**)&ls.lin, ls.lin_bytes, false, true)) return nullptr;
       mx0 = std::max<size_t>(mx0, 2 * HN + 2 * HP); mx3 = std::max<size_t>(mx3, HP);
       mxLV = std::max(mxLV, HP); mxLH = std::max<size_t>(mxLH, sp.lin_heads);
+      mxSeg = std::max(mxSeg, lin_mma_floats(sp.lin_heads, (sp.lin_vdim + 15) / 16, sp.lin_dim, kLmSegs));
     } else if (sp.mixer == DSK_MIX_HGRN2) {
       const size_t HN = (size_t)sp.lin_heads * sp.lin_dim, HP = (size_t)sp.lin_heads * sp.lin_vdim;
       ls.lin_bytes = HN * sp.lin_vdim * 4;
@@ -1293,6 +1297,7 @@ static dsk_state* state_create(dsk_model* m) {
       mx0 = std::max<size_t>(mx0, ssd_proj(sp)); mx1 = std::max<size_t>(mx1, ssd_channels(sp));
       mx2 = std::max<size_t>(mx2, ssd_inner(sp)); mx3 = std::max<size_t>(mx3, ssd_inner(sp));
       mxLH = std::max<size_t>(mxLH, sp.ssm_heads);
+      mxSeg = std::max(mxSeg, lin_mma_floats(sp.ssm_heads, (sp.ssm_vdim + 15) / 16, sp.ssm_state, kLmSegs));
     } else {
       if (M->runs[r].owner_run == (int)r) {
         ls.cache_bytes = (size_t)L.ring * sp.att_kv_rank * 4;
@@ -1381,6 +1386,7 @@ static dsk_state* state_create(dsk_model* m) {
   }
   rc |= salloc(S, (void**)&S->x, Tc * c.dim * 4) | salloc(S, (void**)&S->h, Tc * c.dim * 4);
   if (c.loop_embed && c.loop_times > 1) rc |= salloc(S, (void**)&S->emb, Tc * c.dim * 4);
+  if (mxSeg && Tc >= 64) rc |= salloc(S, (void**)&S->lseg, mxSeg * 4);
   if (mxLH) rc |= salloc(S, (void**)&S->lrec, (Tc + kLinBlk - 1) / kLinBlk * mxLH * kRecFloats * 4) | salloc(S, (void**)&S->lout, Tc * mxLV * 4);
   for (const HLayer& L : M->L)
     if (L.sp.mixer2 && !S->side && (cudaStreamCreateWithFlags(&S->side, cudaStreamNonBlocking) != cudaSuccess || cudaEventCreateWithFlags(&S->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
@@ -1771,13 +1777,42 @@ static void launch_hgrn2(const dsk_layer_spec& sp, const float* proj, int ld, fl
 #undef DSK_LIN
 }
 
-// the walk over the blocks of a step (lin_scan): lanes per channel group by the key size, warps per CTA by how many CTAs there are
 static size_t ssd_gram_smem(const dsk_layer_spec& s) {
   return ((size_t)2 * kLinBlk * (((s.ssm_state + 3) & ~3) + 4) + (size_t)2 * kLinBlk * (s.ssm_heads / s.ssm_groups)) * 4;
 }
+// Whether lin_mma walks a portion, and in how many segments.  Times of a block in us, 128 (64) key entries: walked for results 2.0 (1.35), for the end state alone 1.4 (0.9), a round of
+// CTAs each, and 8 for the launch, 5 for a second; lin_scan 7.7, a block 1.1 and 1.3 more where 64 heads of 64 channels fill the chip.  Whole walks of 2048 tokens: 64 heads of 64 channels 312 (lin_scan) and 215, 16 of 128 187 and 114; 600
+// tokens, 16 heads of 64, 64 entries 46 and 23; 100 tokens 20 and 22: not taken.
+static int lin_mma_segments(const float* q, const float* k, int ldq, int hs, const float* v, int ldv, int T, int H, int N, int P, bool extra, const float* seg) {
+  auto al = [](const float* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  if (!seg || (N != 64 && N != 128) || P % 4 || ldq % 4 || hs % 4 || ldv % 4 || !al(q) || !al(k) || !al(v)) return 0;
+  const int nb = (T + kLinBlk - 1) / kLinBlk, ctas = H * ((P + (extra ? 1 : 0) + kLmCh - 1) / kLmCh);
+  const double full = N == 128 ? 2.0 : 1.35, ends = N == 128 ? 1.4 : 0.9;
+  double best = 7.7 + nb * (1.1 + 1.3 * (double)H * P * N / (64.0 * 64 * 128));
+  int segs = 0;
+  for (int n = 1; n <= kLmSegs; n++) {
+    const int per = (nb + n - 1) / n, rounds = (ctas * n + g_sm_count - 1) / g_sm_count, first = (ctas * (n - 1) + g_sm_count - 1) / g_sm_count;
+    const double cost = per * (rounds * full + first * ends) + (n > 1 ? 13 : 8);
+    if ((nb + per - 1) / per == n && cost < best) { best = cost; segs = n; }
+  }
+  return segs;
+}
+static void launch_lin_mma(LinMmaP p, int N, int nseg, cudaStream_t st) {
+  const int nb = (p.T + kLinBlk - 1) / kLinBlk, cg = (p.groups + kLmGroups - 1) / kLmGroups;
+  p.nseg = nseg; p.per = (nb + nseg - 1) / nseg;
+  auto* kernel = N == 64 ? lin_mma<8> : lin_mma<16>;
+  const size_t smem = N == 64 ? LinMma<8>::SMEM : LinMma<16>::SMEM;
+  for (p.mode = nseg > 1 ? 0 : 1; p.mode < 2; p.mode++) launch_next(kernel, dim3((unsigned)p.H, (unsigned)cg, (unsigned)(p.mode ? nseg : nseg - 1)), kLmThreads, smem, st)(p);
+}
+
+// the walk over the blocks of a step (lin_scan): lanes per channel group by the key size, warps per CTA by how many CTAs there are
 static void launch_lin_scan(bool delta, const float* q, const float* k, int ldq, int hs, int rep, const float* v, int ldv, const float* rec, float* state,
-                            float* out, int ldo, int T, int H, int N, int P, cudaStream_t st, float* nst = nullptr, float* den = nullptr, int sn = 0, int sp = 1) {
+                            float* out, int ldo, int T, int H, int N, int P, cudaStream_t st, float* seg, float* nst = nullptr, float* den = nullptr, int sn = 0, int sp = 1) {
   if (!sn) sn = P;                    // state rows [N][P] of a head, unless said otherwise
+  if (const int n = delta ? 0 : lin_mma_segments(q, k, ldq, hs, v, ldv, T, H, N, P, nst != nullptr, seg)) {
+    launch_lin_mma(LinMmaP{q, k, v, rec, state, out, nst, den, seg, ldq, hs, rep, ldv, ldo, T, H, P, sn, sp, (P + (nst ? 1 : 0) + 15) / 16, n, 0, 0}, N, n, st);
+    return;
+  }
   const int TPC = N <= 32 ? 8 : N <= 64 ? 16 : 32, RQ = N <= 128 ? 1 : 2;
   int CPT = N > 128 ? 4 : 2;          // value channels per lane
   if (const char* e = getenv("DSK_LIN_CPT")) CPT = atoi(e) == 4 || N > 128 ? 4 : 2;   // A/B switch
@@ -1820,7 +1855,7 @@ static void gdn_forward(State* S, const HLayer& L, LayerState& ls, int ldp, cons
   const int nb = (T + kLinBlk - 1) / kLinBlk;
   const size_t smem = (size_t)(2 * kLinBlk * (NP + 4) + 2 * kLinBlk * kLinBlk + 8 * kLinBlk * kLinBlk) * 4;
   launch_next(gdn_prepare, dim3((unsigned)nb, (unsigned)(G + (RV + 255) / 256)), 256, smem, st)(D, S->lq, S->lk, S->lv, NP, S->lrec);
-  launch_lin_scan(true, S->lq, S->lk, G * NP, NP, H / G, S->lv, RV, S->lrec, ls.lin, S->lout, RV, T, H, N, P, st);
+  launch_lin_scan(true, S->lq, S->lk, G * NP, NP, H / G, S->lv, RV, S->lrec, ls.lin, S->lout, RV, T, H, N, P, st, nullptr);
   if (sp.gdn_conv > 1) { launch_next(conv_ring_store, (CH + 127) / 128, 128, 0, st)(S->b0, ldp, (int)a.dq, ls.hist, D.ring, T, CH, sp.gdn_conv, S->d_ctl); S->launches++; }
   launch_next(head_rmsnorm, (unsigned)(((long long)T * H + 7) / 8), 256, 0, st)(S->lout, RV, L.lin_norm, out, ldo, T, H, P, eps, S->b0 + a.dg, ldp, alpha, 0, 0, nullptr, nullptr, out16);
   S->launches += 3;
@@ -1837,7 +1872,7 @@ static void lightning_forward(State* S, const HLayer& L, LayerState& ls, int ldp
     return;
   }
   launch_next(lin_gram, dim3((unsigned)((T + kLinBlk - 1) / kLinBlk), (unsigned)H), 256, (size_t)2 * kLinBlk * (((N + 3) & ~3) + 4) * 4, st)(S->b0, S->b0 + HN, ldp, L.log_decay, T, H, N, S->lrec);
-  launch_lin_scan(false, S->b0, S->b0 + HN, ldp, N, 1, S->b0 + 2 * HN, ldp, S->lrec, ls.lin, S->lout, HP, T, H, N, P, st);
+  launch_lin_scan(false, S->b0, S->b0 + HN, ldp, N, 1, S->b0 + 2 * HN, ldp, S->lrec, ls.lin, S->lout, HP, T, H, N, P, st, S->lseg);
   S->launches += 2;
 }
 
@@ -1855,7 +1890,7 @@ static void mlstm_forward(State* S, const HLayer& L, LayerState& ls, int ldp, co
   float *gi = S->lgate, *gf = gi + (size_t)H * T, *gm = gf + (size_t)H * T;
   launch_next(mlstm_gates, H, 256, 0, st)(S->b0, ldp, (int)a.i, (int)a.f, sp.lin_gate_cap, T, H, gi, gf, gm, mst);
   launch_next(mlstm_gram, dim3((unsigned)((T + kLinBlk - 1) / kLinBlk), (unsigned)H), 256, (size_t)2 * kLinBlk * (((N + 3) & ~3) + 4) * 4, st)(S->b0, S->b0 + HN, ldp, gi, gf, gm, T, H, N, S->lrec);
-  launch_lin_scan(false, S->b0, S->b0 + HN, ldp, N, 1, S->b0 + 2 * HN, ldp, S->lrec, ls.lin, S->lout, HP, T, H, N, P, st, nst, S->lden);
+  launch_lin_scan(false, S->b0, S->b0 + HN, ldp, N, 1, S->b0 + 2 * HN, ldp, S->lrec, ls.lin, S->lout, HP, T, H, N, P, st, S->lseg, nst, S->lden);
   launch_next(head_rmsnorm, (unsigned)(((long long)T * H + 7) / 8), 256, 0, st)(S->lout, HP, L.mnorm, out, HP, T, H, P, eps, S->b0 + a.g, ldp, 1.f, P, 1, S->lden, gm, out16);
   S->launches += 4;
 }
@@ -2466,7 +2501,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         const int H = sp.ssm_heads, N = sp.ssm_state, P = sp.ssm_vdim, G = sp.ssm_groups;
         launch_next(ssd_gram, dim3((unsigned)((T + kLinBlk - 1) / kLinBlk), (unsigned)G), 256, ssd_gram_smem(sp), st)(
             S->b1 + inner + G * N, S->b1 + inner, ch, S->b0 + inner + ch, pw, L.dt_bias, L.A_log, T, H, N, H / G, S->lrec);
-        launch_lin_scan(false, S->b1 + inner + G * N, S->b1 + inner, ch, N, H / G, S->b1, ch, S->lrec, ls.ssm, S->b2, inner, T, H, N, P, st, nullptr, nullptr, 1, N);
+        launch_lin_scan(false, S->b1 + inner + G * N, S->b1 + inner, ch, N, H / G, S->b1, ch, S->lrec, ls.ssm, S->b2, inner, T, H, N, P, st, S->lseg, nullptr, nullptr, 1, N);
         if (inner % 4 == 0 && ch % 4 == 0 && pw % 4 == 0 && P % 4 == 0)
           launch_next(ssd_gate<4>, dim3((unsigned)T, (unsigned)((inner + 1023) / 1024)), 256, 0, st)(S->b2, S->b1, ch, S->b0, pw, L.D, inner, P);
         else launch_next(ssd_gate<1>, dim3((unsigned)T, (unsigned)((inner + 255) / 256)), 256, 0, st)(S->b2, S->b1, ch, S->b0, pw, L.D, inner, P);

@@ -129,6 +129,21 @@ def test_recurrence_in_blocks(mk_hybrid, ho, value):  # noqa: F811
     m.reset()
 
 
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+def test_recurrence_in_segments(mk_hybrid, ho, value):  # noqa: F811
+    ssd = {"type": "mamba2", "mixer": {"heads": 3, "vdim": 20, "state": 64, "groups": 1, "conv": 3, "norm_groups": 1}, "mlp": None}
+    cfg = ho.small_config(layers=[ssd] * 2, width=36, norm={"eps": 1e-5, "groups": 1})
+    m, W = mk_hybrid(cfg, seed=4, chunk=400, edit=lambda W: poisoned(W, value, 50))
+    toks = tokens_for(cfg, 400, 5)
+    toks[toks == 50] = 7
+    for at in (1, 30, 201, 399):
+        t = toks.copy()
+        t[at] = 50
+        m.reset()
+        assert ahead_of_the_poison(m, ho.run, cfg, W, t, at, [400]) < F32_TOL
+    m.reset()
+
+
 @pytest.mark.parametrize("router", ["sigmoid", "groups"])
 def test_routed_rows(mk, mk_hybrid, no, ho, router):  # noqa: F811
     """A token whose router scores are NaN gets experts that exist, and the others theirs: in short steps, and in portions, where rows are put into

@@ -7,6 +7,8 @@ from test_gpu_hybrid import F32_TOL, ho, mk, rel, tokens_for  # noqa: F401
 from test_gpu_netusun import in_portions
 from test_gpu_netusun import mk as mk_netusun  # noqa: F401
 from test_gpu_netusun import no  # noqa: F401
+from test_gpu_zetivik import mk as mk_zetivik  # noqa: F401
+from test_gpu_zetivik import zo  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -22,6 +24,42 @@ def test_recurrence_in_blocks(mk, ho, heads, vdim, state, groups):  # noqa: F811
     toks = tokens_for(cfg, 90, 11)
     exp = ho.run(cfg, W, toks)[0]
     for sizes in ([64, 26], [5, 17, 1, 1, 33], [4, 16, 32], [15, 49]):
+        assert rel(in_portions(m, toks, sizes), exp) < F32_TOL
+
+
+# walks in segments on the tensor cores: 64 and 128 key entries, channels that end inside a group of 16 or need a second CTA, heads sharing a group, one to eight segments, the
+# last one short or ragged; a portion that begins in a decoded state and is followed by tokens
+@pytest.mark.parametrize("heads,vdim,state,groups", [(4, 4, 64, 2), (2, 68, 128, 1), (6, 60, 128, 3), (40, 16, 64, 1)])
+def test_recurrence_in_segments(mk, ho, heads, vdim, state, groups):  # noqa: F811
+    cfg = ho.small_config(layers=[ssd(heads, vdim, state, groups)] * 2, width=36, norm={"eps": 1e-5, "groups": 1})
+    m, W = mk(cfg, seed=state + heads, chunk=600)
+    toks = tokens_for(cfg, 600, 11)
+    exp = ho.run(cfg, W, toks)[0]
+    for sizes in ([600], [7, 577], [161, 1, 1, 437], [270, 329]):
+        assert rel(in_portions(m, toks, sizes), exp) < F32_TOL
+
+
+@pytest.mark.parametrize("heads,dim,vdim", [(4, 64, 64), (3, 128, 60), (2, 64, 16), (2, 128, 12)])   # the normaliser's column: first of a CTA, last of a group, first of one, inside one
+def test_matrix_memory_in_segments(mk_netusun, no, heads, dim, vdim):  # noqa: F811
+    def edit(W):                                             # gates at the cap next to keeping everything
+        W["l0.mix.f.b"][0] = -60.0
+        W["l0.mix.i.b"][1] = 60.0
+    cfg = no.model_config([no.mem(heads=heads, dim=dim, vdim=vdim, gate_cap=40.0), no.mem(heads=heads, dim=dim, vdim=vdim)], width=40, vocab=97)
+    m, W = mk_netusun(cfg, seed=dim, chunk=500, edit=edit)
+    toks = tokens_for(cfg, 500, 9)
+    exp = no.run(cfg, W, toks)[0]
+    for sizes in ([500], [9, 480], [290, 1, 209]):
+        assert rel(in_portions(m, toks, sizes), exp) < F32_TOL
+
+
+@pytest.mark.parametrize("heads,dim,vdim", [(4, 64, 64), (3, 128, 100)])
+def test_lightning_in_segments(mk_zetivik, zo, heads, dim, vdim):  # noqa: F811
+    decay = [0.0, 1.0, 1e-20, 0.999][:heads]
+    cfg = zo.model_config([zo.light(heads=heads, dim=dim, vdim=vdim, decay=decay)], width=40, vocab=97)
+    m, W = mk_zetivik(cfg, seed=dim, chunk=500)
+    toks = tokens_for(cfg, 500, 9)
+    exp = zo.run(cfg, W, toks)[0]
+    for sizes in ([500], [9, 480], [290, 1, 209]):
         assert rel(in_portions(m, toks, sizes), exp) < F32_TOL
 
 
