@@ -375,31 +375,43 @@ struct GemmP {
 };
 enum { BAND_NONE, BAND_COLS, BAND_DEPTH };
 
+// num / (1 + e^-v) for num = 1 or v without the branch that a division has, which kept a lane's values from running next to one another: the intrinsic's reciprocal, one Newton
+// step, the quotient corrected by its remainder (exact in an fma).  What is not finite takes the intrinsic's word, denominators past its range are scaled.
+__device__ __forceinline__ float logistic_times(float v, float num) {
+  const float e = 1.f + expf(-v), s = e > 1e30f ? 5.421010862e-20f : 1.f, d = e * s, y = num * s, r0 = __fdividef(1.f, d), r = fmaf(r0, fmaf(-d, r0, 1.f), r0);   // (2^-64)
+  const float q = y * r, c = fmaf(fmaf(-d, q, y), r, q);
+  return fabsf(c) <= 3.4e38f ? c : y * r0;
+}
+// MANY: many values a thread, next to one another (logistic_times, no branches); else a thread ends one value, where the division's few instructions are faster.  Equal bits.
+template <bool MANY> __device__ __forceinline__ float logistic(float v, float num) { return MANY ? logistic_times(v, num) : num / (1.f + expf(-v)); }
 // the epilogues that join two matrices' results
-template <int EPI>
+template <int EPI, bool MANY = false>
 __device__ __forceinline__ float dual_value(const GemmP& P, float v, float v2) {
   if (EPI == HEPI_GEGLU) return gelu_tanh_f(v) * v2;
-  if (EPI == HEPI_SWIGLU) return silu_f(v) * v2;
+  if (EPI == HEPI_SWIGLU) return logistic<MANY>(v, v) * v2;
   const float g = fminf(v, P.lim), u = fminf(fmaxf(v2, -P.lim), P.lim);   // HEPI_GLU
-  return g * sigmoid_f(1.702f * g) * (u + 1.f);
+  return g * logistic<MANY>(1.702f * g, 1.f) * (u + 1.f);
 }
 // what C[row cr][n] becomes, from the result v of a single product and, for the epilogues on top of it, what C holds
-template <typename WT, int EPI>
+template <typename WT, int EPI, bool MANY = false>
 __device__ __forceinline__ float final_value(const GemmP& P, int cr, int n, float v, float old) {
   if (P.bias) v += P.bias[n];
   if (EPI == HEPI_STORE) return P.alpha * v;
   if (EPI == HEPI_ADD) return old + P.alpha * v;
-  if (EPI == HEPI_XIELU) return v > 0.f ? fmaf(P.act_a * v, v, 0.5f * v) : fmaf(P.act_b, expm1f(v) - v, 0.5f * v);
+  if (EPI == HEPI_XIELU) {
+    if (!MANY) return v > 0.f ? fmaf(P.act_a * v, v, 0.5f * v) : fmaf(P.act_b, expm1f(v) - v, 0.5f * v);
+    float e = expm1f(v > 0.f ? 0.f : v);
+    asm volatile("" : "+f"(e));
+    return fmaf(v > 0.f ? P.act_a * v : P.act_b, v > 0.f ? v : e - v, 0.5f * v);
+  }
   if (EPI == HEPI_RELU2) { const float r = fmaxf(v, 0.f); return r * r; }
-  if (EPI == HEPI_SIGMUL) return old * sigmoid_f(v);
-  if (EPI == HEPI_SILU_SIG) return n < P.aux_off ? silu_f(v) : sigmoid_f(v);
+  if (EPI == HEPI_SIGMUL) return old * logistic<MANY>(v, 1.f);
+  if (EPI == HEPI_SILU_SIG) return logistic<MANY>(v, n < P.aux_off ? v : 1.f);
   if (EPI == HEPI_SOFTCAP) return P.lim * tanhf(P.alpha * v / P.lim);
   if (EPI == HEPI_LINGATE) {
     const int hn = P.aux_off;
-    if (n < hn) return silu_f(v);
-    if (n >= 2 * hn) return v;
-    const float lo = reinterpret_cast<const float*>(P.aux)[n - hn];
-    return fmaf(1.f - lo, sigmoid_f(v), lo);
+    const float r = logistic<MANY>(v, n < hn ? v : 1.f), lo = n >= hn && n < 2 * hn ? reinterpret_cast<const float*>(P.aux)[n - hn] : 0.f;
+    return n < hn ? r : n < 2 * hn ? fmaf(1.f - lo, r, lo) : v;
   }
   const WT* aux = reinterpret_cast<const WT*>(P.aux);   // HEPI_GELU_MUL
   return gelu_tanh_f(v) * to_f<WT>(aux[(size_t)P.aux_row[cr] * P.aux_ld + P.aux_off + n]);

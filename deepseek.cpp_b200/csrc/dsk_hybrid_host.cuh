@@ -1581,7 +1581,7 @@ static void launch_tc5(State* S, int epi, const GemmP& P, int tile_cap, cudaStre
   T.stages = std::min(kTcMaxStages, kTcRing / ((kTcRows + T.bn) * kTcDepth * 2));
   T.n_mt = mt; T.rows_per_expert = P.tiles ? (int)(P.sW / P.ldw) : 0;
   T.C16 = P.C16; T.ldc16 = P.N; T.err = S->h_err;
-  T.wide = P.C16 ? P.N % 8 == 0 && (reinterpret_cast<uintptr_t>(P.C16) & 15) == 0 : P.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(P.C) & 31) == 0;
+  T.wide = P.C16 ? P.N % 4 == 0 && (reinterpret_cast<uintptr_t>(P.C16) & 7) == 0 : P.ldc % 4 == 0 && (reinterpret_cast<uintptr_t>(P.C) & 15) == 0;
   const int brows = dual ? T.bn / 2 : T.bn;
   const long long wrows = P.tiles ? (long long)T.rows_per_expert * P.n_expert : P.N;
   CUtensorMap mA, mB, mB2;

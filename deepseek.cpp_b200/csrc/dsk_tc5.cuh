@@ -2,9 +2,9 @@
 // operands, tcgen05.mma into TMEM and the epilogues of dsk_hybrid.cuh.
 //
 // One CTA per SM walks output tiles of 128 rows x bn columns (bn = 32 .. 256, picked by the host for the grid it gives).  Warp 0 copies
-// 64-deep slices of both operands into a ring of shared memory (128-byte swizzle), one thread of warp 1 issues the products, warps 2 - 5 read
-// the finished accumulators (two in TMEM: a tile's epilogue runs under the next tile's products), apply the epilogue and store: a lane its own
-// row in 32-byte pieces, ragged blocks turned through shared memory.
+// 64-deep slices of both operands into a ring of shared memory (128-byte swizzle), one thread of warp 1 issues the products, warps 2 - 9 (two a row
+// block, every second block of 32 columns) read the finished accumulators (two in TMEM: a tile's epilogue runs under the next tile's products), turn them through shared
+// memory, apply the epilogue and store 128 bytes of a row by eight lanes.
 // The activations are rounded to bf16 (as gemm_mma rounds them while staging) and, in routed products, put into expert order by one
 // pass ahead of the product (bf16_rows), or by the epilogue of the product that made them (TcP::C16): every column tile then reads half
 // the bytes, by TMA, instead of gathering and converting fp32 rows again.
@@ -12,6 +12,9 @@
 // (ring fill 1300 to 3000 cycles, 36 cycles a column to store); narrow tiles by the two issuing threads.  Those are elected lanes that count stages and parities:
 // lanes picked by number, which divided by the number of stages, took 650 cycles a slice at any width, now 535 at 256 columns, 340 at 128, 285 at 64, 270 at 32
 // (512 x 2048 x 2048: 21 -> 14.5 us, 45 x 1024 x 4096: 29 -> 17 us).
+// Epilogues: a warp a row block whose lanes each stored their own row met 32 lines a store and hid no latency, and a value's branches (a division's, expm1's, the sign's) kept
+// those of a lane from running next to one another.  Two warps, stores along rows, no branches, the same bits (2048 x 2048 x 2048 with cold operands, launch and all, us): plain 26.6 -> 24.6,
+// on top of C 32.8 -> 28.7, gate on C 57 -> 31; 512 x 8192 x 2048 xIELU 51 -> 37; 777 x 3072 x 1024 linear-recurrence gates 63 -> 31.
 #pragma once
 
 #include <cuda.h>   // CUtensorMap
@@ -21,9 +24,9 @@
 namespace dsk {
 namespace hy {
 
-constexpr int kTcRows = 128, kTcDepth = 64, kTcThreads = 192, kTcMaxStages = 10;
+constexpr int kTcRows = 128, kTcDepth = 64, kTcEpi = 8, kTcThreads = 64 + 32 * kTcEpi, kTcMaxStages = 10;   // kTcEpi: warps that finish tiles
 constexpr int kTcRing = 192 * 1024;                                  // operand ring
-constexpr int kTcTurn = 4 * 32 * 33 * 4;                             // epilogue: a 32 x 32 block per warp
+constexpr int kTcTurn = kTcEpi * 32 * 32 * 4;                           // epilogue: a 32 x 32 block per warp
 constexpr int kTcSmem = 1024 + kTcRing + kTcTurn + 256;              // (+ alignment, + barriers)
 constexpr long long kTcWaitCycles = 1ll << 32;                       // how long a wait polls a barrier before it gives up (two seconds)
 
@@ -31,7 +34,7 @@ struct TcP {
   int bn, stages, n_mt, rows_per_expert;   // column tile, ring stages, row tiles (no tile list), weight rows between experts
   __nv_bfloat16* C16;                      // non-null: results go here as bf16, row = position in the product (no c_map), pitch ldc16
   int ldc16;
-  int wide;                                // rows of C (C16) take 32-byte (16-byte) accesses at columns that are multiples of eight
+  int wide;                                // rows of C (C16) take 16-byte (8-byte) accesses at columns that are multiples of four
   int* err;                                // host-visible word: set when a wait gave up
 };
 
@@ -109,7 +112,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc5(const GemmP P, const T
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(gbase + kTcRing + kTcTurn + 16 * kTcMaxStages + 40);
   if (threadIdx.x == 0) {
     for (int s = 0; s < T.stages; s++) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, 1); }
-    for (int b = 0; b < 2; b++) { mbar_init(done0 + 8 * b, 1); mbar_init(drained0 + 8 * b, 4); }
+    for (int b = 0; b < 2; b++) { mbar_init(done0 + 8 * b, 1); mbar_init(drained0 + 8 * b, kTcEpi); }
     mbar_init(flushed0, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -181,8 +184,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc5(const GemmP P, const T
     }
     __syncwarp();
   } else {
-    const int quad = warp & 3;                               // a warp reads the TMEM lanes of its place in a group of four
-    float* turn = reinterpret_cast<float*>(gbase + kTcRing) + (warp - 2) * 32 * 33;
+    const int quad = warp & 3, first = ((warp - 2) >> 2) * 32;   // a warp reads the TMEM lanes of its place in a group of four, every second block of 32 columns
+    float* turn = reinterpret_cast<float*>(gbase + kTcRing) + (warp - 2) * 32 * 32;
     int nth = 0;
     for (int tile = blockIdx.x; tile < total; tile += gridDim.x, nth++) {
       const int buf = nth & 1, mt = row_tile(tile), n0 = column(tile);
@@ -191,34 +194,36 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc5(const GemmP P, const T
       const int mine = min(32, nrows - quad * 32);            // rows of this warp
       int cr_lane = row0 + quad * 32 + lane;
       if (!T.C16 && P.c_map && lane < mine) cr_lane = P.c_map[cr_lane];
-      // A lane has one row of the accumulator.  Where rows of C take 32-byte stores it writes its 32 columns of a block by itself; ragged blocks and
-      // odd pitches are turned through shared memory so that a warp stores along rows (turning every block and storing 64 or 128 bytes at a time was what
-      // bound a tile: the expert products of 2048 tokens took 240 + 150 us a layer, now 225 + 115).  Epilogues on top of what C holds read it a block ahead
-      // (the first under the products; a 2048 x 2048 product of 2048 tokens onto the stream: 50 -> 38 us).
-      float* crow = P.C + (lane < mine ? (size_t)cr_lane * P.ldc : 0) + n0;
-      __nv_bfloat16* crow16 = T.C16 + (lane < mine ? (size_t)cr_lane * T.ldc16 : 0) + n0;
+      // A lane has one row of the accumulator.  Blocks of 32 x 32 are turned through shared memory (16-byte pieces, piece j of row r at place j ^ (r & 7): no bank is met
+      // twice), so that eight lanes hold 128 bytes of a row.  Epilogues on top of what C holds read it a block ahead (the first under the products).
+      const int sub = lane >> 3, piece = lane & 7;           // this lane's rows 4 i + sub, columns 4 piece .. + 3 of a turned block
+      int to[8];
+#pragma unroll
+      for (int i = 0; i < 8; i++) to[i] = __shfl_sync(0xffffffffu, cr_lane, 4 * i + sub);
       constexpr bool ON_C = EPI == HEPI_ADD || EPI == HEPI_SIGMUL;
-      float held[ON_C ? 32 : 1];
+      float4 held[ON_C ? 8 : 1];
       auto fetch_c = [&](int c0) {
         if constexpr (ON_C) {
-          if (T.wide && n0 + c0 + 32 <= P.N && lane < mine) {
+          if (c0 < cols && T.wide && n0 + c0 + 32 <= P.N) {
 #pragma unroll
-            for (int q = 0; q < 32; q += 8) load8(crow + c0 + q, held + q);
+            for (int i = 0; i < 8; i++)
+              if (4 * i + sub < mine) held[i] = *reinterpret_cast<const float4*>(P.C + (size_t)to[i] * P.ldc + n0 + c0 + 4 * piece);
           }
         }
       };
-      fetch_c(0);
+      fetch_c(first);
       const bool ok = tc_wait(done0 + 8 * buf, (nth >> 1) & 1, T.err);   // (every lane polls: the loads below are warp-wide)
       if (!__all_sync(0xffffffffu, ok)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      for (int c0 = 0; c0 < cols; c0 += 32) {
+      if (first >= cols && lane == 0) tc_arrive(drained0 + 8 * buf);
+      for (int c0 = first; c0 < cols; c0 += 8 * kTcEpi) {
         uint32_t r[32];
         const uint32_t at = tmem + ((uint32_t)(quad * 32) << 16) + buf * 256 + c0;
         tc_load32(at, r);
         uint32_t r2[DUAL ? 32 : 1];
         if constexpr (DUAL) tc_load32(at + cols, r2);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (c0 + 32 >= cols) {                               // the accumulator is read: the next tile but one may have it
+        if (c0 + 8 * kTcEpi >= cols) {                             // the accumulator is read: the next tile but one may have it
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
           if (lane == 0) tc_arrive(drained0 + 8 * buf);
@@ -228,49 +233,52 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc5(const GemmP P, const T
         for (int c = 0; c < 32; c++) v[c] = __uint_as_float(r[c]);
         if constexpr (DUAL) {
 #pragma unroll
-          for (int c = 0; c < 32; c++) v[c] = dual_value<EPI>(P, v[c], __uint_as_float(r2[c]));
+          for (int c = 0; c < 32; c++) v[c] = dual_value<EPI, true>(P, v[c], __uint_as_float(r2[c]));
         }
+#pragma unroll
+        for (int j = 0; j < 8; j++) *reinterpret_cast<float4*>(turn + lane * 32 + (j ^ (lane & 7)) * 4) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        __syncwarp();
         if (T.wide && n0 + c0 + 32 <= P.N) {
-          if (lane < mine) {
-            if constexpr (!DUAL) {
+          const int n = n0 + c0 + 4 * piece;
+          float4 x[8];
 #pragma unroll
-              for (int c = 0; c < 32; c++) v[c] = final_value<__nv_bfloat16, EPI>(P, cr_lane, n0 + c0 + c, v[c], ON_C ? held[ON_C ? c : 0] : 0.f);
+          for (int i = 0; i < 8; i++) x[i] = *reinterpret_cast<const float4*>(turn + (4 * i + sub) * 32 + (piece ^ ((4 * i + sub) & 7)) * 4);
+          if constexpr (!DUAL) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+              const float4 old = ON_C ? held[ON_C ? i : 0] : make_float4(0.f, 0.f, 0.f, 0.f);
+              x[i].x = final_value<__nv_bfloat16, EPI, true>(P, to[i], n, x[i].x, old.x);
+              x[i].y = final_value<__nv_bfloat16, EPI, true>(P, to[i], n + 1, x[i].y, old.y);
+              x[i].z = final_value<__nv_bfloat16, EPI, true>(P, to[i], n + 2, x[i].z, old.z);
+              x[i].w = final_value<__nv_bfloat16, EPI, true>(P, to[i], n + 3, x[i].w, old.w);
             }
+          }
+          fetch_c(c0 + 8 * kTcEpi);
+#pragma unroll
+          for (int i = 0; i < 8; i++) {
+            if (4 * i + sub >= mine) continue;
             if (T.C16) {
-#pragma unroll
-              for (int q = 0; q < 32; q += 8) {
-                uint4 o;
-                uint32_t* w = reinterpret_cast<uint32_t*>(&o);
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                  const __nv_bfloat162 pr = __floats2bfloat162_rn(v[q + 2 * u], v[q + 2 * u + 1]);
-                  w[u] = *reinterpret_cast<const uint32_t*>(&pr);
-                }
-                *reinterpret_cast<uint4*>(crow16 + c0 + q) = o;
-              }
+              const __nv_bfloat162 lo = __floats2bfloat162_rn(x[i].x, x[i].y), hi = __floats2bfloat162_rn(x[i].z, x[i].w);
+              *reinterpret_cast<uint2*>(T.C16 + (size_t)to[i] * T.ldc16 + n) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
             } else {
-              if (c0 + 32 < cols) fetch_c(c0 + 32);
-#pragma unroll
-              for (int q = 0; q < 32; q += 8) store8(crow + c0 + q, v + q);
+              *reinterpret_cast<float4*>(P.C + (size_t)to[i] * P.ldc + n) = x[i];
             }
           }
         } else {
-#pragma unroll
-          for (int c = 0; c < 32; c++) turn[lane * 33 + c] = v[c];
-          __syncwarp();
           const int n = n0 + c0 + lane;
 #pragma unroll 4
           for (int i = 0; i < 32; i++) {
             const int cr = __shfl_sync(0xffffffffu, cr_lane, i);
             if (i < mine && n < P.N) {
               float* c = P.C + (size_t)cr * P.ldc + n;
-              const float old = ON_C ? *c : 0.f, x = DUAL ? turn[i * 33 + lane] : final_value<__nv_bfloat16, EPI>(P, cr, n, turn[i * 33 + lane], old);
+              const float got = turn[i * 32 + ((lane >> 2) ^ (i & 7)) * 4 + (lane & 3)], old = ON_C ? *c : 0.f;
+              const float x = DUAL ? got : final_value<__nv_bfloat16, EPI, true>(P, cr, n, got, old);
               if (T.C16) T.C16[(size_t)cr * T.ldc16 + n] = __float2bfloat16_rn(x);
               else *c = x;
             }
           }
-          __syncwarp();
         }
+        __syncwarp();
       }
     }
   }

@@ -5,10 +5,12 @@ import numpy as np
 import pytest
 
 import test_gpu_netusun as netusun
+import test_gpu_rutulix as rutulix
 from test_gpu_hybrid import F32_TOL, att_layer, ho, mk, model_cfg, rel, ssd_layer, tokens_for  # noqa: F401
 from test_gpu_netusun import no  # noqa: F401
+from test_gpu_rutulix import ro  # noqa: F401
 
-mk_netusun = netusun.mk
+mk_netusun, mk_rutulix = netusun.mk, rutulix.mk
 
 pytestmark = pytest.mark.gpu
 
@@ -45,3 +47,22 @@ def test_norms_of_closing_blocks(mk_netusun, no, width):  # noqa: F811
     toks = tokens_for(cfg, 21, 5)
     exp = no.run(cfg, W, toks)
     assert rel(m.forward_chunk(toks, 0, range(21)), exp[0] if isinstance(exp, tuple) else exp) < F32_TOL
+
+
+# ends of column tiles of bf16 products on the tensor cores: last blocks of 4, 8 and 28 columns, of an odd number, tiles of one block and of several for the two warps that share a row
+# block's columns; plain, gated, on top of the rows, gates on what lies there
+@pytest.mark.parametrize("width,ff,vocab,tokens", [(40, 36, 131, 33), (72, 132, 132, 129), (136, 100, 260, 200), (520, 284, 97, 70)])
+def test_ends_of_column_tiles(mk_netusun, no, width, ff, vocab, tokens):  # noqa: F811
+    cfg = no.model_config([no.att(heads=3, dim=12, vdim=12, size=40, mlp=no.dense(ff)), no.mem(heads=2, dim=9, vdim=14, mlp=no.moe(5, 2, ff + 4, shared=ff)), no.lat(mlp=no.dense(ff + 1))],
+                          width=width, vocab=vocab)
+    m, W = mk_netusun(cfg, seed=ff, chunk=256, quant="bf16")
+    toks = tokens_for(cfg, tokens, 3)
+    assert netusun.close_bf16(m.forward_chunk(toks, 0, range(tokens)), no.run(cfg, W, toks)[0], no.rounding_noise(cfg, W, toks))
+
+
+@pytest.mark.parametrize("width,ff,tokens", [(40, 36, 45), (72, 260, 130), (136, 1028, 200)])   # xIELU: activations without a branch, rounded as they are stored
+def test_activations_of_column_tiles(mk_rutulix, ro, width, ff, tokens):  # noqa: F811
+    cfg = ro.model_config([ro.att(ff=ff), ro.att(heads=4, dim=10, ff=ff + 8)], width=width, vocab=131)
+    m, W = mk_rutulix(cfg, seed=ff, chunk=256, quant="bf16")
+    toks = tokens_for(cfg, tokens, 3)
+    assert rutulix.close_bf16(m.forward_chunk(toks, 0, range(tokens)), ro.run(cfg, W, toks)[0])
