@@ -228,11 +228,14 @@ __global__ void __launch_bounds__(256) group_rmsnorm(const float* __restrict__ i
 #pragma unroll
     for (int k = 0; k < 16; k++) {
       const int i = threadIdx.x + 256 * k;
-      if (i < n) {
-        if (o16) o16[(size_t)t * n + i] = __float2bfloat16_rn(v[k] * sc * gt[k]);
-        else o[i] = from_f<OT>(mode == 0 ? v[k] * sc * gt[k] : to_f<OT>(o[i]) + alpha * (v[k] * sc * gt[k]));
-      }
+      if (i < n && !o16) o[i] = from_f<OT>(mode == 0 ? v[k] * sc * gt[k] : to_f<OT>(o[i]) + alpha * (v[k] * sc * gt[k]));
     }
+    if (o16)
+#pragma unroll
+      for (int k = 0; k < 16; k++) {
+        const int i = threadIdx.x + 256 * k;
+        if (i < n) o16[(size_t)t * n + i] = __float2bfloat16_rn(v[k] * sc * gt[k]);
+      }
     return;
   }
   // a CTA per group, everything it reads in flight ahead of the sum (a decoded token's 4 groups one after the other, each with two waits for
@@ -1849,7 +1852,10 @@ __global__ void __launch_bounds__(256) rms_open(float* __restrict__ x, const flo
   }
   const float sc = 1.f / sqrtf(block_sum(ss, red) / (float)n + eps);
 #pragma unroll
-  for (int k = 0; k < kLnRegs; k++) { const int i = threadIdx.x + 256 * k; if (i < n) { hr[i] = v[k] * sc * wt[k]; if (h16) h16[(size_t)blockIdx.x * n + i] = __float2bfloat16_rn(v[k] * sc * wt[k]); } }
+  for (int k = 0; k < kLnRegs; k++) { const int i = threadIdx.x + 256 * k; if (i < n) hr[i] = v[k] * sc * wt[k]; }
+  if (h16)                                                   // (a loop of its own: a decoded token has none)
+#pragma unroll
+    for (int k = 0; k < kLnRegs; k++) { const int i = threadIdx.x + 256 * k; if (i < n) h16[(size_t)blockIdx.x * n + i] = __float2bfloat16_rn(v[k] * sc * wt[k]); }
   for (int i = threadIdx.x + 256 * kLnRegs; i < n; i += 256) { hr[i] = xr[i] * sc * w[i]; if (h16) h16[(size_t)blockIdx.x * n + i] = __float2bfloat16_rn(xr[i] * sc * w[i]); }
 }
 
@@ -1914,7 +1920,10 @@ __global__ void __launch_bounds__(NT) rms_add_norm(const float* __restrict__ y, 
   if (!wh) return;
   sc = 1.f / sqrtf(block_sum(ss, red) / (float)n + eps);
 #pragma unroll
-  for (int k = 0; k < KR; k++) { const int i = threadIdx.x + NT * k; if (i < n) { const float r = u[k] * sc * (EARLY ? b_w[EARLY ? k : 0] : wh[i]); h[t * n + i] = r; if (h16) h16[t * n + i] = __float2bfloat16_rn(r); } }
+  for (int k = 0; k < KR; k++) { const int i = threadIdx.x + NT * k; if (i < n) { u[k] = u[k] * sc * (EARLY ? b_w[EARLY ? k : 0] : wh[i]); h[t * n + i] = u[k]; } }
+  if (h16)
+#pragma unroll
+    for (int k = 0; k < KR; k++) { const int i = threadIdx.x + NT * k; if (i < n) h16[t * n + i] = __float2bfloat16_rn(u[k]); }
 }
 
 // the T rows of a step (pitch ls) copied to rows of pitch ld
