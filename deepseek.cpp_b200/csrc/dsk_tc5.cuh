@@ -9,7 +9,7 @@
 // pass ahead of the product (bf16_rows), or by the epilogue of the product that made them (TcP::C16): every column tile then reads half
 // the bytes, by TMA, instead of gathering and converting fp32 rows again.
 // Bound: large products by the tensor pipe (2048 x 8192 x 8192: 1325 TFLOP/s, a 64-deep slice 640 cycles); one-tile grids by what is not under the products
-// (ring fill 1300 to 3000 cycles, 36 cycles a column to store); narrow tiles by the two issuing threads.  Those are elected lanes that count stages and parities:
+// (ring fill 1300 to 3000 cycles, the one epilogue); narrow tiles by the two issuing threads.  Those are elected lanes that count stages and parities:
 // lanes picked by number, which divided by the number of stages, took 650 cycles a slice at any width, now 535 at 256 columns, 340 at 128, 285 at 64, 270 at 32
 // (512 x 2048 x 2048: 21 -> 14.5 us, 45 x 1024 x 4096: 29 -> 17 us).
 // Epilogues: a warp a row block whose lanes each stored their own row met 32 lines a store and hid no latency, and a value's branches (a division's, expm1's, the sign's) kept
