@@ -1807,10 +1807,11 @@ static void launch_lin_mma(LinMmaP p, int N, int nseg, cudaStream_t st) {
 
 // the walk over the blocks of a step (lin_scan): lanes per channel group by the key size, warps per CTA by how many CTAs there are
 static void launch_lin_scan(bool delta, const float* q, const float* k, int ldq, int hs, int rep, const float* v, int ldv, const float* rec, float* state,
-                            float* out, int ldo, int T, int H, int N, int P, cudaStream_t st, float* seg, float* nst = nullptr, float* den = nullptr, int sn = 0, int sp = 1) {
+                            float* out, int ldo, int T, int H, int N, int P, cudaStream_t st, State* S, float* nst = nullptr, float* den = nullptr, int sn = 0, int sp = 1) {
   if (!sn) sn = P;                    // state rows [N][P] of a head, unless said otherwise
-  if (const int n = delta ? 0 : lin_mma_segments(q, k, ldq, hs, v, ldv, T, H, N, P, nst != nullptr, seg)) {
-    launch_lin_mma(LinMmaP{q, k, v, rec, state, out, nst, den, seg, ldq, hs, rep, ldv, ldo, T, H, P, sn, sp, (P + (nst ? 1 : 0) + 15) / 16, n, 0, 0}, N, n, st);
+  if (const int n = delta ? 0 : lin_mma_segments(q, k, ldq, hs, v, ldv, T, H, N, P, nst != nullptr, S->lseg)) {
+    if (n > 1) S->launches++;                // (callers count one)
+    launch_lin_mma(LinMmaP{q, k, v, rec, state, out, nst, den, S->lseg, ldq, hs, rep, ldv, ldo, T, H, P, sn, sp, (P + (nst ? 1 : 0) + 15) / 16, n, 0, 0}, N, n, st);
     return;
   }
   const int TPC = N <= 32 ? 8 : N <= 64 ? 16 : 32, RQ = N <= 128 ? 1 : 2;
@@ -1855,7 +1856,7 @@ static void gdn_forward(State* S, const HLayer& L, LayerState& ls, int ldp, cons
   const int nb = (T + kLinBlk - 1) / kLinBlk;
   const size_t smem = (size_t)(2 * kLinBlk * (NP + 4) + 2 * kLinBlk * kLinBlk + 8 * kLinBlk * kLinBlk) * 4;
   launch_next(gdn_prepare, dim3((unsigned)nb, (unsigned)(G + (RV + 255) / 256)), 256, smem, st)(D, S->lq, S->lk, S->lv, NP, S->lrec);
-  launch_lin_scan(true, S->lq, S->lk, G * NP, NP, H / G, S->lv, RV, S->lrec, ls.lin, S->lout, RV, T, H, N, P, st, nullptr);
+  launch_lin_scan(true, S->lq, S->lk, G * NP, NP, H / G, S->lv, RV, S->lrec, ls.lin, S->lout, RV, T, H, N, P, st, S);
   if (sp.gdn_conv > 1) { launch_next(conv_ring_store, (CH + 127) / 128, 128, 0, st)(S->b0, ldp, (int)a.dq, ls.hist, D.ring, T, CH, sp.gdn_conv, S->d_ctl); S->launches++; }
   launch_next(head_rmsnorm, (unsigned)(((long long)T * H + 7) / 8), 256, 0, st)(S->lout, RV, L.lin_norm, out, ldo, T, H, P, eps, S->b0 + a.dg, ldp, alpha, 0, 0, nullptr, nullptr, out16);
   S->launches += 3;
@@ -1872,7 +1873,7 @@ static void lightning_forward(State* S, const HLayer& L, LayerState& ls, int ldp
     return;
   }
   launch_next(lin_gram, dim3((unsigned)((T + kLinBlk - 1) / kLinBlk), (unsigned)H), 256, (size_t)2 * kLinBlk * (((N + 3) & ~3) + 4) * 4, st)(S->b0, S->b0 + HN, ldp, L.log_decay, T, H, N, S->lrec);
-  launch_lin_scan(false, S->b0, S->b0 + HN, ldp, N, 1, S->b0 + 2 * HN, ldp, S->lrec, ls.lin, S->lout, HP, T, H, N, P, st, S->lseg);
+  launch_lin_scan(false, S->b0, S->b0 + HN, ldp, N, 1, S->b0 + 2 * HN, ldp, S->lrec, ls.lin, S->lout, HP, T, H, N, P, st, S);
   S->launches += 2;
 }
 
@@ -1890,7 +1891,7 @@ static void mlstm_forward(State* S, const HLayer& L, LayerState& ls, int ldp, co
   float *gi = S->lgate, *gf = gi + (size_t)H * T, *gm = gf + (size_t)H * T;
   launch_next(mlstm_gates, H, 256, 0, st)(S->b0, ldp, (int)a.i, (int)a.f, sp.lin_gate_cap, T, H, gi, gf, gm, mst);
   launch_next(mlstm_gram, dim3((unsigned)((T + kLinBlk - 1) / kLinBlk), (unsigned)H), 256, (size_t)2 * kLinBlk * (((N + 3) & ~3) + 4) * 4, st)(S->b0, S->b0 + HN, ldp, gi, gf, gm, T, H, N, S->lrec);
-  launch_lin_scan(false, S->b0, S->b0 + HN, ldp, N, 1, S->b0 + 2 * HN, ldp, S->lrec, ls.lin, S->lout, HP, T, H, N, P, st, S->lseg, nst, S->lden);
+  launch_lin_scan(false, S->b0, S->b0 + HN, ldp, N, 1, S->b0 + 2 * HN, ldp, S->lrec, ls.lin, S->lout, HP, T, H, N, P, st, S, nst, S->lden);
   launch_next(head_rmsnorm, (unsigned)(((long long)T * H + 7) / 8), 256, 0, st)(S->lout, HP, L.mnorm, out, HP, T, H, P, eps, S->b0 + a.g, ldp, 1.f, P, 1, S->lden, gm, out16);
   S->launches += 4;
 }
@@ -2501,7 +2502,7 @@ static int enqueue_chunk(dsk_model* m, dsk_state* s, int T, int n_want, float* t
         const int H = sp.ssm_heads, N = sp.ssm_state, P = sp.ssm_vdim, G = sp.ssm_groups;
         launch_next(ssd_gram, dim3((unsigned)((T + kLinBlk - 1) / kLinBlk), (unsigned)G), 256, ssd_gram_smem(sp), st)(
             S->b1 + inner + G * N, S->b1 + inner, ch, S->b0 + inner + ch, pw, L.dt_bias, L.A_log, T, H, N, H / G, S->lrec);
-        launch_lin_scan(false, S->b1 + inner + G * N, S->b1 + inner, ch, N, H / G, S->b1, ch, S->lrec, ls.ssm, S->b2, inner, T, H, N, P, st, S->lseg, nullptr, nullptr, 1, N);
+        launch_lin_scan(false, S->b1 + inner + G * N, S->b1 + inner, ch, N, H / G, S->b1, ch, S->lrec, ls.ssm, S->b2, inner, T, H, N, P, st, S, nullptr, nullptr, 1, N);
         if (inner % 4 == 0 && ch % 4 == 0 && pw % 4 == 0 && P % 4 == 0)
           launch_next(ssd_gate<4>, dim3((unsigned)T, (unsigned)((inner + 1023) / 1024)), 256, 0, st)(S->b2, S->b1, ch, S->b0, pw, L.D, inner, P);
         else launch_next(ssd_gate<1>, dim3((unsigned)T, (unsigned)((inner + 255) / 256)), 256, 0, st)(S->b2, S->b1, ch, S->b0, pw, L.D, inner, P);
