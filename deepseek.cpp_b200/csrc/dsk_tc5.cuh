@@ -192,8 +192,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc5(const GemmP P, const T
       int row0 = mt * kTcRows, nrows = min(kTcRows, P.M - row0);
       if (P.tiles) { const int4 t = P.tiles[mt]; row0 = t.y; nrows = t.z; }
       const int mine = min(32, nrows - quad * 32);            // rows of this warp
-      int cr_lane = row0 + quad * 32 + lane;
-      if (!T.C16 && P.c_map && lane < mine) cr_lane = P.c_map[cr_lane];
+      // (lanes behind the last row have the first one's: epilogues look up what belongs to a row ahead of asking whether the row is stored)
+      int cr_lane = row0 + (lane < mine ? quad * 32 + lane : 0);
+      if (!T.C16 && P.c_map) cr_lane = P.c_map[cr_lane];
       // A lane has one row of the accumulator.  Blocks of 32 x 32 are turned through shared memory (16-byte pieces, piece j of row r at place j ^ (r & 7): no bank is met
       // twice), so that eight lanes hold 128 bytes of a row.  Epilogues on top of what C holds read it a block ahead (the first under the products).
       const int sub = lane >> 3, piece = lane & 7;           // this lane's rows 4 i + sub, columns 4 piece .. + 3 of a turned block

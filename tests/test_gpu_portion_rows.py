@@ -6,7 +6,7 @@ import pytest
 
 import test_gpu_netusun as netusun
 import test_gpu_rutulix as rutulix
-from test_gpu_hybrid import F32_TOL, att_layer, ho, mk, model_cfg, rel, ssd_layer, tokens_for  # noqa: F401
+from test_gpu_hybrid import F32_TOL, att_layer, close_bf16, ho, mk, model_cfg, rel, ssd_layer, tokens_for  # noqa: F401
 from test_gpu_netusun import no  # noqa: F401
 from test_gpu_rutulix import ro  # noqa: F401
 
@@ -66,3 +66,13 @@ def test_activations_of_column_tiles(mk_rutulix, ro, width, ff, tokens):  # noqa
     m, W = mk_rutulix(cfg, seed=ff, chunk=256, quant="bf16")
     toks = tokens_for(cfg, tokens, 3)
     assert rutulix.close_bf16(m.forward_chunk(toks, 0, range(tokens)), ro.run(cfg, W, toks)[0])
+
+
+# a gate whose values are looked up by a row's token, more columns than the narrow products take: rows past the portion's end belong to no token (portions of a few rows, of a tile
+# less one, of a row more, smaller than the chunk; fewer tokens in the vocabulary than rows in a chunk)
+@pytest.mark.parametrize("width,side,vocab,tokens,chunk", [(40, 104, 31, 40, 60), (64, 100, 53, 5, 8), (72, 256, 53, 127, 200), (40, 128, 97, 129, 129)])
+def test_rows_looked_up_by_token(mk, ho, width, side, vocab, tokens, chunk):  # noqa: F811
+    cfg = model_cfg([ssd_layer(heads=2, vdim=8, state=8), att_layer()], width=width, vocab=vocab, side=side)
+    m, W = mk(cfg, seed=side, chunk=chunk, quant="bf16")
+    toks = tokens_for(cfg, tokens, 3)
+    assert close_bf16(m.forward_chunk(toks, 0, range(tokens)), ho.run(cfg, W, toks)[0])
