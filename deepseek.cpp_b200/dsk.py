@@ -7,6 +7,7 @@ machine without libdsk.so, or calling it without a GPU, raises — there is no C
 """
 from __future__ import annotations
 
+import collections
 import ctypes as C
 import os
 import subprocess
@@ -584,49 +585,78 @@ class _Results:
     LEAST, UNIT, MOST = 64 << 10, 4 << 10, 8 << 20
 
     def __init__(self, L, nbytes: int):
-        self.L, self.lock, self.closed, self.live = L, threading.RLock(), False, 0
+        self.L, self.lock, self.closed = L, threading.Lock(), False
         nbytes = -(-min(nbytes, self.MOST) // self.UNIT) * self.UNIT if nbytes >= self.LEAST else 0
         self.base = L.dsk_host_alloc(nbytes) if nbytes else None
-        self.holes = [(0, nbytes)] if self.base else []              # (offset, bytes), ascending
+        self._holes = [(0, nbytes)] if self.base else []             # (offset, bytes), ascending; changed under the lock alone
+        self._live = 0
+        self._back = collections.deque()                             # parts that came back: a finaliser may run at any point of any thread, also inside rows(), and only appends
 
     def rows(self, shape):
         """An array that the caller writes all of."""
         need = int(np.prod(shape)) * 4
         size, at = -(-need // self.UNIT) * self.UNIT, None
-        if need >= self.LEAST:
+        if need >= self.LEAST and not self.closed:
             with self.lock:
-                i = next((i for i, h in enumerate(self.holes) if h[1] >= size), None)
+                self._drain()
+                i = next((i for i, h in enumerate(self._holes) if h[1] >= size), None)
                 if i is not None and not self.closed:
-                    at, room = self.holes[i]
-                    self.holes[i:i + 1] = [(at + size, room - size)] if room > size else []
-                    self.live += 1
+                    at, room = self._holes[i]
+                    self._holes[i:i + 1] = [(at + size, room - size)] if room > size else []
+                    self._live += 1
+            if self.closed:
+                self._settle()
         if at is None:
             return np.empty(shape, dtype=np.float32)
         raw = (C.c_float * (need // 4)).from_address(self.base + at)
-        weakref.finalize(raw, self._back, at, size).atexit = False
+        weakref.finalize(raw, self._came_back, at, size).atexit = False
         return np.frombuffer(raw, dtype=np.float32).reshape(shape)
 
-    def _back(self, at, size):
-        with self.lock:
-            self.live -= 1
+    def _came_back(self, at, size):
+        self._back.append((at, size))
+        if self.closed:
+            self._settle()
+
+    def _drain(self):
+        """What came back joins the holes; behind a closed model the last part gives the memory back.  Under the lock."""
+        while self._back:
+            self._live -= 1
             merged = []
-            for h in sorted(self.holes + [(at, size)]):
+            for h in sorted(self._holes + [self._back.popleft()]):
                 if merged and sum(merged[-1]) == h[0]:
                     merged[-1] = (merged[-1][0], merged[-1][1] + h[1])
                 else:
                     merged.append(h)
-            self.holes = merged
-            self._give_back()
-
-    def _give_back(self):
-        if self.closed and not self.live and self.base:
+            self._holes = merged
+        if self.closed and not self._live and self.base:
             self.L.dsk_host_free(self.base)
-            self.base, self.holes = None, []
+            self.base, self._holes = None, []
+
+    def _settle(self):
+        """Drains now, unless somebody is at it, who then looks again behind the lock."""
+        while self.lock.acquire(blocking=False):
+            try:
+                self._drain()
+            finally:
+                self.lock.release()
+            if not self._back:
+                return
+
+    @property
+    def holes(self):
+        self._settle()
+        return list(self._holes)
+
+    @property
+    def live(self):
+        self._settle()
+        return self._live
 
     def close(self):
+        self.closed = True
         with self.lock:
-            self.closed = True
-            self._give_back()
+            self._drain()
+        self._settle()
 
 
 class Model:
