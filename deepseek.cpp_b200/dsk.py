@@ -793,7 +793,8 @@ class Model:
         rows [len(want), vocab] (and, with layers=True, the residual stream after every layer run [layer runs, n, dim])."""
         tok = np.ascontiguousarray(tokens, dtype=np.int32)
         w = np.ascontiguousarray(list(want), dtype=np.int32)
-        out = self._results.rows((len(w), self.cfg.vocab_size))
+        shape = (len(w), self.cfg.vocab_size)
+        out = self._results.rows(shape) if self._results else np.empty(shape, dtype=np.float32)   # (a model that is not finished: the library's to refuse)
         tr = np.zeros((self.L.dsk_model_layer_runs(self.h), len(tok), self.cfg.dim), dtype=np.float32) if layers else None
         _ck(self.L.dsk_forward_chunk(self.h, state or self.s, tok.ctypes.data_as(i32p), len(tok), pos0,
                                      w.ctypes.data_as(i32p) if len(w) else None, len(w),

@@ -50,3 +50,13 @@ def test_memory_is_bounded_and_given_back(mk, no):  # noqa: F811
     m._logits = None
     gc.collect()
     assert r.base is None
+
+
+def test_model_that_is_not_finished(no):  # noqa: F811
+    import dsk
+    cfg = no.model_config([no.att()], width=40, vocab=97)
+    hc, specs = dsk.ARCHITECTURES[cfg["architecture"]](cfg, quant="fp32", max_seq_len=64, chunk=16)
+    m = dsk.Model(hc, device=0, layers=specs)
+    with pytest.raises(dsk.DskError):
+        m.forward_chunk([1, 2, 3], 0, range(3))
+    m.close()
