@@ -69,6 +69,7 @@ __global__ void __launch_bounds__(kLmThreads, 1) lin_mma(const LinMmaP P) {
   const int nb = (P.T + C - 1) / C, b0 = seg * P.per, b1 = min(nb, b0 + P.per);
   const bool outputs = P.mode == 1;
   if (threadIdx.x < 2) bad[threadIdx.x] = -1;
+  __syncthreads();                                           // (the staging warps mark the first block ahead of the barrier that all meet on)
   grid_enter();
   if (warp >= 2 * kLmGroups) {
     const int st = threadIdx.x - 64 * kLmGroups;

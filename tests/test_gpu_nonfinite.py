@@ -6,6 +6,8 @@ import pytest
 from test_gpu_hybrid import ho  # noqa: F401
 from test_gpu_hybrid import mk as mk_hybrid  # noqa: F401
 from test_gpu_netusun import F32_TOL, in_portions, mk, no, rel, tokens_for  # noqa: F401
+from test_gpu_zetivik import mk as mk_zetivik  # noqa: F401
+from test_gpu_zetivik import zo  # noqa: F401
 
 pytestmark = pytest.mark.gpu
 
@@ -141,6 +143,66 @@ def test_recurrence_in_segments(mk_hybrid, ho, value):  # noqa: F811
         t[at] = 50
         m.reset()
         assert ahead_of_the_poison(m, ho.run, cfg, W, t, at, [400]) < F32_TOL
+    m.reset()
+
+
+def segments_model(kind, mk, no, mk_zetivik, zo, edit):  # noqa: F811
+    """Recurrences whose walks run in segments on the tensor cores: (oracle's run, config, model, weights)."""
+    if kind.startswith("lightning"):
+        heads, dim, vdim = (3, 64, 20) if kind == "lightning_64" else (2, 128, 68)
+        cfg = zo.model_config([zo.light(heads=heads, dim=dim, vdim=vdim, decay=[0.999, 1.0, 0.5][:heads])], width=40, vocab=97)
+        return (zo.run, cfg) + mk_zetivik(cfg, seed=4, chunk=500, edit=edit)
+    heads, dim, vdim = (3, 64, 64) if kind == "matrix_64" else (2, 128, 12)
+    cfg = no.model_config([no.mem(heads=heads, dim=dim, vdim=vdim)], width=40, vocab=97)
+    return (no.run, cfg) + mk(cfg, seed=4, chunk=500, edit=edit)
+
+
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+@pytest.mark.parametrize("kind", ["lightning_64", "lightning_128", "matrix_64", "matrix_128"])
+def test_walks_in_segments(mk, no, mk_zetivik, zo, kind, value):  # noqa: F811
+    run, cfg, m, W = segments_model(kind, mk, no, mk_zetivik, zo, lambda W: poisoned(W, value, 50))
+    toks = tokens_for(cfg, 500, 5)
+    toks[toks == 50] = 7
+    for at in (1, 66, 200, 499):
+        t = toks.copy()
+        t[at] = 50
+        m.reset()
+        assert ahead_of_the_poison(m, run, cfg, W, t, at, [500]) < F32_TOL
+    m.reset()
+
+
+@pytest.mark.parametrize("kind", ["lightning_64", "lightning_128", "matrix_64", "matrix_128"])
+def test_values_past_bfloat16_in_segments(mk, no, mk_zetivik, zo, kind):  # noqa: F811
+    """One value of one token next to the largest fp32 number, finite but an infinity in bfloat16, against keys and queries so small that what it leaves in the state
+    is ordinary: blocks with such a value update the state by fused multiply-adds, the first one of a segment too."""
+    largest = 3.3985e38                                      # (bfloat16 rounds to an infinity from 3.3962e38 on)
+
+    def edit(W):
+        W["embed"] = np.array(W["embed"])
+        W["embed"][:, 3] = W["embed"][:, 5] = 0.0            # columns that token 50 has to itself: the value's weights read nothing else
+        W["embed"][50, 3], W["embed"][50, 5] = 3.0, 0.125
+        h = zo.rms(W["embed"][50], cfg_eps) * (1.0 + W["l0.norm1"] if kind.startswith("lightning") else W["l0.norm1"])
+        for n in "qk":
+            W["l0.mix." + n] = W["l0.mix." + n] * 1e-18
+        v = np.array(W["l0.mix.v"])
+        v[2] = 0.0
+        v[2, 3] = zo.bf16_to_f64(zo.to_bf16(np.array([0.995 * largest / h[3]])))[0]
+        v[2, 5] = (largest - v[2, 3] * h[3]) / h[5]
+        W["l0.mix.v"] = v
+        if kind.startswith("matrix"):
+            W["l0.mix.f.b"] = W["l0.mix.f.b"] * 0.0 + 8.0    # (kept for the rest of the sequence)
+    cfg_eps = 1e-5
+    run, cfg, m, W = segments_model(kind, mk, no, mk_zetivik, zo, edit)
+    assert cfg["norm"]["eps"] == cfg_eps
+    toks = tokens_for(cfg, 500, 5)
+    toks[toks == 50] = 7
+    for at in (2, 64, 130, 260, 450):
+        t = toks.copy()
+        t[at] = 50
+        exp = run(cfg, W, t)[0]
+        assert np.all(np.isfinite(exp))
+        m.reset()
+        assert rel(in_portions(m, t, [500]), exp) < F32_TOL
     m.reset()
 
 
