@@ -2158,6 +2158,19 @@ extern "C" int dsk_dequantize_row(int quant, const void* blocks, int k, float* o
   return 0;
 }
 
+extern "C" int dsk_logistic(const float* v, int n, int times_v, float* out_many, float* out_plain) {
+  if (need_device()) return -1;
+  if (!v || n <= 0 || !out_many || !out_plain) return fail(-1, "bad arguments");
+  Tmp t;
+  float *dv = t.up<float>(v, n), *dm = t.up<float>(nullptr, n), *dp = t.up<float>(nullptr, n);
+  if (!dv || !dm || !dp) return fail(-2, "allocation failed");
+  hy::logistic_values<<<(unsigned)(((size_t)n + 255) / 256), 256>>>(dv, n, times_v, dm, dp);
+  CK(cudaGetLastError());
+  CK(cudaMemcpy(out_many, dm, (size_t)n * 4, cudaMemcpyDeviceToHost));
+  CK(cudaMemcpy(out_plain, dp, (size_t)n * 4, cudaMemcpyDeviceToHost));
+  return 0;
+}
+
 // rope / rope_v3 on one head's rotary slice (the reference always calls them with d == head_dim == qk_rope_head_dim,
 // src/infer.cpp:956-972): run as the RoPE prologue of the attention stage on a head with no `nope` part
 extern "C" int dsk_rope(float* vec, int d, int head_dim, int pos, float theta, int v3) {

@@ -378,15 +378,22 @@ struct GemmP {
 };
 enum { BAND_NONE, BAND_COLS, BAND_DEPTH };
 
-// num / (1 + e^-v) for num = 1 or v without the branch that a division has, which kept a lane's values from running next to one another: the intrinsic's reciprocal, one Newton
-// step, the quotient corrected by its remainder (exact in an fma).  What is not finite takes the intrinsic's word, denominators past its range are scaled.
+// num / (1 + e^-v) for num = 1 or v without the branch that a division has, which kept a lane's values from running next to one another: a quotient by iterative refinement.
+// r is the intrinsic's reciprocal, documented to be within two last places (2^-22) for denominators up to 2^126; larger ones are scaled by 2^-64, and num with them.
+// q = num r is off by about as much, its residual num - q d is exact in one fma, and q + residual r is off by 2^-43 of itself ahead of its one rounding: half a last
+// place and 2^-19 of one.  Where that is not finite (an infinite num or denominator, NaN), q has what the division has.
 __device__ __forceinline__ float logistic_times(float v, float num) {
-  const float e = 1.f + expf(-v), s = e > 1e30f ? 5.421010862e-20f : 1.f, d = e * s, y = num * s, r0 = __fdividef(1.f, d), r = fmaf(r0, fmaf(-d, r0, 1.f), r0);   // (2^-64)
-  const float q = y * r, c = fmaf(fmaf(-d, q, y), r, q);
-  return fabsf(c) <= 3.4e38f ? c : y * r0;
+  const float e = 1.f + expf(-v), s = e > 0x1p100f ? 0x1p-64f : 1.f, d = e * s, y = num * s, r = __fdividef(1.f, d), q = y * r;
+  const float c = fmaf(fmaf(-d, q, y), r, q);
+  return fabsf(c) <= 3.4e38f ? copysignf(c, num) : q;        // (the residual of -0 is +0)
 }
-// MANY: many values a thread, next to one another (logistic_times, no branches); else a thread ends one value, where the division's few instructions are faster.  Equal bits.
+// MANY: many values a thread, next to one another (logistic_times, no branches); else a thread ends one value, where the division's few instructions are faster.
 template <bool MANY> __device__ __forceinline__ float logistic(float v, float num) { return MANY ? logistic_times(v, num) : num / (1.f + expf(-v)); }
+// out[i] = 1 / (1 + e^-v[i]), or v[i] times that, as MANY and as the division
+__global__ void logistic_values(const float* __restrict__ v, int n, int times_v, float* __restrict__ many, float* __restrict__ plain) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) { many[i] = logistic<true>(v[i], times_v ? v[i] : 1.f); plain[i] = logistic<false>(v[i], times_v ? v[i] : 1.f); }
+}
 // the epilogues that join two matrices' results
 template <int EPI, bool MANY = false>
 __device__ __forceinline__ float dual_value(const GemmP& P, float v, float v2) {

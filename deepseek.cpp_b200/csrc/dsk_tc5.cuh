@@ -13,7 +13,7 @@
 // lanes picked by number, which divided by the number of stages, took 650 cycles a slice at any width, now 535 at 256 columns, 340 at 128, 285 at 64, 270 at 32
 // (512 x 2048 x 2048: 21 -> 14.5 us, 45 x 1024 x 4096: 29 -> 17 us).
 // Epilogues: a warp a row block whose lanes each stored their own row met 32 lines a store and hid no latency, and a value's branches (a division's, expm1's, the sign's) kept
-// those of a lane from running next to one another.  Two warps, stores along rows, no branches, the same bits (2048 x 2048 x 2048 with cold operands, launch and all, us): plain 26.6 -> 24.6,
+// those of a lane from running next to one another.  Two warps, stores along rows, no branches (2048 x 2048 x 2048 with cold operands, launch and all, us): plain 26.6 -> 24.6,
 // on top of C 32.8 -> 28.7, gate on C 57 -> 31; 512 x 8192 x 2048 xIELU 51 -> 37; 777 x 3072 x 1024 linear-recurrence gates 63 -> 31.
 #pragma once
 

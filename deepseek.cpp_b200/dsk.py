@@ -974,6 +974,15 @@ def rope(vec, head_dim, pos, theta, v3):
     return v
 
 
+def logistic(v, times_v):
+    """(1 / (1 + e^-v), or v times that, as the ends of matrix products take it, many values a thread; the same by a division)"""
+    init(_inited or 0)
+    v = np.ascontiguousarray(v, dtype=np.float32)
+    many, plain = np.zeros_like(v), np.zeros_like(v)
+    _ck(lib().dsk_logistic(_fp(v), v.size, int(times_v), _fp(many), _fp(plain)))
+    return many, plain
+
+
 def moe_gate(logits, bias, n_active, norm_topk_prob, scale, sigmoid, topk_method, n_group, topk_group):
     init(_inited or 0)
     x = np.ascontiguousarray(logits, dtype=np.float32).copy()

@@ -369,6 +369,8 @@ int dsk_moe_gate(float* logits, const float* bias, int n_routed, int n_active, i
 /* attn over all heads — src/infer.cpp:728-762 / mha_cpu 1143-1164.  kcache/vcache fp16 (kv_len rows). */
 int dsk_attn(const float* q, const uint16_t* kcache, const uint16_t* vcache, int n_heads, int head_dim,
              int v_head_dim, int kv_len, float* out);
+/* 1 / (1 + e^-v), or v times that (times_v), of n values: as the ends of matrix products take it, many values a thread, and by a division. */
+int dsk_logistic(const float* v, int n, int times_v, float* out_many, float* out_plain);
 
 /* ---- measurement hook (bench.py roofline): times `iters` back-to-back launches of ONE GEMV stage of the decode
  * interpreter (production tile plan, TMA ring, warp-per-tile reduction) on a (d x n) matrix of synthetic weights

@@ -242,3 +242,25 @@ def test_full_size_properties(dsk):
     for r in rows[:16] % (d // 8):
         exp = P.matmul(x, wq[r:r + 1], "q2_k", 1, n)
         assert abs(yq[r] - exp[0]) <= 2e-5 * max(1.0, abs(exp[0]))
+
+
+@pytest.mark.parametrize("times_v", [0, 1])
+def test_logistic_of_many_values(dsk, times_v):
+    """The logistic function at the ends of matrix products, a quotient by refinement: against float64 and against the division.  expf is within two last places, its sum with 1
+    rounds once, the quotient once: 3 x 2^-23 of the value, two last places where it is subnormal."""
+    rng = np.random.RandomState(3)
+    with np.errstate(over="ignore"):
+        edges = np.array([0.0, 1e-45, 1e-40, 1.2e-38, 1e-10, 1.0, 16.0, 43.6, 44.4, 69.3, 87.3, 87.4, 88.0, 88.7, 88.72, 88.73, 89.0, 103.0, 104.0, 1e30, 3.4e38, 3.4028235e38, np.inf], np.float32)
+    v = np.concatenate([edges, -edges, [np.nan], rng.uniform(-110, 110, 1 << 20), rng.randn(1 << 20) * 4, np.exp(rng.uniform(-100, 88, 1 << 20)) * rng.choice([-1.0, 1.0], 1 << 20)]).astype(np.float32)
+    many, plain = dsk.logistic(v, times_v)
+    x = v.astype(np.float64)
+    with np.errstate(over="ignore", invalid="ignore"):
+        exact = (x if times_v else 1.0) / (1.0 + np.exp(-x))
+    assert np.array_equal(np.isnan(many), np.isnan(plain)) and np.array_equal(np.isinf(many), np.isinf(plain))
+    fin = np.isfinite(plain)
+    gone = fin & (np.abs(exact) < 3e-37) & (v < -88.0)       # e^-v is an infinity from 88.73 on: zero for a number that is none
+    assert np.array_equal(many[gone] == 0.0, plain[gone] == 0.0) and np.array_equal(np.signbit(many[fin]), np.signbit(plain[fin]))
+    near = fin & ~gone
+    assert np.all(np.abs(many[near] - exact[near]) <= 3.01 * 2.0 ** -23 * np.abs(exact[near]) + 2.0 ** -148)
+    apart = np.abs(many[fin].view(np.int32).astype(np.int64) - plain[fin].view(np.int32))
+    assert apart.max() <= 1 and np.count_nonzero(apart) <= 1e-5 * v.size
