@@ -579,38 +579,19 @@ _DT = {"F32": 0, "F16": 1, "BF16": 2, "F8_E5M2": 3, "F8_E4M3": 4, "I32": 5, "I16
 
 class _Results:
     """float32 arrays in pinned host memory for a model's logits: the GPU writes them directly (a pageable array takes a second copy, some 100 us a
-    megabyte, and its fresh pages as much again).  Memory for a decoded token's row is taken when the model is finished, more, for the rows of portions, by a
-    result that finds no room, at least as much again as there is (so a few times) and `most` bytes in all; an array's part comes back when the last reference to it
-    is gone.  Results that find no room then (of a program that keeps them all, or larger ones) and small ones are ordinary arrays.  Measured: 300 rows of 2000 behind a
-    prompt of 777 tokens 1030 us as zeroed pageable arrays, 953 as empty ones, 802 here, and 0.7 to 1 ms more where a piece is taken."""
+    megabyte, and its fresh pages as much again).  One piece of memory, taken when the model is finished; an array's part comes back when the last reference to it
+    is gone.  Results that find no room (of a program that keeps them all, or larger ones) and small ones are ordinary arrays.  Measured: 300 rows of 2000 behind a prompt
+    of 777 tokens 1030 us as zeroed pageable arrays, 953 as empty ones, 802 here; 8 MB take 1 to 2 ms when the model is finished (taken by the results that need
+    them instead, first passes were 0.4 to 2.6 ms longer)."""
     LEAST, UNIT, MOST = 64 << 10, 4 << 10, 8 << 20
 
-    def __init__(self, L, first: int, most: int):
+    def __init__(self, L, nbytes: int):
         self.L, self.lock, self.closed = L, threading.Lock(), False
-        self._most = -(-min(most, self.MOST) // self.UNIT) * self.UNIT
-        self._blocks = []                                            # (offset, bytes, address); offsets count through all of them
-        self._taken = 0                                              # bytes of them
-        self._holes = []                                             # (offset, bytes) inside of a block, ascending; changed under the lock alone
+        nbytes = -(-min(nbytes, self.MOST) // self.UNIT) * self.UNIT if nbytes >= self.LEAST else 0
+        self.base = L.dsk_host_alloc(nbytes) if nbytes else None
+        self._holes = [(0, nbytes)] if self.base else []             # (offset, bytes), ascending; changed under the lock alone
         self._live = 0
         self._back = collections.deque()                             # parts that came back: a finaliser may run at any point of any thread, also inside rows(), and only appends
-        if first >= self.LEAST:
-            self._take(-(-first // self.UNIT) * self.UNIT)
-
-    def _take(self, size):
-        """A block of `size` bytes, or as many as there are already."""
-        size = max(size, min(self._taken, self._most - self._taken))
-        if self._taken + size > self._most:
-            return
-        address = self.L.dsk_host_alloc(size)
-        if not address:
-            self._most = self._taken                                 # (not asked for again)
-            return
-        self._blocks.append((self._taken, size, address))
-        self._holes.append((self._taken, size))
-        self._taken += size
-
-    def _hole(self, size):
-        return next((i for i, h in enumerate(self._holes) if h[1] >= size), None)
 
     def rows(self, shape):
         """An array that the caller writes all of."""
@@ -619,19 +600,16 @@ class _Results:
         if need >= self.LEAST and not self.closed:
             with self.lock:
                 self._drain()
-                if self._hole(size) is None and not self.closed:
-                    self._take(size)
-                i = self._hole(size)
+                i = next((i for i, h in enumerate(self._holes) if h[1] >= size), None)
                 if i is not None and not self.closed:
                     at, room = self._holes[i]
                     self._holes[i:i + 1] = [(at + size, room - size)] if room > size else []
                     self._live += 1
-                    address = next(a + at - o for o, n, a in self._blocks if o <= at < o + n)
             if self.closed:
                 self._settle()
         if at is None:
             return np.empty(shape, dtype=np.float32)
-        raw = (C.c_float * (need // 4)).from_address(address)
+        raw = (C.c_float * (need // 4)).from_address(self.base + at)
         weakref.finalize(raw, self._came_back, at, size).atexit = False
         return np.frombuffer(raw, dtype=np.float32).reshape(shape)
 
@@ -644,22 +622,16 @@ class _Results:
         """What came back joins the holes; behind a closed model the last part gives the memory back.  Under the lock."""
         while self._back:
             self._live -= 1
-            self._holes = self._merged(self._holes + [self._back.popleft()], [o for o, _, _ in self._blocks])
-        if self.closed and not self._live:
-            for _, _, address in self._blocks:
-                self.L.dsk_host_free(address)
-            self._blocks, self._holes = [], []
-
-    @staticmethod
-    def _merged(holes, starts=()):
-        """Ascending, neighbours joined but for those at `starts`."""
-        merged = []
-        for h in sorted(holes):
-            if merged and sum(merged[-1]) == h[0] and h[0] not in starts:
-                merged[-1] = (merged[-1][0], merged[-1][1] + h[1])
-            else:
-                merged.append(h)
-        return merged
+            merged = []
+            for h in sorted(self._holes + [self._back.popleft()]):
+                if merged and sum(merged[-1]) == h[0]:
+                    merged[-1] = (merged[-1][0], merged[-1][1] + h[1])
+                else:
+                    merged.append(h)
+            self._holes = merged
+        if self.closed and not self._live and self.base:
+            self.L.dsk_host_free(self.base)
+            self.base, self._holes = None, []
 
     def _settle(self):
         """Drains now, unless somebody is at it, who then looks again behind the lock."""
@@ -672,16 +644,9 @@ class _Results:
                 return
 
     @property
-    def base(self):
-        """Address of the first block, if there is one."""
-        self._settle()
-        return self._blocks[0][2] if self._blocks else None
-
-    @property
     def holes(self):
-        """(offset, bytes) of what is free, memory that is not taken yet behind what is."""
         self._settle()
-        return self._merged(self._holes + ([(self._taken, self._most - self._taken)] if self._taken < self._most else []))
+        return list(self._holes)
 
     @property
     def live(self):
@@ -758,8 +723,8 @@ class Model:
         if not self.s:
             raise DskError(self.L.dsk_last_error().decode())
         if self._results is None:   # a decoded token's row, and what two portions return (the first one's is often still held when the second one's is made)
-            row, most = self.cfg.vocab_size * 4, 5 * min(self.cfg.chunk, 256) // 2 if isinstance(self.cfg, HybridConfig) else 0
-            self._results = _Results(self.L, row, (1 + most) * (row + _Results.UNIT))
+            most = 5 * min(self.cfg.chunk, 256) // 2 if isinstance(self.cfg, HybridConfig) else 0
+            self._results = _Results(self.L, (1 + most) * (self.cfg.vocab_size * 4 + _Results.UNIT))
         self._logits = self._results.rows(self.cfg.vocab_size)
 
     def comm_init(self, unique_id: bytes):

@@ -58,7 +58,7 @@ def thresholds():
 @pytest.mark.parametrize("seed", range(6))
 def test_collected_in_the_middle_of_a_call(thresholds, seed):
     rng, mem = random.Random(seed), HostMemory()
-    res = dsk._Results(mem, 100000, 2 << 20)
+    res = dsk._Results(mem, 2 << 20)
     whole, held = res.holes, []
     for _ in range(3000):
         thresholds(rng.randint(2, 60), 2, 2)
@@ -86,7 +86,7 @@ def test_collected_in_the_middle_of_a_call(thresholds, seed):
 
 def test_threads():
     mem = HostMemory()
-    res = dsk._Results(mem, 0, 4 << 20)
+    res = dsk._Results(mem, 4 << 20)
     whole, wrong = res.holes, []
 
     def work(k):
@@ -113,41 +113,18 @@ def test_threads():
 
 def test_small_and_large_results_are_ordinary_arrays():
     mem = HostMemory()
-    res = dsk._Results(mem, 0, 1 << 20)
+    res = dsk._Results(mem, 1 << 20)
     assert not pinned(mem, res.rows((1, 10))) and not pinned(mem, res.rows((1, 1 << 20))) and pinned(mem, res.rows((4, 20000)))
     res.close()
     gc.collect()
     assert not mem.blocks and not pinned(mem, res.rows((4, 20000)))
 
 
-@pytest.mark.parametrize("first", [0, 1000, 80000])
-def test_memory_is_taken_when_a_result_needs_it(first):
-    mem = HostMemory()
-    taken = lambda: sum(len(b) for b in mem.blocks.values())  # noqa: E731
-    res = dsk._Results(mem, first, 3 << 20)
-    small, large = res.rows(1000), res.rows((100, 20000))
-    assert taken() == (81920 if first == 80000 else 0) and not pinned(mem, small) and not pinned(mem, large)
-    row = res.rows(20000)
-    assert pinned(mem, row) and taken() == 81920             # (the row that is asked for first has it to itself)
-    a = res.rows((5, 20000))
-    assert pinned(mem, a) and taken() == 81920 + 401408
-    held = [row, a] + [res.rows((5, 20000)) for _ in range(10)]
-    check(mem, res, held)
-    assert sum(pinned(mem, h) for h in held) == 8 and taken() == 3 << 20 and len(mem.blocks) <= 5          # (7 x 401408 + 81920 of 3 MB)
-    del held, a, row
-    gc.collect()
-    n = len(mem.blocks)
-    assert pinned(mem, res.rows((5, 20000))) and len(mem.blocks) == n
-    res.close()
-    gc.collect()
-    assert not mem.blocks
-
-
 def test_no_pinned_memory_to_be_had():
     class Refusing(HostMemory):
         def dsk_host_alloc(self, n):
             return None
-    res = dsk._Results(Refusing(), 100000, 1 << 20)
+    res = dsk._Results(Refusing(), 1 << 20)
     a = res.rows((4, 20000))
     a[:] = 1.0
     assert res.live == 0 and res.base is None
