@@ -1780,19 +1780,30 @@ static void launch_hgrn2(const dsk_layer_spec& sp, const float* proj, int ld, fl
 static size_t ssd_gram_smem(const dsk_layer_spec& s) {
   return ((size_t)2 * kLinBlk * (((s.ssm_state + 3) & ~3) + 4) + (size_t)2 * kLinBlk * (s.ssm_heads / s.ssm_groups)) * 4;
 }
-// Whether lin_mma walks a portion, and in how many segments.  Times of a block in us, 128 (64) key entries: walked for results 2.0 (1.35), for the end state alone 1.4 (0.9), a round of
-// CTAs each, and 8 for the launch, 5 for a second; lin_scan 7.7, a block 1.1 and 1.3 more where 64 heads of 64 channels fill the chip.  Whole walks of 2048 tokens: 64 heads of 64 channels 312 (lin_scan) and 215, 16 of 128 187 and 114; 600
-// tokens, 16 heads of 64, 64 entries 46 and 23; 100 tokens 20 and 22: not taken.
+// lin_scan: warps of a CTA and CTAs, by value channels that a warp has (CW) and by how many CTAs there are; extra: a column more, the normaliser
+struct LinScanShape { int warps, ctas; };
+static LinScanShape lin_scan_shape(int H, int P, bool extra, int CW) {
+  int warps = std::max(1, std::min(8, (P + CW - 1) / CW));
+  while (warps > 2 && H * ((P + warps * CW - 1) / (warps * CW)) < g_sm_count) warps = (warps + 1) / 2;
+  return {warps, H * ((P + (extra ? 1 : 0) + warps * CW - 1) / (warps * CW))};
+}
+// Whether lin_mma walks a portion, and in how many segments (0: lin_scan does).  us: lin_scan 8 for the launch, and a block by the warps w that an SM has, 0.95 for 2, 1.1 for 4,
+// 1.4 for 8, 2.4 for 16, 4.8 for 32; lin_mma, 128 (64) key entries, a block walked for results 1.95 (1.25), for the end state alone 1.1 (0.6), a round of CTAs each, 6 for the launch, 11
+// for two, 0.8 a segment that states are joined over.  Measured over 4 to 64 heads of 32 to 128 channels, 64 and 128 entries, with and without the normaliser, 48 to 2048 tokens (354
+// walks): what this takes is 0.3 % above the fastest on average, once 4 % above lin_scan.  2048 tokens, lin_scan and lin_mma: 64 heads of 64 channels 312 and 222 (two segments), 16 of
+// 128 186 and 116 (four), 16 of 128 with the normaliser, whose column takes a third CTA, 188 and 152 (three), 4 of 64 with 64 entries 134 and 46 (eight), 64 of 128 with the normaliser 637
+// and 532 (three); 600 tokens, 16 of 64 with 64 entries 46 and 23; 100 tokens, 8 of 128 with 128 entries 17 and 21: not taken; 48 tokens, 32 of 64 with 64 entries 12.8 and 10.1 (one walk).
 static int lin_mma_segments(const float* q, const float* k, int ldq, int hs, const float* v, int ldv, int T, int H, int N, int P, bool extra, const float* seg) {
   auto al = [](const float* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   if (!seg || (N != 64 && N != 128) || P % 4 || ldq % 4 || hs % 4 || ldv % 4 || !al(q) || !al(k) || !al(v)) return 0;
   const int nb = (T + kLinBlk - 1) / kLinBlk, ctas = H * ((P + (extra ? 1 : 0) + kLmCh - 1) / kLmCh);
-  const double full = N == 128 ? 2.0 : 1.35, ends = N == 128 ? 1.4 : 0.9;
-  double best = 7.7 + nb * (1.1 + 1.3 * (double)H * P * N / (64.0 * 64 * 128));
+  const LinScanShape scan = lin_scan_shape(H, P, extra, N == 64 ? 4 : 2);
+  const double full = N == 128 ? 1.95 : 1.25, ends = N == 128 ? 1.1 : 0.6, w = scan.warps * ((scan.ctas + g_sm_count - 1) / g_sm_count);
+  double best = 8 + nb * std::max(0.8 + 0.075 * w, 0.15 * w);
   int segs = 0;
   for (int n = 1; n <= kLmSegs; n++) {
     const int per = (nb + n - 1) / n, rounds = (ctas * n + g_sm_count - 1) / g_sm_count, first = (ctas * (n - 1) + g_sm_count - 1) / g_sm_count;
-    const double cost = per * (rounds * full + first * ends) + (n > 1 ? 13 : 8);
+    const double cost = per * (rounds * full + first * ends) + (n > 1 ? 11 + 0.8 * n : 6);
     if ((nb + per - 1) / per == n && cost < best) { best = cost; segs = n; }
   }
   return segs;
@@ -1818,8 +1829,7 @@ static void launch_lin_scan(bool delta, const float* q, const float* k, int ldq,
   int CPT = N > 128 ? 4 : 2;          // value channels per lane
   if (const char* e = getenv("DSK_LIN_CPT")) CPT = atoi(e) == 4 || N > 128 ? 4 : 2;   // A/B switch
   const int CW = CPT * (32 / TPC);
-  int warps = std::max(1, std::min(8, (P + CW - 1) / CW));
-  while (warps > 2 && H * ((P + warps * CW - 1) / (warps * CW)) < 148) warps = (warps + 1) / 2;
+  int warps = lin_scan_shape(H, P, nst != nullptr, CW).warps;
   if (const char* e = getenv("DSK_LIN_WARPS")) warps = std::max(1, std::min(8, atoi(e)));   // A/B switch
   const int PB = warps * CW;
   const dim3 grid((unsigned)H, (unsigned)((P + (nst ? 1 : 0) + PB - 1) / PB));

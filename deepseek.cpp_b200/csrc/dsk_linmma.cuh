@@ -7,8 +7,9 @@
 // Segments: the state is linear in what came before, so that every segment but the last is first walked from zero for its end state alone (mode 0), and then all are walked
 // from their true starts, which each works out from those (mode 1).
 // Bound: the chain of a block (products of a sum wait for one another, then a barrier) and the issue slots of its warps: 204 products and 64 numbers into parts.  FMAs of the whole state
-// by every token, with their operands from shared memory, bound lin_scan: 2048 tokens, 64 heads of 64 channels and 128 entries 312 us, here 215; 16 heads of 128 channels 187, 114; 600
-// tokens, 16 heads of 64 channels and entries 46, 23.  The first two in one walk 252 and 248: where heads are few, the segments are the gain.  Two blocks of loads ahead instead of one: the same.
+// by every token, with their operands from shared memory, bound lin_scan: 2048 tokens, 64 heads of 64 channels and 128 entries 312 us, here 222 in two segments and 257 in one walk;
+// 16 heads of 128 channels 186, 116 in four and 255 in one, where heads are few the segments are the gain; with the matrix memory's normaliser, a column in a third CTA a head, 188 and 152
+// (three); 600 tokens, 16 heads of 64 channels and entries 46, 23.  Two blocks of loads ahead instead of one: the same.
 // Error against 64 bits 1.7e-7 of the largest result, lin_scan's 2.8e-7.  lin_scan stays for other sizes and for short steps, where the two launches and the first split cost more.
 // Values that are not finite: results that come out so are summed again from the numbers, as lin_scan sums them, and blocks with such keys or values update the state with FMAs.
 #pragma once

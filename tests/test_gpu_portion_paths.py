@@ -39,6 +39,17 @@ def test_recurrence_in_segments(mk, ho, heads, vdim, state, groups):  # noqa: F8
         assert rel(in_portions(m, toks, sizes), exp) < F32_TOL
 
 
+# the same in one walk, which short portions of many heads take
+@pytest.mark.parametrize("heads,vdim,state,groups", [(32, 64, 64, 4), (32, 128, 128, 2)])
+def test_recurrence_in_one_walk(mk, ho, heads, vdim, state, groups):  # noqa: F811
+    cfg = ho.small_config(layers=[ssd(heads, vdim, state, groups)], width=36, norm={"eps": 1e-5, "groups": 1})
+    m, W = mk(cfg, seed=state + heads, chunk=80)
+    toks = tokens_for(cfg, 130, 11)
+    exp = ho.run(cfg, W, toks)[0]
+    for sizes in ([48, 80], [7, 50, 73]):
+        assert rel(in_portions(m, toks, sizes), exp) < F32_TOL
+
+
 @pytest.mark.parametrize("heads,dim,vdim", [(4, 64, 64), (3, 128, 60), (2, 64, 16), (2, 128, 12)])   # the normaliser's column: first of a CTA, last of a group, first of one, inside one
 def test_matrix_memory_in_segments(mk_netusun, no, heads, dim, vdim):  # noqa: F811
     def edit(W):                                             # gates at the cap next to keeping everything
