@@ -164,7 +164,7 @@ struct State {
   cudaEvent_t in_ev[2] = {nullptr, nullptr};   // its copy is through
   // attention of portions in one kernel (pattn): split keys and values of the visible positions, queries it takes at a time
   __nv_bfloat16 *k16 = nullptr, *v16 = nullptr;
-  float* ppart = nullptr;                    // partial softmax results of shares of the keys: up to 148 CTAs of 128 rows (launches that fill the chip are not split)
+  float* ppart = nullptr;                    // partial softmax results of shares of the keys: a CTA of 128 rows an SM (launches that fill the chip are not split)
   int pattn_q = 0;
   // bf16 products of portions: activations rounded for the product that follows, hidden rows of a feed-forward, and a host word that a wait
   // which gave up sets
@@ -1344,7 +1344,7 @@ static dsk_state* state_create(dsk_model* m) {
         if (!takes_pattn(L.sp, bf16)) continue;
         const PattnSize z = pattn_size(L.sp, bf16);
         const size_t n = visible(L.sp, q);
-        shares = std::max<size_t>(shares, (size_t)148 * 128 * (z.V + 2) / (z.Vp / (z.VN * 8)));
+        shares = std::max<size_t>(shares, (size_t)g_sm_count * 128 * (z.V + 2) / (z.Vp / (z.VN * 8)));
         k16 = std::max(k16, n * z.G * z.Dp * z.parts); v16 = std::max(v16, n * z.G * z.Vp * z.parts);
         if (L.sp.mixer != DSK_MIX_GQA) { kup = std::max(kup, n * z.G * L.sp.att_dim); vup = std::max(vup, n * z.G * z.V); }
       }
@@ -1555,7 +1555,7 @@ static void launch_tc5(State* S, int epi, const GemmP& P, int tile_cap, cudaStre
   if (!A16 && P.A == S->mirror && P.lda == S->width && P.K == S->width) {
     A16 = S->h16;
     if (P.a_map) {
-      launch_next(gather_rows16, (unsigned)std::min<long long>(((long long)P.M * (P.K / 8) + 255) / 256, 148 * 8), 256, 0, st)(S->h16, P.a_map, P.a_div, S->a16, P.M, P.K);
+      launch_next(gather_rows16, (unsigned)std::min<long long>(((long long)P.M * (P.K / 8) + 255) / 256, g_sm_count * 8), 256, 0, st)(S->h16, P.a_map, P.a_div, S->a16, P.M, P.K);
       S->launches++;
       A16 = S->a16;
     }
@@ -1563,7 +1563,7 @@ static void launch_tc5(State* S, int epi, const GemmP& P, int tile_cap, cudaStre
   if (!A16) {
     const int vec = P.lda % 4 == 0 && (reinterpret_cast<uintptr_t>(P.A) & 15) == 0;
     const long long n = (long long)P.M * (P.K / 8);
-    launch_next(bf16_rows, (unsigned)std::min<long long>((n + 255) / 256, 148 * 8), 256, 0, st)(P.A, P.lda, P.a_map, P.a_div, S->a16, P.M, P.K, vec);
+    launch_next(bf16_rows, (unsigned)std::min<long long>((n + 255) / 256, g_sm_count * 8), 256, 0, st)(P.A, P.lda, P.a_map, P.a_div, S->a16, P.M, P.K, vec);
     S->launches++;
     A16 = S->a16;
   }
@@ -1575,8 +1575,8 @@ static void launch_tc5(State* S, int epi, const GemmP& P, int tile_cap, cudaStre
   for (int bn = 256; bn >= 32; bn /= 2) {
     if (dual && bn < 64) break;
     const int cols = dual ? bn / 2 : bn;
-    const long long tiles = (long long)mt * ((P.N + cols - 1) / cols), cost = (tiles + 147) / 148 * (bn + 64);
-    if (best < 0 || cost < best) { best = cost; T.bn = bn; grid = std::min<long long>(tiles, 148); }
+    const long long tiles = (long long)mt * ((P.N + cols - 1) / cols), cost = (tiles + g_sm_count - 1) / g_sm_count * (bn + 64);
+    if (best < 0 || cost < best) { best = cost; T.bn = bn; grid = std::min<long long>(tiles, g_sm_count); }
   }
   T.stages = std::min(kTcMaxStages, kTcRing / ((kTcRows + T.bn) * kTcDepth * 2));
   T.n_mt = mt; T.rows_per_expert = P.tiles ? (int)(P.sW / P.ldw) : 0;
@@ -1602,8 +1602,8 @@ template <typename WT>
 static void launch_gemv(int epi, const GemmP& P, int Z, cudaStream_t st) {
   if (gemv_one_ok<WT>(P)) {
     const int n = std::max(P.N, P.n_shared > 0 ? P.sN : 0);
-    const int R = (long long)n * Z >= (Z == 1 ? 16384 : 148 * 64) ? 2 : 1;   // rows per warp: two where one each would be more warps than the chip holds at a time
-    const dim3 grid((unsigned)std::max(1, std::min((n + 8 * R - 1) / (8 * R), 148 * 8)), (unsigned)Z);
+    const int R = (long long)n * Z >= (Z == 1 ? 16384 : g_sm_count * 64) ? 2 : 1;   // rows per warp: two where one each would be more warps than the chip holds at a time
+    const dim3 grid((unsigned)std::max(1, std::min((n + 8 * R - 1) / (8 * R), g_sm_count * 8)), (unsigned)Z);
 #define DSK_GEMV1(E) do { if (R == 2) launch_next(gemv_one<WT, E, 2>, grid, 256, 0, st)(P); else launch_next(gemv_one<WT, E, 1>, grid, 256, 0, st)(P); } while (0)
     switch (epi) {
       case HEPI_STORE: DSK_GEMV1(HEPI_STORE); break;
@@ -1621,7 +1621,7 @@ static void launch_gemv(int epi, const GemmP& P, int Z, cudaStream_t st) {
     }
 #undef DSK_GEMV1
   } else {
-    const dim3 grid((unsigned)std::max(1, std::min((std::max(P.N, P.n_shared > 0 ? P.sN : 0) + 7) / 8, 148 * 8)), (unsigned)Z);
+    const dim3 grid((unsigned)std::max(1, std::min((std::max(P.N, P.n_shared > 0 ? P.sN : 0) + 7) / 8, g_sm_count * 8)), (unsigned)Z);
     switch (epi) {
       case HEPI_STORE: launch_next(gemv_rows<WT, HEPI_STORE>, grid, 256, 0, st)(P); break;
       case HEPI_ADD: launch_next(gemv_rows<WT, HEPI_ADD>, grid, 256, 0, st)(P); break;
@@ -1737,7 +1737,7 @@ static void launch_scan(const dsk_layer_spec& sp, const float* proj, int ld_proj
   const int H = sp.ssm_heads, P = sp.ssm_vdim, N = sp.ssm_state, G = sp.ssm_groups;
   const int inner = H * P;
   int PB = std::min(P, 64);   // value channels per CTA: fewer when the heads alone would leave most SMs idle
-  while (PB > 32 && H * ((P + PB - 1) / PB) < 148) PB /= 2;   // (measured: 32 channels per CTA is the best split at 64 heads x 64)
+  while (PB > 32 && H * ((P + PB - 1) / PB) < g_sm_count) PB /= 2;   // (measured: 32 channels per CTA is the best split at 64 heads x 64)
   if (const char* e = getenv("DSK_SCAN_PB")) PB = std::max(1, std::min(std::min(P, 64), atoi(e)));   // A/B switch
   const dim3 grid((unsigned)H, (unsigned)((P + PB - 1) / PB));
   const int threads = ((PB * 8 + 31) / 32) * 32;
@@ -1759,7 +1759,7 @@ static void launch_hgrn2(const dsk_layer_spec& sp, const float* proj, int ld, fl
   int TPC = N >= 256 ? 32 : N >= 64 ? 16 : 8;
   if (const char* e = getenv("DSK_LIN_TPC")) { const int v = atoi(e); if ((v == 8 || v == 16 || v == 32) && N >= 4 * v) TPC = v; }   // A/B switch
   int PB = std::min(P, 512 / TPC);   // value channels per CTA
-  while (PB > 16 && H * ((P + PB - 1) / PB) < 148) PB /= 2;
+  while (PB > 16 && H * ((P + PB - 1) / PB) < g_sm_count) PB /= 2;
   if (PB == 16 && H * ((P + 15) / 16) < 74) PB = 8;
   if (const char* e = getenv("DSK_LIN_PB")) PB = std::max(1, std::min(std::min(P, 512 / TPC), atoi(e)));   // A/B switch
   const dim3 grid((unsigned)H, (unsigned)((P + PB - 1) / PB));
@@ -1921,7 +1921,7 @@ static void launch_decode_attn(State* S, DecodeAttn P, bool latent, cudaStream_t
     // Shares of the keys: one a tile, but no more CTAs than run at a time (three an SM).  With a CTA per tile and key head, 16 key heads behind a window of 4096
     // were 1024 CTAs, waiting for a place and mostly without a key of theirs: two such layers (width 1024) and their head took 120 us a token behind 30 keys and
     // 150 behind 2000, gqa_attn with its four key heads a CTA 117 and 139, this 109 and 135.
-    const int rows = (T + P.TQ - 1) / P.TQ * P.G * ((rep + P.HB - 1) / P.HB), most = std::max(1, std::min(kAttnSplitMax, 3 * 148 / rows)), per = (tiles + most - 1) / most;
+    const int rows = (T + P.TQ - 1) / P.TQ * P.G * ((rep + P.HB - 1) / P.HB), most = std::max(1, std::min(kAttnSplitMax, 3 * g_sm_count / rows)), per = (tiles + most - 1) / most;
     P.NS = (tiles + per - 1) / per;
   }
   P.part = S->part;
@@ -1972,7 +1972,7 @@ static void launch_pattn5(State* S, const PattnSize& z, PattnP& A, cudaStream_t 
   const int smem = p5_smem(z.parts, nch, vb, kst, vst), qb = (A.T + kP5Rows - 1) / kP5Rows, zc = z.Vp / (vb * 64);
   // shares of the keys where the query blocks leave SMs idle, of at least four tiles (joining them takes about as long as three)
   const long long ctas = (long long)qb * A.H * zc, tiles = (std::min<long long>(A.Lk, (long long)A.span + kP5Rows) + kP5Keys - 1) / kP5Keys;
-  const long long most = std::min({148 / ctas, tiles / 4, (long long)kAttnSplitMax});
+  const long long most = std::min({g_sm_count / ctas, tiles / 4, (long long)kAttnSplitMax});
   A.NS = most > 1 && (tiles + most - 1) / most + 3 < tiles ? (int)most : 1;
   A.part = S->ppart;
   CUtensorMap mK, mV;
@@ -1996,9 +1996,9 @@ static void launch_pattn(State* S, const PattnSize& z, const PackP& K, PattnP& A
     const int ck = pattn_smem(z.parts, cw, z.Dp, z.VN, 4) <= (size_t)kPattnSmemMax ? 4 : 2;
     if (pattn_smem(z.parts, cw, z.Dp, z.VN, ck) > (size_t)kPattnSmemMax) continue;
     const long long ctas = (long long)((A.T + 16 * cw - 1) / (16 * cw)) * A.H * zc, tiles = (std::min<long long>(K.Lk, (long long)A.span + 16 * cw) + 8 * ck - 1) / (8 * ck);
-    const long long most = std::max<long long>(1, std::min({148 / ctas, tiles / 4, (long long)kAttnSplitMax}));
+    const long long most = std::max<long long>(1, std::min({g_sm_count / ctas, tiles / 4, (long long)kAttnSplitMax}));
     for (long long ns = 1; ns <= most; ns += std::max<long long>(1, most - 1)) {   // (joining shares takes about as long as a tile)
-      const long long cost = (ctas * ns + 147) / 148 * (cw == 8 ? 6 : cw == 4 ? 5 : 7) * ((tiles + ns - 1) / ns + (ns > 1)) * ck;
+      const long long cost = (ctas * ns + g_sm_count - 1) / g_sm_count * (cw == 8 ? 6 : cw == 4 ? 5 : 7) * ((tiles + ns - 1) / ns + (ns > 1)) * ck;
       if (!w || cost < best) { best = cost; w = cw; nk = ck; A.NS = (int)ns; }
     }
   }
