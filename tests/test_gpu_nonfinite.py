@@ -51,6 +51,34 @@ def test_products(no, value, tokens):  # noqa: F811
         assert np.all(np.abs(got[fin & ~near, 77] - exp[fin & ~near, 77]) <= 1e-4 * np.abs(value))
 
 
+# the same where the CTAs of a cluster share a product's depth: the sums of all of them are joined, and looked at, by the CTA that has the row (column: in the first share, one in the
+# middle, the ragged last)
+@pytest.mark.parametrize("value", [np.inf, np.nan, -3.4e38, 3.39e38])
+@pytest.mark.parametrize("tokens,column", [(5, 3), (40, 700), (131, 1099)])
+def test_products_of_shared_depth(no, value, tokens, column):  # noqa: F811
+    cfg = no.model_config([no.att(heads=2, dim=16, vdim=16, mlp=None)], width=1100, vocab=150)
+    W = no.random_weights(cfg, 3)
+    toks = tokens_for(cfg, tokens, 3)
+    toks[toks == 77] = 5
+    exp, layers = no.run(cfg, W, toks)
+    h = np.array([no.rms(x, cfg["norm"]["eps"]) * W["final.norm"] for x in layers[-1]])
+    W["embed"] = np.array(W["embed"])
+    W["embed"][77, column] = value
+    with np.errstate(over="ignore", invalid="ignore"):
+        col = np.float64(np.float32(value)) * h[:, column] + h @ np.where(np.arange(1100) == column, 0.0, W["embed"][77])
+        exp[:, 77] = np.where(np.abs(col) > 3.4028e38, np.copysign(np.inf, col), col) if not np.isnan(value) else np.nan
+    m = matrix_model(no, cfg, W, 256)
+    got = m.forward_chunk(toks, 0, range(tokens))
+    m.close()
+    others = np.arange(150) != 77
+    assert rel(got[:, others], exp[:, others]) < F32_TOL
+    fin = np.isfinite(exp[:, 77])
+    near = np.abs(np.abs(col) / 3.4028e38 - 1.0) < 1e-3 if np.isfinite(value) else np.zeros(tokens, bool)
+    assert np.array_equal(got[~fin & ~near, 77], exp[~fin & ~near, 77], equal_nan=True)
+    if np.any(fin & ~near):
+        assert np.all(np.abs(got[fin & ~near, 77] - exp[fin & ~near, 77]) <= 1e-4 * np.abs(value))
+
+
 def poisoned(W, value, row):
     W["embed"][row, 1] = value
 
@@ -110,6 +138,64 @@ def test_latents_in_bf16(mk_hybrid, ho, value):  # noqa: F811
         t[at] = 50
         m.reset()
         got = m.forward_chunk(t, 0, range(64))
+        others = np.arange(cfg["vocab"]) != 50
+        assert np.all(np.isfinite(got[:at, others])) and rel(got[:at, others], base[:at, others]) < 2e-2   # (rows that are summed again: weights not rounded)
+    m.reset()
+
+
+# heads of 64 entries and more (pattn5): blocks of 64 and 128 value columns, depth in one, two and three pieces, one block of queries and several, whose rows in front of the token share
+# a tile with it
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+@pytest.mark.parametrize("kind", ["grouped", "own_keys", "latent", "deep_latent"])
+def test_attention_of_wide_heads(mk, no, kind, value):  # noqa: F811
+    layer = {"grouped": lambda: no.att(heads=4, kv_heads=2, dim=64, vdim=64, size=50), "own_keys": lambda: no.att(heads=2, kv_heads=2, dim=100, vdim=150, size=None),
+             "latent": lambda: no.lat(heads=2, dim=64, rot_dim=8, vdim=70), "deep_latent": lambda: no.lat(heads=2, dim=128, rot_dim=64, vdim=128)}[kind]
+    cfg = no.model_config([layer(), layer()], width=48, vocab=97)
+    m, W = mk(cfg, seed=4, chunk=256, edit=lambda W: poisoned(W, value, 90))
+    for sizes in ([40], [200], [70, 90]):
+        n = sum(sizes)
+        toks = tokens_for(cfg, n, 5)
+        toks[toks == 90] = 7
+        for at in (1, 31, n // 2 + 3, n - 1):
+            t = toks.copy()
+            t[at] = 90
+            m.reset()
+            assert ahead_of_the_poison(m, no.run, cfg, W, t, at, sizes) < F32_TOL
+    m.reset()
+
+
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+@pytest.mark.parametrize("kind", ["grouped", "own_keys", "latent"])
+def test_shares_of_the_keys_of_wide_heads(mk, no, kind, value):  # noqa: F811
+    layer = {"grouped": lambda: no.att(heads=4, kv_heads=2, dim=64, vdim=64, size=None), "own_keys": lambda: no.att(heads=2, kv_heads=2, dim=100, vdim=150, size=300),
+             "latent": lambda: no.lat(heads=2, dim=64, rot_dim=8, vdim=128)}[kind]
+    cfg = no.model_config([layer(), layer()], width=48, vocab=97)
+    m, W = mk(cfg, seed=4, chunk=300, context=700, edit=lambda W: poisoned(W, value, 90))
+    toks = tokens_for(cfg, 560, 5)
+    toks[toks == 90] = 7
+    for at in (20, 420, 500, 558):
+        t = toks.copy()
+        t[at] = 90
+        m.reset()
+        assert ahead_of_the_poison(m, no.run, cfg, W, t, at, [300, 100, 160]) < F32_TOL
+    m.reset()
+
+
+@pytest.mark.parametrize("value", [np.inf, np.nan])
+@pytest.mark.parametrize("dim,vdim,size,sizes", [(64, 64, 30, [130]), (128, 128, 400, [300, 40])])   # (300 keys behind 40 queries: shares)
+def test_latents_of_wide_heads_in_bf16(mk_hybrid, ho, value, dim, vdim, size, sizes):  # noqa: F811
+    att = {"type": "latent_attention", "mixer": {"heads": 3, "dim": dim, "vdim": vdim, "kv_rank": 40, "mask": {"size": size}, "scale": 0.1}, "mlp": None}
+    cfg = ho.small_config(layers=[att] * 2, width=36, norm={"eps": 1e-5, "groups": 1})
+    m, W = mk_hybrid(cfg, seed=4, quant="bf16", chunk=300, context=500, edit=lambda W: poisoned(W, value, 50))
+    n = sum(sizes)
+    toks = tokens_for(cfg, n, 5)
+    toks[toks == 50] = 7
+    base = in_portions(m, toks, sizes)
+    for at in (1, 33, n // 2, n - 1):
+        t = toks.copy()
+        t[at] = 50
+        m.reset()
+        got = in_portions(m, t, sizes)
         others = np.arange(cfg["vocab"]) != 50
         assert np.all(np.isfinite(got[:at, others])) and rel(got[:at, others], base[:at, others]) < 2e-2   # (rows that are summed again: weights not rounded)
     m.reset()

@@ -2,6 +2,9 @@
 or 128), against the float64 statement: steps that continue a sequence inside a window, several column groups, heads too deep for the kernel."""
 import pytest
 
+from test_gpu_hybrid import close_bf16 as close_rows
+from test_gpu_hybrid import ho  # noqa: F401
+from test_gpu_hybrid import mk as mk_hybrid  # noqa: F401
 from test_gpu_netusun import F32_TOL, close_bf16, in_portions, mk, no, rel, tokens_for  # noqa: F401
 from test_gpu_sakusun import mk as mk_sakusun  # noqa: F401
 from test_gpu_sakusun import so  # noqa: F401
@@ -101,3 +104,13 @@ def test_blocks_of_128_queries_with_a_rotated_part(mk, no, dim, rot_dim, vdim, t
     m, W = mk(cfg, seed=dim, chunk=512, context=600)
     toks = tokens_for(cfg, tokens, 6)
     assert rel(m.forward_chunk(toks, 0, range(tokens)), no.run(cfg, W, toks)[0]) < F32_TOL
+
+
+# latent attention of bf16 models, operands in one part: blocks of 64 and 128 value columns, depths that end inside a piece of 64, windows inside and over a tile, shares of the keys
+@pytest.mark.parametrize("dim,vdim,size,sizes", [(64, 64, 50, [127, 33]), (65, 70, 300, [128, 129]), (128, 128, 200, [300]), (100, 150, 33, [257]), (192, 20, 1000, [130, 126]), (64, 128, 1000, [600, 40])])
+def test_blocks_of_128_queries_in_one_part(mk_hybrid, ho, dim, vdim, size, sizes):  # noqa: F811
+    att = {"type": "latent_attention", "mixer": {"heads": 2, "dim": dim, "vdim": vdim, "kv_rank": 48, "mask": {"size": size}, "scale": dim ** -0.5}, "mlp": None}
+    cfg = ho.small_config(layers=[att] * 2, width=48, norm={"eps": 1e-5, "groups": 1})
+    m, W = mk_hybrid(cfg, seed=dim, quant="bf16", chunk=640, context=700)
+    toks = tokens_for(cfg, sum(sizes), 5)
+    assert close_rows(in_portions(m, toks, sizes), ho.run(cfg, W, toks)[0])
