@@ -1666,7 +1666,7 @@ static void launch_split(State* state, int epi, const GemmP& P, int Z, int tile_
     if (c == 1 || cost < best) { best = cost; S = c; }
   }
   const dim3 grid((unsigned)(nt * S), (unsigned)mt, (unsigned)Z);
-  // (a short depth takes no more of an SM than it has slices: short steps' next kernels start beside it)
+  // (a short depth takes no more shared memory than it has slices, the rest is L1: a prompt of 1500 tokens with mixed heads 1594 -> 1589 us, fp32 prompts and 45 tokens the same)
   const int stages = std::max(1, std::min(kSplitStages, (slices + S - 1) / S));
 #define DSK_SPLIT(E) case E: if (S > 1) launch_next(gemm_split<E, true>, grid, kSplitThreads, split_smem(stages), st, (unsigned)S)(P, stages, S, state->h_err); \
     else launch_next(gemm_split<E, false>, grid, kSplitThreads, split_smem(stages), st)(P, stages, 1, state->h_err); break

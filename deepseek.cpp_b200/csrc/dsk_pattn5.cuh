@@ -1,15 +1,18 @@
-// dsk_pattn5.cuh — softmax attention of portions on the 5th-generation tensor cores, for blocks of 128 queries (pattn has the smaller ones, heads of more than 192 entries
-// and shares of the keys).
+// dsk_pattn5.cuh — softmax attention of portions on the 5th-generation tensor cores, for heads of 64 to 192 entries (a rotated part counted) whatever the number of queries; where the query
+// blocks leave SMs idle, the keys are cut into shares that latent_swa_merge joins.  pattn has the other heads: smaller ones would be half padding, larger ones do not fit.
 //
 // A CTA has 128 query rows of a head and walks their visible keys in tiles of 32.  Operands in PARTS bf16 parts as in pattn.  Keys and values come by TMA from what pattn_pack
-// made; one thread issues the products:
+// made; products:
 //   scores: the parts of a tile's keys are rows of one operand, [Q0 K0 | Q0 K1 | Q0 K2], [Q1 K0 | Q1 K1] and Q2 K0 on columns of one accumulator, as in gemm_split; the leading products
 //   of every 64 entries of depth have an accumulator of their own, so that a score is a sum of few long-rounded pieces joined in registers;
 //   values: the weights' parts are the operand in TMEM, written there by the softmax; the six pairs of a tile add up smallest first, and a tile's 32 keys leave TMEM before the next one's.
 // Eight warps have the softmax (two threads a row), four the output rows in registers (scaled and added to tile by tile).  Two accumulators for scores: a tile's products run under
 // the softmax of the one ahead.  Copies of keys and of values, products for scores and for values have a thread each: with one thread for all products a tile took 3950 to 5900
 // cycles, of which it waited 1000 for barriers in turn.
-// Bound: the tensor pipe at its narrow instructions (a tile 2300 cycles at 128 entries and 3000 at 192 by themselves; 3250 and 4300 here) and, at a part, the softmax (2000).
+// Bound: a tile's narrow tensor core instructions, which take longer than they are counted (2300 cycles at 128 entries and 3000 at 192 by themselves; 3250 and 4300 here), one behind the other with
+// the softmax (2000, what binds at a part).  Counters, 1024 queries of 16 heads, 128 + 128 entries, all keys, three parts: on the busiest SM the tensor pipe is active for 52 % of its
+// cycles and fed for 60 %; issue slots 40 %, L1 28 %, DRAM 2 %.  512 threads have 128 registers each at launch, and no more:
+// 44 bytes (two blocks of value columns) or 20 to 24 (one) are spilled, with 1.2 or 0.6 KB of loads in the code.
 // Measured, us, pattn and this: 2048 queries, 16 heads, 128 + 128 entries, window 1024, capped 433 and 148; 192 + 128 entries, all keys 576 and 183; 777 queries, 64 + 64
 // entries, window 512 99 and 42; 300 queries 54 and 25; 64 queries 19 and 15; one part, 2048 queries, 128 + 128, window 1024 108 and 91.  Error against 64 bits over those 0.74 to 1 times
 // pattn's (64 entries in one accumulator, and not in two of 32: up to 1.3 times).

@@ -9,8 +9,8 @@
 // so that 24 KB per 16 values of depth come out of shared memory and not 36.  Four warps read a finished slice's 3 x 64 columns (two accumulators in TMEM: the
 // next slice's products run meanwhile) and add them, smallest first, to what they hold in registers: a sum of n elements sees n / 64 roundings at its own size, and
 // inside of 64 elements the leading products are four additions of the tensor core.
-// Bound: the banks of shared memory, some 2000 cycles a slice: 768 for the operands of the products (which take 890 by themselves), 576 for the parts, 384 for the numbers
-// on their way through L1, the rest for rows' addresses and results.  Measured, us, before (the same six products on mma.sync, two CTAs of 128 x 64 an SM) and now, rows x columns x
+// A slice takes some 2000 cycles, its products 890 by themselves: the rest is splitting, for every column tile again, through L1 and the banks of shared memory (768 cycles for the operands of
+// the products, 576 for the parts, 384 for the numbers on their way).  Counters, 600 x 4672 x 1024: L1's data pipe 60 % of an SM's active cycles, issue slots 43 %, tensor pipe 27 %, DRAM 3 %.  Measured, us, before (the same six products on mma.sync, two CTAs of 128 x 64 an SM) and now, rows x columns x
 // depth: 600 x 4160 x 1024 139 and 72, 600 x 1024 x 2816 140 and 57, 45 x 1024 x 4096 203 and 27 (four CTAs share a tile's depth, 61 by one), 5 x 1024 x 1024 53 and 12, 1024 x 128 x
 // 512 30 and 13; 64 x 100 x 36 8 and 9.  Error against 64 bits, normal operands, depth 1024 / 2816 / 4096: 1.5, 2.4, 2.9e-7 before, 1.0, 1.4, 1.6e-7 now; positive ones, depth 512 /
 // 1000: 1.0 and 1.3e-7 before, 0.9 and 1.0e-7 now.  Tried: numbers past L1 (3 to 10 % longer), rows' addresses in registers (they spill), eight or twelve splitting warps (84 and 60
