@@ -5,10 +5,10 @@
 // A CTA has 128 rows x 64 columns.  Sixteen warps read 64-deep slices of both operands as fp32 (four groups of four, half a slice each, the next one's numbers
 // on their way while this one's are split), and put the parts into a ring of three stages (K-major rows of 128 bytes, swizzled).  One thread issues the products: a part of A
 // against several parts of W in one instruction, as the parts of W are rows of one operand and the sums of different order columns of one accumulator:
-//   [A0 W0 | A0 W1 | A0 W2],  [A1 W0 | A1 W1] on columns 64 ..,  A2 W0 on columns 128 ..
+//   [A0 W0 | A0 W1 | A0 W2],  [A1 W0 | A1 W1] on columns 64 ..,  A2 W0 on columns 128 ..    (kSplitHalves: A0 W0 of every second half slice on columns 192 ..)
 // so that 24 KB per 16 values of depth come out of shared memory and not 36.  Four warps read a finished slice's 3 x 64 columns (two accumulators in TMEM: the
 // next slice's products run meanwhile) and add them, smallest first, to what they hold in registers: a sum of n elements sees n / 64 roundings at its own size, and
-// inside of 64 elements the leading products are four additions of the tensor core.
+// inside of 64 elements (32, where a product has few of them: kSplitHalves) the leading products are four (two) additions of the tensor core.
 // A slice takes some 2000 cycles, its products 890 by themselves: the rest is splitting, for every column tile again, through L1 and the banks of shared memory (768 cycles for the operands of
 // the products, 576 for the parts, 384 for the numbers on their way).  Counters, 600 x 4672 x 1024: L1's data pipe 60 % of an SM's active cycles, issue slots 43 %, tensor pipe 27 %, DRAM 3 %.  Measured, us, before (the same six products on mma.sync, two CTAs of 128 x 64 an SM) and now, rows x columns x
 // depth: 600 x 4160 x 1024 139 and 72, 600 x 1024 x 2816 140 and 57, 45 x 1024 x 4096 203 and 27 (four CTAs share a tile's depth, 61 by one), 5 x 1024 x 1024 53 and 12, 1024 x 128 x
@@ -35,6 +35,11 @@ __device__ __noinline__ float plain_dot(const float* a, const float* w, int k_lo
 }
 
 constexpr int kSplitN = 64, kSplitDepth = 64, kSplitStages = 3;
+// Products of fewer slices than this have an accumulator of its own for the leading products of every half slice: where the slices are few, the tensor core's own, truncated, additions are
+// a sum's largest errors.  Error against 64 bits of depths 64 / 128 / 256 / 384, the six products on mma.sync (additions of 16 values, joined in registers), whole slices, halves: normal
+// operands 6.3, 7.4, 9.0, 10.4e-8; 6.9, 7.4, 8.1, 8.5; 5.1, 5.9, 7.0; positive ones 5.7, 6.1, 7.2, 8.8; 8.2, 8.1, 8.1, 8.5; 5.1, 5.3, 5.8.  Halves everywhere: an fp32 prompt of 600 tokens
+// (depths of 1024 and 2816) 734 -> 766 us.
+constexpr int kSplitHalves = 6;
 constexpr int kSplitPartA = kTcRows * 128, kSplitPartW = kSplitN * 128;              // bytes of a part of a slice
 constexpr int kSplitStage = 3 * (kSplitPartA + kSplitPartW);
 constexpr int kSplitGroups = 4, kSplitWarps = 4 * kSplitGroups, kSplitThreads = (kSplitWarps + 4 + 4) * 32;   // splitting, summing, issuing (one of the last four warps)
@@ -201,6 +206,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split(const GemmP P, in
   }
   const int all = nrows > 0 ? (k_hi - k_lo + kSplitDepth - 1) / kSplitDepth : 0, per = (all + S - 1) / S;   // slices of the tile, of a share
   const int nk = max(0, min(per, all - share * per)), k_from = k_lo + share * per * kSplitDepth;
+  const bool halves = all < kSplitHalves;
   if (warp < kSplitWarps) {
     if (vec) split_walk<true>(rows, gbase, full0, empty0, k_from, P.K, nk, nrows, stages, err);
     else split_walk<false>(rows, gbase, full0, empty0, k_from, P.K, nk, nrows, stages, err);
@@ -220,7 +226,11 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split(const GemmP P, in
         const uint64_t d0 = tc_desc(a), d1 = tc_desc(a + kSplitPartA), d2 = tc_desc(a + 2 * kSplitPartA), dw = tc_desc(a + 3 * kSplitPartA);
 #pragma unroll
         for (int k = 0; k < kSplitDepth / 16; k++) {
-          tc_mma(d, d0 + 2 * k, dw + 2 * k, idesc | (3u * kSplitN / 8 << 17), k > 0);
+          if (k < kSplitDepth / 32 || !halves) tc_mma(d, d0 + 2 * k, dw + 2 * k, idesc | (3u * kSplitN / 8 << 17), k > 0);
+          else {                                             // the second half's leading products by themselves
+            tc_mma(d + 3 * kSplitN, d0 + 2 * k, dw + 2 * k, idesc | (1u * kSplitN / 8 << 17), k > kSplitDepth / 32);
+            tc_mma(d + kSplitN, d0 + 2 * k, dw + (kSplitPartW >> 4) + 2 * k, idesc | (2u * kSplitN / 8 << 17), true);
+          }
           tc_mma(d + kSplitN, d1 + 2 * k, dw + 2 * k, idesc | (2u * kSplitN / 8 << 17), true);
           tc_mma(d + 2 * kSplitN, d2 + 2 * k, dw + 2 * k, idesc | (1u * kSplitN / 8 << 17), true);
         }
@@ -255,6 +265,12 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemm_split(const GemmP P, in
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
         for (int c = 0; c < 16; c++) acc[c0 + c] += __uint_as_float(t0[c]) + (__uint_as_float(t1[c]) + __uint_as_float(t2[c]));
+        if (halves) {
+          tc_load16(from + 3 * kSplitN + c0, t0);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int c = 0; c < 16; c++) acc[c0 + c] += __uint_as_float(t0[c]);
+        }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();

@@ -1,5 +1,6 @@
 """fp32 products of portions in three bf16 parts on the tensor cores, at the edges of their tiles (128 rows, split 64 at a time; 64 columns, gated ones 32; 64-deep slices in
 halves of 32, three of them in the ring), against the float64 statement of a small model made of them."""
+import numpy as np
 import pytest
 
 from test_gpu_netusun import F32_TOL, in_portions, mk, no, rel, tokens_for  # noqa: F401
@@ -33,3 +34,17 @@ def test_shared_depth(mk, no, width, ff, tokens):  # noqa: F811
     m, W = mk(cfg, seed=width, chunk=512)
     toks = tokens_for(cfg, tokens, 4)
     assert rel(m.forward_chunk(toks, 0, range(tokens)), no.run(cfg, W, toks)[0]) < F32_TOL
+
+
+# Products of few slices, positive operands: the tensor core truncates its additions, so that results are too small on average, by 4.1e-8 with additions of 16 values joined in registers, by
+# 3.5e-8 with accumulators of 32 values, by 7e-8 with accumulators of 64.  (The norm ahead of the product has errors of either sign, one a row.)
+@pytest.mark.parametrize("width", [48, 64, 128, 200, 320])
+def test_truncation_of_few_slices(mk, no, width):  # noqa: F811
+    def edit(W):
+        W["embed"], W["final.norm"] = np.abs(W["embed"]), np.abs(W["final.norm"])
+        W["l0.mix.o"] = W["l0.mix.o"] * 0.0                  # the stream is the embedding
+    cfg = no.model_config([no.att(heads=1, dim=16, vdim=16, mlp=None)], width=width, vocab=500)
+    m, W = mk(cfg, seed=width, chunk=512, edit=edit)
+    toks = tokens_for(cfg, 500, 3)
+    got, exp = m.forward_chunk(toks, 0, range(500)), no.run(cfg, W, toks)[0]
+    assert np.all(exp > 0) and abs(float(np.mean(got.astype(np.float64) / exp - 1.0))) < 5e-8
