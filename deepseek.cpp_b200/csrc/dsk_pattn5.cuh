@@ -4,7 +4,7 @@
 // A CTA has 128 query rows of a head and walks their visible keys in tiles of 32.  Operands in PARTS bf16 parts as in pattn.  Keys and values come by TMA from what pattn_pack
 // made; products:
 //   scores: the parts of a tile's keys are rows of one operand, [Q0 K0 | Q0 K1 | Q0 K2], [Q1 K0 | Q1 K1] and Q2 K0 on columns of one accumulator, as in gemm_split; the leading products
-//   of every 64 entries of depth have an accumulator of their own, so that a score is a sum of few long-rounded pieces joined in registers;
+//   of every 32 to 64 entries of depth have an accumulator of their own, so that a score is a sum of few long-rounded pieces joined in registers;
 //   values: the weights' parts are the operand in TMEM, written there by the softmax; the six pairs of a tile add up smallest first, and a tile's 32 keys leave TMEM before the next one's.
 // Eight warps have the softmax (two threads a row), four the output rows in registers (scaled and added to tile by tile).  Two accumulators for scores: a tile's products run under
 // the softmax of the one ahead.  Copies of keys and of values, products for scores and for values have a thread each: with one thread for all products a tile took 3950 to 5900
@@ -14,8 +14,9 @@
 // cycles and fed for 60 %; issue slots 40 %, L1 28 %, DRAM 2 %.  512 threads have 128 registers each at launch, and no more:
 // 44 bytes (two blocks of value columns) or 20 to 24 (one) are spilled, with 1.2 or 0.6 KB of loads in the code.
 // Measured, us, pattn and this: 2048 queries, 16 heads, 128 + 128 entries, window 1024, capped 433 and 148; 192 + 128 entries, all keys 576 and 183; 777 queries, 64 + 64
-// entries, window 512 99 and 42; 300 queries 54 and 25; 64 queries 19 and 15; one part, 2048 queries, 128 + 128, window 1024 108 and 91.  Error against 64 bits over those 0.74 to 1 times
-// pattn's (64 entries in one accumulator, and not in two of 32: up to 1.3 times).
+// entries, window 512 99 and 42; 300 queries 54 and 25; 64 queries 19 and 15; one part, 2048 queries, 128 + 128, window 1024 108 and 91.  Error against 64 bits 0.77 to 1.06 times
+// pattn's over 64, 80, 96, 128, 160 and 192 entries, normal operands, biased ones, positive values and scores three and nine times as large (64 entries in one accumulator, and not in two of 32:
+// up to 1.3 times; 80 in accumulators of 64 and 16, and not of 48 and 32: up to 1.11; 128 in three instead of two: 1.04 instead of 1.06, and 82 -> 91 us).
 #pragma once
 
 #include "dsk_pattn.cuh"
@@ -109,8 +110,9 @@ __global__ void __launch_bounds__(kP5Threads, 1) pattn5(const __grid_constant__ 
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_slot;
-  // columns: scores [2][main of 64 entries | two of lower order | mains of the other entries], weights' parts, values
-  const int mains = PARTS == 3 ? max(nch, 2) : nch, s_cols = (PARTS == 3 ? mains + 2 : mains) * kP5Keys;   // (64 entries alone: two of 32)
+  // columns: scores [2][main of the first entries | two of lower order | mains of the other entries], weights' parts, values.  As many mains as pieces of 64 entries, two at least, of
+  // equal depth (three parts)
+  const int all_steps = (P.Dp + 15) / 16, mains = PARTS == 3 ? max(nch, 2) : nch, per_main = PARTS == 3 ? (all_steps + mains - 1) / mains : 4, s_cols = (PARTS == 3 ? mains + 2 : mains) * kP5Keys;
   const uint32_t p_at = tmem + 320, o_at = tmem + 384;
   if (warp >= 12) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
@@ -124,18 +126,18 @@ __global__ void __launch_bounds__(kP5Threads, 1) pattn5(const __grid_constant__ 
       for (int i = 0; i < n && alive; i++) {
         if (!tc_wait(sempty + 8 * (i & 1), ((i >> 1) & 1) ^ 1, err)) break;
         const uint32_t d = tmem + (i & 1) * s_cols;
+        int main = 0, nth = 0;
         for (int c = 0; c < nch; c++) {
           alive = tc_wait(kfull + 8 * at, turn, err);
           if (!alive) break;
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           const uint64_t k0 = tc_desc(ks + at * kbytes), a0 = tc_desc(q0s + c * kP5Rows * 128), a1 = tc_desc(q0s + (nch + c) * kP5Rows * 128),
                          a2 = tc_desc(q0s + (2 * nch + c) * kP5Rows * 128);
-          const int steps = min(4, (P.Dp - c * 64 + 15) / 16);
+          const int steps = min(4, all_steps - c * 4);
           for (int k = 0; k < steps; k++) {
             if (PARTS == 1) tc_mma(d + c * kP5Keys, a0 + 2 * k, k0 + 2 * k, idesc | n1, k > 0);
             else {
-              const int main = nch > 1 ? c : k >> 1;                        // leading products of their own accumulator
-              const bool add = nch > 1 ? k > 0 : k & 1;
+              const bool add = nth > 0;                                     // main: the accumulator of this step's leading products, of which it is the nth
               if (main == 0) tc_mma(d, a0 + 2 * k, k0 + 2 * k, idesc | 3 * n1, add);
               else {
                 tc_mma(d + (2 + main) * kP5Keys, a0 + 2 * k, k0 + 2 * k, idesc | n1, add);
@@ -143,6 +145,7 @@ __global__ void __launch_bounds__(kP5Threads, 1) pattn5(const __grid_constant__ 
               }
               tc_mma(d + kP5Keys, a1 + 2 * k, k0 + 2 * k, idesc | 2 * n1, true);
               tc_mma(d + 2 * kP5Keys, a2 + 2 * k, k0 + 2 * k, idesc | n1, true);
+              if (++nth == per_main) { nth = 0; main++; }
             }
           }
           tc_commit(kempty + 8 * at);
