@@ -1694,7 +1694,8 @@ static void linear(State* S, bool bf16, int epi, const GemmP& P, int Z, cudaStre
     // (a CTA of gemm_narrow has 16 rows: under 448 they are too few.  Steps of 256 / 384 / 512 / 1024 tokens, two layers with 64 experts and a token input of
     // 32, width 2048: 714 / 819 / 873 / 1126 us with it, 650 / 806 / 895 / 1221 with the products of warps; width 1024: 519 / 669 / 738 / 786 and 506 / 654 / 749 / 832)
     // (fp32 ones of some more are faster in three parts, their depth shared by a cluster.  64 columns, us, gemm_narrow and gemm_split: 2048 rows 2048 deep 31 and 19, 448 rows
-    // 2048 deep 21 and 14, 777 rows 1024 deep 12 and 12)
+    // 2048 deep 21 and 14, 777 rows 1024 deep 12 and 12.  Error against 64 bits, depth 512 / 1024 / 2048: normal operands 15.6, 21.1, 29.4e-8 and 8.9, 10.3, 12.6e-8, all of one sign 6.0,
+    // 7.2, 9.1e-8 and 8.4, 9.2, 10.8e-8)
     if (!bf16 && P.M >= kNarrowMin && (long long)P.M * P.K >= 900000) {
       launch_split(S, epi, P, 1, 0, st);
       S->launches++;
