@@ -1794,17 +1794,19 @@ static LinScanShape lin_scan_shape(int H, int P, bool extra, int CW) {
 // walks): what this takes is 0.3 % above the fastest on average, once 4 % above lin_scan.  2048 tokens, lin_scan and lin_mma: 64 heads of 64 channels 312 and 222 (two segments), 16 of
 // 128 186 and 116 (four), 16 of 128 with the normaliser, whose column takes a third CTA, 188 and 152 (three), 4 of 64 with 64 entries 134 and 46 (eight), 64 of 128 with the normaliser 637
 // and 532 (three); 600 tokens, 16 of 64 with 64 entries 46 and 23; 100 tokens, 8 of 128 with 128 entries 17 and 21: not taken; 48 tokens, 32 of 64 with 64 entries 12.8 and 10.1 (one walk).
+// In chained steps launches hide under one another: a set of numbers of their own, over 256 walks of 33 to 256 tokens between the kernels around them 0.6 % above the fastest on average.
 static int lin_mma_segments(const float* q, const float* k, int ldq, int hs, const float* v, int ldv, int T, int H, int N, int P, bool extra, const float* seg) {
   auto al = [](const float* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
   if (!seg || (N != 64 && N != 128) || P % 4 || ldq % 4 || hs % 4 || ldv % 4 || !al(q) || !al(k) || !al(v)) return 0;
   const int nb = (T + kLinBlk - 1) / kLinBlk, ctas = H * ((P + (extra ? 1 : 0) + kLmCh - 1) / kLmCh);
   const LinScanShape scan = lin_scan_shape(H, P, extra, N == 64 ? 4 : 2);
-  const double full = N == 128 ? 1.95 : 1.25, ends = N == 128 ? 1.1 : 0.6, w = scan.warps * ((scan.ctas + g_sm_count - 1) / g_sm_count);
-  double best = 8 + nb * std::max(0.8 + 0.075 * w, 0.15 * w);
+  const bool chained = chain_step;
+  const double full = N == 128 ? (chained ? 2.1 : 1.95) : chained ? 1.15 : 1.25, ends = N == 128 ? 1.1 : 0.6, w = scan.warps * ((scan.ctas + g_sm_count - 1) / g_sm_count);
+  double best = (chained ? 7 : 8) + nb * std::max(0.8 + 0.075 * w, 0.15 * w);
   int segs = 0;
   for (int n = 1; n <= kLmSegs; n++) {
     const int per = (nb + n - 1) / n, rounds = (ctas * n + g_sm_count - 1) / g_sm_count, first = (ctas * (n - 1) + g_sm_count - 1) / g_sm_count;
-    const double cost = per * (rounds * full + first * ends) + (n > 1 ? 11 + 0.8 * n : 6);
+    const double cost = per * (rounds * full + first * ends) + (chained ? (n > 1 ? 9 + 0.5 * n : 5) : n > 1 ? 11 + 0.8 * n : 6);
     if ((nb + per - 1) / per == n && cost < best) { best = cost; segs = n; }
   }
   return segs;
@@ -1835,6 +1837,7 @@ static void launch_lin_scan(bool delta, const float* q, const float* k, int ldq,
   const int PB = warps * CW;
   const dim3 grid((unsigned)H, (unsigned)((P + (nst ? 1 : 0) + PB - 1) / PB));
   const size_t smem = lin_scan_smem(4 * TPC * RQ, PB, warps, CW);
+  if (!delta) plain_next = true;   // (its CTAs, few and long, would double up on the SMs that the kernel ahead leaves first: 200 tokens of 16 heads of 64 channels and entries with the normaliser 31 and 27 us)
 #define DSK_LSCAN(D, A, B, C) launch_next(lin_scan<D, A, B, C>, grid, 32 * (warps + kLinStage), smem, st)(q, k, ldq, hs, rep, v, ldv, rec, state, out, ldo, T, H, N, P, PB, nst, den, sn, sp)
 #define DSK_LSCANS(D) do { if (N > 128) DSK_LSCAN(D, 32, 2, 4); else if (CPT == 2) { if (N <= 32) DSK_LSCAN(D, 8, 1, 2); else if (N <= 64) DSK_LSCAN(D, 16, 1, 2); else DSK_LSCAN(D, 32, 1, 2); } \
   else { if (N <= 32) DSK_LSCAN(D, 8, 1, 4); else if (N <= 64) DSK_LSCAN(D, 16, 1, 4); else DSK_LSCAN(D, 32, 1, 4); } } while (0)
