@@ -581,7 +581,7 @@ class _Results:
     """float32 arrays in pinned host memory for a model's logits: the GPU writes them directly (a pageable array takes a second copy, some 100 us a
     megabyte, and its fresh pages as much again).  One piece of memory, taken when the model is finished; an array's part comes back when the last reference to it
     is gone.  Results that find no room (of a program that keeps them all, or larger ones) and small ones are ordinary arrays.  Measured: 300 rows of 2000 behind a prompt
-    of 777 tokens 1030 us as zeroed pageable arrays, 953 as empty ones, 802 here; 8 MB take 1 to 2 ms when the model is finished (taken by the results that need
+    of 777 tokens 1030 us as zeroed pageable arrays, 953 as empty ones, 802 here; 8 MB take 1 to 3 ms when the model is finished (taken by the results that need
     them instead, first passes were 0.4 to 2.6 ms longer)."""
     LEAST, UNIT, MOST = 64 << 10, 4 << 10, 8 << 20
 
